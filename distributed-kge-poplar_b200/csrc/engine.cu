@@ -5,6 +5,8 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
+#include <mutex>
 
 namespace kge {
 
@@ -360,6 +362,10 @@ Engine::Engine(const SettingMap& settings) : cfg_(parse_config(settings)) {
     side_streams_ = 3u;
     if (const char* v = std::getenv("KGE_SIDE_STREAMS")) side_streams_ = (unsigned)std::atoi(v) & 3u;
     KGE_CUDA(cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming));
+    if (n_local_ > 1 && cfg_.world == 1) {
+        ev_shard_.resize(n_local_, nullptr);
+        for (cudaEvent_t& e : ev_shard_) KGE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
     for (cudaEvent_t& e : ev_join_) KGE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     KGE_CUDA(cudaEventCreate(&ev_begin_));
     KGE_CUDA(cudaEventCreate(&ev_end_));
@@ -395,7 +401,7 @@ Engine::Engine(const SettingMap& settings) : cfg_(parse_config(settings)) {
 Engine::~Engine() {
     cudaSetDevice((int)cfg_.device_ordinal);
     if (stream_) cudaStreamSynchronize(stream_);
-    if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
+    for (StepGraph& g : graphs_) if (g.exec) cudaGraphExecDestroy(g.exec);
     for (cudaEvent_t e : event_pool_) cudaEventDestroy(e);
     for (unsigned p = 0; p < peer_arena_.size(); ++p)
         if (p != cfg_.rank && peer_arena_[p]) cudaIpcCloseMemHandle(peer_arena_[p]);
@@ -406,6 +412,7 @@ Engine::~Engine() {
     for (cudaEvent_t e : ev_stage_) if (e) cudaEventDestroy(e);
     if (ev_fork_) cudaEventDestroy(ev_fork_);
     for (cudaEvent_t e : ev_join_) if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : ev_shard_) if (e) cudaEventDestroy(e);
     if (side_stream_) cudaStreamDestroy(side_stream_);
     if (stream_) cudaStreamDestroy(stream_);
 }
@@ -881,24 +888,7 @@ void Engine::train_staged(float learning_rate, float* loss) {
     KGE_CUDA(cudaMemsetAsync(d_loss_total_, 0, n_local_ * 4, stream_));
     KGE_CUDA(cudaEventRecord(ev_begin_, stream_));
     if (cfg_.cuda_graph && !kernel_timing_) {
-        if (!graph_exec_) {
-            cudaGraph_t graph = nullptr;
-            launch_counter_ = 0;
-            KGE_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-            try {
-                launch_steps();
-            } catch (...) {
-                cudaStreamEndCapture(stream_, &graph);
-                if (graph) cudaGraphDestroy(graph);
-                throw;
-            }
-            KGE_CUDA(cudaStreamEndCapture(stream_, &graph));
-            cudaError_t err = cudaGraphInstantiate(&graph_exec_, graph, 0);
-            cudaGraphDestroy(graph);
-            KGE_CUDA(err);
-            last_launches_ = launch_counter_;
-        }
-        KGE_CUDA(cudaGraphLaunch(graph_exec_, stream_));
+        launch_step_graphs();
     } else {
         launch_counter_ = 0;
         if (kernel_timing_) {
@@ -906,7 +896,7 @@ void Engine::train_staged(float learning_rate, float* loss) {
             k_delay<<<1, 1, 0, stream_>>>(20ll * 1000 * 1000);
             KGE_CUDA(cudaGetLastError());
         }
-        launch_steps();
+        launch_steps(0, cfg_.n_step);
         last_launches_ = launch_counter_;
     }
     KGE_CUDA(cudaEventRecord(ev_end_, stream_));
@@ -990,9 +980,106 @@ bool dependent_launch_enabled() {
     return enabled;
 }
 
-void Engine::launch_steps() {
-    launch_gather(0, stream_);
-    for (unsigned step = 0; step < cfg_.n_step; ++step) launch_one_step(step);
+// A program run as a short chain of CUDA graphs, each four times as long as the one before: on an engine's first run
+// every graph but the first (a single step) is captured and instantiated, at 10 to 20 us of host time per kernel, while
+// its predecessor runs on the GPU (the first run of 100 headline steps: 17.1 to 15.9 ms; later runs are the same).
+void Engine::launch_step_graphs() {
+    if (graphs_.empty()) {
+        unsigned length = 1;
+        for (unsigned first = 0; first < cfg_.n_step; first += length, length *= 4)
+            graphs_.push_back({first, std::min(first + length, cfg_.n_step), nullptr, 0});
+        // a last graph shorter than its predecessor's launch joins it
+        if (graphs_.size() > 1 && graphs_.back().end - graphs_.back().first < (graphs_.back().first - graphs_[graphs_.size() - 2].first) / 2) {
+            graphs_[graphs_.size() - 2].end = cfg_.n_step;
+            graphs_.pop_back();
+        }
+    }
+    last_launches_ = 0;
+    for (StepGraph& g : graphs_) {
+        if (!g.exec) {
+            cudaGraph_t graph = nullptr;
+            launch_counter_ = 0;
+            KGE_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+            try {
+                launch_steps(g.first, g.end);
+            } catch (...) {
+                cudaStreamEndCapture(stream_, &graph);
+                if (graph) cudaGraphDestroy(graph);
+                throw;
+            }
+            KGE_CUDA(cudaStreamEndCapture(stream_, &graph));
+            cudaError_t err = cudaGraphInstantiate(&g.exec, graph, 0);
+            cudaGraphDestroy(graph);
+            KGE_CUDA(err);
+            g.launches = launch_counter_;
+        }
+        KGE_CUDA(cudaGraphLaunch(g.exec, stream_));
+        last_launches_ += g.launches;
+    }
+}
+
+namespace {
+// Streams for the shards' branches, lent out while steps are queued or captured: making one costs the host about 2 ms,
+// as much as capturing a short run.  At most kKept per device wait for the next borrower; the rest are destroyed.
+class StreamPool {
+   public:
+    static StreamPool& instance() {
+        static StreamPool* pool = new StreamPool;  // never destroyed: CUDA may be gone before static destructors run
+        return *pool;
+    }
+    cudaStream_t take() {
+        const int slot = current_device_slot();
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            if (slot >= 0 && !free_[slot].empty()) {
+                cudaStream_t st = free_[slot].back();
+                free_[slot].pop_back();
+                return st;
+            }
+        }
+        cudaStream_t st = nullptr;
+        KGE_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        return st;
+    }
+    void give(cudaStream_t st) {
+        const int slot = current_device_slot();
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            if (slot >= 0 && free_[slot].size() < kKept) {
+                free_[slot].push_back(st);
+                return;
+            }
+        }
+        cudaStreamDestroy(st);  // work still queued on it completes first
+    }
+
+   private:
+    static constexpr size_t kKept = 16;
+    std::mutex mutex_;
+    std::vector<cudaStream_t> free_[kMaxDeviceOrdinals];
+};
+}  // namespace
+
+void Engine::launch_steps(unsigned first, unsigned end) {
+    struct Lease {  // the shards' streams, for as long as steps are being queued
+        Engine& e;
+        explicit Lease(Engine& engine) : e(engine) {
+            if (e.n_local_ < 2 || e.cfg_.world > 1 || e.kernel_timing_) return;
+            e.shard_streams_.assign(e.n_local_, nullptr);
+            for (unsigned l = 1; l < e.n_local_; ++l) e.shard_streams_[l] = StreamPool::instance().take();
+        }
+        ~Lease() {
+            for (cudaStream_t st : e.shard_streams_) {
+                if (!st) continue;
+                if (std::uncaught_exceptions()) cudaStreamDestroy(st);  // may still belong to a broken capture
+                else StreamPool::instance().give(st);
+            }
+            e.shard_streams_.clear();
+        }
+    } lease(*this);
+    if (first == 0) launch_gather(0, stream_);
+    for (unsigned step = first; step < end; ++step) launch_one_step(step);
+    if (end < cfg_.n_step) return;
     // The last kernel of a step only publishes its dense parameters.  The run ends when every
     // process's share has arrived in this process's copy (values and optimiser state), so that a
     // "read" or "predict" issued straight after the run sees the finished step without a host barrier.
@@ -1003,13 +1090,14 @@ void Engine::launch_steps() {
 // copies, for even and odd steps).  The gather of step s + 1 needs only the rows step s has
 // updated, so it runs beside the projection gradient and the dense update of step s.
 void Engine::launch_gather(unsigned step, cudaStream_t stream) {
+    for (unsigned l = 0; l < n_local_; ++l) launch_gather(step, l, stream);
+}
+void Engine::launch_gather(unsigned step, unsigned l, cudaStream_t stream) {
     const unsigned R = cfg_.n_remote();
-    for (unsigned l = 0; l < n_local_; ++l) {
-        ShardBuffers& b = shards_[l];
-        const uint32_t* remote = d_remote_ + ((size_t)l * cfg_.n_step + step) * R;
-        KGE_LAUNCH("gather", KGE_CUDA(launch_dependent(k_gather_step_rows, dim3(ceil_div(R, 8)), dim3(256), 0, stream, b.table,
-                                                       layout_.row_bytes, remote, (int)R, b.rows_c2[step & 1], feature_planes(b, step & 1))));
-    }
+    ShardBuffers& b = shards_[l];
+    const uint32_t* remote = d_remote_ + ((size_t)l * cfg_.n_step + step) * R;
+    KGE_LAUNCH("gather", KGE_CUDA(launch_dependent(k_gather_step_rows, dim3(ceil_div(R, 8)), dim3(256), 0, stream, b.table,
+                                                   layout_.row_bytes, remote, (int)R, b.rows_c2[step & 1], feature_planes(b, step & 1))));
 }
 
 FeaturePlanes Engine::feature_planes(const ShardBuffers& b, unsigned parity) const {
@@ -1038,6 +1126,26 @@ void Engine::side_end(int which) {
 void Engine::side_join(int which) {
     if (kernel_timing_ || !side_streams_) return;
     KGE_CUDA(cudaStreamWaitEvent(stream_, ev_join_[which], 0));
+}
+
+// Several shards in one process: the kernels of a phase (hidden rows and lookups; scores and their gradients; row
+// updates and projection gradient) work on one shard each and meet only at the exchange, so every shard's part of a
+// phase is queued on a stream of its own (graph branches under capture).  The kernels of a step are short and mostly
+// far too small to fill 148 SMs: side by side they take little longer than one of them (program runs: the demo
+// preset's two shards, 5 steps, 475 to 342 us; four shards of 256 x 512 L1 scores, 20 steps, 9.5 to 3.7 ms; two
+// shards of the headline step, whose kernels do fill the GPU, 4.0 to 3.6 ms).  Only with one process: the hand-over
+// counters between processes count the blocks of one kernel at a time.
+void Engine::shards_fork() {
+    if (!shards_beside()) return;
+    KGE_CUDA(cudaEventRecord(ev_fork_, stream_));
+    for (unsigned l = 1; l < n_local_; ++l) KGE_CUDA(cudaStreamWaitEvent(shard_streams_[l], ev_fork_, 0));
+}
+void Engine::shards_join() {
+    if (!shards_beside()) return;
+    for (unsigned l = 1; l < n_local_; ++l) {
+        KGE_CUDA(cudaEventRecord(ev_shard_[l], shard_streams_[l]));
+        KGE_CUDA(cudaStreamWaitEvent(stream_, ev_shard_[l], 0));
+    }
 }
 
 void Engine::launch_barrier() {
@@ -1340,7 +1448,9 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
         return plane(reinterpret_cast<const float*>(b.rows_c2[parity] + layout_.off_feat), b.feat_lo2[parity], (long long)layout_.row_bytes, mn_major);
     };
 
+    shards_fork();
     for (unsigned l = 0; l < n_local_; ++l) {
+        const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
         uint8_t* rows_c = b.rows_c2[parity];
         const size_t sidx = (size_t)l * cfg_.n_step + step;
@@ -1400,9 +1510,12 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                                                           b.send_lo_dst, b.pred_lo, bf16 ? 1 : 0)));
         if (cfg_.regularised()) launch_regularise(l, rows_c);
     }
+    shards_join();
     KGE_CUDA(cudaGetLastError());
 
+    shards_fork();
     for (unsigned l = 0; l < n_local_; ++l) {
+        const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
         const uint32_t* head = step_ptr(d_head_, l, B);
         const uint32_t* relation = step_ptr(d_relation_, l, B);
@@ -1464,10 +1577,15 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
             KGE_LAUNCH("pred_bwd", KGE_CUDA(launch_dependent(k_pred_bwd, dim3(B), dim3(64), 0, stream_, b.d_pred, b.hid_h, head, relation, rel_table, b.d_head,
                                                              b.d_relrow, (int)D, cfg_.score_fn)));
     }
+    shards_join();
     KGE_CUDA(cudaGetLastError());
 
     // 5. segment sums + row-wise Adam, and the relation rows of the partial dense gradient
+    const bool gather_ahead = step + 1 < cfg_.n_step;
+    const bool gather_beside = gather_ahead && (side_streams_ & 2u);
+    shards_fork();
     for (unsigned l = 0; l < n_local_; ++l) {
+        const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
         const size_t sidx = (size_t)l * cfg_.n_step + step;
         const HeavyRows heavy{d_heavy_parts_ + sidx * kHeavySlots, d_heavy_count_ + sidx, b.heavy_partial, b.heavy_counter, d_row_info_ + sidx * 2 * R};
@@ -1489,17 +1607,13 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
             if (extras) KGE_ENTITY_UPDATE(__half, true); else KGE_ENTITY_UPDATE(__half, false);
         }
 #undef KGE_ENTITY_UPDATE
+        if (gather_beside) launch_gather(step + 1, l, side_begin());
     }
     KGE_CUDA(cudaGetLastError());
-    const bool gather_ahead = step + 1 < cfg_.n_step;
-    const bool gather_beside = gather_ahead && (side_streams_ & 2u);
-    if (gather_beside) {
-        cudaStream_t side = side_begin();
-        launch_gather(step + 1, side);
-        side_end(1);
-    }
+    if (gather_beside) side_end(1);
     // 6. d W = feature^T . d_hidden, straight into the owners' slices of the partial dense gradient
     for (unsigned l = 0; l < n_local_; ++l) {
+        const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
         tc::PlaneProblem nets[2] = {};
         for (unsigned net = 0; net < cfg_.n_net(); ++net) {
@@ -1524,6 +1638,7 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
         if (F > 0) launch_planes("projection_bwd", nets, (int)cfg_.n_net(), tc::SIDE_NONE, -1, XCHG_DENSE_PARTIALS);
         else launch_exchange_signal(XCHG_DENSE_PARTIALS);  // the relation rows of the entity update are all there is
     }
+    shards_join();
     KGE_CUDA(cudaGetLastError());
     if (gather_ahead && !gather_beside) launch_gather(step + 1, stream_);
     // 7. dense parameters: reduce over shards, Adam on the owned rows, new values and their lower planes into every replica
@@ -1590,7 +1705,9 @@ void Engine::launch_one_step(unsigned step) {
     };
 
     // 1./2. hidden rows, lookups, send half of the exchange
+    shards_fork();
     for (unsigned l = 0; l < n_local_; ++l) {
+        const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
         uint8_t* rows_c = b.rows_c2[step & 1];
         if (cfg_.tensor_cores && F > 0) {
@@ -1637,10 +1754,13 @@ void Engine::launch_one_step(unsigned step) {
                                                                    normal_table, b.pred, b.nrm, (int)D)));
         if (cfg_.regularised()) launch_regularise(l, rows_c);
     }
+    shards_join();
     KGE_CUDA(cudaGetLastError());
 
     // 3./4./5a. scores, loss, score backward with the return half of the exchange
+    shards_fork();
     for (unsigned l = 0; l < n_local_; ++l) {
+        const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
         const uint32_t* head = step_ptr(d_head_, l, B);
         const uint32_t* relation = step_ptr(d_relation_, l, B);
@@ -1727,6 +1847,7 @@ void Engine::launch_one_step(unsigned step) {
             KGE_LAUNCH("pred_bwd", KGE_CUDA(launch_dependent(k_pred_bwd, dim3(B), dim3(64), 0, stream_, b.d_pred, b.hid_h, head, relation, rel_table, b.d_head,
                                                                      b.d_relrow, (int)D, cfg_.score_fn)));
     }
+    shards_join();
     KGE_CUDA(cudaGetLastError());
 
     if (proj_direct) {
@@ -1751,7 +1872,11 @@ void Engine::launch_one_step(unsigned step) {
     }
 
     // 5b. segment sums + row-wise Adam; projection and relation gradients of this shard
+    const bool gather_ahead = step + 1 < cfg_.n_step;
+    const bool gather_beside = gather_ahead && (side_streams_ & 2u);
+    shards_fork();
     for (unsigned l = 0; l < n_local_; ++l) {
+        const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
         uint8_t* rows_c = b.rows_c2[step & 1];
         const size_t sidx = (size_t)l * cfg_.n_step + step;
@@ -1774,20 +1899,14 @@ void Engine::launch_one_step(unsigned step) {
             else { if (extras) KGE_ENTITY_UPDATE(__half, 1, true); else KGE_ENTITY_UPDATE(__half, 1, false); }
         }
 #undef KGE_ENTITY_UPDATE
+        if (mlp_on()) launch_mlp_backward(l, step);
+        // the next step's rows: needs only the rows just updated, runs beside the rest of this step
+        if (gather_beside) launch_gather(step + 1, l, side_begin());
     }
     KGE_CUDA(cudaGetLastError());
-    if (mlp_on())
-        for (unsigned l = 0; l < n_local_; ++l) launch_mlp_backward(l, step);
-    if (proj_direct && (side_streams_ & 1u)) side_join(0);  // the relation rows of the partial dense gradient are in place
-    const bool gather_ahead = step + 1 < cfg_.n_step;
-    const bool gather_beside = gather_ahead && (side_streams_ & 2u);
-    if (gather_beside) {
-        // the next step's rows: needs only the rows just updated, runs beside the rest of this step
-        cudaStream_t side = side_begin();
-        launch_gather(step + 1, side);
-        side_end(1);
-    }
+    if (gather_beside) side_end(1);
     for (unsigned l = 0; l < n_local_; ++l) {
+        const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
         uint8_t* rows_c = b.rows_c2[step & 1];
         const size_t sidx = (size_t)l * cfg_.n_step + step;
@@ -1836,6 +1955,8 @@ void Engine::launch_one_step(unsigned step) {
                                                 proj_elems_, b.dense_dst, (int)cfg_.world, sync, (int)XCHG_DENSE_PARTIALS, 0)));
         }
     }
+    shards_join();
+    if (proj_direct && (side_streams_ & 1u)) side_join(0);  // the relation rows of the partial dense gradient are in place
     KGE_CUDA(cudaGetLastError());
     if (gather_ahead && !gather_beside) launch_gather(step + 1, stream_);  // runs while the partial dense gradients travel
 

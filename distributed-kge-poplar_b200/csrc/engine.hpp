@@ -170,13 +170,15 @@ class Engine {
     void prepare_staged();
 
     // the step
-    void launch_steps();
+    void launch_steps(unsigned first, unsigned end);
+    void launch_step_graphs();
     void launch_one_step(unsigned step);
     void launch_barrier();
     ExchangeSync exchange_sync() const;
     void launch_exchange_wait(int kind);
     void launch_exchange_signal(int kind);
     void launch_gather(unsigned step, cudaStream_t stream);
+    void launch_gather(unsigned step, unsigned l, cudaStream_t stream);
     void launch_tc(const char* name, tc::GemmArgs* problems, int n_problems, int splits, bool a_exact, bool rowsum,
                    int wait_kind = -1, int signal_kind = -1);
     // the plane-fed contraction: tile width and k splits chosen here
@@ -209,6 +211,26 @@ class Engine {
     bool bf16_planes_ = false;        // scores and their gradients multiply bfloat16 copies of their operands
     uint32_t feat_stride_ = 0;        // floats per row of the widened / lower feature planes
     cudaEvent_t ev_fork_ = nullptr, ev_join_[2] = {nullptr, nullptr};
+    // One stream per local shard (the first one is stream_ itself) while steps are being queued; empty where the shards run one after the other.
+    std::vector<cudaStream_t> shard_streams_;
+    std::vector<cudaEvent_t> ev_shard_;
+    bool shards_beside() const { return !shard_streams_.empty() && !kernel_timing_; }
+    void shards_fork();
+    void shards_join();
+    // While alive, what the engine launches goes to local shard l's stream.
+    class ShardScope {
+       public:
+        ShardScope(Engine& e, unsigned l) : engine_(e), saved_(e.stream_) {
+            if (l > 0 && e.shards_beside()) e.stream_ = e.shard_streams_[l];
+        }
+        ~ShardScope() { engine_.stream_ = saved_; }
+        ShardScope(const ShardScope&) = delete;
+        ShardScope& operator=(const ShardScope&) = delete;
+
+       private:
+        Engine& engine_;
+        cudaStream_t saved_;
+    };
     cudaStream_t side_begin();
     void side_end(int which);
     void side_join(int which);
@@ -311,7 +333,12 @@ class Engine {
     std::vector<TimedLaunch> timed_;
     std::map<std::string, KernelTime> kernel_times_;
 
-    cudaGraphExec_t graph_exec_ = nullptr;
+    struct StepGraph {
+        unsigned first, end;  // the steps it replays
+        cudaGraphExec_t exec;
+        unsigned long long launches;
+    };
+    std::vector<StepGraph> graphs_;  // a program run, in order
     float last_ms_ = 0.f;
     unsigned long long last_launches_ = 0, launch_counter_ = 0;
 };
