@@ -406,6 +406,7 @@ Engine::~Engine() {
     for (unsigned p = 0; p < peer_arena_.size(); ++p)
         if (p != cfg_.rank && peer_arena_[p]) cudaIpcCloseMemHandle(peer_arena_[p]);
     for (void* p : allocations_) cudaFree(p);
+    for (cudaEvent_t e : ev_io_) if (e) cudaEventDestroy(e);
     if (pinned_) cudaFreeHost(pinned_);
     if (ev_begin_) cudaEventDestroy(ev_begin_);
     if (ev_end_) cudaEventDestroy(ev_end_);
@@ -430,11 +431,12 @@ void Engine::allocate() {
     dense_lo_ = (float*)(arena_ + arena_offset_dense(3));
 
     shards_.resize(n_local_);
-    const size_t table_bytes = (size_t)cfg_.n_entity * layout_.row_bytes;
+    table_stride_ = round_up((size_t)cfg_.n_entity * layout_.row_bytes, 256);
+    uint8_t* tables = (uint8_t*)device_alloc(n_local_ * table_stride_);
+    KGE_CUDA(cudaMemset(tables, 0, n_local_ * table_stride_));
     for (unsigned l = 0; l < n_local_; ++l) {
         ShardBuffers& b = shards_[l];
-        b.table = (uint8_t*)device_alloc(table_bytes);
-        KGE_CUDA(cudaMemset(b.table, 0, table_bytes));
+        b.table = tables + l * table_stride_;
         for (uint8_t*& rows : b.rows_c2) rows = (uint8_t*)device_alloc((size_t)R * layout_.row_bytes);
         b.hid_h = (float*)device_alloc((size_t)R * D * 4);
         b.hid_t = two_nets || dropout_on() ? (float*)device_alloc((size_t)R * D * 4) : b.hid_h;  // dropout: each call has its own mask
@@ -506,10 +508,7 @@ void Engine::allocate() {
         d_xchg_trace_ = (unsigned long long*)device_alloc(bytes);
         KGE_CUDA(cudaMemset(d_xchg_trace_, 0, bytes));
     }
-    d_tc_status_ = (unsigned*)device_alloc(2 * sizeof(unsigned));  // read back together after every run
-    d_status_ = d_tc_status_ + 1;
     KGE_CUDA(cudaMemset(d_epoch_, 0, sizeof(unsigned)));
-    KGE_CUDA(cudaMemset(d_tc_status_, 0, 2 * sizeof(unsigned)));
     {
         // room for the two problems of the largest paired launch, kTcMaxSplits partial tiles each
         const size_t per_problem = std::max<size_t>({(size_t)R * D, (size_t)(std::max(B, T)) * D, (size_t)cfg_.f * D, (size_t)B * T});
@@ -523,11 +522,29 @@ void Engine::allocate() {
     d_replicas_lo_ = (float**)device_alloc(sizeof(float*) * cfg_.world);
 
     const size_t steps = (size_t)n_local_ * cfg_.n_step;
-    d_remote_ = (uint32_t*)device_alloc(steps * R * 4);
-    d_a2a_ = (uint32_t*)device_alloc(steps * T * 4);
-    d_head_ = (uint32_t*)device_alloc(steps * B * 4);
-    d_relation_ = (uint32_t*)device_alloc(steps * B * 4);
-    d_tail_ = (uint32_t*)device_alloc(steps * B * 4);
+    {
+        size_t at = 0;
+        const size_t stream_words[5] = {steps * R, steps * T, steps * B, steps * B, steps * B};
+        for (int i = 0; i < 5; ++i) stage_at_[i] = at, at += round_up(stream_words[i], 4);
+        keys_at_ = at;
+        sizes_at_ = keys_at_ + cfg_.n_step;
+        loss_at_ = sizes_at_ + cfg_.n_step;
+        status_at_ = loss_at_ + n_local_;
+        run_words_ = status_at_ + 2;
+        d_run_ = (uint32_t*)device_alloc(run_words_ * 4);
+        KGE_CUDA(cudaMemset(d_run_ + loss_at_, 0, (run_words_ - loss_at_) * 4));
+        KGE_CUDA(cudaMallocHost((void**)&pinned_, run_words_ * 4));
+    }
+    d_remote_ = d_run_ + stage_at_[0];
+    d_a2a_ = d_run_ + stage_at_[1];
+    d_head_ = d_run_ + stage_at_[2];
+    d_relation_ = d_run_ + stage_at_[3];
+    d_tail_ = d_run_ + stage_at_[4];
+    d_step_key_ = d_run_ + keys_at_;
+    d_step_size_ = reinterpret_cast<float*>(d_run_ + sizes_at_);
+    d_loss_total_ = reinterpret_cast<float*>(d_run_ + loss_at_);
+    d_tc_status_ = d_run_ + status_at_;
+    d_status_ = d_tc_status_ + 1;
     d_ent_perm_ = (uint32_t*)device_alloc(steps * (B + T) * 4);
     d_ent_off_ = (uint32_t*)device_alloc(steps * (R + 1) * 4);
     d_rel_perm_ = (uint32_t*)device_alloc(steps * B * 4);
@@ -537,9 +554,6 @@ void Engine::allocate() {
     d_row_info_ = (uint4*)device_alloc(steps * 2 * R * sizeof(uint4));
     d_heavy_count_ = (uint32_t*)device_alloc(steps * 4);
     KGE_CUDA(cudaMemset(d_heavy_count_, 0, steps * 4));
-    d_step_size_ = (float*)device_alloc(cfg_.n_step * 4);
-    d_step_key_ = (uint32_t*)device_alloc(cfg_.n_step * 4);
-    d_loss_total_ = (float*)device_alloc(n_local_ * 4);
     d_loss_last_ = (float*)device_alloc(n_local_ * 4);
     d_loss_counter_ = (unsigned*)device_alloc(n_local_ * sizeof(unsigned));
     KGE_CUDA(cudaMemset(d_loss_counter_, 0, n_local_ * sizeof(unsigned)));
@@ -552,10 +566,6 @@ void Engine::allocate() {
 
     const size_t rw = (size_t)n_local_ * cfg_.rw_batch;
     d_rw_idx_ = (uint32_t*)device_alloc(std::max<size_t>(rw, (size_t)n_local_ * cfg_.predict_hr * 2) * 4);
-    d_rw_data_ = (uint8_t*)device_alloc(rw * cfg_.row_width() * 4);
-
-    pinned_bytes_ = steps * ((size_t)R + T + 3 * B) * 4 + 2 * cfg_.n_step * 4 + 256;  // index streams | step keys | step sizes | loss
-    KGE_CUDA(cudaMallocHost((void**)&pinned_, pinned_bytes_));
     KGE_CUDA(cudaDeviceSynchronize());
 }
 
@@ -701,6 +711,8 @@ void Engine::run(const std::string& command, std::vector<HostArray>& arrays, con
     if (command == "read_entity") return cmd_read_entity(arrays);
     if (command == "write_entity") return cmd_write_entity(arrays, false);
     if (command == "write_entity_rows") return cmd_write_entity(arrays, true);
+    if (command == "read_entity_range") return cmd_entity_range(arrays, true);
+    if (command == "write_entity_range") return cmd_entity_range(arrays, false);
     if (command == "initialise_entities") return cmd_initialise_entities();
     if (command == "entity_layout") {
         // `layout` u32 [4]: bytes of a stored row, rows per shard, local shards, the first local shard
@@ -721,11 +733,24 @@ void Engine::run(const std::string& command, std::vector<HostArray>& arrays, con
 void Engine::cmd_train_step_loop(std::vector<HostArray>& arrays) {
     HostArray& lr = find_array(arrays, "learning_rate", KGE_F32, {n_local_});
     HostArray& loss = find_array(arrays, "loss", KGE_F32, {n_local_});
-    stage_batch(arrays);
+    stage_batch(arrays, static_cast<const float*>(lr.data));
     train_staged(static_cast<const float*>(lr.data)[0], static_cast<float*>(loss.data));
 }
 
-void Engine::stage_batch(std::vector<HostArray>& arrays) {
+// The words of the coming run that change with it: Adam step sizes (src/fructose/frnn.cpp:42-59, in fp32), the steps'
+// numbers, and zeros for the loss totals.
+void Engine::write_run_words(float learning_rate) {
+    uint32_t* keys = pinned_ + keys_at_;
+    float* sizes = reinterpret_cast<float*>(pinned_ + sizes_at_);
+    for (unsigned i = 0; i < cfg_.n_step; ++i) {
+        const float t = (float)(step_ + 1 + i);
+        keys[i] = (uint32_t)(step_ + 1 + i);
+        sizes[i] = (std::sqrt(1.0f - std::pow(cfg_.beta_v, t)) / (1.0f - std::pow(cfg_.beta_m, t))) * learning_rate;
+    }
+    std::memset(pinned_ + loss_at_, 0, n_local_ * 4);
+}
+
+void Engine::stage_batch(std::vector<HostArray>& arrays, const float* learning_rate) {
     KGE_CUDA(cudaSetDevice((int)cfg_.device_ordinal));
     const size_t n = n_local_, S = cfg_.n_step, B = cfg_.batch_size, T = cfg_.n_tail(), R = cfg_.n_remote();
     HostArray& remote = find_array(arrays, "remote", KGE_U32, {n, S, R});
@@ -742,33 +767,33 @@ void Engine::stage_batch(std::vector<HostArray>& arrays) {
                 fail(KGE_INVALID_ARGUMENT, msg() << "'" << a.name << "' holds index " << p[i] << " at position " << i
                                                  << ", which is not below " << what << " (" << limit << ")");
     };
-    // One pass per stream: copy into the pinned buffer and take the maximum (a loop without an exit,
-    // which the compiler vectorises); only a stream with a bad index is walked again for its position.
-    // A batch that fails a check is not staged: the engine refuses to train until one passes all five.
+    // One pass per stream copies into the pinned buffer and takes the maximum; only a stream with a bad index is
+    // walked again for its position.  A batch that fails a check is not staged: the engine refuses to train until one
+    // passes all five.
     staged_ = false;
-    KGE_CUDA(cudaStreamSynchronize(stream_));  // the pinned buffer may still be in flight
-    uint8_t* stage = pinned_;
-    struct Upload { const HostArray* a; uint32_t* dst; uint32_t limit; const char* what; };
-    const Upload uploads[5] = {{&remote, d_remote_, cfg_.n_entity, "model.n_entity"},
-                               {&a2a, d_a2a_, (uint32_t)R, "the number of gathered rows"},
-                               {&head, d_head_, (uint32_t)R, "the number of gathered rows"},
-                               {&relation, d_relation_, cfg_.n_relation_type, "model.n_relation_type"},
-                               {&tail, d_tail_, (uint32_t)T, "n_shard * a2a_size"}};
-    for (const Upload& u : uploads) {
-        const uint32_t* __restrict__ src = static_cast<const uint32_t*>(u.a->data);
-        uint32_t* __restrict__ out = reinterpret_cast<uint32_t*>(stage);
+    run_words_uploaded_ = false;
+    if (uploads_pending_) KGE_CUDA(cudaStreamSynchronize(stream_));  // the pinned buffer may still be in flight
+    uploads_pending_ = true;
+    struct Upload { const HostArray* a; uint32_t limit; const char* what; };
+    const Upload uploads[5] = {{&remote, cfg_.n_entity, "model.n_entity"}, {&a2a, (uint32_t)R, "the number of gathered rows"},
+                               {&head, (uint32_t)R, "the number of gathered rows"}, {&relation, cfg_.n_relation_type, "model.n_relation_type"},
+                               {&tail, (uint32_t)T, "n_shard * a2a_size"}};
+    // Up to 256 KB one transfer carries everything, the run's words included (a transfer costs the host 3 us, the link
+    // 1 us); above that each stream travels while the next one is copied and checked.
+    const bool one_transfer = keys_at_ * 4 <= 256 * 1024;
+    for (int i = 0; i < 5; ++i) {
+        const Upload& u = uploads[i];
+        uint32_t* out = pinned_ + stage_at_[i];
         const size_t count = u.a->count();
-        uint32_t highest = 0;
-        for (size_t i = 0; i < count; ++i) {
-            const uint32_t v = src[i];
-            out[i] = v;
-            highest = v > highest ? v : highest;
-        }
-        if (highest >= u.limit) check_below(*u.a, u.limit, u.what);
-        // the transfer of this stream runs while the next one is copied and checked
-        KGE_CUDA(cudaMemcpyAsync(u.dst, stage, count * 4, cudaMemcpyHostToDevice, stream_));
-        stage += count * 4;
+        if (copy_and_max(out, static_cast<const uint32_t*>(u.a->data), count) >= u.limit) check_below(*u.a, u.limit, u.what);
+        if (!one_transfer) KGE_CUDA(cudaMemcpyAsync(d_run_ + stage_at_[i], out, count * 4, cudaMemcpyHostToDevice, stream_));
     }
+    if (learning_rate) {
+        write_run_words(*learning_rate);
+        run_words_uploaded_ = true;
+    }
+    const size_t from = one_transfer ? 0 : keys_at_, to = learning_rate ? status_at_ : keys_at_;
+    if (to > from) KGE_CUDA(cudaMemcpyAsync(d_run_ + from, pinned_ + from, (to - from) * 4, cudaMemcpyHostToDevice, stream_));
     prepare_staged();
 }
 
@@ -853,6 +878,7 @@ void Engine::cmd_sample_batch(std::vector<HostArray>& arrays, bool train) {
         loss = &find_array(arrays, "loss", KGE_F32, {n});
     }
     KGE_CUDA(cudaSetDevice((int)cfg_.device_ordinal));
+    run_words_uploaded_ = false;
     sample_and_stage(static_cast<const uint32_t*>(seed.data)[0]);
     struct Stream { const char* name; uint32_t* device; std::vector<size_t> shape; };
     const Stream streams[5] = {{"remote", d_remote_, {n, S, R}}, {"a2a", d_a2a_, {n, S, cfg_.n_shard, cfg_.a2a_size}},
@@ -861,9 +887,8 @@ void Engine::cmd_sample_batch(std::vector<HostArray>& arrays, bool train) {
         for (HostArray& a : arrays)
             if (a.name == st.name) {
                 HostArray& out = find_array(arrays, st.name, KGE_U32, st.shape);
-                KGE_CUDA(cudaMemcpyAsync(out.data, st.device, out.count() * 4, cudaMemcpyDeviceToHost, stream_));
+                copy_out(out.data, st.device, out.count() * 4, out.count() * 4, 1);
             }
-    KGE_CUDA(cudaStreamSynchronize(stream_));
     if (train) train_staged(static_cast<const float*>(lr->data)[0], static_cast<float*>(loss->data));
 }
 
@@ -873,19 +898,13 @@ void Engine::train_staged(float learning_rate, float* loss) {
     require_usable();
     if (!staged_) fail(KGE_LOGIC_ERROR, "kge_train_staged called before kge_stage_batch");
     if (!connected_) fail(KGE_LOGIC_ERROR, "world_size > 1 but kge_comm_connect has not been called");
-    // Adam step sizes of the staged steps (src/fructose/frnn.cpp:42-59), in fp32.
-    float* sizes = reinterpret_cast<float*>(pinned_ + pinned_bytes_ - 256 - (size_t)cfg_.n_step * 4);
-    for (unsigned i = 0; i < cfg_.n_step; ++i) {
-        const float t = (float)(step_ + 1 + i);
-        sizes[i] = (std::sqrt(1.0f - std::pow(cfg_.beta_v, t)) / (1.0f - std::pow(cfg_.beta_m, t))) * learning_rate;
+    if (!run_words_uploaded_) {
+        if (uploads_pending_) KGE_CUDA(cudaStreamSynchronize(stream_));
+        uploads_pending_ = true;
+        write_run_words(learning_rate);
+        KGE_CUDA(cudaMemcpyAsync(d_run_ + keys_at_, pinned_ + keys_at_, (status_at_ - keys_at_) * 4, cudaMemcpyHostToDevice, stream_));
     }
-    KGE_CUDA(cudaMemcpyAsync(d_step_size_, sizes, (size_t)cfg_.n_step * 4, cudaMemcpyHostToDevice, stream_));
-    if (dropout_on()) {
-        uint32_t* keys = reinterpret_cast<uint32_t*>(sizes) - cfg_.n_step;
-        for (unsigned i = 0; i < cfg_.n_step; ++i) keys[i] = (uint32_t)(step_ + 1 + i);
-        KGE_CUDA(cudaMemcpyAsync(d_step_key_, keys, (size_t)cfg_.n_step * 4, cudaMemcpyHostToDevice, stream_));
-    }
-    KGE_CUDA(cudaMemsetAsync(d_loss_total_, 0, n_local_ * 4, stream_));
+    run_words_uploaded_ = false;
     KGE_CUDA(cudaEventRecord(ev_begin_, stream_));
     if (cfg_.cuda_graph && !kernel_timing_) {
         launch_step_graphs();
@@ -900,22 +919,19 @@ void Engine::train_staged(float learning_rate, float* loss) {
         last_launches_ = launch_counter_;
     }
     KGE_CUDA(cudaEventRecord(ev_end_, stream_));
-    float* host_loss = reinterpret_cast<float*>(pinned_ + pinned_bytes_ - 256);
-    if (loss)
-        KGE_CUDA(cudaMemcpyAsync(host_loss, d_loss_total_, n_local_ * 4, cudaMemcpyDeviceToHost, stream_));
+    // the loss totals and the status words are neighbours: one transfer brings both
+    KGE_CUDA(cudaMemcpyAsync(pinned_ + loss_at_, d_run_ + loss_at_, (run_words_ - loss_at_) * 4, cudaMemcpyDeviceToHost, stream_));
     KGE_CUDA(cudaStreamSynchronize(stream_));
-    KGE_CUDA(cudaEventElapsedTime(&last_ms_, ev_begin_, ev_end_));
-    if (stage_fresh_) {
-        // the sort-and-segment preparation belongs to the step (it is the backward of the row
-        // gather): its device time counts towards the first run of a staged batch
-        float stage_ms = 0.f;
-        KGE_CUDA(cudaEventElapsedTime(&stage_ms, ev_stage_[0], ev_stage_[1]));
-        last_ms_ += stage_ms;
-        stage_fresh_ = false;
-    }
+    uploads_pending_ = false;
+    ms_pending_ = true;
+    // the sort-and-segment preparation belongs to the step (it is the backward of the row
+    // gather): its device time counts towards the first run of a staged batch
+    ms_counts_stage_ = stage_fresh_;
+    stage_fresh_ = false;
     timing_collect();
     step_ += cfg_.n_step;
-    check_device_status();
+    raise_device_status(pinned_ + status_at_);
+    const float* host_loss = reinterpret_cast<const float*>(pinned_ + loss_at_);
     if (loss)
         for (unsigned l = 0; l < n_local_; ++l) loss[l] = host_loss[l] / (float)cfg_.n_step;
 }
@@ -924,9 +940,12 @@ void Engine::train_staged(float learning_rate, float* loss) {
 // up leaves this engine's kernels out of step with the other processes' (their hand-over epochs
 // disagree from then on), so the engine refuses further device commands: it must be rebuilt.
 void Engine::check_device_status() {
-    unsigned status[2] = {0, 0};  // [0] the tensor-core pipeline, [1] the hand-overs between processes
-    KGE_CUDA(cudaMemcpyAsync(status, d_tc_status_, sizeof(status), cudaMemcpyDeviceToHost, stream_));
+    KGE_CUDA(cudaMemcpyAsync(pinned_ + status_at_, d_tc_status_, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream_));
     KGE_CUDA(cudaStreamSynchronize(stream_));
+    raise_device_status(pinned_ + status_at_);
+}
+void Engine::raise_device_status(const unsigned* words) {
+    const unsigned status[2] = {words[0], words[1]};  // [0] the tensor-core pipeline, [1] the hand-overs between processes
     if (!status[0] && !status[1]) return;
     poisoned_ = true;
     KGE_CUDA(cudaMemset(d_tc_status_, 0, sizeof(status)));
@@ -958,6 +977,15 @@ void Engine::kernel_time(size_t index, const char** name, float* ms, unsigned lo
 }
 
 void Engine::last_run_stats(float* ms, unsigned long long* launches) const {
+    if (ms_pending_) {
+        KGE_CUDA(cudaEventElapsedTime(&last_ms_, ev_begin_, ev_end_));
+        if (ms_counts_stage_) {
+            float stage_ms = 0.f;
+            KGE_CUDA(cudaEventElapsedTime(&stage_ms, ev_stage_[0], ev_stage_[1]));
+            last_ms_ += stage_ms;
+        }
+        ms_pending_ = false;
+    }
     if (ms) *ms = last_ms_;
     if (launches) *launches = last_launches_;
 }
@@ -1988,6 +2016,136 @@ void Engine::launch_one_step(unsigned step) {
 // ---------------------------------------------------------------------------
 // Table and variable I/O
 
+// rows x row_bytes from device memory (rows src_pitch apart) into the caller's contiguous array, in pieces: while one
+// piece crosses the link the previous one is copied out of pinned memory (1.4 MB: 180 us as a plain pageable copy, 70 us).
+void Engine::copy_out(void* dst, const void* src, size_t src_pitch, size_t row_bytes, size_t rows) {
+    if (src_pitch == row_bytes) row_bytes *= rows, rows = 1;
+    const size_t per_row = rows == 1 ? kIoPiece : std::max<size_t>(1, (kIoPiece - 256) / row_bytes);  // bytes of one long row, or rows, per piece
+    const size_t total = rows == 1 ? row_bytes : rows;
+    const size_t piece_bytes = rows == 1 ? kIoPiece : round_up(per_row * row_bytes, 256);
+    const PinnedBlock block(piece_bytes * kIoSlots);
+    const size_t pieces = (total + per_row - 1) / per_row;
+    HostTeam* const team = team_for(total * (rows == 1 ? 1 : row_bytes));
+    size_t issued = 0;
+    auto issue = [&](size_t i) {
+        uint8_t* slot = block.data() + (i % kIoSlots) * piece_bytes;
+        const uint8_t* from = static_cast<const uint8_t*>(src) + i * per_row * (rows == 1 ? 1 : src_pitch);
+        const size_t count = std::min(per_row, total - i * per_row);
+        if (rows == 1) KGE_CUDA(cudaMemcpyAsync(slot, from, count, cudaMemcpyDeviceToHost, stream_));
+        else KGE_CUDA(cudaMemcpy2DAsync(slot, row_bytes, from, src_pitch, row_bytes, count, cudaMemcpyDeviceToHost, stream_));
+        KGE_CUDA(cudaEventRecord(io_event(i), stream_));
+    };
+    for (size_t i = 0; i < pieces; ++i) {
+        for (; issued < pieces && issued < i + kIoSlots; ++issued) issue(issued);
+        KGE_CUDA(cudaEventSynchronize(io_event(i)));
+        const size_t unit = rows == 1 ? 1 : row_bytes, count = std::min(per_row, total - i * per_row);
+        team_copy(team, static_cast<uint8_t*>(dst) + i * per_row * unit, block.data() + (i % kIoSlots) * piece_bytes, count * unit);
+    }
+}
+
+// The other way.  Returns when the transfers are complete.
+void Engine::copy_in(void* dst, size_t dst_pitch, const void* src, size_t row_bytes, size_t rows) {
+    if (dst_pitch == row_bytes) row_bytes *= rows, rows = 1;
+    const size_t per_piece = rows == 1 ? kIoPiece : std::max<size_t>(1, (kIoPiece - 256) / row_bytes), total = rows == 1 ? row_bytes : rows;
+    const size_t unit = rows == 1 ? 1 : row_bytes, piece_bytes = round_up(per_piece * unit, 256);
+    HostTeam* const team = team_for(total * unit);
+    const PinnedBlock block(piece_bytes * kIoSlots);
+    for (size_t i = 0, at = 0; at < total; ++i, at += per_piece) {
+        uint8_t* slot = block.data() + (i % kIoSlots) * piece_bytes;
+        const size_t count = std::min(per_piece, total - at);
+        if (i >= kIoSlots) KGE_CUDA(cudaEventSynchronize(io_event(i)));
+        team_copy(team, slot, static_cast<const uint8_t*>(src) + at * unit, count * unit);
+        if (rows == 1) KGE_CUDA(cudaMemcpyAsync(static_cast<uint8_t*>(dst) + at, slot, count, cudaMemcpyHostToDevice, stream_));
+        else KGE_CUDA(cudaMemcpy2DAsync(static_cast<uint8_t*>(dst) + at * dst_pitch, dst_pitch, slot, row_bytes, row_bytes, count, cudaMemcpyHostToDevice, stream_));
+        KGE_CUDA(cudaEventRecord(io_event(i), stream_));
+    }
+    KGE_CUDA(cudaStreamSynchronize(stream_));
+}
+
+cudaEvent_t Engine::io_event(size_t piece) {
+    cudaEvent_t& e = ev_io_[piece % kIoSlots];
+    if (!e) KGE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return e;
+}
+
+// Whole rows in the host's element type: `per_shard` rows of every local shard, named by h_idx [n_local, per_shard] or
+// (null) the rows first, first + 1, ...  A piece is converted on the GPU, crosses the link and is copied to the caller,
+// each while the next one does the step before.  Pieces up to 64 KB are written by the kernel straight into pinned
+// memory: that saves a transfer's start but moves only 12 GB/s (the copy engine 45).
+void Engine::read_rows(const uint32_t* h_idx, uint32_t first, size_t per_shard, int dtype, void* out) {
+    const size_t W = cfg_.row_width(), row_out = W * (dtype == KGE_F32 ? 4 : 2), total = n_local_ * per_shard;
+    if (!total) return;
+    const size_t per_piece = std::max<size_t>(1, (kIoPiece - 512) / (row_out + 4)), idx_bytes = round_up(per_piece * 4, 256);
+    const size_t piece_bytes = idx_bytes + round_up(per_piece * row_out, 256), pieces = (total + per_piece - 1) / per_piece;
+    const PinnedBlock block(piece_bytes * kIoSlots);
+    HostTeam* const team = team_for(total * row_out);
+    DeviceBlock staging;
+    size_t issued = 0;
+    for (size_t i = 0; i < pieces; ++i) {
+        for (; issued < pieces && issued < i + kIoSlots; ++issued) {
+            uint8_t* slot = block.data() + (issued % kIoSlots) * piece_bytes;
+            const size_t at = issued * per_piece, count = std::min(per_piece, total - at);
+            uint32_t* idx = nullptr;
+            if (h_idx) {
+                idx = reinterpret_cast<uint32_t*>(slot);
+                std::memcpy(idx, h_idx + at, count * 4);
+            }
+            const RowSource rows{shards_[0].table, table_stride_, idx, first, at, per_shard};
+            const unsigned grid = (unsigned)count;
+            const bool staged = count * row_out > kIoDirectBytes && piece_bytes <= kIoPiece;
+            uint8_t* to = staged ? staging.get() + (issued % kIoSlots) * kIoPiece : slot + idx_bytes;
+            if (dtype == KGE_F32)
+                KGE_DISPATCH_ROW(cfg_, k_read_rows<ST, FT, float><<<grid, 128, 0, stream_>>>(rows, layout_, reinterpret_cast<float*>(to)));
+            else
+                k_read_rows<__half, __half, __half><<<grid, 128, 0, stream_>>>(rows, layout_, reinterpret_cast<__half*>(to));
+            KGE_CUDA(cudaGetLastError());
+            if (staged) KGE_CUDA(cudaMemcpyAsync(slot + idx_bytes, to, count * row_out, cudaMemcpyDeviceToHost, stream_));
+            KGE_CUDA(cudaEventRecord(io_event(issued), stream_));
+        }
+        if (team && i == 0) team_touch(*team, out, total * row_out);
+        KGE_CUDA(cudaEventSynchronize(io_event(i)));
+        const size_t at = i * per_piece;
+        team_copy(team, static_cast<uint8_t*>(out) + at * row_out, block.data() + (i % kIoSlots) * piece_bytes + idx_bytes, std::min(per_piece, total - at) * row_out);
+    }
+}
+
+// The other way: fresh rows with the given features (as "write_entity"), or whole rows.
+void Engine::write_rows(const uint32_t* h_idx, uint32_t first, size_t per_shard, int dtype, const void* data, bool whole_rows) {
+    const size_t per_row = whole_rows ? cfg_.row_width() : cfg_.f, row_in = per_row * (dtype == KGE_F32 ? 4 : 2), total = n_local_ * per_shard;
+    if (!total) return;
+    const size_t per_piece = std::max<size_t>(1, (kIoPiece - 256) / std::max<size_t>(row_in, 64)), piece_bytes = round_up(per_piece * row_in, 256);
+    const PinnedBlock block(piece_bytes * kIoSlots);
+    HostTeam* const team = team_for(total * row_in);
+    DeviceBlock staging;
+    const float stddev = cfg_.init_scale / (float)cfg_.d;  // src/poplar_kge.cpp:865
+    if (h_idx) copy_in(d_rw_idx_, total * 4, h_idx, total * 4, 1);  // all of them: a slot looks for later ones with its row
+    for (size_t i = 0, at = 0; at < total; ++i, at += per_piece) {
+        uint8_t* slot = block.data() + (i % kIoSlots) * piece_bytes;
+        const size_t count = std::min(per_piece, total - at);
+        if (i >= kIoSlots) KGE_CUDA(cudaEventSynchronize(io_event(i)));
+        if (row_in) team_copy(team, slot, static_cast<const uint8_t*>(data) + at * row_in, count * row_in);
+        const RowSource rows{shards_[0].table, table_stride_, h_idx ? d_rw_idx_ + at : nullptr, first, at, per_shard};
+        const unsigned grid = (unsigned)count;
+        if (count * row_in > kIoDirectBytes && piece_bytes <= kIoPiece) {  // shorter pieces are read by the kernel across the link
+            uint8_t* to = staging.get() + (i % kIoSlots) * kIoPiece;
+            KGE_CUDA(cudaMemcpyAsync(to, slot, count * row_in, cudaMemcpyHostToDevice, stream_));
+            slot = to;
+        }
+        if (dtype == KGE_F32) {
+            using IT = float;
+            if (whole_rows) KGE_DISPATCH_ROW(cfg_, k_write_rows<ST, FT, IT><<<grid, 128, 0, stream_>>>(rows, layout_, (const IT*)slot));
+            else KGE_DISPATCH_ROW(cfg_, k_write_entity<ST, FT, IT><<<grid, 128, 0, stream_>>>(rows, layout_, (const IT*)slot, cfg_.seed, shard0_, stddev));
+        } else {
+            using IT = __half;
+            if (whole_rows) KGE_DISPATCH_ROW(cfg_, k_write_rows<ST, FT, IT><<<grid, 128, 0, stream_>>>(rows, layout_, (const IT*)slot));
+            else KGE_DISPATCH_ROW(cfg_, k_write_entity<ST, FT, IT><<<grid, 128, 0, stream_>>>(rows, layout_, (const IT*)slot, cfg_.seed, shard0_, stddev));
+        }
+        KGE_CUDA(cudaGetLastError());
+        KGE_CUDA(cudaEventRecord(io_event(i), stream_));
+    }
+    KGE_CUDA(cudaStreamSynchronize(stream_));
+}
+
 void Engine::cmd_read_entity(std::vector<HostArray>& arrays) {
     const size_t n = n_local_, rw = cfg_.rw_batch, W = cfg_.row_width();
     HostArray& idx = find_array(arrays, "read_indices", KGE_U32, {n, rw});
@@ -1998,22 +2156,28 @@ void Engine::cmd_read_entity(std::vector<HostArray>& arrays) {
         if (h[i] >= cfg_.n_entity)
             fail(KGE_INVALID_ARGUMENT, msg() << "'read_indices' holds index " << h[i] << ", not below model.n_entity ("
                                              << cfg_.n_entity << ")");
-    KGE_CUDA(cudaStreamSynchronize(stream_));
-    KGE_CUDA(cudaMemcpyAsync(d_rw_idx_, idx.data, n * rw * 4, cudaMemcpyHostToDevice, stream_));
-    const size_t elem = out_dtype == KGE_F32 ? 4 : 2;
-    for (unsigned l = 0; l < n; ++l) {
-        const uint32_t* di = d_rw_idx_ + l * rw;
-        void* dout = d_rw_data_ + l * rw * W * elem;
-        if (out_dtype == KGE_F32) {
-            KGE_DISPATCH_ROW(cfg_, k_read_rows<ST, FT, float><<<(unsigned)rw, 128, 0, stream_>>>(shards_[l].table, layout_, di,
-                                                                                                 (float*)dout));
-        } else {
-            k_read_rows<__half, __half, __half><<<(unsigned)rw, 128, 0, stream_>>>(shards_[l].table, layout_, di, (__half*)dout);
-        }
+    read_rows(h, 0, rw, out_dtype, out.data);
+}
+
+// "read_entity_range" / "write_entity_range": what "read_entity" / "write_entity" do to the rows `row_range` u32 [2] =
+// (first, count) of every local shard, whatever rw_batch_size: read_data [n, count, 3D+F] in the state type;
+// write_features [n, count, F], float32 or float16.
+void Engine::cmd_entity_range(std::vector<HostArray>& arrays, bool read) {
+    HostArray& range = find_array(arrays, "row_range", KGE_U32, {2});
+    const size_t n = n_local_, first = static_cast<const uint32_t*>(range.data)[0], count = static_cast<const uint32_t*>(range.data)[1];
+    if (first + count > cfg_.n_entity)
+        fail(KGE_INVALID_ARGUMENT, msg() << "'row_range' covers rows [" << first << ", " << first + count << "), not within model.n_entity (" << cfg_.n_entity << ")");
+    if (read) {
+        const int out_dtype = cfg_.state_type == ST_F32 ? KGE_F32 : KGE_F16;
+        HostArray& out = find_array(arrays, "read_data", out_dtype, {n, count, cfg_.row_width()});
+        return read_rows(nullptr, (uint32_t)first, count, out_dtype, out.data);
     }
-    KGE_CUDA(cudaGetLastError());
-    KGE_CUDA(cudaMemcpyAsync(out.data, d_rw_data_, n * rw * W * elem, cudaMemcpyDeviceToHost, stream_));
-    KGE_CUDA(cudaStreamSynchronize(stream_));
+    HostArray* data = nullptr;
+    for (HostArray& a : arrays)
+        if (a.name == "write_features") data = &a;
+    if (!data) fail(KGE_INVALID_ARGUMENT, "Key not found 'write_features'");
+    find_array(arrays, "write_features", data->dtype == KGE_F16 ? KGE_F16 : KGE_F32, {n, count, cfg_.f});
+    write_rows(nullptr, (uint32_t)first, count, data->dtype, data->data, false);
 }
 
 // "dump_entity_rows" / "restore_entity_rows": a contiguous range of one local shard's table as it
@@ -2060,28 +2224,7 @@ void Engine::cmd_write_entity(std::vector<HostArray>& arrays, bool whole_rows) {
         if (h[i] >= cfg_.n_entity)
             fail(KGE_INVALID_ARGUMENT, msg() << "'write_indices' holds index " << h[i] << ", not below model.n_entity ("
                                              << cfg_.n_entity << ")");
-    const size_t elem = data->dtype == KGE_F32 ? 4 : 2, per_row = shape[2];
-    KGE_CUDA(cudaStreamSynchronize(stream_));
-    KGE_CUDA(cudaMemcpyAsync(d_rw_idx_, idx.data, n * rw * 4, cudaMemcpyHostToDevice, stream_));
-    KGE_CUDA(cudaMemcpyAsync(d_rw_data_, data->data, n * rw * per_row * elem, cudaMemcpyHostToDevice, stream_));
-    const float stddev = cfg_.init_scale / (float)cfg_.d;  // src/poplar_kge.cpp:865
-    for (unsigned l = 0; l < n; ++l) {
-        const uint32_t* di = d_rw_idx_ + l * rw;
-        const uint8_t* din = d_rw_data_ + l * rw * per_row * elem;
-        uint8_t* table = shards_[l].table;
-        const unsigned g = (unsigned)rw;
-        if (data->dtype == KGE_F32) {
-            using IT = float;
-            if (whole_rows) KGE_DISPATCH_ROW(cfg_, k_write_rows<ST, FT, IT><<<g, 128, 0, stream_>>>(table, layout_, di, (int)rw, (const IT*)din));
-            else KGE_DISPATCH_ROW(cfg_, k_write_entity<ST, FT, IT><<<g, 128, 0, stream_>>>(table, layout_, di, (int)rw, (const IT*)din, cfg_.seed, shard0_ + l, stddev));
-        } else {
-            using IT = __half;
-            if (whole_rows) KGE_DISPATCH_ROW(cfg_, k_write_rows<ST, FT, IT><<<g, 128, 0, stream_>>>(table, layout_, di, (int)rw, (const IT*)din));
-            else KGE_DISPATCH_ROW(cfg_, k_write_entity<ST, FT, IT><<<g, 128, 0, stream_>>>(table, layout_, di, (int)rw, (const IT*)din, cfg_.seed, shard0_ + l, stddev));
-        }
-    }
-    KGE_CUDA(cudaGetLastError());
-    KGE_CUDA(cudaStreamSynchronize(stream_));
+    write_rows(h, 0, rw, data->dtype, data->data, whole_rows);
 }
 
 void Engine::cmd_initialise_entities() {
@@ -2100,7 +2243,6 @@ void Engine::cmd_read_write_variable(std::vector<HostArray>& arrays, const std::
         if (v.name == name) var = &v;
     if (!var) fail(KGE_INVALID_ARGUMENT, msg() << "Key not found '" << name << "'");
     HostArray& value = find_array(arrays, "value", var->dtype, var->shape);
-    KGE_CUDA(cudaStreamSynchronize(stream_));
     if (var->kind == 3) {  // step: one counter, presented per shard
         uint32_t* p = static_cast<uint32_t*>(value.data);
         if (write) {
@@ -2122,15 +2264,15 @@ void Engine::cmd_read_write_variable(std::vector<HostArray>& arrays, const std::
     float* host = static_cast<float*>(value.data);
     if (write) {
         // on the engine's stream, so that the kernel that derives the lower plane is ordered behind the copy
-        KGE_CUDA(cudaMemcpy2DAsync(base + var->offset, D * 4, host, cols * 4, cols * 4, n_rows, cudaMemcpyHostToDevice, stream_));
+        copy_in(base + var->offset, D * 4, host, cols * 4, n_rows);
         if (var->kind == 0) refresh_lower_plane(var->offset, n_rows * D);
-        KGE_CUDA(cudaStreamSynchronize(stream_));
         return;
     }
     if (var->kind == 0 || cfg_.world == 1) {
-        KGE_CUDA(cudaMemcpy2D(host, cols * 4, base + var->offset, D * 4, cols * 4, n_rows, cudaMemcpyDeviceToHost));
+        copy_out(host, base + var->offset, D * 4, cols * 4, n_rows);
         return;
     }
+    KGE_CUDA(cudaStreamSynchronize(stream_));
     // Optimiser state lives with the process that owns the row (src/poplar_kge.cpp:329-339): row r of
     // the dense vector with process r % world.  Collect each owner's rows through its mapped arena.
     for (size_t p = 0; p < W; ++p) {

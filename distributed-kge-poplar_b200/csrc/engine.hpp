@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "common.hpp"
+#include "host_io.hpp"
 #include "kernels.cuh"
 #include "tc_gemm.cuh"
 #include "tc_planes.cuh"
@@ -101,7 +102,7 @@ class Engine {
     void comm_export(void* out) const;
     void comm_connect(const void* handles, size_t world);
 
-    void stage_batch(std::vector<HostArray>& arrays);
+    void stage_batch(std::vector<HostArray>& arrays) { stage_batch(arrays, nullptr); }
     void train_staged(float learning_rate, float* loss);
     void last_run_stats(float* ms, unsigned long long* launches) const;
     void set_kernel_timing(bool on);
@@ -159,6 +160,7 @@ class Engine {
     // commands
     void cmd_train_step_loop(std::vector<HostArray>& arrays);
     void cmd_read_entity(std::vector<HostArray>& arrays);
+    void cmd_entity_range(std::vector<HostArray>& arrays, bool read);
     void cmd_copy_entity_range(std::vector<HostArray>& arrays, bool to_host);
     void cmd_write_entity(std::vector<HostArray>& arrays, bool whole_rows);
     void cmd_read_write_variable(std::vector<HostArray>& arrays, const std::string& name, bool write);
@@ -166,6 +168,8 @@ class Engine {
     void cmd_initialise_entities();
     void cmd_load_triples(std::vector<HostArray>& arrays);
     void cmd_sample_batch(std::vector<HostArray>& arrays, bool train);
+    void stage_batch(std::vector<HostArray>& arrays, const float* learning_rate);
+    void write_run_words(float learning_rate);
     void sample_and_stage(uint32_t seed);
     void prepare_staged();
 
@@ -188,6 +192,7 @@ class Engine {
     void refresh_lower_plane(size_t offset, size_t count);
     FeaturePlanes feature_planes(const ShardBuffers& b, unsigned parity) const;
     void check_device_status();
+    void raise_device_status(const unsigned* words);
     void require_usable() const;
     void timing_begin(const char* name);
     void timing_end();
@@ -240,6 +245,7 @@ class Engine {
     bool poisoned_ = false;                         // a device-side wait gave up: the engine must be rebuilt
     std::vector<void*> allocations_;
     std::vector<ShardBuffers> shards_;
+    size_t table_stride_ = 0;  // bytes between the local shards' tables
 
     // peer-visible arena
     uint8_t* arena_ = nullptr;
@@ -300,8 +306,13 @@ class Engine {
     unsigned* d_reg_counter_ = nullptr;
     void launch_regularise(unsigned l, const uint8_t* rows_c);
     RelationRows with_regularisers(RelationRows rr, unsigned l, unsigned step) const;
-    uint8_t* pinned_ = nullptr;
-    size_t pinned_bytes_ = 0;
+    // What crosses to the GPU before a run and what comes back, laid out alike in pinned and in device memory: the five
+    // index streams, then the run's words (step numbers, Adam step sizes, the loss totals' zeros), then the two status
+    // words.  Offsets in 32-bit words.
+    uint32_t *pinned_ = nullptr, *d_run_ = nullptr;
+    size_t stage_at_[5] = {}, keys_at_ = 0, sizes_at_ = 0, loss_at_ = 0, status_at_ = 0, run_words_ = 0;
+    bool uploads_pending_ = false;      // transfers out of `pinned_` may still be under way
+    bool run_words_uploaded_ = false;   // the coming run's words went up with its index streams
     bool staged_ = false;
     // the training triples for the on-device sampler ("load_triples"), bucketed by (head shard, tail shard)
     SamplerData sampler_{};
@@ -317,7 +328,21 @@ class Engine {
     float *p_feat_ = nullptr, *p_chunk_lo_ = nullptr, *p_query_lo_ = nullptr;  // planes of a pass: widened / lower features, lower hidden rows, lower queries
 
     uint32_t* d_rw_idx_ = nullptr;
-    uint8_t* d_rw_data_ = nullptr;
+
+    // Transfers of callers' arrays in pieces through pinned blocks: the link, the GPU and the host's copies overlap.
+    static constexpr size_t kIoPiece = 512 << 10;
+    static constexpr unsigned kIoSlots = 8;
+    static constexpr size_t kIoDirectBytes = 64 << 10;
+    static_assert(kIoPiece * kIoSlots <= DeviceBlock::kBytes && kIoPiece * kIoSlots <= PinnedPool::kBlock, "a transfer's pieces fit a block");
+    static constexpr size_t kTeamBytes = 16 << 20;  // from here on the helpers share the copying
+    HostTeam* team_for(size_t bytes) { return bytes >= kTeamBytes ? &team_ : nullptr; }
+    HostTeam team_;
+    cudaEvent_t ev_io_[kIoSlots] = {};
+    cudaEvent_t io_event(size_t piece);
+    void copy_out(void* dst, const void* src, size_t src_pitch, size_t row_bytes, size_t rows);
+    void copy_in(void* dst, size_t dst_pitch, const void* src, size_t row_bytes, size_t rows);
+    void read_rows(const uint32_t* h_idx, uint32_t first, size_t per_shard, int dtype, void* out);
+    void write_rows(const uint32_t* h_idx, uint32_t first, size_t per_shard, int dtype, const void* data, bool whole_rows);
 
     struct TimedLaunch {
         const char* name;
@@ -339,7 +364,8 @@ class Engine {
         unsigned long long launches;
     };
     std::vector<StepGraph> graphs_;  // a program run, in order
-    float last_ms_ = 0.f;
+    mutable float last_ms_ = 0.f;
+    mutable bool ms_pending_ = false, ms_counts_stage_ = false;  // the last run's events have not been read yet
     unsigned long long last_launches_ = 0, launch_counter_ = 0;
 };
 

@@ -2410,43 +2410,65 @@ __device__ __forceinline__ float4 philox_normal4(uint32_t seed, uint32_t stream,
     return make_float4(r0 * c0, r0 * s0, r1 * c1, r1 * s1);
 }
 
-// A slot writes only if no later slot names the same row, so duplicate indices (the
-// overflow slots that the host redirects to row 0, src/python/poplar_kge.py:546-552)
-// resolve to the last one in order, deterministically.
-__device__ __forceinline__ bool is_last_writer(const uint32_t* idx, int n, int j) {
-    const uint32_t mine = idx[j];
-    for (int k = j + 1; k < n; ++k)
-        if (idx[k] == mine) return false;
-    return true;
+// Which table row slot j of a piece of a transfer stands for: the slots at, at + 1, ... of n_local x per_shard, with
+// their rows in idx[j] or (null) counted up from `first` in every shard.
+struct RowSource {
+    uint8_t* tables;  // the local shards' tables, `stride` bytes apart
+    size_t stride;
+    const uint32_t* idx;
+    uint32_t first;
+    size_t at, per_shard;
+};
+struct RowSlot {
+    uint32_t row, shard, slot;  // slot: within the shard
+};
+__device__ __forceinline__ RowSlot row_slot(const RowSource& s, unsigned j) {
+    const size_t g = s.at + j, l = g / s.per_shard;
+    RowSlot r;
+    r.shard = (uint32_t)l;
+    r.slot = (uint32_t)(g - l * s.per_shard);
+    r.row = s.idx ? s.idx[j] : s.first + r.slot;
+    return r;
 }
 
-// write_entity: fresh embedding ~ N(0, std), zero moments, features from the host array.
+// A slot writes only if no later slot of its shard names the same row, so duplicate indices (the
+// overflow slots that the host redirects to row 0, src/python/poplar_kge.py:546-552)
+// resolve to the last one in order, deterministically.  All threads of the block look.
+__device__ __forceinline__ bool is_last_writer(const RowSource& s, unsigned j, const RowSlot& r) {
+    if (!s.idx) return true;
+    const uint32_t left = (uint32_t)s.per_shard - r.slot;
+    bool later = false;
+    for (uint32_t k = 1 + threadIdx.x; k < left; k += blockDim.x) later |= s.idx[j + k] == r.row;
+    return !__syncthreads_or(later);
+}
+
+// write_entity: fresh embedding ~ N(0, std), zero moments, features from the host array (in pinned memory).
 template <class ST, class FT, class IT>
 __global__ void __launch_bounds__(128)
-k_write_entity(uint8_t* __restrict__ table, RowLayout L, const uint32_t* __restrict__ idx, int n,
-               const IT* __restrict__ features, uint32_t seed, uint32_t shard, float stddev) {
+k_write_entity(RowSource rows, RowLayout L, const IT* __restrict__ features, uint32_t seed, uint32_t shard0, float stddev) {
     const int j = blockIdx.x;
-    __shared__ int go;
-    if (threadIdx.x == 0) go = is_last_writer(idx, n, j) ? 1 : 0;
-    __syncthreads();
-    if (!go) return;
-    const size_t row = idx[j];
-    ST* xv = reinterpret_cast<ST*>(table + row * L.row_bytes);
-    ST* mv = reinterpret_cast<ST*>(table + row * L.row_bytes + L.off_m);
-    ST* qv = reinterpret_cast<ST*>(table + row * L.row_bytes + L.off_q);
-    FT* fv = reinterpret_cast<FT*>(table + row * L.row_bytes + L.off_feat);
+    const RowSlot s = row_slot(rows, j);
+    if (!is_last_writer(rows, j, s)) return;
+    uint8_t* base = rows.tables + s.shard * rows.stride + (size_t)s.row * L.row_bytes;
+    ST* mv = reinterpret_cast<ST*>(base + L.off_m);
+    ST* qv = reinterpret_cast<ST*>(base + L.off_q);
+    FT* fv = reinterpret_cast<FT*>(base + L.off_feat);
     const int D = L.d, F = L.f;
+    const IT* __restrict__ src = features + (size_t)j * F;
+    const bool vec = (F & 3) == 0;
+    if (vec)
+        for (int c = threadIdx.x * 4; c < F; c += blockDim.x * 4) store4(fv + c, load4(src + c));
+    else
+        for (int c = threadIdx.x; c < F; c += blockDim.x) store_from_float(fv + c, load_as_float(src + c));
     for (int c4 = threadIdx.x; c4 * 4 < D; c4 += blockDim.x) {
-        const float4 z = philox_normal4(seed, shard, (uint32_t)row, (uint32_t)c4);
+        const float4 z = philox_normal4(seed, shard0 + s.shard, s.row, (uint32_t)c4);
         const float zz[4] = {z.x, z.y, z.z, z.w};
         for (int u = 0; u < 4 && c4 * 4 + u < D; ++u) {
-            store_value<ST>(L, reinterpret_cast<uint8_t*>(xv), c4 * 4 + u, stddev * zz[u]);
+            store_value<ST>(L, base, c4 * 4 + u, stddev * zz[u]);
             store_from_float(mv + c4 * 4 + u, 0.f);
             store_from_float(qv + c4 * 4 + u, 0.f);
         }
     }
-    for (int c = threadIdx.x; c < F; c += blockDim.x)
-        store_from_float(fv + c, load_as_float(features + (size_t)j * F + c));
 }
 
 // initialise_entities: every row of the shard on the device, no host data.  Embeddings as
@@ -2483,20 +2505,16 @@ k_init_table(uint8_t* __restrict__ table, RowLayout L, size_t n_rows, uint32_t s
     }
 }
 
-// write_entity_rows: whole rows [value | m | sqrt(v) | feature] from the host array.
+// write_entity_rows: whole rows [value | m | sqrt(v) | feature] from the host array (in pinned memory).
 template <class ST, class FT, class IT>
 __global__ void __launch_bounds__(128)
-k_write_rows(uint8_t* __restrict__ table, RowLayout L, const uint32_t* __restrict__ idx, int n,
-             const IT* __restrict__ data) {
+k_write_rows(RowSource rows, RowLayout L, const IT* __restrict__ data) {
     const int j = blockIdx.x;
-    __shared__ int go;
-    if (threadIdx.x == 0) go = is_last_writer(idx, n, j) ? 1 : 0;
-    __syncthreads();
-    if (!go) return;
-    const size_t row = idx[j];
+    const RowSlot s = row_slot(rows, j);
+    if (!is_last_writer(rows, j, s)) return;
     const int D = L.d, F = L.f, W = 3 * D + F;
     const IT* __restrict__ src = data + (size_t)j * W;
-    uint8_t* base = table + row * L.row_bytes;
+    uint8_t* base = rows.tables + s.shard * rows.stride + (size_t)s.row * L.row_bytes;
     for (int c = threadIdx.x; c < W; c += blockDim.x) {
         const float v = load_as_float(src + c);
         if (c < D) store_value<ST>(L, base, c, v);
@@ -2506,16 +2524,27 @@ k_write_rows(uint8_t* __restrict__ table, RowLayout L, const uint32_t* __restric
     }
 }
 
-// read_entity: whole rows out, in the host array's element type.
+// read_entity: whole rows out, in the host array's element type, into pinned memory: four elements per store where the
+// segments allow it, so that a warp's stores make whole 128-byte writes on the link.
 template <class ST, class FT, class OT>
 __global__ void __launch_bounds__(128)
-k_read_rows(const uint8_t* __restrict__ table, RowLayout L, const uint32_t* __restrict__ idx,
-            OT* __restrict__ out) {
+k_read_rows(RowSource rows, RowLayout L, OT* __restrict__ out) {
     const int j = blockIdx.x;
-    const size_t row = idx[j];
+    const RowSlot s = row_slot(rows, j);
     const int D = L.d, F = L.f, W = 3 * D + F;
-    const uint8_t* base = table + row * L.row_bytes;
+    const uint8_t* base = rows.tables + s.shard * rows.stride + (size_t)s.row * L.row_bytes;
     OT* __restrict__ dst = out + (size_t)j * W;
+    if (((D | F) & 3) == 0) {
+        for (int c = threadIdx.x * 4; c < W; c += blockDim.x * 4) {
+            float4 v;
+            if (c < D) v = L.value_bf16 ? load4(reinterpret_cast<const __nv_bfloat16*>(base) + c) : load4(reinterpret_cast<const ST*>(base) + c);
+            else if (c < 2 * D) v = load4(reinterpret_cast<const ST*>(base + L.off_m) + (c - D));
+            else if (c < 3 * D) v = load4(reinterpret_cast<const ST*>(base + L.off_q) + (c - 2 * D));
+            else v = load4(reinterpret_cast<const FT*>(base + L.off_feat) + (c - 3 * D));
+            store4(dst + c, v);
+        }
+        return;
+    }
     for (int c = threadIdx.x; c < W; c += blockDim.x) {
         float v;
         if (c < D) v = load_value<ST>(L, base, c);

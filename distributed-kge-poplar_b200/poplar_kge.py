@@ -448,8 +448,10 @@ class Engine:
         return array.view(np.int16) if array.dtype == np.float16 else array
 
     def _rw_indices(self, offset: int) -> np.ndarray:
-        idx = np.arange(offset, offset + self.settings.execution.rw_batch_size, dtype=np.uint32)
-        idx[idx >= self.settings.model.n_entity] = 0  # overflow slots go to the padding row
+        count, n_entity = self.settings.execution.rw_batch_size, self.settings.model.n_entity
+        idx = np.arange(offset, offset + count, dtype=np.uint32)
+        if offset + count > n_entity:
+            idx[idx >= n_entity] = 0  # overflow slots go to the padding row
         return np.ascontiguousarray(np.broadcast_to(idx, (self.n_local, idx.size)))
 
     def random_normal(self, shape: Shape, dtype: Union[str, np.dtype] = "float32") -> np.ndarray:
@@ -473,7 +475,7 @@ class Engine:
 
     def read_variable(self, name: str) -> np.ndarray:
         dtype = self.variable_to_dtype[name]
-        value = np.full(self.variable_to_shape[name], np.nan if dtype.kind == "f" else 0, dtype=dtype)
+        value = np.empty(self.variable_to_shape[name], dtype=dtype)
         self.engine.run("read", dict(name=name, value=value))
         return value
 
@@ -513,6 +515,11 @@ class Engine:
         self.engine.run("write_entity", dict(write_indices=idx, write_features=self._as_engine_array(data)))
         self.uninitialized_entity_data[idx[0]] = False
 
+    def _write_features(self, first: int, features: np.ndarray) -> None:
+        """``write_entity`` for any number of consecutive rows: ``[n_local, count, feature_size]``."""
+        self.engine.run("write_entity_range", dict(row_range=np.array([first, features.shape[1]], np.uint32),
+                                                   write_features=self._as_engine_array(features)))
+
     def write_entity_rows(self, offset: int, data: np.ndarray) -> None:
         """Write whole rows ``[n_local, rw_batch_size, 3*d + f]`` (value | adam_m | sqrt(adam_v) | feature)."""
         self._expect_shape("write_entity_rows(data)", data, self._local_shape(self.settings.entity_data_r_shape))
@@ -522,7 +529,7 @@ class Engine:
 
     def read_entity(self, offset: int) -> np.ndarray:
         idx = self._rw_indices(offset)
-        out = np.zeros(self._local_shape(self.settings.entity_data_r_shape), dtype=self.settings.execution.dtype)
+        out = np.empty(self._local_shape(self.settings.entity_data_r_shape), dtype=self.settings.execution.dtype)
         self.engine.run("read_entity", dict(read_indices=idx, read_data=self._as_engine_array(out)))
         return out[:, : self.settings.model.n_entity - offset]
 
@@ -531,7 +538,10 @@ class Engine:
 
     def read_entity_all(self) -> np.ndarray:
         """All rows of the local shards (large models: this is the whole table in host memory)."""
-        return np.concatenate([self.read_entity(o) for o in self._chunk_offsets()], axis=1)
+        n_entity = self.settings.model.n_entity
+        out = np.empty((self.n_local, n_entity, self.settings.entity_data_r_size), dtype=self.settings.execution.dtype)
+        self.engine.run("read_entity_range", dict(row_range=np.array([0, n_entity], np.uint32), read_data=self._as_engine_array(out)))
+        return out
 
     def _padded_chunk(self, array: np.ndarray, offset: int) -> np.ndarray:
         rw = self.settings.execution.rw_batch_size
@@ -543,8 +553,19 @@ class Engine:
     def initialise_all(self, entity_features: np.ndarray) -> None:
         """Reset the variables, then stream all features ``[n_local, n_entity, f]`` into the table."""
         self.initialise_variables()
-        for offset in self._chunk_offsets():
-            self.write_entity(offset, self._padded_chunk(entity_features, offset).astype(self.settings.execution.dtype))
+        s, features = self.settings, np.asarray(entity_features)
+        n_entity, rw = s.model.n_entity, s.execution.rw_batch_size
+        if features.shape[1] != n_entity:  # fewer or more rows than the table has: chunk by chunk, padded with zeros
+            for offset in self._chunk_offsets():
+                self.write_entity(offset, self._padded_chunk(features, offset).astype(s.execution.dtype))
+            return
+        self._expect_shape("initialise_all(entity_features)", features, (self.n_local, n_entity, s.model.entity_feature_size))
+        if features.dtype not in (np.float32, np.float16):
+            features = features.astype(s.execution.dtype)
+        self._write_features(0, features)
+        if n_entity % rw:  # the last chunk's overflow slots, whose features are zero, name the padding row
+            self._write_features(0, np.zeros((self.n_local, 1, features.shape[2]), features.dtype))
+        self.uninitialized_entity_data[:] = False
 
     def write_all_rows(self, entity_data: np.ndarray) -> None:
         """Stream whole rows ``[n_local, n_entity, 3*d + f]`` into the table."""

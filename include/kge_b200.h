@@ -92,6 +92,9 @@ const char* kge_last_error(const kge_engine* engine);
  * (src/poplar_kge.cpp:977-991).  Commands added to the reference's:
  *   "write_entity_rows" (write_indices u32 [n, rw], write_data [n, rw, 3D+F]) writes whole
  *     rows, embedding and optimiser state included, which the reference cannot do from the host.
+ *   "read_entity_range" / "write_entity_range" (row_range u32 [2] = first row, count; read_data
+ *     [n, count, 3D+F] or write_features [n, count, F]) do what "read_entity" / "write_entity" do
+ *     for any number of consecutive rows, in pieces whose copies and transfers overlap.
  *   "initialise_entities" (no arrays) fills every row on the device: embeddings as
  *     "write_entity" draws them, features ~ N(0, 1), optimiser state zero.  It stands in for
  *     the reference's host loop that streams all features through "write_entity"

@@ -274,3 +274,29 @@ def test_sharded_checkpoint_resumes_bit_exactly(tmp_path):
     with pytest.raises(ValueError, match="shard_range"):
         engine.engine.run("dump_entity_rows", dict(shard_range=np.array([0, m.n_entity - 1, 2], np.uint32),
                                                    rows=np.zeros((2, engine._entity_layout()[0] // 4), np.uint32)))
+
+
+@pytest.mark.parametrize("n_shard,n_entity,d,f,rw", [(1, 700, 300, 770, 1024), (2, 1501, 34, 21, 64), (2, 90, 8, 6, 45), (3, 2, 4, 0, 1)])
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+def test_whole_table_transfers_equal_chunked_ones(n_shard, n_entity, d, f, rw, dtype):
+    """Rows move between the host and the table in pieces of about a megabyte: one piece or several, pieces that
+    span shards, row widths with and without a remainder of four, chunks that overflow onto the padding row."""
+    settings = kge.Settings.create_demo()
+    settings.seed = 3
+    m, e = settings.model, settings.execution
+    m.n_shard, m.n_entity, m.embedding_size, m.entity_feature_size = n_shard, n_entity, d, f - f % n_shard
+    m.n_relation_type, e.rw_batch_size, e.dtype = 4 * n_shard, rw, dtype
+    settings.prepare()
+    f = m.entity_feature_size
+    features = np.random.RandomState(1).standard_normal((n_shard, n_entity, f)).astype(np.float32)
+    counts = np.full(n_shard, n_entity - 1)
+    whole, chunked = kge.Engine(settings, counts), kge.Engine(settings, counts)
+    whole.initialise_all(features)
+    for offset in chunked._chunk_offsets():
+        chunked.write_entity(offset, chunked._padded_chunk(features, offset).astype(dtype))
+    got = whole.read_entity_all()
+    want = np.concatenate([chunked.read_entity(o) for o in chunked._chunk_offsets()], axis=1)
+    assert got.dtype == want.dtype == np.dtype(dtype)
+    np.testing.assert_array_equal(got, want)
+    np.testing.assert_array_equal(got[:, 1:, 3 * d :], features[:, 1:].astype(dtype))
+    assert np.any(got[..., :d]) and not np.any(got[..., d : 3 * d])
