@@ -247,13 +247,9 @@ int kge_op_pairwise_grad(int fn, const float* a, const float* b, const float* gr
         to_device(dg, coeff.data(), m * n * 4);
         PairBwdArgs pa{};
         pa.D = (int)k;
-        pa.tiles_m0 = (int)blocks_for(m, 32);
         pa.p[0] = {da.as<float>(), db.as<float>(), dg.as<float>(), (int)m, (int)n, (int)n, 1, dga.as<float>(), nullptr, 1};
         pa.p[1] = {db.as<float>(), da.as<float>(), dg.as<float>(), (int)n, (int)m, 1, (int)n, dgb.as<float>(), nullptr, 1};
-        dim3 grid(blocks_for(m, 32) + blocks_for(n, 32), blocks_for(k, 64));
-        if (fn == DIST_L1) k_pair_bwd<DIST_L1><<<grid, 128>>>(pa);
-        else if (fn == DIST_L2) k_pair_bwd<DIST_L2><<<grid, 128>>>(pa);
-        else k_pair_bwd<DIST_DOT><<<grid, 128>>>(pa);
+        KGE_CUDA(launch_pair_bwd(fn, pa, nullptr));
         finish_kernels();
         to_host(grad_a, dga, m * k * 4);
         to_host(grad_b, dgb, n * k * 4);

@@ -378,8 +378,6 @@ Engine::Engine(const SettingMap& settings) : cfg_(parse_config(settings)) {
     if (mlp_on()) planes_ = false;  // the MLP sits between the projection and the lookups: the step of separate kernels
     if (cfg_.score_fn == SCORE_TRANSH) {
         planes_ = false;  // its score has no contraction form: the step of separate kernels
-        if (transh_score_smem() > 200 * 1024) fail(KGE_INVALID_ARGUMENT, "TransH: model.embedding_size is limited to 1600");
-        KGE_CUDA(cudaFuncSetAttribute(k_transh_score, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)transh_score_smem()));
     }
     // With one shard in all a dense gradient has a single contributor: the projection gradient's contraction and the
     // relation rows' blocks of the entity update apply the Adam step themselves and k_dense_update is not launched.
@@ -1575,11 +1573,9 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
         if (l1) {
             PairBwdArgs pa{};
             pa.D = (int)D;
-            pa.tiles_m0 = (int)ceil_div(B, 32);
             pa.p[0] = {b.pred, b.tails, b.coeff, (int)B, (int)T, (int)T, 1, b.d_pred, nullptr, 1};
             pa.p[1] = {b.tails, b.pred, b.coeff, (int)T, (int)B, 1, (int)T, nullptr, b.grad_dst, (int)cfg_.a2a_size};
-            dim3 bgrid(ceil_div(B, 32) + ceil_div(T, 32), ceil_div(D, 64));
-            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_dependent(k_pair_bwd<DIST_L1>, dim3(bgrid), dim3(128), 0, stream_, pa)));
+            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_pair_bwd(DIST_L1, pa, stream_)));
             launch_exchange_signal(XCHG_TAIL_GRADS);
         } else {
             //   dot:  d_pred = C . tails,                          d_tails = C^T . pred
@@ -1795,16 +1791,12 @@ void Engine::launch_one_step(unsigned step) {
         const uint32_t* tail = step_ptr(d_tail_, l, B);
         PairBwdArgs pa{};
         pa.D = (int)D;
-        pa.tiles_m0 = (int)ceil_div(B, 32);
         pa.p[0] = {b.pred, b.tails, b.coeff, (int)B, (int)T, (int)T, 1, b.d_pred, nullptr, 1};
         pa.p[1] = {b.tails, b.pred, b.coeff, (int)T, (int)B, 1, (int)T, nullptr, b.grad_dst, (int)cfg_.a2a_size};
-        dim3 bgrid(ceil_div(B, 32) + ceil_div(T, 32), ceil_div(D, 64));
         const bool tc_score = cfg_.tensor_cores && cfg_.dist_fn == DIST_DOT;
         const bool tc_bwd = cfg_.tensor_cores && cfg_.dist_fn != DIST_L1;
         if (transh) {
-            const dim3 grid(ceil_div(B, kTranshRows), std::max(1u, std::min(ceil_div(T, 8), 2 * 148 / std::max(1u, ceil_div(B, kTranshRows)))));
-            KGE_LAUNCH("score", KGE_CUDA(launch_dependent(k_transh_score, grid, dim3(256), transh_score_smem(), stream_, b.pred, b.nrm, b.tails, b.raw,
-                                                          b.pair_s, b.pair_u, (int)B, (int)T, (int)D, sync)));
+            KGE_LAUNCH("score", KGE_CUDA(launch_transh_score(b.pred, b.nrm, b.tails, b.raw, b.pair_s, b.pair_u, (int)B, (int)T, (int)D, sync, stream_)));
         } else if (tc_score) {
             tc::GemmArgs g{};
             g.A = tc::make_operand(b.pred, (long long)D * 4, false, false);
@@ -1846,16 +1838,12 @@ void Engine::launch_one_step(unsigned step) {
             launch_tc("score_bwd", both, 2, tc_splits((ceil_div(B, 128) + ceil_div(T, 128)) * ceil_div(D, 64), std::min(B, T)), false, l2,
                       -1, XCHG_TAIL_GRADS);
         } else if (transh) {
-            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_dependent(k_transh_bwd, dim3(B + T), dim3(128), 0, stream_, b.pred, b.nrm, b.tails, b.coeff, b.pair_s,
-                                                              b.pair_u, b.d_pred, b.d_nrm, b.grad_dst, (int)cfg_.a2a_size, (int)B, (int)T, (int)D)));
+            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_transh_bwd(TranshBwdArgs{b.pred, b.nrm, b.tails, b.coeff, b.pair_s, b.pair_u, b.d_pred, b.d_nrm, b.grad_dst,
+                                                                               (int)cfg_.a2a_size, (int)B, (int)T, (int)D, 0}, stream_)));
             launch_exchange_signal(XCHG_TAIL_GRADS);
         } else {
-        switch (cfg_.dist_fn) {
-            case DIST_L1: KGE_LAUNCH("score_bwd", KGE_CUDA(launch_dependent(k_pair_bwd<DIST_L1>, dim3(bgrid), dim3(128), 0, stream_, pa))); break;
-            case DIST_L2: KGE_LAUNCH("score_bwd", KGE_CUDA(launch_dependent(k_pair_bwd<DIST_L2>, dim3(bgrid), dim3(128), 0, stream_, pa))); break;
-            default: KGE_LAUNCH("score_bwd", KGE_CUDA(launch_dependent(k_pair_bwd<DIST_DOT>, dim3(bgrid), dim3(128), 0, stream_, pa))); break;
-        }
-        launch_exchange_signal(XCHG_TAIL_GRADS);
+            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_pair_bwd(cfg_.dist_fn, pa, stream_)));
+            launch_exchange_signal(XCHG_TAIL_GRADS);
         }
         if (transh) {
             KGE_LAUNCH("pred_bwd", KGE_CUDA(launch_dependent(k_transh_pred_bwd, dim3(B), dim3(64), 0, stream_, b.d_pred, b.d_nrm, b.hid_h, head, relation,
@@ -2432,9 +2420,8 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
                                                                     p_chunk_hidden_, nullptr)));
             if (mlp_on()) launch_mlp_forward(b.table, nullptr, start, c, two_nets ? 1 : 0, p_chunk_hidden_, p_mlp_cat_, p_mlp_pre_, p_mlp_out_);
             if (cfg_.score_fn == SCORE_TRANSH) {
-                const dim3 grid(ceil_div((unsigned)Q, kTranshRows), std::max(1u, std::min(ceil_div(c, 8u), 2 * 148 / std::max(1u, ceil_div((unsigned)Q, kTranshRows)))));
-                KGE_LAUNCH("predict_score", k_transh_score<<<grid, 256, transh_score_smem(), stream_>>>(
-                                                queries, queries + Q * D, p_chunk_hidden_, p_raw_, nullptr, nullptr, (int)Q, (int)c, (int)D, ExchangeSync{}));
+                KGE_LAUNCH("predict_score", KGE_CUDA(launch_transh_score(queries, queries + Q * D, p_chunk_hidden_, p_raw_, nullptr, nullptr, (int)Q, (int)c, (int)D,
+                                                                         ExchangeSync{}, stream_)));
             } else
             KGE_LAUNCH("predict_score", KGE_CUDA(launch_score(cfg_.dist_fn, queries, p_chunk_hidden_, p_raw_, (int)Q, (int)c, (int)D, stream_)));
             launch_topk(b, c, start, last, tp, false);

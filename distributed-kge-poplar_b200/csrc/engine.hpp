@@ -286,7 +286,6 @@ class Engine {
     uint4* d_row_info_ = nullptr;  // [n_local * n_step][R][2] per gathered row: offsets, flags, table row, first four lookups
     float *d_step_size_ = nullptr, *d_loss_total_ = nullptr, *d_loss_last_ = nullptr;
     unsigned* d_loss_counter_ = nullptr;
-    size_t transh_score_smem() const { return (size_t)2 * kTranshRows * cfg_.d * sizeof(float); }
     bool mlp_on() const { return cfg_.mlp > 0 && cfg_.f > 0; }
     void launch_mlp_forward(const uint8_t* rows, const uint32_t* index, uint32_t start, unsigned n_rows, int net, float* hid,
                             float* cat, float* pre, float* out);

@@ -802,7 +802,7 @@ inline cudaError_t launch_loss(const float* raw, const uint32_t* label, float* c
 // Problem 0 is the gradient of the predicted tails (x = pred, y = tails, C = coeff);
 // problem 1 the gradient of the tails (x = tails, y = pred, C = coeff transposed), whose
 // rows go straight to the shard that owns them: the return half of the exchange
-// (src/pag/pag.cpp:925-932).  32 rows x 64 columns per block, n in slices of 32.
+// (src/pag/pag.cpp:925-932).
 struct PairBwdProblem {
     const float* X;
     const float* Y;
@@ -816,107 +816,180 @@ struct PairBwdProblem {
 struct PairBwdArgs {
     PairBwdProblem p[2];
     int D;
-    int tiles_m0;
+    int tiles_m0;  // set by launch_pair_bwd
 };
 
-template <int FN>
-__global__ void __launch_bounds__(128) k_pair_bwd(PairBwdArgs args) {
-    grid_dependency_sync();
-    constexpr int BM = 32, BD = 64, BN = 32;
-    __shared__ float Cs[BM][BN + 1];
-    __shared__ __align__(16) float Ys[BN][BD];
-    const int which = (int)blockIdx.x >= args.tiles_m0 ? 1 : 0;
-    const PairBwdProblem& pr = args.p[which];
-    const int D = args.D;
-    const int m0 = ((int)blockIdx.x - (which ? args.tiles_m0 : 0)) * BM, d0 = blockIdx.y * BD;
-    const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-    const bool vec = (D & 3) == 0;
+// Two neighbouring fp32 values in one 64-bit register pair: the FP32 pipe takes both in one instruction.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// a - b, rounded once.
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, 0xbf800000bf800000ull, a); }
+// 1 where x > 0, else 0 (0 and NaN included): x times infinity, clamped to [0, 1], where a NaN becomes 0.
+__device__ __forceinline__ float positive(float x, float infinity) {
+    float r;
+    asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(infinity));
+    return r;
+}
+// sign(e) of either value: 1, 0 or -1.  Comparisons run at half the FP32 pipe's rate; these products run at the full one.
+__device__ __forceinline__ f32x2 sign2(f32x2 e) {
+    const float inf = __int_as_float(0x7f800000);
+    const float2 v = unpack2(e);
+    return sub2(pack2(positive(v.x, inf), positive(v.y, inf)), pack2(positive(v.x, -inf), positive(v.y, -inf)));
+}
+constexpr int kPairCols = 64, kPairWarps = 8;  // columns and warps of a block of the two backward kernels below
 
-    float x[4][4], acc[4][4];
+// dst[r][c] = src[r * stride + c] for r < rows, c < cols of a ROWS x COLS array, zeros elsewhere; asynchronous where vec.
+template <int ROWS, int COLS>
+__device__ __forceinline__ void stage_rows(float* dst, const float* __restrict__ src, size_t stride, int rows, int cols, bool vec) {
+    constexpr int kQuads = COLS / 4;
+    for (int q = threadIdx.x; q < ROWS * kQuads; q += 32 * kPairWarps) {
+        const int r = q / kQuads, c = q % kQuads * 4;
+        float* to = dst + q * 4;
+        const float* from = src + (size_t)r * stride + c;
+        if (vec && r < rows && c < cols) {
+            score_copy16(to, from);
+        } else {
+            float v[4];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int m = m0 + ty * 4 + a;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int k = d0 + tx * 4 + b;
-            x[a][b] = (m < pr.M && k < D) ? pr.X[(size_t)m * D + k] : 0.f;
-            acc[a][b] = 0.f;
+            for (int u = 0; u < 4; ++u) v[u] = r < rows && c + u < cols ? from[u] : 0.f;
+            *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
         }
     }
-    const bool n_fast = pr.c_stride_n == 1;
-    for (int n0 = 0; n0 < pr.N; n0 += BN) {
-        __syncthreads();
+}
+__device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void stage_wait_previous() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+// Columns k and k + 1 of a row, zeros past the end.
+__device__ __forceinline__ f32x2 load_pair(const float* __restrict__ row, int k, int D) { return pack2(k < D ? row[k] : 0.f, k + 1 < D ? row[k + 1] : 0.f); }
+__device__ __forceinline__ void store_pair(float* __restrict__ row, int k, int D, f32x2 v) {
+    const float2 f = unpack2(v);
+    if (k + 1 < D && (D & 1) == 0) {
+        *reinterpret_cast<float2*>(row + k) = f;
+    } else {
+        if (k < D) row[k] = f.x;
+        if (k + 1 < D) row[k + 1] = f.y;
+    }
+}
+
+// A warp takes ROWS rows of 64 columns (a lane two of them) and adds the terms up in the order of n, which is part of the
+// result: the coefficients of a softmax row add up to zero, so where (nearly) all differences of a column have one sign
+// the L1 gradient is the rounding left over from that sum, and Adam's first steps of a parameter do not depend on a
+// gradient's size.  (Dividing n over warps was no faster and moved relations by 1e-3.)  The block walks n in chunks of
+// 64, both operands staged in shared memory one chunk ahead.  Bound by the FP32 pipe, 4 issue slots a term, as many as
+// shared memory's wavefronts with one row per warp; two rows share a warp's reads of Y where the problem has blocks
+// enough for it.  The form before, 32 x 64 tiles of 128 threads without the look-ahead, had 48 blocks for a
+// 256 x 512 x 100 problem and stalled on every chunk (61 us for 256 x 320 x 64).
+constexpr int kPairChunk = 64;
+
+template <int FN, int ROWS>
+__global__ void __launch_bounds__(32 * kPairWarps, 3) k_pair_bwd(PairBwdArgs args) {
+    grid_dependency_sync();
+    constexpr int kRows = ROWS * kPairWarps, kCs = kRows * kPairChunk, kStage = kCs + kPairChunk * kPairCols;
+    __shared__ __align__(16) float smem[2][kStage];  // C [kRows][chunk] or [chunk][kRows] | Y [chunk][cols]
+    const int D = args.D, col_tiles = (D + kPairCols - 1) / kPairCols, tile_m = (int)blockIdx.x / col_tiles;
+    const int which = tile_m >= args.tiles_m0 ? 1 : 0;
+    const PairBwdProblem& pr = args.p[which];
+    const int M = pr.M, N = pr.N, m0 = (tile_m - (which ? args.tiles_m0 : 0)) * kRows, k0 = (int)blockIdx.x % col_tiles * kPairCols;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = m0 + warp * ROWS, k = k0 + lane * 2;
+    const bool n_fast = pr.c_stride_n == 1, y_vec = (D & 3) == 0;  // else c_stride_m is 1
+    const int c_stride = n_fast ? pr.c_stride_m : pr.c_stride_n;
+    const bool c_vec = ((c_stride | (n_fast ? N : M)) & 3) == 0;
+    auto stage = [&](int n0, float* to) {
+        if (n_fast) stage_rows<kRows, kPairChunk>(to, pr.C + (size_t)m0 * c_stride + n0, c_stride, M - m0, N - n0, c_vec);
+        else stage_rows<kPairChunk, kRows>(to, pr.C + (size_t)n0 * c_stride + m0, c_stride, N - n0, M - m0, c_vec);
+        stage_rows<kPairChunk, kPairCols>(to + kCs, pr.Y + (size_t)n0 * D + k0, D, N - n0, D - k0, y_vec);
+    };
+    f32x2 x[ROWS], acc[ROWS];
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {
-            const int idx = t + it * 128;
-            const int m = n_fast ? (idx >> 5) : (idx & 31);
-            const int n = n_fast ? (idx & 31) : (idx >> 5);
-            const int gm = m0 + m, gn = n0 + n;
-            float v = 0.f;
-            if (gm < pr.M && gn < pr.N)
-                v = pr.C[(size_t)gm * pr.c_stride_m + (size_t)gn * pr.c_stride_n];
-            Cs[m][n] = v;
-        }
-#pragma unroll
-        for (int it = 0; it < 4; ++it) {
-            const int idx = t + it * 128, k4 = (idx & 15) * 4, n = idx >> 4;
-            const int gn = n0 + n, gk = d0 + k4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (gn < pr.N) {
-                const float* src = pr.Y + (size_t)gn * D + gk;
-                if (vec && gk + 3 < D) {
-                    v = load4(src);
-                } else {
-                    if (gk + 0 < D) v.x = src[0];
-                    if (gk + 1 < D) v.y = src[1];
-                    if (gk + 2 < D) v.z = src[2];
-                    if (gk + 3 < D) v.w = src[3];
-                }
-            }
-            store4(&Ys[n][k4], v);
-        }
+    for (int r = 0; r < ROWS; ++r) {
+        x[r] = m + r < M ? load_pair(pr.X + (size_t)(m + r) * D, k, D) : 0ull;
+        acc[r] = 0ull;
+    }
+    stage(0, smem[0]);
+    stage_commit();
+    for (int n0 = 0, half = 0; n0 < N; n0 += kPairChunk, half ^= 1) {
+        if (n0 + kPairChunk < N) stage(n0 + kPairChunk, smem[half ^ 1]);
+        stage_commit();
+        stage_wait_previous();
         __syncthreads();
+        const float* cs = smem[half] + (n_fast ? warp * ROWS * kPairChunk : warp * ROWS);
+        const float* ys = smem[half] + kCs + lane * 2;
 #pragma unroll 4
-        for (int nn = 0; nn < BN; ++nn) {
-            const float4 yv = load4(&Ys[nn][tx * 4]);
-            const float yr[4] = {yv.x, yv.y, yv.z, yv.w};
+        for (int n = 0; n < kPairChunk; n += 4) {
+            float c[ROWS][4];
+            if (n_fast) {
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const float c = Cs[ty * 4 + a][nn];
+                for (int r = 0; r < ROWS; ++r) {
+                    const float4 q = load4(cs + r * kPairChunk + n);
+                    c[r][0] = q.x; c[r][1] = q.y; c[r][2] = q.z; c[r][3] = q.w;
+                }
+            } else {
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
-                    if (FN == DIST_L1) {
-                        const float d = x[a][b] - yr[b];
-                        acc[a][b] += d > 0.f ? c : (d < 0.f ? -c : 0.f);
-                    } else if (FN == DIST_L2) {
-                        acc[a][b] = fmaf(c, x[a][b] - yr[b], acc[a][b]);
-                    } else {
-                        acc[a][b] = fmaf(c, yr[b], acc[a][b]);
-                    }
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                    for (int r = 0; r < ROWS; ++r) c[r][u] = cs[(n + u) * kRows + r];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const f32x2 y = *reinterpret_cast<const f32x2*>(ys + (n + u) * kPairCols);
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) {
+                    const f32x2 cc = pack2(c[r][u], c[r][u]);
+                    if (FN == DIST_DOT) acc[r] = fma2(cc, y, acc[r]);
+                    else if (FN == DIST_L2) acc[r] = fma2(cc, sub2(x[r], y), acc[r]);
+                    else acc[r] = fma2(cc, sign2(sub2(x[r], y)), acc[r]);
                 }
             }
         }
+        __syncthreads();
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int m = m0 + ty * 4 + a;
-        if (m >= pr.M) continue;
+    for (int r = 0; r < ROWS; ++r) {
+        if (m + r >= M) continue;
         float* dst;
         if (pr.out_blocks) {
-            const int blk = m / pr.block_rows;
-            dst = pr.out_blocks[blk] + (size_t)(m - blk * pr.block_rows) * D;
+            const int blk = (m + r) / pr.block_rows;
+            dst = pr.out_blocks[blk] + (size_t)(m + r - blk * pr.block_rows) * D;
         } else {
-            dst = pr.out + (size_t)m * D;
+            dst = pr.out + (size_t)(m + r) * D;
         }
-        const int k = d0 + tx * 4;
-        if (vec && k + 3 < D) {
-            store4(dst + k, make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]));
-        } else {
-#pragma unroll
-            for (int b = 0; b < 4; ++b)
-                if (k + b < D) dst[k + b] = acc[a][b];
-        }
+        store_pair(dst, k, D, acc[r]);
     }
+}
+
+template <int FN>
+inline cudaError_t launch_pair_bwd(PairBwdArgs args, cudaStream_t stream) {
+    const int col_tiles = (args.D + kPairCols - 1) / kPairCols;
+    auto tiles = [&](int which, int rows) { return (args.p[which].M + rows * kPairWarps - 1) / (rows * kPairWarps); };
+    // two rows per warp where that still leaves two blocks per SM
+    const int rows = (tiles(0, 2) + tiles(1, 2)) * col_tiles >= 2 * 148 ? 2 : 1;
+    args.tiles_m0 = tiles(0, rows);
+    const dim3 grid((args.tiles_m0 + tiles(1, rows)) * col_tiles), block(32 * kPairWarps);
+    if (rows == 2) return launch_dependent(k_pair_bwd<FN, 2>, grid, block, 0, stream, args);
+    return launch_dependent(k_pair_bwd<FN, 1>, grid, block, 0, stream, args);
+}
+inline cudaError_t launch_pair_bwd(int fn, const PairBwdArgs& args, cudaStream_t stream) {
+    if (fn == DIST_L1) return launch_pair_bwd<DIST_L1>(args, stream);
+    if (fn == DIST_L2) return launch_pair_bwd<DIST_L2>(args, stream);
+    return launch_pair_bwd<DIST_DOT>(args, stream);
 }
 
 // Gradients of the head vector and of the relation row for the multiplicative score

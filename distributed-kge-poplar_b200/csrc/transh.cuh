@@ -7,8 +7,7 @@
 // Four kernels: the predicted tails of a batch, the pairwise distances with the two [B, T]
 // matrices the backward needs (s_ij = n_i . t_j and u_ij = sum_k sign(e_ijk) n_ik), the gradients
 // of the distance with respect to pt, n and the tails, and the backward of the prediction down to
-// the head rows, the translation rows and the raw normals.  Plain FP32-pipe kernels: a row of the
-// output per block, the other index walked in order, so every sum has a fixed order.
+// the head rows, the translation rows and the raw normals.  FP32-pipe kernels; every sum has a fixed order.
 #pragma once
 
 #include "kernels.cuh"
@@ -42,93 +41,246 @@ k_transh_predict(const float* __restrict__ hid_h, const uint32_t* __restrict__ h
     }
 }
 
-// raw[i, j] = sum_k |e_ijk|, and (when asked for) S[i, j] = n_i . t_j, U[i, j] = sum_k sign(e_ijk) n_ik.
-// A block holds 16 query rows (pt and n) in shared memory and walks the tails; a warp per tail, the
-// lanes split k.  `y_index` (optional) names the tail rows (predict scores chunks of the table's
-// hidden rows in place).
-constexpr int kTranshRows = 16;
+// raw[i, j] = sum_k |e_ijk|, and (BACKWARD) S[i, j] = n_i . t_j, U[i, j] = sum_k sign(e_ijk) n_ik.
+// A warp owns 4 x 8 outputs with its lanes along k (lane l has k = l, l + 32, ...), so that a row is read in whole
+// 128-byte lines and held by the lanes for all outputs of the tile; the 32 sums of a quantity are then reduced over the
+// lanes by halving: a step exchanges half of a lane's sums with its partner and adds, 31 exchanges for 32 sums instead
+// of 160, and leaves lane l with output l.  Bound by the FP32 pipe and the latency of the rows' loads (a lane's sums
+// fill the registers of two blocks per SM).  512 x 768 x 128: 316 us with a warp per tail, a query after the other and
+// three full reductions each; 39 us this way.
+constexpr int kTranshRows = 4, kTranshCols = 8, kTranshWarps = 8;
 
-static __global__ void __launch_bounds__(256)
+// sums[o] of all lanes added up for o = 0 .. 31; lane l returns the total of sums[l].
+__device__ __forceinline__ float reduce_to_lanes(float (&sums)[32]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = 16; half > 0; half >>= 1) {
+        const bool upper = (lane & half) != 0;
+#pragma unroll
+        for (int o = 0; o < half; ++o) {
+            const float give = upper ? sums[o] : sums[o + half], keep = upper ? sums[o + half] : sums[o];
+            sums[o] = keep + __shfl_xor_sync(0xffffffffu, give, half);
+        }
+    }
+    return sums[0];
+}
+
+template <bool BACKWARD>
+__global__ void __launch_bounds__(32 * kTranshWarps, 2)
 k_transh_score(const float* __restrict__ pt, const float* __restrict__ nrm, const float* __restrict__ tails, float* __restrict__ raw,
                float* __restrict__ S, float* __restrict__ U, int B, int T, int D, ExchangeSync sync) {
     grid_dependency_sync();
     exchange_wait(sync, XCHG_TAILS);  // the tails come from the other processes
-    extern __shared__ float smem[];
-    float* sp = smem;                       // [kTranshRows][D]
-    float* sn = smem + kTranshRows * D;     // [kTranshRows][D]
-    const int i0 = blockIdx.x * kTranshRows, rows = min(kTranshRows, B - i0);
-    for (int idx = threadIdx.x; idx < rows * D; idx += 256) {
-        sp[idx] = pt[(size_t)i0 * D + idx];
-        sn[idx] = nrm[(size_t)i0 * D + idx];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i0 = blockIdx.x * kTranshRows, j0 = (blockIdx.y * kTranshWarps + warp) * kTranshCols;
+    if (j0 >= T) return;
+    // rows past the end read the last one (predict's largest operand, 4096 rows a pass, keeps the offsets below 2^32)
+    uint32_t row_i[kTranshRows], row_j[kTranshCols];
+#pragma unroll
+    for (int a = 0; a < kTranshRows; ++a) row_i[a] = (uint32_t)min(i0 + a, B - 1) * (uint32_t)D;
+#pragma unroll
+    for (int b = 0; b < kTranshCols; ++b) row_j[b] = (uint32_t)min(j0 + b, T - 1) * (uint32_t)D;
+    const int i = i0 + lane / kTranshCols, j = j0 + lane % kTranshCols;  // the output whose totals this lane ends up with
+    const bool live = i < B && j < T;
+    const size_t out = (size_t)i * T + j;
+
+    // two neighbouring tails at a time
+    constexpr int kPairs = kTranshCols / 2;
+    f32x2 s2[kTranshRows][kPairs];
+#pragma unroll
+    for (int a = 0; a < kTranshRows; ++a)
+#pragma unroll
+        for (int b = 0; b < kPairs; ++b) s2[a][b] = 0ull;
+    for (int k = lane; k < D; k += 32) {
+        f32x2 t[kPairs];
+#pragma unroll
+        for (int b = 0; b < kPairs; ++b) t[b] = pack2(tails[row_j[2 * b] + k], tails[row_j[2 * b + 1] + k]);
+#pragma unroll
+        for (int a = 0; a < kTranshRows; ++a) {
+            const float n = nrm[row_i[a] + k];
+#pragma unroll
+            for (int b = 0; b < kPairs; ++b) s2[a][b] = fma2(pack2(n, n), t[b], s2[a][b]);
+        }
     }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int j = blockIdx.y * 8 + warp; j < T; j += gridDim.y * 8) {
-        const float* __restrict__ t = tails + (size_t)j * D;
-        for (int a = 0; a < rows; ++a) {
-            float s = 0.f;
-            for (int k = lane; k < D; k += 32) s += sn[a * D + k] * t[k];
-            s = warp_sum(s);
-            float dist = 0.f, u = 0.f;
-            for (int k = lane; k < D; k += 32) {
-                const float n = sn[a * D + k], e = sp[a * D + k] - t[k] + n * s;
-                dist += fabsf(e);
-                u += e > 0.f ? n : (e < 0.f ? -n : 0.f);
+    float sums[32];
+    auto spread = [&](const f32x2 (&v)[kTranshRows][kPairs]) {
+#pragma unroll
+        for (int a = 0; a < kTranshRows; ++a)
+#pragma unroll
+            for (int b = 0; b < kPairs; ++b) {
+                const float2 f = unpack2(v[a][b]);
+                sums[a * kTranshCols + 2 * b] = f.x;
+                sums[a * kTranshCols + 2 * b + 1] = f.y;
             }
-            dist = warp_sum(dist);
-            u = warp_sum(u);
-            if (lane == 0) {
-                const size_t o = (size_t)(i0 + a) * T + j;
-                raw[o] = dist;
-                if (S) S[o] = s;
-                if (U) U[o] = u;
+    };
+    spread(s2);
+    const float s_mine = reduce_to_lanes(sums);
+    if (BACKWARD && live) S[out] = s_mine;
+    f32x2 u2[kTranshRows][kPairs];
+#pragma unroll
+    for (int a = 0; a < kTranshRows; ++a)
+#pragma unroll
+        for (int b = 0; b < kPairs; ++b) {
+            const int o = a * kTranshCols + 2 * b;
+            s2[a][b] = pack2(__shfl_sync(0xffffffffu, s_mine, o), __shfl_sync(0xffffffffu, s_mine, o + 1));
+            sums[o] = sums[o + 1] = 0.f;
+            u2[a][b] = 0ull;
+        }
+    for (int k = lane; k < D; k += 32) {
+        f32x2 t[kPairs];
+#pragma unroll
+        for (int b = 0; b < kPairs; ++b) t[b] = pack2(tails[row_j[2 * b] + k], tails[row_j[2 * b + 1] + k]);
+#pragma unroll
+        for (int a = 0; a < kTranshRows; ++a) {
+            const float p = pt[row_i[a] + k], n = nrm[row_i[a] + k];
+            const f32x2 pp = pack2(p, p), nn = pack2(n, n);
+#pragma unroll
+            for (int b = 0; b < kPairs; ++b) {
+                const int o = a * kTranshCols + 2 * b;
+                const f32x2 e = fma2(nn, s2[a][b], sub2(pp, t[b]));
+                const float2 f = unpack2(e);
+                sums[o] += fabsf(f.x);
+                sums[o + 1] += fabsf(f.y);
+                if (BACKWARD) u2[a][b] = fma2(nn, sign2(e), u2[a][b]);
             }
         }
+    }
+    const float dist = reduce_to_lanes(sums);
+    if (live) raw[out] = dist;
+    if (BACKWARD) {
+        spread(u2);
+        const float total = reduce_to_lanes(sums);
+        if (live) U[out] = total;
     }
 }
 
-// Gradients of the distances times C [B, T] (C = d loss / d raw):
-//   rows i (blockIdx.x < B):  d_pt_ik = sum_j C_ij sg_ijk,   d_n_ik = sum_j C_ij (sg_ijk S_ij + U_ij t_jk)
-//   rows j (the others):      d_t_jk  = sum_i C_ij (-sg_ijk + U_ij n_ik), stored to the shard that owns tail j
-// with sg_ijk = sign(pt_ik - t_jk + n_ik S_ij) recomputed.  One block per output row, a thread per column.
-static __global__ void __launch_bounds__(128)
-k_transh_bwd(const float* __restrict__ pt, const float* __restrict__ nrm, const float* __restrict__ tails, const float* __restrict__ C,
-             const float* __restrict__ S, const float* __restrict__ U, float* __restrict__ d_pt, float* __restrict__ d_n,
-             float* const* __restrict__ d_tail_blocks, int block_rows, int B, int T, int D) {
-    grid_dependency_sync();
-    const int m = blockIdx.x;
-    if (m < B) {
-        const int i = m;
-        for (int k = threadIdx.x; k < D; k += 128) {
-            const float p = pt[(size_t)i * D + k], n = nrm[(size_t)i * D + k];
-            float acc_p = 0.f, acc_n = 0.f;
-            for (int j = 0; j < T; ++j) {
-                const size_t o = (size_t)i * T + j;
-                const float c = C[o], s = S[o], u = U[o], t = tails[(size_t)j * D + k];
-                const float e = p - t + n * s;
-                const float sg = e > 0.f ? 1.f : (e < 0.f ? -1.f : 0.f);
-                acc_p += c * sg;
-                acc_n += c * (sg * s + u * t);
+// S and U null: the distances alone (predict).
+inline cudaError_t launch_transh_score(const float* pt, const float* nrm, const float* tails, float* raw, float* S, float* U, int B, int T, int D,
+                                       const ExchangeSync& sync, cudaStream_t stream) {
+    constexpr int kCols = kTranshCols * kTranshWarps;
+    const dim3 grid((B + kTranshRows - 1) / kTranshRows, (T + kCols - 1) / kCols), block(32 * kTranshWarps);
+    if (S) return launch_dependent(k_transh_score<true>, grid, block, 0, stream, pt, nrm, tails, raw, S, U, B, T, D, sync);
+    return launch_dependent(k_transh_score<false>, grid, block, 0, stream, pt, nrm, tails, raw, S, U, B, T, D, sync);
+}
+
+// Gradients of the distances times C [B, T] (C = d loss / d raw), with sg_ijk = sign(pt_ik - t_jk + n_ik S_ij):
+//   rows i:  d_pt_ik = sum_j C_ij sg_ijk,   d_n_ik = sum_j C_ij (sg_ijk S_ij + U_ij t_jk)
+//   rows j:  d_t_jk  = sum_i C_ij (U_ij n_ik - sg_ijk), stored to the shard that owns tail j
+// In k_pair_bwd's form: 64 columns per block, two per lane, sums in order, the operands staged one chunk ahead.  The
+// first blocks take the rows i (one per warp, chunks of 64 tails), the others the rows j (two per warp, which share the
+// reads of pt and n; chunks of 32 triples).  512 x 768 x 128: 153 us with a block per output row and a thread per column.
+struct TranshBwdArgs {
+    const float *pt, *nrm, *tails, *C, *S, *U;
+    float *d_pt, *d_n;
+    float* const* d_tail_blocks;
+    int block_rows, B, T, D, blocks_i;
+};
+constexpr int kTranshChunkI = 64, kTranshChunkJ = 32;
+constexpr int kTranshStage = 3 * kPairWarps * kTranshChunkI + kTranshChunkI * kPairCols;  // floats of one chunk
+static_assert(3 * 2 * kPairWarps * kTranshChunkJ + 2 * kTranshChunkJ * kPairCols <= kTranshStage, "both kinds of rows use the same memory");
+
+__device__ __forceinline__ void transh_bwd_triples(const TranshBwdArgs& g, int block, float (*smem)[kTranshStage]) {
+    constexpr int kChunk = kTranshChunkI, kPlane = kPairWarps * kChunk;
+    const int D = g.D, T = g.T, col_tiles = (D + kPairCols - 1) / kPairCols;
+    const int i0 = block / col_tiles * kPairWarps, k0 = block % col_tiles * kPairCols;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = i0 + warp, k = k0 + lane * 2;
+    const bool t_vec = (D & 3) == 0, c_vec = (T & 3) == 0;
+    auto stage = [&](int j0, float* to) {
+        const float* planes[3] = {g.C, g.S, g.U};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) stage_rows<kPairWarps, kChunk>(to + q * kPlane, planes[q] + (size_t)i0 * T + j0, T, g.B - i0, T - j0, c_vec);
+        stage_rows<kChunk, kPairCols>(to + 3 * kPlane, g.tails + (size_t)j0 * D + k0, D, T - j0, D - k0, t_vec);
+    };
+    f32x2 p = 0ull, n = 0ull, acc_p = 0ull, acc_n = 0ull;
+    if (i < g.B) {
+        p = load_pair(g.pt + (size_t)i * D, k, D);
+        n = load_pair(g.nrm + (size_t)i * D, k, D);
+    }
+    stage(0, smem[0]);
+    stage_commit();
+    for (int j0 = 0, half = 0; j0 < T; j0 += kChunk, half ^= 1) {
+        if (j0 + kChunk < T) stage(j0 + kChunk, smem[half ^ 1]);
+        stage_commit();
+        stage_wait_previous();
+        __syncthreads();
+        const float* c = smem[half] + warp * kChunk;
+        const float* t = smem[half] + 3 * kPlane + lane * 2;
+#pragma unroll 2
+        for (int j = 0; j < kChunk; j += 4) {
+            const float4 qc = load4(c + j), qs = load4(c + kPlane + j), qu = load4(c + 2 * kPlane + j);
+            const float cj[4] = {qc.x, qc.y, qc.z, qc.w}, sj[4] = {qs.x, qs.y, qs.z, qs.w}, uj[4] = {qu.x, qu.y, qu.z, qu.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const f32x2 tj = *reinterpret_cast<const f32x2*>(t + (j + u) * kPairCols);
+                const f32x2 cc = pack2(cj[u], cj[u]), ss = pack2(sj[u], sj[u]), uu = pack2(uj[u], uj[u]);
+                const f32x2 sg = sign2(fma2(n, ss, sub2(p, tj)));
+                acc_p = fma2(cc, sg, acc_p);
+                acc_n = fma2(cc, fma2(sg, ss, mul2(uu, tj)), acc_n);
             }
-            d_pt[(size_t)i * D + k] = acc_p;
-            d_n[(size_t)i * D + k] = acc_n;
         }
-        return;
+        __syncthreads();
     }
-    const int j = m - B;
-    float* __restrict__ dst = d_tail_blocks[j / block_rows] + (size_t)(j % block_rows) * D;
-    for (int k = threadIdx.x; k < D; k += 128) {
-        const float t = tails[(size_t)j * D + k];
-        float acc = 0.f;
-        for (int i = 0; i < B; ++i) {
-            const size_t o = (size_t)i * T + j;
-            const float c = C[o], s = S[o], u = U[o], n = nrm[(size_t)i * D + k];
-            const float e = pt[(size_t)i * D + k] - t + n * s;
-            const float sg = e > 0.f ? 1.f : (e < 0.f ? -1.f : 0.f);
-            acc += c * (u * n - sg);
+    if (i >= g.B) return;
+    store_pair(g.d_pt + (size_t)i * D, k, D, acc_p);
+    store_pair(g.d_n + (size_t)i * D, k, D, acc_n);
+}
+
+__device__ __forceinline__ void transh_bwd_tails(const TranshBwdArgs& g, int block, float (*smem)[kTranshStage]) {
+    constexpr int kChunk = kTranshChunkJ, kRows = 2 * kPairWarps, kPlane = kRows * kChunk, kWide = kChunk * kPairCols;
+    const int D = g.D, T = g.T, B = g.B, col_tiles = (D + kPairCols - 1) / kPairCols;
+    const int j0 = block / col_tiles * kRows, k0 = block % col_tiles * kPairCols;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = j0 + 2 * warp, k = k0 + lane * 2;
+    const bool vec = (D & 3) == 0, c_vec = (T & 3) == 0;
+    auto stage = [&](int i0, float* to) {
+        const float* planes[3] = {g.C, g.S, g.U};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) stage_rows<kChunk, kRows>(to + q * kPlane, planes[q] + (size_t)i0 * T + j0, T, B - i0, T - j0, c_vec);
+        stage_rows<kChunk, kPairCols>(to + 3 * kPlane, g.pt + (size_t)i0 * D + k0, D, B - i0, D - k0, vec);
+        stage_rows<kChunk, kPairCols>(to + 3 * kPlane + kWide, g.nrm + (size_t)i0 * D + k0, D, B - i0, D - k0, vec);
+    };
+    f32x2 t[2], acc[2] = {0ull, 0ull};
+#pragma unroll
+    for (int r = 0; r < 2; ++r) t[r] = j + r < T ? load_pair(g.tails + (size_t)(j + r) * D, k, D) : 0ull;
+    stage(0, smem[0]);
+    stage_commit();
+    for (int i0 = 0, half = 0; i0 < B; i0 += kChunk, half ^= 1) {
+        if (i0 + kChunk < B) stage(i0 + kChunk, smem[half ^ 1]);
+        stage_commit();
+        stage_wait_previous();
+        __syncthreads();
+        const float* c = smem[half] + 2 * warp;
+        const float* p = smem[half] + 3 * kPlane + lane * 2;
+#pragma unroll 4
+        for (int i = 0; i < kChunk; ++i) {
+            const f32x2 pi = *reinterpret_cast<const f32x2*>(p + i * kPairCols), ni = *reinterpret_cast<const f32x2*>(p + kWide + i * kPairCols);
+            const float2 qc = *reinterpret_cast<const float2*>(c + i * kRows), qs = *reinterpret_cast<const float2*>(c + kPlane + i * kRows),
+                         qu = *reinterpret_cast<const float2*>(c + 2 * kPlane + i * kRows);
+            const float cj[2] = {qc.x, qc.y}, sj[2] = {qs.x, qs.y}, uj[2] = {qu.x, qu.y};
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const f32x2 sg = sign2(fma2(ni, pack2(sj[r], sj[r]), sub2(pi, t[r])));
+                acc[r] = fma2(pack2(cj[r], cj[r]), fma2(pack2(uj[r], uj[r]), ni, sg ^ 0x8000000080000000ull), acc[r]);
+            }
         }
-        dst[k] = acc;
+        __syncthreads();
     }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+        if (j + r < T) store_pair(g.d_tail_blocks[(j + r) / g.block_rows] + (size_t)((j + r) % g.block_rows) * D, k, D, acc[r]);
+}
+
+static __global__ void __launch_bounds__(32 * kPairWarps, 3) k_transh_bwd(TranshBwdArgs g) {
+    grid_dependency_sync();
+    __shared__ __align__(16) float smem[2][kTranshStage];
+    if ((int)blockIdx.x < g.blocks_i) transh_bwd_triples(g, blockIdx.x, smem);
+    else transh_bwd_tails(g, (int)blockIdx.x - g.blocks_i, smem);
+}
+
+inline cudaError_t launch_transh_bwd(TranshBwdArgs g, cudaStream_t stream) {
+    const int col_tiles = (g.D + kPairCols - 1) / kPairCols;
+    g.blocks_i = (g.B + kPairWarps - 1) / kPairWarps * col_tiles;
+    const int blocks_j = (g.T + 2 * kPairWarps - 1) / (2 * kPairWarps) * col_tiles;
+    return launch_dependent(k_transh_bwd, dim3(g.blocks_i + blocks_j), dim3(32 * kPairWarps), 0, stream, g);
 }
 
 // Backward of k_transh_predict for triple i:
