@@ -166,36 +166,40 @@ inline cudaError_t launch_transh_score(const float* pt, const float* nrm, const 
 // Gradients of the distances times C [B, T] (C = d loss / d raw), with sg_ijk = sign(pt_ik - t_jk + n_ik S_ij):
 //   rows i:  d_pt_ik = sum_j C_ij sg_ijk,   d_n_ik = sum_j C_ij (sg_ijk S_ij + U_ij t_jk)
 //   rows j:  d_t_jk  = sum_i C_ij (U_ij n_ik - sg_ijk), stored to the shard that owns tail j
-// In k_pair_bwd's form: 64 columns per block, two per lane, sums in order, the operands staged one chunk ahead.  The
-// first blocks take the rows i (one per warp, chunks of 64 tails), the others the rows j (two per warp, which share the
-// reads of pt and n; chunks of 32 triples).  512 x 768 x 128: 153 us with a block per output row and a thread per column.
+// In k_pair_bwd's form (sums in order, the operands staged one chunk ahead) but with one column per lane, 32 per block:
+// a packed instruction occupies the FP32 pipe twice as long, so pairs would only halve the warps that hide latency.  The first blocks take the rows i (one per
+// warp, chunks of 64 tails), the others the rows j (two per warp, which share the reads of pt and n; chunks of 32
+// triples).  512 x 768 x 128: 153 us with a block per output row and a thread per column, 87 us with pairs,
+// 61 us this way.
 struct TranshBwdArgs {
     const float *pt, *nrm, *tails, *C, *S, *U;
     float *d_pt, *d_n;
     float* const* d_tail_blocks;
     int block_rows, B, T, D, blocks_i;
 };
-constexpr int kTranshChunkI = 64, kTranshChunkJ = 32;
-constexpr int kTranshStage = 3 * kPairWarps * kTranshChunkI + kTranshChunkI * kPairCols;  // floats of one chunk
-static_assert(3 * 2 * kPairWarps * kTranshChunkJ + 2 * kTranshChunkJ * kPairCols <= kTranshStage, "both kinds of rows use the same memory");
+constexpr int kTranshBwdCols = 32, kTranshChunkI = 64, kTranshChunkJ = 32;
+constexpr int kTranshStage = 3 * kPairWarps * kTranshChunkI + kTranshChunkI * kTranshBwdCols;  // floats of one chunk
+static_assert(3 * 2 * kPairWarps * kTranshChunkJ + 2 * kTranshChunkJ * kTranshBwdCols <= kTranshStage, "both kinds of rows use the same memory");
+
+__device__ __forceinline__ float sign_of(float e) {
+    const float inf = __int_as_float(0x7f800000);
+    return positive(e, inf) - positive(e, -inf);
+}
 
 __device__ __forceinline__ void transh_bwd_triples(const TranshBwdArgs& g, int block, float (*smem)[kTranshStage]) {
-    constexpr int kChunk = kTranshChunkI, kPlane = kPairWarps * kChunk;
-    const int D = g.D, T = g.T, col_tiles = (D + kPairCols - 1) / kPairCols;
-    const int i0 = block / col_tiles * kPairWarps, k0 = block % col_tiles * kPairCols;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = i0 + warp, k = k0 + lane * 2;
-    const bool t_vec = (D & 3) == 0, c_vec = (T & 3) == 0;
+    constexpr int kChunk = kTranshChunkI, kPlane = kPairWarps * kChunk, kCols = kTranshBwdCols;
+    const int D = g.D, T = g.T, col_tiles = (D + kCols - 1) / kCols;
+    const int i0 = block / col_tiles * kPairWarps, k0 = block % col_tiles * kCols;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = i0 + warp, k = k0 + lane;
+    const bool t_vec = (D & 3) == 0, c_vec = (T & 3) == 0, live = i < g.B && k < D;
     auto stage = [&](int j0, float* to) {
         const float* planes[3] = {g.C, g.S, g.U};
 #pragma unroll
         for (int q = 0; q < 3; ++q) stage_rows<kPairWarps, kChunk>(to + q * kPlane, planes[q] + (size_t)i0 * T + j0, T, g.B - i0, T - j0, c_vec);
-        stage_rows<kChunk, kPairCols>(to + 3 * kPlane, g.tails + (size_t)j0 * D + k0, D, T - j0, D - k0, t_vec);
+        stage_rows<kChunk, kCols>(to + 3 * kPlane, g.tails + (size_t)j0 * D + k0, D, T - j0, D - k0, t_vec);
     };
-    f32x2 p = 0ull, n = 0ull, acc_p = 0ull, acc_n = 0ull;
-    if (i < g.B) {
-        p = load_pair(g.pt + (size_t)i * D, k, D);
-        n = load_pair(g.nrm + (size_t)i * D, k, D);
-    }
+    const float p = live ? g.pt[(size_t)i * D + k] : 0.f, n = live ? g.nrm[(size_t)i * D + k] : 0.f;
+    float acc_p = 0.f, acc_n = 0.f;
     stage(0, smem[0]);
     stage_commit();
     for (int j0 = 0, half = 0; j0 < T; j0 += kChunk, half ^= 1) {
@@ -204,43 +208,41 @@ __device__ __forceinline__ void transh_bwd_triples(const TranshBwdArgs& g, int b
         stage_wait_previous();
         __syncthreads();
         const float* c = smem[half] + warp * kChunk;
-        const float* t = smem[half] + 3 * kPlane + lane * 2;
+        const float* t = smem[half] + 3 * kPlane + lane;
 #pragma unroll 2
         for (int j = 0; j < kChunk; j += 4) {
             const float4 qc = load4(c + j), qs = load4(c + kPlane + j), qu = load4(c + 2 * kPlane + j);
             const float cj[4] = {qc.x, qc.y, qc.z, qc.w}, sj[4] = {qs.x, qs.y, qs.z, qs.w}, uj[4] = {qu.x, qu.y, qu.z, qu.w};
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const f32x2 tj = *reinterpret_cast<const f32x2*>(t + (j + u) * kPairCols);
-                const f32x2 cc = pack2(cj[u], cj[u]), ss = pack2(sj[u], sj[u]), uu = pack2(uj[u], uj[u]);
-                const f32x2 sg = sign2(fma2(n, ss, sub2(p, tj)));
-                acc_p = fma2(cc, sg, acc_p);
-                acc_n = fma2(cc, fma2(sg, ss, mul2(uu, tj)), acc_n);
+                const float tj = t[(j + u) * kCols], sg = sign_of(fmaf(n, sj[u], p - tj));
+                acc_p = fmaf(cj[u], sg, acc_p);
+                acc_n = fmaf(cj[u], fmaf(sg, sj[u], uj[u] * tj), acc_n);
             }
         }
         __syncthreads();
     }
-    if (i >= g.B) return;
-    store_pair(g.d_pt + (size_t)i * D, k, D, acc_p);
-    store_pair(g.d_n + (size_t)i * D, k, D, acc_n);
+    if (!live) return;
+    g.d_pt[(size_t)i * D + k] = acc_p;
+    g.d_n[(size_t)i * D + k] = acc_n;
 }
 
 __device__ __forceinline__ void transh_bwd_tails(const TranshBwdArgs& g, int block, float (*smem)[kTranshStage]) {
-    constexpr int kChunk = kTranshChunkJ, kRows = 2 * kPairWarps, kPlane = kRows * kChunk, kWide = kChunk * kPairCols;
-    const int D = g.D, T = g.T, B = g.B, col_tiles = (D + kPairCols - 1) / kPairCols;
-    const int j0 = block / col_tiles * kRows, k0 = block % col_tiles * kPairCols;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = j0 + 2 * warp, k = k0 + lane * 2;
+    constexpr int kChunk = kTranshChunkJ, kRows = 2 * kPairWarps, kPlane = kRows * kChunk, kCols = kTranshBwdCols, kWide = kChunk * kCols;
+    const int D = g.D, T = g.T, B = g.B, col_tiles = (D + kCols - 1) / kCols;
+    const int j0 = block / col_tiles * kRows, k0 = block % col_tiles * kCols;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = j0 + 2 * warp, k = k0 + lane;
     const bool vec = (D & 3) == 0, c_vec = (T & 3) == 0;
     auto stage = [&](int i0, float* to) {
         const float* planes[3] = {g.C, g.S, g.U};
 #pragma unroll
         for (int q = 0; q < 3; ++q) stage_rows<kChunk, kRows>(to + q * kPlane, planes[q] + (size_t)i0 * T + j0, T, B - i0, T - j0, c_vec);
-        stage_rows<kChunk, kPairCols>(to + 3 * kPlane, g.pt + (size_t)i0 * D + k0, D, B - i0, D - k0, vec);
-        stage_rows<kChunk, kPairCols>(to + 3 * kPlane + kWide, g.nrm + (size_t)i0 * D + k0, D, B - i0, D - k0, vec);
+        stage_rows<kChunk, kCols>(to + 3 * kPlane, g.pt + (size_t)i0 * D + k0, D, B - i0, D - k0, vec);
+        stage_rows<kChunk, kCols>(to + 3 * kPlane + kWide, g.nrm + (size_t)i0 * D + k0, D, B - i0, D - k0, vec);
     };
-    f32x2 t[2], acc[2] = {0ull, 0ull};
+    float t[2], acc[2] = {0.f, 0.f};
 #pragma unroll
-    for (int r = 0; r < 2; ++r) t[r] = j + r < T ? load_pair(g.tails + (size_t)(j + r) * D, k, D) : 0ull;
+    for (int r = 0; r < 2; ++r) t[r] = j + r < T && k < D ? g.tails[(size_t)(j + r) * D + k] : 0.f;
     stage(0, smem[0]);
     stage_commit();
     for (int i0 = 0, half = 0; i0 < B; i0 += kChunk, half ^= 1) {
@@ -249,27 +251,24 @@ __device__ __forceinline__ void transh_bwd_tails(const TranshBwdArgs& g, int blo
         stage_wait_previous();
         __syncthreads();
         const float* c = smem[half] + 2 * warp;
-        const float* p = smem[half] + 3 * kPlane + lane * 2;
-#pragma unroll 4
+        const float* p = smem[half] + 3 * kPlane + lane;
+#pragma unroll 8
         for (int i = 0; i < kChunk; ++i) {
-            const f32x2 pi = *reinterpret_cast<const f32x2*>(p + i * kPairCols), ni = *reinterpret_cast<const f32x2*>(p + kWide + i * kPairCols);
+            const float pi = p[i * kCols], ni = p[kWide + i * kCols];
             const float2 qc = *reinterpret_cast<const float2*>(c + i * kRows), qs = *reinterpret_cast<const float2*>(c + kPlane + i * kRows),
                          qu = *reinterpret_cast<const float2*>(c + 2 * kPlane + i * kRows);
             const float cj[2] = {qc.x, qc.y}, sj[2] = {qs.x, qs.y}, uj[2] = {qu.x, qu.y};
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const f32x2 sg = sign2(fma2(ni, pack2(sj[r], sj[r]), sub2(pi, t[r])));
-                acc[r] = fma2(pack2(cj[r], cj[r]), fma2(pack2(uj[r], uj[r]), ni, sg ^ 0x8000000080000000ull), acc[r]);
-            }
+            for (int r = 0; r < 2; ++r) acc[r] = fmaf(cj[r], fmaf(uj[r], ni, -sign_of(fmaf(ni, sj[r], pi - t[r]))), acc[r]);
         }
         __syncthreads();
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r)
-        if (j + r < T) store_pair(g.d_tail_blocks[(j + r) / g.block_rows] + (size_t)((j + r) % g.block_rows) * D, k, D, acc[r]);
+        if (j + r < T && k < D) g.d_tail_blocks[(j + r) / g.block_rows][(size_t)((j + r) % g.block_rows) * D + k] = acc[r];
 }
 
-static __global__ void __launch_bounds__(32 * kPairWarps, 3) k_transh_bwd(TranshBwdArgs g) {
+static __global__ void __launch_bounds__(32 * kPairWarps, 4) k_transh_bwd(TranshBwdArgs g) {
     grid_dependency_sync();
     __shared__ __align__(16) float smem[2][kTranshStage];
     if ((int)blockIdx.x < g.blocks_i) transh_bwd_triples(g, blockIdx.x, smem);
@@ -277,7 +276,7 @@ static __global__ void __launch_bounds__(32 * kPairWarps, 3) k_transh_bwd(Transh
 }
 
 inline cudaError_t launch_transh_bwd(TranshBwdArgs g, cudaStream_t stream) {
-    const int col_tiles = (g.D + kPairCols - 1) / kPairCols;
+    const int col_tiles = (g.D + kTranshBwdCols - 1) / kTranshBwdCols;
     g.blocks_i = (g.B + kPairWarps - 1) / kPairWarps * col_tiles;
     const int blocks_j = (g.T + 2 * kPairWarps - 1) / (2 * kPairWarps) * col_tiles;
     return launch_dependent(k_transh_bwd, dim3(g.blocks_i + blocks_j), dim3(32 * kPairWarps), 0, stream, g);
