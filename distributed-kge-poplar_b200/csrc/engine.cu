@@ -2289,7 +2289,9 @@ void Engine::ensure_predict_buffers() {
     // Rows per pass over the table.  On the tensor cores: 148 tiles of 128 rows, so that the hidden
     // rows' contraction (2 column tiles) and the scores' (10 query tiles at 1250 queries) both fill
     // whole waves of 148 blocks.
-    predict_chunk_ = predict_planes_ ? 148u * 128u : 4096u;
+    // Elsewhere as many as 64 MB of scores hold, between 4096 and 65536: few queries make short kernels.
+    predict_chunk_ = predict_planes_ ? 148u * 128u : (unsigned)std::min<size_t>(65536, std::max<size_t>(4096, ((size_t)16 << 20) / Q / 128 * 128));
+    predict_chunk_ = std::min(predict_chunk_, (unsigned)round_up(cfg_.n_entity, 128));
     if (const char* v = std::getenv("KGE_PREDICT_PASS_ROWS")) predict_chunk_ = std::max(64u, (unsigned)std::atoi(v) / 4u * 4u);
     p_chunk_hidden_ = (float*)device_alloc((size_t)predict_chunk_ * D * 4);
     p_raw_ = (float*)device_alloc(Q * predict_chunk_ * 4);
@@ -2321,9 +2323,13 @@ void Engine::ensure_predict_buffers() {
 // full bandwidth, then one warp per query on what it left.
 void Engine::launch_topk(ShardBuffers& b, unsigned c, uint32_t start, uint32_t last, const TopkParams& tp, bool filtered) {
     const unsigned Q = (unsigned)tp.n_query;
-    const dim3 fgrid(std::max(1u, std::min(ceil_div(c, 4 * 256), 8u)), Q);
-    if (!filtered)  // else the score kernel's epilogue has left the candidates
+    if (start == 1) {  // nothing ranked yet: parts of at least 512 scores, as many lists as the candidates have room for
+        const unsigned parts = std::max(1u, std::min({(unsigned)kTopkCandidates / (unsigned)tp.n_best, ceil_div(c, 512u), 64u}));
+        KGE_LAUNCH("predict_topk", k_topk_seed<<<dim3(ceil_div(Q, 4), parts), 128, 0, stream_>>>(p_raw_, (int)c, start, last, p_cand_, p_cand_count_, tp));
+    } else if (!filtered) {  // else the score kernel's epilogue has left the candidates
+        const dim3 fgrid(std::max(1u, std::min(ceil_div(c, 4 * 256), 8u)), Q);
         KGE_LAUNCH("predict_topk", k_topk_filter<<<fgrid, 256, 0, stream_>>>(p_raw_, (int)c, start, last, b.topk_state, b.topk_count, p_cand_, p_cand_count_, tp));
+    }
     KGE_LAUNCH("predict_topk", k_topk_update<<<ceil_div(Q, 4), 128, 0, stream_>>>(p_raw_, (int)c, start, last, b.topk_state, b.topk_count, tp, p_cand_,
                                                                                  p_cand_count_));
 }
@@ -2432,13 +2438,20 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
         KGE_CUDA(cudaGetLastError());
     }
     launch_barrier();
-    const size_t result_bytes = n * cfg_.n_shard * hr * nb * 4;
-    KGE_CUDA(cudaMemcpyAsync(scores.data, arena_ + arena_offset_predict(1), result_bytes, cudaMemcpyDeviceToHost, stream_));
-    KGE_CUDA(cudaMemcpyAsync(indices.data, arena_ + arena_offset_predict(2), result_bytes, cudaMemcpyDeviceToHost, stream_));
-    KGE_CUDA(cudaStreamSynchronize(stream_));
+    const size_t result_bytes = n * cfg_.n_shard * hr * nb * 4, slot = round_up(result_bytes, 256);
+    if (2 * slot + 256 <= PinnedPool::kBlock) {  // results and status words in one wait
+        const PinnedBlock block;
+        KGE_CUDA(cudaMemcpyAsync(block.data(), arena_ + arena_offset_predict(1), slot + result_bytes, cudaMemcpyDeviceToHost, stream_));
+        check_device_status();
+        std::memcpy(scores.data, block.data(), result_bytes);
+        std::memcpy(indices.data, block.data() + slot, result_bytes);
+    } else {
+        copy_out(scores.data, arena_ + arena_offset_predict(1), result_bytes, result_bytes, 1);
+        copy_out(indices.data, arena_ + arena_offset_predict(2), result_bytes, result_bytes, 1);
+        check_device_status();
+    }
     timing_collect();
     last_launches_ = launch_counter_;
-    check_device_status();
 }
 
 // One pass of predict on the tensor cores: hidden rows of the table rows [start, start + c) as the

@@ -620,6 +620,111 @@ k_score_wide(const float* __restrict__ P, const float* __restrict__ Tl, float* _
     }
 }
 
+// The same scores where there are enough of them to fill the GPU with tiles (ranking): a block owns 64 x 128 outputs, its
+// 8 warps 32 x 32 each, with k_score_wide's register tile; all of them walk all of k in chunks of 32 staged one ahead.
+// Each chunk is summed by itself and added to the total, as k_score_wide adds its warps' chunks.  Bound by the FP32
+// pipe.  (k_score_wide divides the chunks over its warps, half of which have none at 100 columns, and its blocks pay a
+// reduction for every 1024 outputs: 32 queries x 4 shards x 4096 rows x 100 columns took 13 us a pass.)
+constexpr int kScoreTileP = 64, kScoreTileT = 128;
+constexpr int kScoreTileStage = (kScoreTileP + kScoreTileT) * kScoreStride;
+constexpr size_t kScoreTileSmem = 2 * kScoreTileStage * sizeof(float);
+
+template <int FN>
+__global__ void __launch_bounds__(256, 2)
+k_score_tile(const float* __restrict__ P, const float* __restrict__ Tl, float* __restrict__ raw, int B, int T, int D) {
+    grid_dependency_sync();
+    extern __shared__ __align__(16) float score_smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ty = lane >> 2, tx = lane & 3;
+    const int i0 = blockIdx.y * kScoreTileP, j0 = blockIdx.x * kScoreTileT;
+    auto stage = [&](int k0, float* to) {
+#pragma unroll
+        for (int it = 0; it < (kScoreTileP + kScoreTileT) * 8 / 256; ++it) {
+            const int q = threadIdx.x + it * 256, row = q >> 3, k4 = (q & 7) * 4;
+            const bool is_p = row < kScoreTileP;
+            const int g = is_p ? i0 + row : j0 + row - kScoreTileP;
+            float* d = to + row * kScoreStride + k4;
+            if (g < (is_p ? B : T) && k0 + k4 < D) score_copy16(d, (is_p ? P : Tl) + (size_t)g * D + k0 + k4);
+            else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    float total[4][8];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 8; ++b) total[a][b] = 0.f;
+    const int row_p = (warp >> 2) * 32 + ty, row_t = kScoreTileP + (warp & 3) * 32 + tx;
+    stage(0, score_smem);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int k0 = 0, half = 0; k0 < D; k0 += 32, half ^= 1) {
+        if (k0 + 32 < D) stage(k0 + 32, score_smem + (half ^ 1) * kScoreTileStage);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const float* Ps = score_smem + half * kScoreTileStage + row_p * kScoreStride;
+        const float* Ts = score_smem + half * kScoreTileStage + row_t * kScoreStride;
+        float acc[4][8];
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
+#pragma unroll 1
+        for (int k4 = 0; k4 < 32; k4 += 4) {
+            float4 pv[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) pv[a] = load4(Ps + 8 * a * kScoreStride + k4);
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const float4 tv = load4(Ts + 4 * b * kScoreStride + k4);
+                const float tr[4] = {tv.x, tv.y, tv.z, tv.w};
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    const float pr[4] = {pv[a].x, pv[a].y, pv[a].z, pv[a].w};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        if (FN == DIST_L1) {
+                            acc[a][b] += fabsf(pr[c] - tr[c]);
+                        } else if (FN == DIST_L2) {
+                            const float d = pr[c] - tr[c];
+                            acc[a][b] = fmaf(d, d, acc[a][b]);
+                        } else {
+                            acc[a][b] = fmaf(pr[c], tr[c], acc[a][b]);
+                        }
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 8; ++b) total[a][b] += acc[a][b];
+        __syncthreads();
+    }
+    // through shared memory, so that whole rows are stored
+    constexpr int kOut = kScoreTileT + 4;
+    static_assert(kScoreTileP * kOut <= 2 * kScoreTileStage, "the outputs fit");
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 8; ++b)
+            score_smem[(row_p + 8 * a) * kOut + row_t - kScoreTileP + 4 * b] = FN == DIST_L2 ? sqrtf(total[a][b]) : total[a][b];
+    __syncthreads();
+    const bool vec = (T & 3) == 0;
+    for (int q = threadIdx.x; q < kScoreTileP * kScoreTileT / 4; q += 256) {
+        const int row = q / (kScoreTileT / 4), col = q % (kScoreTileT / 4) * 4, i = i0 + row, j = j0 + col;
+        if (i >= B || j >= T) continue;
+        const float4 v = load4(score_smem + row * kOut + col);
+        float* dst = raw + (size_t)i * T + j;
+        if (vec) {
+            store4(dst, v);
+        } else {
+            const float t[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (j + u < T) dst[u] = t[u];
+        }
+    }
+}
+
 // Picks the kernel: the 16-byte-copy form when the rows allow it, the general form otherwise.
 // `sync` with world > 1: the kernel waits for the tail rows of the other processes (only the
 // 16-byte-copy form can; returns cudaErrorNotSupported otherwise so that the caller waits first).
@@ -635,9 +740,14 @@ inline cudaError_t launch_score(const float* P, const float* Tl, float* raw, int
     const int slot = current_device_slot();
     if (slot < 0 || !configured[slot]) {
         cudaError_t err = cudaFuncSetAttribute(k_score_wide<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreWideSmem);
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(k_score_tile<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreTileSmem);
         if (err != cudaSuccess) return err;
         if (slot >= 0) configured[slot] = true;
     }
+    // whole tiles from two blocks per SM on; below that, and where tails are waited for, the k range is divided too
+    const dim3 tiles((T + kScoreTileT - 1) / kScoreTileT, (B + kScoreTileP - 1) / kScoreTileP);
+    if (sync.world <= 1 && (size_t)tiles.x * tiles.y >= 2 * 148)
+        return launch_dependent(k_score_tile<FN>, tiles, dim3(256), kScoreTileSmem, stream, P, Tl, raw, B, T, D);
     return launch_dependent(k_score_wide<FN>, dim3((T + 31) / 32, (B + 31) / 32), dim3(32 * kScoreWarps), kScoreWideSmem, stream,
                             P, Tl, raw, B, T, D, sync);
 }
@@ -2155,25 +2265,44 @@ __device__ __forceinline__ float topk_score(unsigned long long key) {
 }
 __device__ __forceinline__ uint32_t topk_index(unsigned long long key) { return ~(uint32_t)key; }
 
-// Sorts the warp's buffer in descending key order (empty slots hold key 0, which sorts last).
+// Sorts the warp's buffer in descending key order (empty slots hold key 0, which sorts last): a bitonic network on eight
+// keys per lane, key p of the network in lane p / 8, so that 21 of its 36 stages stay inside a lane and the other 15
+// exchange through shuffles.  (In shared memory, a compare-exchange per visit, a sort took 10 us, most of a merge.)
 __device__ __forceinline__ void warp_sort_desc(unsigned long long* buf) {
+    constexpr int kPerLane = kTopkCapacity / 32;
     const int lane = threadIdx.x & 31;
+    unsigned long long v[kPerLane];
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < kPerLane; ++r) v[r] = buf[r * 32 + lane];  // in any order: they are about to be sorted
+    __syncwarp();
+#pragma unroll
     for (int k = 2; k <= kTopkCapacity; k <<= 1) {
+#pragma unroll
         for (int j = k >> 1; j > 0; j >>= 1) {
-            __syncwarp();
-            for (int i = lane; i < kTopkCapacity; i += 32) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = buf[i], b = buf[ixj];
-                    const bool descending = (i & k) == 0;
-                    if ((a < b) == descending) {
-                        buf[i] = b;
-                        buf[ixj] = a;
-                    }
+            if (j >= kPerLane) {
+                const bool lower = ((lane * kPerLane) & j) == 0, descending = ((lane * kPerLane) & k) == 0;
+                const bool keep_larger = lower == descending;
+#pragma unroll
+                for (int r = 0; r < kPerLane; ++r) {
+                    const unsigned long long other = __shfl_xor_sync(0xffffffffu, v[r], j / kPerLane);
+                    v[r] = (v[r] > other) == keep_larger ? v[r] : other;
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < kPerLane; ++r) {
+                    if (r & j) continue;
+                    const bool descending = ((lane * kPerLane + r) & k) == 0;
+                    const unsigned long long a = v[r], b = v[r | j];
+                    const bool swap = (a < b) == descending;
+                    v[r] = swap ? b : a;
+                    v[r | j] = swap ? a : b;
                 }
             }
         }
     }
+#pragma unroll
+    for (int r = 0; r < kPerLane; r += 2) *reinterpret_cast<ulonglong2*>(buf + lane * kPerLane + r) = make_ulonglong2(v[r], v[r + 1]);
     __syncwarp();
 }
 
@@ -2187,8 +2316,8 @@ struct TopkParams {
 // (four scores per thread) and leaves, per query, the keys that beat the query's cut-off as it
 // stands before the batch in `cand` (at most kTopkCandidates; the count goes on past that).
 // k_topk_update, one warp per query, then merges those few keys; a query whose candidates did not
-// fit (the first batches, before a cut-off exists) scans its row of scores itself, as it would
-// without the filter.  The candidates' order in `cand` depends on timing, the merged result does
+// fit scans its row of scores itself.  In a ranking's first batch, before a cut-off exists, k_topk_seed
+// takes the filter's place.  The candidates' order in `cand` depends on timing, the merged result does
 // not: it is the n_best largest keys of the old list and the candidates, and keys are unique.
 constexpr int kTopkCandidates = 1024;
 
@@ -2234,94 +2363,105 @@ k_topk_filter(const float* __restrict__ raw, int n_cols, uint32_t first_row, uin
     }
 }
 
+// One warp's list: up to kTopkCapacity keys in shared memory, sorted down to the n_best largest when it fills.
+struct TopkList {
+    unsigned long long* buf;
+    int count, n_best;
+    unsigned long long cutoff;  // keys up to it cannot be among the n_best
+
+    __device__ __noinline__ void sort() {
+        const int lane = threadIdx.x & 31;
+        warp_sort_desc(buf);
+        count = min(count, n_best);
+        for (int i = count + lane; i < kTopkCapacity; i += 32) buf[i] = 0ull;
+        __syncwarp();
+        cutoff = count >= n_best ? buf[n_best - 1] : 0ull;
+    }
+    // One key per lane (0: none).
+    __device__ __forceinline__ void add(unsigned long long key) {
+        if (__ballot_sync(0xffffffffu, key > cutoff) != 0) insert(key);
+    }
+    __device__ __noinline__ void insert(unsigned long long key) {
+        const int lane = threadIdx.x & 31;
+        if (count + 32 > kTopkCapacity) sort();
+        const bool pass = key > cutoff;
+        const unsigned mask = __ballot_sync(0xffffffffu, pass);
+        if (pass) buf[count + __popc(mask & ((1u << lane) - 1))] = key;
+        count += __popc(mask);
+        __syncwarp();
+    }
+    // The scores of columns [begin, end) of a query's row.
+    __device__ __forceinline__ void scan(const float* __restrict__ row, int begin, int end, uint32_t first_row, uint32_t last_valid_row, const TopkParams& tp) {
+        const int lane = threadIdx.x & 31;
+        constexpr int kAhead = 8;  // scores fetched before the first of them is looked at: the loads overlap
+        for (int base0 = begin; base0 < end; base0 += 32 * kAhead) {
+            float ahead[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int j = base0 + 32 * u + lane;
+                ahead[u] = j < end ? row[j] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const int j = base0 + 32 * u + lane;
+                unsigned long long key = 0ull;
+                if (j < end && first_row + (uint32_t)j <= last_valid_row)
+                    key = topk_key(tp.score_is_gamma_minus ? tp.gamma - ahead[u] : ahead[u], first_row + (uint32_t)j);
+                add(key);
+            }
+        }
+    }
+};
+
+// The first batch of a ranking, when no query has a cut-off: gridDim.y warps per query each scan a part of its row and
+// leave their n_best keys (0 for missing ones) as candidates, which k_topk_update merges like any other.  One warp per
+// query took 25 us for every 4096 scores, on as many SMs as there are groups of four queries.
+static __global__ void __launch_bounds__(128)
+k_topk_seed(const float* __restrict__ raw, int n_cols, uint32_t first_row, uint32_t last_valid_row, unsigned long long* __restrict__ cand,
+            int* __restrict__ cand_count, TopkParams tp) {
+    __shared__ __align__(16) unsigned long long buffers[4][kTopkCapacity];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * 4 + warp;
+    if (q >= tp.n_query) return;
+    TopkList list{buffers[warp], 0, tp.n_best, 0ull};
+    for (int i = lane; i < kTopkCapacity; i += 32) list.buf[i] = 0ull;
+    __syncwarp();
+    const int part = ((n_cols + (int)gridDim.y - 1) / (int)gridDim.y + 31) / 32 * 32, begin = (int)blockIdx.y * part;
+    list.scan(raw + (size_t)q * n_cols, begin, min(n_cols, begin + part), first_row, last_valid_row, tp);
+    list.sort();
+    unsigned long long* __restrict__ out = cand + (size_t)q * kTopkCandidates + (size_t)blockIdx.y * tp.n_best;
+    for (int i = lane; i < tp.n_best; i += 32) out[i] = list.buf[i];
+    if (blockIdx.y == 0 && lane == 0) cand_count[q] = (int)gridDim.y * tp.n_best;
+}
+
 // raw [n_query, n_cols] holds distances / dot products against rows first_row .. first_row+n_cols-1;
 // rows above last_valid_row are padding of the shard and are skipped (src/poplar_kge.cpp:836-842).
 // state [n_query, kTopkCapacity] keys, counts [n_query].  4 warps per block, one query each.
-// cand / cand_count (may be null): the filter's output for this batch; the counts are cleared for the next.
+// cand / cand_count: the filter's or the seed's output for this batch; the counts are cleared for the next.
 static __global__ void __launch_bounds__(128)
 k_topk_update(const float* __restrict__ raw, int n_cols, uint32_t first_row, uint32_t last_valid_row,
               unsigned long long* __restrict__ state, int* __restrict__ counts, TopkParams tp,
               const unsigned long long* __restrict__ cand, int* __restrict__ cand_count) {
-    __shared__ unsigned long long buffers[4][kTopkCapacity];
+    __shared__ __align__(16) unsigned long long buffers[4][kTopkCapacity];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int q = blockIdx.x * 4 + warp;
     if (q >= tp.n_query) return;
-    unsigned long long* buf = buffers[warp];
-    unsigned long long* mine = state + (size_t)q * kTopkCapacity;
-    int count = counts[q];
-    for (int i = lane; i < kTopkCapacity; i += 32) buf[i] = i < count ? mine[i] : 0ull;
-    __syncwarp();
-    unsigned long long cutoff = count >= tp.n_best ? buf[tp.n_best - 1] : 0ull;
-    const int n_cand = cand_count ? cand_count[q] : kTopkCandidates + 1;
-    __syncwarp();
-    if (cand_count && lane == 0) cand_count[q] = 0;
+    const int n_cand = cand_count[q];
     if (n_cand == 0) return;  // nothing in this batch beats the cut-off: the list stands
+    unsigned long long* mine = state + (size_t)q * kTopkCapacity;
+    TopkList list{buffers[warp], counts[q], tp.n_best, 0ull};
+    for (int i = lane; i < kTopkCapacity; i += 32) list.buf[i] = i < list.count ? mine[i] : 0ull;
+    __syncwarp();
+    if (list.count >= tp.n_best) list.cutoff = list.buf[tp.n_best - 1];
+    if (lane == 0) cand_count[q] = 0;
     if (n_cand <= kTopkCandidates) {
-        // the filter's keys for this query: all beat the old cut-off; the cut-off rises as they are merged
         const unsigned long long* __restrict__ keys = cand + (size_t)q * kTopkCandidates;
-        for (int base = 0; base < n_cand; base += 32) {
-            const unsigned long long key = base + lane < n_cand ? keys[base + lane] : 0ull;
-            const bool pass = key > cutoff;
-            if (__ballot_sync(0xffffffffu, pass) == 0) continue;
-            if (count + 32 > kTopkCapacity) {
-                warp_sort_desc(buf);
-                count = min(count, tp.n_best);
-                for (int i = count + lane; i < kTopkCapacity; i += 32) buf[i] = 0ull;
-                __syncwarp();
-                cutoff = count >= tp.n_best ? buf[tp.n_best - 1] : 0ull;
-            }
-            const bool still = pass && key > cutoff;
-            const unsigned mask2 = __ballot_sync(0xffffffffu, still);
-            if (still) buf[count + __popc(mask2 & ((1u << lane) - 1))] = key;
-            count += __popc(mask2);
-            __syncwarp();
-        }
-        warp_sort_desc(buf);
-        count = min(count, tp.n_best);
-        for (int i = lane; i < kTopkCapacity; i += 32) mine[i] = i < count ? buf[i] : 0ull;
-        if (lane == 0) counts[q] = count;
-        return;
+        for (int base = 0; base < n_cand; base += 32) list.add(base + lane < n_cand ? keys[base + lane] : 0ull);
+    } else {  // more than the candidate list holds
+        list.scan(raw + (size_t)q * n_cols, 0, n_cols, first_row, last_valid_row, tp);
     }
-    const float* __restrict__ row = raw + (size_t)q * n_cols;
-    constexpr int kAhead = 8;  // scores fetched before the first of them is looked at: the loads overlap
-    for (int base0 = 0; base0 < n_cols; base0 += 32 * kAhead) {
-    float ahead[kAhead];
-#pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-        const int j = base0 + 32 * u + lane;
-        ahead[u] = j < n_cols ? row[j] : 0.f;
-    }
-#pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-        const int base = base0 + 32 * u;
-        if (base >= n_cols) break;
-        const int j = base + lane;
-        unsigned long long key = 0ull;
-        if (j < n_cols && first_row + (uint32_t)j <= last_valid_row) {
-            const float v = ahead[u];
-            key = topk_key(tp.score_is_gamma_minus ? tp.gamma - v : v, first_row + (uint32_t)j);
-        }
-        const bool pass = key > cutoff;
-        const unsigned mask = __ballot_sync(0xffffffffu, pass);
-        if (mask == 0) continue;
-        if (count + 32 > kTopkCapacity) {  // no room for a full ballot: sort down to n_best first
-            warp_sort_desc(buf);
-            count = min(count, tp.n_best);
-            for (int i = count + lane; i < kTopkCapacity; i += 32) buf[i] = 0ull;
-            __syncwarp();
-            cutoff = count >= tp.n_best ? buf[tp.n_best - 1] : 0ull;
-        }
-        const bool still = pass && key > cutoff;
-        const unsigned mask2 = __ballot_sync(0xffffffffu, still);
-        if (still) buf[count + __popc(mask2 & ((1u << lane) - 1))] = key;
-        count += __popc(mask2);
-        __syncwarp();
-    }
-    }
-    warp_sort_desc(buf);
-    count = min(count, tp.n_best);
-    for (int i = lane; i < kTopkCapacity; i += 32) mine[i] = i < count ? buf[i] : 0ull;
-    if (lane == 0) counts[q] = count;
+    list.sort();
+    for (int i = lane; i < tp.n_best; i += 32) mine[i] = list.buf[i];
+    if (lane == 0) counts[q] = list.count;
 }
 
 // Writes each query's sorted candidates to the shard that asked: query q = (asking shard, slot)
