@@ -668,7 +668,7 @@ k_score_tile(const float* __restrict__ P, const float* __restrict__ Tl, float* _
 #pragma unroll
             for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
 #pragma unroll 1
-        for (int k4 = 0; k4 < 32; k4 += 4) {
+        for (int k4 = 0; k4 < min(32, D - k0); k4 += 4) {
             float4 pv[4];
 #pragma unroll
             for (int a = 0; a < 4; ++a) pv[a] = load4(Ps + 8 * a * kScoreStride + k4);
@@ -2267,39 +2267,51 @@ __device__ __forceinline__ uint32_t topk_index(unsigned long long key) { return 
 
 // Sorts the warp's buffer in descending key order (empty slots hold key 0, which sorts last): a bitonic network on eight
 // keys per lane, key p of the network in lane p / 8, so that 21 of its 36 stages stay inside a lane and the other 15
-// exchange through shuffles.  (In shared memory, a compare-exchange per visit, a sort took 10 us, most of a merge.)
+// exchange through shuffles.  The outer stages are rolled: a sort is run by few warps, now and then, and 40 KB of
+// straight-line code took longer to fetch than to run.  (In shared memory, one compare-exchange per visit: 10 us.)
+__device__ __forceinline__ void order_desc(unsigned long long& a, unsigned long long& b, bool descending) {
+    const bool swap = (a < b) == descending;
+    const unsigned long long t = swap ? b : a;
+    b = swap ? a : b;
+    a = t;
+}
 __device__ __forceinline__ void warp_sort_desc(unsigned long long* buf) {
     constexpr int kPerLane = kTopkCapacity / 32;
+    static_assert(kPerLane == 8, "stages of 4, 2 and 1 inside a lane");
     const int lane = threadIdx.x & 31;
     unsigned long long v[kPerLane];
     __syncwarp();
 #pragma unroll
     for (int r = 0; r < kPerLane; ++r) v[r] = buf[r * 32 + lane];  // in any order: they are about to be sorted
     __syncwarp();
+    auto inside = [&](bool descending) {
 #pragma unroll
-    for (int k = 2; k <= kTopkCapacity; k <<= 1) {
+        for (int j = 4; j > 0; j >>= 1)
 #pragma unroll
+            for (int r = 0; r < kPerLane; ++r)
+                if (!(r & j)) order_desc(v[r], v[r | j], descending);
+    };
+#pragma unroll
+    for (int r = 0; r < kPerLane; r += 2) order_desc(v[r], v[r + 1], (r & 2) == 0);
+#pragma unroll
+    for (int j = 2; j > 0; j >>= 1)
+#pragma unroll
+        for (int r = 0; r < kPerLane; ++r)
+            if (!(r & j)) order_desc(v[r], v[r | j], (r & 4) == 0);
+    inside((lane & 1) == 0);
+#pragma unroll 1
+    for (int k = 2; k <= 32; k <<= 1) {  // in lanes
+        const bool descending = (lane & k) == 0;
+#pragma unroll 1
         for (int j = k >> 1; j > 0; j >>= 1) {
-            if (j >= kPerLane) {
-                const bool lower = ((lane * kPerLane) & j) == 0, descending = ((lane * kPerLane) & k) == 0;
-                const bool keep_larger = lower == descending;
+            const bool keep_larger = ((lane & j) == 0) == descending;
 #pragma unroll
-                for (int r = 0; r < kPerLane; ++r) {
-                    const unsigned long long other = __shfl_xor_sync(0xffffffffu, v[r], j / kPerLane);
-                    v[r] = (v[r] > other) == keep_larger ? v[r] : other;
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < kPerLane; ++r) {
-                    if (r & j) continue;
-                    const bool descending = ((lane * kPerLane + r) & k) == 0;
-                    const unsigned long long a = v[r], b = v[r | j];
-                    const bool swap = (a < b) == descending;
-                    v[r] = swap ? b : a;
-                    v[r | j] = swap ? a : b;
-                }
+            for (int r = 0; r < kPerLane; ++r) {
+                const unsigned long long other = __shfl_xor_sync(0xffffffffu, v[r], j);
+                v[r] = (v[r] > other) == keep_larger ? v[r] : other;
             }
         }
+        inside(descending);
     }
 #pragma unroll
     for (int r = 0; r < kPerLane; r += 2) *reinterpret_cast<ulonglong2*>(buf + lane * kPerLane + r) = make_ulonglong2(v[r], v[r + 1]);
@@ -2390,6 +2402,46 @@ struct TopkList {
         count += __popc(mask);
         __syncwarp();
     }
+    // A lower bound of the n_best-th largest of n keys, before any of them is in the list: among the 32 lanes' largest (n_best
+    // up to 32) or four largest keys there are n_best that reach it.  Most keys then never enter the list, which is
+    // sorted once instead of every time that 256 keys have come together.
+    template <class Key>
+    __device__ __forceinline__ void raise_cutoff(int n, Key&& key_of) {
+        const int lane = threadIdx.x & 31;
+        const bool few = n_best <= 32;
+        unsigned long long top[4] = {0ull, 0ull, 0ull, 0ull};
+        for (int i = lane; i < n; i += 32) {
+            unsigned long long key = key_of(i);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (r > 0 && few) break;
+                const unsigned long long less = key < top[r] ? key : top[r];
+                top[r] = key < top[r] ? top[r] : key;
+                key = less;
+            }
+        }
+        if (few) {
+#pragma unroll 1
+            for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll 1
+                for (int j = k >> 1; j > 0; j >>= 1) {
+                    const unsigned long long other = __shfl_xor_sync(0xffffffffu, top[0], j);
+                    const bool keep_larger = ((lane & j) == 0) == ((lane & k) == 0);
+                    top[0] = (top[0] > other) == keep_larger ? top[0] : other;
+                }
+            top[0] = __shfl_sync(0xffffffffu, top[0], n_best - 1);
+        } else {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) buf[r * 32 + lane] = top[r];
+            for (int i = 128 + lane; i < kTopkCapacity; i += 32) buf[i] = 0ull;
+            warp_sort_desc(buf);
+            top[0] = buf[n_best - 1];
+            __syncwarp();
+            for (int i = lane; i < 128; i += 32) buf[i] = 0ull;
+            __syncwarp();
+        }
+        if (top[0] > 0ull && top[0] - 1 > cutoff) cutoff = top[0] - 1;  // the bound itself passes
+    }
     // The scores of columns [begin, end) of a query's row.
     __device__ __forceinline__ void scan(const float* __restrict__ row, int begin, int end, uint32_t first_row, uint32_t last_valid_row, const TopkParams& tp) {
         const int lane = threadIdx.x & 31;
@@ -2426,7 +2478,13 @@ k_topk_seed(const float* __restrict__ raw, int n_cols, uint32_t first_row, uint3
     for (int i = lane; i < kTopkCapacity; i += 32) list.buf[i] = 0ull;
     __syncwarp();
     const int part = ((n_cols + (int)gridDim.y - 1) / (int)gridDim.y + 31) / 32 * 32, begin = (int)blockIdx.y * part;
-    list.scan(raw + (size_t)q * n_cols, begin, min(n_cols, begin + part), first_row, last_valid_row, tp);
+    const float* __restrict__ row = raw + (size_t)q * n_cols;
+    const int end = min(n_cols, begin + part);
+    list.raise_cutoff(end - begin, [&](int i) {
+        const uint32_t table_row = first_row + (uint32_t)(begin + i);
+        return table_row <= last_valid_row ? topk_key(tp.score_is_gamma_minus ? tp.gamma - row[begin + i] : row[begin + i], table_row) : 0ull;
+    });
+    list.scan(row, begin, end, first_row, last_valid_row, tp);
     list.sort();
     unsigned long long* __restrict__ out = cand + (size_t)q * kTopkCandidates + (size_t)blockIdx.y * tp.n_best;
     for (int i = lane; i < tp.n_best; i += 32) out[i] = list.buf[i];
@@ -2435,8 +2493,8 @@ k_topk_seed(const float* __restrict__ raw, int n_cols, uint32_t first_row, uint3
 
 // raw [n_query, n_cols] holds distances / dot products against rows first_row .. first_row+n_cols-1;
 // rows above last_valid_row are padding of the shard and are skipped (src/poplar_kge.cpp:836-842).
-// state [n_query, kTopkCapacity] keys, counts [n_query].  4 warps per block, one query each.
-// cand / cand_count: the filter's or the seed's output for this batch; the counts are cleared for the next.
+// state [n_query, kTopkCapacity] keys, counts [n_query]: the first n_best (or fewer) sorted, what came later behind them.
+// 4 warps per block, one query each.  cand / cand_count: the filter's or the seed's output for this batch; the counts are cleared for the next.
 static __global__ void __launch_bounds__(128)
 k_topk_update(const float* __restrict__ raw, int n_cols, uint32_t first_row, uint32_t last_valid_row,
               unsigned long long* __restrict__ state, int* __restrict__ counts, TopkParams tp,
@@ -2448,19 +2506,31 @@ k_topk_update(const float* __restrict__ raw, int n_cols, uint32_t first_row, uin
     const int n_cand = cand_count[q];
     if (n_cand == 0) return;  // nothing in this batch beats the cut-off: the list stands
     unsigned long long* mine = state + (size_t)q * kTopkCapacity;
-    TopkList list{buffers[warp], counts[q], tp.n_best, 0ull};
+    const unsigned long long* __restrict__ keys = cand + (size_t)q * kTopkCandidates;
+    const int old_count = counts[q];
+    if (old_count >= tp.n_best && old_count + n_cand <= kTopkCapacity) {
+        // room behind the sorted n_best: a later merge or k_topk_finish sorts; the cut-off stays the older, lower one
+        for (int i = lane; i < n_cand; i += 32) mine[old_count + i] = keys[i];
+        if (lane == 0) {
+            cand_count[q] = 0;
+            counts[q] = old_count + n_cand;
+        }
+        return;
+    }
+    TopkList list{buffers[warp], old_count, tp.n_best, 0ull};
     for (int i = lane; i < kTopkCapacity; i += 32) list.buf[i] = i < list.count ? mine[i] : 0ull;
     __syncwarp();
-    if (list.count >= tp.n_best) list.cutoff = list.buf[tp.n_best - 1];
+    const bool ranked = list.count >= tp.n_best;
+    if (ranked) list.sort();
     if (lane == 0) cand_count[q] = 0;
     if (n_cand <= kTopkCandidates) {
-        const unsigned long long* __restrict__ keys = cand + (size_t)q * kTopkCandidates;
+        if (list.count == 0 && n_cand > kTopkCapacity) list.raise_cutoff(n_cand, [&](int i) { return keys[i]; });
         for (int base = 0; base < n_cand; base += 32) list.add(base + lane < n_cand ? keys[base + lane] : 0ull);
     } else {  // more than the candidate list holds
         list.scan(raw + (size_t)q * n_cols, 0, n_cols, first_row, last_valid_row, tp);
     }
-    list.sort();
-    for (int i = lane; i < tp.n_best; i += 32) mine[i] = list.buf[i];
+    if (!ranked) list.sort();
+    for (int i = lane; i < list.count; i += 32) mine[i] = list.buf[i];
     if (lane == 0) counts[q] = list.count;
 }
 
@@ -2471,16 +2541,20 @@ static __global__ void __launch_bounds__(128)
 k_topk_finish(const unsigned long long* __restrict__ state, const int* __restrict__ counts, int n_query,
               int queries_per_shard, int n_best, float* const* __restrict__ score_blocks,
               uint32_t* const* __restrict__ index_blocks) {
+    __shared__ __align__(16) unsigned long long keys[kTopkCapacity];
     const int q = blockIdx.x;
     if (q >= n_query) return;
     const int shard = q / queries_per_shard, slot = q - shard * queries_per_shard;
     float* __restrict__ so = score_blocks[shard] + (size_t)slot * n_best;
     uint32_t* __restrict__ io = index_blocks[shard] + (size_t)slot * n_best;
     const int count = counts[q];
+    for (int i = threadIdx.x; i < kTopkCapacity; i += blockDim.x) keys[i] = i < count ? state[(size_t)q * kTopkCapacity + i] : 0ull;
+    __syncthreads();
+    if (count > n_best && threadIdx.x < 32) warp_sort_desc(keys);
+    __syncthreads();
     for (int i = threadIdx.x; i < n_best; i += blockDim.x) {
-        const unsigned long long key = state[(size_t)q * kTopkCapacity + i];
-        so[i] = i < count ? topk_score(key) : -1e6f;
-        io[i] = i < count ? topk_index(key) : 0u;
+        so[i] = i < count ? topk_score(keys[i]) : -1e6f;
+        io[i] = i < count ? topk_index(keys[i]) : 0u;
     }
 }
 
