@@ -858,7 +858,7 @@ void Engine::sample_and_stage(uint32_t seed) {
     if (!sampler_.triples) fail(KGE_LOGIC_ERROR, "no training triples: run \"load_triples\" first");
     k_sample_batch<<<(unsigned)(n_local_ * cfg_.n_step), 512, 0, stream_>>>(sampler_, seed, sample_run_++, (int)cfg_.n_shard, (int)shard0_,
                                                                              (int)cfg_.n_step, (int)cfg_.batch_size, (int)cfg_.a2a_size,
-                                                                             d_remote_, d_a2a_, d_head_, d_relation_, d_tail_);
+                                                                             d_remote_, d_a2a_, d_head_, d_relation_, d_tail_, cfg_.n_entity - 1);
     KGE_CUDA(cudaGetLastError());
     prepare_staged();
 }

@@ -1158,38 +1158,94 @@ k_pred_bwd(const float* __restrict__ d_pred, const float* __restrict__ hid_h,
 // order is unique) and records where each row's segment starts; the same for the B
 // relation lookups.  The scatter-add of src/pag/pag.cpp:721-743 then becomes one
 // sequential sum per row in a fixed order: no float atomics.
-// One block per (shard-step); bitonic sort of (row << 32 | position) keys in shared memory.
+// One block per (shard-step).
 constexpr int kMaxSortItems = 4096;
+constexpr int kSortThreads = 512, kSortWarps = kSortThreads / 32;
 
-__device__ __forceinline__ void bitonic_sort(unsigned long long* keys, int padded) {
-    for (int k = 2; k <= padded; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
+// A stable sort of up to kMaxSortItems positions by their keys, one block, in passes over six bits of the key.  A warp
+// owns a contiguous part of the positions and ranks them 32 at a time among the warp's equal digits (six ballots); the
+// 64 x 16 counts are scanned digit by digit, so equal keys stay in position order.  As many passes as the largest key
+// has bits for: two for the 4096 rows of a step, where a bitonic network in shared memory ran 78 stages (two sorts
+// of 1280 keys and one of 512 took 80 us, 160 us at 3072, a third of that with the launch this way).
+struct BlockSort {
+    uint32_t key[kMaxSortItems];
+    uint16_t idx[2][kMaxSortItems];
+    uint32_t count[64 * kSortWarps];  // [digit][warp]
+    uint32_t warp_total[kSortWarps];
+
+    // Sorts the positions 0 .. n - 1 by key (filled by the caller, who has synchronised); all keys are below 2^bits.
+    // Returns the sorted positions.
+    __device__ const uint16_t* sort(int n, int bits) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int per_warp = (n + kSortThreads - 1) / kSortThreads * 32, begin = warp * per_warp;
+        uint16_t *in = idx[0], *out = idx[1];
+        for (int i = threadIdx.x; i < n; i += kSortThreads) in[i] = (uint16_t)i;
+        for (int shift = 0; shift < bits; shift += 6) {
+            for (int i = threadIdx.x; i < 64 * kSortWarps; i += kSortThreads) count[i] = 0u;
             __syncthreads();
-            for (int i = threadIdx.x; i < padded; i += blockDim.x) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = keys[i], b = keys[ixj];
-                    const bool ascending = (i & k) == 0;
-                    if ((a > b) == ascending) {
-                        keys[i] = b;
-                        keys[ixj] = a;
-                    }
+            uint32_t place[kMaxSortItems / kSortThreads], pos[kMaxSortItems / kSortThreads];
+#pragma unroll
+            for (int it = 0; it < kMaxSortItems / kSortThreads; ++it) {
+                const int i = begin + it * 32 + lane;
+                const bool live = it * 32 < per_warp && i < n;
+                if (!__any_sync(0xffffffffu, live)) break;
+                pos[it] = live ? in[i] : 0u;
+                const uint32_t digit = (key[pos[it]] >> shift) & 63u;
+                uint32_t same = __ballot_sync(0xffffffffu, live);
+                if (!live) same = ~same;
+#pragma unroll
+                for (int b = 0; b < 6; ++b) {
+                    const uint32_t ones = __ballot_sync(0xffffffffu, (digit >> b) & 1u);
+                    same &= (digit >> b) & 1u ? ones : ~ones;
                 }
+                uint32_t* const cell = count + digit * kSortWarps + warp;
+                const uint32_t before = *cell;
+                __syncwarp();
+                if (live && lane == __ffs(same) - 1) *cell = before + __popc(same);
+                __syncwarp();
+                place[it] = before + __popc(same & ((1u << lane) - 1u));
             }
+            __syncthreads();
+            // exclusive scan over (digit, warp), two neighbours per thread
+            const uint2 mine = *reinterpret_cast<const uint2*>(count + 2 * threadIdx.x);
+            uint32_t sum = mine.x + mine.y;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t left = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += left;
+            }
+            if (lane == 31) warp_total[warp] = sum;
+            __syncthreads();
+            uint32_t base = 0;
+            for (int w = 0; w < warp; ++w) base += warp_total[w];
+            base += sum - mine.x - mine.y;
+            *reinterpret_cast<uint2*>(count + 2 * threadIdx.x) = make_uint2(base, base + mine.x);
+            __syncthreads();
+#pragma unroll
+            for (int it = 0; it < kMaxSortItems / kSortThreads; ++it) {
+                const int i = begin + it * 32 + lane;
+                if (it * 32 < per_warp && i < n) out[count[((key[pos[it]] >> shift) & 63u) * kSortWarps + warp] + place[it]] = (uint16_t)pos[it];
+            }
+            __syncthreads();
+            uint16_t* const t = in;
+            in = out;
+            out = t;
         }
+        __syncthreads();
+        return in;
     }
-    __syncthreads();
-}
-
-__device__ __forceinline__ int lower_bound_key(const unsigned long long* keys, int n,
-                                                unsigned long long target) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (keys[mid] < target) lo = mid + 1; else hi = mid;
+    // The first of the n sorted positions whose key is not below `target`.
+    __device__ int lower_bound(const uint16_t* sorted, int n, uint32_t target) const {
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key[sorted[mid]] < target) lo = mid + 1; else hi = mid;
+        }
+        return lo;
     }
-    return lo;
-}
+};
+static_assert(kMaxSortItems <= 65536 && 2 * kSortThreads == 64 * kSortWarps, "positions in 16 bits, two counts per thread");
+__device__ __forceinline__ int bits_below(uint32_t limit) { return limit <= 1u ? 0 : 32 - __clz(limit - 1u); }
 
 // Rows with more than kHeavyMin lookups are cut into parts of kHeavyPart lookups, at most kHeavySlots
 // parts per shard and step (see k_entity_update).
@@ -1197,14 +1253,14 @@ constexpr int kHeavySlots = 112;
 constexpr int kHeavyMin = 12;
 constexpr int kHeavyPart = 16;
 
-static __global__ void __launch_bounds__(512)
+static __global__ void __launch_bounds__(kSortThreads)
 k_prepare_segments(const uint32_t* __restrict__ head, const uint32_t* __restrict__ a2a_idx,
                    const uint32_t* __restrict__ relation, const uint32_t* __restrict__ remote, int B,
                    int T, int R, int n_rel, uint32_t* __restrict__ ent_perm,
                    uint32_t* __restrict__ ent_off, uint32_t* __restrict__ rel_perm,
                    uint32_t* __restrict__ rel_off, uint32_t* __restrict__ first_slot,
                    uint4* __restrict__ heavy_parts, uint32_t* __restrict__ heavy_count, uint4* __restrict__ row_info) {
-    __shared__ unsigned long long keys[kMaxSortItems];
+    __shared__ BlockSort bs;
     const int s = blockIdx.x;
     head += (size_t)s * B;
     relation += (size_t)s * B;
@@ -1214,30 +1270,20 @@ k_prepare_segments(const uint32_t* __restrict__ head, const uint32_t* __restrict
     rel_perm += (size_t)s * B;
     rel_off += (size_t)s * (n_rel + 1);
 
-    int n = B + T, padded = 1;
-    while (padded < n) padded <<= 1;
-    for (int i = threadIdx.x; i < padded; i += blockDim.x) {
-        unsigned long long key = ~0ull;
-        if (i < B) key = ((unsigned long long)head[i] << 32) | (unsigned)i;
-        else if (i < n) key = ((unsigned long long)a2a_idx[i - B] << 32) | (unsigned)i;
-        keys[i] = key;
-    }
-    bitonic_sort(keys, padded);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) ent_perm[i] = (uint32_t)keys[i];
-    for (int r = threadIdx.x; r <= R; r += blockDim.x)
-        ent_off[r] = (uint32_t)lower_bound_key(keys, n, (unsigned long long)r << 32);
+    const int n = B + T;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) bs.key[i] = min(i < B ? head[i] : a2a_idx[i - B], (uint32_t)R);  // lookups past the rows (an operator's caller may pass some): behind them
+    __syncthreads();
+    const uint16_t* sorted = bs.sort(n, bits_below((uint32_t)R + 1u));
+    for (int i = threadIdx.x; i < n; i += blockDim.x) ent_perm[i] = sorted[i];
+    for (int r = threadIdx.x; r <= R; r += blockDim.x) ent_off[r] = (uint32_t)bs.lower_bound(sorted, n, (uint32_t)r);
     __syncthreads();
 
     if (rel_perm) {  // null: the caller has no relation lookups (the operator form of the scatter-add)
-        n = B;
-        padded = 1;
-        while (padded < n) padded <<= 1;
-        for (int i = threadIdx.x; i < padded; i += blockDim.x)
-            keys[i] = i < n ? (((unsigned long long)relation[i] << 32) | (unsigned)i) : ~0ull;
-        bitonic_sort(keys, padded);
-        for (int i = threadIdx.x; i < n; i += blockDim.x) rel_perm[i] = (uint32_t)keys[i];
-        for (int r = threadIdx.x; r <= n_rel; r += blockDim.x)
-            rel_off[r] = (uint32_t)lower_bound_key(keys, n, (unsigned long long)r << 32);
+        for (int i = threadIdx.x; i < B; i += blockDim.x) bs.key[i] = relation[i];
+        __syncthreads();
+        sorted = bs.sort(B, bits_below((uint32_t)n_rel));
+        for (int i = threadIdx.x; i < B; i += blockDim.x) rel_perm[i] = sorted[i];
+        for (int r = threadIdx.x; r <= n_rel; r += blockDim.x) rel_off[r] = (uint32_t)bs.lower_bound(sorted, B, (uint32_t)r);
     }
     if (!remote) return;
     __syncthreads();
@@ -1248,15 +1294,28 @@ k_prepare_segments(const uint32_t* __restrict__ head, const uint32_t* __restrict
     // writes are identical, and one write reproduces them.
     remote += (size_t)s * R;
     first_slot += (size_t)s * R;
-    n = R;
-    padded = 1;
-    while (padded < n) padded <<= 1;
-    for (int i = threadIdx.x; i < padded; i += blockDim.x)
-        keys[i] = i < n ? (((unsigned long long)remote[i] << 32) | (unsigned)i) : ~0ull;
-    bitonic_sort(keys, padded);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const bool first = i == 0 || (keys[i - 1] >> 32) != (keys[i] >> 32);
-        first_slot[(uint32_t)keys[i]] = first ? 1u : 0u;
+    // The sampler's order (ascending, the padding last) needs no sort.
+    bool in_order = true;
+    for (int i = threadIdx.x; i < R; i += blockDim.x) {
+        const uint32_t row = remote[i], before = i ? remote[i - 1] : 0u;
+        in_order = in_order && (row > before ? i == 0 || before != 0u : row == 0u);  // nothing but padding after padding
+    }
+    if (__syncthreads_and(in_order)) {
+        for (int i = threadIdx.x; i < R; i += blockDim.x) first_slot[i] = remote[i] != 0u || i == 0 || remote[i - 1] != 0u ? 1u : 0u;
+    } else {
+        __shared__ uint32_t s_highest;
+        if (threadIdx.x == 0) s_highest = 0u;
+        __syncthreads();
+        uint32_t highest = 0;
+        for (int i = threadIdx.x; i < R; i += blockDim.x) {
+            bs.key[i] = remote[i];
+            highest = max(highest, remote[i]);
+        }
+        atomicMax(&s_highest, highest);
+        __syncthreads();
+        sorted = bs.sort(R, 32 - __clz(s_highest));
+        for (int i = threadIdx.x; i < R; i += blockDim.x)
+            first_slot[sorted[i]] = i == 0 || bs.key[sorted[i - 1]] != bs.key[sorted[i]] ? 1u : 0u;
     }
     if (heavy_parts) {
     // Rows with many lookups are cut into parts for k_entity_update (bit 1 of first_slot marks them).
@@ -2595,12 +2654,12 @@ __device__ __forceinline__ unsigned long long sampler_draw(uint32_t seed, uint32
 
 constexpr uint32_t kNegativeSlot = 0x80000000u;  // slot numbers of negatives, apart from those of positives
 
-static __global__ void __launch_bounds__(512)
+static __global__ void __launch_bounds__(kSortThreads)
 k_sample_batch(SamplerData sd, uint32_t seed, uint32_t run, int n_shard, int shard0, int n_step, int B, int a2a,
                uint32_t* __restrict__ remote, uint32_t* __restrict__ a2a_out, uint32_t* __restrict__ head,
-               uint32_t* __restrict__ relation, uint32_t* __restrict__ tail) {
-    __shared__ unsigned long long keys[kMaxSortItems];
-    __shared__ uint32_t s_scan[512];
+               uint32_t* __restrict__ relation, uint32_t* __restrict__ tail, uint32_t highest_row) {
+    __shared__ BlockSort bs;
+    __shared__ uint32_t s_scan[kSortThreads];
     const int l = blockIdx.x / n_step, step = blockIdx.x % n_step, s = shard0 + l;
     const int pos = B / n_shard, neg = a2a - pos, T = n_shard * a2a, R = B + T;
     const size_t sidx = (size_t)l * n_step + step;
@@ -2609,34 +2668,32 @@ k_sample_batch(SamplerData sd, uint32_t seed, uint32_t run, int n_shard, int sha
     head += sidx * B;
     relation += sidx * B;
     tail += sidx * B;
-    int padded = 1;
-    while (padded < R) padded <<= 1;
-    for (int p = threadIdx.x; p < padded; p += blockDim.x) {
-        unsigned long long key = ~0ull;
+    for (int p = threadIdx.x; p < R; p += blockDim.x) {
+        uint32_t row;
         if (p < B) {
             const int ts = p / pos, k = p - ts * pos;
             const uint32_t bucket = (uint32_t)(s * n_shard + ts);
             const size_t idx = sd.bucket_offset[bucket] + sampler_draw(seed, run, (uint32_t)s, (uint32_t)step, (uint32_t)ts, (uint32_t)k) % sd.bucket_count[bucket];
-            key = ((unsigned long long)sd.triples[idx] << 32) | (unsigned)p;
+            row = sd.triples[idx];
             relation[p] = sd.triples[sd.n_triples + idx];
             tail[p] = (uint32_t)(ts * a2a + k);  // where the exchange puts this positive's tail (:257-263)
         } else if (p < 2 * B) {
             const int q = p - B, hs = q / pos, k = q - hs * pos;
             const uint32_t bucket = (uint32_t)(hs * n_shard + s);
             const size_t idx = sd.bucket_offset[bucket] + sampler_draw(seed, run, (uint32_t)hs, (uint32_t)step, (uint32_t)s, (uint32_t)k) % sd.bucket_count[bucket];
-            key = ((unsigned long long)sd.triples[2 * sd.n_triples + idx] << 32) | (unsigned)p;
-        } else if (p < R) {
+            row = sd.triples[2 * sd.n_triples + idx];
+        } else {
             const int q = p - 2 * B, hs = q / neg, k = q - hs * neg;
-            const uint32_t row = 1u + (uint32_t)(sampler_draw(seed, run, (uint32_t)hs, (uint32_t)step, (uint32_t)s, kNegativeSlot | (uint32_t)k) % sd.shard_count[s]);
-            key = ((unsigned long long)row << 32) | (unsigned)p;
+            row = 1u + (uint32_t)(sampler_draw(seed, run, (uint32_t)hs, (uint32_t)step, (uint32_t)s, kNegativeSlot | (uint32_t)k) % sd.shard_count[s]);
         }
-        keys[p] = key;
+        bs.key[p] = row;
     }
-    bitonic_sort(keys, padded);
+    __syncthreads();
+    const uint16_t* const sorted = bs.sort(R, 32 - __clz(highest_row));
     // rank of every sorted entry among the distinct rows: an exclusive scan of "starts a new row"
-    const int per_thread = (padded + (int)blockDim.x - 1) / (int)blockDim.x, first = threadIdx.x * per_thread;
+    const int per_thread = (R + (int)blockDim.x - 1) / (int)blockDim.x, first = threadIdx.x * per_thread;
     uint32_t mine = 0;
-    for (int i = first; i < first + per_thread && i < R; ++i) mine += (i == 0 || (keys[i] >> 32) != (keys[i - 1] >> 32)) ? 1u : 0u;
+    for (int i = first; i < first + per_thread && i < R; ++i) mine += i == 0 || bs.key[sorted[i]] != bs.key[sorted[i - 1]] ? 1u : 0u;
     s_scan[threadIdx.x] = mine;
     __syncthreads();
     for (int o = 1; o < (int)blockDim.x; o <<= 1) {  // Hillis-Steele inclusive scan over the threads' counts
@@ -2648,9 +2705,10 @@ k_sample_batch(SamplerData sd, uint32_t seed, uint32_t run, int n_shard, int sha
     uint32_t rank = s_scan[threadIdx.x] - mine;  // distinct rows before this thread's first entry
     const uint32_t n_unique = s_scan[blockDim.x - 1];
     for (int i = first; i < first + per_thread && i < R; ++i) {
-        const bool starts = i == 0 || (keys[i] >> 32) != (keys[i - 1] >> 32);
-        if (starts) remote[rank++] = (uint32_t)(keys[i] >> 32);
-        const uint32_t p = (uint32_t)keys[i], slot = rank - 1;
+        const uint32_t p = sorted[i];
+        const bool starts = i == 0 || bs.key[p] != bs.key[sorted[i - 1]];
+        if (starts) remote[rank++] = bs.key[p];
+        const uint32_t slot = rank - 1;
         if (p < (uint32_t)B) {
             head[p] = slot;
         } else if (p < (uint32_t)(2 * B)) {
