@@ -1,0 +1,79 @@
+"""Kernels at the sizes where their tiles, chunks and lists begin, end and change over."""
+
+import numpy as np
+import pytest
+
+from distributed_kge_poplar_b200 import capi
+from helpers import assert_close, engine_settings, make_oracle, random_state, write_state
+from oracle import step_oracle as so
+from oracle.step_oracle import StepConfig
+from test_predict_gpu import RW, _clear, _predict
+
+pytestmark = pytest.mark.gpu
+RTOL = 1e-5
+
+
+@pytest.mark.parametrize("fn", [capi.L1, capi.L2, capi.DOT], ids=["l1", "l2", "dot"])
+@pytest.mark.parametrize("shape", [(64, 37889, 4), (65, 18950, 36), (1, 37890, 32)])
+def test_scores_in_whole_tiles(fn, shape):
+    """Enough 64 x 128 tiles to fill the GPU: full and ragged tiles, one chunk of k and a remainder."""
+    m, n, k = shape
+    rng = np.random.RandomState(n)
+    a, b = rng.normal(size=(m, k)).astype(np.float32), rng.normal(size=(n, k)).astype(np.float32)
+    b[7] = a[0]
+    a64, b64 = a.astype(np.float64), b.astype(np.float64)
+    want = {capi.L1: so.l1_distance, capi.L2: so.l2_distance, capi.DOT: lambda x, y: x @ y.T}[fn](a64, b64)
+    assert_close(capi.op_pairwise(fn, a, b), want, RTOL, f"scores {shape}")
+
+
+@pytest.mark.parametrize("shape", [(1, 64, 64), (8, 65, 63), (9, 63, 65), (17, 129, 2), (600, 590, 250)])
+def test_l1_gradients_add_up_in_order(shape):
+    """Chunks of 64 and column tiles of 64 with and without a remainder; one and two rows per warp.  The terms are added
+    in index order, so the result has the bits of a plain fp32 loop."""
+    m, n, k = shape
+    rng = np.random.RandomState(m + n + k)
+    a, b = rng.normal(size=(m, k)).astype(np.float32), rng.normal(size=(n, k)).astype(np.float32)
+    b[-1] = a[0]
+    g = rng.normal(size=(m, n)).astype(np.float32)
+    want_a, want_b = np.zeros_like(a), np.zeros_like(b)
+    for j in range(n):
+        want_a += g[:, j : j + 1] * np.sign(a - b[j])
+    for i in range(m):
+        want_b += g[i, :, None] * np.sign(b - a[i])
+    got_a, got_b = capi.op_pairwise_grad(capi.L1, a, b, g)
+    np.testing.assert_array_equal(got_a, want_a)
+    np.testing.assert_array_equal(got_b, want_b)
+
+
+@pytest.mark.parametrize("n,rows", [(1, 1), (31, 2), (32, 63), (33, 64), (511, 65), (512, 4095), (513, 4096), (4095, 3), (4096, 4097)])
+def test_lookups_are_sorted_stably(n, rows):
+    """Radix passes of six bits (1, 63, 64, 65, 4095 ... rows), warps with no, some and all of their positions."""
+    rng = np.random.RandomState(n)
+    idx = (rows * rng.random_sample(n) ** 3).astype(np.uint32)
+    grad = rng.normal(size=(n, 5)).astype(np.float32)
+    want = np.zeros((rows, 5), np.float32)
+    np.add.at(want, idx, grad)
+    np.testing.assert_array_equal(capi.op_scatter_add_rows(grad, idx, rows), want)
+
+
+@pytest.mark.parametrize("score_fn,distance_fn", [("TransE", "L1"), ("TransE", "L2"), ("DistMult", "MatMul")])
+@pytest.mark.parametrize("n_best", [1, 32, 33, 128])
+@pytest.mark.parametrize("pass_rows", [256, 640])
+def test_ranking_lists(monkeypatch, score_fn, distance_fn, n_best, pass_rows):
+    """First scans, appended merges and full lists: the shortest and longest lists, and the change from one to four
+    largest keys per lane."""
+    monkeypatch.setenv("KGE_PREDICT_PASS_ROWS", str(pass_rows))
+    cfg = StepConfig(n_shard=2, n_entity=1500, n_relation_type=4, embedding_size=16, entity_feature_size=0, batch_size=8, a2a_size=6,
+                     score_fn=score_fn, distance_fn=distance_fn, gamma=8.0)
+    state = random_state(cfg, 3, warm=True)
+    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW, **{"execution.predict_hr_batch_size": 9, "execution.predict_n_best": n_best}))
+    write_state(engine, cfg, state, RW)
+    rng = np.random.RandomState(1)
+    queries = np.stack([np.arange(18) % 2, 1 + rng.randint(1499, size=18), rng.randint(4, size=18)], axis=1)
+    counts = np.array([1499, 700])
+    got_idx, got_score = _predict(engine, cfg, queries, counts, 9, n_best)
+    engine.close()
+    want_idx, want_score = make_oracle(cfg, state).predict(queries, counts, n_best)
+    assert_close(got_score, want_score, RTOL, "ranking: scores")
+    clear = _clear(want_score) if n_best > 1 else np.ones_like(want_score, bool)
+    np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
