@@ -391,11 +391,12 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// EPI >= 0: an instantiation for the training step's contractions, whose epilogue is known at
-// compile time and which always run with fp32 planes and a k split over a cluster.  A block runs
+// EPI >= 0: an instantiation whose epilogue, operand type and k split are known at compile time.  A block runs
 // this kernel once on an SM whose instruction cache has never seen it, and most of it is
 // straight-line code executed once: what the instantiation does not need is not fetched.
-template <int BN, int SIDE, int EPI = -1>
+// SPLIT: 0 no k split; else the k range is split over a cluster and a block finishes at most SPLIT units per thread
+// (3: up to 30 rows, five or more splits; 7: up to 64 rows).  BF16: bfloat16 operands.
+template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, bool BF16 = false>
 __global__ void __launch_bounds__(kPlThreads, 1)
 k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneMaps maps) {
     constexpr bool kLean = EPI >= 0;
@@ -426,7 +427,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr uint32_t kATile = kBM * 128, kBTile = BN * 128;
     const int k_begin = blockIdx.z * g.k_per_split, k_end = min(g.K, k_begin + g.k_per_split);
-    const int bf16 = kLean ? 0 : gp.bf16, slice_k = bf16 ? 64 : kBK;
+    const int bf16 = kLean ? (BF16 ? 1 : 0) : gp.bf16, slice_k = bf16 ? 64 : kBK;
     const int n_slices = max(0, (k_end - k_begin + slice_k - 1) / slice_k);
     const bool a_two = pp.A.lo != nullptr, b_two = pp.B.lo != nullptr;
     // a ring stage: A hi [| A lo] | B hi [| B lo]
@@ -458,7 +459,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     grid_dependency_sync();
     exchange_wait(gp.sync, gp.wait_kind);
     const uint32_t tmem_base = tmem_slot;
-    if (!kLean && g.epilogue == EPI_ADD_TABLE_VALUE && g.cluster_splits <= 1 && tid >= 64 && tid < 64 + kBM && m0 + tid - 64 < g.M) {
+    if ((kLean ? EPI == EPI_ADD_TABLE_VALUE && SPLIT == 0 : g.epilogue == EPI_ADD_TABLE_VALUE && g.cluster_splits <= 1) && tid >= 64 && tid < 64 + kBM && m0 + tid - 64 < g.M) {
         // A whole tile without a k split (predict's hidden rows): the table values that the epilogue
         // adds are asked into L2 now, a row per thread, so that the finishing loop, which fetches
         // them one unit after the other, waits for L2 and not for DRAM.
@@ -603,7 +604,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
         // barrier (arrive here, wait before the copies are issued).  Without a k split the block is
         // the only owner: its rows take the same way through shared memory, which turns one thread's
         // row of the accumulator into whole rows stored by neighbouring threads.
-        const bool clustered = kLean || g.cluster_splits > 1;
+        const bool clustered = kLean ? SPLIT > 0 : g.cluster_splits > 1;
         if (clustered) cluster_arrive_relaxed();
         const int n_split = clustered ? g.cluster_splits : 1, rank = clustered ? (int)cluster_rank() : 0;
         const int rows_each = (kBM + n_split - 1) / n_split;
@@ -689,8 +690,8 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
         if (clustered) fence_async_shared();  // the copy engine reads what the threads have just written
         const int r_begin = rank * rows_each, r_end = min(kBM, r_begin + rows_each);
         constexpr int kQuads = BN / 4;
-        // a split owns at most 64 rows x BN / 4 quads (22 rows in the training step's instantiations: six splits or more)
-        constexpr int kUnits = ((kLean ? 22 : 64) * kQuads + kPlThreads - 1) / kPlThreads;
+        // a split owns at most 64 rows x BN / 4 quads
+        constexpr int kUnits = kLean && SPLIT > 0 ? SPLIT : (64 * kQuads + kPlThreads - 1) / kPlThreads;
         const int n_units = max(0, r_end - r_begin) * kQuads;
         float xv[kUnits][4];
         if (clustered) {
@@ -753,6 +754,21 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
 #pragma unroll
             for (int i = 0; i < kUnits; ++i)
                 if (tid + i * kPlThreads < n_units) finish_unit(tid + i * kPlThreads, xv[i]);
+        } else if (kLean && EPI != EPI_L2_DISTANCE) {
+            // the epilogue's second operand is fetched for four units at a time
+#pragma unroll 1
+            for (int u0 = tid; u0 < n_units; u0 += 4 * kPlThreads) {
+                float x[4][4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int u = u0 + i * kPlThreads, mm = m0 + u / kQuads, nn = n0 + (u % kQuads) * 4;
+                    x[i][0] = x[i][1] = x[i][2] = x[i][3] = 0.f;
+                    if (u < n_units && mm < g.M && nn < g.N) load_x_four(g, mm, nn, x[i], EPI);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (u0 + i * kPlThreads < n_units) finish_unit(u0 + i * kPlThreads, x[i]);
+            }
         } else if (SIDE == SIDE_NORMS || (g.epilogue == EPI_STORE && g.out_blocks == nullptr && !routing)) {
             // the staged rows are finished (distances, or a plain product): whole rows go out in 16-byte pieces
 #pragma unroll 4
@@ -823,12 +839,12 @@ inline bool planes_aligned(const PlaneOperand& op) {
     return reinterpret_cast<uintptr_t>(op.hi) % 16 == 0 && reinterpret_cast<uintptr_t>(op.lo) % 16 == 0 && op.row_stride_bytes % 16 == 0;
 }
 
-template <int BN, int SIDE, int EPI = -1>
+template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, bool BF16 = false>
 inline cudaError_t configure_planes() {
     static bool configured[kMaxDeviceOrdinals] = {};
     const int slot = current_device_slot();
     if (slot >= 0 && configured[slot]) return cudaSuccess;
-    cudaError_t err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem_bytes());
+    cudaError_t err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem_bytes());
     if (err == cudaSuccess && slot >= 0) configured[slot] = true;
     return err;
 }
@@ -918,12 +934,19 @@ inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, 
     return cudaSuccess;
 }
 
-template <int SIDE, int EPI>
+template <int SIDE, int EPI, int SPLIT, bool BF16 = false>
 inline cudaError_t launch_lean(const PlaneLaunch& l, cudaStream_t stream) {
-    cudaError_t err = configure_planes<128, SIDE, EPI>();
+    cudaError_t err = configure_planes<128, SIDE, EPI, SPLIT, BF16>();
     if (err != cudaSuccess) return err;
-    return launch_dependent_cluster(k_tc_planes<128, SIDE, EPI>, l.grid, dim3(kPlThreads), plane_smem_bytes(), stream, (unsigned)l.splits, l.gp,
-                                    l.maps);
+    return launch_dependent_cluster(k_tc_planes<128, SIDE, EPI, SPLIT, BF16>, l.grid, dim3(kPlThreads), plane_smem_bytes(), stream, (unsigned)l.splits,
+                                    l.gp, l.maps);
+}
+// By the number of k splits: five or more leave at most 26 rows of a tile to a block.
+template <int SIDE, int EPI>
+inline cudaError_t launch_lean_split(const PlaneLaunch& l, cudaStream_t stream) {
+    if (l.splits >= 5) return launch_lean<SIDE, EPI, 3>(l, stream);
+    if (l.splits >= 2) return launch_lean<SIDE, EPI, 7>(l, stream);
+    return launch_lean<SIDE, EPI, 0>(l, stream);
 }
 
 template <int SIDE>
@@ -933,15 +956,22 @@ inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
         for (int i = 0; i < 2; ++i)
             if (l.gp.p[i].A.mn_major || l.gp.p[i].B.mn_major || l.gp.p[i].g.out_blocks) return cudaErrorInvalidValue;
     if (l.tile_n == 128) {
-        // the training step's contractions (fp32 planes, k split over a cluster, one epilogue for the launch)
+        // one epilogue for the launch: the instantiation for it
         const int epilogue = l.gp.p[0].g.epilogue;
-        const bool lean = SIDE != SIDE_NORMS && !l.gp.bf16 && l.splits >= 6 && l.gp.p[1].g.epilogue == epilogue;
-        if constexpr (SIDE == SIDE_NONE) {
-            if (lean && epilogue == EPI_ADD_TABLE_VALUE) return launch_lean<SIDE_NONE, EPI_ADD_TABLE_VALUE>(l, stream);
-            if (lean && epilogue == EPI_DENSE_ADAM) return launch_lean<SIDE_NONE, EPI_DENSE_ADAM>(l, stream);
-            if (lean && epilogue == EPI_STORE) return launch_lean<SIDE_NONE, EPI_STORE>(l, stream);
-        } else if constexpr (SIDE == SIDE_ROWSUM) {
-            if (lean && epilogue == EPI_ROWSUM_X_MINUS) return launch_lean<SIDE_ROWSUM, EPI_ROWSUM_X_MINUS>(l, stream);
+        if (l.gp.p[1].g.epilogue == epilogue) {
+            if constexpr (SIDE == SIDE_NONE) {
+                if (l.gp.bf16) {
+                    if (epilogue == EPI_STORE) return l.splits > 1 ? launch_lean<SIDE_NONE, EPI_STORE, 7, true>(l, stream) : launch_lean<SIDE_NONE, EPI_STORE, 0, true>(l, stream);
+                } else {
+                    if (epilogue == EPI_ADD_TABLE_VALUE) return launch_lean_split<SIDE_NONE, EPI_ADD_TABLE_VALUE>(l, stream);
+                    if (epilogue == EPI_DENSE_ADAM) return launch_lean_split<SIDE_NONE, EPI_DENSE_ADAM>(l, stream);
+                    if (epilogue == EPI_STORE) return launch_lean_split<SIDE_NONE, EPI_STORE>(l, stream);
+                }
+            } else if constexpr (SIDE == SIDE_ROWSUM) {
+                if (epilogue == EPI_ROWSUM_X_MINUS) return launch_lean_split<SIDE_ROWSUM, EPI_ROWSUM_X_MINUS>(l, stream);
+            } else {
+                if (epilogue == EPI_L2_DISTANCE && l.splits == 1) return launch_lean<SIDE_NORMS, EPI_L2_DISTANCE, 0>(l, stream);
+            }
         }
         cudaError_t err = configure_planes<128, SIDE>();
         if (err != cudaSuccess) return err;
