@@ -862,15 +862,18 @@ k_loss(const float* __restrict__ raw, const uint32_t* __restrict__ label, float*
     const bool adv = lp.adversarial_scale > 0.f;
     if (adv) {
         float mx = -INFINITY;
+#pragma unroll 4
         for (int j = threadIdx.x; j < T; j += THREADS)
             mx = fmaxf(mx, lp.adversarial_scale * score_of(j) + (j == lab ? -10000.f : 0.f));
         adv_max = block_max<THREADS>(mx, scratch);
         float sum = 0.f;
+#pragma unroll 4
         for (int j = threadIdx.x; j < T; j += THREADS)
             sum += expf(lp.adversarial_scale * score_of(j) + (j == lab ? -10000.f : 0.f) - adv_max);
         adv_sum = block_sum<THREADS>(sum, scratch);
     }
     float part = 0.f;
+#pragma unroll 4
     for (int j = threadIdx.x; j < T; j += THREADS) {
         const float s = score_of(j);
         const bool pos = j == lab;
@@ -899,7 +902,12 @@ inline cudaError_t launch_loss(const float* raw, const uint32_t* label, float* c
                                float* loss_total, float* loss_last, unsigned* counter, float* coeff_lo, int lo_bf16, int B, cudaStream_t stream,
                                const float* extra_loss = nullptr) {
     // One block per row keeps about 130 thousand threads in flight for the metric's 512 x 768 scores; a warp
-    // per row (a sixth as many threads, each with a serial chain of exponentials) measured 4 us slower.
+    // per row (a sixth as many threads, each with a serial chain of exponentials) measured 4 us slower.  A long row of
+    // log-sigmoids, whose chains are longest, gets twice the threads: 256 x 1536 self-adversarial scores 12.7 to 9.5 us
+    // (a softmax row of that length was 1 us slower with them).
+    if (lp.loss_fn == LOSS_LOGSIGMOID && lp.n_tail >= 1024)
+        return launch_dependent(k_loss<512>, dim3((unsigned)B), dim3(512), 0, stream, raw, label, coeff, loss_rows, lp, inv_normaliser, loss_total,
+                                loss_last, counter, coeff_lo, lo_bf16, extra_loss);
     return launch_dependent(k_loss<256>, dim3((unsigned)B), dim3(256), 0, stream, raw, label, coeff, loss_rows, lp, inv_normaliser, loss_total,
                             loss_last, counter, coeff_lo, lo_bf16, extra_loss);
 }
