@@ -1298,7 +1298,8 @@ void Engine::launch_planes(const char* name, tc::PlaneProblem* problems, int n_p
     int max_n = 0, max_k = 0;
     unsigned tiles = 0;
     for (int i = 0; i < n_problems; ++i) max_n = std::max(max_n, problems[i].g.N);
-    const int tile_n = max_n > 64 ? 128 : 64;
+    const bool half = problems[0].A.elem_bytes == 16;  // float16 planes: whole tiles of 128 x 128 (launch_prepared)
+    const int tile_n = max_n > 64 || half ? 128 : 64;
     for (int i = 0; i < n_problems; ++i) {
         tiles += ceil_div((unsigned)problems[i].g.M, 128) * ceil_div((unsigned)max_n, (unsigned)tile_n);
         max_k = std::max(max_k, problems[i].g.K);
@@ -1306,10 +1307,11 @@ void Engine::launch_planes(const char* name, tc::PlaneProblem* problems, int n_p
     int splits = (int)std::min<unsigned>({std::max(1u, 148u / std::max(1u, tiles)), std::max(1u, (unsigned)max_k / 64u),
                                           (unsigned)tc::kMaxClusterSplits});
     while (splits > 1 && (unsigned)tc::max_resident_plane_clusters(splits) < tiles) --splits;
+    if (half) splits = 1;
     for (int i = 0; i < n_problems; ++i) {
         tc::GemmArgs& g = problems[i].g;
         g.status = d_tc_status_;
-        const unsigned slice = problems[i].A.elem_bytes == 2 ? 64u : 32u;  // bf16 slices are 64 deep
+        const unsigned slice = problems[i].A.elem_bytes == 2 || half ? 64u : 32u;  // slices of 16-bit operands are 64 deep
         g.k_per_split = (int)std::max<size_t>(slice, round_up(ceil_div((unsigned)g.K, (unsigned)splits), slice));
     }
     timing_begin(name);
@@ -2280,6 +2282,12 @@ void Engine::refresh_lower_plane(size_t offset, size_t count) {
     KGE_CUDA(cudaStreamSynchronize(stream_));
 }
 
+// Where a pass has a wave of 128 x 128 tiles its contractions run on float16 planes (tc::HalfRows): the fp16 features as
+// they lie in the table, everything else in two parts, half the instructions and bytes of the TF32 planes and no copy of
+// the features.  Smaller passes divide k over a cluster, which those instantiations do not.  A pass of 18944 rows and
+// 1250 queries, d 256, f 768: 308 -> 178 us.
+static bool fills_gpu(unsigned m, unsigned n) { return ceil_div(m, 128) * ceil_div(n, 128) >= 148; }
+
 void Engine::ensure_predict_buffers() {
     if (p_raw_) return;
     const size_t Q = (size_t)cfg_.n_shard * cfg_.predict_hr, D = cfg_.d;
@@ -2299,6 +2307,15 @@ void Engine::ensure_predict_buffers() {
         p_chunk_lo_ = (float*)device_alloc((size_t)predict_chunk_ * D * 4);
         p_query_lo_ = (float*)device_alloc(Q * D * 4);
         if (cfg_.f) p_feat_ = (float*)device_alloc((size_t)predict_chunk_ * feat_stride_ * 4);
+        p_half_stride_ = (int)round_up(D, 8);
+        p_half_q_ = (__half*)device_alloc(2 * Q * p_half_stride_ * sizeof(__half));
+        p_half_q_info_ = (float2*)device_alloc(Q * sizeof(float2));
+        p_half_t_ = (__half*)device_alloc(2 * (size_t)predict_chunk_ * p_half_stride_ * sizeof(__half));
+        p_half_t_info_ = (float2*)device_alloc(predict_chunk_ * sizeof(float2));
+        if (cfg_.f && cfg_.feature_type == ST_F16) {
+            p_half_w_ = (__half*)device_alloc(2 * (size_t)cfg_.f * p_half_stride_ * sizeof(__half));
+            p_half_w_info_ = (float2*)device_alloc(D * sizeof(float2));
+        }
     }
     if (mlp_on()) {
         const size_t rows = std::max<size_t>(cfg_.predict_hr, predict_chunk_);
@@ -2405,8 +2422,15 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
 
     // 2. stream each local shard's rows past all queries
     const float* queries = (const float*)(arena_ + arena_offset_predict(0));
+    unsigned longest = 0;  // rows of the command's longest pass
+    for (unsigned l = 0; l < n; ++l) longest = std::max(longest, (unsigned)std::min<uint32_t>(predict_chunk_, h_count[l]));
     if (predict_planes_) {
         KGE_LAUNCH("predict_planes", k_lower_plane<<<(unsigned)std::min<size_t>((Q * D + 255) / 256, 148 * 8), 256, 0, stream_>>>(queries, Q * D, p_query_lo_));
+        if (fills_gpu((unsigned)Q, longest)) KGE_LAUNCH("predict_planes", tc::k_half_rows<<<ceil_div((unsigned)Q, 8), 256, 0, stream_>>>(queries, (int)Q, (int)D, p_half_stride_, p_half_q_,
+                                                                                                    p_half_q_ + Q * p_half_stride_, p_half_q_info_));
+        if (p_half_w_ && fills_gpu(longest, (unsigned)D))
+            KGE_LAUNCH("predict_planes", tc::k_half_columns<<<ceil_div((unsigned)D, 32), 256, 0, stream_>>>(
+                                             W_tail, (int)cfg_.f, (int)D, p_half_stride_, p_half_w_, p_half_w_ + (size_t)cfg_.f * p_half_stride_, p_half_w_info_));
     }
     TopkParams tp{(int)Q, (int)nb, score_is_gamma_minus_distance(cfg_.score_fn) ? 1 : 0, cfg_.gamma};
     for (unsigned l = 0; l < n; ++l) {
@@ -2465,7 +2489,22 @@ bool Engine::predict_pass_planes(ShardBuffers& b, uint32_t start, unsigned c, ui
                                  int net) {
     const unsigned D = cfg_.d, F = cfg_.f;
     const uint8_t* rows = b.table + (size_t)start * layout_.row_bytes;
-    if (F > 0) {
+    const bool hidden_half = F > 0 && p_half_w_ && fills_gpu(c, D), score_half = fills_gpu(Q, c);
+    auto half_plane = [&](const __half* hi, const __half* lo, bool mn_major) {
+        return tc::PlaneOperand{reinterpret_cast<const float*>(hi), reinterpret_cast<const float*>(lo), (long long)p_half_stride_ * 2, mn_major ? 1 : 0, 16};
+    };
+    if (hidden_half) {
+        tc::PlaneProblem p{};
+        p.A = tc::PlaneOperand{reinterpret_cast<const float*>(rows + layout_.off_feat), nullptr, (long long)layout_.row_bytes, 0, 16};
+        p.B = half_plane(p_half_w_, p_half_w_ + (size_t)F * p_half_stride_, true);
+        p.half_b.info = p_half_w_info_;
+        p.g.M = (int)c; p.g.N = (int)D; p.g.K = (int)F;
+        p.g.epilogue = tc::EPI_ADD_TABLE_VALUE;
+        p.g.out = p_chunk_hidden_; p.g.ldc = D; p.g.block_rows = 1;
+        p.g.x_base = rows; p.g.x_row_stride_bytes = layout_.row_bytes;
+        p.g.x_is_half = cfg_.value_bf16 ? 2 : (cfg_.state_type == ST_F16 ? 1 : 0);
+        launch_planes("predict_hidden", &p, 1, tc::SIDE_NONE, -1, -1);
+    } else if (F > 0) {
         FeaturePlanes fp{};
         const bool half_features = cfg_.feature_type == ST_F16;
         (half_features ? fp.wide : fp.lo) = p_feat_;
@@ -2490,11 +2529,20 @@ bool Engine::predict_pass_planes(ShardBuffers& b, uint32_t start, unsigned c, ui
         KGE_LAUNCH("predict_hidden", KGE_DISPATCH_ROW(cfg_, k_hidden<ST, FT><<<hgrid, 256, 0, stream_>>>(
                                                                 b.table, layout_, nullptr, start, (int)c, nullptr, nullptr, p_chunk_hidden_, nullptr)));
     }
-    KGE_LAUNCH("predict_planes", k_lower_plane<<<(unsigned)std::min<size_t>(((size_t)c * D + 255) / 256, 148 * 16), 256, 0, stream_>>>(
-                                     p_chunk_hidden_, (size_t)c * D, p_chunk_lo_));
     tc::PlaneProblem s{};
-    s.A = tc::PlaneOperand{queries, p_query_lo_, (long long)D * 4, 0, 0};
-    s.B = tc::PlaneOperand{p_chunk_hidden_, p_chunk_lo_, (long long)D * 4, 0, 0};
+    if (score_half) {
+        __half* const lo = p_half_t_ + (size_t)predict_chunk_ * p_half_stride_;
+        KGE_LAUNCH("predict_planes", tc::k_half_rows<<<ceil_div(c, 8), 256, 0, stream_>>>(p_chunk_hidden_, (int)c, (int)D, p_half_stride_, p_half_t_, lo, p_half_t_info_));
+        s.A = half_plane(p_half_q_, p_half_q_ + (size_t)Q * p_half_stride_, false);
+        s.B = half_plane(p_half_t_, lo, false);
+        s.half_a = tc::HalfRows{p_half_q_info_, queries, (long long)D * 4};
+        s.half_b = tc::HalfRows{p_half_t_info_, p_chunk_hidden_, (long long)D * 4};
+    } else {
+        KGE_LAUNCH("predict_planes", k_lower_plane<<<(unsigned)std::min<size_t>(((size_t)c * D + 255) / 256, 148 * 16), 256, 0, stream_>>>(
+                                         p_chunk_hidden_, (size_t)c * D, p_chunk_lo_));
+        s.A = tc::PlaneOperand{queries, p_query_lo_, (long long)D * 4, 0, 0};
+        s.B = tc::PlaneOperand{p_chunk_hidden_, p_chunk_lo_, (long long)D * 4, 0, 0};
+    }
     s.g.M = (int)Q; s.g.N = (int)c; s.g.K = (int)D;
     const bool l2 = cfg_.dist_fn == DIST_L2;
     s.g.epilogue = l2 ? tc::EPI_L2_DISTANCE : tc::EPI_STORE;

@@ -324,6 +324,10 @@ class Engine {
     // table rows scored per pass: 4096 on the FP32 pipe, 16384 when hidden rows and scores are tensor-core contractions
     unsigned predict_chunk_ = 4096;
     bool predict_planes_ = false;
+    // float16 planes (hi | lo, rows of p_half_stride_) and scales of the queries, a pass's hidden rows and the tails' projection
+    __half *p_half_q_ = nullptr, *p_half_t_ = nullptr, *p_half_w_ = nullptr;
+    float2 *p_half_q_info_ = nullptr, *p_half_t_info_ = nullptr, *p_half_w_info_ = nullptr;
+    int p_half_stride_ = 0;
     float *p_feat_ = nullptr, *p_chunk_lo_ = nullptr, *p_query_lo_ = nullptr;  // planes of a pass: widened / lower features, lower hidden rows, lower queries
 
     uint32_t* d_rw_idx_ = nullptr;

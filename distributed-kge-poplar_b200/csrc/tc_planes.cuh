@@ -47,7 +47,8 @@ struct PlaneOperand {
     long long row_stride_bytes;  // multiple of 16
     int mn_major;                // 0: stored [mn][k], k contiguous; 1: stored [k][mn], mn contiguous
     // 2: `hi` points at bfloat16 values, one plane, multiplied by tcgen05.mma.kind::f16 (the 2e-2 tier:
-    // bf16 embeddings with fp32 accumulation); 0 or 4: fp32 values as above.  One kind per launch.
+    // bf16 embeddings with fp32 accumulation); 0 or 4: fp32 values as above; 16: `hi` and `lo` point at float16 values
+    // (see HalfRows).  One kind per launch.
     int elem_bytes;
 };
 
@@ -67,10 +68,21 @@ struct TopkFilterArgs {
     float gamma;
 };
 
+// What belongs to an operand of float16 planes.  Every row (k-major) or column (mn-major) of the operand's [mn][k] view is
+// scaled by a power of two that brings its largest value to [2^13, 2^14), and split into two float16 parts: 22 bits of
+// every value down to 2^-15 of the row's largest, as in two TF32 planes, and below that an error of 2^-38 of the largest,
+// far under the rounding of the fp32 sums; in half the bytes and with products of 16 k per instruction instead of 8.
+struct HalfRows {
+    const float2* info;    // [mn] {squared norm of the values, what undoes the scale}; null: {-, 1}
+    const float* values;   // the fp32 rows themselves (L2 distances that cancel are recomputed from them)
+    long long stride_bytes;
+};
+
 struct PlaneProblem {
     PlaneOperand A, B;
     GemmArgs g;
     TopkFilterArgs filter;
+    HalfRows half_a, half_b;
 };
 
 // Folded into the epilogue of hidden = value + feature . W: the lookups of the step and the send
@@ -108,7 +120,7 @@ struct PlanePair {
     int wait_kind, signal_kind;
     RouteArgs route;
     int n_stages[2];  // ring stages of each problem (2 to kPlMaxStages), as many as the shared memory holds
-    int bf16;         // the operands are bfloat16 planes: 64-deep slices, kind::f16 products
+    int bf16;         // 1: the operands are bfloat16 planes, 2: float16 planes: 64-deep slices, kind::f16 products
 };
 
 struct PlaneMaps {
@@ -165,6 +177,9 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint
 __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
+
+// The same for float16 inputs (format 0).
+__host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
 
 // The copies of one slice of one plane: [ROWS x 32 k] fp32 or [ROWS x 64 k] bf16 (16 KB for 128 rows either way).
 template <int ROWS>
@@ -395,8 +410,8 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // this kernel once on an SM whose instruction cache has never seen it, and most of it is
 // straight-line code executed once: what the instantiation does not need is not fetched.
 // SPLIT: 0 no k split; else the k range is split over a cluster and a block finishes at most SPLIT units per thread
-// (3: up to 30 rows, five or more splits; 7: up to 64 rows).  BF16: bfloat16 operands.
-template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, bool BF16 = false>
+// (3: up to 30 rows, five or more splits; 7: up to 64 rows).  TYPE: 0 fp32 planes, 1 one bfloat16 plane, 2 float16 planes.
+template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, int TYPE = 0>
 __global__ void __launch_bounds__(kPlThreads, 1)
 k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneMaps maps) {
     constexpr bool kLean = EPI >= 0;
@@ -410,7 +425,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     __shared__ __align__(16) float s_colsum[2][BN];  // read in 16-byte pieces
     __shared__ unsigned long long s_cutoff[SIDE == SIDE_NORMS ? kBM : 1];  // the tile's queries' top-k cut-offs (TopkFilterArgs)
     __shared__ float s_cut_score[SIDE == SIDE_NORMS ? kBM : 1];            // their scores: a score below it cannot pass
-    constexpr bool ROWSUM = SIDE != SIDE_NONE;
+    constexpr bool ROWSUM = SIDE != SIDE_NONE && TYPE != 2;  // with float16 planes the norms come with the operands
 
     const int which = (int)blockIdx.x >= gp.tiles_m0 ? 1 : 0;
     const PlaneProblem& pp = gp.p[which];
@@ -427,7 +442,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr uint32_t kATile = kBM * 128, kBTile = BN * 128;
     const int k_begin = blockIdx.z * g.k_per_split, k_end = min(g.K, k_begin + g.k_per_split);
-    const int bf16 = kLean ? (BF16 ? 1 : 0) : gp.bf16, slice_k = bf16 ? 64 : kBK;
+    const int bf16 = kLean ? TYPE : gp.bf16, slice_k = bf16 ? 64 : kBK;
     const int n_slices = max(0, (k_end - k_begin + slice_k - 1) / slice_k);
     const bool a_two = pp.A.lo != nullptr, b_two = pp.B.lo != nullptr;
     // a ring stage: A hi [| A lo] | B hi [| B lo]
@@ -518,7 +533,23 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
                 const uint64_t db_hi = pp.B.mn_major ? make_mnmajor_sw128_desc(b_hi) : make_kmajor_sw128_desc(b_hi);
                 const uint64_t db_lo = pp.B.mn_major ? make_mnmajor_sw128_desc(b_lo) : make_kmajor_sw128_desc(b_lo);
                 uint32_t accumulate = 0u;
-                if (bf16) {
+                if (kLean && TYPE == 2) {
+                    // two float16 planes per operand (A may have one), twelve 16-deep products per 64-deep slice
+                    const uint32_t idesc16 = make_idesc_f16(kBM, BN) | (pp.A.mn_major ? (1u << 15) : 0u) | (pp.B.mn_major ? (1u << 16) : 0u);
+                    const uint64_t sa = pp.A.mn_major ? (2048 >> 4) : (32 >> 4), sb = pp.B.mn_major ? (2048 >> 4) : (32 >> 4);
+                    const uint64_t a0 = pp.A.mn_major ? make_mnmajor_sw128_desc16(a_hi) : make_kmajor_sw128_desc(a_hi);
+                    const uint64_t a1 = pp.A.mn_major ? make_mnmajor_sw128_desc16(a_lo) : make_kmajor_sw128_desc(a_lo);
+                    const uint64_t b0 = pp.B.mn_major ? make_mnmajor_sw128_desc16(b_hi) : make_kmajor_sw128_desc(b_hi);
+                    const uint64_t b1 = pp.B.mn_major ? make_mnmajor_sw128_desc16(b_lo) : make_kmajor_sw128_desc(b_lo);
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks) {
+                        const uint64_t ka = (uint64_t)ks * sa, kb = (uint64_t)ks * sb;
+                        if (b_two) { umma_bf16(tmem_acc, a0 + ka, b1 + kb, idesc16, accumulate); accumulate = 1u; }
+                        if (a_two) { umma_bf16(tmem_acc, a1 + ka, b0 + kb, idesc16, accumulate); accumulate = 1u; }
+                        umma_bf16(tmem_acc, a0 + ka, b0 + kb, idesc16, accumulate);
+                        accumulate = 1u;
+                    }
+                } else if (bf16) {
                     // one bf16 plane per operand, four 16-deep products per 64-deep slice
                     const uint32_t idesc16 = make_idesc_bf16(kBM, BN) | (pp.A.mn_major ? (1u << 15) : 0u) | (pp.B.mn_major ? (1u << 16) : 0u);
                     const uint64_t da = pp.A.mn_major ? make_mnmajor_sw128_desc16(a_hi) : make_kmajor_sw128_desc(a_hi);
@@ -579,8 +610,20 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
 #pragma unroll
                 for (int j = 0; j < 32; ++j) acc[c * 32 + j] += __uint_as_float(r[c][j]);
         }
+        if (TYPE == 2 && half == 0) {
+            // {squared norm, undo scale} of the tile's rows and columns
+            const HalfRows &ha = pp.half_a, &hb = pp.half_b;
+            const float2 of_a = ha.info && m0 + row < g.M ? ha.info[m0 + row] : make_float2(0.f, 1.f);
+            s_rowsum[0][row] = of_a.x;
+            s_rowsum[1][row] = of_a.y;
+            if (row < BN) {
+                const float2 of_b = hb.info && n0 + row < g.N ? hb.info[n0 + row] : make_float2(0.f, 1.f);
+                s_colsum[0][row] = of_b.x;
+                s_colsum[1][row] = of_b.y;
+            }
+        }
         if (ROWSUM) s_rowsum[half][row] = row_part;
-        if (SIDE == SIDE_NORMS && row < BN) s_colsum[half][row] = col_part;
+        if (SIDE == SIDE_NORMS && TYPE != 2 && row < BN) s_colsum[half][row] = col_part;
     }
     __syncthreads();  // every slice has been read from TMEM (so the ring is idle); the row sums are in place
 
@@ -626,17 +669,21 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
         const bool whole_tile = SIDE == SIDE_NORMS && !clustered && acc_warp;
         const bool filtering = whole_tile && pp.filter.cand != nullptr && m < g.M;
         if (whole_tile) {
-            const float an = s_rowsum[0][row] + s_rowsum[1][row];
+            const float an = TYPE == 2 ? s_rowsum[0][row] : s_rowsum[0][row] + s_rowsum[1][row];
+            const float undo_a = TYPE == 2 ? s_rowsum[1][row] : 1.f;
             const float cut = filtering ? s_cut_score[row] : __int_as_float(0x7f800000);
             const float sign = pp.filter.score_is_gamma_minus ? -1.f : 1.f, offset = pp.filter.score_is_gamma_minus ? pp.filter.gamma : 0.f;
 #pragma unroll
             for (int j0 = 0; j0 < CPT; j0 += 4) {
                 const int tc0 = (nc0 - n0) + j0;  // tile column of acc[j0]
                 const float4 c0 = *reinterpret_cast<const float4*>(&s_colsum[0][tc0]), c1 = *reinterpret_cast<const float4*>(&s_colsum[1][tc0]);
-                const float bn[4] = {c0.x + c1.x, c0.y + c1.y, c0.z + c1.z, c0.w + c1.w};
+                const float bn[4] = {TYPE == 2 ? c0.x : c0.x + c1.x, TYPE == 2 ? c0.y : c0.y + c1.y, TYPE == 2 ? c0.z : c0.z + c1.z,
+                                     TYPE == 2 ? c0.w : c0.w + c1.w};
+                const float undo_b[4] = {c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
-                    const float both = an + bn[t], d2 = both - 2.f * acc[j0 + t];
+                    const float dot = TYPE == 2 ? acc[j0 + t] * undo_a * undo_b[t] : acc[j0 + t];
+                    const float both = an + bn[t], d2 = both - 2.f * dot;
                     direct_bits[(j0 + t) >> 5] |= (uint32_t)(d2 < 0.2f * both) << ((j0 + t) & 31);
                     float dist;
                     asm("sqrt.approx.f32 %0, %1;" : "=f"(dist) : "f"(fmaxf(d2, 0.f)));
@@ -644,6 +691,11 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
                     pass_bits[(j0 + t) >> 5] |= (uint32_t)(fmaf(sign, dist, offset) >= cut) << ((j0 + t) & 31);
                 }
             }
+        }
+        if (TYPE == 2 && SIDE == SIDE_NONE && acc_warp) {
+            const float undo_a = s_rowsum[1][row];
+#pragma unroll
+            for (int j = 0; j < CPT; ++j) acc[j] = acc[j] * undo_a * s_colsum[1][nc0 - n0 + j];
         }
         if (acc_warp) {
             // 16-byte chunk c of tile row `row` lies at chunk c ^ (row & 7): the lanes of a warp hold
@@ -656,7 +708,11 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
                 *reinterpret_cast<float4*>(mine + (((c0 + (j >> 2)) ^ (row & 7)) << 2)) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
             if (ROWSUM && nc0 == n0) staging[(size_t)owner * slot_floats + off_rowsum + local] = s_rowsum[0][row] + s_rowsum[1][row];
             if (whole_tile && m < g.M) {
-                const float* a_row = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(pp.A.hi) + (size_t)m * pp.A.row_stride_bytes);
+                const uint8_t* const a_values = reinterpret_cast<const uint8_t*>(TYPE == 2 ? pp.half_a.values : pp.A.hi);
+                const uint8_t* const b_values = reinterpret_cast<const uint8_t*>(TYPE == 2 ? pp.half_b.values : pp.B.hi);
+                const size_t a_stride = (size_t)(TYPE == 2 ? pp.half_a.stride_bytes : pp.A.row_stride_bytes);
+                const size_t b_stride = (size_t)(TYPE == 2 ? pp.half_b.stride_bytes : pp.B.row_stride_bytes);
+                const float* a_row = reinterpret_cast<const float*>(a_values + (size_t)m * a_stride);
 #pragma unroll
                 for (int w = 0; w < CPT / 32; ++w) {
                     uint32_t todo = direct_bits[w] | (filtering ? pass_bits[w] : 0u);
@@ -666,7 +722,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
                         if (col >= g.N) continue;
                         float* cell = mine + (((tcol >> 2) ^ (row & 7)) << 2) + (tcol & 3);
                         if ((direct_bits[w] >> bit) & 1u) {
-                            const float d2 = l2_squared_direct(a_row, reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(pp.B.hi) + (size_t)col * pp.B.row_stride_bytes), g.K);
+                            const float d2 = l2_squared_direct(a_row, reinterpret_cast<const float*>(b_values + (size_t)col * b_stride), g.K);
                             *cell = sqrtf(d2);
                         }
                         if (filtering) {
@@ -805,6 +861,77 @@ static __global__ void __launch_bounds__(256) k_split_planes(const float* __rest
     }
 }
 
+// The float16 planes of an operand (HalfRows).  The scale 2^(s - 127) for values up to `largest`, as a biased exponent:
+// the largest lands in [2^13, 2^14); no scaling of a row that holds infinities or NaNs.
+__device__ __forceinline__ uint32_t half_scale_exponent(float largest) {
+    const uint32_t e = (__float_as_uint(largest) >> 23) & 255u;
+    return e == 255u ? 127u : min(253u, 267u - e);
+}
+__device__ __forceinline__ float power_of_two(uint32_t biased) { return __uint_as_float(biased << 23); }
+__device__ __forceinline__ void half_split(float v, __half& hi, __half& lo) {
+    hi = __float2half_rn(v);
+    lo = __float2half_rn(v - __half2float(hi));
+}
+
+// x [rows, D] (D a multiple of 4) into hi and lo [rows, stride], a warp per row; bound by memory (65536 x 256: 128 MB).
+static __global__ void __launch_bounds__(256)
+k_half_rows(const float* __restrict__ x, int rows, int D, int stride, __half* __restrict__ hi, __half* __restrict__ lo, float2* __restrict__ info) {
+    const int r = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= rows) return;
+    const float* __restrict__ row = x + (size_t)r * D;
+    float largest = 0.f, square = 0.f;
+    for (int c = lane * 4; c < D; c += 128) {
+        const float4 v = load4(row + c);
+        largest = fmaxf(fmaxf(largest, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+        square += (v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w);
+    }
+    for (int o = 16; o > 0; o >>= 1) largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, o));
+    square = warp_sum(square);
+    const uint32_t s = square != square ? 127u : half_scale_exponent(largest);  // (fmaxf drops NaNs)
+    const float scale = power_of_two(s);
+    for (int c = lane * 4; c < D; c += 128) {  // from L1
+        const float4 v = load4(row + c);
+        __half h[4], l[4];
+        half_split(v.x * scale, h[0], l[0]);
+        half_split(v.y * scale, h[1], l[1]);
+        half_split(v.z * scale, h[2], l[2]);
+        half_split(v.w * scale, h[3], l[3]);
+        *reinterpret_cast<uint2*>(hi + (size_t)r * stride + c) = *reinterpret_cast<const uint2*>(h);
+        *reinterpret_cast<uint2*>(lo + (size_t)r * stride + c) = *reinterpret_cast<const uint2*>(l);
+    }
+    if (lane == 0) info[r] = make_float2(square, power_of_two(254u - s));
+}
+
+// w [F, D] into hi and lo [F, stride], scaled by columns: 32 columns per block, eight rows at a time.
+static __global__ void __launch_bounds__(256)
+k_half_columns(const float* __restrict__ w, int F, int D, int stride, __half* __restrict__ hi, __half* __restrict__ lo, float2* __restrict__ info) {
+    __shared__ float part[8][32];
+    const int lane = threadIdx.x & 31, group = threadIdx.x >> 5, c = (int)blockIdx.x * 32 + lane;
+    float largest = 0.f;
+    bool odd = false;
+    if (c < D)
+#pragma unroll 4
+        for (int f = group; f < F; f += 8) {
+            const float v = fabsf(w[(size_t)f * D + c]);
+            odd = odd || !(v <= 3.4028235e38f);
+            largest = fmaxf(largest, v);
+        }
+    part[group][lane] = odd ? __int_as_float(0x7f800000) : largest;
+    __syncthreads();
+    for (int g = 0; g < 8; ++g) largest = fmaxf(largest, part[g][lane]);
+    if (c >= D) return;
+    const uint32_t s = half_scale_exponent(largest);
+    const float scale = power_of_two(s);
+#pragma unroll 4
+    for (int f = group; f < F; f += 8) {
+        __half h, l;
+        half_split(w[(size_t)f * D + c] * scale, h, l);
+        hi[(size_t)f * stride + c] = h;
+        lo[(size_t)f * stride + c] = l;
+    }
+    if (group == 0) info[c] = make_float2(0.f, power_of_two(254u - s));
+}
+
 // What a producing kernel stores for four neighbouring values.
 __device__ __forceinline__ void store_planes4(float* hi, float* lo, size_t e, float a, float b, float c, float d) {
     const float4 h = make_float4(tf32_hi(a), tf32_hi(b), tf32_hi(c), tf32_hi(d));
@@ -821,14 +948,14 @@ inline cudaError_t make_plane_map(const float* base, const PlaneOperand& op, int
     EncodeTiledFn encode = encode_tiled_fn();
     if (!encode) return cudaErrorNotSupported;
     if (reinterpret_cast<uintptr_t>(base) % 16 || op.row_stride_bytes % 16) return cudaErrorInvalidValue;
-    const bool bf16 = op.elem_bytes == 2;
+    const bool bf16 = op.elem_bytes == 2 || op.elem_bytes == 16;  // 16-bit elements
     const cuuint64_t dims[2] = {(cuuint64_t)(op.mn_major ? mn : k), (cuuint64_t)(op.mn_major ? k : mn)};
     const cuuint64_t strides[1] = {(cuuint64_t)op.row_stride_bytes};
     // 128 bytes along the contiguous dimension; a slice is 32 k deep in fp32 and 64 k deep in bf16
     const cuuint32_t inner = bf16 ? 64u : 32u;
     const cuuint32_t box[2] = {inner, (cuuint32_t)(op.mn_major ? inner : rows)};
     const cuuint32_t elem[2] = {1, 1};
-    const CUresult r = encode(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims,
+    const CUresult r = encode(map, op.elem_bytes == 16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims,
                               strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                               op.mn_major && !bf16 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -839,12 +966,12 @@ inline bool planes_aligned(const PlaneOperand& op) {
     return reinterpret_cast<uintptr_t>(op.hi) % 16 == 0 && reinterpret_cast<uintptr_t>(op.lo) % 16 == 0 && op.row_stride_bytes % 16 == 0;
 }
 
-template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, bool BF16 = false>
+template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, int TYPE = 0>
 inline cudaError_t configure_planes() {
     static bool configured[kMaxDeviceOrdinals] = {};
     const int slot = current_device_slot();
     if (slot >= 0 && configured[slot]) return cudaSuccess;
-    cudaError_t err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem_bytes());
+    cudaError_t err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem_bytes());
     if (err == cudaSuccess && slot >= 0) configured[slot] = true;
     return err;
 }
@@ -912,11 +1039,13 @@ inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, 
         tiles_m += (problems[1].g.M + kBM - 1) / kBM;
         tiles_n = std::max(tiles_n, (problems[1].g.N + tile_n - 1) / tile_n);
     }
-    gp.bf16 = problems[0].A.elem_bytes == 2 ? 1 : 0;
+    auto type_of = [](const PlaneOperand& op) { return op.elem_bytes == 16 ? 2 : op.elem_bytes == 2 ? 1 : 0; };
+    gp.bf16 = type_of(problems[0].A);
     for (int i = 0; i < 2; ++i) {
         PlaneProblem& q = gp.p[i];
-        if ((q.A.elem_bytes == 2) != (gp.bf16 != 0) || (q.B.elem_bytes == 2) != (gp.bf16 != 0)) return cudaErrorInvalidValue;
-        if (gp.bf16 && (q.A.lo || q.B.lo || q.g.k_per_split % 64)) return cudaErrorInvalidValue;
+        if (type_of(q.A) != gp.bf16 || type_of(q.B) != gp.bf16) return cudaErrorInvalidValue;
+        if (gp.bf16 == 1 && (q.A.lo || q.B.lo)) return cudaErrorInvalidValue;
+        if (gp.bf16 && q.g.k_per_split % 64) return cudaErrorInvalidValue;
         q.g.ws = nullptr;
         q.g.cluster_splits = splits > 1 ? splits : 0;
         if (!planes_aligned(q.A) || !planes_aligned(q.B)) return cudaErrorInvalidValue;
@@ -934,11 +1063,11 @@ inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, 
     return cudaSuccess;
 }
 
-template <int SIDE, int EPI, int SPLIT, bool BF16 = false>
+template <int SIDE, int EPI, int SPLIT, int TYPE = 0>
 inline cudaError_t launch_lean(const PlaneLaunch& l, cudaStream_t stream) {
-    cudaError_t err = configure_planes<128, SIDE, EPI, SPLIT, BF16>();
+    cudaError_t err = configure_planes<128, SIDE, EPI, SPLIT, TYPE>();
     if (err != cudaSuccess) return err;
-    return launch_dependent_cluster(k_tc_planes<128, SIDE, EPI, SPLIT, BF16>, l.grid, dim3(kPlThreads), plane_smem_bytes(), stream, (unsigned)l.splits,
+    return launch_dependent_cluster(k_tc_planes<128, SIDE, EPI, SPLIT, TYPE>, l.grid, dim3(kPlThreads), plane_smem_bytes(), stream, (unsigned)l.splits,
                                     l.gp, l.maps);
 }
 // By the number of k splits: five or more leave at most 26 rows of a tile to a block.
@@ -951,17 +1080,28 @@ inline cudaError_t launch_lean_split(const PlaneLaunch& l, cudaStream_t stream) 
 
 template <int SIDE>
 inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
-    if (SIDE != SIDE_NONE && l.gp.bf16) return cudaErrorInvalidValue;  // the side sums read fp32 tiles
+    if (SIDE != SIDE_NONE && l.gp.bf16 == 1) return cudaErrorInvalidValue;  // the side sums read fp32 tiles
     if (SIDE == SIDE_NORMS)
         for (int i = 0; i < 2; ++i)
             if (l.gp.p[i].A.mn_major || l.gp.p[i].B.mn_major || l.gp.p[i].g.out_blocks) return cudaErrorInvalidValue;
+    if (l.gp.bf16 == 2) {  // whole tiles of one problem only (ranking)
+        const int epilogue = l.gp.p[0].g.epilogue;
+        if (l.tile_n != 128 || l.splits != 1) return cudaErrorInvalidValue;
+        if constexpr (SIDE == SIDE_NONE) {
+            if (epilogue == EPI_ADD_TABLE_VALUE) return launch_lean<SIDE_NONE, EPI_ADD_TABLE_VALUE, 0, 2>(l, stream);
+            if (epilogue == EPI_STORE) return launch_lean<SIDE_NONE, EPI_STORE, 0, 2>(l, stream);
+        } else if constexpr (SIDE == SIDE_NORMS) {
+            if (epilogue == EPI_L2_DISTANCE) return launch_lean<SIDE_NORMS, EPI_L2_DISTANCE, 0, 2>(l, stream);
+        }
+        return cudaErrorInvalidValue;
+    }
     if (l.tile_n == 128) {
         // one epilogue for the launch: the instantiation for it
         const int epilogue = l.gp.p[0].g.epilogue;
         if (l.gp.p[1].g.epilogue == epilogue) {
             if constexpr (SIDE == SIDE_NONE) {
                 if (l.gp.bf16) {
-                    if (epilogue == EPI_STORE) return l.splits > 1 ? launch_lean<SIDE_NONE, EPI_STORE, 7, true>(l, stream) : launch_lean<SIDE_NONE, EPI_STORE, 0, true>(l, stream);
+                    if (epilogue == EPI_STORE) return l.splits > 1 ? launch_lean<SIDE_NONE, EPI_STORE, 7, 1>(l, stream) : launch_lean<SIDE_NONE, EPI_STORE, 0, 1>(l, stream);
                 } else {
                     if (epilogue == EPI_ADD_TABLE_VALUE) return launch_lean_split<SIDE_NONE, EPI_ADD_TABLE_VALUE>(l, stream);
                     if (epilogue == EPI_DENSE_ADAM) return launch_lean_split<SIDE_NONE, EPI_DENSE_ADAM>(l, stream);

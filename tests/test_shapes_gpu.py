@@ -77,3 +77,26 @@ def test_ranking_lists(monkeypatch, score_fn, distance_fn, n_best, pass_rows):
     assert_close(got_score, want_score, RTOL, "ranking: scores")
     clear = _clear(want_score) if n_best > 1 else np.ones_like(want_score, bool)
     np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
+
+
+@pytest.mark.parametrize("score_fn,distance_fn", [("TransE", "L2"), ("DistMult", "MatMul")])
+@pytest.mark.parametrize("queries,rows,size,features", [(129, 9473, 20, 0), (130, 9500, 132, 70), (5, 18945, 12, 9)])
+def test_ranking_in_whole_tiles(monkeypatch, score_fn, distance_fn, queries, rows, size, features):
+    """Passes with 148 and more tiles (float16 planes): ragged rows, columns and depths, rows of very different size, and
+    a last pass below 148."""
+    monkeypatch.setenv("KGE_PREDICT_PASS_ROWS", str(rows // 4 * 4))
+    n_entity = rows + 300
+    cfg = StepConfig(n_shard=1, n_entity=n_entity, n_relation_type=4, embedding_size=size, entity_feature_size=features, batch_size=8, a2a_size=6,
+                     score_fn=score_fn, distance_fn=distance_fn, gamma=8.0)
+    state = random_state(cfg, 3, fp16_features=True, warm=True)
+    state["entity_data"][0, 1::3, :size] *= 1e-3
+    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW, feature_dtype="float16", **{"execution.predict_hr_batch_size": queries, "execution.predict_n_best": 10}))
+    write_state(engine, cfg, state, RW)
+    rng = np.random.RandomState(1)
+    hr = np.stack([np.zeros(queries, int), 1 + rng.randint(n_entity - 1, size=queries), rng.randint(4, size=queries)], axis=1)
+    got_idx, got_score = _predict(engine, cfg, hr, np.array([n_entity - 1]), queries, 10)
+    engine.close()
+    want_idx, want_score = make_oracle(cfg, state).predict(hr, np.array([n_entity - 1]), 10)
+    assert_close(got_score, want_score, RTOL, "ranking: scores")
+    clear = _clear(want_score)
+    np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
