@@ -135,7 +135,12 @@ constexpr int kPlTmemSlots = 4;
 // Dynamic shared memory of a block: the operand ring (the partial rows of a cluster's k split land
 // in the same memory once the ring is idle), after alignment to 1024 bytes.
 constexpr size_t kPlRingBytes = 220 * 1024;
-constexpr size_t plane_smem_bytes() { return 1024 + kPlRingBytes; }
+// Float16 planes: a ring of six single planes (16 KB each), so that two blocks fit on an SM and one's mainloop runs under
+// the other's epilogue; they share TMEM, two accumulators each.
+constexpr int kPlHalfSlots = 6;
+constexpr int kPlHalfTmemSlots = 2;
+constexpr size_t plane_smem_bytes(int type = 0) { return 1024 + (type == 2 ? (size_t)kPlHalfSlots * 128 * 128 : kPlRingBytes); }
+static_assert((128 * 128 + 128 + 128) * 4 <= kPlHalfSlots * 128 * 128, "a staged tile and its sums");
 static_assert(2 * ((size_t)(kBM + kMaxClusterRows) * (128 + 1) + 8 * 128) * 4 <= 150 * 1024, "the sent and the received rows of a k split");
 static_assert(150 * 1024 + 64 * 128 * 4 <= 184 * 1024 && (128 * 128 + 128 + 128) * 4 <= 72 * 1024 && 72 * 1024 + 128 * 128 * 4 <= 184 * 1024 && 184 * 1024 + (2 * 4096 + kBM + 1) * 4 <= kPlRingBytes, "finished rows and staged lookups behind them");
 
@@ -402,6 +407,14 @@ __device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&r)[32
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -411,14 +424,19 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // straight-line code executed once: what the instantiation does not need is not fetched.
 // SPLIT: 0 no k split; else the k range is split over a cluster and a block finishes at most SPLIT units per thread
 // (3: up to 30 rows, five or more splits; 7: up to 64 rows).  TYPE: 0 fp32 planes, 1 one bfloat16 plane, 2 float16 planes.
+//
+// TYPE 2 (whole tiles, many per SM): at one block per SM a 128 x 128 tile of d 256 took 11 us, of which the products are
+// 1.7; the rest is start, first loads and epilogue.  Two blocks per SM, hence the smaller ring and 96 registers: 1250 x 18944 scores of
+// d 256 110 -> 82 us, 18944 x 256 hidden rows of f 768 46 -> 31 us.
 template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, int TYPE = 0>
-__global__ void __launch_bounds__(kPlThreads, 1)
+__global__ void __launch_bounds__(kPlThreads, TYPE == 2 ? 2 : 1)
 k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneMaps maps) {
     constexpr bool kLean = EPI >= 0;
     static_assert(BN == 64 || BN == 128, "tile widths: 64 or 128 columns");
     constexpr int CPT = BN / 2;  // accumulator columns per accumulating thread: a warp reads one half of its 32 lanes' columns
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t bar_full[kPlMaxStages], bar_empty[kPlMaxStages], bar_acc_ready[kPlTmemSlots], bar_acc_free[kPlTmemSlots];
+    constexpr int kBars = TYPE == 2 ? kPlHalfSlots : kPlMaxStages;
+    __shared__ uint64_t bar_full[kBars], bar_empty[kBars], bar_acc_ready[kPlTmemSlots], bar_acc_free[kPlTmemSlots];
     __shared__ uint64_t bar_reduce;
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(16) float s_rowsum[2][kBM];
@@ -450,7 +468,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     const int n_stages = gp.n_stages[which];
 
     if (tid == 0) {
-        for (int s = 0; s < kPlMaxStages; ++s) {
+        for (int s = 0; s < kBars; ++s) {
             mbar_init(&bar_full[s], 1);
             mbar_init(&bar_empty[s], ROWSUM ? 1 + kPlAccWarps : 1);
         }
@@ -466,7 +484,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
         if (a_two) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.a_lo[which])) : "memory");
         if (b_two) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.b_lo[which])) : "memory");
     }
-    constexpr int n_slots = kPlTmemSlots;
+    constexpr int n_slots = TYPE == 2 ? kPlHalfTmemSlots : kPlTmemSlots;
     if (warp == 0) tmem_alloc(&tmem_slot, (uint32_t)(n_slots * BN));
     tc_fence_before();
     __syncthreads();
@@ -502,7 +520,80 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     for (int j = 0; j < CPT; ++j) acc[j] = 0.f;
     float row_part = 0.f, col_part = 0.f;
 
-    if (warp == 0) {
+    // TYPE 2: a slice's planes B lo, A hi[, A lo], B hi, each in the next slot of the ring and given back after its last product
+    const int n_planes = a_two ? 4 : 3;
+    if (TYPE == 2 && warp == 0) {
+        for (int i = 0, kc = 0; kc < n_slices; ++kc) {
+            const int k0 = k_begin + kc * slice_k;
+            for (int j = 0; j < n_planes; ++j, ++i) {
+                const int s = i % kPlHalfSlots, use = i / kPlHalfSlots;
+                if (use >= 1) mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), g.status, 6u);
+                if (lane == 0) {
+                    uint8_t* slot = smem + (size_t)s * kATile;
+                    mbar_arrive_expect(&bar_full[s], kATile);
+                    if (j == 0 || j == n_planes - 1)
+                        tma_plane_tile<BN>(slot, j == 0 ? &maps.b_lo[which] : &maps.b_hi[which], pp.B.mn_major, 1, n0, k0, &bar_full[s]);
+                    else
+                        tma_plane_tile<kBM>(slot, j == 1 ? &maps.a_hi[which] : &maps.a_lo[which], pp.A.mn_major, 1, m0, k0, &bar_full[s]);
+                }
+                __syncwarp();
+            }
+        }
+    } else if (TYPE == 2 && warp == 1) {
+        const uint32_t idesc = make_idesc_f16(kBM, BN) | (pp.A.mn_major ? (1u << 15) : 0u) | (pp.B.mn_major ? (1u << 16) : 0u);
+        const uint64_t sa = pp.A.mn_major ? (2048 >> 4) : (32 >> 4), sb = pp.B.mn_major ? (2048 >> 4) : (32 >> 4);
+        for (int i0 = 0, kc = 0; kc < n_slices; ++kc, i0 += n_planes) {
+            const int t = kc % n_slots;
+            if (kc >= n_slots) mbar_wait(&bar_acc_free[t], (uint32_t)(((kc / n_slots) - 1) & 1), g.status, 4u);
+            const uint32_t tmem_acc = tmem_base + (uint32_t)(t * BN);
+            uint32_t accumulate = 0u;
+            auto arrived = [&](int j) {
+                const int i = i0 + j;
+                mbar_wait(&bar_full[i % kPlHalfSlots], (uint32_t)((i / kPlHalfSlots) & 1), g.status, 3u);
+            };
+            auto multiply = [&](int ja, int jb) {  // four 16-deep products of a 64-deep slice
+                const uint32_t a = smem_u32(smem + (size_t)((i0 + ja) % kPlHalfSlots) * kATile), b = smem_u32(smem + (size_t)((i0 + jb) % kPlHalfSlots) * kATile);
+                const uint64_t da = pp.A.mn_major ? make_mnmajor_sw128_desc16(a) : make_kmajor_sw128_desc(a);
+                const uint64_t db = pp.B.mn_major ? make_mnmajor_sw128_desc16(b) : make_kmajor_sw128_desc(b);
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) {
+                    umma_bf16(tmem_acc, da + (uint64_t)ks * sa, db + (uint64_t)ks * sb, idesc, accumulate);
+                    accumulate = 1u;
+                }
+            };
+            auto give_back = [&](int j) { umma_commit(&bar_empty[(i0 + j) % kPlHalfSlots]); };
+            const int b_hi = n_planes - 1;
+            // small cross terms first, the large hi*hi term last
+            arrived(0);
+            arrived(1);
+            tc_fence_after();
+            if (lane == 0) {
+                multiply(1, 0);
+                give_back(0);
+            }
+            __syncwarp();
+            if (a_two) {
+                arrived(2);
+                arrived(b_hi);
+                tc_fence_after();
+                if (lane == 0) {
+                    multiply(2, b_hi);
+                    give_back(2);
+                }
+                __syncwarp();
+            } else {
+                arrived(b_hi);
+                tc_fence_after();
+            }
+            if (lane == 0) {
+                multiply(1, b_hi);
+                give_back(1);
+                give_back(b_hi);
+                umma_commit(&bar_acc_ready[t]);
+            }
+            __syncwarp();
+        }
+    } else if (warp == 0) {
         for (int kc = 0; kc < n_slices; ++kc) {
             const int s = kc % n_stages, use = kc / n_stages;
             if (use >= 1) mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), g.status, 6u);
@@ -533,23 +624,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
                 const uint64_t db_hi = pp.B.mn_major ? make_mnmajor_sw128_desc(b_hi) : make_kmajor_sw128_desc(b_hi);
                 const uint64_t db_lo = pp.B.mn_major ? make_mnmajor_sw128_desc(b_lo) : make_kmajor_sw128_desc(b_lo);
                 uint32_t accumulate = 0u;
-                if (kLean && TYPE == 2) {
-                    // two float16 planes per operand (A may have one), twelve 16-deep products per 64-deep slice
-                    const uint32_t idesc16 = make_idesc_f16(kBM, BN) | (pp.A.mn_major ? (1u << 15) : 0u) | (pp.B.mn_major ? (1u << 16) : 0u);
-                    const uint64_t sa = pp.A.mn_major ? (2048 >> 4) : (32 >> 4), sb = pp.B.mn_major ? (2048 >> 4) : (32 >> 4);
-                    const uint64_t a0 = pp.A.mn_major ? make_mnmajor_sw128_desc16(a_hi) : make_kmajor_sw128_desc(a_hi);
-                    const uint64_t a1 = pp.A.mn_major ? make_mnmajor_sw128_desc16(a_lo) : make_kmajor_sw128_desc(a_lo);
-                    const uint64_t b0 = pp.B.mn_major ? make_mnmajor_sw128_desc16(b_hi) : make_kmajor_sw128_desc(b_hi);
-                    const uint64_t b1 = pp.B.mn_major ? make_mnmajor_sw128_desc16(b_lo) : make_kmajor_sw128_desc(b_lo);
-#pragma unroll
-                    for (int ks = 0; ks < 4; ++ks) {
-                        const uint64_t ka = (uint64_t)ks * sa, kb = (uint64_t)ks * sb;
-                        if (b_two) { umma_bf16(tmem_acc, a0 + ka, b1 + kb, idesc16, accumulate); accumulate = 1u; }
-                        if (a_two) { umma_bf16(tmem_acc, a1 + ka, b0 + kb, idesc16, accumulate); accumulate = 1u; }
-                        umma_bf16(tmem_acc, a0 + ka, b0 + kb, idesc16, accumulate);
-                        accumulate = 1u;
-                    }
-                } else if (bf16) {
+                if (bf16) {
                     // one bf16 plane per operand, four 16-deep products per 64-deep slice
                     const uint32_t idesc16 = make_idesc_bf16(kBM, BN) | (pp.A.mn_major ? (1u << 15) : 0u) | (pp.B.mn_major ? (1u << 16) : 0u);
                     const uint64_t da = pp.A.mn_major ? make_mnmajor_sw128_desc16(a_hi) : make_kmajor_sw128_desc(a_hi);
@@ -598,6 +673,19 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
             mbar_wait(&bar_acc_ready[t], (uint32_t)((kc / n_slots) & 1), g.status, 1u);
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * BN + half * CPT);
+            if constexpr (TYPE == 2) {  // 16 columns at a time: registers for two blocks
+#pragma unroll
+                for (int c = 0; c < CPT / 16; ++c) {
+                    uint32_t r[16];
+                    tmem_ld16_issue(taddr + (uint32_t)(c * 16), r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) acc[c * 16 + j] += __uint_as_float(r[j]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_acc_free[t]);
+            } else {
             uint32_t r[CPT / 32][32];
 #pragma unroll
             for (int c = 0; c < CPT / 32; ++c) tmem_ld32_issue(taddr + (uint32_t)(c * 32), r[c]);
@@ -609,6 +697,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
             for (int c = 0; c < CPT / 32; ++c)
 #pragma unroll
                 for (int j = 0; j < 32; ++j) acc[c * 32 + j] += __uint_as_float(r[c][j]);
+            }
         }
         if (TYPE == 2 && half == 0) {
             // {squared norm, undo scale} of the tile's rows and columns
@@ -629,7 +718,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
 
     // Routing (hidden rows to their lookups): the finished rows and the staged lookups live in the
     // idle ring, behind what the k-split exchange uses.
-    const bool routing = (!kLean || EPI == EPI_ADD_TABLE_VALUE) && gp.route.perm != nullptr && gp.route.mode[which] != 0;
+    const bool routing = TYPE != 2 && (!kLean || EPI == EPI_ADD_TABLE_VALUE) && gp.route.perm != nullptr && gp.route.mode[which] != 0;
     float* fin = reinterpret_cast<float*>(smem + 150 * 1024);                              // [<= 64 rows][BN], or [128][BN] at offset 0 without a k split
     uint32_t* s_look = reinterpret_cast<uint32_t*>(smem + 184 * 1024);                      // [kRouteMaxLookups]
     uint32_t* s_rel = s_look + kRouteMaxLookups;                                            // [kRouteMaxLookups]
@@ -971,7 +1060,9 @@ inline cudaError_t configure_planes() {
     static bool configured[kMaxDeviceOrdinals] = {};
     const int slot = current_device_slot();
     if (slot >= 0 && configured[slot]) return cudaSuccess;
-    cudaError_t err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem_bytes());
+    cudaError_t err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem_bytes(TYPE));
+    if (err == cudaSuccess && TYPE == 2)  // room for two blocks
+        err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, TYPE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (err == cudaSuccess && slot >= 0) configured[slot] = true;
     return err;
 }
@@ -1045,6 +1136,7 @@ inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, 
         PlaneProblem& q = gp.p[i];
         if (type_of(q.A) != gp.bf16 || type_of(q.B) != gp.bf16) return cudaErrorInvalidValue;
         if (gp.bf16 == 1 && (q.A.lo || q.B.lo)) return cudaErrorInvalidValue;
+        if (gp.bf16 == 2 && !q.B.lo) return cudaErrorInvalidValue;  // B always has two planes
         if (gp.bf16 && q.g.k_per_split % 64) return cudaErrorInvalidValue;
         q.g.ws = nullptr;
         q.g.cluster_splits = splits > 1 ? splits : 0;
@@ -1067,7 +1159,7 @@ template <int SIDE, int EPI, int SPLIT, int TYPE = 0>
 inline cudaError_t launch_lean(const PlaneLaunch& l, cudaStream_t stream) {
     cudaError_t err = configure_planes<128, SIDE, EPI, SPLIT, TYPE>();
     if (err != cudaSuccess) return err;
-    return launch_dependent_cluster(k_tc_planes<128, SIDE, EPI, SPLIT, TYPE>, l.grid, dim3(kPlThreads), plane_smem_bytes(), stream, (unsigned)l.splits,
+    return launch_dependent_cluster(k_tc_planes<128, SIDE, EPI, SPLIT, TYPE>, l.grid, dim3(kPlThreads), plane_smem_bytes(TYPE), stream, (unsigned)l.splits,
                                     l.gp, l.maps);
 }
 // By the number of k splits: five or more leave at most 26 rows of a tile to a block.
