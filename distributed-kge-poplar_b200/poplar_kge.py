@@ -741,13 +741,23 @@ class Engine:
             predict_relation=np.ascontiguousarray(idx_relation[:, :, 1], dtype=np.uint32),
             predict_entity_count=np.ascontiguousarray(self.shard_to_entity_count[self.local_shards], dtype=np.uint32),
             predict_scores=scores, predict_indices=indices))
-        shard_idx = np.empty(indices.shape + (2,), dtype=np.uint32)
-        shard_idx[..., 0] = np.arange(n, dtype=np.uint32)[None, :, None, None]
-        shard_idx[..., 1] = indices
-        merged = Predictions(
-            shard_idx=shard_idx.transpose(0, 2, 1, 3, 4).reshape(self.n_local, e.predict_hr_batch_size, -1, 2),
-            score=scores.transpose(0, 2, 1, 3).reshape(self.n_local, e.predict_hr_batch_size, -1))
-        return merged.topk(e.predict_n_best).sort()
+        k, width = e.predict_n_best, n * e.predict_n_best
+        shape = (self.n_local, e.predict_hr_batch_size, k)
+        shard_idx = np.empty((shape[0] * shape[1], k, 2), dtype=np.uint32)
+        if n == 1:  # the engine's list is sorted, equal scores by row: there is nothing to merge
+            shard_idx[..., 0] = 0
+            shard_idx[..., 1] = indices.reshape(-1, k)
+            return Predictions(shard_idx=shard_idx.reshape(shape + (2,)), score=scores.reshape(shape))
+        # The shards' lists side by side, merged as Predictions.topk().sort() does; the orders are applied to the scores
+        # first and the candidates are gathered once, which halves the time on the host.
+        flat = scores.transpose(0, 2, 1, 3).reshape(-1, width)
+        first = (np.arange(flat.shape[0]) * width)[:, None]
+        best = np.argpartition(flat, -k, axis=1)[:, -k:]
+        order = np.take_along_axis(best, np.argsort(flat.ravel().take(first + best), axis=1)[:, ::-1], axis=1)
+        np.floor_divide(order, k, out=shard_idx[..., 0], casting="unsafe")
+        order += first
+        shard_idx[..., 1] = indices.transpose(0, 2, 1, 3).ravel().take(order)
+        return Predictions(shard_idx=shard_idx.reshape(shape + (2,)), score=flat.ravel().take(order).reshape(shape))
 
     def predict_chunks(self, query_shards: np.ndarray) -> int:
         """Engine "predict" calls needed for queries whose head shards are ``query_shards``: the
