@@ -120,7 +120,7 @@ struct PlanePair {
     int wait_kind, signal_kind;
     RouteArgs route;
     int n_stages[2];  // ring stages of each problem (2 to kPlMaxStages), as many as the shared memory holds
-    int bf16;         // 1: the operands are bfloat16 planes, 2: float16 planes: 64-deep slices, kind::f16 products
+    int bf16;         // 1: the operands are bfloat16 planes, 2: float16 planes (k_half_tiles): 64-deep slices, kind::f16 products
 };
 
 struct PlaneMaps {
@@ -135,12 +135,7 @@ constexpr int kPlTmemSlots = 4;
 // Dynamic shared memory of a block: the operand ring (the partial rows of a cluster's k split land
 // in the same memory once the ring is idle), after alignment to 1024 bytes.
 constexpr size_t kPlRingBytes = 220 * 1024;
-// Float16 planes: a ring of six single planes (16 KB each), so that two blocks fit on an SM and one's mainloop runs under
-// the other's epilogue; they share TMEM, two accumulators each.
-constexpr int kPlHalfSlots = 6;
-constexpr int kPlHalfTmemSlots = 2;
-constexpr size_t plane_smem_bytes(int type = 0) { return 1024 + (type == 2 ? (size_t)kPlHalfSlots * 128 * 128 : kPlRingBytes); }
-static_assert((128 * 128 + 128 + 128) * 4 <= kPlHalfSlots * 128 * 128, "a staged tile and its sums");
+constexpr size_t plane_smem_bytes() { return 1024 + kPlRingBytes; }
 static_assert(2 * ((size_t)(kBM + kMaxClusterRows) * (128 + 1) + 8 * 128) * 4 <= 150 * 1024, "the sent and the received rows of a k split");
 static_assert(150 * 1024 + 64 * 128 * 4 <= 184 * 1024 && (128 * 128 + 128 + 128) * 4 <= 72 * 1024 && 72 * 1024 + 128 * 128 * 4 <= 184 * 1024 && 184 * 1024 + (2 * 4096 + kBM + 1) * 4 <= kPlRingBytes, "finished rows and staged lookups behind them");
 
@@ -407,14 +402,6 @@ __device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&r)[32
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr)
-        : "memory");
-}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
@@ -423,27 +410,22 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // this kernel once on an SM whose instruction cache has never seen it, and most of it is
 // straight-line code executed once: what the instantiation does not need is not fetched.
 // SPLIT: 0 no k split; else the k range is split over a cluster and a block finishes at most SPLIT units per thread
-// (3: up to 30 rows, five or more splits; 7: up to 64 rows).  TYPE: 0 fp32 planes, 1 one bfloat16 plane, 2 float16 planes.
-//
-// TYPE 2 (whole tiles, many per SM): at one block per SM a 128 x 128 tile of d 256 took 11 us, of which the products are
-// 1.7; the rest is start, first loads and epilogue.  Two blocks per SM, hence the smaller ring and 96 registers: 1250 x 18944 scores of
-// d 256 110 -> 82 us, 18944 x 256 hidden rows of f 768 46 -> 31 us.
-template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, int TYPE = 0>
-__global__ void __launch_bounds__(kPlThreads, TYPE == 2 ? 2 : 1)
+// (3: up to 30 rows, five or more splits; 7: up to 64 rows).  BF16: bfloat16 operands.
+template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, bool BF16 = false>
+__global__ void __launch_bounds__(kPlThreads, 1)
 k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneMaps maps) {
     constexpr bool kLean = EPI >= 0;
     static_assert(BN == 64 || BN == 128, "tile widths: 64 or 128 columns");
     constexpr int CPT = BN / 2;  // accumulator columns per accumulating thread: a warp reads one half of its 32 lanes' columns
     extern __shared__ uint8_t smem_raw[];
-    constexpr int kBars = TYPE == 2 ? kPlHalfSlots : kPlMaxStages;
-    __shared__ uint64_t bar_full[kBars], bar_empty[kBars], bar_acc_ready[kPlTmemSlots], bar_acc_free[kPlTmemSlots];
+    __shared__ uint64_t bar_full[kPlMaxStages], bar_empty[kPlMaxStages], bar_acc_ready[kPlTmemSlots], bar_acc_free[kPlTmemSlots];
     __shared__ uint64_t bar_reduce;
     __shared__ uint32_t tmem_slot;
     __shared__ __align__(16) float s_rowsum[2][kBM];
     __shared__ __align__(16) float s_colsum[2][BN];  // read in 16-byte pieces
     __shared__ unsigned long long s_cutoff[SIDE == SIDE_NORMS ? kBM : 1];  // the tile's queries' top-k cut-offs (TopkFilterArgs)
     __shared__ float s_cut_score[SIDE == SIDE_NORMS ? kBM : 1];            // their scores: a score below it cannot pass
-    constexpr bool ROWSUM = SIDE != SIDE_NONE && TYPE != 2;  // with float16 planes the norms come with the operands
+    constexpr bool ROWSUM = SIDE != SIDE_NONE;
 
     const int which = (int)blockIdx.x >= gp.tiles_m0 ? 1 : 0;
     const PlaneProblem& pp = gp.p[which];
@@ -460,7 +442,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr uint32_t kATile = kBM * 128, kBTile = BN * 128;
     const int k_begin = blockIdx.z * g.k_per_split, k_end = min(g.K, k_begin + g.k_per_split);
-    const int bf16 = kLean ? TYPE : gp.bf16, slice_k = bf16 ? 64 : kBK;
+    const int bf16 = kLean ? (BF16 ? 1 : 0) : gp.bf16, slice_k = bf16 ? 64 : kBK;
     const int n_slices = max(0, (k_end - k_begin + slice_k - 1) / slice_k);
     const bool a_two = pp.A.lo != nullptr, b_two = pp.B.lo != nullptr;
     // a ring stage: A hi [| A lo] | B hi [| B lo]
@@ -468,7 +450,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     const int n_stages = gp.n_stages[which];
 
     if (tid == 0) {
-        for (int s = 0; s < kBars; ++s) {
+        for (int s = 0; s < kPlMaxStages; ++s) {
             mbar_init(&bar_full[s], 1);
             mbar_init(&bar_empty[s], ROWSUM ? 1 + kPlAccWarps : 1);
         }
@@ -484,7 +466,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
         if (a_two) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.a_lo[which])) : "memory");
         if (b_two) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.b_lo[which])) : "memory");
     }
-    constexpr int n_slots = TYPE == 2 ? kPlHalfTmemSlots : kPlTmemSlots;
+    constexpr int n_slots = kPlTmemSlots;
     if (warp == 0) tmem_alloc(&tmem_slot, (uint32_t)(n_slots * BN));
     tc_fence_before();
     __syncthreads();
@@ -520,80 +502,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     for (int j = 0; j < CPT; ++j) acc[j] = 0.f;
     float row_part = 0.f, col_part = 0.f;
 
-    // TYPE 2: a slice's planes B lo, A hi[, A lo], B hi, each in the next slot of the ring and given back after its last product
-    const int n_planes = a_two ? 4 : 3;
-    if (TYPE == 2 && warp == 0) {
-        for (int i = 0, kc = 0; kc < n_slices; ++kc) {
-            const int k0 = k_begin + kc * slice_k;
-            for (int j = 0; j < n_planes; ++j, ++i) {
-                const int s = i % kPlHalfSlots, use = i / kPlHalfSlots;
-                if (use >= 1) mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), g.status, 6u);
-                if (lane == 0) {
-                    uint8_t* slot = smem + (size_t)s * kATile;
-                    mbar_arrive_expect(&bar_full[s], kATile);
-                    if (j == 0 || j == n_planes - 1)
-                        tma_plane_tile<BN>(slot, j == 0 ? &maps.b_lo[which] : &maps.b_hi[which], pp.B.mn_major, 1, n0, k0, &bar_full[s]);
-                    else
-                        tma_plane_tile<kBM>(slot, j == 1 ? &maps.a_hi[which] : &maps.a_lo[which], pp.A.mn_major, 1, m0, k0, &bar_full[s]);
-                }
-                __syncwarp();
-            }
-        }
-    } else if (TYPE == 2 && warp == 1) {
-        const uint32_t idesc = make_idesc_f16(kBM, BN) | (pp.A.mn_major ? (1u << 15) : 0u) | (pp.B.mn_major ? (1u << 16) : 0u);
-        const uint64_t sa = pp.A.mn_major ? (2048 >> 4) : (32 >> 4), sb = pp.B.mn_major ? (2048 >> 4) : (32 >> 4);
-        for (int i0 = 0, kc = 0; kc < n_slices; ++kc, i0 += n_planes) {
-            const int t = kc % n_slots;
-            if (kc >= n_slots) mbar_wait(&bar_acc_free[t], (uint32_t)(((kc / n_slots) - 1) & 1), g.status, 4u);
-            const uint32_t tmem_acc = tmem_base + (uint32_t)(t * BN);
-            uint32_t accumulate = 0u;
-            auto arrived = [&](int j) {
-                const int i = i0 + j;
-                mbar_wait(&bar_full[i % kPlHalfSlots], (uint32_t)((i / kPlHalfSlots) & 1), g.status, 3u);
-            };
-            auto multiply = [&](int ja, int jb) {  // four 16-deep products of a 64-deep slice
-                const uint32_t a = smem_u32(smem + (size_t)((i0 + ja) % kPlHalfSlots) * kATile), b = smem_u32(smem + (size_t)((i0 + jb) % kPlHalfSlots) * kATile);
-                const uint64_t da = pp.A.mn_major ? make_mnmajor_sw128_desc16(a) : make_kmajor_sw128_desc(a);
-                const uint64_t db = pp.B.mn_major ? make_mnmajor_sw128_desc16(b) : make_kmajor_sw128_desc(b);
-#pragma unroll
-                for (int ks = 0; ks < 4; ++ks) {
-                    umma_bf16(tmem_acc, da + (uint64_t)ks * sa, db + (uint64_t)ks * sb, idesc, accumulate);
-                    accumulate = 1u;
-                }
-            };
-            auto give_back = [&](int j) { umma_commit(&bar_empty[(i0 + j) % kPlHalfSlots]); };
-            const int b_hi = n_planes - 1;
-            // small cross terms first, the large hi*hi term last
-            arrived(0);
-            arrived(1);
-            tc_fence_after();
-            if (lane == 0) {
-                multiply(1, 0);
-                give_back(0);
-            }
-            __syncwarp();
-            if (a_two) {
-                arrived(2);
-                arrived(b_hi);
-                tc_fence_after();
-                if (lane == 0) {
-                    multiply(2, b_hi);
-                    give_back(2);
-                }
-                __syncwarp();
-            } else {
-                arrived(b_hi);
-                tc_fence_after();
-            }
-            if (lane == 0) {
-                multiply(1, b_hi);
-                give_back(1);
-                give_back(b_hi);
-                umma_commit(&bar_acc_ready[t]);
-            }
-            __syncwarp();
-        }
-    } else if (warp == 0) {
+    if (warp == 0) {
         for (int kc = 0; kc < n_slices; ++kc) {
             const int s = kc % n_stages, use = kc / n_stages;
             if (use >= 1) mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), g.status, 6u);
@@ -673,19 +582,6 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
             mbar_wait(&bar_acc_ready[t], (uint32_t)((kc / n_slots) & 1), g.status, 1u);
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * BN + half * CPT);
-            if constexpr (TYPE == 2) {  // 16 columns at a time: registers for two blocks
-#pragma unroll
-                for (int c = 0; c < CPT / 16; ++c) {
-                    uint32_t r[16];
-                    tmem_ld16_issue(taddr + (uint32_t)(c * 16), r);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) acc[c * 16 + j] += __uint_as_float(r[j]);
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_acc_free[t]);
-            } else {
             uint32_t r[CPT / 32][32];
 #pragma unroll
             for (int c = 0; c < CPT / 32; ++c) tmem_ld32_issue(taddr + (uint32_t)(c * 32), r[c]);
@@ -697,28 +593,15 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
             for (int c = 0; c < CPT / 32; ++c)
 #pragma unroll
                 for (int j = 0; j < 32; ++j) acc[c * 32 + j] += __uint_as_float(r[c][j]);
-            }
-        }
-        if (TYPE == 2 && half == 0) {
-            // {squared norm, undo scale} of the tile's rows and columns
-            const HalfRows &ha = pp.half_a, &hb = pp.half_b;
-            const float2 of_a = ha.info && m0 + row < g.M ? ha.info[m0 + row] : make_float2(0.f, 1.f);
-            s_rowsum[0][row] = of_a.x;
-            s_rowsum[1][row] = of_a.y;
-            if (row < BN) {
-                const float2 of_b = hb.info && n0 + row < g.N ? hb.info[n0 + row] : make_float2(0.f, 1.f);
-                s_colsum[0][row] = of_b.x;
-                s_colsum[1][row] = of_b.y;
-            }
         }
         if (ROWSUM) s_rowsum[half][row] = row_part;
-        if (SIDE == SIDE_NORMS && TYPE != 2 && row < BN) s_colsum[half][row] = col_part;
+        if (SIDE == SIDE_NORMS && row < BN) s_colsum[half][row] = col_part;
     }
     __syncthreads();  // every slice has been read from TMEM (so the ring is idle); the row sums are in place
 
     // Routing (hidden rows to their lookups): the finished rows and the staged lookups live in the
     // idle ring, behind what the k-split exchange uses.
-    const bool routing = TYPE != 2 && (!kLean || EPI == EPI_ADD_TABLE_VALUE) && gp.route.perm != nullptr && gp.route.mode[which] != 0;
+    const bool routing = (!kLean || EPI == EPI_ADD_TABLE_VALUE) && gp.route.perm != nullptr && gp.route.mode[which] != 0;
     float* fin = reinterpret_cast<float*>(smem + 150 * 1024);                              // [<= 64 rows][BN], or [128][BN] at offset 0 without a k split
     uint32_t* s_look = reinterpret_cast<uint32_t*>(smem + 184 * 1024);                      // [kRouteMaxLookups]
     uint32_t* s_rel = s_look + kRouteMaxLookups;                                            // [kRouteMaxLookups]
@@ -758,21 +641,17 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
         const bool whole_tile = SIDE == SIDE_NORMS && !clustered && acc_warp;
         const bool filtering = whole_tile && pp.filter.cand != nullptr && m < g.M;
         if (whole_tile) {
-            const float an = TYPE == 2 ? s_rowsum[0][row] : s_rowsum[0][row] + s_rowsum[1][row];
-            const float undo_a = TYPE == 2 ? s_rowsum[1][row] : 1.f;
+            const float an = s_rowsum[0][row] + s_rowsum[1][row];
             const float cut = filtering ? s_cut_score[row] : __int_as_float(0x7f800000);
             const float sign = pp.filter.score_is_gamma_minus ? -1.f : 1.f, offset = pp.filter.score_is_gamma_minus ? pp.filter.gamma : 0.f;
 #pragma unroll
             for (int j0 = 0; j0 < CPT; j0 += 4) {
                 const int tc0 = (nc0 - n0) + j0;  // tile column of acc[j0]
                 const float4 c0 = *reinterpret_cast<const float4*>(&s_colsum[0][tc0]), c1 = *reinterpret_cast<const float4*>(&s_colsum[1][tc0]);
-                const float bn[4] = {TYPE == 2 ? c0.x : c0.x + c1.x, TYPE == 2 ? c0.y : c0.y + c1.y, TYPE == 2 ? c0.z : c0.z + c1.z,
-                                     TYPE == 2 ? c0.w : c0.w + c1.w};
-                const float undo_b[4] = {c1.x, c1.y, c1.z, c1.w};
+                const float bn[4] = {c0.x + c1.x, c0.y + c1.y, c0.z + c1.z, c0.w + c1.w};
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
-                    const float dot = TYPE == 2 ? acc[j0 + t] * undo_a * undo_b[t] : acc[j0 + t];
-                    const float both = an + bn[t], d2 = both - 2.f * dot;
+                    const float both = an + bn[t], d2 = both - 2.f * acc[j0 + t];
                     direct_bits[(j0 + t) >> 5] |= (uint32_t)(d2 < 0.2f * both) << ((j0 + t) & 31);
                     float dist;
                     asm("sqrt.approx.f32 %0, %1;" : "=f"(dist) : "f"(fmaxf(d2, 0.f)));
@@ -780,11 +659,6 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
                     pass_bits[(j0 + t) >> 5] |= (uint32_t)(fmaf(sign, dist, offset) >= cut) << ((j0 + t) & 31);
                 }
             }
-        }
-        if (TYPE == 2 && SIDE == SIDE_NONE && acc_warp) {
-            const float undo_a = s_rowsum[1][row];
-#pragma unroll
-            for (int j = 0; j < CPT; ++j) acc[j] = acc[j] * undo_a * s_colsum[1][nc0 - n0 + j];
         }
         if (acc_warp) {
             // 16-byte chunk c of tile row `row` lies at chunk c ^ (row & 7): the lanes of a warp hold
@@ -797,11 +671,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
                 *reinterpret_cast<float4*>(mine + (((c0 + (j >> 2)) ^ (row & 7)) << 2)) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
             if (ROWSUM && nc0 == n0) staging[(size_t)owner * slot_floats + off_rowsum + local] = s_rowsum[0][row] + s_rowsum[1][row];
             if (whole_tile && m < g.M) {
-                const uint8_t* const a_values = reinterpret_cast<const uint8_t*>(TYPE == 2 ? pp.half_a.values : pp.A.hi);
-                const uint8_t* const b_values = reinterpret_cast<const uint8_t*>(TYPE == 2 ? pp.half_b.values : pp.B.hi);
-                const size_t a_stride = (size_t)(TYPE == 2 ? pp.half_a.stride_bytes : pp.A.row_stride_bytes);
-                const size_t b_stride = (size_t)(TYPE == 2 ? pp.half_b.stride_bytes : pp.B.row_stride_bytes);
-                const float* a_row = reinterpret_cast<const float*>(a_values + (size_t)m * a_stride);
+                const float* a_row = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(pp.A.hi) + (size_t)m * pp.A.row_stride_bytes);
 #pragma unroll
                 for (int w = 0; w < CPT / 32; ++w) {
                     uint32_t todo = direct_bits[w] | (filtering ? pass_bits[w] : 0u);
@@ -811,7 +681,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
                         if (col >= g.N) continue;
                         float* cell = mine + (((tcol >> 2) ^ (row & 7)) << 2) + (tcol & 3);
                         if ((direct_bits[w] >> bit) & 1u) {
-                            const float d2 = l2_squared_direct(a_row, reinterpret_cast<const float*>(b_values + (size_t)col * b_stride), g.K);
+                            const float d2 = l2_squared_direct(a_row, reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(pp.B.hi) + (size_t)col * pp.B.row_stride_bytes), g.K);
                             *cell = sqrtf(d2);
                         }
                         if (filtering) {
@@ -950,6 +820,278 @@ static __global__ void __launch_bounds__(256) k_split_planes(const float* __rest
     }
 }
 
+// Ring of single planes of k_half_tiles ([128 rows] x [64 k] float16 each) and, behind it, the tile that is being finished.
+constexpr int kHalfSlots = 9;
+constexpr int kHalfPlane = 128 * 128;
+constexpr int kHalfAccWarps = 16;  // 32 columns of a row per thread
+constexpr int kHalfThreads = 32 * (2 + kHalfAccWarps);
+constexpr size_t half_smem_bytes() { return 1024 + (size_t)kHalfSlots * kHalfPlane + (size_t)kBM * 128 * 4; }
+
+__device__ __forceinline__ void accumulating_warps_sync() {
+    __syncwarp();
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kHalfAccWarps) : "memory");
+}
+
+// Whole tiles of 128 x 128 of one contraction on float16 planes (HalfRows), many per SM: ranking's hidden rows and scores.
+// A block works through every gridDim-th tile.  One warp fetches planes and one multiplies, as far ahead as the ring and
+// the four accumulators in TMEM reach (all of the next tile at d 256), while sixteen warps add up the slices' products and
+// finish the tile.  Bound by those warps (distances, staging, stores), not by the products (1.7 us of a tile of d 256).
+// 1250 x 18944 scores of d 256: 110 us with a block per tile, 82 with two such blocks per SM, 76 now.
+template <int EPI>
+__global__ void __launch_bounds__(kHalfThreads, 1)
+k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneMaps maps) {
+    static_assert(EPI == EPI_STORE || EPI == EPI_L2_DISTANCE || EPI == EPI_ADD_TABLE_VALUE, "ranking's epilogues");
+    constexpr int BN = 128, CPT = BN / 4, kQuads = BN / 4, kAccThreads = 32 * kHalfAccWarps;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t bar_full[kHalfSlots], bar_empty[kHalfSlots], bar_acc_ready[kPlTmemSlots], bar_acc_free[kPlTmemSlots];
+    __shared__ uint32_t tmem_slot;
+    __shared__ __align__(16) float s_col[2][BN];  // the columns' squared norms, and what undoes their scales
+    const PlaneProblem& pp = gp.p[0];
+    const GemmArgs& g = pp.g;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tiles_m = (g.M + kBM - 1) / kBM, n_tiles = tiles_m * ((g.N + BN - 1) / BN), n_slices = (g.K + 63) / 64;
+    const bool a_two = pp.A.lo != nullptr;
+    const int n_planes = a_two ? 4 : 3;  // of a slice, in this order: B lo, A hi[, A lo], B hi
+    uint8_t* const ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    float* const staging = reinterpret_cast<float*>(ring + (size_t)kHalfSlots * kHalfPlane);
+
+    if (tid == 0) {
+        for (int s = 0; s < kHalfSlots; ++s) {
+            mbar_init(&bar_full[s], 1);
+            mbar_init(&bar_empty[s], 1);
+        }
+        for (int t = 0; t < kPlTmemSlots; ++t) {
+            mbar_init(&bar_acc_ready[t], 1);
+            mbar_init(&bar_acc_free[t], kHalfAccWarps);
+        }
+        mbar_fence_init();
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.a_hi[0])) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.b_hi[0])) : "memory");
+        if (a_two) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.a_lo[0])) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps.b_lo[0])) : "memory");
+    }
+    if (warp == 0) tmem_alloc(&tmem_slot, (uint32_t)(kPlTmemSlots * BN));
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    grid_dependency_sync();
+    const uint32_t tmem_base = tmem_slot;
+
+    if (warp == 0) {
+        int i = 0;  // planes so far
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            const int m0 = tile % tiles_m * kBM, n0 = tile / tiles_m * BN;
+            for (int kc = 0; kc < n_slices; ++kc)
+                for (int j = 0; j < n_planes; ++j, ++i) {
+                    const int s = i % kHalfSlots, use = i / kHalfSlots;
+                    if (use >= 1) mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), g.status, 6u);
+                    if (lane == 0) {
+                        uint8_t* slot = ring + (size_t)s * kHalfPlane;
+                        mbar_arrive_expect(&bar_full[s], kHalfPlane);
+                        if (j == 0 || j == n_planes - 1)
+                            tma_plane_tile<BN>(slot, j == 0 ? &maps.b_lo[0] : &maps.b_hi[0], pp.B.mn_major, 1, n0, kc * 64, &bar_full[s]);
+                        else
+                            tma_plane_tile<kBM>(slot, j == 1 ? &maps.a_hi[0] : &maps.a_lo[0], pp.A.mn_major, 1, m0, kc * 64, &bar_full[s]);
+                    }
+                    __syncwarp();
+                }
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = make_idesc_f16(kBM, BN) | (pp.A.mn_major ? (1u << 15) : 0u) | (pp.B.mn_major ? (1u << 16) : 0u);
+        const uint64_t sa = pp.A.mn_major ? (2048 >> 4) : (32 >> 4), sb = pp.B.mn_major ? (2048 >> 4) : (32 >> 4);
+        int i0 = 0, c = 0;  // planes and slices so far
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x)
+            for (int kc = 0; kc < n_slices; ++kc, ++c, i0 += n_planes) {
+                const int t = c % kPlTmemSlots;
+                if (c >= kPlTmemSlots) mbar_wait(&bar_acc_free[t], (uint32_t)((c / kPlTmemSlots - 1) & 1), g.status, 4u);
+                const uint32_t tmem_acc = tmem_base + (uint32_t)(t * BN);
+                uint32_t accumulate = 0u;
+                auto arrived = [&](int j) { mbar_wait(&bar_full[(i0 + j) % kHalfSlots], (uint32_t)(((i0 + j) / kHalfSlots) & 1), g.status, 3u); };
+                auto multiply = [&](int ja, int jb) {  // four 16-deep products of a 64-deep slice
+                    const uint32_t a = smem_u32(ring + (size_t)((i0 + ja) % kHalfSlots) * kHalfPlane), b = smem_u32(ring + (size_t)((i0 + jb) % kHalfSlots) * kHalfPlane);
+                    const uint64_t da = pp.A.mn_major ? make_mnmajor_sw128_desc16(a) : make_kmajor_sw128_desc(a);
+                    const uint64_t db = pp.B.mn_major ? make_mnmajor_sw128_desc16(b) : make_kmajor_sw128_desc(b);
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks) {
+                        umma_bf16(tmem_acc, da + (uint64_t)ks * sa, db + (uint64_t)ks * sb, idesc, accumulate);
+                        accumulate = 1u;
+                    }
+                };
+                // a plane's slot is given back after its last product
+                auto give_back = [&](int j) { umma_commit(&bar_empty[(i0 + j) % kHalfSlots]); };
+                const int b_hi = n_planes - 1;
+                arrived(0);  // small cross terms first, the large hi * hi term last
+                arrived(1);
+                tc_fence_after();
+                if (lane == 0) {
+                    multiply(1, 0);
+                    give_back(0);
+                }
+                __syncwarp();
+                if (a_two) arrived(2);
+                arrived(b_hi);
+                tc_fence_after();
+                if (lane == 0) {
+                    if (a_two) {
+                        multiply(2, b_hi);
+                        give_back(2);
+                    }
+                    multiply(1, b_hi);
+                    give_back(1);
+                    give_back(b_hi);
+                    umma_commit(&bar_acc_ready[t]);
+                }
+                __syncwarp();
+            }
+    } else {
+        // a thread holds a quarter of the columns of one row
+        const int quarter = warp & 3, part = (warp - 2) >> 2, row = quarter * 32 + lane, at = tid - 64;
+        const bool filter = EPI == EPI_L2_DISTANCE && pp.filter.cand != nullptr;
+        // what belongs to a tile's rows and columns is loaded one tile ahead
+        struct {
+            float2 a, b;
+            unsigned long long key;
+            int count;
+        } next = {};
+        auto look_up = [&](int tile) {
+            if (tile >= n_tiles) return;
+            const int m = tile % tiles_m * kBM + row, n = tile / tiles_m * BN + at;
+            next.a = pp.half_a.info && m < g.M ? pp.half_a.info[m] : make_float2(0.f, 1.f);
+            if (at < BN) next.b = pp.half_b.info && n < g.N ? pp.half_b.info[n] : make_float2(0.f, 1.f);
+            if (filter && m < g.M) {
+                next.count = pp.filter.counts[m];
+                next.key = pp.filter.state[(size_t)m * kTopkCapacity + pp.filter.n_best - 1];
+            }
+        };
+        look_up(blockIdx.x);
+        const bool aligned = (g.N & 3) == 0 && (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(g.out) & 15) == 0;
+        int c = 0;
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            const int m0 = tile % tiles_m * kBM, n0 = tile / tiles_m * BN, m = m0 + row;
+            const float2 of_a = next.a;
+            if (at < BN) {
+                s_col[0][at] = next.b.x;
+                s_col[1][at] = next.b.y;
+            }
+            if (EPI == EPI_ADD_TABLE_VALUE && at < kBM && m0 + at < g.M) {
+                // the table values that the finishing loop adds are asked into L2 while the products run
+                const int elem = g.x_is_half ? 2 : 4;
+                const size_t xr = g.x_gather ? g.x_gather[m0 + at] : (size_t)g.x_row_base + (size_t)(m0 + at);
+                const uint8_t* x = g.x_base + xr * (size_t)g.x_row_stride_bytes + (size_t)n0 * elem;
+                const int bytes = min(BN, g.N - n0) * elem;
+                for (int o = 0; o < bytes; o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(x + o));
+            }
+            unsigned long long cutoff = ~0ull;
+            float cut = __int_as_float(0x7f800000);  // the score of the query's cut-off key; none: nothing passes
+            if (filter && m < g.M) {
+                cutoff = next.count >= pp.filter.n_best ? next.key : 0ull;
+                // no cut-off yet: every score is a candidate and the query scans its row of scores itself
+                if (cutoff != 0ull) cut = topk_score(cutoff);
+                else if (n0 == 0 && part == 0) pp.filter.cand_count[m] = kTopkCandidates + 1;
+            }
+            look_up(tile + (int)gridDim.x);
+            float acc[CPT];
+#pragma unroll
+            for (int j = 0; j < CPT; ++j) acc[j] = 0.f;
+            for (int kc = 0; kc < n_slices; ++kc, ++c) {
+                const int t = c % kPlTmemSlots;
+                mbar_wait(&bar_acc_ready[t], (uint32_t)((c / kPlTmemSlots) & 1), g.status, 1u);
+                __syncwarp();
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(t * BN + part * CPT);
+                uint32_t r[32];
+                tmem_ld32_issue(taddr, r);
+                tmem_ld_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_acc_free[t]);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) acc[j] += __uint_as_float(r[j]);
+            }
+            accumulating_warps_sync();  // s_col is complete; the rows of the tile before have left the staging
+            uint32_t direct_bits = 0, pass_bits = 0;  // the rare cases: recomputed distances, scores that reach the cut-off
+            if (EPI == EPI_L2_DISTANCE) {
+                // The square root is the approximate one (relative error 2^-23, exact at zero): the form's own error is larger.
+                const float sign = pp.filter.score_is_gamma_minus ? -1.f : 1.f, offset = pp.filter.score_is_gamma_minus ? pp.filter.gamma : 0.f;
+#pragma unroll
+                for (int j0 = 0; j0 < CPT; j0 += 4) {
+                    const float4 norms = *reinterpret_cast<const float4*>(&s_col[0][part * CPT + j0]), undo = *reinterpret_cast<const float4*>(&s_col[1][part * CPT + j0]);
+                    const float bn[4] = {norms.x, norms.y, norms.z, norms.w}, undo_b[4] = {undo.x, undo.y, undo.z, undo.w};
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        const float both = of_a.x + bn[t], d2 = both - 2.f * (acc[j0 + t] * of_a.y * undo_b[t]);
+                        direct_bits |= (uint32_t)(d2 < 0.2f * both) << (j0 + t);
+                        float dist;
+                        asm("sqrt.approx.f32 %0, %1;" : "=f"(dist) : "f"(fmaxf(d2, 0.f)));
+                        acc[j0 + t] = dist;
+                        pass_bits |= (uint32_t)(fmaf(sign, dist, offset) >= cut) << (j0 + t);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < CPT; ++j) acc[j] = acc[j] * of_a.y * s_col[1][part * CPT + j];
+            }
+            // 16-byte chunk c of tile row `row` lies at chunk c ^ (row & 7): the lanes of a warp hold
+            // 32 different rows, and this spreads their stores over all banks
+            float* const mine = staging + (size_t)row * BN;
+#pragma unroll
+            for (int j = 0; j < CPT; j += 4)
+                *reinterpret_cast<float4*>(mine + (((part * (CPT / 4) + (j >> 2)) ^ (row & 7)) << 2)) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+            if (EPI == EPI_L2_DISTANCE && m < g.M) {
+                const float* a_row = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(pp.half_a.values) + (size_t)m * pp.half_a.stride_bytes);
+                uint32_t todo = direct_bits | (filter ? pass_bits : 0u);
+                while (todo) {
+                    const int bit = __ffs(todo) - 1, tcol = part * CPT + bit, col = n0 + tcol;
+                    todo &= todo - 1;
+                    if (col >= g.N) continue;
+                    float* cell = mine + (((tcol >> 2) ^ (row & 7)) << 2) + (tcol & 3);
+                    if ((direct_bits >> bit) & 1u)
+                        *cell = sqrtf(l2_squared_direct(a_row, reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(pp.half_b.values) + (size_t)col * pp.half_b.stride_bytes), g.K));
+                    if (filter) {
+                        const TopkFilterArgs& f = pp.filter;
+                        const float score = f.score_is_gamma_minus ? f.gamma - *cell : *cell;
+                        const uint32_t table_row = f.first_row + (uint32_t)col;
+                        // without a cut-off the query scans for itself (its count is past the capacity already)
+                        if (cutoff == 0ull || table_row > f.last_valid_row) continue;
+                        const unsigned long long key = topk_key(score, table_row);
+                        if (key > cutoff) {  // ties with the cut-off are decided by the keys
+                            const int slot = atomicAdd(f.cand_count + m, 1);
+                            if (slot < kTopkCandidates) f.cand[(size_t)m * kTopkCandidates + slot] = key;
+                        }
+                    }
+                }
+            }
+            accumulating_warps_sync();
+            constexpr int kBatch = 8;  // whole rows go out in 16-byte pieces, eight at a time
+#pragma unroll 1
+            for (int u0 = at; u0 < kBM * kQuads; u0 += kBatch * kAccThreads) {
+                float x[kBatch][4];
+                if (EPI == EPI_ADD_TABLE_VALUE) {
+#pragma unroll
+                    for (int i = 0; i < kBatch; ++i) {
+                        const int u = u0 + i * kAccThreads, mm = m0 + u / kQuads, nn = n0 + u % kQuads * 4;
+                        x[i][0] = x[i][1] = x[i][2] = x[i][3] = 0.f;
+                        if (mm < g.M && nn < g.N) load_x_four(g, mm, nn, x[i], EPI);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < kBatch; ++i) {
+                    const int u = u0 + i * kAccThreads, local = u / kQuads, q = u % kQuads, mm = m0 + local, nn = n0 + q * 4;
+                    const float4 v = *reinterpret_cast<const float4*>(staging + (size_t)local * BN + ((q ^ (local & 7)) << 2));
+                    float four[4] = {v.x, v.y, v.z, v.w};
+                    if (mm >= g.M || nn >= g.N) continue;
+                    if (EPI == EPI_ADD_TABLE_VALUE) finish_four(g, g.out, mm, nn, four, x[i], 0.f, EPI);
+                    else if (aligned) *reinterpret_cast<float4*>(g.out + (size_t)mm * g.ldc + nn) = v;
+                    else store_four(g, mm, nn, four);
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem_base, (uint32_t)(kPlTmemSlots * BN));
+}
+
 // The float16 planes of an operand (HalfRows).  The scale 2^(s - 127) for values up to `largest`, as a biased exponent:
 // the largest lands in [2^13, 2^14); no scaling of a row that holds infinities or NaNs.
 __device__ __forceinline__ uint32_t half_scale_exponent(float largest) {
@@ -1044,8 +1186,8 @@ inline cudaError_t make_plane_map(const float* base, const PlaneOperand& op, int
     const cuuint32_t inner = bf16 ? 64u : 32u;
     const cuuint32_t box[2] = {inner, (cuuint32_t)(op.mn_major ? inner : rows)};
     const cuuint32_t elem[2] = {1, 1};
-    const CUresult r = encode(map, op.elem_bytes == 16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims,
-                              strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const CUresult r = encode(map, op.elem_bytes == 16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2,
+                              const_cast<float*>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                               op.mn_major && !bf16 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
@@ -1055,14 +1197,12 @@ inline bool planes_aligned(const PlaneOperand& op) {
     return reinterpret_cast<uintptr_t>(op.hi) % 16 == 0 && reinterpret_cast<uintptr_t>(op.lo) % 16 == 0 && op.row_stride_bytes % 16 == 0;
 }
 
-template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, int TYPE = 0>
+template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, bool BF16 = false>
 inline cudaError_t configure_planes() {
     static bool configured[kMaxDeviceOrdinals] = {};
     const int slot = current_device_slot();
     if (slot >= 0 && configured[slot]) return cudaSuccess;
-    cudaError_t err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem_bytes(TYPE));
-    if (err == cudaSuccess && TYPE == 2)  // room for two blocks
-        err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, TYPE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    cudaError_t err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem_bytes());
     if (err == cudaSuccess && slot >= 0) configured[slot] = true;
     return err;
 }
@@ -1135,9 +1275,8 @@ inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, 
     for (int i = 0; i < 2; ++i) {
         PlaneProblem& q = gp.p[i];
         if (type_of(q.A) != gp.bf16 || type_of(q.B) != gp.bf16) return cudaErrorInvalidValue;
-        if (gp.bf16 == 1 && (q.A.lo || q.B.lo)) return cudaErrorInvalidValue;
-        if (gp.bf16 == 2 && !q.B.lo) return cudaErrorInvalidValue;  // B always has two planes
-        if (gp.bf16 && q.g.k_per_split % 64) return cudaErrorInvalidValue;
+        if (gp.bf16 == 1 && (q.A.lo || q.B.lo || q.g.k_per_split % 64)) return cudaErrorInvalidValue;
+        if (gp.bf16 == 2 && (!q.B.lo || n_problems != 1 || splits != 1 || tile_n != 128)) return cudaErrorInvalidValue;
         q.g.ws = nullptr;
         q.g.cluster_splits = splits > 1 ? splits : 0;
         if (!planes_aligned(q.A) || !planes_aligned(q.B)) return cudaErrorInvalidValue;
@@ -1155,11 +1294,11 @@ inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, 
     return cudaSuccess;
 }
 
-template <int SIDE, int EPI, int SPLIT, int TYPE = 0>
+template <int SIDE, int EPI, int SPLIT, bool BF16 = false>
 inline cudaError_t launch_lean(const PlaneLaunch& l, cudaStream_t stream) {
-    cudaError_t err = configure_planes<128, SIDE, EPI, SPLIT, TYPE>();
+    cudaError_t err = configure_planes<128, SIDE, EPI, SPLIT, BF16>();
     if (err != cudaSuccess) return err;
-    return launch_dependent_cluster(k_tc_planes<128, SIDE, EPI, SPLIT, TYPE>, l.grid, dim3(kPlThreads), plane_smem_bytes(TYPE), stream, (unsigned)l.splits,
+    return launch_dependent_cluster(k_tc_planes<128, SIDE, EPI, SPLIT, BF16>, l.grid, dim3(kPlThreads), plane_smem_bytes(), stream, (unsigned)l.splits,
                                     l.gp, l.maps);
 }
 // By the number of k splits: five or more leave at most 26 rows of a tile to a block.
@@ -1170,21 +1309,29 @@ inline cudaError_t launch_lean_split(const PlaneLaunch& l, cudaStream_t stream) 
     return launch_lean<SIDE, EPI, 0>(l, stream);
 }
 
+template <int EPI>
+inline cudaError_t launch_half(const PlaneLaunch& l, cudaStream_t stream) {
+    static bool configured[kMaxDeviceOrdinals] = {};
+    const int slot = current_device_slot();
+    if (slot < 0 || !configured[slot]) {
+        const cudaError_t err = cudaFuncSetAttribute(k_half_tiles<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)half_smem_bytes());
+        if (err != cudaSuccess) return err;
+        if (slot >= 0) configured[slot] = true;
+    }
+    return launch_dependent(k_half_tiles<EPI>, dim3(std::min(148u, l.grid.x * l.grid.y)), dim3(kHalfThreads), half_smem_bytes(), stream, l.gp, l.maps);
+}
+
 template <int SIDE>
 inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
     if (SIDE != SIDE_NONE && l.gp.bf16 == 1) return cudaErrorInvalidValue;  // the side sums read fp32 tiles
     if (SIDE == SIDE_NORMS)
         for (int i = 0; i < 2; ++i)
             if (l.gp.p[i].A.mn_major || l.gp.p[i].B.mn_major || l.gp.p[i].g.out_blocks) return cudaErrorInvalidValue;
-    if (l.gp.bf16 == 2) {  // whole tiles of one problem only (ranking)
+    if (l.gp.bf16 == 2) {
         const int epilogue = l.gp.p[0].g.epilogue;
-        if (l.tile_n != 128 || l.splits != 1) return cudaErrorInvalidValue;
-        if constexpr (SIDE == SIDE_NONE) {
-            if (epilogue == EPI_ADD_TABLE_VALUE) return launch_lean<SIDE_NONE, EPI_ADD_TABLE_VALUE, 0, 2>(l, stream);
-            if (epilogue == EPI_STORE) return launch_lean<SIDE_NONE, EPI_STORE, 0, 2>(l, stream);
-        } else if constexpr (SIDE == SIDE_NORMS) {
-            if (epilogue == EPI_L2_DISTANCE) return launch_lean<SIDE_NORMS, EPI_L2_DISTANCE, 0, 2>(l, stream);
-        }
+        if (SIDE == SIDE_NONE && epilogue == EPI_ADD_TABLE_VALUE) return launch_half<EPI_ADD_TABLE_VALUE>(l, stream);
+        if (SIDE == SIDE_NONE && epilogue == EPI_STORE) return launch_half<EPI_STORE>(l, stream);
+        if (SIDE == SIDE_NORMS && epilogue == EPI_L2_DISTANCE) return launch_half<EPI_L2_DISTANCE>(l, stream);
         return cudaErrorInvalidValue;
     }
     if (l.tile_n == 128) {
@@ -1193,7 +1340,7 @@ inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
         if (l.gp.p[1].g.epilogue == epilogue) {
             if constexpr (SIDE == SIDE_NONE) {
                 if (l.gp.bf16) {
-                    if (epilogue == EPI_STORE) return l.splits > 1 ? launch_lean<SIDE_NONE, EPI_STORE, 7, 1>(l, stream) : launch_lean<SIDE_NONE, EPI_STORE, 0, 1>(l, stream);
+                    if (epilogue == EPI_STORE) return l.splits > 1 ? launch_lean<SIDE_NONE, EPI_STORE, 7, true>(l, stream) : launch_lean<SIDE_NONE, EPI_STORE, 0, true>(l, stream);
                 } else {
                     if (epilogue == EPI_ADD_TABLE_VALUE) return launch_lean_split<SIDE_NONE, EPI_ADD_TABLE_VALUE>(l, stream);
                     if (epilogue == EPI_DENSE_ADAM) return launch_lean_split<SIDE_NONE, EPI_DENSE_ADAM>(l, stream);
