@@ -152,6 +152,15 @@ __device__ __forceinline__ uint64_t make_mnmajor_sw128_desc(uint32_t smem_addr) 
     return d;
 }
 
+// One lane of a converged warp, always the same.  Where a single lane issues TMA copies and MMAs the branch must be this
+// one: of `lane == 0` the compiler does not know that it leaves one lane, and it wraps each of these instructions, which
+// take their operands from the warp's uniform registers, in a loop over the active lanes.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}" : "=r"(one));
+    return one != 0;
+}
+
 // MN-major tile of 16-bit elements under the ordinary 128-byte swizzle: atoms of 8 k-rows x 128 B
 // (64 elements along mn); a box holds 64 k-rows (8 KB), the next 64 mn are 8192 B further, the
 // next 8 k 1024 B further.
@@ -506,7 +515,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
         for (int kc = 0; kc < n_slices; ++kc) {
             const int s = kc % n_stages, use = kc / n_stages;
             if (use >= 1) mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), g.status, 6u);
-            if (lane == 0) {
+            if (elect_one()) {
                 uint8_t* stage = smem + (size_t)s * stage_bytes;
                 const int k0 = k_begin + kc * slice_k;
                 mbar_arrive_expect(&bar_full[s], stage_bytes);
@@ -525,7 +534,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
             mbar_wait(&bar_full[s], (uint32_t)((kc / n_stages) & 1), g.status, 3u);
             if (kc >= n_slots) mbar_wait(&bar_acc_free[t], (uint32_t)(((kc / n_slots) - 1) & 1), g.status, 4u);
             tc_fence_after();
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t a_hi = smem_u32(smem + (size_t)s * stage_bytes), a_lo = a_hi + kATile, b_hi = a_hi + off_b, b_lo = b_hi + kBTile;
                 const uint32_t tmem_acc = tmem_base + (uint32_t)(t * BN);
                 const uint64_t da_hi = pp.A.mn_major ? make_mnmajor_sw128_desc(a_hi) : make_kmajor_sw128_desc(a_hi);
@@ -836,7 +845,8 @@ __device__ __forceinline__ void accumulating_warps_sync() {
 // A block works through every gridDim-th tile.  One warp fetches planes and one multiplies, as far ahead as the ring and
 // the four accumulators in TMEM reach (all of the next tile at d 256), while sixteen warps add up the slices' products and
 // finish the tile.  Bound by those warps (distances, staging, stores), not by the products (1.7 us of a tile of d 256).
-// 1250 x 18944 scores of d 256: 110 us with a block per tile, 82 with two such blocks per SM, 76 now.
+// 1250 x 18944 scores of d 256: 110 us with a block per tile, 82 with two such blocks per SM, 68 now; 18944 x 256 hidden
+// rows of f 768: 46, 31, 34.  (TMA copies and MMAs issued by an elected lane: see elect_one.)
 template <int EPI>
 __global__ void __launch_bounds__(kHalfThreads, 1)
 k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneMaps maps) {
@@ -885,7 +895,7 @@ k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ Plane
                 for (int j = 0; j < n_planes; ++j, ++i) {
                     const int s = i % kHalfSlots, use = i / kHalfSlots;
                     if (use >= 1) mbar_wait(&bar_empty[s], (uint32_t)((use - 1) & 1), g.status, 6u);
-                    if (lane == 0) {
+                    if (elect_one()) {
                         uint8_t* slot = ring + (size_t)s * kHalfPlane;
                         mbar_arrive_expect(&bar_full[s], kHalfPlane);
                         if (j == 0 || j == n_planes - 1)
@@ -923,7 +933,7 @@ k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ Plane
                 arrived(0);  // small cross terms first, the large hi * hi term last
                 arrived(1);
                 tc_fence_after();
-                if (lane == 0) {
+                if (elect_one()) {
                     multiply(1, 0);
                     give_back(0);
                 }
@@ -931,7 +941,7 @@ k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ Plane
                 if (a_two) arrived(2);
                 arrived(b_hi);
                 tc_fence_after();
-                if (lane == 0) {
+                if (elect_one()) {
                     if (a_two) {
                         multiply(2, b_hi);
                         give_back(2);
