@@ -2347,8 +2347,18 @@ void Engine::launch_topk(ShardBuffers& b, unsigned c, uint32_t start, uint32_t l
         const dim3 fgrid(std::max(1u, std::min(ceil_div(c, 4 * 256), 8u)), Q);
         KGE_LAUNCH("predict_topk", k_topk_filter<<<fgrid, 256, 0, stream_>>>(p_raw_, (int)c, start, last, b.topk_state, b.topk_count, p_cand_, p_cand_count_, tp));
     }
-    KGE_LAUNCH("predict_topk", k_topk_update<<<ceil_div(Q, 4), 128, 0, stream_>>>(p_raw_, (int)c, start, last, b.topk_state, b.topk_count, tp, p_cand_,
-                                                                                 p_cand_count_));
+    // On the tensor cores the merge (13 us for 1250 queries) runs beside the next pass's hidden rows, which it has nothing
+    // to do with; the next scores wait for it (join_topk).
+    const cudaStream_t st = predict_planes_ ? side_begin() : stream_;
+    KGE_LAUNCH("predict_topk", k_topk_update<<<ceil_div(Q, 4), 128, 0, st>>>(p_raw_, (int)c, start, last, b.topk_state, b.topk_count, tp, p_cand_,
+                                                                            p_cand_count_));
+    if (predict_planes_) side_end(0);
+    topk_beside_ = predict_planes_;
+}
+
+void Engine::join_topk() {
+    if (topk_beside_) side_join(0);
+    topk_beside_ = false;
 }
 
 // Ranks every real row of the local shards as a tail for the queries of all shards
@@ -2456,6 +2466,7 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
             KGE_LAUNCH("predict_score", KGE_CUDA(launch_score(cfg_.dist_fn, queries, p_chunk_hidden_, p_raw_, (int)Q, (int)c, (int)D, stream_)));
             launch_topk(b, c, start, last, tp, false);
         }
+        join_topk();
         KGE_LAUNCH("predict_finish", k_topk_finish<<<(unsigned)Q, 128, 0, stream_>>>(
                                          b.topk_state, b.topk_count, (int)Q, (int)hr, (int)nb, b.predict_score_dst,
                                          b.predict_index_dst));
@@ -2549,6 +2560,7 @@ bool Engine::predict_pass_planes(ShardBuffers& b, uint32_t start, unsigned c, ui
     s.g.out = p_raw_; s.g.ldc = c; s.g.block_rows = 1;
     const bool filtered = l2 && filter_in_scores_;
     if (filtered) s.filter = tc::TopkFilterArgs{b.topk_state, b.topk_count, p_cand_, p_cand_count_, start, last, tp.n_best, tp.score_is_gamma_minus, tp.gamma};
+    join_topk();
     launch_planes("predict_score", &s, 1, l2 ? tc::SIDE_NORMS : tc::SIDE_NONE, -1, -1);
     KGE_CUDA(cudaGetLastError());
     return filtered;

@@ -293,6 +293,7 @@ class Engine {
     unsigned long long* p_cand_ = nullptr;  // [Q, kTopkCandidates] a batch's keys above each query's cut-off
     int* p_cand_count_ = nullptr;
     void launch_topk(ShardBuffers& b, unsigned c, uint32_t start, uint32_t last, const TopkParams& tp, bool filtered);
+    void join_topk();
     float *p_mlp_cat_ = nullptr, *p_mlp_pre_ = nullptr, *p_mlp_out_ = nullptr;  // predict's MLP buffers
     bool filter_in_scores_ = true;  // predict's L2 score contraction also filters the scores against the queries' cut-offs (KGE_PREDICT_FILTER_IN_SCORES=0: k_topk_filter)
     bool heavy_route_ = false;  // rows with many lookups are routed in parts by k_route_heavy (KGE_ROUTE_POPULAR_ROWS=0: by the hidden kernel's epilogue)
@@ -328,6 +329,7 @@ class Engine {
     __half *p_half_q_ = nullptr, *p_half_t_ = nullptr, *p_half_w_ = nullptr;
     float2 *p_half_q_info_ = nullptr, *p_half_t_info_ = nullptr, *p_half_w_info_ = nullptr;
     int p_half_stride_ = 0;
+    bool topk_beside_ = false;  // a pass's merge is on the side stream
     float *p_feat_ = nullptr, *p_chunk_lo_ = nullptr, *p_query_lo_ = nullptr;  // planes of a pass: widened / lower features, lower hidden rows, lower queries
 
     uint32_t* d_rw_idx_ = nullptr;
