@@ -809,10 +809,10 @@ def run_predict(args) -> None:
             "e2e": {"value": queries_per_gpu * world / per_step, "unit": "queries/s", "h2d_bytes_per_step": int(2 * 4 * queries_per_gpu),
                     "d2h_bytes_per_step": int(2 * scores.nbytes * (queries_per_gpu // hr))},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "tensor", "kernel": "k_tc_planes (hidden rows and L2 scores of a pass)", "achieved": flop / per_step / world / 1e12,
+            "roofline": {"bound": "tensor", "kernel": "k_half_tiles (hidden rows and L2 scores of a pass)", "achieved": flop / per_step / world / 1e12,
                          "peak": peaks["tensor_tflops"], "unit": "TFLOP/s", "frac": flop / per_step / world / 1e12 / peaks["tensor_tflops"],
                          "peak_source": peaks["source"], "traffic": None,
-                         "algorithmic_flops_per_step": flop, "peak_note": "dense bf16 sustained; fp32 products run as three TF32 products"},
+                         "algorithmic_flops_per_step": flop, "peak_note": "dense bf16 sustained; fp32 products run as three float16 products, fp16 features as two"},
             "clocks": clocks, "best_score_of_first_query": float(best[0, 0]),
         }), flush=True)
     if world > 1:
