@@ -5,8 +5,8 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <exception>
 #include <mutex>
+#include <optional>
 
 namespace kge {
 
@@ -903,6 +903,7 @@ void Engine::train_staged(float learning_rate, float* loss) {
         KGE_CUDA(cudaMemcpyAsync(d_run_ + keys_at_, pinned_ + keys_at_, (status_at_ - keys_at_) * 4, cudaMemcpyHostToDevice, stream_));
     }
     run_words_uploaded_ = false;
+    std::optional<ShardStreams> streams;
     KGE_CUDA(cudaEventRecord(ev_begin_, stream_));
     if (cfg_.cuda_graph && !kernel_timing_) {
         launch_step_graphs();
@@ -913,6 +914,7 @@ void Engine::train_staged(float learning_rate, float* loss) {
             k_delay<<<1, 1, 0, stream_>>>(20ll * 1000 * 1000);
             KGE_CUDA(cudaGetLastError());
         }
+        streams.emplace(*this);
         launch_steps(0, cfg_.n_step);
         last_launches_ = launch_counter_;
     }
@@ -920,6 +922,7 @@ void Engine::train_staged(float learning_rate, float* loss) {
     // the loss totals and the status words are neighbours: one transfer brings both
     KGE_CUDA(cudaMemcpyAsync(pinned_ + loss_at_, d_run_ + loss_at_, (run_words_ - loss_at_) * 4, cudaMemcpyDeviceToHost, stream_));
     KGE_CUDA(cudaStreamSynchronize(stream_));
+    if (streams) streams->give_back();
     uploads_pending_ = false;
     ms_pending_ = true;
     // the sort-and-segment preparation belongs to the step (it is the backward of the row
@@ -1006,46 +1009,8 @@ bool dependent_launch_enabled() {
     return enabled;
 }
 
-// A program run as a short chain of CUDA graphs, each four times as long as the one before: on an engine's first run
-// every graph but the first (a single step) is captured and instantiated, at 10 to 20 us of host time per kernel, while
-// its predecessor runs on the GPU (the first run of 100 headline steps: 17.1 to 15.9 ms; later runs are the same).
-void Engine::launch_step_graphs() {
-    if (graphs_.empty()) {
-        unsigned length = 1;
-        for (unsigned first = 0; first < cfg_.n_step; first += length, length *= 4)
-            graphs_.push_back({first, std::min(first + length, cfg_.n_step), nullptr, 0});
-        // a last graph shorter than its predecessor's launch joins it
-        if (graphs_.size() > 1 && graphs_.back().end - graphs_.back().first < (graphs_.back().first - graphs_[graphs_.size() - 2].first) / 2) {
-            graphs_[graphs_.size() - 2].end = cfg_.n_step;
-            graphs_.pop_back();
-        }
-    }
-    last_launches_ = 0;
-    for (StepGraph& g : graphs_) {
-        if (!g.exec) {
-            cudaGraph_t graph = nullptr;
-            launch_counter_ = 0;
-            KGE_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-            try {
-                launch_steps(g.first, g.end);
-            } catch (...) {
-                cudaStreamEndCapture(stream_, &graph);
-                if (graph) cudaGraphDestroy(graph);
-                throw;
-            }
-            KGE_CUDA(cudaStreamEndCapture(stream_, &graph));
-            cudaError_t err = cudaGraphInstantiate(&g.exec, graph, 0);
-            cudaGraphDestroy(graph);
-            KGE_CUDA(err);
-            g.launches = launch_counter_;
-        }
-        KGE_CUDA(cudaGraphLaunch(g.exec, stream_));
-        last_launches_ += g.launches;
-    }
-}
-
 namespace {
-// Streams for the shards' branches, lent out while steps are queued or captured: making one costs the host about 2 ms,
+// Streams for the shards' branches, lent out while steps are queued or captured (Engine::ShardStreams): making one costs the host about 2 ms,
 // as much as capturing a short run.  At most kKept per device wait for the next borrower; the rest are destroyed.
 class StreamPool {
    public:
@@ -1086,23 +1051,66 @@ class StreamPool {
 };
 }  // namespace
 
-void Engine::launch_steps(unsigned first, unsigned end) {
-    struct Lease {  // the shards' streams, for as long as steps are being queued
-        Engine& e;
-        explicit Lease(Engine& engine) : e(engine) {
-            if (e.n_local_ < 2 || e.cfg_.world > 1 || e.kernel_timing_) return;
-            e.shard_streams_.assign(e.n_local_, nullptr);
-            for (unsigned l = 1; l < e.n_local_; ++l) e.shard_streams_[l] = StreamPool::instance().take();
+// The shards' streams, from before the first step is queued until the streams are out of the capture that recorded the
+// steps, or until the steps themselves are over: StreamPool serves every engine of the process, and an engine on another
+// thread may borrow a stream the moment it is back.  After an error they are destroyed, not lent again.
+Engine::ShardStreams::ShardStreams(Engine& e) : engine_(e) {
+    if (e.n_local_ < 2 || e.cfg_.world > 1 || e.kernel_timing_) return;
+    e.shard_streams_.assign(e.n_local_, nullptr);
+    for (unsigned l = 1; l < e.n_local_; ++l) e.shard_streams_[l] = StreamPool::instance().take();
+}
+void Engine::ShardStreams::give_back() {
+    for (cudaStream_t st : engine_.shard_streams_)
+        if (st) StreamPool::instance().give(st);
+    engine_.shard_streams_.clear();
+}
+Engine::ShardStreams::~ShardStreams() {
+    for (cudaStream_t st : engine_.shard_streams_)
+        if (st) cudaStreamDestroy(st);
+    engine_.shard_streams_.clear();
+}
+
+// A program run as a short chain of CUDA graphs, each four times as long as the one before: on an engine's first run
+// every graph but the first (a single step) is captured and instantiated, at 10 to 20 us of host time per kernel, while
+// its predecessor runs on the GPU (the first run of 100 headline steps: 17.1 to 15.9 ms; later runs are the same).
+void Engine::launch_step_graphs() {
+    if (graphs_.empty()) {
+        unsigned length = 1;
+        for (unsigned first = 0; first < cfg_.n_step; first += length, length *= 4)
+            graphs_.push_back({first, std::min(first + length, cfg_.n_step), nullptr, 0});
+        // a last graph shorter than its predecessor's launch joins it
+        if (graphs_.size() > 1 && graphs_.back().end - graphs_.back().first < (graphs_.back().first - graphs_[graphs_.size() - 2].first) / 2) {
+            graphs_[graphs_.size() - 2].end = cfg_.n_step;
+            graphs_.pop_back();
         }
-        ~Lease() {
-            for (cudaStream_t st : e.shard_streams_) {
-                if (!st) continue;
-                if (std::uncaught_exceptions()) cudaStreamDestroy(st);  // may still belong to a broken capture
-                else StreamPool::instance().give(st);
+    }
+    last_launches_ = 0;
+    for (StepGraph& g : graphs_) {
+        if (!g.exec) {
+            cudaGraph_t graph = nullptr;
+            launch_counter_ = 0;
+            ShardStreams streams(*this);
+            KGE_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+            try {
+                launch_steps(g.first, g.end);
+            } catch (...) {
+                cudaStreamEndCapture(stream_, &graph);
+                if (graph) cudaGraphDestroy(graph);
+                throw;
             }
-            e.shard_streams_.clear();
+            KGE_CUDA(cudaStreamEndCapture(stream_, &graph));
+            streams.give_back();
+            cudaError_t err = cudaGraphInstantiate(&g.exec, graph, 0);
+            cudaGraphDestroy(graph);
+            KGE_CUDA(err);
+            g.launches = launch_counter_;
         }
-    } lease(*this);
+        KGE_CUDA(cudaGraphLaunch(g.exec, stream_));
+        last_launches_ += g.launches;
+    }
+}
+
+void Engine::launch_steps(unsigned first, unsigned end) {
     if (first == 0) launch_gather(0, stream_);
     for (unsigned step = first; step < end; ++step) launch_one_step(step);
     if (end < cfg_.n_step) return;

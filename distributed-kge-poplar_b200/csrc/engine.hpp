@@ -222,6 +222,17 @@ class Engine {
     bool shards_beside() const { return !shard_streams_.empty() && !kernel_timing_; }
     void shards_fork();
     void shards_join();
+    class ShardStreams {  // fills shard_streams_ from the process's pool
+       public:
+        explicit ShardStreams(Engine& e);
+        ~ShardStreams();
+        ShardStreams(const ShardStreams&) = delete;
+        ShardStreams& operator=(const ShardStreams&) = delete;
+        void give_back();
+
+       private:
+        Engine& engine_;
+    };
     // While alive, what the engine launches goes to local shard l's stream.
     class ShardScope {
        public:

@@ -586,3 +586,42 @@ def test_bf16_values_with_float32_optimiser_state(name):
     values = got_state["entity_data"][..., :d]
     np.testing.assert_array_equal(values, _bf16_round(values))
     engine.close()
+
+
+def test_engines_on_two_threads_capture_their_first_runs_side_by_side():
+    """Two engines with several shards record their first program runs at the same time, each with branches on streams
+    that a pool lends to both: the results are those of the same runs one after the other, bit for bit."""
+    import threading
+
+    def fresh(i):
+        case = CASES["config1_transe_l1"]
+        cfg, state, engine, batch = _build({**case, "seed": 40 + i}, n_step=6, warm=True, pad=2)
+        return cfg, engine, batch
+
+    want = []
+    for i in range(2):
+        cfg, engine, batch = fresh(i)
+        loss = [_run_engine(engine, cfg, batch, 1e-3) for _ in range(3)]
+        want.append((loss, read_state(engine, cfg, RW, cfg.n_shard)))
+        engine.close()
+    for _ in range(4):
+        made = [fresh(i) for i in range(2)]
+        start, got = threading.Barrier(2), [None, None]
+
+        def work(i):
+            cfg, engine, batch = made[i]
+            start.wait()
+            got[i] = [_run_engine(engine, cfg, batch, 1e-3) for _ in range(3)]
+
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for i, (cfg, engine, _) in enumerate(made):
+            assert got[i] is not None, "the run on this thread failed"
+            np.testing.assert_array_equal(got[i], want[i][0])
+            state = read_state(engine, cfg, RW, cfg.n_shard)
+            for name, value in want[i][1].items():
+                np.testing.assert_array_equal(state[name], value, err_msg=name)
+            engine.close()
