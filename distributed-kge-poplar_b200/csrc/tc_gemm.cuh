@@ -30,6 +30,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "exchange.cuh"
 #include "pdl.cuh"
 
@@ -1112,11 +1114,10 @@ inline cudaError_t make_operand_map(const Operand& op, int mn, int k, int rows, 
 // How many clusters of `splits` blocks of the pipelined kernel the device can hold at once
 // (a cluster needs its blocks on SMs of one GPC, one block per SM).  0 when the query fails.
 inline int max_resident_clusters(int splits) {
-    static int cached[kMaxDeviceOrdinals][kMaxClusterSplits + 1] = {};
-    static bool known[kMaxDeviceOrdinals][kMaxClusterSplits + 1] = {};
+    static std::atomic<int> known[kMaxDeviceOrdinals][kMaxClusterSplits + 1] = {};  // the answer plus one, 0 = not asked yet
     if (splits < 1 || splits > kMaxClusterSplits) return 0;
     const int slot = current_device_slot();
-    if (slot >= 0 && known[slot][splits]) return cached[slot][splits];
+    if (const int answer = slot >= 0 ? known[slot][splits].load() : 0) return answer - 1;
     auto kernel = k_tc_gemm_async<64, false, false>;
     int n = 0;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes_async<64>()) == cudaSuccess) {
@@ -1136,10 +1137,7 @@ inline int max_resident_clusters(int splits) {
             (void)cudaGetLastError();
         }
     }
-    if (slot >= 0) {
-        known[slot][splits] = true;
-        cached[slot][splits] = n;
-    }
+    if (slot >= 0) known[slot][splits].store(n + 1);
     return n;
 }
 

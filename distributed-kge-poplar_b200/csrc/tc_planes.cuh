@@ -1220,11 +1220,10 @@ inline cudaError_t configure_planes() {
 // How many clusters of `splits` blocks of k_tc_planes the current device holds at once (one block
 // per SM whatever the tile width, so one instantiation answers for all).
 inline int max_resident_plane_clusters(int splits) {
-    static int cached[kMaxDeviceOrdinals][kMaxClusterSplits + 1] = {};
-    static bool known[kMaxDeviceOrdinals][kMaxClusterSplits + 1] = {};
+    static std::atomic<int> known[kMaxDeviceOrdinals][kMaxClusterSplits + 1] = {};  // the answer plus one, 0 = not asked yet
     if (splits < 1 || splits > kMaxClusterSplits) return 0;
     const int slot = current_device_slot();
-    if (slot >= 0 && known[slot][splits]) return cached[slot][splits];
+    if (const int answer = slot >= 0 ? known[slot][splits].load() : 0) return answer - 1;
     int n = 0;
     if (configure_planes<128, SIDE_NONE>() == cudaSuccess) {
         cudaLaunchConfig_t config = {};
@@ -1243,10 +1242,7 @@ inline int max_resident_plane_clusters(int splits) {
             (void)cudaGetLastError();
         }
     }
-    if (slot >= 0) {
-        known[slot][splits] = true;
-        cached[slot][splits] = n;
-    }
+    if (slot >= 0) known[slot][splits].store(n + 1);
     return n;
 }
 
