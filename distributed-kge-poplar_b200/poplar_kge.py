@@ -550,6 +550,8 @@ class Engine:
             chunk = np.pad(chunk, [(0, 0), (0, rw - chunk.shape[1]), (0, 0)])
         return chunk
 
+    CONVERT_CHUNK_BYTES = 64 << 20
+
     def initialise_all(self, entity_features: np.ndarray) -> None:
         """Reset the variables, then stream all features ``[n_local, n_entity, f]`` into the table."""
         self.initialise_variables()
@@ -560,11 +562,15 @@ class Engine:
                 self.write_entity(offset, self._padded_chunk(features, offset).astype(s.execution.dtype))
             return
         self._expect_shape("initialise_all(entity_features)", features, (self.n_local, n_entity, s.model.entity_feature_size))
-        if features.dtype not in (np.float32, np.float16):
-            features = features.astype(s.execution.dtype)
-        self._write_features(0, features)
+        if features.dtype in (np.float32, np.float16) and features.flags.c_contiguous:
+            self._write_features(0, features)
+        else:  # another type or a strided view: converted in parts, never the whole array at once
+            count = max(1, self.CONVERT_CHUNK_BYTES // max(1, self.n_local * features.shape[2] * features.dtype.itemsize))
+            for first in range(0, n_entity, count):
+                part = features[:, first : first + count]
+                self._write_features(first, part if part.dtype in (np.float32, np.float16) else part.astype(s.execution.dtype))
         if n_entity % rw:  # the last chunk's overflow slots, whose features are zero, name the padding row
-            self._write_features(0, np.zeros((self.n_local, 1, features.shape[2]), features.dtype))
+            self._write_features(0, np.zeros((self.n_local, 1, features.shape[2]), s.execution.dtype))
         self.uninitialized_entity_data[:] = False
 
     def write_all_rows(self, entity_data: np.ndarray) -> None:

@@ -193,3 +193,38 @@ def test_documented_switches_are_the_ones_the_sources_read():
             read |= set(re.findall(r'environ(?:\.get)?\(?\[?"(KGE_[A-Z0-9_]+)"', text))
     assert read, "no switch found: the patterns above no longer match the sources"
     assert documented == read
+
+
+@pytest.mark.parametrize("kind", ["float64", "strided", "float16_strided", "big_endian"])
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+def test_features_of_another_type_or_layout_are_converted_in_parts(kind, dtype):
+    """No call that initialise_all makes holds more than a part's rows of a feature array that has to be converted, and
+    the parts cover every row once, in the table's order."""
+    settings = kge.Settings.create_demo()
+    m, e = settings.model, settings.execution
+    m.n_shard, m.n_entity, m.entity_feature_size, e.rw_batch_size, e.dtype = 2, 1003, 6, 50, dtype
+    features = np.random.RandomState(0).standard_normal((2, 1003, 6))
+    want = features.astype(np.float16 if kind == "float16_strided" else np.float32).astype(dtype)
+    given = {"float64": lambda: features, "strided": lambda: np.repeat(features.astype(np.float32), 2, axis=2)[..., ::2],
+             "float16_strided": lambda: np.asfortranarray(features.astype(np.float16)), "big_endian": lambda: features.astype(">f4")}[kind]()
+    calls = []
+
+    class Recorder:
+        def run(self, command, arrays):
+            assert command == "write_entity_range"
+            calls.append((int(arrays["row_range"][0]), arrays["write_features"].copy()))
+
+    engine = object.__new__(kge.Engine)
+    engine.settings, engine.n_local, engine.engine, engine.CONVERT_CHUNK_BYTES = settings, 2, Recorder(), 20_000
+    engine.initialise_variables = lambda: None
+    engine.uninitialized_entity_data = np.ones(1003, bool)
+    engine.initialise_all(given)
+    got, covered = np.zeros((2, 1003, 6), dtype), np.zeros(1003, int)
+    for first, part in calls[:-1]:
+        assert part.nbytes <= 20_000 and part.flags.c_contiguous
+        part = part.view(np.float16) if part.dtype == np.int16 else part
+        got[:, first : first + part.shape[1]] = part.astype(dtype)
+        covered[first : first + part.shape[1]] += 1
+    assert np.all(covered == 1)
+    np.testing.assert_allclose(got, want, rtol=1e-3 if dtype == "float16" else 1e-7)
+    assert calls[-1][0] == 0 and calls[-1][1].shape == (2, 1, 6) and not calls[-1][1].any()  # the padding row
