@@ -367,9 +367,8 @@ Engine::Engine(const SettingMap& settings) : cfg_(parse_config(settings)) {
         for (cudaEvent_t& e : ev_shard_) KGE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     for (cudaEvent_t& e : ev_join_) KGE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    KGE_CUDA(cudaEventCreate(&ev_begin_));
-    KGE_CUDA(cudaEventCreate(&ev_end_));
-    for (cudaEvent_t& e : ev_stage_) KGE_CUDA(cudaEventCreate(&e));
+    for (RunEvents& r : ev_runs_)
+        for (cudaEvent_t* e : {&r.begin, &r.end, &r.stage[0], &r.stage[1]}) KGE_CUDA(cudaEventCreate(e));
     // The plane-fed contraction needs 16-byte rows in every operand and the lookups of a block of
     // hidden rows to fit its staging area.
     planes_ = cfg_.tensor_cores && cfg_.d % 4 == 0 && cfg_.batch_size % 4 == 0 && cfg_.n_tail() % 4 == 0 &&
@@ -406,9 +405,8 @@ Engine::~Engine() {
     for (void* p : allocations_) cudaFree(p);
     for (cudaEvent_t e : ev_io_) if (e) cudaEventDestroy(e);
     if (pinned_) cudaFreeHost(pinned_);
-    if (ev_begin_) cudaEventDestroy(ev_begin_);
-    if (ev_end_) cudaEventDestroy(ev_end_);
-    for (cudaEvent_t e : ev_stage_) if (e) cudaEventDestroy(e);
+    for (const RunEvents& r : ev_runs_)
+        for (cudaEvent_t e : {r.begin, r.end, r.stage[0], r.stage[1]}) if (e) cudaEventDestroy(e);
     if (ev_fork_) cudaEventDestroy(ev_fork_);
     for (cudaEvent_t e : ev_join_) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : ev_shard_) if (e) cudaEventDestroy(e);
@@ -798,12 +796,12 @@ void Engine::stage_batch(std::vector<HostArray>& arrays, const float* learning_r
 // The sort-and-segment tables of the staged index streams (the backward of the row gather).
 void Engine::prepare_staged() {
     const size_t n = n_local_, S = cfg_.n_step, B = cfg_.batch_size, T = cfg_.n_tail(), R = cfg_.n_remote();
-    KGE_CUDA(cudaEventRecord(ev_stage_[0], stream_));
+    KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].stage[0], stream_));
     k_prepare_segments<<<(unsigned)(n * S), 512, 0, stream_>>>(
         d_head_, d_a2a_, d_relation_, d_remote_, (int)B, (int)T, (int)R, (int)cfg_.n_relation_type, d_ent_perm_,
         d_ent_off_, d_rel_perm_, d_rel_off_, d_first_slot_, split_popular_rows_ ? d_heavy_parts_ : nullptr, d_heavy_count_, d_row_info_);
     KGE_CUDA(cudaGetLastError());
-    KGE_CUDA(cudaEventRecord(ev_stage_[1], stream_));
+    KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].stage[1], stream_));
     staged_ = true;
     stage_fresh_ = true;
 }
@@ -904,7 +902,7 @@ void Engine::train_staged(float learning_rate, float* loss) {
     }
     run_words_uploaded_ = false;
     std::optional<ShardStreams> streams;
-    KGE_CUDA(cudaEventRecord(ev_begin_, stream_));
+    KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].begin, stream_));
     if (cfg_.cuda_graph && !kernel_timing_) {
         launch_step_graphs();
     } else {
@@ -918,7 +916,7 @@ void Engine::train_staged(float learning_rate, float* loss) {
         launch_steps(0, cfg_.n_step);
         last_launches_ = launch_counter_;
     }
-    KGE_CUDA(cudaEventRecord(ev_end_, stream_));
+    KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].end, stream_));
     // the loss totals and the status words are neighbours: one transfer brings both
     KGE_CUDA(cudaMemcpyAsync(pinned_ + loss_at_, d_run_ + loss_at_, (run_words_ - loss_at_) * 4, cudaMemcpyDeviceToHost, stream_));
     KGE_CUDA(cudaStreamSynchronize(stream_));
@@ -929,6 +927,7 @@ void Engine::train_staged(float learning_rate, float* loss) {
     // gather): its device time counts towards the first run of a staged batch
     ms_counts_stage_ = stage_fresh_;
     stage_fresh_ = false;
+    ev_run_ ^= 1;
     timing_collect();
     step_ += cfg_.n_step;
     raise_device_status(pinned_ + status_at_);
@@ -979,10 +978,11 @@ void Engine::kernel_time(size_t index, const char** name, float* ms, unsigned lo
 
 void Engine::last_run_stats(float* ms, unsigned long long* launches) const {
     if (ms_pending_) {
-        KGE_CUDA(cudaEventElapsedTime(&last_ms_, ev_begin_, ev_end_));
+        const RunEvents& run = ev_runs_[ev_run_ ^ 1];
+        KGE_CUDA(cudaEventElapsedTime(&last_ms_, run.begin, run.end));
         if (ms_counts_stage_) {
             float stage_ms = 0.f;
-            KGE_CUDA(cudaEventElapsedTime(&stage_ms, ev_stage_[0], ev_stage_[1]));
+            KGE_CUDA(cudaEventElapsedTime(&stage_ms, run.stage[0], run.stage[1]));
             last_ms_ += stage_ms;
         }
         ms_pending_ = false;

@@ -250,8 +250,13 @@ class Engine {
     cudaStream_t side_begin();
     void side_end(int which);
     void side_join(int which);
-    cudaEvent_t ev_begin_ = nullptr, ev_end_ = nullptr;
-    cudaEvent_t ev_stage_[2] = {nullptr, nullptr};  // around the segment preparation of a staged batch
+    // Around a program run and around the segment preparation of its batch, read only when last_run_stats asks.  Two sets
+    // in turn: what is staged or begun after a run leaves the events of that run as they are.
+    struct RunEvents {
+        cudaEvent_t begin = nullptr, end = nullptr, stage[2] = {nullptr, nullptr};
+    };
+    RunEvents ev_runs_[2];
+    unsigned ev_run_ = 0;                           // the set of the coming run; the other one is the last run's
     bool stage_fresh_ = false;                      // its time has not been counted towards a run yet
     bool poisoned_ = false;                         // a device-side wait gave up: the engine must be rebuilt
     std::vector<void*> allocations_;

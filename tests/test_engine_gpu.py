@@ -625,3 +625,21 @@ def test_engines_on_two_threads_capture_their_first_runs_side_by_side():
             for name, value in want[i][1].items():
                 np.testing.assert_array_equal(state[name], value, err_msg=name)
             engine.close()
+
+
+def test_a_batch_staged_after_a_run_leaves_its_time_alone():
+    """The time of a run is read when it is asked for: neither the staging of the next batch, which may still be under
+    way, nor a refused one changes it."""
+    cfg, _, engine, batch = _build(CASES["config1_transe_l1"], n_step=200, warm=True)
+    engine.stage_batch(batch)
+    engine.train_staged(1e-3)
+    engine.stage_batch(batch)
+    first = engine.last_run_stats()
+    assert first[0] > 0
+    with pytest.raises(ValueError, match="not below"):
+        engine.stage_batch({**batch, "head": batch["head"] + np.uint32(cfg.n_remote)})
+    engine.stage_batch(batch)
+    assert engine.last_run_stats() == first
+    engine.train_staged(1e-3)
+    assert engine.last_run_stats() != first
+    engine.close()
