@@ -176,8 +176,7 @@ int kge_train_staged(kge_engine* engine, float learning_rate, float* loss) {
 
 int kge_last_run_stats(kge_engine* engine, float* device_ms, unsigned long long* kernel_launches) {
     if (!engine) return KGE_INVALID_ARGUMENT;
-    engine->impl->last_run_stats(device_ms, kernel_launches);
-    return KGE_OK;
+    return guarded(engine->last_error, [&] { engine->impl->last_run_stats(device_ms, kernel_launches); });
 }
 
 int kge_set_kernel_timing(kge_engine* engine, int on) {

@@ -1,0 +1,80 @@
+"""Calls of the CUDA runtime that fail, made to fail on the host: a preloaded library answers the n-th call of a function
+with an error code and passes every other call on.  No kernel is disturbed."""
+
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+ROOT = Path(__file__).resolve().parents[1]
+
+SHIM = r"""
+#include <dlfcn.h>
+#include <stdlib.h>
+static void *runtime(const char *name) { return dlsym(dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD), name); }
+static int due(const char *variable, int *calls) {  /* FAIL_<function>="n": the n-th call and all later ones, "n!": that one */
+    const char *at = getenv(variable);
+    if (!at) return 0;
+    const int n = atoi(at);
+    ++*calls;
+    return at[1] == '!' ? *calls == n : *calls >= n;
+}
+int cudaGraphInstantiate(void **exec, void *graph, unsigned long long flags) {
+    static int calls;
+    if (due("FAIL_cudaGraphInstantiate", &calls)) return 2; /* out of memory */
+    return ((int (*)(void **, void *, unsigned long long))runtime("cudaGraphInstantiate"))(exec, graph, flags);
+}
+int cudaGraphLaunch(void *exec, void *stream) {
+    static int calls;
+    if (due("FAIL_cudaGraphLaunch", &calls)) return 2;
+    return ((int (*)(void *, void *))runtime("cudaGraphLaunch"))(exec, stream);
+}
+int cudaEventElapsedTime(float *ms, void *begin, void *end) {
+    static int calls;
+    if (due("FAIL_cudaEventElapsedTime", &calls)) return 600; /* not ready */
+    return ((int (*)(float *, void *, void *))runtime("cudaEventElapsedTime"))(ms, begin, end);
+}
+"""
+
+PRELUDE = """
+import sys
+sys.path[:0] = [{root!r}, {tests!r}]
+import numpy as np
+from distributed_kge_poplar_b200 import capi
+from helpers import read_state
+from test_engine_gpu import CASES, RW, _build, _run_engine
+"""
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    folder = tmp_path_factory.mktemp("shim")
+    (folder / "shim.c").write_text(SHIM)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", str(folder / "shim.c"), "-o", str(folder / "shim.so"), "-ldl"], check=True)
+    return folder / "shim.so"
+
+
+def _run(shim, body, **fail):
+    env = dict(os.environ, LD_PRELOAD=str(shim), **{f"FAIL_{name}": value for name, value in fail.items()})
+    script = PRELUDE.format(root=str(ROOT), tests=str(ROOT / "tests")) + body
+    done = subprocess.run([sys.executable, "-c", script], env=env, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stdout[-2000:] + done.stderr[-2000:]
+    return done.stdout
+
+
+def test_a_failing_event_read_is_an_error_code(shim):
+    """An exception that left the C entry would end the process."""
+    out = _run(shim, """
+cfg, _, engine, batch = _build(CASES["config1_transe_l1"])
+_run_engine(engine, cfg, batch, 1e-3)
+try:
+    engine.last_run_stats()
+    print("no error")
+except RuntimeError as e:
+    print("raised", e)
+assert engine.last_run_stats()[0] > 0
+""", cudaEventElapsedTime="1!")
+    assert out.startswith("raised") and "cudaEventElapsedTime" in out
