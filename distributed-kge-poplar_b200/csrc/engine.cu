@@ -902,24 +902,32 @@ void Engine::train_staged(float learning_rate, float* loss) {
     }
     run_words_uploaded_ = false;
     std::optional<ShardStreams> streams;
-    KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].begin, stream_));
-    if (cfg_.cuda_graph && !kernel_timing_) {
-        launch_step_graphs();
-    } else {
-        launch_counter_ = 0;
-        if (kernel_timing_) {
-            // hold the stream while the host queues the run, so the event pairs bracket kernels only
-            k_delay<<<1, 1, 0, stream_>>>(20ll * 1000 * 1000);
-            KGE_CUDA(cudaGetLastError());
+    steps_queued_ = false;
+    try {
+        KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].begin, stream_));
+        if (cfg_.cuda_graph && !kernel_timing_) {
+            launch_step_graphs();
+        } else {
+            launch_counter_ = 0;
+            if (kernel_timing_) {
+                // hold the stream while the host queues the run, so the event pairs bracket kernels only
+                k_delay<<<1, 1, 0, stream_>>>(20ll * 1000 * 1000);
+                KGE_CUDA(cudaGetLastError());
+            }
+            streams.emplace(*this);
+            steps_queued_ = true;
+            launch_steps(0, cfg_.n_step);
+            last_launches_ = launch_counter_;
         }
-        streams.emplace(*this);
-        launch_steps(0, cfg_.n_step);
-        last_launches_ = launch_counter_;
+        KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].end, stream_));
+        // the loss totals and the status words are neighbours: one transfer brings both
+        KGE_CUDA(cudaMemcpyAsync(pinned_ + loss_at_, d_run_ + loss_at_, (run_words_ - loss_at_) * 4, cudaMemcpyDeviceToHost, stream_));
+        KGE_CUDA(cudaStreamSynchronize(stream_));
+    } catch (...) {
+        // some of the steps have moved the rows, and the step counter has not followed
+        if (steps_queued_) unusable_ = "an earlier program run failed after some of its steps: this engine's state is between two runs and it must be rebuilt";
+        throw;
     }
-    KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].end, stream_));
-    // the loss totals and the status words are neighbours: one transfer brings both
-    KGE_CUDA(cudaMemcpyAsync(pinned_ + loss_at_, d_run_ + loss_at_, (run_words_ - loss_at_) * 4, cudaMemcpyDeviceToHost, stream_));
-    KGE_CUDA(cudaStreamSynchronize(stream_));
     if (streams) streams->give_back();
     uploads_pending_ = false;
     ms_pending_ = true;
@@ -947,7 +955,7 @@ void Engine::check_device_status() {
 void Engine::raise_device_status(const unsigned* words) {
     const unsigned status[2] = {words[0], words[1]};  // [0] the tensor-core pipeline, [1] the hand-overs between processes
     if (!status[0] && !status[1]) return;
-    poisoned_ = true;
+    unusable_ = "a device-side wait of an earlier command gave up: this engine is out of step with the other processes and must be rebuilt";
     KGE_CUDA(cudaMemset(d_tc_status_, 0, sizeof(status)));
     if (status[0]) fail(KGE_DEVICE_STATUS, msg() << "a bounded wait on the tensor-core pipeline gave up (code " << status[0] << ")");
     fail(KGE_DEVICE_STATUS, msg() << "a device-side wait for rank " << (status[1] - 1)
@@ -955,9 +963,7 @@ void Engine::raise_device_status(const unsigned* words) {
 }
 
 void Engine::require_usable() const {
-    if (poisoned_)
-        fail(KGE_LOGIC_ERROR, "a device-side wait of an earlier command gave up: this engine is out of step with the other "
-                              "processes and must be rebuilt");
+    if (unusable_) fail(KGE_LOGIC_ERROR, unusable_);
 }
 
 void Engine::set_kernel_timing(bool on) {
@@ -1086,28 +1092,44 @@ void Engine::launch_step_graphs() {
     }
     last_launches_ = 0;
     for (StepGraph& g : graphs_) {
-        if (!g.exec) {
-            cudaGraph_t graph = nullptr;
+        if (!g.exec && !record_graph(g)) {  // no room for it: the rest of this run goes out kernel by kernel
+            steps_queued_ = true;
             launch_counter_ = 0;
-            ShardStreams streams(*this);
-            KGE_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-            try {
-                launch_steps(g.first, g.end);
-            } catch (...) {
-                cudaStreamEndCapture(stream_, &graph);
-                if (graph) cudaGraphDestroy(graph);
-                throw;
-            }
-            KGE_CUDA(cudaStreamEndCapture(stream_, &graph));
-            streams.give_back();
-            cudaError_t err = cudaGraphInstantiate(&g.exec, graph, 0);
-            cudaGraphDestroy(graph);
-            KGE_CUDA(err);
-            g.launches = launch_counter_;
+            launch_steps(g.first, cfg_.n_step);
+            last_launches_ += launch_counter_;
+            return;
         }
         KGE_CUDA(cudaGraphLaunch(g.exec, stream_));
+        steps_queued_ = true;
         last_launches_ += g.launches;
     }
+}
+
+// Captures and instantiates the steps of `g`; false where the driver has no memory for the graph.
+bool Engine::record_graph(StepGraph& g) {
+    cudaGraph_t graph = nullptr;
+    launch_counter_ = 0;
+    {
+        ShardStreams streams(*this);
+        KGE_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+        try {
+            launch_steps(g.first, g.end);
+        } catch (...) {
+            cudaStreamEndCapture(stream_, &graph);
+            if (graph) cudaGraphDestroy(graph);
+            throw;
+        }
+        KGE_CUDA(cudaStreamEndCapture(stream_, &graph));
+        streams.give_back();
+    }
+    const cudaError_t err = cudaGraphInstantiate(&g.exec, graph, 0);
+    cudaGraphDestroy(graph);
+    g.launches = launch_counter_;
+    if (err == cudaSuccess) return true;
+    g.exec = nullptr;
+    if (err != cudaErrorMemoryAllocation) KGE_CUDA(err);
+    cudaGetLastError();
+    return false;
 }
 
 void Engine::launch_steps(unsigned first, unsigned end) {

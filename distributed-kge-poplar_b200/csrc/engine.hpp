@@ -258,7 +258,8 @@ class Engine {
     RunEvents ev_runs_[2];
     unsigned ev_run_ = 0;                           // the set of the coming run; the other one is the last run's
     bool stage_fresh_ = false;                      // its time has not been counted towards a run yet
-    bool poisoned_ = false;                         // a device-side wait gave up: the engine must be rebuilt
+    const char* unusable_ = nullptr;                // why the engine must be rebuilt, once a command has left it in an undefined state
+    bool steps_queued_ = false;                     // the run in hand has launched work that changes the state
     std::vector<void*> allocations_;
     std::vector<ShardBuffers> shards_;
     size_t table_stride_ = 0;  // bytes between the local shards' tables
@@ -385,6 +386,7 @@ class Engine {
         unsigned long long launches;
     };
     std::vector<StepGraph> graphs_;  // a program run, in order
+    bool record_graph(StepGraph& g);
     mutable float last_ms_ = 0.f;
     mutable bool ms_pending_ = false, ms_counts_stage_ = false;  // the last run's events have not been read yet
     unsigned long long last_launches_ = 0, launch_counter_ = 0;

@@ -78,3 +78,40 @@ except RuntimeError as e:
 assert engine.last_run_stats()[0] > 0
 """, cudaEventElapsedTime="1!")
     assert out.startswith("raised") and "cudaEventElapsedTime" in out
+
+
+def test_a_graph_that_finds_no_memory_leaves_the_run_whole(shim):
+    """The second graph of a run cannot be made: its steps go out as plain launches, and later runs as graphs again."""
+    _run(shim, """
+case = CASES["config1_transe_l1"]
+cfg, _, engine, batch = _build(case, n_step=6, warm=True)
+_, _, plain, _ = _build(case, n_step=6, warm=True, cuda_graph=False)
+for run in range(4):
+    got, want = _run_engine(engine, cfg, batch, 1e-3), _run_engine(plain, cfg, batch, 1e-3)
+    np.testing.assert_array_equal(got, want)
+    assert engine.last_run_stats()[1] == plain.last_run_stats()[1], "launches"
+a, b = (read_state(e, cfg, RW, cfg.n_shard) for e in (engine, plain))
+for name in a:
+    np.testing.assert_array_equal(a[name], b[name], err_msg=name)
+""", cudaGraphInstantiate="2!")
+
+
+def test_a_run_that_fails_half_way_makes_the_engine_unusable(shim):
+    """The first of a run's graphs has moved the rows when the second cannot be launched."""
+    _run(shim, """
+cfg, _, engine, batch = _build(CASES["config1_transe_l1"], n_step=6, warm=True)
+for run in range(3):
+    try:
+        _run_engine(engine, cfg, batch, 1e-3)
+    except RuntimeError as e:
+        assert "cudaGraphLaunch" in str(e), e
+        break
+else:
+    raise SystemExit("no launch failed")
+try:
+    _run_engine(engine, cfg, batch, 1e-3)
+except RuntimeError as e:
+    assert "must be rebuilt" in str(e), e
+else:
+    raise SystemExit("the engine trains on")
+""", cudaGraphLaunch="2!")
