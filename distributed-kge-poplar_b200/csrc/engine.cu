@@ -905,9 +905,10 @@ void Engine::train_staged(float learning_rate, float* loss) {
     steps_queued_ = false;
     try {
         KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].begin, stream_));
-        if (cfg_.cuda_graph && !kernel_timing_) {
+        if (cfg_.cuda_graph && !kernel_timing_ && launched_before_) {
             launch_step_graphs();
         } else {
+            launched_before_ = true;
             launch_counter_ = 0;
             if (kernel_timing_) {
                 // hold the stream while the host queues the run, so the event pairs bracket kernels only
@@ -1076,9 +1077,15 @@ Engine::ShardStreams::~ShardStreams() {
     engine_.shard_streams_.clear();
 }
 
-// A program run as a short chain of CUDA graphs, each four times as long as the one before: on an engine's first run
-// every graph but the first (a single step) is captured and instantiated, at 10 to 20 us of host time per kernel, while
-// its predecessor runs on the GPU (the first run of 100 headline steps: 17.1 to 15.9 ms; later runs are the same).
+// A program run as a short chain of CUDA graphs, each four times as long as the one before: on the run that makes them,
+// every graph but the first (a single step) is captured and instantiated while its predecessor runs on the GPU.  That is
+// an engine's second run; the first goes out as plain launches, at about 3 us of host time each, while a graph costs 12 us
+// per kernel in a chain and up to 22 us among the branches of several shards (capture 1, instantiation 9 to 19, upload 2).
+// Milliseconds of an engine's first / second / later run, graphs made in the first and in the second:
+//   demo preset, 5 steps of 2 shards   1.45 / 0.31 / 0.29    0.58 / 1.46 / 0.29
+//   4 shards of TransE-L1, 20 steps    13.8 / 1.95 / 1.91    2.75 / 13.1 / 1.92
+//   2 shards of the headline, 20       7.36 / 3.66 / 2.98    4.26 / 7.14 / 3.00
+//   headline model, 100 steps          16.9 / 8.36 / 7.79    9.08 / 15.4 / 7.80
 void Engine::launch_step_graphs() {
     if (graphs_.empty()) {
         unsigned length = 1;

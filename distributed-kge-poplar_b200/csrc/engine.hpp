@@ -387,6 +387,7 @@ class Engine {
     };
     std::vector<StepGraph> graphs_;  // a program run, in order
     bool record_graph(StepGraph& g);
+    bool launched_before_ = false;  // the first program run has gone out as plain launches
     mutable float last_ms_ = 0.f;
     mutable bool ms_pending_ = false, ms_counts_stage_ = false;  // the last run's events have not been read yet
     unsigned long long last_launches_ = 0, launch_counter_ = 0;

@@ -70,7 +70,7 @@ typedef struct kge_array {
  *       n_shard / world_size consecutive shards; default 0 / 1)
  *   execution.feature_dtype ("float16" | "float32"; storage type of the feature part of a
  *       row; default = execution.dtype)
- *   execution.cuda_graph (bool, default true: replay the step loop as one CUDA graph)
+ *   execution.cuda_graph (bool, default true: replay the step loop as CUDA graphs from an engine's second run on)
  * `artefact_dir` takes the place of gp_folder (the codelet folder); it is accepted and ignored.
  */
 int kge_create(const kge_setting* settings, size_t n_settings, const char* artefact_dir,

@@ -643,3 +643,21 @@ def test_a_batch_staged_after_a_run_leaves_its_time_alone():
     engine.train_staged(1e-3)
     assert engine.last_run_stats() != first
     engine.close()
+
+
+@pytest.mark.parametrize("name", ["config1_transe_l1", "transe_l2_softmax_features", "long_k_split", "transh_logsigmoid"])
+@pytest.mark.parametrize("n_step", [1, 2, 7])
+def test_launched_recorded_and_replayed_runs_are_the_same(name, n_step):
+    """An engine's first run goes out as plain launches, the second makes the graphs, the third replays them; one, two and
+    three graphs.  Bit for bit what an engine without graphs computes."""
+    cfg, _, graphs, batch = _build(CASES[name], n_step=n_step, warm=True, pad=2)
+    _, _, plain, _ = _build(CASES[name], n_step=n_step, warm=True, pad=2, cuda_graph=False)
+    for run in range(4):
+        b = batch if run != 2 else random_batch(cfg, n_step, 5, pad=2)
+        np.testing.assert_array_equal(_run_engine(graphs, cfg, b, 1e-3), _run_engine(plain, cfg, b, 1e-3))
+        assert graphs.last_run_stats()[1] == plain.last_run_stats()[1]
+        a, b_ = read_state(graphs, cfg, RW, cfg.n_shard), read_state(plain, cfg, RW, cfg.n_shard)
+        for key in a:
+            np.testing.assert_array_equal(a[key], b_[key], err_msg=f"run {run}: {key}")
+    graphs.close()
+    plain.close()
