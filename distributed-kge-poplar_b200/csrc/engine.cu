@@ -194,6 +194,8 @@ Config parse_config(const SettingMap& s) {
         fail(KGE_INVALID_ARGUMENT, "ComplEx and RotatE need an even 'model.embedding_size'");
     if (c.score_fn == SCORE_ROTATE && c.dist_fn == DIST_DOT)
         fail(KGE_INVALID_ARGUMENT, "RotatE scores by a distance: 'model.distance_fn' must be 'L1' or 'L2'");
+    if (c.score_fn == SCORE_TRANSH && c.d >= UINT32_MAX / kMaxSortItems)
+        fail(KGE_INVALID_ARGUMENT, msg() << "TransH: 'model.embedding_size' is limited to " << UINT32_MAX / kMaxSortItems - 1);
     if (c.n_tail() < 2) fail(KGE_INVALID_ARGUMENT, "n_shard * a2a_size must be at least 2");
     if ((size_t)c.batch_size + c.n_tail() > (size_t)kMaxSortItems)
         fail(KGE_INVALID_ARGUMENT, msg() << "batch_size + n_shard * a2a_size (" << c.n_remote()
@@ -2338,6 +2340,7 @@ void Engine::ensure_predict_buffers() {
     predict_chunk_ = predict_planes_ ? 148u * 128u : (unsigned)std::min<size_t>(65536, std::max<size_t>(4096, ((size_t)16 << 20) / Q / 128 * 128));
     predict_chunk_ = std::min(predict_chunk_, (unsigned)round_up(cfg_.n_entity, 128));
     if (const char* v = std::getenv("KGE_PREDICT_PASS_ROWS")) predict_chunk_ = std::max(64u, (unsigned)std::atoi(v) / 4u * 4u);
+    if (cfg_.score_fn == SCORE_TRANSH) predict_chunk_ = std::min(predict_chunk_, (unsigned)kTranshMaxTails);
     p_chunk_hidden_ = (float*)device_alloc((size_t)predict_chunk_ * D * 4);
     p_raw_ = (float*)device_alloc(Q * predict_chunk_ * 4);
     if (predict_planes_) {

@@ -10,6 +10,8 @@
 // the head rows, the translation rows and the raw normals.  FP32-pipe kernels; every sum has a fixed order.
 #pragma once
 
+#include <algorithm>
+
 #include "kernels.cuh"
 
 namespace kge {
@@ -49,6 +51,7 @@ k_transh_predict(const float* __restrict__ hid_h, const uint32_t* __restrict__ h
 // fill the registers of two blocks per SM).  512 x 768 x 128: 316 us with a warp per tail, a query after the other and
 // three full reductions each; 39 us this way.
 constexpr int kTranshRows = 4, kTranshCols = 8, kTranshWarps = 8;
+constexpr int kTranshMaxTails = 65535 * kTranshCols * kTranshWarps;  // per launch
 
 // sums[o] of all lanes added up for o = 0 .. 31; lane l returns the total of sums[l].
 __device__ __forceinline__ float reduce_to_lanes(float (&sums)[32]) {
@@ -74,12 +77,21 @@ k_transh_score(const float* __restrict__ pt, const float* __restrict__ nrm, cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i0 = blockIdx.x * kTranshRows, j0 = (blockIdx.y * kTranshWarps + warp) * kTranshCols;
     if (j0 >= T) return;
-    // rows past the end read the last one (predict's largest operand, 4096 rows a pass, keeps the offsets below 2^32)
+    // Rows as 32-bit offsets, past the end the last one.  A training step's rows (4096 of 2^20 columns at most) lie within
+    // 2^32 of the first; those of a ranking pass, which may be any number, are counted from the block's own first rows.
+    int from_i = 0, from_j = 0;
+    if constexpr (!BACKWARD) {
+        from_i = i0;
+        from_j = (int)blockIdx.y * kTranshWarps * kTranshCols;
+        pt += (size_t)from_i * D;
+        nrm += (size_t)from_i * D;
+        tails += (size_t)from_j * D;
+    }
     uint32_t row_i[kTranshRows], row_j[kTranshCols];
 #pragma unroll
-    for (int a = 0; a < kTranshRows; ++a) row_i[a] = (uint32_t)min(i0 + a, B - 1) * (uint32_t)D;
+    for (int a = 0; a < kTranshRows; ++a) row_i[a] = (uint32_t)(min(i0 + a, B - 1) - from_i) * (uint32_t)D;
 #pragma unroll
-    for (int b = 0; b < kTranshCols; ++b) row_j[b] = (uint32_t)min(j0 + b, T - 1) * (uint32_t)D;
+    for (int b = 0; b < kTranshCols; ++b) row_j[b] = (uint32_t)(min(j0 + b, T - 1) - from_j) * (uint32_t)D;
     const int i = i0 + lane / kTranshCols, j = j0 + lane % kTranshCols;  // the output whose totals this lane ends up with
     const bool live = i < B && j < T;
     const size_t out = (size_t)i * T + j;
@@ -159,6 +171,8 @@ inline cudaError_t launch_transh_score(const float* pt, const float* nrm, const 
                                        const ExchangeSync& sync, cudaStream_t stream) {
     constexpr int kCols = kTranshCols * kTranshWarps;
     const dim3 grid((B + kTranshRows - 1) / kTranshRows, (T + kCols - 1) / kCols), block(32 * kTranshWarps);
+    if (S && (uint64_t)std::max(B, T) * D > UINT32_MAX) return cudaErrorInvalidValue;
+    if (T > kTranshMaxTails) return cudaErrorInvalidValue;
     if (S) return launch_dependent(k_transh_score<true>, grid, block, 0, stream, pt, nrm, tails, raw, S, U, B, T, D, sync);
     return launch_dependent(k_transh_score<false>, grid, block, 0, stream, pt, nrm, tails, raw, S, U, B, T, D, sync);
 }

@@ -228,3 +228,11 @@ def test_features_of_another_type_or_layout_are_converted_in_parts(kind, dtype):
     assert np.all(covered == 1)
     np.testing.assert_allclose(got, want, rtol=1e-3 if dtype == "float16" else 1e-7)
     assert calls[-1][0] == 0 and calls[-1][1].shape == (2, 1, 6) and not calls[-1][1].any()  # the padding row
+
+
+def test_transh_refuses_rows_whose_offsets_pass_32_bits():
+    """4096 rows of a step times the columns of a row stay below 2^32 in the kernel that counts them in 32 bits."""
+    settings = engine_settings(StepConfig(n_shard=1, n_entity=50, n_relation_type=4, embedding_size=1 << 20, entity_feature_size=0,
+                                          batch_size=4, a2a_size=3, score_fn="TransH", distance_fn="L1"))
+    with pytest.raises(ValueError, match="TransH: 'model.embedding_size' is limited to 1048574"):
+        capi.CEngine(settings)

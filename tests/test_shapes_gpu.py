@@ -100,3 +100,28 @@ def test_ranking_in_whole_tiles(monkeypatch, score_fn, distance_fn, queries, row
     assert_close(got_score, want_score, RTOL, "ranking: scores")
     clear = _clear(want_score)
     np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
+
+
+def test_transh_ranking_in_one_pass_of_more_than_2_32_values(monkeypatch):
+    """A pass of 1 060 000 rows of 4096 columns: offsets into its hidden rows need more than 32 bits.  Passes of the usual
+    length give the same lists."""
+    rows, size, queries, n_best = 1_060_000, 4096, 8, 128
+    cfg = StepConfig(n_shard=1, n_entity=rows, n_relation_type=2, embedding_size=size, entity_feature_size=0, batch_size=4, a2a_size=4,
+                     score_fn="TransH", distance_fn="L1", gamma=8.0)
+    rng = np.random.RandomState(2)
+    variables = {name: rng.normal(size=(2, size)).astype(np.float32) for name in ("relation_embedding", "relation_normal")}
+    got = []
+    for pass_rows in (None, rows):
+        if pass_rows:
+            monkeypatch.setenv("KGE_PREDICT_PASS_ROWS", str(pass_rows))
+        engine = capi.CEngine(engine_settings(cfg, dtype="float16", rw_batch=RW, **{"execution.predict_hr_batch_size": queries, "execution.predict_n_best": n_best}))
+        engine.run("initialise_entities", {})
+        for name, value in variables.items():
+            engine.run("write", {"value": value}, name=name)
+        hr = np.stack([np.zeros(queries, int), 1 + np.arange(queries) * 1000, np.arange(queries) % 2], axis=1)
+        got.append(_predict(engine, cfg, hr, np.array([rows - 1]), queries, n_best))
+        engine.close()
+    (idx, score), (idx_whole, score_whole) = got
+    assert np.sum(idx[..., 1] >= 2**32 // size) > 0, "no candidate behind the first 2^32 values: the case shows nothing"
+    np.testing.assert_array_equal(score_whole, score)
+    np.testing.assert_array_equal(idx_whole, idx)
