@@ -528,7 +528,7 @@ void Engine::allocate() {
         sizes_at_ = keys_at_ + cfg_.n_step;
         loss_at_ = sizes_at_ + cfg_.n_step;
         status_at_ = loss_at_ + n_local_;
-        run_words_ = status_at_ + 2;
+        run_words_ = status_at_ + 3;
         d_run_ = (uint32_t*)device_alloc(run_words_ * 4);
         KGE_CUDA(cudaMemset(d_run_ + loss_at_, 0, (run_words_ - loss_at_) * 4));
         KGE_CUDA(cudaMallocHost((void**)&pinned_, run_words_ * 4));
@@ -543,6 +543,7 @@ void Engine::allocate() {
     d_loss_total_ = reinterpret_cast<float*>(d_run_ + loss_at_);
     d_tc_status_ = d_run_ + status_at_;
     d_status_ = d_tc_status_ + 1;
+    d_planes_short_ = d_tc_status_ + 2;
     d_ent_perm_ = (uint32_t*)device_alloc(steps * (B + T) * 4);
     d_ent_off_ = (uint32_t*)device_alloc(steps * (R + 1) * 4);
     d_rel_perm_ = (uint32_t*)device_alloc(steps * B * 4);
@@ -2436,12 +2437,23 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
     uint32_t* d_rel = d_rw_idx_ + n * hr;
     KGE_CUDA(cudaMemcpyAsync(d_head, h_head, n * hr * 4, cudaMemcpyHostToDevice, stream_));
     KGE_CUDA(cudaMemcpyAsync(d_rel, h_rel, n * hr * 4, cudaMemcpyHostToDevice, stream_));
+    unsigned longest = 0;  // rows of the command's longest pass
+    for (unsigned l = 0; l < n; ++l) longest = std::max(longest, (unsigned)std::min<uint32_t>(predict_chunk_, h_count[l]));
 
     const bool two_nets = cfg_.n_net() == 2, vec = (D % 4) == 0;
     const float* W_head = cfg_.n_net() >= 1 ? dense_ + dense_bounds_[1] : nullptr;
     const float* W_tail = two_nets ? dense_ + dense_bounds_[2] : W_head;
     const unsigned dtiles = ceil_div((unsigned)D, 64);
     launch_counter_ = 0;
+    const bool half_projection = predict_planes_ && p_half_w_ && fills_gpu(longest, (unsigned)D);
+    if (half_projection) {
+        KGE_CUDA(cudaMemsetAsync(d_planes_short_, 0, 4, stream_));
+        KGE_LAUNCH("predict_planes", tc::k_half_columns<<<ceil_div((unsigned)D, 32), 256, 0, stream_>>>(
+                                         W_tail, (int)cfg_.f, (int)D, p_half_stride_, p_half_w_, p_half_w_ + (size_t)cfg_.f * p_half_stride_, p_half_w_info_, d_planes_short_));
+        KGE_CUDA(cudaGetLastError());
+        KGE_CUDA(cudaMemcpyAsync(pinned_ + status_at_ + 2, d_planes_short_, 4, cudaMemcpyDeviceToHost, stream_));
+        KGE_CUDA(cudaEventRecord(io_event(0), stream_));
+    }
 
     // 1. predicted tails of the local queries, written into every process's gathered query buffer
     for (unsigned l = 0; l < n; ++l) {
@@ -2472,15 +2484,12 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
 
     // 2. stream each local shard's rows past all queries
     const float* queries = (const float*)(arena_ + arena_offset_predict(0));
-    unsigned longest = 0;  // rows of the command's longest pass
-    for (unsigned l = 0; l < n; ++l) longest = std::max(longest, (unsigned)std::min<uint32_t>(predict_chunk_, h_count[l]));
+    if (half_projection) KGE_CUDA(cudaEventSynchronize(io_event(0)));  // the queries are being prepared meanwhile
+    p_half_w_usable_ = half_projection && pinned_[status_at_ + 2] == 0;
     if (predict_planes_) {
         KGE_LAUNCH("predict_planes", k_lower_plane<<<(unsigned)std::min<size_t>((Q * D + 255) / 256, 148 * 8), 256, 0, stream_>>>(queries, Q * D, p_query_lo_));
         if (fills_gpu((unsigned)Q, longest)) KGE_LAUNCH("predict_planes", tc::k_half_rows<<<ceil_div((unsigned)Q, 8), 256, 0, stream_>>>(queries, (int)Q, (int)D, p_half_stride_, p_half_q_,
                                                                                                     p_half_q_ + Q * p_half_stride_, p_half_q_info_));
-        if (p_half_w_ && fills_gpu(longest, (unsigned)D))
-            KGE_LAUNCH("predict_planes", tc::k_half_columns<<<ceil_div((unsigned)D, 32), 256, 0, stream_>>>(
-                                             W_tail, (int)cfg_.f, (int)D, p_half_stride_, p_half_w_, p_half_w_ + (size_t)cfg_.f * p_half_stride_, p_half_w_info_));
     }
     TopkParams tp{(int)Q, (int)nb, score_is_gamma_minus_distance(cfg_.score_fn) ? 1 : 0, cfg_.gamma};
     for (unsigned l = 0; l < n; ++l) {
@@ -2540,7 +2549,7 @@ bool Engine::predict_pass_planes(ShardBuffers& b, uint32_t start, unsigned c, ui
                                  int net) {
     const unsigned D = cfg_.d, F = cfg_.f;
     const uint8_t* rows = b.table + (size_t)start * layout_.row_bytes;
-    const bool hidden_half = F > 0 && p_half_w_ && fills_gpu(c, D), score_half = fills_gpu(Q, c);
+    const bool hidden_half = F > 0 && p_half_w_usable_ && fills_gpu(c, D), score_half = fills_gpu(Q, c);
     auto half_plane = [&](const __half* hi, const __half* lo, bool mn_major) {
         return tc::PlaneOperand{reinterpret_cast<const float*>(hi), reinterpret_cast<const float*>(lo), (long long)p_half_stride_ * 2, mn_major ? 1 : 0, 16};
     };

@@ -273,6 +273,7 @@ class Engine {
     unsigned long long* d_xchg_trace_ = nullptr;  // optional time stamps of the hand-overs (KGE_EXCHANGE_TRACE=1)
     unsigned* d_xchg_words_ = nullptr;  // [XCHG_KINDS] published epochs, [XCHG_KINDS] finished-block counters
     unsigned* d_tc_status_ = nullptr;
+    unsigned* d_planes_short_ = nullptr;  // beside the status words: the tails' projection is beyond the float16 planes
     // split-k workspace of the tensor-core contractions (shared by all of them: one stream)
     float *tc_ws_ = nullptr, *tc_ws_rowsum_ = nullptr;
     size_t tc_ws_floats_ = 0;
@@ -325,7 +326,7 @@ class Engine {
     RelationRows with_regularisers(RelationRows rr, unsigned l, unsigned step) const;
     // What crosses to the GPU before a run and what comes back, laid out alike in pinned and in device memory: the five
     // index streams, then the run's words (step numbers, Adam step sizes, the loss totals' zeros), then the two status
-    // words.  Offsets in 32-bit words.
+    // words and ranking's flag.  Offsets in 32-bit words.
     uint32_t *pinned_ = nullptr, *d_run_ = nullptr;
     size_t stage_at_[5] = {}, keys_at_ = 0, sizes_at_ = 0, loss_at_ = 0, status_at_ = 0, run_words_ = 0;
     bool uploads_pending_ = false;      // transfers out of `pinned_` may still be under way
@@ -346,6 +347,7 @@ class Engine {
     __half *p_half_q_ = nullptr, *p_half_t_ = nullptr, *p_half_w_ = nullptr;
     float2 *p_half_q_info_ = nullptr, *p_half_t_info_ = nullptr, *p_half_w_info_ = nullptr;
     int p_half_stride_ = 0;
+    bool p_half_w_usable_ = false;  // by the ranking in hand
     bool topk_beside_ = false;  // a pass's merge is on the side stream
     float *p_feat_ = nullptr, *p_chunk_lo_ = nullptr, *p_query_lo_ = nullptr;  // planes of a pass: widened / lower features, lower hidden rows, lower queries
 

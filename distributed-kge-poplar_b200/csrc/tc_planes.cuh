@@ -69,12 +69,16 @@ struct TopkFilterArgs {
 };
 
 // What belongs to an operand of float16 planes.  Every row (k-major) or column (mn-major) of the operand's [mn][k] view is
-// scaled by a power of two that brings its largest value to [2^13, 2^14), and split into two float16 parts: 22 bits of
-// every value down to 2^-15 of the row's largest, as in two TF32 planes, and below that an error of 2^-38 of the largest,
-// far under the rounding of the fp32 sums; in half the bytes and with products of 16 k per instruction instead of 8.
+// scaled by a power of two that brings its largest value to [2^13, 2^14), and split into a float16 and 2^kHalfLoScale times
+// what that leaves, another float16: 22 bits of every value down to 2^-27 of the row's largest, as in two TF32 planes; in
+// half the bytes and with products of 16 k per instruction instead of 8.  Smaller values have an error of 2^-51 of the
+// largest at most.  Where that could show, the result comes from elsewhere: L2 distances do not notice (their own terms
+// are at least as large as the largest value's square, and what cancels is recomputed); a dot product so small that the
+// rows' largest values must have met zeros is recomputed (kHalfDirect); and a projection with such values keeps its TF32
+// planes (k_half_columns tells).
 struct HalfRows {
-    const float2* info;    // [mn] {squared norm of the values, what undoes the scale}; null: {-, 1}
-    const float* values;   // the fp32 rows themselves (L2 distances that cancel are recomputed from them)
+    const float2* info;    // [mn] {squared norm of the values, what undoes the scale (0: all values are zero)}; null: {-, 1}
+    const float* values;   // the fp32 rows themselves (distances and products that cancel are recomputed from them)
     long long stride_bytes;
 };
 
@@ -180,6 +184,16 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a_desc, uint
         "setp.ne.b32 p, %4, 0;\n"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
         ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// The same with the accumulator as it was before the product scaled by 2^-SCALE.
+template <int SCALE>
+__device__ __forceinline__ void umma_16bit_onto_scaled(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+    asm volatile(
+        "{\n.reg .pred p;\n"
+        "setp.eq.b32 p, 0, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n}"
+        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "n"(SCALE)
         : "memory");
 }
 // Instruction descriptor for bf16 inputs (format 1 at bits 7-9 and 10-12), fp32 accumulator.
@@ -330,6 +344,20 @@ static __device__ __noinline__ float l2_squared_direct(const float* __restrict__
         const float d = a[k] - b[k];
         s0 = fmaf(d, d, s0);
     }
+    return s0 + s1;
+}
+// Likewise the dot product.
+static __device__ __noinline__ float dot_direct(const float* __restrict__ a, const float* __restrict__ b, int K) {
+    float s0 = 0.f, s1 = 0.f;
+    int k = 0;
+    for (; k + 3 < K; k += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(b + k);
+        s0 = fmaf(x.x, y.x, s0);
+        s1 = fmaf(x.y, y.y, s1);
+        s0 = fmaf(x.z, y.z, s0);
+        s1 = fmaf(x.w, y.w, s1);
+    }
+    for (; k < K; ++k) s0 = fmaf(a[k], b[k], s0);
     return s0 + s1;
 }
 
@@ -834,6 +862,12 @@ constexpr int kHalfSlots = 9;
 constexpr int kHalfPlane = 128 * 128;
 constexpr int kHalfAccWarps = 16;  // 32 columns of a row per thread
 constexpr int kHalfThreads = 32 * (2 + kHalfAccWarps);
+// The lower plane holds 2^13 times the remainder (at most 4 of values below 2^14): it stays a normal number 13 bits longer.
+constexpr int kHalfLoScale = 13;
+// A scaled dot product of K terms below kHalfDirect * K is recomputed: the lower planes' last bits, and the product of two
+// remainders that is left out, come to at most 1.25 * 2^-21 per term, 2^-22 of what is kept.  Of rows whose values are alike one
+// pair in 300 000 is that small (K 256).
+constexpr float kHalfDirect = 4.f;
 constexpr size_t half_smem_bytes() { return 1024 + (size_t)kHalfSlots * kHalfPlane + (size_t)kBM * 128 * 4; }
 
 __device__ __forceinline__ void accumulating_warps_sync() {
@@ -917,13 +951,16 @@ k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ Plane
                 const uint32_t tmem_acc = tmem_base + (uint32_t)(t * BN);
                 uint32_t accumulate = 0u;
                 auto arrived = [&](int j) { mbar_wait(&bar_full[(i0 + j) % kHalfSlots], (uint32_t)(((i0 + j) / kHalfSlots) & 1), g.status, 3u); };
-                auto multiply = [&](int ja, int jb) {  // four 16-deep products of a 64-deep slice
+                // four 16-deep products of a 64-deep slice; the cross terms come first, at 2^kHalfLoScale times their size
+                auto multiply = [&](int ja, int jb, bool onto_cross_terms = false) {
                     const uint32_t a = smem_u32(ring + (size_t)((i0 + ja) % kHalfSlots) * kHalfPlane), b = smem_u32(ring + (size_t)((i0 + jb) % kHalfSlots) * kHalfPlane);
                     const uint64_t da = pp.A.mn_major ? make_mnmajor_sw128_desc16(a) : make_kmajor_sw128_desc(a);
                     const uint64_t db = pp.B.mn_major ? make_mnmajor_sw128_desc16(b) : make_kmajor_sw128_desc(b);
 #pragma unroll
                     for (int ks = 0; ks < 4; ++ks) {
-                        umma_bf16(tmem_acc, da + (uint64_t)ks * sa, db + (uint64_t)ks * sb, idesc, accumulate);
+                        const uint64_t ka = da + (uint64_t)ks * sa, kb = db + (uint64_t)ks * sb;
+                        if (onto_cross_terms && ks == 0) umma_16bit_onto_scaled<kHalfLoScale>(tmem_acc, ka, kb, idesc);
+                        else umma_bf16(tmem_acc, ka, kb, idesc, accumulate);
                         accumulate = 1u;
                     }
                 };
@@ -946,7 +983,7 @@ k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ Plane
                         multiply(2, b_hi);
                         give_back(2);
                     }
-                    multiply(1, b_hi);
+                    multiply(1, b_hi, true);
                     give_back(1);
                     give_back(b_hi);
                     umma_commit(&bar_acc_ready[t]);
@@ -1019,7 +1056,7 @@ k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ Plane
                 for (int j = 0; j < 32; ++j) acc[j] += __uint_as_float(r[j]);
             }
             accumulating_warps_sync();  // s_col is complete; the rows of the tile before have left the staging
-            uint32_t direct_bits = 0, pass_bits = 0;  // the rare cases: recomputed distances, scores that reach the cut-off
+            uint32_t direct_bits = 0, pass_bits = 0;  // the rare cases: recomputed pairs, scores that reach the cut-off
             if (EPI == EPI_L2_DISTANCE) {
                 // The square root is the approximate one (relative error 2^-23, exact at zero): the form's own error is larger.
                 const float sign = pp.filter.score_is_gamma_minus ? -1.f : 1.f, offset = pp.filter.score_is_gamma_minus ? pp.filter.gamma : 0.f;
@@ -1038,8 +1075,13 @@ k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ Plane
                     }
                 }
             } else {
+                const float few = EPI == EPI_STORE && of_a.y != 0.f ? kHalfDirect * (float)g.K : 0.f;
 #pragma unroll
-                for (int j = 0; j < CPT; ++j) acc[j] = acc[j] * of_a.y * s_col[1][part * CPT + j];
+                for (int j = 0; j < CPT; ++j) {
+                    const float undo_b = s_col[1][part * CPT + j];
+                    if (EPI == EPI_STORE) direct_bits |= (uint32_t)(fabsf(acc[j]) < few && undo_b != 0.f) << j;
+                    acc[j] = acc[j] * of_a.y * undo_b;
+                }
             }
             // 16-byte chunk c of tile row `row` lies at chunk c ^ (row & 7): the lanes of a warp hold
             // 32 different rows, and this spreads their stores over all banks
@@ -1047,7 +1089,7 @@ k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ Plane
 #pragma unroll
             for (int j = 0; j < CPT; j += 4)
                 *reinterpret_cast<float4*>(mine + (((part * (CPT / 4) + (j >> 2)) ^ (row & 7)) << 2)) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-            if (EPI == EPI_L2_DISTANCE && m < g.M) {
+            if (EPI != EPI_ADD_TABLE_VALUE && m < g.M) {
                 const float* a_row = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(pp.half_a.values) + (size_t)m * pp.half_a.stride_bytes);
                 uint32_t todo = direct_bits | (filter ? pass_bits : 0u);
                 while (todo) {
@@ -1055,8 +1097,10 @@ k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ Plane
                     todo &= todo - 1;
                     if (col >= g.N) continue;
                     float* cell = mine + (((tcol >> 2) ^ (row & 7)) << 2) + (tcol & 3);
-                    if ((direct_bits >> bit) & 1u)
-                        *cell = sqrtf(l2_squared_direct(a_row, reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(pp.half_b.values) + (size_t)col * pp.half_b.stride_bytes), g.K));
+                    if ((direct_bits >> bit) & 1u) {
+                        const float* b_row = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(pp.half_b.values) + (size_t)col * pp.half_b.stride_bytes);
+                        *cell = EPI == EPI_STORE ? dot_direct(a_row, b_row, g.K) : sqrtf(l2_squared_direct(a_row, b_row, g.K));
+                    }
                     if (filter) {
                         const TopkFilterArgs& f = pp.filter;
                         const float score = f.score_is_gamma_minus ? f.gamma - *cell : *cell;
@@ -1111,7 +1155,12 @@ __device__ __forceinline__ uint32_t half_scale_exponent(float largest) {
 __device__ __forceinline__ float power_of_two(uint32_t biased) { return __uint_as_float(biased << 23); }
 __device__ __forceinline__ void half_split(float v, __half& hi, __half& lo) {
     hi = __float2half_rn(v);
-    lo = __float2half_rn(v - __half2float(hi));
+    lo = __float2half_rn((v - __half2float(hi)) * (float)(1 << kHalfLoScale));
+}
+// Whether that has lost more of `value` (scaled: v) than two TF32 planes would, 2^-21 of it.
+__device__ __forceinline__ bool half_split_is_short(float value, float v, __half hi, __half lo) {
+    const float left = (v - __half2float(hi)) * (float)(1 << kHalfLoScale) - __half2float(lo);  // exact
+    return fabsf(left) > fabsf(v) / (float)(1 << (21 - kHalfLoScale)) || (value != 0.f && fabsf(v) < 1e-20f);
 }
 
 // x [rows, D] (D a multiple of 4) into hi and lo [rows, stride], a warp per row; bound by memory (65536 x 256: 128 MB).
@@ -1140,12 +1189,14 @@ k_half_rows(const float* __restrict__ x, int rows, int D, int stride, __half* __
         *reinterpret_cast<uint2*>(hi + (size_t)r * stride + c) = *reinterpret_cast<const uint2*>(h);
         *reinterpret_cast<uint2*>(lo + (size_t)r * stride + c) = *reinterpret_cast<const uint2*>(l);
     }
-    if (lane == 0) info[r] = make_float2(square, power_of_two(254u - s));
+    if (lane == 0) info[r] = make_float2(square, largest == 0.f ? 0.f : power_of_two(254u - s));
 }
 
-// w [F, D] into hi and lo [F, stride], scaled by columns: 32 columns per block, eight rows at a time.
+// w [F, D] into hi and lo [F, stride], scaled by columns: 32 columns per block, eight rows at a time.  *short_of becomes 1 if a
+// value is too far below its column's largest for the planes (it is left alone otherwise).
 static __global__ void __launch_bounds__(256)
-k_half_columns(const float* __restrict__ w, int F, int D, int stride, __half* __restrict__ hi, __half* __restrict__ lo, float2* __restrict__ info) {
+k_half_columns(const float* __restrict__ w, int F, int D, int stride, __half* __restrict__ hi, __half* __restrict__ lo, float2* __restrict__ info,
+               unsigned* __restrict__ short_of) {
     __shared__ float part[8][32];
     const int lane = threadIdx.x & 31, group = threadIdx.x >> 5, c = (int)blockIdx.x * 32 + lane;
     float largest = 0.f;
@@ -1166,11 +1217,13 @@ k_half_columns(const float* __restrict__ w, int F, int D, int stride, __half* __
 #pragma unroll 4
     for (int f = group; f < F; f += 8) {
         __half h, l;
-        half_split(w[(size_t)f * D + c] * scale, h, l);
+        const float value = w[(size_t)f * D + c], v = value * scale;
+        half_split(v, h, l);
+        if (half_split_is_short(value, v, h, l)) *short_of = 1u;
         hi[(size_t)f * stride + c] = h;
         lo[(size_t)f * stride + c] = l;
     }
-    if (group == 0) info[c] = make_float2(0.f, power_of_two(254u - s));
+    if (group == 0) info[c] = make_float2(0.f, largest == 0.f ? 0.f : power_of_two(254u - s));
 }
 
 // What a producing kernel stores for four neighbouring values.
@@ -1335,6 +1388,7 @@ inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
             if (l.gp.p[i].A.mn_major || l.gp.p[i].B.mn_major || l.gp.p[i].g.out_blocks) return cudaErrorInvalidValue;
     if (l.gp.bf16 == 2) {
         const int epilogue = l.gp.p[0].g.epilogue;
+        if (epilogue != EPI_ADD_TABLE_VALUE && (!l.gp.p[0].half_a.values || !l.gp.p[0].half_b.values)) return cudaErrorInvalidValue;
         if (SIDE == SIDE_NONE && epilogue == EPI_ADD_TABLE_VALUE) return launch_half<EPI_ADD_TABLE_VALUE>(l, stream);
         if (SIDE == SIDE_NONE && epilogue == EPI_STORE) return launch_half<EPI_STORE>(l, stream);
         if (SIDE == SIDE_NORMS && epilogue == EPI_L2_DISTANCE) return launch_half<EPI_L2_DISTANCE>(l, stream);

@@ -79,6 +79,16 @@ def test_ranking_lists(monkeypatch, score_fn, distance_fn, n_best, pass_rows):
     np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
 
 
+def _rank_whole_tiles(cfg, state, queries, counts):
+    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW, feature_dtype="float16", **{"execution.predict_hr_batch_size": len(queries), "execution.predict_n_best": 10}))
+    write_state(engine, cfg, state, RW)
+    engine.set_kernel_timing(True)
+    got = _predict(engine, cfg, queries, counts, len(queries), 10)
+    assert "predict_planes" in engine.kernel_times(), "the tensor cores have not ranked"
+    engine.close()
+    return got
+
+
 @pytest.mark.parametrize("score_fn,distance_fn", [("TransE", "L2"), ("DistMult", "MatMul")])
 @pytest.mark.parametrize("queries,rows,size,features", [(129, 9473, 20, 0), (130, 9500, 132, 70), (5, 18945, 12, 9)])
 def test_ranking_in_whole_tiles(monkeypatch, score_fn, distance_fn, queries, rows, size, features):
@@ -86,16 +96,13 @@ def test_ranking_in_whole_tiles(monkeypatch, score_fn, distance_fn, queries, row
     a last pass below 148."""
     monkeypatch.setenv("KGE_PREDICT_PASS_ROWS", str(rows // 4 * 4))
     n_entity = rows + 300
-    cfg = StepConfig(n_shard=1, n_entity=n_entity, n_relation_type=4, embedding_size=size, entity_feature_size=features, batch_size=8, a2a_size=6,
+    cfg = StepConfig(n_shard=1, n_entity=n_entity, n_relation_type=4, embedding_size=size, entity_feature_size=features, batch_size=8, a2a_size=8,
                      score_fn=score_fn, distance_fn=distance_fn, gamma=8.0)
     state = random_state(cfg, 3, fp16_features=True, warm=True)
     state["entity_data"][0, 1::3, :size] *= 1e-3
-    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW, feature_dtype="float16", **{"execution.predict_hr_batch_size": queries, "execution.predict_n_best": 10}))
-    write_state(engine, cfg, state, RW)
     rng = np.random.RandomState(1)
     hr = np.stack([np.zeros(queries, int), 1 + rng.randint(n_entity - 1, size=queries), rng.randint(4, size=queries)], axis=1)
-    got_idx, got_score = _predict(engine, cfg, hr, np.array([n_entity - 1]), queries, 10)
-    engine.close()
+    got_idx, got_score = _rank_whole_tiles(cfg, state, hr, np.array([n_entity - 1]))
     want_idx, want_score = make_oracle(cfg, state).predict(hr, np.array([n_entity - 1]), 10)
     assert_close(got_score, want_score, RTOL, "ranking: scores")
     clear = _clear(want_score)
@@ -125,3 +132,57 @@ def test_transh_ranking_in_one_pass_of_more_than_2_32_values(monkeypatch):
     assert np.sum(idx[..., 1] >= 2**32 // size) > 0, "no candidate behind the first 2^32 values: the case shows nothing"
     np.testing.assert_array_equal(score_whole, score)
     np.testing.assert_array_equal(idx_whole, idx)
+
+
+@pytest.mark.parametrize("score_fn,distance_fn", [("TransE", "L2"), ("DistMult", "MatMul")])
+@pytest.mark.parametrize("spread", [6, 12, 20])
+def test_ranking_rows_with_columns_of_very_different_size(monkeypatch, score_fn, distance_fn, spread):
+    """Passes on float16 planes whose rows range over 2^(2 * spread).  For products the queries range the other way round,
+    so that every column counts alike: 2^12 fits the planes, 2^24 needs all of them, and at 2^40 the values that matter lie
+    below their last bit and the pair is recomputed.  1e-5, as two TF32 planes keep it."""
+    rows, size, n_query = 9473, 132, 129
+    monkeypatch.setenv("KGE_PREDICT_PASS_ROWS", str(rows // 4 * 4))
+    cfg = StepConfig(n_shard=1, n_entity=rows, n_relation_type=4, embedding_size=size, entity_feature_size=0, batch_size=8, a2a_size=8,
+                     score_fn=score_fn, distance_fn=distance_fn, gamma=8.0)
+    state = random_state(cfg, 5)
+    scale = np.exp2(np.random.RandomState(6).permutation(np.linspace(-spread, spread, size).round())).astype(np.float32)
+    state["entity_data"][..., :size] *= scale
+    state["relation_embedding"] *= scale if distance_fn == "L2" else 1 / scale**2
+    rng = np.random.RandomState(1)
+    queries = np.stack([np.zeros(n_query, int), 1 + rng.randint(rows - 1, size=n_query), rng.randint(4, size=n_query)], axis=1)
+    got_idx, got_score = _rank_whole_tiles(cfg, state, queries, np.array([rows - 1]))
+    want_idx, want_score = make_oracle(cfg, state).predict(queries, np.array([rows - 1]), 10)
+    assert_close(got_score, want_score, RTOL, "ranking: scores")
+    clear = _clear(want_score)
+    np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
+
+
+@pytest.mark.parametrize("spread,masked", [(6, False), (12, False), (12, True), (25, True)])
+def test_ranking_with_a_projection_of_very_different_rows(monkeypatch, spread, masked):
+    """The hidden rows' contraction: projection rows that range over 2^(2 * spread) against features that range the other
+    way round (float16, so over 2^24 at most), or whose features are zero where the projection is large: what is left lies
+    2^spread below the largest value of its column.  At 2^25 the planes are too short and the pass takes the TF32 ones."""
+    rows, size, features, n_query = 9500, 132, 70, 130
+    monkeypatch.setenv("KGE_PREDICT_PASS_ROWS", str(rows // 4 * 4))
+    cfg = StepConfig(n_shard=1, n_entity=rows, n_relation_type=4, embedding_size=size, entity_feature_size=features, batch_size=8, a2a_size=8,
+                     score_fn="DistMult", distance_fn="MatMul", gamma=8.0)
+    state = random_state(cfg, 7, fp16_features=True)
+    state["entity_data"][..., :size] *= 1e-3  # the scores show the projection
+    feat = state["entity_data"][..., 3 * size :]
+    if masked:
+        large = np.arange(features) % 2 == 0
+        feat[..., large] = 0
+        state["feature_projection"][large] *= np.float32(2.0 ** (2 * spread - 6))
+        state["feature_projection"][~large] *= np.float32(2.0**-6)
+        feat *= np.float32(2.0**6)
+    else:
+        scale = np.exp2(np.random.RandomState(8).permutation(np.linspace(-spread, spread, features).round())).astype(np.float32)
+        feat[...] = (feat * scale).astype(np.float16).astype(np.float32)
+        state["feature_projection"] /= scale[:, None]
+    rng = np.random.RandomState(1)
+    queries = np.stack([np.zeros(n_query, int), 1 + rng.randint(rows - 1, size=n_query), rng.randint(4, size=n_query)], axis=1)
+    got_idx, got_score = _rank_whole_tiles(cfg, state, queries, np.array([rows - 1]))
+    want_idx, want_score = make_oracle(cfg, state).predict(queries, np.array([rows - 1]), 10)
+    assert_close(got_score, want_score, RTOL, "ranking: scores")
+    clear = _clear(want_score)
+    np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
