@@ -878,9 +878,11 @@ __device__ __forceinline__ void accumulating_warps_sync() {
 // Whole tiles of 128 x 128 of one contraction on float16 planes (HalfRows), many per SM: ranking's hidden rows and scores.
 // A block works through every gridDim-th tile.  One warp fetches planes and one multiplies, as far ahead as the ring and
 // the four accumulators in TMEM reach (all of the next tile at d 256), while sixteen warps add up the slices' products and
-// finish the tile.  Bound by those warps (distances, staging, stores), not by the products (1.7 us of a tile of d 256).
-// 1250 x 18944 scores of d 256: 110 us with a block per tile, 82 with two such blocks per SM, 68 now; 18944 x 256 hidden
-// rows of f 768: 46, 31, 34.  (TMA copies and MMAs issued by an elected lane: see elect_one.)
+// finish the tile.  Bound by the latency of a tile's chain: planes in, products (1.7 us of a tile of d 256), accumulators out
+// of TMEM, distances, staging, stores.  1250 x 18944 scores of d 256: 110 us with a block per tile, 82 with two such blocks
+// per SM, 68 now; 18944 x 256 hidden rows of f 768: 46, 31, 34.  (TMA copies and MMAs issued by an elected lane: see
+// elect_one.)  Both forms with the elected lane, launch latency included: scores 92.6 us with two blocks per SM and 83.6
+// in this form, hidden rows 35.5 and 39.3; one kernel serves both launches, at 5 of the pass's 120 us less than the other form.
 template <int EPI>
 __global__ void __launch_bounds__(kHalfThreads, 1)
 k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneMaps maps) {
@@ -1160,7 +1162,8 @@ __device__ __forceinline__ void half_split(float v, __half& hi, __half& lo) {
 // Whether that has lost more of `value` (scaled: v) than two TF32 planes would, 2^-21 of it.
 __device__ __forceinline__ bool half_split_is_short(float value, float v, __half hi, __half lo) {
     const float left = (v - __half2float(hi)) * (float)(1 << kHalfLoScale) - __half2float(lo);  // exact
-    return fabsf(left) > fabsf(v) / (float)(1 << (21 - kHalfLoScale)) || (value != 0.f && fabsf(v) < 1e-20f);
+    const bool lost = fabsf(left) > fabsf(v) / (float)(1 << (21 - kHalfLoScale)), vanished = fabsf(v) < 1e-20f;
+    return lost | (vanished & (value != 0.f));
 }
 
 // x [rows, D] (D a multiple of 4) into hi and lo [rows, stride], a warp per row; bound by memory (65536 x 256: 128 MB).
@@ -1214,15 +1217,17 @@ k_half_columns(const float* __restrict__ w, int F, int D, int stride, __half* __
     if (c >= D) return;
     const uint32_t s = half_scale_exponent(largest);
     const float scale = power_of_two(s);
+    bool is_short = false;
 #pragma unroll 4
     for (int f = group; f < F; f += 8) {
         __half h, l;
         const float value = w[(size_t)f * D + c], v = value * scale;
         half_split(v, h, l);
-        if (half_split_is_short(value, v, h, l)) *short_of = 1u;
+        is_short |= half_split_is_short(value, v, h, l);  // (no branch: the loop's loads overlap)
         hi[(size_t)f * stride + c] = h;
         lo[(size_t)f * stride + c] = l;
     }
+    if (is_short) *short_of = 1u;
     if (group == 0) info[c] = make_float2(0.f, largest == 0.f ? 0.f : power_of_two(254u - s));
 }
 
