@@ -2325,7 +2325,7 @@ void Engine::refresh_lower_plane(size_t offset, size_t count) {
 // Where a pass has a wave of 128 x 128 tiles its contractions run on float16 planes (tc::HalfRows): the fp16 features as
 // they lie in the table, everything else in two parts, half the instructions and bytes of the TF32 planes and no copy of
 // the features.  Smaller passes divide k over a cluster, which those instantiations do not.  A pass of 18944 rows and
-// 1250 queries, d 256, f 768: 308 -> 135 us.
+// 1250 queries, d 256, f 768: 308 us on TF32 planes, 120 us.
 static bool fills_gpu(unsigned m, unsigned n) { return ceil_div(m, 128) * ceil_div(n, 128) >= 148; }
 
 void Engine::ensure_predict_buffers() {

@@ -937,7 +937,9 @@ struct PairBwdArgs {
     int tiles_m0;  // set by launch_pair_bwd
 };
 
-// Two neighbouring fp32 values in one 64-bit register pair: the FP32 pipe takes both in one instruction.
+// Two neighbouring fp32 values in one 64-bit register pair.  An instruction issues both and holds the FP32 pipe as long as
+// two would: half the issue slots, the same pipe time.  The pair gradients and TransH's scores are faster with it, TransH's
+// gradients slower (k_transh_bwd).
 using f32x2 = unsigned long long;
 __device__ __forceinline__ f32x2 pack2(float lo, float hi) {
     f32x2 r;
@@ -952,11 +954,6 @@ __device__ __forceinline__ float2 unpack2(f32x2 v) {
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     f32x2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 // a - b, rounded once.
@@ -2795,7 +2792,8 @@ __device__ __forceinline__ bool is_last_writer(const RowSource& s, unsigned j, c
     return !__syncthreads_or(later);
 }
 
-// write_entity: fresh embedding ~ N(0, std), zero moments, features from the host array (in pinned memory).
+// write_entity: fresh embedding ~ N(0, std), zero moments, features from the host array's piece (in pinned memory up to 64 KB,
+// else in device memory).
 template <class ST, class FT, class IT>
 __global__ void __launch_bounds__(128)
 k_write_entity(RowSource rows, RowLayout L, const IT* __restrict__ features, uint32_t seed, uint32_t shard0, float stddev) {
@@ -2858,7 +2856,7 @@ k_init_table(uint8_t* __restrict__ table, RowLayout L, size_t n_rows, uint32_t s
     }
 }
 
-// write_entity_rows: whole rows [value | m | sqrt(v) | feature] from the host array (in pinned memory).
+// write_entity_rows: whole rows [value | m | sqrt(v) | feature] from the host array's piece (as write_entity's).
 template <class ST, class FT, class IT>
 __global__ void __launch_bounds__(128)
 k_write_rows(RowSource rows, RowLayout L, const IT* __restrict__ data) {
@@ -2877,8 +2875,8 @@ k_write_rows(RowSource rows, RowLayout L, const IT* __restrict__ data) {
     }
 }
 
-// read_entity: whole rows out, in the host array's element type, into pinned memory: four elements per store where the
-// segments allow it, so that a warp's stores make whole 128-byte writes on the link.
+// read_entity: whole rows out, in the host array's element type, into a piece in pinned memory (up to 64 KB) or device memory:
+// four elements per store where the segments allow it, so that a warp's stores make whole 128-byte writes, on the link too.
 template <class ST, class FT, class OT>
 __global__ void __launch_bounds__(128)
 k_read_rows(RowSource rows, RowLayout L, OT* __restrict__ out) {

@@ -181,9 +181,9 @@ inline cudaError_t launch_transh_score(const float* pt, const float* nrm, const 
 //   rows i:  d_pt_ik = sum_j C_ij sg_ijk,   d_n_ik = sum_j C_ij (sg_ijk S_ij + U_ij t_jk)
 //   rows j:  d_t_jk  = sum_i C_ij (U_ij n_ik - sg_ijk), stored to the shard that owns tail j
 // In k_pair_bwd's form (sums in order, the operands staged one chunk ahead) but with one column per lane, 32 per block:
-// a packed instruction occupies the FP32 pipe twice as long, so pairs would only halve the warps that hide latency.  The first blocks take the rows i (one per
-// warp, chunks of 64 tails), the others the rows j (two per warp, which share the reads of pt and n; chunks of 32
-// triples).  512 x 768 x 128: 153 us with a block per output row and a thread per column, 87 us with pairs,
+// a packed instruction holds the FP32 pipe twice as long, so pairs only halve the warps that hide latency.  The first blocks
+// take the rows i (one per warp, chunks of 64 tails), the others the rows j (two per warp, which share the reads of pt and
+// n; chunks of 32 triples).  512 x 768 x 128: 153 us with a block per output row and a thread per column, 87 us with pairs,
 // 61 us this way.
 struct TranshBwdArgs {
     const float *pt, *nrm, *tails, *C, *S, *U;
