@@ -90,7 +90,7 @@ def test_predict_in_many_passes_matches_oracle(monkeypatch, score_fn, distance_f
     monkeypatch.setenv("KGE_PREDICT_PASS_ROWS", "100")
     monkeypatch.setenv("KGE_PREDICT_FILTER_IN_SCORES", filter_in_scores)
     cfg = StepConfig(n_shard=2, n_entity=700, n_relation_type=6, embedding_size=36, entity_feature_size=12,
-                     batch_size=6, a2a_size=4, score_fn=score_fn, distance_fn=distance_fn, gamma=5.0)
+                     batch_size=8, a2a_size=4, score_fn=score_fn, distance_fn=distance_fn, gamma=5.0)
     hr, n_best = 8, 60
     state = random_state(cfg, 22, warm=False)
     engine = capi.CEngine(engine_settings(cfg, rw_batch=RW, **{"execution.predict_hr_batch_size": hr, "execution.predict_n_best": n_best}))
@@ -99,7 +99,9 @@ def test_predict_in_many_passes_matches_oracle(monkeypatch, score_fn, distance_f
     counts = np.array([699, 655])
     rng = np.random.RandomState(5)
     queries = np.stack([rng.randint(2, size=13), 1 + rng.randint(600, size=13), rng.randint(6, size=13)], axis=1)
+    engine.set_kernel_timing(True)
     got_idx, got_score = _predict(engine, cfg, queries, counts, hr, n_best)
+    assert "predict_planes" in engine.kernel_times(), "the tensor cores have not ranked"
     want_idx, want_score = oracle.predict(queries, counts, n_best)
     np.testing.assert_allclose(got_score, want_score, rtol=1e-5, atol=1e-5)
     clear = _clear(want_score)

@@ -109,6 +109,33 @@ def test_ranking_in_whole_tiles(monkeypatch, score_fn, distance_fn, queries, row
     np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
 
 
+@pytest.mark.parametrize("score_fn,distance_fn", [("TransE", "L2"), ("DistMult", "MatMul")])
+@pytest.mark.parametrize("filter_in_scores", ["1", "0"])
+def test_ranking_in_several_passes_of_whole_tiles(monkeypatch, score_fn, distance_fn, filter_in_scores):
+    """From the second pass on every query has a cut-off, and scores reach the lists through the filter inside the
+    whole-tile kernel or the kernel of its own; rows that equal the best candidate tie with it in every pass."""
+    monkeypatch.setenv("KGE_PREDICT_PASS_ROWS", "9472")
+    monkeypatch.setenv("KGE_PREDICT_FILTER_IN_SCORES", filter_in_scores)
+    rows, size, n_query = 3 * 9472 + 1, 20, 130
+    cfg = StepConfig(n_shard=1, n_entity=rows, n_relation_type=4, embedding_size=size, entity_feature_size=0, batch_size=8, a2a_size=8,
+                     score_fn=score_fn, distance_fn=distance_fn, gamma=8.0)
+    state = random_state(cfg, 9)
+    for first in (50, 9000, 15000, 28000):  # pairs of equal rows, the second a pass or a few rows later
+        state["entity_data"][0, first + 400] = state["entity_data"][0, first]
+    rng = np.random.RandomState(1)
+    queries = np.stack([np.zeros(n_query, int), 1 + rng.randint(rows - 1, size=n_query), rng.randint(4, size=n_query)], axis=1)
+    queries[:4, 1] = [50, 9000, 15000, 28000]
+    state["relation_embedding"][0] = 0 if distance_fn == "L2" else 1  # the queries' own rows are the best candidates
+    queries[:4, 2] = 0
+    got_idx, got_score = _rank_whole_tiles(cfg, state, queries, np.array([rows - 1]))
+    want_idx, want_score = make_oracle(cfg, state).predict(queries, np.array([rows - 1]), 10)
+    assert_close(got_score, want_score, RTOL, "ranking: scores")
+    clear = _clear(want_score)
+    np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
+    if distance_fn == "L2":
+        np.testing.assert_array_equal(got_idx[:4, :2, 1], [[r, r + 400] for r in (50, 9000, 15000, 28000)])
+
+
 def test_transh_ranking_in_one_pass_of_more_than_2_32_values(monkeypatch):
     """A pass of 1 060 000 rows of 4096 columns: offsets into its hidden rows need more than 32 bits.  Passes of the usual
     length give the same lists."""
