@@ -797,6 +797,10 @@ def run_predict(args) -> None:
     engine.close()
     if rank == 0:
         per_step = seconds / args.steps
+        # which contraction kernel a full pass runs on (148 tiles of 128 x 128 and more: the whole-tile one), hidden rows and scores
+        pass_tiles = -(-min(148 * 128, rows - 1) // 128)
+        on_tiles = [pass_tiles * -(-n // 128) >= 148 for n in (D, hr * world)]
+        names = [k for k, on in (("k_half_tiles", any(on_tiles)), ("k_tc_planes", not all(on_tiles))) if on]
         pairs = queries_per_gpu * world * (rows - 1) * world   # every query against every row of every shard
         flop = pairs * (2 * D) + (rows - 1) * world * 2 * F * D * (queries_per_gpu // hr)  # scores + hidden rows of every pass
         peaks = measured_peaks()
@@ -809,10 +813,10 @@ def run_predict(args) -> None:
             "e2e": {"value": queries_per_gpu * world / per_step, "unit": "queries/s", "h2d_bytes_per_step": int(2 * 4 * queries_per_gpu),
                     "d2h_bytes_per_step": int(2 * scores.nbytes * (queries_per_gpu // hr))},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "tensor", "kernel": "k_half_tiles (hidden rows and L2 scores of a pass)", "achieved": flop / per_step / world / 1e12,
+            "roofline": {"bound": "tensor", "kernel": " and ".join(names) + " (hidden rows and L2 scores of a pass)", "achieved": flop / per_step / world / 1e12,
                          "peak": peaks["tensor_tflops"], "unit": "TFLOP/s", "frac": flop / per_step / world / 1e12 / peaks["tensor_tflops"],
                          "peak_source": peaks["source"], "traffic": None,
-                         "algorithmic_flops_per_step": flop, "peak_note": "dense bf16 sustained; fp32 products run as three float16 products, fp16 features as two"},
+                         "algorithmic_flops_per_step": flop, "peak_note": "dense bf16 sustained; fp32 products run as three products (float16 in k_half_tiles, TF32 in k_tc_planes), fp16 features as two"},
             "clocks": clocks, "best_score_of_first_query": float(best[0, 0]),
         }), flush=True)
     if world > 1:
