@@ -645,11 +645,11 @@ def test_a_batch_staged_after_a_run_leaves_its_time_alone():
     engine.close()
 
 
-@pytest.mark.parametrize("name", ["config1_transe_l1", "transe_l2_softmax_features", "long_k_split", "transh_logsigmoid"])
-@pytest.mark.parametrize("n_step", [1, 2, 7])
+@pytest.mark.parametrize("name,n_step", [(name, 2) for name in CASES] + [("config1_transe_l1", 1), ("config1_transe_l1", 7),
+                                                                        ("long_k_split", 1), ("long_k_split", 7), ("long_k_split", 30)])
 def test_launched_recorded_and_replayed_runs_are_the_same(name, n_step):
-    """An engine's first run goes out as plain launches, the second makes the graphs, the third replays them; one, two and
-    three graphs.  Bit for bit what an engine without graphs computes."""
+    """An engine's first run goes out as plain launches, the second makes the graphs, the third replays them; runs of
+    one, two and three graphs.  Bit for bit what an engine without graphs computes."""
     cfg, _, graphs, batch = _build(CASES[name], n_step=n_step, warm=True, pad=2)
     _, _, plain, _ = _build(CASES[name], n_step=n_step, warm=True, pad=2, cuda_graph=False)
     for run in range(4):
