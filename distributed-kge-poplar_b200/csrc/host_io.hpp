@@ -9,6 +9,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -193,7 +194,17 @@ class PinnedPool {
     std::vector<uint8_t*> free_;
 };
 
-// A block of the pool for the length of a scope.  Its transfers must have completed when the scope ends.
+// Whether a scope is being left by an exception that came up inside it: its transfers may still be under way, so its
+// blocks are not lent to anyone else but freed, for which CUDA waits.
+class LeftByException {
+   public:
+    explicit operator bool() const { return std::uncaught_exceptions() > at_entry_; }
+
+   private:
+    const int at_entry_ = std::uncaught_exceptions();
+};
+
+// A block of the pool for the length of a scope.  Its transfers must have completed when the scope ends as it should.
 class PinnedBlock {
    public:
     explicit PinnedBlock(size_t bytes = PinnedPool::kBlock) : pooled_(bytes <= PinnedPool::kBlock) {
@@ -201,7 +212,7 @@ class PinnedBlock {
         else KGE_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&data_), bytes, cudaHostAllocPortable));
     }
     ~PinnedBlock() {
-        if (pooled_) PinnedPool::instance().give(data_);
+        if (pooled_ && !left_by_exception_) PinnedPool::instance().give(data_);
         else cudaFreeHost(data_);
     }
     PinnedBlock(const PinnedBlock&) = delete;
@@ -209,6 +220,7 @@ class PinnedBlock {
     uint8_t* data() const { return data_; }
 
    private:
+    LeftByException left_by_exception_;
     bool pooled_;
     uint8_t* data_ = nullptr;
 };
@@ -221,7 +233,7 @@ class DeviceBlock {
     DeviceBlock() = default;
     ~DeviceBlock() {
         if (!data_) return;
-        {
+        if (!left_by_exception_) {
             std::lock_guard<std::mutex> lock(pool().mutex);
             if (slot_ >= 0 && pool().free[slot_].size() < kKept) {
                 pool().free[slot_].push_back(data_);
@@ -257,6 +269,7 @@ class DeviceBlock {
         static Pool* p = new Pool;
         return *p;
     }
+    LeftByException left_by_exception_;
     uint8_t* data_ = nullptr;
     int slot_ = -1;
 };

@@ -13,6 +13,7 @@ ROOT = Path(__file__).resolve().parents[1]
 
 SHIM = r"""
 #include <dlfcn.h>
+#include <stdio.h>
 #include <stdlib.h>
 static void *runtime(const char *name) { return dlsym(dlopen("libcudart.so.12", RTLD_LAZY | RTLD_NOLOAD), name); }
 static int due(const char *variable, int *calls) {  /* FAIL_<function>="n": the n-th call and all later ones, "n!": that one */
@@ -31,6 +32,15 @@ int cudaGraphLaunch(void *exec, void *stream) {
     static int calls;
     if (due("FAIL_cudaGraphLaunch", &calls)) return 2;
     return ((int (*)(void *, void *))runtime("cudaGraphLaunch"))(exec, stream);
+}
+int cudaEventRecord(void *event, void *stream) {
+    static int calls;
+    if (due("FAIL_cudaEventRecord", &calls)) return 2;
+    return ((int (*)(void *, void *))runtime("cudaEventRecord"))(event, stream);
+}
+int cudaHostAlloc(void **p, size_t bytes, unsigned flags) {
+    if (getenv("SHOW_cudaHostAlloc")) puts("cudaHostAlloc"), fflush(stdout);
+    return ((int (*)(void **, size_t, unsigned))runtime("cudaHostAlloc"))(p, bytes, flags);
 }
 int cudaEventElapsedTime(float *ms, void *begin, void *end) {
     static int calls;
@@ -115,3 +125,33 @@ except RuntimeError as e:
 else:
     raise SystemExit("the engine trains on")
 """, cudaGraphLaunch="2!")
+
+
+@pytest.mark.parametrize("command", ["read_entity_range", "read"])
+def test_blocks_of_a_failed_transfer_are_not_lent_again(shim, command):
+    """The transfer into the pinned block is under way when the event behind it fails: the block is freed, and the next
+    transfers take others, and in the end a new one."""
+    out = _run(shim, f"""
+import os
+cfg, state, engine, batch = _build(CASES["config1_transe_l1"])
+rows = np.zeros((cfg.n_shard, 300, cfg.row_size), np.float32)
+value = np.zeros((cfg.n_relation_type, cfg.embedding_size), np.float32)
+arrays, name = (dict(row_range=np.array([1, 300], np.uint32), read_data=rows), None) if {command!r} != "read" else (dict(value=value), "relation_embedding")
+engine.run({command!r}, arrays, name=name)
+os.environ["SHOW_cudaHostAlloc"] = "1"
+print("again", flush=True)
+engine.run({command!r}, arrays, name=name)
+os.environ["FAIL_cudaEventRecord"] = "1"
+for block in range(4):  # as many as the pool keeps
+    try:
+        engine.run({command!r}, arrays, name=name)
+        raise SystemExit("nothing failed")
+    except RuntimeError:
+        pass
+print("failed", flush=True)
+del os.environ["FAIL_cudaEventRecord"]
+engine.run({command!r}, arrays, name=name)
+np.testing.assert_array_equal(rows[..., : cfg.embedding_size] if name is None else value,
+                              state["entity_data"][:, 1:301, : cfg.embedding_size] if name is None else state[name])
+""")
+    assert out.split()[0] == "again" and out.split()[-2:] == ["failed", "cudaHostAlloc"]
