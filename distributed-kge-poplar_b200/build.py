@@ -16,6 +16,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
@@ -52,13 +53,12 @@ def build(force: bool = False, verbose: bool = False) -> None:
     if verbose:
         common += ["-Xptxas", "-v"]
     if force or _newer_than(LIB, lib_sources + headers + [Path(__file__)]):
-        objects = []
-        for src in lib_sources:
-            obj = HERE / "build" / (src.stem + ".o")
-            obj.parent.mkdir(exist_ok=True)
-            if force or _newer_than(obj, [src, *headers, Path(__file__)]):
-                _run([NVCC, *common, "-c", src, "-o", obj], verbose)
-            objects.append(obj)
+        objects = [HERE / "build" / (src.stem + ".o") for src in lib_sources]
+        objects[0].parent.mkdir(exist_ok=True)
+        stale = [[NVCC, *common, "-c", src, "-o", obj] for src, obj in zip(lib_sources, objects)
+                 if force or _newer_than(obj, [src, *headers, Path(__file__)])]
+        with ThreadPoolExecutor() as pool:  # the sources side by side
+            list(pool.map(lambda cmd: _run(cmd, verbose), stale))
         _run([NVCC, "-shared", *ARCH, "-o", LIB, *objects, "-cudart", "shared"], verbose)
     binding = CSRC / "pybind_module.cpp"
     if binding.exists() and (force or _newer_than(MODULE, [binding, LIB, *headers])):

@@ -285,7 +285,7 @@ int kge_op_scatter_add_rows(const float* grad_rows, const uint32_t* indices, siz
         // All n lookups are passed as "head" lookups; there are no tail and no relation lookups.
         k_prepare_segments<<<1, 512>>>(di.as<uint32_t>(), di.as<uint32_t>(), nullptr, nullptr, (int)n, 0,
                                        (int)rows, 0, dperm.as<uint32_t>(), doff.as<uint32_t>(),
-                                       nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+                                       nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
         k_segment_sum_rows<<<(unsigned)rows, 128>>>(dg.as<float>(), dperm.as<uint32_t>(), doff.as<uint32_t>(), width,
                                                     dout.as<float>());
         finish_kernels();
@@ -713,7 +713,7 @@ int kge_op_scatter_add_rows_noalloc(const float* grad_rows, const uint32_t* indi
         // Every entry the second kernel reads (perm[0, n) and offsets[0, rows]) is rewritten by the
         // first, so nothing left by an earlier call is ever read and nothing needs clearing.
         k_prepare_segments<<<1, 512, 0, stream>>>(indices, indices, nullptr, nullptr, (int)n, 0, (int)rows, 0, scratch->perm,
-                                                  scratch->offsets, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+                                                  scratch->offsets, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
         k_segment_sum_rows<<<(unsigned)rows, 128, 0, stream>>>(grad_rows, scratch->perm, scratch->offsets, width, grad_table);
         KGE_CUDA(cudaGetLastError());
     });

@@ -380,6 +380,8 @@ Engine::Engine(const SettingMap& settings) : cfg_(parse_config(settings)) {
     if (cfg_.score_fn == SCORE_TRANSH) {
         planes_ = false;  // its score has no contraction form: the step of separate kernels
     }
+    // Without features a hidden row is the stored value: the lookups and the row update read the table itself.
+    direct_rows_ = planes_ && cfg_.f == 0 && !cfg_.regularised();
     // With one shard in all a dense gradient has a single contributor: the projection gradient's contraction and the
     // relation rows' blocks of the entity update apply the Adam step themselves and k_dense_update is not launched.
     fuse_dense_ = fuse_dense_env_ && planes_ && cfg_.n_shard == 1 && cfg_.world == 1;
@@ -435,7 +437,8 @@ void Engine::allocate() {
     for (unsigned l = 0; l < n_local_; ++l) {
         ShardBuffers& b = shards_[l];
         b.table = tables + l * table_stride_;
-        for (uint8_t*& rows : b.rows_c2) rows = (uint8_t*)device_alloc((size_t)R * layout_.row_bytes);
+        if (!direct_rows_)
+            for (uint8_t*& rows : b.rows_c2) rows = (uint8_t*)device_alloc((size_t)R * layout_.row_bytes);
         b.hid_h = (float*)device_alloc((size_t)R * D * 4);
         b.hid_t = two_nets || dropout_on() ? (float*)device_alloc((size_t)R * D * 4) : b.hid_h;  // dropout: each call has its own mask
         b.pred = (float*)device_alloc((size_t)B * D * 4);
@@ -549,6 +552,7 @@ void Engine::allocate() {
     d_rel_perm_ = (uint32_t*)device_alloc(steps * B * 4);
     d_rel_off_ = (uint32_t*)device_alloc(steps * (cfg_.n_relation_type + 1) * 4);
     d_first_slot_ = (uint32_t*)device_alloc(steps * R * 4);
+    if (direct_rows_) d_lookup_row_ = (uint32_t*)device_alloc(steps * (B + T) * 4);
     d_heavy_parts_ = (uint4*)device_alloc(steps * kHeavySlots * sizeof(uint4));
     d_row_info_ = (uint4*)device_alloc(steps * 2 * R * sizeof(uint4));
     d_heavy_count_ = (uint32_t*)device_alloc(steps * 4);
@@ -802,7 +806,7 @@ void Engine::prepare_staged() {
     KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].stage[0], stream_));
     k_prepare_segments<<<(unsigned)(n * S), 512, 0, stream_>>>(
         d_head_, d_a2a_, d_relation_, d_remote_, (int)B, (int)T, (int)R, (int)cfg_.n_relation_type, d_ent_perm_,
-        d_ent_off_, d_rel_perm_, d_rel_off_, d_first_slot_, split_popular_rows_ ? d_heavy_parts_ : nullptr, d_heavy_count_, d_row_info_);
+        d_ent_off_, d_rel_perm_, d_rel_off_, d_first_slot_, split_popular_rows_ ? d_heavy_parts_ : nullptr, d_heavy_count_, d_row_info_, d_lookup_row_);
     KGE_CUDA(cudaGetLastError());
     KGE_CUDA(cudaEventRecord(ev_runs_[ev_run_].stage[1], stream_));
     staged_ = true;
@@ -1159,6 +1163,7 @@ void Engine::launch_gather(unsigned step, cudaStream_t stream) {
     for (unsigned l = 0; l < n_local_; ++l) launch_gather(step, l, stream);
 }
 void Engine::launch_gather(unsigned step, unsigned l, cudaStream_t stream) {
+    if (direct_rows_) return;
     const unsigned R = cfg_.n_remote();
     ShardBuffers& b = shards_[l];
     const uint32_t* remote = d_remote_ + ((size_t)l * cfg_.n_step + step) * R;
@@ -1489,6 +1494,18 @@ void Engine::launch_dropout(unsigned l, unsigned step, const uint8_t* rows_c) {
                                                         (int)R, dropout_params(l, step))));
 }
 
+// What the lookups of local shard l read: the table's values, or the hidden rows.
+LookupRows Engine::lookup_rows(unsigned l, unsigned step) const {
+    const ShardBuffers& b = shards_[l];
+    const size_t B = cfg_.batch_size, T = cfg_.n_tail(), sidx = (size_t)l * cfg_.n_step + step;
+    if (direct_rows_) {
+        const uint32_t* row = d_lookup_row_ + sidx * (B + T);
+        return LookupRows{b.table, b.table, row, row + B, layout_.row_bytes};
+    }
+    return LookupRows{reinterpret_cast<const uint8_t*>(b.hid_h), reinterpret_cast<const uint8_t*>(b.hid_t), d_head_ + sidx * B, d_a2a_ + sidx * T, (uint32_t)(cfg_.d * 4)};
+}
+int Engine::lookup_type() const { return !direct_rows_ ? 0 : cfg_.value_bf16 ? 2 : cfg_.state_type == ST_F16 ? 1 : 0; }
+
 // The training step with its contractions on the plane-fed kernel: seven launches on the step's
 // chain (hidden + lookups + send, scores, loss, score gradients + return, segment sums + Adam +
 // relation gradients, projection gradient, dense update) and the next step's gather beside the
@@ -1522,8 +1539,6 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
         ShardBuffers& b = shards_[l];
         uint8_t* rows_c = b.rows_c2[parity];
         const size_t sidx = (size_t)l * cfg_.n_step + step;
-        const uint32_t* a2a = step_ptr(d_a2a_, l, T);
-        const uint32_t* head = step_ptr(d_head_, l, B);
         const uint32_t* relation = step_ptr(d_relation_, l, B);
         // 1. hidden = value + feature . W, and from its epilogue the lookups and the send half of the exchange
         const bool fused_route = F > 0 && cfg_.score_fn != SCORE_COMPLEX && cfg_.score_fn != SCORE_ROTATE && !dropout_on();
@@ -1565,17 +1580,35 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                                                                     (const uint32_t*)(d_ent_perm_ + sidx * (B + T)), relation, rel_table, b.send_dst, b.send_lo_dst,
                                                                     b.pred, b.pred_lo, (int)B, (int)cfg_.a2a_size, (int)D, cfg_.score_fn, bf16 ? 1 : 0, sync)));
         } else {
-            // no features: the hidden rows are the gathered values
             launch_exchange_wait(XCHG_DENSE_PARAMS);
-            dim3 grid(ceil_div(R, 64), ceil_div(D, 64), 1);
-            KGE_LAUNCH("hidden", KGE_DISPATCH_ROW(cfg_, KGE_CUDA(launch_dependent(k_hidden<ST, FT>, dim3(grid), dim3(256), 0, stream_, rows_c, layout_,
-                                                                                  nullptr, 0u, (int)R, nullptr, nullptr, b.hid_h, b.hid_t))));
+            if (!direct_rows_) {  // the hidden rows are the gathered values
+                dim3 grid(ceil_div(R, 64), ceil_div(D, 64), 1);
+                KGE_LAUNCH("hidden", KGE_DISPATCH_ROW(cfg_, KGE_CUDA(launch_dependent(k_hidden<ST, FT>, dim3(grid), dim3(256), 0, stream_, rows_c, layout_,
+                                                                                      nullptr, 0u, (int)R, nullptr, nullptr, b.hid_h, b.hid_t))));
+            }
         }
         if (dropout_on()) launch_dropout(l, step, rows_c);
-        if (!fused_route)
-            KGE_LAUNCH("route", KGE_CUDA(launch_dependent(k_route<4>, dim3(T + B), dim3(64), 0, stream_, b.hid_h, b.hid_t, a2a, head, relation, rel_table,
-                                                          b.send_dst, b.pred, (int)T, (int)cfg_.a2a_size, (int)B, (int)D, cfg_.score_fn, sync,
-                                                          b.send_lo_dst, b.pred_lo, bf16 ? 1 : 0)));
+        if (!fused_route) {
+            LookupSizes sizes{};
+            sizes.rel_table = rel_table;
+            sizes.B = (int)B; sizes.T = (int)T; sizes.a2a = (int)cfg_.a2a_size; sizes.D = (int)D; sizes.R = (int)R;
+            sizes.lo_bf16 = bf16 ? 1 : 0;
+            sizes.prefetch = direct_rows_ && step > 0;  // the first step's index streams come from the kernel in front
+            sizes.sync = sync;
+            ShardArgs<LookupArgs> shard{};
+            LookupArgs& a = shard.s[0];
+            a.rows = lookup_rows(l, step);
+            a.relation = relation;
+            a.send_dst = b.send_dst;
+            a.send_lo_dst = l1 ? nullptr : b.send_lo_dst;
+            a.pred = b.pred;
+            a.pred_lo = l1 ? nullptr : b.pred_lo;
+            if (direct_rows_ && step + 1 == cfg_.n_step) {  // kge_debug_fetch shows the last step's hidden rows
+                a.remote = step_ptr(d_remote_, l, R);
+                a.hid = b.hid_h;
+            }
+            KGE_LAUNCH("lookup", KGE_CUDA(launch_lookup(shard, 1, sizes, cfg_.score_fn, lookup_type(), stream_)));
+        }
         if (cfg_.regularised()) launch_regularise(l, rows_c);
     }
     shards_join();
@@ -1585,7 +1618,6 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
     for (unsigned l = 0; l < n_local_; ++l) {
         const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
-        const uint32_t* head = step_ptr(d_head_, l, B);
         const uint32_t* relation = step_ptr(d_relation_, l, B);
         const uint32_t* tail = step_ptr(d_tail_, l, B);
         // 2. scores
@@ -1639,15 +1671,19 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
             h.g.x_base = reinterpret_cast<const uint8_t*>(b.tails); h.g.x_row_stride_bytes = (long long)D * 4;
             launch_planes("score_bwd", both, 2, l2 ? tc::SIDE_ROWSUM : tc::SIDE_NONE, -1, XCHG_TAIL_GRADS);
         }
-        if (cfg_.score_fn != SCORE_TRANSE)
-            KGE_LAUNCH("pred_bwd", KGE_CUDA(launch_dependent(k_pred_bwd, dim3(B), dim3(64), 0, stream_, b.d_pred, b.hid_h, head, relation, rel_table, b.d_head,
-                                                             b.d_relrow, (int)D, cfg_.score_fn)));
+        if (cfg_.score_fn != SCORE_TRANSE) {
+            ShardArgs<LookupBwdArgs> shard{};
+            shard.s[0] = LookupBwdArgs{lookup_rows(l, step), relation, b.d_pred, b.d_head, b.d_relrow, nullptr, nullptr, nullptr};
+            KGE_LAUNCH("lookup_bwd", KGE_CUDA(launch_lookup_bwd(shard, 1, rel_table, nullptr, (int)B, (int)D, cfg_.score_fn, lookup_type(), stream_)));
+        }
     }
     shards_join();
     KGE_CUDA(cudaGetLastError());
 
     // 5. segment sums + row-wise Adam, and the relation rows of the partial dense gradient
-    const bool gather_ahead = step + 1 < cfg_.n_step;
+    const bool gather_ahead = step + 1 < cfg_.n_step && !direct_rows_;
+    // with the table's own rows nothing reads the hidden rows' gradients but kge_debug_fetch, which shows the last step's
+    const bool keep_d_hid = !direct_rows_ || step + 1 == cfg_.n_step;
     const bool gather_beside = gather_ahead && (side_streams_ & 2u);
     shards_fork();
     for (unsigned l = 0; l < n_local_; ++l) {
@@ -1661,16 +1697,16 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                                                                dense_lr_mod_[0], b.loss_rows, (int)B, 1.0f / normaliser, d_loss_total_ + l, d_loss_last_ + l,
                                                                d_reg_loss_ ? d_reg_loss_ + 2 * l : nullptr}, l, step);
         const dim3 grid(kHeavySlots + ceil_div(R, kRowsPerBlock) + n_rel + 1), block(64 * kSegmentLanes);  // + the loss block
-#define KGE_ENTITY_UPDATE(ST_, EXTRAS_)                                                                                                          \
-    KGE_LAUNCH("entity_update", KGE_CUDA(launch_dependent(k_entity_update<ST_, 4, EXTRAS_>, grid, block, 0, stream_, b.table, b.rows_c2[parity], layout_, \
+#define KGE_ENTITY_UPDATE(ST_, ...)                                                                                                          \
+    KGE_LAUNCH("entity_update", KGE_CUDA(launch_dependent(k_entity_update<ST_, 4, __VA_ARGS__>, grid, block, 0, stream_, b.table, b.rows_c2[parity], layout_, \
                                          step_ptr(d_remote_, l, R), d_ent_perm_ + sidx * (B + T), d_ent_off_ + sidx * (R + 1), d_first_slot_ + sidx * R,      \
-                                         b.d_head, b.grad_recv, (int)B, b.d_hid_h, b.d_hid_t, d_step_size_ + step, entity_lr_mod_, adam_, sync, heavy,       \
+                                         b.d_head, b.grad_recv, (int)B, keep_d_hid ? b.d_hid_h : nullptr, b.d_hid_t, d_step_size_ + step, entity_lr_mod_, adam_, sync, heavy, \
                                          (int)R, rr)))
         const bool extras = cfg_.regularised() || dropout_on() || mlp_on();
         if (cfg_.state_type == ST_F32) {
-            if (extras) KGE_ENTITY_UPDATE(float, true); else KGE_ENTITY_UPDATE(float, false);
+            if (extras) KGE_ENTITY_UPDATE(float, true); else if (direct_rows_) KGE_ENTITY_UPDATE(float, false, true); else KGE_ENTITY_UPDATE(float, false);
         } else {
-            if (extras) KGE_ENTITY_UPDATE(__half, true); else KGE_ENTITY_UPDATE(__half, false);
+            if (extras) KGE_ENTITY_UPDATE(__half, true); else if (direct_rows_) KGE_ENTITY_UPDATE(__half, false, true); else KGE_ENTITY_UPDATE(__half, false);
         }
 #undef KGE_ENTITY_UPDATE
         if (gather_beside) launch_gather(step + 1, l, side_begin());

@@ -11,6 +11,7 @@
 #include "common.hpp"
 #include "host_io.hpp"
 #include "kernels.cuh"
+#include "lookup.cuh"
 #include "tc_gemm.cuh"
 #include "tc_planes.cuh"
 #include "transh.cuh"
@@ -190,6 +191,8 @@ class Engine {
                        const tc::RouteArgs* route = nullptr);
     void launch_step_planes(unsigned step, const LossParams& lp, float normaliser);
     void refresh_lower_plane(size_t offset, size_t count);
+    LookupRows lookup_rows(unsigned l, unsigned step) const;
+    int lookup_type() const;
     FeaturePlanes feature_planes(const ShardBuffers& b, unsigned parity) const;
     void check_device_status();
     void raise_device_status(const unsigned* words);
@@ -212,6 +215,7 @@ class Engine {
     cudaStream_t side_stream_ = nullptr;
     unsigned side_streams_ = 0;
     bool split_popular_rows_ = true;  // rows with many lookups are summed in parts by several blocks
+    bool direct_rows_ = false;        // lookups and row update read the table: no gathered copy, no hidden rows
     bool planes_ = false;             // the step's contractions run on the plane-fed tensor-core kernel
     bool bf16_planes_ = false;        // scores and their gradients multiply bfloat16 copies of their operands
     uint32_t feat_stride_ = 0;        // floats per row of the widened / lower feature planes
@@ -301,6 +305,7 @@ class Engine {
     uint32_t *d_ent_perm_ = nullptr, *d_ent_off_ = nullptr, *d_rel_perm_ = nullptr,
              *d_rel_off_ = nullptr, *d_first_slot_ = nullptr, *d_heavy_count_ = nullptr;
     uint4* d_heavy_parts_ = nullptr;
+    uint32_t* d_lookup_row_ = nullptr;  // [n_local * n_step][B + T] table rows by lookup (direct_rows_)
     uint4* d_row_info_ = nullptr;  // [n_local * n_step][R][2] per gathered row: offsets, flags, table row, first four lookups
     float *d_step_size_ = nullptr, *d_loss_total_ = nullptr, *d_loss_last_ = nullptr;
     unsigned* d_loss_counter_ = nullptr;

@@ -1264,7 +1264,8 @@ k_prepare_segments(const uint32_t* __restrict__ head, const uint32_t* __restrict
                    int T, int R, int n_rel, uint32_t* __restrict__ ent_perm,
                    uint32_t* __restrict__ ent_off, uint32_t* __restrict__ rel_perm,
                    uint32_t* __restrict__ rel_off, uint32_t* __restrict__ first_slot,
-                   uint4* __restrict__ heavy_parts, uint32_t* __restrict__ heavy_count, uint4* __restrict__ row_info) {
+                   uint4* __restrict__ heavy_parts, uint32_t* __restrict__ heavy_count, uint4* __restrict__ row_info,
+                   uint32_t* __restrict__ lookup_row) {
     __shared__ BlockSort bs;
     const int s = blockIdx.x;
     head += (size_t)s * B;
@@ -1276,6 +1277,8 @@ k_prepare_segments(const uint32_t* __restrict__ head, const uint32_t* __restrict
     rel_off += (size_t)s * (n_rel + 1);
 
     const int n = B + T;
+    if (lookup_row)  // the table row of every lookup, for a step whose lookups read the table
+        for (int i = threadIdx.x; i < n; i += blockDim.x) lookup_row[(size_t)s * n + i] = remote[(size_t)s * R + (i < B ? head[i] : a2a_idx[i - B])];
     for (int i = threadIdx.x; i < n; i += blockDim.x) bs.key[i] = min(i < B ? head[i] : a2a_idx[i - B], (uint32_t)R);  // lookups past the rows (an operator's caller may pass some): behind them
     __syncthreads();
     const uint16_t* sorted = bs.sort(n, bits_below((uint32_t)R + 1u));
@@ -1380,7 +1383,7 @@ k_prepare_segments(const uint32_t* __restrict__ head, const uint32_t* __restrict
 // update and the write-back (src/pag/pag.cpp:721-743; src/poplar_kge.cpp:695-704;
 // src/fructose/frnn.cpp:61-90).  One block per gathered row.  Every gathered row is
 // updated, rows with a zero gradient and the padding row included, as in the reference.
-// d_hid_h / d_hid_t keep the hidden-row gradients for the projection backward.
+// d_hid_h / d_hid_t keep the hidden-row gradients for the projection backward (null: there is none).
 //
 // Entity popularity is skewed: the shard that holds a step's most popular entity sees one row
 // with hundreds of lookups, and a single block would add them sixteen at a time while the rest of
@@ -1682,7 +1685,8 @@ __device__ __forceinline__ void relation_row_sum(const RelationRows& rr, int rho
 
 // EXTRAS: the regularisers' terms, the dropout masks and the deferred row update are compiled in
 // (they cost 20 registers, a third of the resident blocks, which the plain step does not pay).
-template <class ST, int V, bool EXTRAS = false>
+// DIRECT: the step makes no gathered copy; the state before the update is the table row, which only its first slot touches.
+template <class ST, int V, bool EXTRAS = false, bool DIRECT = false>
 __global__ void __launch_bounds__(64 * kSegmentLanes, EXTRAS ? 2 : 4)
 k_entity_update(uint8_t* __restrict__ table, const uint8_t* __restrict__ rows_c, RowLayout L,
                 const uint32_t* __restrict__ remote, const uint32_t* __restrict__ perm,
@@ -1742,14 +1746,16 @@ k_entity_update(uint8_t* __restrict__ table, const uint8_t* __restrict__ rows_c,
             slot_word = first_slot[r]; q0 = off[r]; q1 = off[r + 1]; row = remote[r];
         }
         if (slot_word & 2u) return;  // its lookups are summed part by part by the first blocks
+        if (!d_hid_h && !(slot_word & 1u)) return;  // a padding slot behind the first one, and nobody reads its gradient
     }
-    ST* __restrict__ xv = reinterpret_cast<ST*>(table + row * L.row_bytes);
-    ST* __restrict__ mv = reinterpret_cast<ST*>(table + row * L.row_bytes + L.off_m);
-    ST* __restrict__ qv = reinterpret_cast<ST*>(table + row * L.row_bytes + L.off_q);
+    ST* xv = reinterpret_cast<ST*>(table + row * L.row_bytes);
+    ST* mv = reinterpret_cast<ST*>(table + row * L.row_bytes + L.off_m);
+    ST* qv = reinterpret_cast<ST*>(table + row * L.row_bytes + L.off_q);
     // the state before the update comes from the step's gathered copy (slot r), not from the table
-    const ST* __restrict__ xs = reinterpret_cast<const ST*>(rows_c + (size_t)r * L.row_bytes);
-    const ST* __restrict__ ms = reinterpret_cast<const ST*>(rows_c + (size_t)r * L.row_bytes + L.off_m);
-    const ST* __restrict__ qs = reinterpret_cast<const ST*>(rows_c + (size_t)r * L.row_bytes + L.off_q);
+    const uint8_t* const state = DIRECT ? table + row * L.row_bytes : rows_c + (size_t)r * L.row_bytes;
+    const ST* xs = reinterpret_cast<const ST*>(state);
+    const ST* ms = reinterpret_cast<const ST*>(state + L.off_m);
+    const ST* qs = reinterpret_cast<const ST*>(state + L.off_q);
     const float alpha = *step_size * lr_modifier;
     const bool writes_row = (slot_word & 1u) != 0;
 
@@ -1838,7 +1844,9 @@ k_entity_update(uint8_t* __restrict__ table, const uint8_t* __restrict__ rows_c,
                 gt[u] = (keep_t >> bit) & 1u ? gt[u] * rr.drop.scale : 0.f;
             }
         }
-        if (V == 4) {
+        if (!d_hid_h) {
+            // no features: nothing reads the hidden rows' gradients
+        } else if (V == 4) {
             if (d_hid_t) {
                 const float4 a = make_float4(gh[0], gh[1 % V], gh[2 % V], gh[3 % V]), b = make_float4(gt[0], gt[1 % V], gt[2 % V], gt[3 % V]);
                 store4(d_hid_h + o, a);

@@ -1,0 +1,60 @@
+"""The training step in the forms its sizes choose: rows read straight from the table, widths around a warp's pieces."""
+
+import numpy as np
+import pytest
+
+from distributed_kge_poplar_b200 import capi
+from helpers import assert_close, engine_settings, make_oracle, random_batch, random_state, read_rows, read_state, write_state
+from oracle.step_oracle import StepConfig
+
+pytestmark = pytest.mark.gpu
+RW = 64
+
+
+def _config(score_fn, distance_fn, **sizes):
+    return StepConfig(**{**dict(n_shard=1, n_entity=300, n_relation_type=12, embedding_size=16, entity_feature_size=0, batch_size=8, a2a_size=16,
+                                score_fn=score_fn, distance_fn=distance_fn, gamma=6.0, loss_type="logsigmoid"), **sizes})
+
+
+def _two_runs(cfg, seed, rtol, rel_rtol=None, dtype="float32", n_step=2, pad=3, feature_dtype=None, **extra):
+    """Two program runs (plain launches, then graphs) against the oracle."""
+    store = np.float32 if dtype == "float32" else np.float16
+    state = random_state(cfg, seed, fp16_features=feature_dtype == "float16" or dtype == "float16", warm=True)
+    state["entity_data"] = state["entity_data"].astype(store).astype(np.float32)
+    engine = capi.CEngine(engine_settings(cfg, n_step=n_step, dtype=dtype, feature_dtype=feature_dtype, rw_batch=RW, **extra))
+    write_state(engine, cfg, state, RW, dtype=store)
+    oracle = make_oracle(cfg, state)
+    for run in range(2):
+        batch = random_batch(cfg, n_step, seed + 1 + run, pad=pad)
+        want = oracle.train_step_loop(1e-3, batch)
+        got = np.zeros(cfg.n_shard, np.float32)
+        engine.run("train_step_loop", dict(learning_rate=np.full(cfg.n_shard, 1e-3, np.float32), loss=got, **batch))
+        assert_close(got, want, rtol, f"loss of run {run}", atol_scale=0)
+    want, d = oracle.get_state(), cfg.embedding_size
+    got = read_state(engine, cfg, RW, cfg.n_shard) if dtype == "float32" else dict(entity_data=read_rows(engine, cfg, RW, cfg.n_shard, store).astype(np.float32))
+    hidden = [engine.debug_fetch("hidden", s, cfg.n_remote * d).reshape(-1, d) for s in range(cfg.n_shard)]
+    d_hidden = [engine.debug_fetch("d_hidden", s, cfg.n_remote * d).reshape(-1, d) for s in range(cfg.n_shard)]
+    raw = [engine.debug_fetch("raw_score", s, cfg.batch_size * cfg.n_tail).reshape(cfg.batch_size, -1) for s in range(cfg.n_shard)]
+    engine.close()
+    for s in range(cfg.n_shard):
+        assert_close(hidden[s], oracle.last["hidden"][s], rtol, f"hidden[{s}]")
+        scores = cfg.gamma - raw[s] if cfg.score_fn in ("TransE", "RotatE", "TransH") else raw[s]
+        assert_close(scores, oracle.last["scores"][s], rtol, f"scores[{s}]")
+        if cfg.share_feature_networks and cfg.distance_fn != "L1":
+            assert_close(d_hidden[s], oracle.last["d_feature_hidden"][s], rtol, f"d hidden[{s}]")
+    assert_close(got["entity_data"][..., : 3 * d], want["entity_data"][..., : 3 * d], rtol, "rows")
+    for key in set(got) & set(want) - {"entity_data", "step"}:
+        assert_close(got[key], want[key], (rel_rtol if key.startswith("relation") else None) or rtol, key)
+
+
+# the bounds of several steps of the other step tests: 1e-4, and 2e-3 where relation gradients pass through float16
+@pytest.mark.parametrize("score_fn,distance_fn", [("TransE", "L1"), ("TransE", "L2"), ("DistMult", "MatMul"), ("ComplEx", "MatMul"), ("RotatE", "L2")])
+@pytest.mark.parametrize("d", [4, 36, 132, 516])
+def test_rows_straight_from_the_table(score_fn, distance_fn, d):
+    """Without features: a row of one piece, of a warp's pieces and a remainder, and of more than a lane keeps in flight."""
+    _two_runs(_config(score_fn, distance_fn, embedding_size=d), seed=d, rtol=1e-4, rel_rtol=2e-3 if score_fn == "RotatE" else None)
+
+
+def test_rows_straight_from_a_float16_table():
+    # float16 rows: the bound of the other float16 tests
+    _two_runs(_config("ComplEx", "MatMul", embedding_size=36, n_shard=2), seed=5, rtol=2e-2, dtype="float16")
