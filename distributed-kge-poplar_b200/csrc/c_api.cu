@@ -330,12 +330,14 @@ int kge_op_all_to_all(const float* in, size_t n_shard, size_t block, float* out)
             for (size_t d = 0; d < n_shard; ++d) dst[d] = dout.as<float>() + (d * n_shard + s) * block;
             to_device(dtable, dst.data(), n_shard * sizeof(float*));
             const float* rows = din.as<float>() + s * n_shard * block;
-            if (block % 4 == 0)
-                k_route<4><<<(unsigned)n_shard, 64>>>(rows, rows, didx.as<uint32_t>(), nullptr, nullptr, nullptr,
-                                                      dtable.as<float*>(), nullptr, (int)n_shard, 1, 0, (int)block, SCORE_TRANSE, ExchangeSync{});
-            else
-                k_route<1><<<(unsigned)n_shard, 64>>>(rows, rows, didx.as<uint32_t>(), nullptr, nullptr, nullptr,
-                                                      dtable.as<float*>(), nullptr, (int)n_shard, 1, 0, (int)block, SCORE_TRANSE, ExchangeSync{});
+            ShardArgs<LookupArgs> lookups{};
+            lookups.s[0].rows = LookupRows{nullptr, reinterpret_cast<const uint8_t*>(rows), nullptr, didx.as<uint32_t>(), block * 4};
+            lookups.s[0].send_dst = dtable.as<float*>();
+            LookupSizes sizes{};
+            sizes.T = (int)n_shard;
+            sizes.a2a = 1;
+            sizes.D = (int)block;
+            KGE_CUDA(launch_lookup(lookups, 1, sizes, SCORE_TRANSE, 0, nullptr));
             finish_kernels();
         }
         to_host(out, dout, total * 4);
@@ -578,11 +580,9 @@ int kge_microbench_rows(int kind, size_t table_rows, size_t d, const uint32_t* i
         k_fill_pattern<<<1184, 256>>>(table.as<float>(), table_rows * 3 * d, 1u);
         KGE_CUDA(cudaGetLastError());
         to_device(idx, indices, n * 4);
-        const FeaturePlanes no_planes{nullptr, nullptr, 0u, L.off_feat};
-        auto gather = [&] {
-            return launch_dependent(k_gather_step_rows, dim3(blocks_for(n, 8)), dim3(256), 0, nullptr, table.as<uint8_t>(), L.row_bytes,
-                                    idx.as<uint32_t>(), (int)n, rows_c.as<uint8_t>(), no_planes);
-        };
+        ShardArgs<GatherArgs> rows{};
+        rows.s[0] = GatherArgs{table.as<uint8_t>(), idx.as<uint32_t>(), rows_c.as<uint8_t>(), FeaturePlanes{nullptr, nullptr, 0u, L.off_feat}};
+        auto gather = [&] { return launch_dependent(k_gather_step_rows, dim3(blocks_for(n, 8)), dim3(256), 0, nullptr, rows, L.row_bytes, (int)n); };
         if (kind == 0) {
             *mean_us = timed_launches(repeat, gather);
             return;
@@ -609,13 +609,25 @@ int kge_microbench_rows(int kind, size_t table_rows, size_t d, const uint32_t* i
         }
         DeviceBuffer row_info(2 * n * sizeof(uint4));
         to_device(row_info, info.data(), 2 * n * sizeof(uint4));
-        const HeavyRows heavy{nullptr, heavy_count.as<uint32_t>(), nullptr, nullptr, row_info.as<uint4>()};
-        *mean_us = timed_launches(repeat, [&] {
-            return launch_dependent(k_entity_update<float, 4>, dim3((unsigned)(kHeavySlots + blocks_for(n, kRowsPerBlock))), dim3(64 * kSegmentLanes), 0, nullptr, table.as<uint8_t>(),
-                                    rows_c.as<uint8_t>(), L, idx.as<uint32_t>(), perm.as<uint32_t>(), off.as<uint32_t>(), first.as<uint32_t>(),
-                                    grads.as<float>(), grads.as<float>(), (int)n, d_hid.as<float>(), (float*)nullptr, step_size.as<float>(), 1.0f, ap,
-                                    ExchangeSync{}, heavy, (int)n, RelationRows{});
-        });
+        ShardArgs<EntityShard> shard{};
+        EntityShard& u = shard.s[0];
+        u.table = table.as<uint8_t>();
+        u.rows_c = rows_c.as<uint8_t>();
+        u.remote = idx.as<uint32_t>();
+        u.perm = perm.as<uint32_t>();
+        u.off = off.as<uint32_t>();
+        u.first_slot = first.as<uint32_t>();
+        u.d_head = u.grad_recv = grads.as<float>();
+        u.d_hid_h = d_hid.as<float>();
+        u.heavy = HeavyRows{nullptr, heavy_count.as<uint32_t>(), nullptr, nullptr, row_info.as<uint4>()};
+        EntityStep step{};
+        step.L = L;
+        step.B = step.R = (int)n;
+        step.n_shards = 1;
+        step.step_size = step_size.as<float>();
+        step.lr_modifier = 1.0f;
+        step.ap = ap;
+        *mean_us = timed_launches(repeat, [&] { return launch_entity_update<float, 4>(shard, step, nullptr); });
     });
 }
 

@@ -371,23 +371,23 @@ Engine::Engine(const SettingMap& settings) : cfg_(parse_config(settings)) {
     for (cudaEvent_t& e : ev_join_) KGE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (RunEvents& r : ev_runs_)
         for (cudaEvent_t* e : {&r.begin, &r.end, &r.stage[0], &r.stage[1]}) KGE_CUDA(cudaEventCreate(e));
-    // The plane-fed contraction needs 16-byte rows in every operand and the lookups of a block of
-    // hidden rows to fit its staging area.
-    planes_ = cfg_.tensor_cores && cfg_.d % 4 == 0 && cfg_.batch_size % 4 == 0 && cfg_.n_tail() % 4 == 0 &&
-              cfg_.n_remote() <= (unsigned)tc::kRouteMaxLookups;
+    // The step of batched launches: rows of 16 bytes, which its contractions' operands need, and lookups of a block of hidden
+    // rows that fit its staging area.  Scores and coefficients get rows of a multiple of eight, so that any batch will do.
+    planes_ = cfg_.tensor_cores && cfg_.d % 4 == 0 && cfg_.n_remote() <= (unsigned)tc::kRouteMaxLookups;
     if (const char* v = std::getenv("KGE_PLANE_CONTRACTIONS")) planes_ = planes_ && std::atoi(v) != 0;
     if (mlp_on()) planes_ = false;  // the MLP sits between the projection and the lookups: the step of separate kernels
-    if (cfg_.score_fn == SCORE_TRANSH) {
-        planes_ = false;  // its score has no contraction form: the step of separate kernels
-    }
+    score_ld_ = planes_ ? (unsigned)round_up(cfg_.n_tail(), 8) : cfg_.n_tail();
     // Without features a hidden row is the stored value: the lookups and the row update read the table itself.
     direct_rows_ = planes_ && cfg_.f == 0 && !cfg_.regularised();
-    // With one shard in all a dense gradient has a single contributor: the projection gradient's contraction and the
-    // relation rows' blocks of the entity update apply the Adam step themselves and k_dense_update is not launched.
-    fuse_dense_ = fuse_dense_env_ && planes_ && cfg_.n_shard == 1 && cfg_.world == 1;
+    // Shards of one launch.  With several processes the hand-over counters count the blocks of one shard's kernel at a time.
+    group_ = cfg_.world == 1 ? std::min(n_local_, (unsigned)kShardBatch) : 1u;
+    // Where every shard is in every launch no gradient has to wait for another launch: the projection gradient's
+    // contraction (over all shards' rows) and the relation rows' blocks of the entity update apply the Adam step
+    // themselves and k_dense_update is not launched.
+    fuse_dense_ = fuse_dense_env_ && planes_ && cfg_.world == 1 && cfg_.n_shard <= (unsigned)kShardBatch;
     // fp16 features are widened into rows of their own; the lower plane of fp32 features keeps the
     // stride of the rows whose feature part is its upper plane (one stride per operand)
-    bf16_planes_ = planes_ && cfg_.value_bf16 && cfg_.dist_fn == DIST_DOT && cfg_.d % 8 == 0 && cfg_.n_tail() % 8 == 0 && cfg_.batch_size % 8 == 0 &&
+    bf16_planes_ = planes_ && cfg_.value_bf16 && cfg_.dist_fn == DIST_DOT && cfg_.score_fn != SCORE_TRANSH && cfg_.d % 8 == 0 && cfg_.n_tail() % 8 == 0 && cfg_.batch_size % 8 == 0 &&
                    (cfg_.a2a_size * cfg_.d) % 2 == 0;
     feat_stride_ = cfg_.feature_type == ST_F16 ? (uint32_t)round_up(cfg_.f, 4) : layout_.row_bytes / 4;
     allocate();
@@ -434,16 +434,34 @@ void Engine::allocate() {
     table_stride_ = round_up((size_t)cfg_.n_entity * layout_.row_bytes, 256);
     uint8_t* tables = (uint8_t*)device_alloc(n_local_ * table_stride_);
     KGE_CUDA(cudaMemset(tables, 0, n_local_ * table_stride_));
+    const size_t score_elems = (size_t)B * score_ld_;
+    // what the projection's gradient contracts over lies shard behind shard, one operand for all of them
+    uint8_t* rows_all[2] = {nullptr, nullptr};
+    float *wide_all[2] = {nullptr, nullptr}, *lo_all[2] = {nullptr, nullptr}, *d_hid_all[2] = {nullptr, nullptr}, *d_hid_lo_all[2] = {nullptr, nullptr};
+    for (int i = 0; i < 2; ++i) {
+        if (!direct_rows_) rows_all[i] = (uint8_t*)device_alloc((size_t)n_local_ * R * layout_.row_bytes);
+        if (planes_ && cfg_.f) (cfg_.feature_type == ST_F16 ? wide_all : lo_all)[i] = (float*)device_alloc((size_t)n_local_ * R * feat_stride_ * 4);
+        if (i == 1 && !two_nets) continue;
+        d_hid_all[i] = (float*)device_alloc((size_t)n_local_ * R * D * 4);
+        if (planes_ && cfg_.f) d_hid_lo_all[i] = (float*)device_alloc((size_t)n_local_ * R * D * 4);
+    }
     for (unsigned l = 0; l < n_local_; ++l) {
         ShardBuffers& b = shards_[l];
         b.table = tables + l * table_stride_;
-        if (!direct_rows_)
-            for (uint8_t*& rows : b.rows_c2) rows = (uint8_t*)device_alloc((size_t)R * layout_.row_bytes);
+        for (int i = 0; i < 2; ++i) {
+            if (rows_all[i]) b.rows_c2[i] = rows_all[i] + (size_t)l * R * layout_.row_bytes;
+            if (wide_all[i]) b.feat_wide2[i] = wide_all[i] + (size_t)l * R * feat_stride_;
+            if (lo_all[i]) b.feat_lo2[i] = lo_all[i] + (size_t)l * R * feat_stride_;
+        }
+        b.d_hid_h = d_hid_all[0] + (size_t)l * R * D;
+        if (d_hid_all[1]) b.d_hid_t = d_hid_all[1] + (size_t)l * R * D;
+        if (d_hid_lo_all[0]) b.d_hid_h_lo = d_hid_lo_all[0] + (size_t)l * R * D;
+        if (d_hid_lo_all[1]) b.d_hid_t_lo = d_hid_lo_all[1] + (size_t)l * R * D;
         b.hid_h = (float*)device_alloc((size_t)R * D * 4);
         b.hid_t = two_nets || dropout_on() ? (float*)device_alloc((size_t)R * D * 4) : b.hid_h;  // dropout: each call has its own mask
         b.pred = (float*)device_alloc((size_t)B * D * 4);
-        b.raw = (float*)device_alloc((size_t)B * T * 4);
-        b.coeff = (float*)device_alloc((size_t)B * T * 4);
+        b.raw = (float*)device_alloc(score_elems * 4);
+        b.coeff = (float*)device_alloc(score_elems * 4);
         b.d_pred = (float*)device_alloc((size_t)B * D * 4);
         b.d_head = multiplicative ? (float*)device_alloc((size_t)B * D * 4) : b.d_pred;
         b.d_relrow = multiplicative ? (float*)device_alloc((size_t)B * D * 4) : b.d_pred;
@@ -464,8 +482,11 @@ void Engine::allocate() {
             b.nrm = (float*)device_alloc((size_t)B * D * 4);
             b.d_nrm = (float*)device_alloc((size_t)B * D * 4);
             b.d_normrow = (float*)device_alloc((size_t)B * D * 4);
-            b.pair_s = (float*)device_alloc((size_t)B * T * 4);
-            b.pair_u = (float*)device_alloc((size_t)B * T * 4);
+            b.pair_s = (float*)device_alloc(score_elems * 4);
+            b.pair_u = (float*)device_alloc(score_elems * 4);
+            // (what lies behind a row's last column is multiplied with coefficients of zero)
+            KGE_CUDA(cudaMemset(b.pair_s, 0, score_elems * 4));
+            KGE_CUDA(cudaMemset(b.pair_u, 0, score_elems * 4));
         }
         if (cfg_.regularised()) {
             b.reg_val = (float*)device_alloc((size_t)R * D * 4);
@@ -473,8 +494,6 @@ void Engine::allocate() {
             b.reg_t = two_nets || dropout_on() ? (float*)device_alloc((size_t)R * D * 4) : nullptr;
             b.reg_loss_rows = (float*)device_alloc((size_t)R * 4);
         }
-        b.d_hid_h = (float*)device_alloc((size_t)R * D * 4);
-        b.d_hid_t = two_nets ? (float*)device_alloc((size_t)R * D * 4) : nullptr;
         b.proj_partial = (float*)device_alloc(std::max<size_t>(1, cfg_.n_net()) * proj_splits_ * proj_elems_ * 4);
         b.loss_rows = (float*)device_alloc((size_t)B * 4);
         b.tails = (float*)(arena_ + arena_offset_shard(l, 0));
@@ -489,14 +508,8 @@ void Engine::allocate() {
         b.send_lo_dst = (float**)device_alloc(sizeof(float*) * cfg_.n_shard);
         b.tails_lo = (float*)(arena_ + arena_offset_shard(l, 2));
         if (planes_) {
-            for (int par = 0; par < 2; ++par) {
-                if (cfg_.feature_type == ST_F16) b.feat_wide2[par] = (float*)device_alloc((size_t)R * feat_stride_ * 4);
-                else b.feat_lo2[par] = (float*)device_alloc((size_t)R * feat_stride_ * 4);
-            }
             b.pred_lo = (float*)device_alloc((size_t)B * D * 4);
-            b.coeff_lo = (float*)device_alloc((size_t)B * T * 4);
-            b.d_hid_h_lo = (float*)device_alloc((size_t)R * D * 4);
-            b.d_hid_t_lo = two_nets ? (float*)device_alloc((size_t)R * D * 4) : nullptr;
+            b.coeff_lo = (float*)device_alloc(score_elems * 4);
         }
         b.predict_score_dst = (float**)device_alloc(sizeof(float*) * cfg_.n_shard);
         b.predict_index_dst = (uint32_t**)device_alloc(sizeof(uint32_t*) * cfg_.n_shard);
@@ -1015,6 +1028,13 @@ void Engine::last_run_stats(float* ms, unsigned long long* launches) const {
         ++launch_counter_;               \
     } while (0)
 
+// The same for a launch that works on `n` local shards, which counts as the n kernels it stands for.
+#define KGE_LAUNCH_SHARDS(name, n, ...)  \
+    do {                                 \
+        KGE_LAUNCH(name, __VA_ARGS__);   \
+        launch_counter_ += (n) - 1u;     \
+    } while (0)
+
 bool dependent_launch_enabled() {
     static const bool enabled = [] {
         const char* off = std::getenv("KGE_NO_DEPENDENT_LAUNCH");
@@ -1069,7 +1089,7 @@ class StreamPool {
 // steps, or until the steps themselves are over: StreamPool serves every engine of the process, and an engine on another
 // thread may borrow a stream the moment it is back.  After an error they are destroyed, not lent again.
 Engine::ShardStreams::ShardStreams(Engine& e) : engine_(e) {
-    if (e.n_local_ < 2 || e.cfg_.world > 1 || e.kernel_timing_) return;
+    if (e.n_local_ < 2 || e.cfg_.world > 1 || e.kernel_timing_ || e.planes_) return;
     e.shard_streams_.assign(e.n_local_, nullptr);
     for (unsigned l = 1; l < e.n_local_; ++l) e.shard_streams_[l] = StreamPool::instance().take();
 }
@@ -1160,15 +1180,17 @@ void Engine::launch_steps(unsigned first, unsigned end) {
 // copies, for even and odd steps).  The gather of step s + 1 needs only the rows step s has
 // updated, so it runs beside the projection gradient and the dense update of step s.
 void Engine::launch_gather(unsigned step, cudaStream_t stream) {
-    for (unsigned l = 0; l < n_local_; ++l) launch_gather(step, l, stream);
+    for (unsigned l = 0; l < n_local_; l += group_) launch_gather(step, l, std::min(group_, n_local_ - l), stream);
 }
-void Engine::launch_gather(unsigned step, unsigned l, cudaStream_t stream) {
+void Engine::launch_gather(unsigned step, unsigned l0, unsigned n, cudaStream_t stream) {
     if (direct_rows_) return;
     const unsigned R = cfg_.n_remote();
-    ShardBuffers& b = shards_[l];
-    const uint32_t* remote = d_remote_ + ((size_t)l * cfg_.n_step + step) * R;
-    KGE_LAUNCH("gather", KGE_CUDA(launch_dependent(k_gather_step_rows, dim3(ceil_div(R, 8)), dim3(256), 0, stream, b.table,
-                                                   layout_.row_bytes, remote, (int)R, b.rows_c2[step & 1], feature_planes(b, step & 1))));
+    ShardArgs<GatherArgs> shards{};
+    for (unsigned i = 0; i < n; ++i) {
+        const ShardBuffers& b = shards_[l0 + i];
+        shards.s[i] = GatherArgs{b.table, d_remote_ + ((size_t)(l0 + i) * cfg_.n_step + step) * R, b.rows_c2[step & 1], feature_planes(b, step & 1)};
+    }
+    KGE_LAUNCH_SHARDS("gather", n, KGE_CUDA(launch_dependent(k_gather_step_rows, dim3(ceil_div(R, 8), n), dim3(256), 0, stream, shards, layout_.row_bytes, (int)R)));
 }
 
 FeaturePlanes Engine::feature_planes(const ShardBuffers& b, unsigned parity) const {
@@ -1335,11 +1357,11 @@ void Engine::launch_tc(const char* name, tc::GemmArgs* problems, int n_problems,
     KGE_CUDA(err);
 }
 
-// One launch of the plane-fed contraction for one or two problems of the same shape class.  Tiles
+// One launch of the plane-fed contraction for problems of the same shape class, those of `n_shards` local shards.  Tiles
 // are 128 x 128 (128 x 64 for narrow outputs); the k range is split over the blocks of a cluster so
 // that about one block per SM is busy and every split keeps at least two 32-deep slices.
 void Engine::launch_planes(const char* name, tc::PlaneProblem* problems, int n_problems, int side, int wait_kind, int signal_kind,
-                           const tc::RouteArgs* route) {
+                           const tc::Routing* routing, unsigned n_shards) {
     int max_n = 0, max_k = 0;
     unsigned tiles = 0;
     for (int i = 0; i < n_problems; ++i) max_n = std::max(max_n, problems[i].g.N);
@@ -1361,11 +1383,11 @@ void Engine::launch_planes(const char* name, tc::PlaneProblem* problems, int n_p
     }
     timing_begin(name);
     cudaError_t err;
-    if (side == tc::SIDE_ROWSUM) err = tc::launch_planes<tc::SIDE_ROWSUM>(problems, n_problems, splits, tile_n, stream_, exchange_sync(), wait_kind, signal_kind, route);
-    else if (side == tc::SIDE_NORMS) err = tc::launch_planes<tc::SIDE_NORMS>(problems, n_problems, splits, tile_n, stream_, exchange_sync(), wait_kind, signal_kind, route);
-    else err = tc::launch_planes<tc::SIDE_NONE>(problems, n_problems, splits, tile_n, stream_, exchange_sync(), wait_kind, signal_kind, route);
+    if (side == tc::SIDE_ROWSUM) err = tc::launch_planes<tc::SIDE_ROWSUM>(problems, n_problems, splits, tile_n, stream_, exchange_sync(), wait_kind, signal_kind, routing);
+    else if (side == tc::SIDE_NORMS) err = tc::launch_planes<tc::SIDE_NORMS>(problems, n_problems, splits, tile_n, stream_, exchange_sync(), wait_kind, signal_kind, routing);
+    else err = tc::launch_planes<tc::SIDE_NONE>(problems, n_problems, splits, tile_n, stream_, exchange_sync(), wait_kind, signal_kind, routing);
     timing_end();
-    ++launch_counter_;
+    launch_counter_ += n_shards;
     KGE_CUDA(err);
 }
 
@@ -1459,16 +1481,6 @@ void Engine::launch_regularise(unsigned l, const uint8_t* rows_c) {
                                                            b.hid_t, (int)R, rp, b.reg_val, b.reg_h, b.reg_t, b.reg_loss_rows, loss, loss + 1, d_reg_counter_ + l)));
 }
 
-RelationRows Engine::with_regularisers(RelationRows rr, unsigned l, unsigned step) const {
-    const ShardBuffers& b = shards_[l];
-    rr.reg_val = b.reg_val;
-    rr.reg_h = b.reg_h;
-    rr.reg_t = b.reg_t;
-    rr.drop = dropout_params(l, step);
-    rr.defer_grad = b.d_val;
-    return rr;
-}
-
 DropoutParams Engine::dropout_params(unsigned l, unsigned step) const {
     DropoutParams dp{};
     if (!dropout_on()) return dp;
@@ -1506,15 +1518,142 @@ LookupRows Engine::lookup_rows(unsigned l, unsigned step) const {
 }
 int Engine::lookup_type() const { return !direct_rows_ ? 0 : cfg_.value_bf16 ? 2 : cfg_.state_type == ST_F16 ? 1 : 0; }
 
-// The training step with its contractions on the plane-fed kernel: seven launches on the step's
-// chain (hidden + lookups + send, scores, loss, score gradients + return, segment sums + Adam +
-// relation gradients, projection gradient, dense update) and the next step's gather beside the
-// last two.  Every operand of a contraction is the fp32 array its producer wrote (the upper TF32
-// plane) plus a lower plane the same producer wrote next to it.
+// Lookups, predicted tails and the send half of the exchange for local shards whose hidden rows are ready.
+void Engine::launch_lookup(unsigned l0, unsigned n, unsigned step) {
+    const bool companion = planes_ && cfg_.dist_fn != DIST_L1 && cfg_.score_fn != SCORE_TRANSH;  // contractions read pred and tails
+    const size_t B = cfg_.batch_size, R = cfg_.n_remote();
+    LookupSizes sizes{};
+    sizes.rel_table = dense_;
+    sizes.normal_table = dense_ + dense_bounds_[3];
+    sizes.B = (int)B; sizes.T = (int)cfg_.n_tail(); sizes.a2a = (int)cfg_.a2a_size; sizes.D = (int)cfg_.d; sizes.R = (int)R;
+    sizes.lo_bf16 = bf16_planes_ ? 1 : 0;
+    sizes.prefetch = direct_rows_ && step > 0;  // the first step's index streams come from the kernel in front
+    sizes.sync = exchange_sync();
+    ShardArgs<LookupArgs> shards{};
+    for (unsigned i = 0; i < n; ++i) {
+        const ShardBuffers& b = shards_[l0 + i];
+        const size_t sidx = (size_t)(l0 + i) * cfg_.n_step + step;
+        LookupArgs& a = shards.s[i];
+        a.rows = lookup_rows(l0 + i, step);
+        a.relation = d_relation_ + sidx * B;
+        a.send_dst = b.send_dst;
+        a.send_lo_dst = companion ? b.send_lo_dst : nullptr;
+        a.pred = b.pred;
+        a.pred_lo = companion ? b.pred_lo : nullptr;
+        a.nrm = b.nrm;
+        if (direct_rows_ && step + 1 == cfg_.n_step) {  // kge_debug_fetch shows the last step's hidden rows
+            a.remote = d_remote_ + sidx * R;
+            a.hid = b.hid_h;
+        }
+    }
+    KGE_LAUNCH_SHARDS("lookup", n, KGE_CUDA(kge::launch_lookup(shards, (int)n, sizes, cfg_.score_fn, lookup_type(), stream_)));
+}
+
+void Engine::launch_lookup_bwd(unsigned l0, unsigned n, unsigned step) {
+    const size_t B = cfg_.batch_size;
+    ShardArgs<LookupBwdArgs> shards{};
+    for (unsigned i = 0; i < n; ++i) {
+        const ShardBuffers& b = shards_[l0 + i];
+        shards.s[i] = LookupBwdArgs{lookup_rows(l0 + i, step), d_relation_ + ((size_t)(l0 + i) * cfg_.n_step + step) * B, b.d_pred, b.d_head, b.d_relrow, b.nrm, b.d_nrm, b.d_normrow};
+    }
+    KGE_LAUNCH_SHARDS("lookup_bwd", n, KGE_CUDA(kge::launch_lookup_bwd(shards, (int)n, dense_, dense_ + dense_bounds_[3], (int)B, (int)cfg_.d, cfg_.score_fn, lookup_type(), stream_)));
+}
+
+ShardArgs<TranshScoreArgs> Engine::transh_scores(unsigned l0, unsigned n) const {
+    ShardArgs<TranshScoreArgs> shards{};
+    for (unsigned i = 0; i < n; ++i) {
+        const ShardBuffers& b = shards_[l0 + i];
+        shards.s[i] = TranshScoreArgs{b.pred, b.nrm, b.tails, b.raw, b.pair_s, b.pair_u};
+    }
+    return shards;
+}
+ShardArgs<TranshBwdArgs> Engine::transh_gradients(unsigned l0, unsigned n) const {
+    ShardArgs<TranshBwdArgs> shards{};
+    for (unsigned i = 0; i < n; ++i) {
+        const ShardBuffers& b = shards_[l0 + i];
+        shards.s[i] = TranshBwdArgs{b.pred, b.nrm, b.tails, b.coeff, b.pair_s, b.pair_u, b.d_pred, b.d_nrm, b.grad_dst,
+                                    (int)cfg_.a2a_size, (int)cfg_.batch_size, (int)cfg_.n_tail(), (int)cfg_.d, (int)score_ld_, 0};
+    }
+    return shards;
+}
+
+EntityShard Engine::entity_shard(unsigned l, unsigned step, bool keep_d_hid) const {
+    const ShardBuffers& b = shards_[l];
+    const size_t B = cfg_.batch_size, T = cfg_.n_tail(), R = cfg_.n_remote(), sidx = (size_t)l * cfg_.n_step + step;
+    EntityShard e{};
+    e.table = b.table;
+    e.rows_c = b.rows_c2[step & 1];
+    e.remote = d_remote_ + sidx * R;
+    e.perm = d_ent_perm_ + sidx * (B + T);
+    e.off = d_ent_off_ + sidx * (R + 1);
+    e.first_slot = d_first_slot_ + sidx * R;
+    e.d_head = b.d_head;
+    e.grad_recv = b.grad_recv;
+    if (keep_d_hid) {
+        e.d_hid_h = b.d_hid_h;
+        e.d_hid_t = b.d_hid_t;
+        e.d_hid_h_lo = planes_ ? b.d_hid_h_lo : nullptr;
+        e.d_hid_t_lo = planes_ ? b.d_hid_t_lo : nullptr;
+    }
+    e.heavy = HeavyRows{d_heavy_parts_ + sidx * kHeavySlots, d_heavy_count_ + sidx, b.heavy_partial, b.heavy_counter, d_row_info_ + sidx * 2 * R};
+    e.reg_val = b.reg_val;
+    e.reg_h = b.reg_h;
+    e.reg_t = b.reg_t;
+    e.drop = dropout_params(l, step);
+    e.defer_grad = b.d_val;
+    if (planes_) {
+        e.d_relrow[0] = b.d_relrow;
+        e.d_relrow[1] = b.d_normrow;
+        e.rel_perm = d_rel_perm_ + sidx * B;
+        e.rel_off = d_rel_off_ + sidx * (cfg_.n_relation_type + 1);
+        e.dense_dst = b.dense_dst;
+        e.loss_rows = b.loss_rows;
+        e.loss_total = d_loss_total_ + l;
+        e.loss_last = d_loss_last_ + l;
+        e.extra_loss = d_reg_loss_ ? d_reg_loss_ + 2 * l : nullptr;
+    }
+    return e;
+}
+EntityStep Engine::entity_step(unsigned step, unsigned n) const {
+    EntityStep g{};
+    g.L = layout_;
+    g.B = (int)cfg_.batch_size;
+    g.R = (int)cfg_.n_remote();
+    g.n_shards = (int)n;
+    g.step_size = d_step_size_ + step;
+    g.lr_modifier = entity_lr_mod_;
+    g.ap = adam_;
+    g.sync = exchange_sync();
+    if (planes_) {
+        const int parameter[2] = {0, 3};  // the relation table and TransH's normals
+        g.n_rel = (int)cfg_.n_relation_type;
+        g.n_tables = cfg_.score_fn == SCORE_TRANSH ? 2 : 1;
+        g.n_owner = (int)cfg_.world;
+        const unsigned rows = (unsigned)(g.n_rel * g.n_tables);
+        g.rel_blocks = (int)(fuse_dense_ ? ceil_div(rows, n) : rows);
+        for (int t = 0; t < g.n_tables; ++t) {
+            const size_t at = dense_bounds_[parameter[t]];
+            g.dense_row0[t] = (int)(at / cfg_.d);
+            g.rel_lr_modifier[t] = dense_lr_mod_[parameter[t]];
+            if (fuse_dense_) g.rel_w[t] = dense_ + at, g.rel_m[t] = dense_m_ + at, g.rel_v[t] = dense_v_ + at;
+        }
+    }
+    return g;
+}
+
+// The training step of batched launches: six to nine on the step's chain (hidden rows, lookups + send, scores, loss, score
+// gradients + return, the prediction's backward, segment sums + Adam + relation gradients, projection gradient, dense
+// update; what a model has no use for is left out, and the lookups of the elementwise score functions are the hidden
+// kernel's epilogue) and the next step's gather beside the last two.  Every launch works on all local shards, which meet
+// at the exchange (the tails and the tails' gradients), and every operand of a contraction is the fp32 array its producer
+// wrote (the upper TF32 plane) plus a lower plane the same producer wrote next to it.
+// With a stream per shard instead, forked and joined three times a step, and a dense update of its own (us per step,
+// before -> after): demo preset, 2 shards, 40.4 -> 32.3; four shards of 256 x 320 L1 scores, 76.4 -> 67.2; four of 256 x 512
+// fp16 rows, 79.4 -> 83.1; two shards of the headline step 129.5 -> 112.9.
 void Engine::launch_step_planes(unsigned step, const LossParams& lp, float normaliser) {
     const unsigned B = cfg_.batch_size, T = cfg_.n_tail(), R = cfg_.n_remote(), D = cfg_.d, F = cfg_.f;
-    const unsigned n_rel = cfg_.n_relation_type, parity = step & 1;
-    const bool two_nets = cfg_.n_net() == 2, l2 = cfg_.dist_fn == DIST_L2, l1 = cfg_.dist_fn == DIST_L1;
+    const unsigned n_rel = cfg_.n_relation_type, parity = step & 1, n_nets = cfg_.n_net(), ld = score_ld_;
+    const bool transh = cfg_.score_fn == SCORE_TRANSH, dot = cfg_.dist_fn == DIST_DOT && !transh, l2 = cfg_.dist_fn == DIST_L2 && !transh;
     // bf16 embeddings: the dot-product scores and their gradients multiply bfloat16 copies of pred,
     // tails and the coefficients (written by their producers into the companion planes)
     const bool bf16 = bf16_planes_;
@@ -1522,249 +1661,234 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
         return tc::PlaneOperand{values, nullptr, row_elems * 2, mn_major ? 1 : 0, 2};
     };
     const bool half_features = cfg_.feature_type == ST_F16;
-    const float* rel_table = dense_;
     const ExchangeSync sync = exchange_sync();
     auto step_ptr = [&](uint32_t* base, unsigned l, size_t per_step) { return base + ((size_t)l * cfg_.n_step + step) * per_step; };
     auto plane = [](const float* hi, const float* lo, long long stride_bytes, bool mn_major) {
-        return tc::PlaneOperand{hi, lo, stride_bytes, mn_major ? 1 : 0};
+        return tc::PlaneOperand{hi, lo, stride_bytes, mn_major ? 1 : 0, 0};
     };
     auto features = [&](const ShardBuffers& b, bool mn_major) {
         if (half_features) return plane(b.feat_wide2[parity], nullptr, (long long)feat_stride_ * 4, mn_major);
         return plane(reinterpret_cast<const float*>(b.rows_c2[parity] + layout_.off_feat), b.feat_lo2[parity], (long long)layout_.row_bytes, mn_major);
     };
+    tc::PlaneProblem problems[tc::kMaxPlaneProblems];
 
-    shards_fork();
-    for (unsigned l = 0; l < n_local_; ++l) {
-        const ShardScope on_stream(*this, l);
-        ShardBuffers& b = shards_[l];
-        uint8_t* rows_c = b.rows_c2[parity];
-        const size_t sidx = (size_t)l * cfg_.n_step + step;
-        const uint32_t* relation = step_ptr(d_relation_, l, B);
-        // 1. hidden = value + feature . W, and from its epilogue the lookups and the send half of the exchange
-        const bool fused_route = F > 0 && cfg_.score_fn != SCORE_COMPLEX && cfg_.score_fn != SCORE_ROTATE && !dropout_on();
+    // 1. hidden = value + feature . W, and (elementwise score functions) from its epilogue the lookups and the send half of the exchange
+    const bool fused_route = F > 0 && (cfg_.score_fn == SCORE_TRANSE || cfg_.score_fn == SCORE_DISTMULT) && !dropout_on();
+    // rows with many lookups are routed in parts by a kernel of their own, which then publishes the tails
+    const bool heavy_route = fused_route && split_popular_rows_ && heavy_route_;
+    for (unsigned l0 = 0; l0 < n_local_; l0 += group_) {
+        const unsigned n = std::min(group_, n_local_ - l0);
         if (F > 0) {
-            tc::PlaneProblem nets[2] = {};
-            const int n_nets = two_nets ? 2 : 1;
-            for (int net = 0; net < n_nets; ++net) {
-                tc::PlaneProblem& p = nets[net];
-                const size_t w = dense_bounds_[1 + net];
-                p.A = features(b, false);
-                p.B = plane(dense_ + w, dense_lo_ + w, (long long)D * 4, true);
-                tc::GemmArgs& g = p.g;
-                g.M = (int)R; g.N = (int)D; g.K = (int)F;
-                g.epilogue = tc::EPI_ADD_TABLE_VALUE;
-                g.out = net ? b.hid_t : b.hid_h; g.ldc = D; g.block_rows = 1;
-                g.x_base = rows_c; g.x_row_stride_bytes = layout_.row_bytes; g.x_is_half = cfg_.value_bf16 ? 2 : (cfg_.state_type == ST_F16 ? 1 : 0);
+            tc::RouteArgs routes[kShardBatch] = {};
+            for (unsigned i = 0; i < n; ++i) {
+                const ShardBuffers& b = shards_[l0 + i];
+                const size_t sidx = (size_t)(l0 + i) * cfg_.n_step + step;
+                for (unsigned net = 0; net < n_nets; ++net) {
+                    tc::PlaneProblem& p = problems[i * n_nets + net];
+                    p = tc::PlaneProblem{};
+                    const size_t w = dense_bounds_[1 + net];
+                    p.A = features(b, false);
+                    p.B = plane(dense_ + w, dense_lo_ + w, (long long)D * 4, true);
+                    tc::GemmArgs& g = p.g;
+                    g.M = (int)R; g.N = (int)D; g.K = (int)F;
+                    g.epilogue = tc::EPI_ADD_TABLE_VALUE;
+                    g.out = net ? b.hid_t : b.hid_h; g.ldc = D; g.block_rows = 1;
+                    g.x_base = b.rows_c2[parity]; g.x_row_stride_bytes = layout_.row_bytes;
+                    g.x_is_half = cfg_.value_bf16 ? 2 : (cfg_.state_type == ST_F16 ? 1 : 0);
+                }
+                tc::RouteArgs& route = routes[i];
+                route.perm = d_ent_perm_ + sidx * (B + T);
+                route.off = d_ent_off_ + sidx * (R + 1);
+                route.relation = step_ptr(d_relation_, l0 + i, B);
+                route.rel_table = dense_;
+                route.send_dst = b.send_dst;
+                route.send_lo_dst = b.send_lo_dst;
+                route.pred = b.pred;
+                route.pred_lo = b.pred_lo;
+                route.B = (int)B; route.a2a = (int)cfg_.a2a_size; route.n_shard = (int)cfg_.n_shard; route.score_fn = cfg_.score_fn;
+                route.lo_bf16 = bf16 ? 1 : 0;
+                route.first_slot = heavy_route ? step_ptr(d_first_slot_, l0 + i, R) : nullptr;
             }
-            tc::RouteArgs route{};
-            route.perm = d_ent_perm_ + sidx * (B + T);
-            route.off = d_ent_off_ + sidx * (R + 1);
-            route.relation = relation;
-            route.rel_table = rel_table;
-            route.send_dst = b.send_dst;
-            route.send_lo_dst = b.send_lo_dst;
-            route.pred = b.pred;
-            route.pred_lo = b.pred_lo;
-            route.B = (int)B; route.a2a = (int)cfg_.a2a_size; route.n_shard = (int)cfg_.n_shard; route.score_fn = cfg_.score_fn;
-            route.mode[0] = two_nets ? 1 : 3;
-            route.mode[1] = two_nets ? 2 : 0;
-            route.lo_bf16 = bf16 ? 1 : 0;
-            // rows with many lookups are routed in parts by a kernel of their own, which then publishes the tails
-            const bool heavy_route = fused_route && split_popular_rows_ && heavy_route_;
-            route.first_slot = heavy_route ? d_first_slot_ + sidx * R : nullptr;
-            launch_planes("hidden", nets, n_nets, tc::SIDE_NONE, XCHG_DENSE_PARAMS, fused_route && !heavy_route ? XCHG_TAILS : -1,
-                          fused_route ? &route : nullptr);
+            const tc::Routing routing{routes, (int)n, (int)n_nets, {n_nets == 2 ? 1 : 3, 2}};
+            launch_planes("hidden", problems, (int)(n * n_nets), tc::SIDE_NONE, XCHG_DENSE_PARAMS, fused_route && !heavy_route ? XCHG_TAILS : -1,
+                          fused_route ? &routing : nullptr, n);
+        } else {
+            launch_exchange_wait(XCHG_DENSE_PARAMS);
+        }
+        for (unsigned l = l0; l < l0 + n; ++l) {
+            const ShardBuffers& b = shards_[l];
+            const size_t sidx = (size_t)l * cfg_.n_step + step;
+            if (F == 0 && !direct_rows_) {  // the hidden rows are the gathered values
+                dim3 grid(ceil_div(R, 64), ceil_div(D, 64), 1);
+                KGE_LAUNCH("hidden", KGE_DISPATCH_ROW(cfg_, KGE_CUDA(launch_dependent(k_hidden<ST, FT>, dim3(grid), dim3(256), 0, stream_, b.rows_c2[parity],
+                                                                                      layout_, nullptr, 0u, (int)R, nullptr, nullptr, b.hid_h, b.hid_t))));
+            }
             if (heavy_route)
                 KGE_LAUNCH("route_heavy", KGE_CUDA(launch_dependent(k_route_heavy, dim3(kHeavySlots), dim3(256), 0, stream_, (const float*)b.hid_h, (const float*)b.hid_t,
                                                                     (const uint4*)(d_heavy_parts_ + sidx * kHeavySlots), (const uint32_t*)(d_heavy_count_ + sidx),
-                                                                    (const uint32_t*)(d_ent_perm_ + sidx * (B + T)), relation, rel_table, b.send_dst, b.send_lo_dst,
-                                                                    b.pred, b.pred_lo, (int)B, (int)cfg_.a2a_size, (int)D, cfg_.score_fn, bf16 ? 1 : 0, sync)));
-        } else {
-            launch_exchange_wait(XCHG_DENSE_PARAMS);
-            if (!direct_rows_) {  // the hidden rows are the gathered values
-                dim3 grid(ceil_div(R, 64), ceil_div(D, 64), 1);
-                KGE_LAUNCH("hidden", KGE_DISPATCH_ROW(cfg_, KGE_CUDA(launch_dependent(k_hidden<ST, FT>, dim3(grid), dim3(256), 0, stream_, rows_c, layout_,
-                                                                                      nullptr, 0u, (int)R, nullptr, nullptr, b.hid_h, b.hid_t))));
-            }
+                                                                    (const uint32_t*)(d_ent_perm_ + sidx * (B + T)), (const uint32_t*)step_ptr(d_relation_, l, B),
+                                                                    (const float*)dense_, b.send_dst, b.send_lo_dst, b.pred, b.pred_lo, (int)B, (int)cfg_.a2a_size,
+                                                                    (int)D, cfg_.score_fn, bf16 ? 1 : 0, sync)));
+            if (dropout_on()) launch_dropout(l, step, b.rows_c2[parity]);
         }
-        if (dropout_on()) launch_dropout(l, step, rows_c);
-        if (!fused_route) {
-            LookupSizes sizes{};
-            sizes.rel_table = rel_table;
-            sizes.B = (int)B; sizes.T = (int)T; sizes.a2a = (int)cfg_.a2a_size; sizes.D = (int)D; sizes.R = (int)R;
-            sizes.lo_bf16 = bf16 ? 1 : 0;
-            sizes.prefetch = direct_rows_ && step > 0;  // the first step's index streams come from the kernel in front
-            sizes.sync = sync;
-            ShardArgs<LookupArgs> shard{};
-            LookupArgs& a = shard.s[0];
-            a.rows = lookup_rows(l, step);
-            a.relation = relation;
-            a.send_dst = b.send_dst;
-            a.send_lo_dst = l1 ? nullptr : b.send_lo_dst;
-            a.pred = b.pred;
-            a.pred_lo = l1 ? nullptr : b.pred_lo;
-            if (direct_rows_ && step + 1 == cfg_.n_step) {  // kge_debug_fetch shows the last step's hidden rows
-                a.remote = step_ptr(d_remote_, l, R);
-                a.hid = b.hid_h;
-            }
-            KGE_LAUNCH("lookup", KGE_CUDA(launch_lookup(shard, 1, sizes, cfg_.score_fn, lookup_type(), stream_)));
-        }
-        if (cfg_.regularised()) launch_regularise(l, rows_c);
+        if (!fused_route) launch_lookup(l0, n, step);
+        if (cfg_.regularised())
+            for (unsigned l = l0; l < l0 + n; ++l) launch_regularise(l, shards_[l].rows_c2[parity]);
     }
-    shards_join();
     KGE_CUDA(cudaGetLastError());
 
-    shards_fork();
-    for (unsigned l = 0; l < n_local_; ++l) {
-        const ShardScope on_stream(*this, l);
-        ShardBuffers& b = shards_[l];
-        const uint32_t* relation = step_ptr(d_relation_, l, B);
-        const uint32_t* tail = step_ptr(d_tail_, l, B);
+    for (unsigned l0 = 0; l0 < n_local_; l0 += group_) {
+        const unsigned n = std::min(group_, n_local_ - l0);
         // 2. scores
-        if (cfg_.dist_fn == DIST_DOT) {
-            tc::PlaneProblem p{};
-            p.A = bf16 ? plane16(b.pred_lo, D, false) : plane(b.pred, b.pred_lo, (long long)D * 4, false);
-            p.B = bf16 ? plane16(b.tails_lo, D, false) : plane(b.tails, b.tails_lo, (long long)D * 4, false);
-            p.g.M = (int)B; p.g.N = (int)T; p.g.K = (int)D;
-            p.g.epilogue = tc::EPI_STORE; p.g.out = b.raw; p.g.ldc = T; p.g.block_rows = 1;
-            launch_planes("score", &p, 1, tc::SIDE_NONE, XCHG_TAILS, -1);
-        } else if (l2 && cfg_.l2_contraction) {
-            // the L2 distance as |p|^2 + |t|^2 - 2 p.t on the tensor cores (direct form where that cancels)
-            tc::PlaneProblem p{};
-            p.A = plane(b.pred, b.pred_lo, (long long)D * 4, false);
-            p.B = plane(b.tails, b.tails_lo, (long long)D * 4, false);
-            p.g.M = (int)B; p.g.N = (int)T; p.g.K = (int)D;
-            p.g.epilogue = tc::EPI_L2_DISTANCE; p.g.out = b.raw; p.g.ldc = T; p.g.block_rows = 1;
-            launch_planes("score", &p, 1, tc::SIDE_NORMS, XCHG_TAILS, -1);
+        if (transh) {
+            KGE_LAUNCH_SHARDS("score", n, KGE_CUDA(launch_transh_score(transh_scores(l0, n), (int)n, (int)B, (int)T, (int)D, (int)ld, sync, stream_)));
+        } else if (dot || (l2 && cfg_.l2_contraction)) {
+            // (the L2 distance as |p|^2 + |t|^2 - 2 p.t, in the direct form where that cancels)
+            for (unsigned i = 0; i < n; ++i) {
+                const ShardBuffers& b = shards_[l0 + i];
+                tc::PlaneProblem& p = problems[i];
+                p = tc::PlaneProblem{};
+                p.A = bf16 ? plane16(b.pred_lo, D, false) : plane(b.pred, b.pred_lo, (long long)D * 4, false);
+                p.B = bf16 ? plane16(b.tails_lo, D, false) : plane(b.tails, b.tails_lo, (long long)D * 4, false);
+                p.g.M = (int)B; p.g.N = (int)T; p.g.K = (int)D;
+                p.g.epilogue = dot ? tc::EPI_STORE : tc::EPI_L2_DISTANCE;
+                p.g.out = b.raw; p.g.ldc = ld; p.g.block_rows = 1;
+            }
+            launch_planes("score", problems, (int)n, dot ? tc::SIDE_NONE : tc::SIDE_NORMS, XCHG_TAILS, -1, nullptr, n);
         } else {
-            KGE_LAUNCH("score", KGE_CUDA(launch_score(cfg_.dist_fn, b.pred, b.tails, b.raw, (int)B, (int)T, (int)D, stream_, sync)));
+            ShardArgs<ScoreArgs> shards{};
+            for (unsigned i = 0; i < n; ++i) shards.s[i] = ScoreArgs{shards_[l0 + i].pred, shards_[l0 + i].tails, shards_[l0 + i].raw};
+            KGE_LAUNCH_SHARDS("score", n, KGE_CUDA(launch_score(cfg_.dist_fn, shards, (int)n, (int)B, (int)T, (int)D, (int)ld, stream_, sync)));
         }
-        // 3. loss and the coefficients of the score gradients
-        // (the rows' loss terms are added up by a block of the entity update, off the chain)
-        KGE_LAUNCH("loss", KGE_CUDA(launch_loss(b.raw, tail, b.coeff, b.loss_rows, lp, 1.0f / normaliser, nullptr, nullptr,
-                                                d_loss_counter_ + l, l1 ? nullptr : b.coeff_lo, bf16 ? 1 : 0, (int)B, stream_, nullptr)));
+        // 3. loss and the coefficients of the score gradients (the rows' loss terms are added up by a block of the entity update, off the chain)
+        ShardArgs<LossArgs> loss{};
+        for (unsigned i = 0; i < n; ++i) {
+            const ShardBuffers& b = shards_[l0 + i];
+            loss.s[i] = LossArgs{b.raw, step_ptr(d_tail_, l0 + i, B), b.coeff, dot || l2 ? b.coeff_lo : nullptr, b.loss_rows, nullptr, nullptr, nullptr, nullptr};
+        }
+        KGE_LAUNCH_SHARDS("loss", n, KGE_CUDA(launch_loss(loss, (int)n, lp, 1.0f / normaliser, bf16 ? 1 : 0, (int)B, stream_)));
         // 4. score gradients; the tails' rows go straight to the shards that own them
-        if (l1) {
-            PairBwdArgs pa{};
-            pa.D = (int)D;
-            pa.p[0] = {b.pred, b.tails, b.coeff, (int)B, (int)T, (int)T, 1, b.d_pred, nullptr, 1};
-            pa.p[1] = {b.tails, b.pred, b.coeff, (int)T, (int)B, 1, (int)T, nullptr, b.grad_dst, (int)cfg_.a2a_size};
-            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_pair_bwd(DIST_L1, pa, stream_)));
+        if (transh) {
+            KGE_LAUNCH_SHARDS("score_bwd", n, KGE_CUDA(launch_transh_bwd(transh_gradients(l0, n), (int)n, stream_)));
+            launch_exchange_signal(XCHG_TAIL_GRADS);
+        } else if (!dot && !l2) {
+            ShardArgs<PairBwdArgs> shards{};
+            for (unsigned i = 0; i < n; ++i) {
+                const ShardBuffers& b = shards_[l0 + i];
+                PairBwdArgs& pa = shards.s[i];
+                pa.D = (int)D;
+                pa.p[0] = {b.pred, b.tails, b.coeff, (int)B, (int)T, (int)ld, 1, b.d_pred, nullptr, 1};
+                pa.p[1] = {b.tails, b.pred, b.coeff, (int)T, (int)B, 1, (int)ld, nullptr, b.grad_dst, (int)cfg_.a2a_size};
+            }
+            KGE_LAUNCH_SHARDS("score_bwd", n, KGE_CUDA(launch_pair_bwd(DIST_L1, shards, (int)n, stream_)));
             launch_exchange_signal(XCHG_TAIL_GRADS);
         } else {
             //   dot:  d_pred = C . tails,                          d_tails = C^T . pred
             //   L2:   d_pred = rowsum(C) * pred - C . tails,       d_tails = colsum(C) * tails - C^T . pred
-            tc::PlaneProblem both[2] = {};
-            tc::PlaneProblem& g = both[0];
-            g.A = bf16 ? plane16(b.coeff_lo, T, false) : plane(b.coeff, b.coeff_lo, (long long)T * 4, false);
-            g.B = bf16 ? plane16(b.tails_lo, D, true) : plane(b.tails, b.tails_lo, (long long)D * 4, true);
-            g.g.M = (int)B; g.g.N = (int)D; g.g.K = (int)T;
-            g.g.epilogue = l2 ? tc::EPI_ROWSUM_X_MINUS : tc::EPI_STORE;
-            g.g.out = b.d_pred; g.g.ldc = D; g.g.block_rows = 1;
-            g.g.x_base = reinterpret_cast<const uint8_t*>(b.pred); g.g.x_row_stride_bytes = (long long)D * 4;
-            tc::PlaneProblem& h = both[1];
-            h.A = bf16 ? plane16(b.coeff_lo, T, true) : plane(b.coeff, b.coeff_lo, (long long)T * 4, true);
-            h.B = bf16 ? plane16(b.pred_lo, D, true) : plane(b.pred, b.pred_lo, (long long)D * 4, true);
-            h.g.M = (int)T; h.g.N = (int)D; h.g.K = (int)B;
-            h.g.epilogue = g.g.epilogue;
-            h.g.out = nullptr; h.g.out_blocks = b.grad_dst; h.g.block_rows = (int)cfg_.a2a_size; h.g.ldc = D;
-            h.g.x_base = reinterpret_cast<const uint8_t*>(b.tails); h.g.x_row_stride_bytes = (long long)D * 4;
-            launch_planes("score_bwd", both, 2, l2 ? tc::SIDE_ROWSUM : tc::SIDE_NONE, -1, XCHG_TAIL_GRADS);
+            for (unsigned i = 0; i < n; ++i) {
+                const ShardBuffers& b = shards_[l0 + i];
+                tc::PlaneProblem &g = problems[2 * i], &h = problems[2 * i + 1];
+                g = h = tc::PlaneProblem{};
+                g.A = bf16 ? plane16(b.coeff_lo, ld, false) : plane(b.coeff, b.coeff_lo, (long long)ld * 4, false);
+                g.B = bf16 ? plane16(b.tails_lo, D, true) : plane(b.tails, b.tails_lo, (long long)D * 4, true);
+                g.g.M = (int)B; g.g.N = (int)D; g.g.K = (int)T;
+                g.g.epilogue = l2 ? tc::EPI_ROWSUM_X_MINUS : tc::EPI_STORE;
+                g.g.out = b.d_pred; g.g.ldc = D; g.g.block_rows = 1;
+                g.g.x_base = reinterpret_cast<const uint8_t*>(b.pred); g.g.x_row_stride_bytes = (long long)D * 4;
+                h.A = bf16 ? plane16(b.coeff_lo, ld, true) : plane(b.coeff, b.coeff_lo, (long long)ld * 4, true);
+                h.B = bf16 ? plane16(b.pred_lo, D, true) : plane(b.pred, b.pred_lo, (long long)D * 4, true);
+                h.g.M = (int)T; h.g.N = (int)D; h.g.K = (int)B;
+                h.g.epilogue = g.g.epilogue;
+                h.g.out = nullptr; h.g.out_blocks = b.grad_dst; h.g.block_rows = (int)cfg_.a2a_size; h.g.ldc = D;
+                h.g.x_base = reinterpret_cast<const uint8_t*>(b.tails); h.g.x_row_stride_bytes = (long long)D * 4;
+            }
+            launch_planes("score_bwd", problems, (int)(2 * n), l2 ? tc::SIDE_ROWSUM : tc::SIDE_NONE, -1, XCHG_TAIL_GRADS, nullptr, n);
         }
-        if (cfg_.score_fn != SCORE_TRANSE) {
-            ShardArgs<LookupBwdArgs> shard{};
-            shard.s[0] = LookupBwdArgs{lookup_rows(l, step), relation, b.d_pred, b.d_head, b.d_relrow, nullptr, nullptr, nullptr};
-            KGE_LAUNCH("lookup_bwd", KGE_CUDA(launch_lookup_bwd(shard, 1, rel_table, nullptr, (int)B, (int)D, cfg_.score_fn, lookup_type(), stream_)));
-        }
+        if (cfg_.score_fn != SCORE_TRANSE) launch_lookup_bwd(l0, n, step);
     }
-    shards_join();
     KGE_CUDA(cudaGetLastError());
 
-    // 5. segment sums + row-wise Adam, and the relation rows of the partial dense gradient
+    // 5. segment sums + row-wise Adam, and the relation rows of the dense gradient
     const bool gather_ahead = step + 1 < cfg_.n_step && !direct_rows_;
+    const bool gather_beside = gather_ahead && (side_streams_ & 2u);
     // with the table's own rows nothing reads the hidden rows' gradients but kge_debug_fetch, which shows the last step's
     const bool keep_d_hid = !direct_rows_ || step + 1 == cfg_.n_step;
-    const bool gather_beside = gather_ahead && (side_streams_ & 2u);
-    shards_fork();
-    for (unsigned l = 0; l < n_local_; ++l) {
-        const ShardScope on_stream(*this, l);
-        ShardBuffers& b = shards_[l];
-        const size_t sidx = (size_t)l * cfg_.n_step + step;
-        const HeavyRows heavy{d_heavy_parts_ + sidx * kHeavySlots, d_heavy_count_ + sidx, b.heavy_partial, b.heavy_counter, d_row_info_ + sidx * 2 * R};
-        const RelationRows rr = with_regularisers(RelationRows{b.d_relrow, d_rel_perm_ + sidx * B, d_rel_off_ + sidx * (n_rel + 1), b.dense_dst,
-                                                               (int)n_rel, (int)cfg_.world, b.d_hid_h_lo, b.d_hid_t_lo, nullptr, nullptr, nullptr, DropoutParams{}, nullptr,
-                                                               fuse_dense_ ? dense_ : nullptr, fuse_dense_ ? dense_m_ : nullptr, fuse_dense_ ? dense_v_ : nullptr,
-                                                               dense_lr_mod_[0], b.loss_rows, (int)B, 1.0f / normaliser, d_loss_total_ + l, d_loss_last_ + l,
-                                                               d_reg_loss_ ? d_reg_loss_ + 2 * l : nullptr}, l, step);
-        const dim3 grid(kHeavySlots + ceil_div(R, kRowsPerBlock) + n_rel + 1), block(64 * kSegmentLanes);  // + the loss block
-#define KGE_ENTITY_UPDATE(ST_, ...)                                                                                                          \
-    KGE_LAUNCH("entity_update", KGE_CUDA(launch_dependent(k_entity_update<ST_, 4, __VA_ARGS__>, grid, block, 0, stream_, b.table, b.rows_c2[parity], layout_, \
-                                         step_ptr(d_remote_, l, R), d_ent_perm_ + sidx * (B + T), d_ent_off_ + sidx * (R + 1), d_first_slot_ + sidx * R,      \
-                                         b.d_head, b.grad_recv, (int)B, keep_d_hid ? b.d_hid_h : nullptr, b.d_hid_t, d_step_size_ + step, entity_lr_mod_, adam_, sync, heavy, \
-                                         (int)R, rr)))
-        const bool extras = cfg_.regularised() || dropout_on() || mlp_on();
-        if (cfg_.state_type == ST_F32) {
-            if (extras) KGE_ENTITY_UPDATE(float, true); else if (direct_rows_) KGE_ENTITY_UPDATE(float, false, true); else KGE_ENTITY_UPDATE(float, false);
-        } else {
-            if (extras) KGE_ENTITY_UPDATE(__half, true); else if (direct_rows_) KGE_ENTITY_UPDATE(__half, false, true); else KGE_ENTITY_UPDATE(__half, false);
-        }
-#undef KGE_ENTITY_UPDATE
-        if (gather_beside) launch_gather(step + 1, l, side_begin());
+    const bool extras = cfg_.regularised() || dropout_on();
+    for (unsigned l0 = 0; l0 < n_local_; l0 += group_) {
+        const unsigned n = std::min(group_, n_local_ - l0);
+        ShardArgs<EntityShard> shards{};
+        for (unsigned i = 0; i < n; ++i) shards.s[i] = entity_shard(l0 + i, step, keep_d_hid);
+        EntityStep es = entity_step(step, n);
+        es.inv_normaliser = 1.0f / normaliser;
+        auto update = [&](auto state) {
+            using ST = decltype(state);
+            if (extras) return launch_entity_update<ST, 4, true>(shards, es, stream_);
+            if (direct_rows_) return launch_entity_update<ST, 4, false, true>(shards, es, stream_);
+            return launch_entity_update<ST, 4>(shards, es, stream_);
+        };
+        KGE_LAUNCH_SHARDS("entity_update", n, KGE_CUDA(cfg_.state_type == ST_F32 ? update(float{}) : update(__half{})));
+        if (gather_beside) launch_gather(step + 1, l0, n, side_begin());
     }
     KGE_CUDA(cudaGetLastError());
     if (gather_beside) side_end(1);
-    // 6. d W = feature^T . d_hidden, straight into the owners' slices of the partial dense gradient
-    for (unsigned l = 0; l < n_local_; ++l) {
-        const ShardScope on_stream(*this, l);
-        ShardBuffers& b = shards_[l];
-        tc::PlaneProblem nets[2] = {};
-        for (unsigned net = 0; net < cfg_.n_net(); ++net) {
-            tc::PlaneProblem& p = nets[net];
-            p.A = features(b, true);
-            p.B = plane(net ? b.d_hid_t : b.d_hid_h, net ? b.d_hid_t_lo : b.d_hid_h_lo, (long long)D * 4, true);
-            tc::GemmArgs& g = p.g;
-            g.M = (int)F; g.N = (int)D; g.K = (int)R;
-            g.epilogue = tc::EPI_STORE;
-            g.out = nullptr; g.out_blocks = b.dense_dst; g.block_rows = 1; g.block_cyclic = (int)cfg_.world;
-            g.block_row_offset = (int)(n_rel + net * F); g.ldc = D;
-            if (fuse_dense_) {
-                // one shard in all: this gradient is the whole gradient, and the epilogue is the projection's Adam step
-                g.epilogue = tc::EPI_DENSE_ADAM;
-                g.out_blocks = nullptr;
-                g.x_base = reinterpret_cast<const uint8_t*>(dense_ + dense_bounds_[1 + net]);
-                g.x_row_stride_bytes = (long long)D * 4;
-                g.adam = tc::DenseAdamArgs{dense_, dense_lo_, dense_m_, dense_v_, d_step_size_ + step, dense_lr_mod_[1 + net], adam_.beta_m, adam_.beta_v,
-                                           adam_.one_minus_beta_m, adam_.one_minus_beta_v, adam_.epsilon, adam_.weight_decay};
+    // 6. d W = feature^T . d_hidden: the projection's Adam step, over the rows of all shards, or straight into the owners'
+    // slices of each shard's partial dense gradient
+    const unsigned at_once = fuse_dense_ ? n_local_ : group_;
+    for (unsigned l0 = 0; l0 < n_local_; l0 += at_once) {
+        const unsigned n = std::min(at_once, n_local_ - l0), n_problems = fuse_dense_ ? 1 : n;
+        for (unsigned i = 0; i < n_problems; ++i) {
+            const ShardBuffers& b = shards_[l0 + i];
+            for (unsigned net = 0; net < n_nets; ++net) {
+                tc::PlaneProblem& p = problems[i * n_nets + net];
+                p = tc::PlaneProblem{};
+                p.A = features(b, true);
+                p.B = plane(net ? b.d_hid_t : b.d_hid_h, net ? b.d_hid_t_lo : b.d_hid_h_lo, (long long)D * 4, true);
+                tc::GemmArgs& g = p.g;
+                g.M = (int)F; g.N = (int)D; g.K = (int)(fuse_dense_ ? n * R : R);  // (shard behind shard in memory)
+                g.block_row_offset = (int)(n_rel + net * F); g.block_rows = 1; g.ldc = D;
+                if (fuse_dense_) {
+                    g.epilogue = tc::EPI_DENSE_ADAM;
+                    g.x_base = reinterpret_cast<const uint8_t*>(dense_ + dense_bounds_[1 + net]);
+                    g.x_row_stride_bytes = (long long)D * 4;
+                    g.adam = tc::DenseAdamArgs{dense_, dense_lo_, dense_m_, dense_v_, d_step_size_ + step, dense_lr_mod_[1 + net], adam_.beta_m, adam_.beta_v,
+                                               adam_.one_minus_beta_m, adam_.one_minus_beta_v, adam_.epsilon, adam_.weight_decay};
+                } else {
+                    g.epilogue = tc::EPI_STORE;
+                    g.out_blocks = b.dense_dst; g.block_cyclic = (int)cfg_.world;
+                }
             }
         }
-        if (F > 0) launch_planes("projection_bwd", nets, (int)cfg_.n_net(), tc::SIDE_NONE, -1, XCHG_DENSE_PARTIALS);
+        if (F > 0) launch_planes("projection_bwd", problems, (int)(n_problems * n_nets), tc::SIDE_NONE, -1, XCHG_DENSE_PARTIALS, nullptr, n);
         else launch_exchange_signal(XCHG_DENSE_PARTIALS);  // the relation rows of the entity update are all there is
     }
-    shards_join();
     KGE_CUDA(cudaGetLastError());
     if (gather_ahead && !gather_beside) launch_gather(step + 1, stream_);
     // 7. dense parameters: reduce over shards, Adam on the owned rows, new values and their lower planes into every replica
-    if (!fuse_dense_) {
-        DenseUpdateArgs da{};
-        da.sync = sync;
-        da.partials = d_partials_;
-        da.n_partial = (int)cfg_.n_shard;
-        da.replicas = d_replicas_;
-        da.replicas_lo = d_replicas_lo_;
-        da.n_replica = (int)cfg_.world;
-        da.adam_m = dense_m_;
-        da.adam_v = dense_v_;
-        da.n_own = own_rows_;
-        da.row_width = D;
-        for (int i = 0; i <= kDenseParams; ++i) da.bounds[i] = dense_bounds_[i];
-        for (int i = 0; i < kDenseParams; ++i) da.lr_modifier[i] = dense_lr_mod_[i];
-        da.step_size = d_step_size_ + step;
-        da.ap = adam_;
-        const unsigned blocks = (unsigned)std::min<size_t>((own_rows_ * D / 4 + 255) / 256, 148 * 8);
-        KGE_LAUNCH("dense_update", KGE_CUDA(launch_dependent(k_dense_update, dim3(std::max(1u, blocks)), dim3(256), 0, stream_, da, (int)cfg_.rank)));
-    }
+    if (!fuse_dense_) launch_dense_update(step);
     KGE_CUDA(cudaGetLastError());
     if (gather_beside) side_join(1);
+}
+
+// Dense parameters: every process, also one that owns nothing, launches it, since the kernel carries two hand-overs.
+void Engine::launch_dense_update(unsigned step) {
+    DenseUpdateArgs da{};
+    da.sync = exchange_sync();
+    da.partials = d_partials_;
+    da.n_partial = (int)cfg_.n_shard;
+    da.replicas = d_replicas_;
+    da.replicas_lo = planes_ ? d_replicas_lo_ : nullptr;
+    da.n_replica = (int)cfg_.world;
+    da.adam_m = dense_m_;
+    da.adam_v = dense_v_;
+    da.n_own = own_rows_;
+    da.row_width = cfg_.d;
+    for (int i = 0; i <= kDenseParams; ++i) da.bounds[i] = dense_bounds_[i];
+    for (int i = 0; i < kDenseParams; ++i) da.lr_modifier[i] = dense_lr_mod_[i];
+    da.step_size = d_step_size_ + step;
+    da.ap = adam_;
+    // The parameter itself is read from this process's own replica (entry `rank`).
+    const unsigned blocks = (unsigned)std::min<size_t>((own_rows_ * cfg_.d / (cfg_.d % 4 == 0 ? 4 : 1) + 255) / 256, 148 * 8);
+    KGE_LAUNCH("dense_update", KGE_CUDA(launch_dependent(k_dense_update, dim3(std::max(1u, blocks)), dim3(256), 0, stream_, da, (int)cfg_.rank)));
 }
 
 void Engine::launch_one_step(unsigned step) {
@@ -1783,6 +1907,7 @@ void Engine::launch_one_step(unsigned step) {
     lp.score_fn = cfg_.score_fn;
     lp.dist_fn = cfg_.dist_fn;
     lp.n_tail = (int)T;
+    lp.ld = (int)score_ld_;
     lp.gamma = cfg_.gamma;
     lp.adversarial_scale = cfg_.adversarial_scale;
     lp.w_neg = (0.5f * (float)T) / (float)(T - 1);
@@ -1835,25 +1960,11 @@ void Engine::launch_one_step(unsigned step) {
             KGE_LAUNCH("hidden", KGE_DISPATCH_ROW(cfg_, KGE_CUDA(launch_dependent(k_hidden<ST, FT>, dim3(grid), dim3(256), 0, stream_, 
                                                             rows_c, layout_, nullptr, 0u, (int)R, W0, W1, b.hid_h, b.hid_t))));
         }
-        const uint32_t* a2a = step_ptr(d_a2a_, l, T);
-        const uint32_t* head = step_ptr(d_head_, l, B);
-        const uint32_t* relation = step_ptr(d_relation_, l, B);
         if (mlp_on())
             for (unsigned net = 0; net < cfg_.n_net(); ++net)
                 launch_mlp_forward(rows_c, nullptr, 0u, R, (int)net, net ? b.hid_t : b.hid_h, b.mlp_cat[net], b.mlp_pre[net], b.mlp_out);
         if (dropout_on()) launch_dropout(l, step, rows_c);
-        const int route_fn = transh ? SCORE_TRANSE : cfg_.score_fn;  // TransH: the tails are routed, the prediction follows
-        if (vec)
-            KGE_LAUNCH("route", KGE_CUDA(launch_dependent(k_route<4>, dim3(T + B), dim3(64), 0, stream_, b.hid_h, b.hid_t, a2a, head, relation, rel_table,
-                                                                      b.send_dst, b.pred, (int)T, (int)cfg_.a2a_size,
-                                                                      (int)B, (int)D, route_fn, sync, (float* const*)nullptr, (float*)nullptr, 0)));
-        else
-            KGE_LAUNCH("route", KGE_CUDA(launch_dependent(k_route<1>, dim3(T + B), dim3(64), 0, stream_, b.hid_h, b.hid_t, a2a, head, relation, rel_table,
-                                                                      b.send_dst, b.pred, (int)T, (int)cfg_.a2a_size,
-                                                                      (int)B, (int)D, route_fn, sync, (float* const*)nullptr, (float*)nullptr, 0)));
-        if (transh)
-            KGE_LAUNCH("transh_predict", KGE_CUDA(launch_dependent(k_transh_predict, dim3(B), dim3(64), 0, stream_, b.hid_h, head, relation, rel_table,
-                                                                   normal_table, b.pred, b.nrm, (int)D)));
+        launch_lookup(l, 1, step);
         if (cfg_.regularised()) launch_regularise(l, rows_c);
     }
     shards_join();
@@ -1864,8 +1975,6 @@ void Engine::launch_one_step(unsigned step) {
     for (unsigned l = 0; l < n_local_; ++l) {
         const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
-        const uint32_t* head = step_ptr(d_head_, l, B);
-        const uint32_t* relation = step_ptr(d_relation_, l, B);
         const uint32_t* tail = step_ptr(d_tail_, l, B);
         PairBwdArgs pa{};
         pa.D = (int)D;
@@ -1874,7 +1983,7 @@ void Engine::launch_one_step(unsigned step) {
         const bool tc_score = cfg_.tensor_cores && cfg_.dist_fn == DIST_DOT;
         const bool tc_bwd = cfg_.tensor_cores && cfg_.dist_fn != DIST_L1;
         if (transh) {
-            KGE_LAUNCH("score", KGE_CUDA(launch_transh_score(b.pred, b.nrm, b.tails, b.raw, b.pair_s, b.pair_u, (int)B, (int)T, (int)D, sync, stream_)));
+            KGE_LAUNCH("score", KGE_CUDA(launch_transh_score(transh_scores(l, 1), 1, (int)B, (int)T, (int)D, (int)score_ld_, sync, stream_)));
         } else if (tc_score) {
             tc::GemmArgs g{};
             g.A = tc::make_operand(b.pred, (long long)D * 4, false, false);
@@ -1889,8 +1998,9 @@ void Engine::launch_one_step(unsigned step) {
             KGE_LAUNCH("score", KGE_CUDA(launch_score(cfg_.dist_fn, b.pred, b.tails, b.raw, (int)B, (int)T, (int)D, stream_,
                                                       fused_wait ? sync : ExchangeSync{})));
         }
-        KGE_LAUNCH("loss", KGE_CUDA(launch_loss(b.raw, tail, b.coeff, b.loss_rows, lp, 1.0f / normaliser, d_loss_total_ + l, d_loss_last_ + l,
-                                                d_loss_counter_ + l, nullptr, 0, (int)B, stream_, d_reg_loss_ ? d_reg_loss_ + 2 * l : nullptr)));
+        ShardArgs<LossArgs> loss{};
+        loss.s[0] = LossArgs{b.raw, tail, b.coeff, nullptr, b.loss_rows, d_loss_total_ + l, d_loss_last_ + l, d_loss_counter_ + l, d_reg_loss_ ? d_reg_loss_ + 2 * l : nullptr};
+        KGE_LAUNCH("loss", KGE_CUDA(launch_loss(loss, 1, lp, 1.0f / normaliser, 0, (int)B, stream_)));
         if (tc_bwd) {
             // Both input gradients are contractions with the coefficient matrix C [B, T]:
             //   dot:  d_pred = C . tails,                          d_tails = C^T . pred
@@ -1916,16 +2026,14 @@ void Engine::launch_one_step(unsigned step) {
             launch_tc("score_bwd", both, 2, tc_splits((ceil_div(B, 128) + ceil_div(T, 128)) * ceil_div(D, 64), std::min(B, T)), false, l2,
                       -1, XCHG_TAIL_GRADS);
         } else if (transh) {
-            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_transh_bwd(TranshBwdArgs{b.pred, b.nrm, b.tails, b.coeff, b.pair_s, b.pair_u, b.d_pred, b.d_nrm, b.grad_dst,
-                                                                               (int)cfg_.a2a_size, (int)B, (int)T, (int)D, 0}, stream_)));
+            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_transh_bwd(transh_gradients(l, 1), 1, stream_)));
             launch_exchange_signal(XCHG_TAIL_GRADS);
         } else {
             KGE_LAUNCH("score_bwd", KGE_CUDA(launch_pair_bwd(cfg_.dist_fn, pa, stream_)));
             launch_exchange_signal(XCHG_TAIL_GRADS);
         }
+        if (cfg_.score_fn != SCORE_TRANSE) launch_lookup_bwd(l, 1, step);
         if (transh) {
-            KGE_LAUNCH("pred_bwd", KGE_CUDA(launch_dependent(k_transh_pred_bwd, dim3(B), dim3(64), 0, stream_, b.d_pred, b.d_nrm, b.hid_h, head, relation,
-                                                             normal_table, b.nrm, b.d_head, b.d_relrow, b.d_normrow, (int)D)));
             // the normals' rows of the partial dense gradient, behind the relation table and the projections
             const size_t sidx = (size_t)l * cfg_.n_step + step;
             const int normal_row0 = (int)(n_rel + cfg_.n_net() * F);
@@ -1937,9 +2045,7 @@ void Engine::launch_one_step(unsigned step) {
                 KGE_LAUNCH("dense_partial", KGE_CUDA(launch_dependent(k_dense_partial<1>, dim3(n_rel), dim3(64 * kRelationLanes), 0, stream_,
                                                 b.d_normrow, d_rel_perm_ + sidx * B, d_rel_off_ + sidx * (n_rel + 1), (int)n_rel,
                                                 (int)D, b.proj_partial, 0, 1, proj_elems_, b.dense_dst, (int)cfg_.world, sync, -1, normal_row0)));
-        } else if (cfg_.score_fn != SCORE_TRANSE)
-            KGE_LAUNCH("pred_bwd", KGE_CUDA(launch_dependent(k_pred_bwd, dim3(B), dim3(64), 0, stream_, b.d_pred, b.hid_h, head, relation, rel_table, b.d_head,
-                                                                     b.d_relrow, (int)D, cfg_.score_fn)));
+        }
     }
     shards_join();
     KGE_CUDA(cudaGetLastError());
@@ -1972,30 +2078,20 @@ void Engine::launch_one_step(unsigned step) {
     for (unsigned l = 0; l < n_local_; ++l) {
         const ShardScope on_stream(*this, l);
         ShardBuffers& b = shards_[l];
-        uint8_t* rows_c = b.rows_c2[step & 1];
-        const size_t sidx = (size_t)l * cfg_.n_step + step;
-        const uint32_t* remote = step_ptr(d_remote_, l, R);
-        const uint32_t* perm = d_ent_perm_ + sidx * (B + T);
-        const uint32_t* off = d_ent_off_ + sidx * (R + 1);
-        const uint32_t* first = d_first_slot_ + sidx * R;
-        const float* alpha = d_step_size_ + step;
-        const HeavyRows heavy{d_heavy_parts_ + sidx * kHeavySlots, d_heavy_count_ + sidx, b.heavy_partial, b.heavy_counter, d_row_info_ + sidx * 2 * R};
-#define KGE_ENTITY_UPDATE(ST_, V_, EXTRAS_)                                                                                                              \
-    KGE_LAUNCH("entity_update", KGE_CUDA(launch_dependent(k_entity_update<ST_, V_, EXTRAS_>, dim3(ceil_div(R, kRowsPerBlock) + kHeavySlots), dim3(64 * kSegmentLanes), \
-                                         0, stream_, b.table, rows_c, layout_, remote, perm, off, first, b.d_head, b.grad_recv, (int)B, b.d_hid_h, b.d_hid_t, alpha,  \
-                                         entity_lr_mod_, adam_, sync, heavy, (int)R, with_regularisers(RelationRows{}, l, step))))
+        ShardArgs<EntityShard> shard{};
+        shard.s[0] = entity_shard(l, step, true);
+        const EntityStep es = entity_step(step, 1);
         const bool extras = cfg_.regularised() || dropout_on() || mlp_on();
         if (cfg_.state_type == ST_F32) {
-            if (vec) { if (extras) KGE_ENTITY_UPDATE(float, 4, true); else KGE_ENTITY_UPDATE(float, 4, false); }
-            else { if (extras) KGE_ENTITY_UPDATE(float, 1, true); else KGE_ENTITY_UPDATE(float, 1, false); }
+            if (vec) KGE_LAUNCH("entity_update", KGE_CUDA((extras ? launch_entity_update<float, 4, true>(shard, es, stream_) : launch_entity_update<float, 4>(shard, es, stream_))));
+            else KGE_LAUNCH("entity_update", KGE_CUDA((extras ? launch_entity_update<float, 1, true>(shard, es, stream_) : launch_entity_update<float, 1>(shard, es, stream_))));
         } else {
-            if (vec) { if (extras) KGE_ENTITY_UPDATE(__half, 4, true); else KGE_ENTITY_UPDATE(__half, 4, false); }
-            else { if (extras) KGE_ENTITY_UPDATE(__half, 1, true); else KGE_ENTITY_UPDATE(__half, 1, false); }
+            if (vec) KGE_LAUNCH("entity_update", KGE_CUDA((extras ? launch_entity_update<__half, 4, true>(shard, es, stream_) : launch_entity_update<__half, 4>(shard, es, stream_))));
+            else KGE_LAUNCH("entity_update", KGE_CUDA((extras ? launch_entity_update<__half, 1, true>(shard, es, stream_) : launch_entity_update<__half, 1>(shard, es, stream_))));
         }
-#undef KGE_ENTITY_UPDATE
         if (mlp_on()) launch_mlp_backward(l, step);
         // the next step's rows: needs only the rows just updated, runs beside the rest of this step
-        if (gather_beside) launch_gather(step + 1, l, side_begin());
+        if (gather_beside) launch_gather(step + 1, l, 1, side_begin());
     }
     KGE_CUDA(cudaGetLastError());
     if (gather_beside) side_end(1);
@@ -2054,27 +2150,8 @@ void Engine::launch_one_step(unsigned step) {
     KGE_CUDA(cudaGetLastError());
     if (gather_ahead && !gather_beside) launch_gather(step + 1, stream_);  // runs while the partial dense gradients travel
 
-    // 5c. dense parameters: reduce over shards, Adam on the owned slice, publish.  Every process
-    // launches it, also one that owns nothing, since the kernel carries two hand-overs.
-    {
-        DenseUpdateArgs da{};
-        da.sync = sync;
-        da.partials = d_partials_;
-        da.n_partial = (int)cfg_.n_shard;
-        da.replicas = d_replicas_;
-        da.n_replica = (int)cfg_.world;
-        da.adam_m = dense_m_;
-        da.adam_v = dense_v_;
-        da.n_own = own_rows_;
-        da.row_width = D;
-        for (int i = 0; i <= kDenseParams; ++i) da.bounds[i] = dense_bounds_[i];
-        for (int i = 0; i < kDenseParams; ++i) da.lr_modifier[i] = dense_lr_mod_[i];
-        da.step_size = d_step_size_ + step;
-        da.ap = adam_;
-        // The parameter itself is read from this process's own replica (entry `rank`).
-        const unsigned blocks = (unsigned)std::min<size_t>((own_rows_ * D / (vec ? 4 : 1) + 255) / 256, 148 * 8);
-        KGE_LAUNCH("dense_update", KGE_CUDA(launch_dependent(k_dense_update, dim3(std::max(1u, blocks)), dim3(256), 0, stream_, da, (int)cfg_.rank)));
-    }
+    // 5c. dense parameters: reduce over shards, Adam on the owned slice, publish
+    launch_dense_update(step);
     KGE_CUDA(cudaGetLastError());
     if (gather_beside) side_join(1);
 }
@@ -2369,7 +2446,7 @@ void Engine::ensure_predict_buffers() {
     const size_t Q = (size_t)cfg_.n_shard * cfg_.predict_hr, D = cfg_.d;
     p_head_hidden_ = (float*)device_alloc((size_t)cfg_.predict_hr * D * 4);
     // L1 has no contraction form; everything else ranks with the plane-fed tensor-core kernel
-    predict_planes_ = planes_ && cfg_.dist_fn != DIST_L1;
+    predict_planes_ = planes_ && cfg_.dist_fn != DIST_L1 && cfg_.score_fn != SCORE_TRANSH;
     // Rows per pass over the table.  On the tensor cores: 148 tiles of 128 rows, so that the hidden
     // rows' contraction (2 column tiles) and the scores' (10 query tiles at 1250 queries) both fill
     // whole waves of 148 blocks.
@@ -2500,19 +2577,17 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
         if (mlp_on()) launch_mlp_forward(shards_[l].table, d_head + l * hr, 0u, (unsigned)hr, 0, p_head_hidden_, p_mlp_cat_, p_mlp_pre_, p_mlp_out_);
         for (unsigned p = 0; p < cfg_.world; ++p) {
             float* dst = (float*)(peer_arena_[p] + arena_offset_predict(0)) + (size_t)(shard0_ + l) * hr * D;
-            if (cfg_.score_fn == SCORE_TRANSH) {
-                KGE_LAUNCH("predict_query", k_transh_predict<<<(unsigned)hr, 64, 0, stream_>>>(
-                                                p_head_hidden_, d_iota_, d_rel + l * hr, dense_, dense_ + dense_bounds_[3], dst, dst + Q * D, (int)D));
-                continue;
-            }
-            if (vec)
-                KGE_LAUNCH("predict_query", k_route<4><<<(unsigned)hr, 64, 0, stream_>>>(
-                                                p_head_hidden_, p_head_hidden_, nullptr, d_iota_, d_rel + l * hr, dense_, nullptr,
-                                                dst, 0, 1, (int)hr, (int)D, cfg_.score_fn, ExchangeSync{}));
-            else
-                KGE_LAUNCH("predict_query", k_route<1><<<(unsigned)hr, 64, 0, stream_>>>(
-                                                p_head_hidden_, p_head_hidden_, nullptr, d_iota_, d_rel + l * hr, dense_, nullptr,
-                                                dst, 0, 1, (int)hr, (int)D, cfg_.score_fn, ExchangeSync{}));
+            ShardArgs<LookupArgs> query{};
+            query.s[0].rows = LookupRows{reinterpret_cast<const uint8_t*>(p_head_hidden_), nullptr, d_iota_, nullptr, D * 4};
+            query.s[0].relation = d_rel + l * hr;
+            query.s[0].pred = dst;
+            query.s[0].nrm = dst + Q * D;  // TransH
+            LookupSizes sizes{};
+            sizes.rel_table = dense_;
+            sizes.normal_table = dense_ + dense_bounds_[3];
+            sizes.B = (int)hr;
+            sizes.D = (int)D;
+            KGE_LAUNCH("predict_query", KGE_CUDA(kge::launch_lookup(query, 1, sizes, cfg_.score_fn, 0, stream_)));
         }
     }
     KGE_CUDA(cudaGetLastError());
@@ -2545,8 +2620,7 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
                                                                     p_chunk_hidden_, nullptr)));
             if (mlp_on()) launch_mlp_forward(b.table, nullptr, start, c, two_nets ? 1 : 0, p_chunk_hidden_, p_mlp_cat_, p_mlp_pre_, p_mlp_out_);
             if (cfg_.score_fn == SCORE_TRANSH) {
-                KGE_LAUNCH("predict_score", KGE_CUDA(launch_transh_score(queries, queries + Q * D, p_chunk_hidden_, p_raw_, nullptr, nullptr, (int)Q, (int)c, (int)D,
-                                                                         ExchangeSync{}, stream_)));
+                KGE_LAUNCH("predict_score", KGE_CUDA(launch_transh_score(queries, queries + Q * D, p_chunk_hidden_, p_raw_, (int)Q, (int)c, (int)D, stream_)));
             } else
             KGE_LAUNCH("predict_score", KGE_CUDA(launch_score(cfg_.dist_fn, queries, p_chunk_hidden_, p_raw_, (int)Q, (int)c, (int)D, stream_)));
             launch_topk(b, c, start, last, tp, false);
@@ -2688,7 +2762,8 @@ size_t Engine::debug_fetch(const std::string& what, size_t shard, float* out, si
     else fail(KGE_INVALID_ARGUMENT, msg() << "kge_debug_fetch: unknown buffer '" << what << "'");
     if (count > capacity) fail(KGE_INVALID_ARGUMENT, msg() << "kge_debug_fetch: '" << what << "' needs room for " << count << " floats");
     KGE_CUDA(cudaStreamSynchronize(stream_));
-    if (count) KGE_CUDA(cudaMemcpy(out, src, count * 4, cudaMemcpyDeviceToHost));
+    if (count && (src == b.raw || src == b.coeff)) KGE_CUDA(cudaMemcpy2D(out, T * 4, src, score_ld_ * 4, T * 4, B, cudaMemcpyDeviceToHost));
+    else if (count) KGE_CUDA(cudaMemcpy(out, src, count * 4, cudaMemcpyDeviceToHost));
     return count;
 }
 

@@ -183,16 +183,24 @@ class Engine {
     void launch_exchange_wait(int kind);
     void launch_exchange_signal(int kind);
     void launch_gather(unsigned step, cudaStream_t stream);
-    void launch_gather(unsigned step, unsigned l, cudaStream_t stream);
+    void launch_gather(unsigned step, unsigned l0, unsigned n, cudaStream_t stream);
     void launch_tc(const char* name, tc::GemmArgs* problems, int n_problems, int splits, bool a_exact, bool rowsum,
                    int wait_kind = -1, int signal_kind = -1);
     // the plane-fed contraction: tile width and k splits chosen here
     void launch_planes(const char* name, tc::PlaneProblem* problems, int n_problems, int side, int wait_kind, int signal_kind,
-                       const tc::RouteArgs* route = nullptr);
+                       const tc::Routing* routing = nullptr, unsigned n_shards = 1);
     void launch_step_planes(unsigned step, const LossParams& lp, float normaliser);
     void refresh_lower_plane(size_t offset, size_t count);
     LookupRows lookup_rows(unsigned l, unsigned step) const;
     int lookup_type() const;
+    // what the kernels of the step read and write of the local shards l0 .. l0 + n - 1
+    void launch_dense_update(unsigned step);
+    void launch_lookup(unsigned l0, unsigned n, unsigned step);
+    void launch_lookup_bwd(unsigned l0, unsigned n, unsigned step);
+    ShardArgs<TranshScoreArgs> transh_scores(unsigned l0, unsigned n) const;
+    ShardArgs<TranshBwdArgs> transh_gradients(unsigned l0, unsigned n) const;
+    EntityShard entity_shard(unsigned l, unsigned step, bool keep_d_hid) const;
+    EntityStep entity_step(unsigned step, unsigned n) const;
     FeaturePlanes feature_planes(const ShardBuffers& b, unsigned parity) const;
     void check_device_status();
     void raise_device_status(const unsigned* words);
@@ -216,7 +224,9 @@ class Engine {
     unsigned side_streams_ = 0;
     bool split_popular_rows_ = true;  // rows with many lookups are summed in parts by several blocks
     bool direct_rows_ = false;        // lookups and row update read the table: no gathered copy, no hidden rows
-    bool planes_ = false;             // the step's contractions run on the plane-fed tensor-core kernel
+    bool planes_ = false;             // the step of batched launches, its contractions on the plane-fed tensor-core kernel
+    unsigned group_ = 1;              // local shards of one launch
+    unsigned score_ld_ = 0;           // floats between rows of scores, coefficients and TransH's pair matrices
     bool bf16_planes_ = false;        // scores and their gradients multiply bfloat16 copies of their operands
     uint32_t feat_stride_ = 0;        // floats per row of the widened / lower feature planes
     cudaEvent_t ev_fork_ = nullptr, ev_join_[2] = {nullptr, nullptr};
@@ -320,7 +330,7 @@ class Engine {
     float *p_mlp_cat_ = nullptr, *p_mlp_pre_ = nullptr, *p_mlp_out_ = nullptr;  // predict's MLP buffers
     bool filter_in_scores_ = true;  // predict's L2 score contraction also filters the scores against the queries' cut-offs (KGE_PREDICT_FILTER_IN_SCORES=0: k_topk_filter)
     bool heavy_route_ = false;  // rows with many lookups are routed in parts by k_route_heavy (KGE_ROUTE_POPULAR_ROWS=0: by the hidden kernel's epilogue)
-    bool fuse_dense_ = false, fuse_dense_env_ = true;  // single shard: dense Adam steps inside the kernels that produce the gradients (KGE_FUSE_DENSE_UPDATE=0: k_dense_update)
+    bool fuse_dense_ = false, fuse_dense_env_ = true;  // all shards in every launch: dense Adam steps inside the kernels that produce the gradients (KGE_FUSE_DENSE_UPDATE=0: k_dense_update)
     uint32_t* d_step_key_ = nullptr;   // [n_step] numbers of the staged training steps (keys of the dropout masks)
     bool dropout_on() const { return cfg_.dropout > 0.f && cfg_.f > 0; }
     DropoutParams dropout_params(unsigned l, unsigned step) const;
@@ -328,7 +338,6 @@ class Engine {
     float* d_reg_loss_ = nullptr;      // [n_local][2]: the step's regularisation loss, and a sink for its running sum
     unsigned* d_reg_counter_ = nullptr;
     void launch_regularise(unsigned l, const uint8_t* rows_c);
-    RelationRows with_regularisers(RelationRows rr, unsigned l, unsigned step) const;
     // What crosses to the GPU before a run and what comes back, laid out alike in pinned and in device memory: the five
     // index streams, then the run's words (step numbers, Adam step sizes, the loss totals' zeros), then the two status
     // words and ranking's flag.  Offsets in 32-bit words.

@@ -32,6 +32,14 @@ __device__ __forceinline__ float round_to_half(float x) { return __half2float(__
 enum DistFn : int { DIST_L1 = 0, DIST_L2 = 1, DIST_DOT = 2 };
 enum LossFn : int { LOSS_LOGSIGMOID = 0, LOSS_SOFTMAX = 1 };
 
+// What belongs to each of the shards of one process that a launch works on, one per blockIdx.y (.z where y is taken).  The
+// kernels of a step are short and mostly far too small to fill 148 SMs, so the shards of a process share every launch.
+constexpr int kShardBatch = 4;
+template <class A>
+struct ShardArgs {
+    A s[kShardBatch];
+};
+
 // Byte layout of one table row: value | adam_m | sqrt(adam_v) | feature
 // (src/poplar_kge.cpp:405-417).  Every segment starts on a 16-byte boundary and
 // row_bytes is a multiple of 16, so 128-bit accesses are always aligned.
@@ -162,10 +170,20 @@ __device__ __forceinline__ float tf32_upper(float x) { return __uint_as_float(__
 __device__ __forceinline__ float tf32_lower(float x) { return tf32_upper(x - tf32_upper(x)); }
 __device__ __forceinline__ float4 tf32_lower4(float4 v) { return make_float4(tf32_lower(v.x), tf32_lower(v.y), tf32_lower(v.z), tf32_lower(v.w)); }
 
-static __global__ void __launch_bounds__(256)
-k_gather_step_rows(const uint8_t* __restrict__ table, uint32_t row_bytes, const uint32_t* __restrict__ remote, int R,
-                   uint8_t* __restrict__ rows_c, FeaturePlanes fp) {
+struct GatherArgs {
+    const uint8_t* table;
+    const uint32_t* remote;
+    uint8_t* rows_c;
+    FeaturePlanes fp;
+};
+
+static __global__ void __launch_bounds__(256) k_gather_step_rows(const __grid_constant__ ShardArgs<GatherArgs> shards, uint32_t row_bytes, int R) {
     grid_dependency_sync();
+    const GatherArgs& g = shards.s[blockIdx.y];
+    const FeaturePlanes& fp = g.fp;
+    const uint8_t* __restrict__ table = g.table;
+    const uint32_t* __restrict__ remote = g.remote;
+    uint8_t* __restrict__ rows_c = g.rows_c;
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= R) return;
     const uint4* __restrict__ src = reinterpret_cast<const uint4*>(table + (size_t)remote[r] * row_bytes);
@@ -296,86 +314,6 @@ k_hidden(const uint8_t* __restrict__ table, RowLayout L, const uint32_t* __restr
 }
 
 // ---------------------------------------------------------------------------
-// Lookups of the hidden table and the send half of the exchange
-// (src/poplar_kge.cpp:676-684).  Blocks [0, T) copy hidden_t[a2a[q]] straight into the
-// receive buffer of the destination shard (a peer's device memory when that shard lives
-// in another process): `send_dst[d]` already points at this shard's slot of shard d's
-// buffer.  Blocks [T, T+B) form the predicted tail h (+|*|complex*) r into `pred`.
-template <int V>
-__global__ void __launch_bounds__(64)
-k_route(const float* __restrict__ hid_h, const float* __restrict__ hid_t,
-        const uint32_t* __restrict__ a2a_idx, const uint32_t* __restrict__ head,
-        const uint32_t* __restrict__ relation, const float* __restrict__ rel_table,
-        float* const* __restrict__ send_dst, float* __restrict__ pred, int T, int a2a, int B, int D,
-        int score_fn, ExchangeSync sync, float* const* __restrict__ send_lo_dst = nullptr, float* __restrict__ pred_lo = nullptr,
-        int lo_bf16 = 0) {
-    grid_dependency_sync();
-    const int b = blockIdx.x;
-    if (b < T) {
-        const int dst = b / a2a, j = b - dst * a2a;
-        const float* __restrict__ src = hid_t + (size_t)a2a_idx[b] * D;
-        float* __restrict__ out = send_dst[dst] + (size_t)j * D;
-        if (V == 4) {
-            for (int c = threadIdx.x * 4; c < D; c += blockDim.x * 4) {
-                const float4 v = load4(src + c);
-                store4(out + c, v);
-                if (send_lo_dst) {  // the companion plane of the tensor-core operands: lower TF32 part, or the bf16 rounding
-                    if (lo_bf16) store4(reinterpret_cast<__nv_bfloat16*>(send_lo_dst[dst]) + (size_t)j * D + c, v);
-                    else store4(send_lo_dst[dst] + (size_t)j * D + c, tf32_lower4(v));
-                }
-            }
-        } else {
-            for (int c = threadIdx.x; c < D; c += blockDim.x) out[c] = src[c];
-        }
-        exchange_signal(sync, XCHG_TAILS, gridDim.x);  // the tail rows are in their consumers' memory
-        return;
-    }
-    const int i = b - T;
-    if (i >= B) {
-        exchange_signal(sync, XCHG_TAILS, gridDim.x);
-        return;
-    }
-    const float* __restrict__ h = hid_h + (size_t)head[i] * D;
-    const float* __restrict__ r = rel_table + (size_t)relation[i] * D;
-    float* __restrict__ p = pred + (size_t)i * D;
-    if (score_fn == SCORE_COMPLEX || score_fn == SCORE_ROTATE) {
-        const int half = D / 2;
-        for (int c = threadIdx.x; c < half; c += blockDim.x) {
-            const float hr = h[c], hi = h[c + half];
-            float rr, ri;  // the relation as a complex number: stored (ComplEx) or the unit rotation by the stored angle (RotatE)
-            if (score_fn == SCORE_ROTATE) rotate_sin_cos(r[c], ri, rr);
-            else { rr = r[c]; ri = r[c + half]; }
-            p[c] = hr * rr - hi * ri;
-            p[c + half] = hr * ri + hi * rr;
-            if (pred_lo && lo_bf16) {
-                __nv_bfloat16* p16 = reinterpret_cast<__nv_bfloat16*>(pred_lo) + (size_t)i * D;
-                p16[c] = __float2bfloat16_rn(p[c]);
-                p16[c + half] = __float2bfloat16_rn(p[c + half]);
-            } else if (pred_lo) {
-                pred_lo[(size_t)i * D + c] = tf32_lower(p[c]);
-                pred_lo[(size_t)i * D + c + half] = tf32_lower(p[c + half]);
-            }
-        }
-    } else if (V == 4) {
-        for (int c = threadIdx.x * 4; c < D; c += blockDim.x * 4) {
-            const float4 a = load4(h + c), q = load4(r + c);
-            float4 o;
-            if (score_fn == SCORE_TRANSE) {
-                o = make_float4(a.x + q.x, a.y + q.y, a.z + q.z, a.w + q.w);
-            } else {
-                o = make_float4(a.x * q.x, a.y * q.y, a.z * q.z, a.w * q.w);
-            }
-            store4(p + c, o);
-            if (pred_lo && lo_bf16) store4(reinterpret_cast<__nv_bfloat16*>(pred_lo) + (size_t)i * D + c, o);
-            else if (pred_lo) store4(pred_lo + (size_t)i * D + c, tf32_lower4(o));
-        }
-    } else {
-        for (int c = threadIdx.x; c < D; c += blockDim.x)
-            p[c] = score_fn == SCORE_TRANSE ? h[c] + r[c] : h[c] * r[c];
-    }
-    exchange_signal(sync, XCHG_TAILS, gridDim.x);
-}
-
 // The lookups of the rows with many lookups (the parts k_prepare_segments cut them into for the
 // entity update): block p copies hidden row parts[p].x to the lookups perm[parts[p].y .. parts[p].z),
 // heads (+ or * their relation row) into `pred`, tails into the owning shards' buffers, each with
@@ -422,11 +360,17 @@ k_route_heavy(const float* __restrict__ hid_h, const float* __restrict__ hid_t, 
 // src/poplar_extensions/distance.cpp:70-104,151-185 and the codelets' l1dist / l2dist;
 // the dot form is matMul(a, b^T) of src/poplar_kge.cpp:478-479.
 // 32x64 output tile, 32-deep k slices staged in shared memory k-major, 128 threads, 4x4 each.
+struct ScoreArgs {
+    const float *P, *Tl;
+    float* raw;
+};
+
 template <int FN>
-__global__ void __launch_bounds__(128)
-k_score(const float* __restrict__ P, const float* __restrict__ Tl, float* __restrict__ raw, int B,
-        int T, int D) {
+__global__ void __launch_bounds__(128) k_score(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, int D, int ld) {
     grid_dependency_sync();
+    const float* __restrict__ P = shards.s[blockIdx.z].P;
+    const float* __restrict__ Tl = shards.s[blockIdx.z].Tl;
+    float* __restrict__ raw = shards.s[blockIdx.z].raw;
     constexpr int BM = 32, BN = 64, BK = 32;
     __shared__ __align__(16) float Ps[BK][BM];
     __shared__ __align__(16) float Ts[BK][BN];
@@ -512,7 +456,7 @@ k_score(const float* __restrict__ P, const float* __restrict__ Tl, float* __rest
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const int j = j0 + tx * 4 + b;
-            if (j < T) raw[(size_t)i * T + j] = FN == DIST_L2 ? sqrtf(acc[a][b]) : acc[a][b];
+            if (j < T) raw[(size_t)i * ld + j] = FN == DIST_L2 ? sqrtf(acc[a][b]) : acc[a][b];
         }
     }
 }
@@ -535,8 +479,10 @@ __device__ __forceinline__ void score_copy16(float* dst_smem, const float* src) 
 
 template <int FN>
 __global__ void __launch_bounds__(32 * kScoreWarps, 3)
-k_score_wide(const float* __restrict__ P, const float* __restrict__ Tl, float* __restrict__ raw, int B,
-             int T, int D, ExchangeSync sync) {
+k_score_wide(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, int D, int ld, ExchangeSync sync) {
+    const float* __restrict__ P = shards.s[blockIdx.z].P;
+    const float* __restrict__ Tl = shards.s[blockIdx.z].Tl;
+    float* __restrict__ raw = shards.s[blockIdx.z].raw;
     grid_dependency_sync();
     exchange_wait(sync, XCHG_TAILS);  // the tail rows come from the other processes
     extern __shared__ __align__(16) float score_smem[];
@@ -616,7 +562,7 @@ k_score_wide(const float* __restrict__ P, const float* __restrict__ Tl, float* _
         float sum = 0.f;
         for (int w = 0; w < n_active; ++w) sum += red[(w * 32 + prow) * 33 + trow];
         const int i = i0 + prow, j = j0 + trow;
-        if (i < B && j < T) raw[(size_t)i * T + j] = FN == DIST_L2 ? sqrtf(sum) : sum;
+        if (i < B && j < T) raw[(size_t)i * ld + j] = FN == DIST_L2 ? sqrtf(sum) : sum;
     }
 }
 
@@ -631,7 +577,10 @@ constexpr size_t kScoreTileSmem = 2 * kScoreTileStage * sizeof(float);
 
 template <int FN>
 __global__ void __launch_bounds__(256, 2)
-k_score_tile(const float* __restrict__ P, const float* __restrict__ Tl, float* __restrict__ raw, int B, int T, int D) {
+k_score_tile(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, int D, int ld) {
+    const float* __restrict__ P = shards.s[blockIdx.z].P;
+    const float* __restrict__ Tl = shards.s[blockIdx.z].Tl;
+    float* __restrict__ raw = shards.s[blockIdx.z].raw;
     grid_dependency_sync();
     extern __shared__ __align__(16) float score_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ty = lane >> 2, tx = lane & 3;
@@ -708,13 +657,13 @@ k_score_tile(const float* __restrict__ P, const float* __restrict__ Tl, float* _
         for (int b = 0; b < 8; ++b)
             score_smem[(row_p + 8 * a) * kOut + row_t - kScoreTileP + 4 * b] = FN == DIST_L2 ? sqrtf(total[a][b]) : total[a][b];
     __syncthreads();
-    const bool vec = (T & 3) == 0;
+    const bool vec = (ld & 3) == 0;
     for (int q = threadIdx.x; q < kScoreTileP * kScoreTileT / 4; q += 256) {
         const int row = q / (kScoreTileT / 4), col = q % (kScoreTileT / 4) * 4, i = i0 + row, j = j0 + col;
         if (i >= B || j >= T) continue;
         const float4 v = load4(score_smem + row * kOut + col);
-        float* dst = raw + (size_t)i * T + j;
-        if (vec) {
+        float* dst = raw + (size_t)i * ld + j;
+        if (vec && j + 3 < T) {
             store4(dst, v);
         } else {
             const float t[4] = {v.x, v.y, v.z, v.w};
@@ -725,16 +674,21 @@ k_score_tile(const float* __restrict__ P, const float* __restrict__ Tl, float* _
     }
 }
 
-// Picks the kernel: the 16-byte-copy form when the rows allow it, the general form otherwise.
-// `sync` with world > 1: the kernel waits for the tail rows of the other processes (only the
+// Picks the kernel: the 16-byte-copy form when the rows allow it, the general form otherwise.  Rows of the scores begin
+// `ld` floats apart.  `sync` with world > 1: the kernel waits for the tail rows of the other processes (only the
 // 16-byte-copy form can; returns cudaErrorNotSupported otherwise so that the caller waits first).
+inline bool score_rows_aligned(const float* P, const float* Tl, int D) {
+    return (D % 4) == 0 && reinterpret_cast<uintptr_t>(P) % 16 == 0 && reinterpret_cast<uintptr_t>(Tl) % 16 == 0;
+}
+
 template <int FN>
-inline cudaError_t launch_score(const float* P, const float* Tl, float* raw, int B, int T, int D, cudaStream_t stream,
-                                const ExchangeSync& sync = ExchangeSync{}) {
-    const bool aligned = (D % 4) == 0 && reinterpret_cast<uintptr_t>(P) % 16 == 0 && reinterpret_cast<uintptr_t>(Tl) % 16 == 0;
+inline cudaError_t launch_score(const ShardArgs<ScoreArgs>& shards, int n_shards, int B, int T, int D, int ld, cudaStream_t stream, const ExchangeSync& sync) {
+    bool aligned = true;
+    for (int s = 0; s < n_shards; ++s) aligned = aligned && score_rows_aligned(shards.s[s].P, shards.s[s].Tl, D);
+    const unsigned n = (unsigned)n_shards;
     if (!aligned) {
         if (sync.world > 1) return cudaErrorNotSupported;
-        return launch_dependent(k_score<FN>, dim3((T + 63) / 64, (B + 31) / 32), dim3(128), 0, stream, P, Tl, raw, B, T, D);
+        return launch_dependent(k_score<FN>, dim3((T + 63) / 64, (B + 31) / 32, n), dim3(128), 0, stream, shards, B, T, D, ld);
     }
     static bool configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
     const int slot = current_device_slot();
@@ -745,24 +699,25 @@ inline cudaError_t launch_score(const float* P, const float* Tl, float* raw, int
         if (slot >= 0) configured[slot] = true;
     }
     // whole tiles from two blocks per SM on; below that, and where tails are waited for, the k range is divided too
-    const dim3 tiles((T + kScoreTileT - 1) / kScoreTileT, (B + kScoreTileP - 1) / kScoreTileP);
-    if (sync.world <= 1 && (size_t)tiles.x * tiles.y >= 2 * 148)
-        return launch_dependent(k_score_tile<FN>, tiles, dim3(256), kScoreTileSmem, stream, P, Tl, raw, B, T, D);
-    return launch_dependent(k_score_wide<FN>, dim3((T + 31) / 32, (B + 31) / 32), dim3(32 * kScoreWarps), kScoreWideSmem, stream,
-                            P, Tl, raw, B, T, D, sync);
+    const dim3 tiles((T + kScoreTileT - 1) / kScoreTileT, (B + kScoreTileP - 1) / kScoreTileP, n);
+    if (sync.world <= 1 && (size_t)tiles.x * tiles.y * n >= 2 * 148)
+        return launch_dependent(k_score_tile<FN>, tiles, dim3(256), kScoreTileSmem, stream, shards, B, T, D, ld);
+    return launch_dependent(k_score_wide<FN>, dim3((T + 31) / 32, (B + 31) / 32, n), dim3(32 * kScoreWarps), kScoreWideSmem, stream, shards, B, T, D, ld, sync);
 }
-
-inline bool score_rows_aligned(const float* P, const float* Tl, int D) {
-    return (D % 4) == 0 && reinterpret_cast<uintptr_t>(P) % 16 == 0 && reinterpret_cast<uintptr_t>(Tl) % 16 == 0;
-}
-
-inline cudaError_t launch_score(int dist_fn, const float* P, const float* Tl, float* raw, int B, int T, int D, cudaStream_t stream,
+inline cudaError_t launch_score(int dist_fn, const ShardArgs<ScoreArgs>& shards, int n_shards, int B, int T, int D, int ld, cudaStream_t stream,
                                 const ExchangeSync& sync = ExchangeSync{}) {
     switch (dist_fn) {
-        case DIST_L1: return launch_score<DIST_L1>(P, Tl, raw, B, T, D, stream, sync);
-        case DIST_L2: return launch_score<DIST_L2>(P, Tl, raw, B, T, D, stream, sync);
-        default: return launch_score<DIST_DOT>(P, Tl, raw, B, T, D, stream, sync);
+        case DIST_L1: return launch_score<DIST_L1>(shards, n_shards, B, T, D, ld, stream, sync);
+        case DIST_L2: return launch_score<DIST_L2>(shards, n_shards, B, T, D, ld, stream, sync);
+        default: return launch_score<DIST_DOT>(shards, n_shards, B, T, D, ld, stream, sync);
     }
+}
+// One set of rows, the scores without gaps.
+inline cudaError_t launch_score(int dist_fn, const float* P, const float* Tl, float* raw, int B, int T, int D, cudaStream_t stream,
+                                const ExchangeSync& sync = ExchangeSync{}) {
+    ShardArgs<ScoreArgs> shards{};
+    shards.s[0] = ScoreArgs{P, Tl, raw};
+    return launch_score(dist_fn, shards, 1, B, T, D, T, stream, sync);
 }
 
 // ---------------------------------------------------------------------------
@@ -778,11 +733,22 @@ struct LossParams {
     int score_fn;
     int dist_fn;
     int n_tail;
+    int ld;                  // floats between rows of the scores and of the coefficients, whose last ld - n_tail become zeros
     float gamma;
     float softmax_shift;     // correction_weight * (log(n_entity*n_shard-1) - log(n_tail-1)), or 0
     float adversarial_scale; // 0 = off
     float w_pos, w_neg;      // log-sigmoid weights of the label / of the other columns
     float grad_scale;        // loss_scale / normaliser
+};
+
+struct LossArgs {
+    const float* raw;        // [B, ld]
+    const uint32_t* label;   // [B]
+    float *coeff, *coeff_lo; // [B, ld]; coeff_lo: companion plane, null: none
+    float* loss_rows;        // [B]
+    float *loss_total, *loss_last;  // null: a later kernel adds the rows' terms
+    unsigned* counter;
+    const float* extra_loss;
 };
 
 // After its row, the block that finishes last adds the rows' loss terms in row order (a fixed
@@ -812,19 +778,23 @@ __device__ __forceinline__ void finish_step_loss(const float* loss_rows, int B, 
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
-k_loss(const float* __restrict__ raw, const uint32_t* __restrict__ label, float* __restrict__ coeff,
-       float* __restrict__ loss_rows, LossParams lp, float inv_normaliser, float* __restrict__ loss_total,
-       float* __restrict__ loss_last, unsigned* __restrict__ counter, float* __restrict__ coeff_lo, int lo_bf16,
-       const float* __restrict__ extra_loss) {
+k_loss(const __grid_constant__ ShardArgs<LossArgs> shards, LossParams lp, float inv_normaliser, int lo_bf16) {
     grid_dependency_sync();
     __shared__ float scratch[THREADS / 32];
+    const LossArgs& a = shards.s[blockIdx.y];
+    float* __restrict__ loss_rows = a.loss_rows;
     const int i = blockIdx.x, T = lp.n_tail;
-    const float* __restrict__ r = raw + (size_t)i * T;
-    float* __restrict__ c = coeff + (size_t)i * T;
-    // the companion plane for the tensor-core gradients: lower TF32 part, or the bf16 rounding (rows of T bf16)
-    float* __restrict__ c_lo = coeff_lo && !lo_bf16 ? coeff_lo + (size_t)i * T : nullptr;
-    __nv_bfloat16* __restrict__ c16 = coeff_lo && lo_bf16 ? reinterpret_cast<__nv_bfloat16*>(coeff_lo) + (size_t)i * T : nullptr;
-    const int lab = (int)label[i];
+    const float* __restrict__ r = a.raw + (size_t)i * lp.ld;
+    float* __restrict__ c = a.coeff + (size_t)i * lp.ld;
+    // the companion plane for the tensor-core gradients: lower TF32 part, or the bf16 rounding
+    float* __restrict__ c_lo = a.coeff_lo && !lo_bf16 ? a.coeff_lo + (size_t)i * lp.ld : nullptr;
+    __nv_bfloat16* __restrict__ c16 = a.coeff_lo && lo_bf16 ? reinterpret_cast<__nv_bfloat16*>(a.coeff_lo) + (size_t)i * lp.ld : nullptr;
+    for (int j = T + (int)threadIdx.x; j < lp.ld; j += THREADS) {
+        c[j] = 0.f;
+        if (c_lo) c_lo[j] = 0.f;
+        if (c16) c16[j] = __float2bfloat16_rn(0.f);
+    }
+    const int lab = (int)a.label[i];
     const bool transe = score_is_gamma_minus_distance(lp.score_fn);
     auto score_of = [&](int j) { return transe ? lp.gamma - r[j] : r[j]; };
     auto to_coeff = [&](int j, float g_score) {
@@ -854,7 +824,7 @@ k_loss(const float* __restrict__ raw, const uint32_t* __restrict__ label, float*
             if (c16) c16[j] = __float2bfloat16_rn(cj);
             if (j == lab) loss_rows[i] = -logp;
         }
-        if (loss_total) finish_step_loss<THREADS>(loss_rows, (int)gridDim.x, inv_normaliser, loss_total, loss_last, counter, scratch, extra_loss);
+        if (a.loss_total) finish_step_loss<THREADS>(loss_rows, (int)gridDim.x, inv_normaliser, a.loss_total, a.loss_last, a.counter, scratch, a.extra_loss);
         return;
     }
     // log-sigmoid, optionally with self-adversarial weights from a detached softmax
@@ -895,21 +865,18 @@ k_loss(const float* __restrict__ raw, const uint32_t* __restrict__ label, float*
     part = block_sum<THREADS>(part, scratch);
     if (threadIdx.x == 0) loss_rows[i] = -part;
     // (null loss_total: a later kernel of the step adds the rows' terms, off the step's critical chain)
-    if (loss_total) finish_step_loss<THREADS>(loss_rows, (int)gridDim.x, inv_normaliser, loss_total, loss_last, counter, scratch, extra_loss);
+    if (a.loss_total) finish_step_loss<THREADS>(loss_rows, (int)gridDim.x, inv_normaliser, a.loss_total, a.loss_last, a.counter, scratch, a.extra_loss);
 }
 
-inline cudaError_t launch_loss(const float* raw, const uint32_t* label, float* coeff, float* loss_rows, const LossParams& lp, float inv_normaliser,
-                               float* loss_total, float* loss_last, unsigned* counter, float* coeff_lo, int lo_bf16, int B, cudaStream_t stream,
-                               const float* extra_loss = nullptr) {
+inline cudaError_t launch_loss(const ShardArgs<LossArgs>& shards, int n_shards, const LossParams& lp, float inv_normaliser, int lo_bf16, int B,
+                               cudaStream_t stream) {
     // One block per row keeps about 130 thousand threads in flight for the metric's 512 x 768 scores; a warp
     // per row (a sixth as many threads, each with a serial chain of exponentials) measured 4 us slower.  A long row of
     // log-sigmoids, whose chains are longest, gets twice the threads: 256 x 1536 self-adversarial scores 12.7 to 9.5 us
     // (a softmax row of that length was 1 us slower with them).
-    if (lp.loss_fn == LOSS_LOGSIGMOID && lp.n_tail >= 1024)
-        return launch_dependent(k_loss<512>, dim3((unsigned)B), dim3(512), 0, stream, raw, label, coeff, loss_rows, lp, inv_normaliser, loss_total,
-                                loss_last, counter, coeff_lo, lo_bf16, extra_loss);
-    return launch_dependent(k_loss<256>, dim3((unsigned)B), dim3(256), 0, stream, raw, label, coeff, loss_rows, lp, inv_normaliser, loss_total,
-                            loss_last, counter, coeff_lo, lo_bf16, extra_loss);
+    const dim3 grid((unsigned)B, (unsigned)n_shards);
+    if (lp.loss_fn == LOSS_LOGSIGMOID && lp.n_tail >= 1024) return launch_dependent(k_loss<512>, grid, dim3(512), 0, stream, shards, lp, inv_normaliser, lo_bf16);
+    return launch_dependent(k_loss<256>, grid, dim3(256), 0, stream, shards, lp, inv_normaliser, lo_bf16);
 }
 
 // ---------------------------------------------------------------------------
@@ -1015,8 +982,9 @@ __device__ __forceinline__ void store_pair(float* __restrict__ row, int k, int D
 constexpr int kPairChunk = 64;
 
 template <int FN, int ROWS>
-__global__ void __launch_bounds__(32 * kPairWarps, 3) k_pair_bwd(PairBwdArgs args) {
+__global__ void __launch_bounds__(32 * kPairWarps, 3) k_pair_bwd(const __grid_constant__ ShardArgs<PairBwdArgs> shards) {
     grid_dependency_sync();
+    const PairBwdArgs& args = shards.s[blockIdx.y];
     constexpr int kRows = ROWS * kPairWarps, kCs = kRows * kPairChunk, kStage = kCs + kPairChunk * kPairCols;
     __shared__ __align__(16) float smem[2][kStage];  // C [kRows][chunk] or [chunk][kRows] | Y [chunk][cols]
     const int D = args.D, col_tiles = (D + kPairCols - 1) / kPairCols, tile_m = (int)blockIdx.x / col_tiles;
@@ -1026,7 +994,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 3) k_pair_bwd(PairBwdArgs arg
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = m0 + warp * ROWS, k = k0 + lane * 2;
     const bool n_fast = pr.c_stride_n == 1, y_vec = (D & 3) == 0;  // else c_stride_m is 1
     const int c_stride = n_fast ? pr.c_stride_m : pr.c_stride_n;
-    const bool c_vec = ((c_stride | (n_fast ? N : M)) & 3) == 0;
+    const bool c_vec = (c_stride & 3) == 0;  // columns of C between its size and its stride are zero
     auto stage = [&](int n0, float* to) {
         if (n_fast) stage_rows<kRows, kPairChunk>(to, pr.C + (size_t)m0 * c_stride + n0, c_stride, M - m0, N - n0, c_vec);
         else stage_rows<kPairChunk, kRows>(to, pr.C + (size_t)n0 * c_stride + m0, c_stride, N - n0, M - m0, c_vec);
@@ -1091,70 +1059,26 @@ __global__ void __launch_bounds__(32 * kPairWarps, 3) k_pair_bwd(PairBwdArgs arg
 }
 
 template <int FN>
-inline cudaError_t launch_pair_bwd(PairBwdArgs args, cudaStream_t stream) {
-    const int col_tiles = (args.D + kPairCols - 1) / kPairCols;
-    auto tiles = [&](int which, int rows) { return (args.p[which].M + rows * kPairWarps - 1) / (rows * kPairWarps); };
+inline cudaError_t launch_pair_bwd(ShardArgs<PairBwdArgs> shards, int n_shards, cudaStream_t stream) {
+    const PairBwdArgs& first = shards.s[0];  // the shards' sizes are alike
+    const int col_tiles = (first.D + kPairCols - 1) / kPairCols;
+    auto tiles = [&](int which, int rows) { return (first.p[which].M + rows * kPairWarps - 1) / (rows * kPairWarps); };
     // two rows per warp where that still leaves two blocks per SM
-    const int rows = (tiles(0, 2) + tiles(1, 2)) * col_tiles >= 2 * 148 ? 2 : 1;
-    args.tiles_m0 = tiles(0, rows);
-    const dim3 grid((args.tiles_m0 + tiles(1, rows)) * col_tiles), block(32 * kPairWarps);
-    if (rows == 2) return launch_dependent(k_pair_bwd<FN, 2>, grid, block, 0, stream, args);
-    return launch_dependent(k_pair_bwd<FN, 1>, grid, block, 0, stream, args);
+    const int rows = (tiles(0, 2) + tiles(1, 2)) * col_tiles * n_shards >= 2 * 148 ? 2 : 1;
+    for (int s = 0; s < n_shards; ++s) shards.s[s].tiles_m0 = tiles(0, rows);
+    const dim3 grid((tiles(0, rows) + tiles(1, rows)) * col_tiles, (unsigned)n_shards), block(32 * kPairWarps);
+    if (rows == 2) return launch_dependent(k_pair_bwd<FN, 2>, grid, block, 0, stream, shards);
+    return launch_dependent(k_pair_bwd<FN, 1>, grid, block, 0, stream, shards);
+}
+inline cudaError_t launch_pair_bwd(int fn, const ShardArgs<PairBwdArgs>& shards, int n_shards, cudaStream_t stream) {
+    if (fn == DIST_L1) return launch_pair_bwd<DIST_L1>(shards, n_shards, stream);
+    if (fn == DIST_L2) return launch_pair_bwd<DIST_L2>(shards, n_shards, stream);
+    return launch_pair_bwd<DIST_DOT>(shards, n_shards, stream);
 }
 inline cudaError_t launch_pair_bwd(int fn, const PairBwdArgs& args, cudaStream_t stream) {
-    if (fn == DIST_L1) return launch_pair_bwd<DIST_L1>(args, stream);
-    if (fn == DIST_L2) return launch_pair_bwd<DIST_L2>(args, stream);
-    return launch_pair_bwd<DIST_DOT>(args, stream);
-}
-
-// Gradients of the head vector and of the relation row for the multiplicative score
-// functions (backward of src/poplar_kge.cpp:501-510, 567-569).  TransE needs no kernel:
-// both gradients equal d_pred.
-static __global__ void __launch_bounds__(64)
-k_pred_bwd(const float* __restrict__ d_pred, const float* __restrict__ hid_h,
-           const uint32_t* __restrict__ head, const uint32_t* __restrict__ relation,
-           const float* __restrict__ rel_table, float* __restrict__ d_head,
-           float* __restrict__ d_relrow, int D, int score_fn) {
-    grid_dependency_sync();
-    const int i = blockIdx.x;
-    const float* __restrict__ dp = d_pred + (size_t)i * D;
-    const float* __restrict__ h = hid_h + (size_t)head[i] * D;
-    const float* __restrict__ r = rel_table + (size_t)relation[i] * D;
-    float* __restrict__ dh = d_head + (size_t)i * D;
-    float* __restrict__ dr = d_relrow + (size_t)i * D;
-    if (score_fn == SCORE_DISTMULT) {
-        for (int c = threadIdx.x; c < D; c += blockDim.x) {
-            dh[c] = dp[c] * r[c];
-            dr[c] = dp[c] * h[c];
-        }
-    } else if (score_fn == SCORE_ROTATE) {
-        // Backward of src/poplar_kge.cpp:516-530.  The gradients of sine and cosine pass back through
-        // the float16 casts and the float16 sin / cos (src/pag/pag.cpp:552-595, 619-633): rounded to
-        // float16 at each of those points, the angle's gradient is their float16 sum.
-        const int half = D / 2;
-        for (int c = threadIdx.x; c < half; c += blockDim.x) {
-            const float hr = h[c], hi = h[c + half];
-            float s, co;
-            rotate_sin_cos(r[c], s, co);
-            const float gr = dp[c], gi = dp[c + half];
-            dh[c] = gr * co + gi * s;
-            dh[c + half] = -gr * s + gi * co;
-            const float d_sin = round_to_half(-gr * hi + gi * hr), d_cos = round_to_half(gr * hr + gi * hi);
-            const float via_sin = round_to_half(d_sin * co), via_cos = round_to_half(-d_cos * s);
-            dr[c] = round_to_half(via_sin + via_cos);
-            dr[c + half] = 0.f;  // the table keeps rows of D floats; the upper half of an angle row is unused
-        }
-    } else {
-        const int half = D / 2;
-        for (int c = threadIdx.x; c < half; c += blockDim.x) {
-            const float hr = h[c], hi = h[c + half], rr = r[c], ri = r[c + half];
-            const float gr = dp[c], gi = dp[c + half];
-            dh[c] = gr * rr + gi * ri;
-            dh[c + half] = -gr * ri + gi * rr;
-            dr[c] = gr * hr + gi * hi;
-            dr[c + half] = -gr * hi + gi * hr;
-        }
-    }
+    ShardArgs<PairBwdArgs> shards{};
+    shards.s[0] = args;
+    return launch_pair_bwd(fn, shards, 1, stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -1542,74 +1466,86 @@ struct HeavyRows {
     const uint4* row_info;
 };
 
-// The relation part of a shard's dense gradient, summed by blocks appended to the entity update's
-// grid (both depend only on the score gradients): row rho = the sum of the per-triple relation
-// gradients of the triples of relation rho, in position order (backward of the gather at
-// src/poplar_kge.cpp:489), stored into the memory of the process that owns that row of the dense
-// vector (row r to process r % n_owner as its row r / n_owner).  Null d_relrow: no such blocks.
-struct RelationRows {
-    const float* d_relrow;       // [B, D] per-triple gradients
-    const uint32_t* perm;        // triples ordered by relation
-    const uint32_t* off;         // [n_rel + 1]
-    float* const* dense_dst;     // [n_owner] this shard's slot in each owner's receive buffer
-    int n_rel, n_owner;
-    float* d_hid_h_lo;           // lower TF32 planes of the hidden-row gradients (null: not needed)
-    float* d_hid_t_lo;
+// What k_entity_update reads and writes of one shard.
+struct EntityShard {
+    uint8_t* table;
+    const uint8_t* rows_c;            // the step's gathered rows; null with DIRECT
+    const uint32_t *remote, *perm, *off, *first_slot;
+    const float *d_head, *grad_recv;
+    float *d_hid_h, *d_hid_t;         // gradients of the hidden rows (null: nothing reads them; d_hid_t null: one network)
+    float *d_hid_h_lo, *d_hid_t_lo;   // their lower TF32 planes (null: not needed)
+    HeavyRows heavy;
     // Gradients of the norm regularisers (k_regularise), [R, D] each, null when all weights are 0:
     // reg_val joins the value's gradient, reg_h / reg_t the gradient of the feature network's output
     // (reg_t null with a shared network, whose reg_h then holds both calls' terms).
-    const float* reg_val;
-    const float* reg_h;
-    const float* reg_t;
+    const float *reg_val, *reg_h, *reg_t;
     DropoutParams drop;  // threshold 0: none.  Masks the gradients of the feature network's outputs.
     // Non-null: the value's gradient is left here ([R, D]) and the rows are not updated; k_row_adam
     // does that once the rest of the gradient is known (the feature MLP reads the value too).
     float* defer_grad;
-    // Non-null (one shard in all: no other shard's gradient to wait for): a relation row's block applies
-    // the row's Adam step itself instead of handing its sum to k_dense_update.
-    float* rel_w;
-    float* rel_m;
-    float* rel_v;
-    float rel_lr_modifier;
-    // Non-null: one more block at the end of the grid adds the step's loss terms (loss_rows [loss_n], left by
-    // k_loss) in row order into the run's total: beside the row updates instead of at the end of k_loss.
-    const float* loss_rows;
-    int loss_n;
-    float inv_normaliser;
-    float* loss_total;
-    float* loss_last;
+    const float* d_relrow[2];         // [B, D] per-triple gradients of the relation tables' rows (the second one: TransH's normals)
+    const uint32_t *rel_perm, *rel_off;  // triples ordered by relation, [n_rel + 1]
+    float* const* dense_dst;          // [n_owner] this shard's slot in each owner's receive buffer
+    const float* loss_rows;           // [B] loss terms left by k_loss; null: k_loss has added them up
+    float *loss_total, *loss_last;
     const float* extra_loss;
 };
 
-template <int V, int LANES>
-__device__ __forceinline__ void relation_row_sum(const RelationRows& rr, int rho, int D, float (*part)[64 * V], uint32_t* s_perm,
-                                                 const float* __restrict__ step_size, const AdamParams& ap) {
-    const int col = threadIdx.x & 63, lane = threadIdx.x >> 6;
-    const uint32_t q0 = rr.off[rho], q1 = rr.off[rho + 1];
-    // where the row's gradient goes: into its owner's receive buffer, or (one shard in all) straight into the row's Adam step
+// The relation rows of the dense gradient are summed by blocks appended to the grid (they too depend only on the score
+// gradients): a row's gradient is the sum of the per-triple gradients of its relation's triples, in position order
+// (backward of the gather at src/poplar_kge.cpp:489).  Where all shards are in the launch and in this process, a block
+// adds the shards' sums in shard order and applies the row's Adam step; else each shard's sum is stored into the memory
+// of the process that owns that row of the dense vector (row r to process r % n_owner as its row r / n_owner), which
+// k_dense_update waits for.
+struct EntityStep {
+    RowLayout L;
+    int B, R, n_shards;
+    const float* step_size;
+    float lr_modifier;
+    AdamParams ap;
+    ExchangeSync sync;
+    int n_rel, n_tables, n_owner;     // relation rows per table; tables (0: another kernel sums them)
+    int rel_blocks;                   // blocks of a shard that sum relation rows
+    int dense_row0[2];                // a table's first row in the dense vector
+    float *rel_w[2], *rel_m[2], *rel_v[2];  // null: sums go to dense_dst
+    float rel_lr_modifier[2];
+    float inv_normaliser;
+};
+
+// A thread adds up PER strands of a relation's triples: strand s of LANES * PER takes the triples s, s + LANES * PER, ...
+template <int V, int LANES, int PER>
+__device__ __forceinline__ void relation_row_sum(const ShardArgs<EntityShard>& shards, const EntityStep& g, int unit, float (*part)[64 * V], uint32_t* s_perm) {
+    const int D = (int)g.L.d, col = threadIdx.x & 63, lane = threadIdx.x >> 6;
+    const int table = unit >= g.n_rel ? 1 : 0, rho = unit - table * g.n_rel;
+    const bool here = g.rel_w[table] != nullptr;
+    const int first = here ? 0 : (int)blockIdx.y, last = here ? g.n_shards : first + 1;
+    const AdamParams& ap = g.ap;
+    // where the row's gradient goes: into its owner's receive buffer, or straight into the row's Adam step
     auto deliver = [&](int c, float total) {
-        if (!rr.rel_w) {
-            rr.dense_dst[rho % rr.n_owner][(size_t)(rho / rr.n_owner) * D + c] = total;
+        if (!here) {
+            const int row = rho + g.dense_row0[table];
+            shards.s[first].dense_dst[row % g.n_owner][(size_t)(row / g.n_owner) * D + c] = total;
             return;
         }
         const size_t e = (size_t)rho * D + c;
-        const float alpha = *step_size * rr.rel_lr_modifier;
-        const float mo = ap.beta_m * rr.rel_m[e] + ap.one_minus_beta_m * total;
-        const float ve = ap.beta_v * rr.rel_v[e] + ap.one_minus_beta_v * total * total;
-        const float x = rr.rel_w[e];
-        rr.rel_w[e] = x - alpha * (mo / (sqrtf(ve) + ap.epsilon) + ap.weight_decay * x);
-        rr.rel_m[e] = mo;
-        rr.rel_v[e] = ve;
+        const float alpha = *g.step_size * g.rel_lr_modifier[table];
+        const float mo = ap.beta_m * g.rel_m[table][e] + ap.one_minus_beta_m * total;
+        const float ve = ap.beta_v * g.rel_v[table][e] + ap.one_minus_beta_v * total * total;
+        const float x = g.rel_w[table][e];
+        g.rel_w[table][e] = x - alpha * (mo / (sqrtf(ve) + ap.epsilon) + ap.weight_decay * x);
+        g.rel_m[table][e] = mo;
+        g.rel_v[table][e] = ve;
     };
     // four neighbouring columns at once where the rows allow 16-byte accesses
     auto deliver4 = [&](int c, const float (&total)[4]) {
-        if (!rr.rel_w) {
-            store4(rr.dense_dst[rho % rr.n_owner] + (size_t)(rho / rr.n_owner) * D + c, make_float4(total[0], total[1], total[2], total[3]));
+        if (!here) {
+            const int row = rho + g.dense_row0[table];
+            store4(shards.s[first].dense_dst[row % g.n_owner] + (size_t)(row / g.n_owner) * D + c, make_float4(total[0], total[1], total[2], total[3]));
             return;
         }
         const size_t e = (size_t)rho * D + c;
-        const float alpha = *step_size * rr.rel_lr_modifier;
-        const float4 m4 = load4(rr.rel_m + e), v4 = load4(rr.rel_v + e), x4 = load4(rr.rel_w + e);
+        const float alpha = *g.step_size * g.rel_lr_modifier[table];
+        const float4 m4 = load4(g.rel_m[table] + e), v4 = load4(g.rel_v[table] + e), x4 = load4(g.rel_w[table] + e);
         float mo[4] = {m4.x, m4.y, m4.z, m4.w}, ve[4] = {v4.x, v4.y, v4.z, v4.w}, x[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -1617,11 +1553,13 @@ __device__ __forceinline__ void relation_row_sum(const RelationRows& rr, int rho
             ve[u] = ap.beta_v * ve[u] + ap.one_minus_beta_v * total[u] * total[u];
             x[u] = x[u] - alpha * (mo[u] / (sqrtf(ve[u]) + ap.epsilon) + ap.weight_decay * x[u]);
         }
-        store4(rr.rel_w + e, make_float4(x[0], x[1], x[2], x[3]));
-        store4(rr.rel_m + e, make_float4(mo[0], mo[1], mo[2], mo[3]));
-        store4(rr.rel_v + e, make_float4(ve[0], ve[1], ve[2], ve[3]));
+        store4(g.rel_w[table] + e, make_float4(x[0], x[1], x[2], x[3]));
+        store4(g.rel_m[table] + e, make_float4(mo[0], mo[1], mo[2], mo[3]));
+        store4(g.rel_v[table] + e, make_float4(ve[0], ve[1], ve[2], ve[3]));
     };
-    if (q0 == q1) {
+    bool any = false;
+    for (int s = first; s < last; ++s) any = any || shards.s[s].rel_off[rho] != shards.s[s].rel_off[rho + 1];
+    if (!any) {
         if (V == 4) {
             const float zero[4] = {0.f, 0.f, 0.f, 0.f};
             for (int c = threadIdx.x * 4; c < D; c += blockDim.x * 4) deliver4(c, zero);
@@ -1632,53 +1570,62 @@ __device__ __forceinline__ void relation_row_sum(const RelationRows& rr, int rho
     }
     for (int c0 = 0; c0 < D; c0 += 64 * V) {
         const int c = c0 + col * V;
-        float g[V];
+        float totals[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int s = first; s < last; ++s) {
+            const EntityShard& a = shards.s[s];
+            const float* __restrict__ rows = a.d_relrow[table];
+            const uint32_t q0 = a.rel_off[rho], q1 = a.rel_off[rho + 1];
+            if (q0 == q1) continue;
+            float sum[PER][V];
 #pragma unroll
-        for (int u = 0; u < V; ++u) g[u] = 0.f;
-        for (uint32_t base = q0; base < q1; base += 64 * LANES) {
-            const int count = (int)min((uint32_t)(64 * LANES), q1 - base);
-            __syncthreads();
-            if ((int)threadIdx.x < count) s_perm[threadIdx.x] = rr.perm[base + threadIdx.x];
-            __syncthreads();
-            if (c >= D) continue;
-            for (int i = lane; i < count; i += 4 * LANES) {
-                float4 v[4];
+            for (int p = 0; p < PER; ++p)
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int ii = i + u * LANES;
-                    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (ii < count) {
-                        const float* src = rr.d_relrow + (size_t)s_perm[ii] * D + c;
-                        if (V == 4) v[u] = load4(src); else v[u].x = src[0];
+                for (int u = 0; u < V; ++u) sum[p][u] = 0.f;
+            for (uint32_t base = q0; base < q1; base += 64 * LANES) {
+                const int count = (int)min((uint32_t)(64 * LANES), q1 - base);
+                __syncthreads();
+                if ((int)threadIdx.x < count) s_perm[threadIdx.x] = a.rel_perm[base + threadIdx.x];
+                __syncthreads();
+                if (c >= D) continue;
+                for (int i = lane; i < count; i += 4 * LANES) {
+                    float4 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int ii = i + u * LANES;
+                        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (ii < count) {
+                            const float* src = rows + (size_t)s_perm[ii] * D + c;
+                            if (V == 4) v[u] = load4(src); else v[u].x = src[0];
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (i + u * LANES >= count) continue;
+                        float (&strand)[V] = sum[u % PER];
+                        strand[0] += v[u].x;
+                        if (V == 4) { strand[1 % V] += v[u].y; strand[2 % V] += v[u].z; strand[3 % V] += v[u].w; }
                     }
                 }
+            }
+            __syncthreads();
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (i + u * LANES >= count) continue;
-                    g[0] += v[u].x;
-                    if (V == 4) { g[1 % V] += v[u].y; g[2 % V] += v[u].z; g[3 % V] += v[u].w; }
+            for (int p = 0; p < PER; ++p)
+#pragma unroll
+                for (int u = 0; u < V; ++u) part[p * LANES + lane][col * V + u] = sum[p][u];
+            __syncthreads();
+            if (lane == 0 && c < D) {
+#pragma unroll
+                for (int u = 0; u < V; ++u) {
+                    float total = part[0][col * V + u];
+#pragma unroll
+                    for (int l = 1; l < LANES * PER; ++l) total += part[l][col * V + u];
+                    totals[u] += total;
                 }
             }
         }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < V; ++u) part[lane][col * V + u] = g[u];
-        __syncthreads();
         if (lane == 0 && c < D) {
-#pragma unroll
-            float totals[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int u = 0; u < V; ++u) {
-                float total = part[0][col * V + u];
-#pragma unroll
-                for (int l = 1; l < LANES; ++l) total += part[l][col * V + u];
-                totals[u] = total;
-            }
-            if (V == 4) {
-                deliver4(c, totals);
-            } else {
-                deliver(c, totals[0]);
-            }
+            if (V == 4) deliver4(c, totals);
+            else deliver(c, totals[0]);
         }
     }
 }
@@ -1688,35 +1635,47 @@ __device__ __forceinline__ void relation_row_sum(const RelationRows& rr, int rho
 // DIRECT: the step makes no gathered copy; the state before the update is the table row, which only its first slot touches.
 template <class ST, int V, bool EXTRAS = false, bool DIRECT = false>
 __global__ void __launch_bounds__(64 * kSegmentLanes, EXTRAS ? 2 : 4)
-k_entity_update(uint8_t* __restrict__ table, const uint8_t* __restrict__ rows_c, RowLayout L,
-                const uint32_t* __restrict__ remote, const uint32_t* __restrict__ perm,
-                const uint32_t* __restrict__ off,
-                const uint32_t* __restrict__ first_slot, const float* __restrict__ d_head,
-                const float* __restrict__ grad_recv, int B,
-                float* __restrict__ d_hid_h, float* __restrict__ d_hid_t,
-                const float* __restrict__ step_size, float lr_modifier, AdamParams ap, ExchangeSync sync, HeavyRows heavy,
-                int R, RelationRows rr) {
+k_entity_update(const __grid_constant__ ShardArgs<EntityShard> shards, const __grid_constant__ EntityStep g) {
     grid_dependency_sync();
-    const int row_blocks = (R + kRowsPerBlock - 1) / kRowsPerBlock;
+    const EntityShard& rr = shards.s[blockIdx.y];
+    const RowLayout& L = g.L;
+    const AdamParams& ap = g.ap;
+    const int R = g.R, B = g.B, row_blocks = (R + kRowsPerBlock - 1) / kRowsPerBlock;
     if ((int)blockIdx.x >= kHeavySlots + row_blocks) {  // a relation row: needs nothing from the other processes
-        __shared__ float rel_part[kSegmentLanes][64 * V];
+        __shared__ float rel_part[2 * kSegmentLanes][64 * V];
         __shared__ uint32_t rel_perm[64 * kSegmentLanes];
-        const int rho = (int)blockIdx.x - kHeavySlots - row_blocks;
-        if (rho >= rr.n_rel) {  // the loss block
+        const int block = (int)blockIdx.x - kHeavySlots - row_blocks;
+        if (block >= g.rel_blocks) {  // the loss block
             float part = 0.f;
-            for (int i = threadIdx.x; i < rr.loss_n; i += 64 * kSegmentLanes) part += rr.loss_rows[i];
+            for (int i = threadIdx.x; i < B; i += 64 * kSegmentLanes) part += rr.loss_rows[i];
             part = block_sum<64 * kSegmentLanes>(part, &rel_part[0][0]);
             if (threadIdx.x == 0) {
-                const float step_loss = part * rr.inv_normaliser + (rr.extra_loss ? *rr.extra_loss : 0.f);
+                const float step_loss = part * g.inv_normaliser + (rr.extra_loss ? *rr.extra_loss : 0.f);
                 *rr.loss_total += step_loss;
                 *rr.loss_last = step_loss;
             }
             return;
         }
-        relation_row_sum<V, kSegmentLanes>(rr, rho, (int)L.d, rel_part, rel_perm, step_size, ap);
+        // rows whose shards are added up here are dealt out over the shards' blocks
+        const int unit = g.rel_w[0] ? block * g.n_shards + (int)blockIdx.y : block;
+        if (unit >= g.n_rel * g.n_tables) return;
+        // (the order of a sum is part of an L1 model's result, see k_pair_bwd: TransH's have eight strands, the others four)
+        if (g.n_tables > 1) relation_row_sum<V, kSegmentLanes, 2>(shards, g, unit, rel_part, rel_perm);
+        else relation_row_sum<V, kSegmentLanes, 1>(shards, g, unit, rel_part, rel_perm);
         return;
     }
-    exchange_wait(sync, XCHG_TAIL_GRADS);  // grad_recv is written by the other processes
+    uint8_t* __restrict__ table = rr.table;
+    const uint8_t* __restrict__ rows_c = rr.rows_c;
+    const uint32_t* __restrict__ remote = rr.remote;
+    const uint32_t* __restrict__ perm = rr.perm;
+    const uint32_t* __restrict__ off = rr.off;
+    const uint32_t* __restrict__ first_slot = rr.first_slot;
+    const float* __restrict__ d_head = rr.d_head;
+    const float* __restrict__ grad_recv = rr.grad_recv;
+    float* __restrict__ d_hid_h = rr.d_hid_h;
+    float* __restrict__ d_hid_t = rr.d_hid_t;
+    const HeavyRows& heavy = rr.heavy;
+    exchange_wait(g.sync, XCHG_TAIL_GRADS);  // grad_recv is written by the other processes
     // partial sums of the item lanes, [lane][head | tail][64 column threads][V]
     __shared__ float part[kSegmentLanes][2][64 * V];
     __shared__ uint32_t s_perm[64 * kSegmentLanes];
@@ -1756,7 +1715,7 @@ k_entity_update(uint8_t* __restrict__ table, const uint8_t* __restrict__ rows_c,
     const ST* xs = reinterpret_cast<const ST*>(state);
     const ST* ms = reinterpret_cast<const ST*>(state + L.off_m);
     const ST* qs = reinterpret_cast<const ST*>(state + L.off_q);
-    const float alpha = *step_size * lr_modifier;
+    const float alpha = *g.step_size * g.lr_modifier;
     const bool writes_row = (slot_word & 1u) != 0;
 
     // Sums of the lookups [q0, q1) for the columns c .. c+V-1, separately for head and tail lookups;
@@ -1775,26 +1734,26 @@ k_entity_update(uint8_t* __restrict__ table, const uint8_t* __restrict__ rows_c,
             if (c >= D) continue;
             for (int q = lane; q < count; q += 4 * kSegmentLanes) {
                 uint32_t e[4];
-                float4 g[4];
+                float4 v[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) e[u] = q + u * kSegmentLanes < count ? s_perm[q + u * kSegmentLanes] : 0xffffffffu;
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    g[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (e[u] == 0xffffffffu) continue;
                     const float* src = e[u] < (uint32_t)B ? d_head + (size_t)e[u] * D + c
                                                           : grad_recv + (size_t)(e[u] - B) * D + c;
-                    if (V == 4) g[u] = load4(src); else g[u].x = src[0];
+                    if (V == 4) v[u] = load4(src); else v[u].x = src[0];
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     if (e[u] == 0xffffffffu) continue;
                     if (e[u] < (uint32_t)B) {
-                        gh[0] += g[u].x;
-                        if (V == 4) { gh[1 % V] += g[u].y; gh[2 % V] += g[u].z; gh[3 % V] += g[u].w; }
+                        gh[0] += v[u].x;
+                        if (V == 4) { gh[1 % V] += v[u].y; gh[2 % V] += v[u].z; gh[3 % V] += v[u].w; }
                     } else {
-                        gt[0] += g[u].x;
-                        if (V == 4) { gt[1 % V] += g[u].y; gt[2 % V] += g[u].z; gt[3 % V] += g[u].w; }
+                        gt[0] += v[u].x;
+                        if (V == 4) { gt[1 % V] += v[u].y; gt[2 % V] += v[u].z; gt[3 % V] += v[u].w; }
                     }
                 }
             }
@@ -1879,10 +1838,9 @@ k_entity_update(uint8_t* __restrict__ table, const uint8_t* __restrict__ rows_c,
         }
 #pragma unroll
         for (int u = 0; u < V; ++u) {
-            const float g = gv[u];
             float v = qq[u] * qq[u];
-            m[u] = ap.beta_m * m[u] + ap.one_minus_beta_m * g;
-            v = ap.beta_v * v + ap.one_minus_beta_v * g * g;
+            m[u] = ap.beta_m * m[u] + ap.one_minus_beta_m * gv[u];
+            v = ap.beta_v * v + ap.one_minus_beta_v * gv[u] * gv[u];
             x[u] = x[u] - alpha * (m[u] / (sqrtf(v) + ap.epsilon) + ap.weight_decay * x[u]);
             qq[u] = sqrtf(v);
         }
@@ -2003,6 +1961,13 @@ k_entity_update(uint8_t* __restrict__ table, const uint8_t* __restrict__ rows_c,
         }
         finish(c, gh, gt);
     }
+}
+
+template <class ST, int V, bool EXTRAS = false, bool DIRECT = false>
+inline cudaError_t launch_entity_update(const ShardArgs<EntityShard>& shards, const EntityStep& g, cudaStream_t stream) {
+    const int loss_blocks = shards.s[0].loss_rows ? 1 : 0;
+    const dim3 grid((unsigned)(kHeavySlots + (g.R + kRowsPerBlock - 1) / kRowsPerBlock + g.rel_blocks + loss_blocks), (unsigned)g.n_shards);
+    return launch_dependent(k_entity_update<ST, V, EXTRAS, DIRECT>, grid, dim3(64 * kSegmentLanes), 0, stream, shards, g);
 }
 
 // ---------------------------------------------------------------------------

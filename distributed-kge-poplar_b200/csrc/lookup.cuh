@@ -9,19 +9,12 @@
 
 namespace kge {
 
-// Shards of one process that a launch works on, one per blockIdx.y.
-constexpr int kShardBatch = 4;
-template <class A>
-struct ShardArgs {
-    A s[kShardBatch];
-};
-
 // Where the rows that lookups name lie: hidden rows in fp32, or, in a model without features, whose hidden rows are the
 // stored values, the table itself.
 struct LookupRows {
     const uint8_t *head, *tail;           // bases of the rows that head and tail lookups read
     const uint32_t *head_row, *tail_row;  // [B], [T] rows by lookup
-    uint32_t stride;                      // bytes
+    size_t stride;                        // bytes
 };
 
 struct LookupArgs {
@@ -71,6 +64,24 @@ __device__ __forceinline__ void for_row(const VT* __restrict__ src, int D, F f) 
         }
     } else {
         for (int c = lane; c < D; c += 32) f(c, load_as_float(src + c));
+    }
+}
+
+// Sums over a row's columns for a whole warp: add(c, sums) for the columns lane, lane + 64, ... into one set of sums and for
+// lane + 32, lane + 96, ... into another, each then added up over the lanes.  (The order is part of TransH's result, whose
+// L1 gradients turn on the last bit of a score: see k_pair_bwd.)
+template <int N, class F>
+__device__ __forceinline__ void two_strands(int D, float (&sums)[2][N], F add) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 2
+    for (int c = lane; c < D; c += 64) {
+        add(c, sums[0]);
+        if (c + 32 < D) add(c + 32, sums[1]);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        sums[0][i] = warp_sum(sums[0][i]);
+        sums[1][i] = warp_sum(sums[1][i]);
     }
 }
 
@@ -124,14 +135,12 @@ __global__ void __launch_bounds__(256) k_lookup(const __grid_constant__ ShardArg
         } else if (FN == SCORE_TRANSH) {
             // n_i = w_i / |w_i|,  pt_i = h_i - n_i (n_i . h_i) + r_i
             const float* __restrict__ w = g.normal_table + (size_t)a.relation[i] * D;
-            float ww = 0.f, wh = 0.f;
-#pragma unroll 4
-            for (int c = lane; c < D; c += 32) {
-                ww += w[c] * w[c];
-                wh += w[c] * load_as_float(h + c);
-            }
-            ww = warp_sum(ww);
-            wh = warp_sum(wh);
+            float sums[2][2] = {};
+            two_strands(D, sums, [&](int c, float (&sum)[2]) {
+                sum[0] += w[c] * w[c];
+                sum[1] += w[c] * load_as_float(h + c);
+            });
+            const float ww = sums[0][0] + sums[1][0], wh = sums[0][1] + sums[1][1];
             const float inv = 1.f / sqrtf(ww), nh = wh * inv;  // n . h
 #pragma unroll 4
             for (int c = lane; c < D; c += 32) {
@@ -244,20 +253,15 @@ k_lookup_bwd(const __grid_constant__ ShardArgs<LookupBwdArgs> shards, const floa
         const float* __restrict__ w = normal_table + (size_t)a.relation[i] * D;
         const float* __restrict__ n = a.nrm + (size_t)i * D;
         const float* __restrict__ dn = a.d_nrm + (size_t)i * D;
-        float ww = 0.f, nh = 0.f, ndp = 0.f;
-#pragma unroll 4
-        for (int c = lane; c < D; c += 32) {
-            ww += w[c] * w[c];
-            nh += n[c] * load_as_float(h + c);
-            ndp += n[c] * dp[c];
-        }
-        ww = warp_sum(ww);
-        nh = warp_sum(nh);
-        ndp = warp_sum(ndp);
-        float ndn = 0.f;  // n . (total d_n)
-#pragma unroll 4
-        for (int c = lane; c < D; c += 32) ndn += n[c] * (dn[c] - nh * dp[c] - load_as_float(h + c) * ndp);
-        ndn = warp_sum(ndn);
+        float sums[2][3] = {}, last[2][1] = {};
+        two_strands(D, sums, [&](int c, float (&sum)[3]) {
+            sum[0] += w[c] * w[c];
+            sum[1] += n[c] * load_as_float(h + c);
+            sum[2] += n[c] * dp[c];
+        });
+        const float ww = sums[0][0] + sums[1][0], nh = sums[0][1] + sums[1][1], ndp = sums[0][2] + sums[1][2];
+        two_strands(D, last, [&](int c, float (&sum)[1]) { sum[0] += n[c] * (dn[c] - nh * dp[c] - load_as_float(h + c) * ndp); });
+        const float ndn = last[0][0] + last[1][0];  // n . (total d_n)
         const float inv = 1.f / sqrtf(ww);
 #pragma unroll 4
         for (int c = lane; c < D; c += 32) {

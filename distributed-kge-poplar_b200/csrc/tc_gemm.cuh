@@ -682,7 +682,7 @@ __device__ __forceinline__ void finish_four(const GemmArgs& g, float* out_base, 
     } else {
         out_row = out_base + (size_t)m * g.ldc;
     }
-    if ((g.N & 3) == 0 && (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(out_row) & 15) == 0) {
+    if (n + 3 < g.N && (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(out_row) & 15) == 0) {
         *reinterpret_cast<float4*>(out_row + n) = make_float4(acc[0], acc[1], acc[2], acc[3]);
     } else {
 #pragma unroll

@@ -94,9 +94,8 @@ struct PlaneProblem {
 // row they read, `off[r]` is where row r's begin (k_prepare_segments).  Lookup e < B is head lookup
 // e: pred[e] = row (+|*) relation row; lookup e >= B is tail lookup e - B: the row goes to slot
 // (e - B) % a2a of destination shard (e - B) / a2a, whose buffer may be a peer's memory.  Both also
-// get their lo plane (the score gradients read them as tensor-core operands).  mode[p]: what
-// problem p of the launch routes (bit 0 heads, bit 1 tails; separate head / tail networks are two
-// problems).  Null `perm`: no routing.
+// get their lo plane (the score gradients read them as tensor-core operands).  A set belongs to one
+// shard; PlaneSet::route_mode tells what each problem of the launch routes.
 struct RouteArgs {
     const uint32_t* perm;
     const uint32_t* off;
@@ -107,7 +106,6 @@ struct RouteArgs {
     float* pred;
     float* pred_lo;
     int B, a2a, n_shard, score_fn;
-    int mode[2];
     int lo_bf16;  // the companion planes hold the bfloat16 rounding of the rows instead of the lower TF32 part
     // Per gathered row, bit 1 set: the row has so many lookups that they are routed in parts by
     // k_route_heavy (a row that half of a step's lookups name would otherwise keep one block storing
@@ -117,18 +115,23 @@ struct RouteArgs {
 constexpr uint32_t kRouteSkip = 0xffffffffu;
 constexpr int kRouteMaxLookups = 4096;  // lookups one block may have to route (batch_size + n_shard * a2a_size)
 
-struct PlanePair {
-    PlaneProblem p[2];
-    int tiles_m0;  // blocks with blockIdx.x < tiles_m0 work on p[0], the others on p[1]
+// The contractions of one launch: two per shard (the two score gradients, the two feature networks) at most.
+constexpr int kMaxPlaneProblems = 2 * kShardBatch;
+struct PlaneSet {
+    PlaneProblem p[kMaxPlaneProblems];
+    int n_problems;
+    int tiles_end[kMaxPlaneProblems];  // blocks with blockIdx.x below it, and not below the one before, work on p[i]
     ExchangeSync sync;
     int wait_kind, signal_kind;
-    RouteArgs route;
-    int n_stages[2];  // ring stages of each problem (2 to kPlMaxStages), as many as the shared memory holds
+    RouteArgs route[kShardBatch];
+    int route_of[kMaxPlaneProblems];    // which of them a problem's finished rows follow
+    int route_mode[kMaxPlaneProblems];  // bit 0: its head lookups, bit 1: its tail lookups (separate networks are two problems), 0: none
+    int n_stages[kMaxPlaneProblems];    // ring stages of each problem (2 to kPlMaxStages), as many as the shared memory holds
     int bf16;         // 1: the operands are bfloat16 planes, 2: float16 planes (k_half_tiles): 64-deep slices, kind::f16 products
 };
 
 struct PlaneMaps {
-    CUtensorMap a_hi[2], a_lo[2], b_hi[2], b_lo[2];
+    CUtensorMap a_hi[kMaxPlaneProblems], a_lo[kMaxPlaneProblems], b_hi[kMaxPlaneProblems], b_lo[kMaxPlaneProblems];
 };
 
 constexpr int kPlMaxStages = 4;
@@ -287,7 +290,7 @@ __device__ __forceinline__ void route_rows(const RouteArgs& rt, int mode, const 
             float4 o = h[b];
             float *dst, *dst_lo;
             if (head[b]) {
-                // TransE / DistMult: elementwise with the relation row (ComplEx mixes the halves of a row: k_route)
+                // TransE / DistMult: elementwise with the relation row (ComplEx mixes the halves of a row: k_lookup)
                 if (rt.score_fn == 0) o = make_float4(o.x + r[b].x, o.y + r[b].y, o.z + r[b].z, o.w + r[b].w);
                 else o = make_float4(o.x * r[b].x, o.y * r[b].y, o.z * r[b].z, o.w * r[b].w);
                 dst = rt.pred + (size_t)e * D;
@@ -393,7 +396,7 @@ __device__ __forceinline__ void l2_distance_four(const PlaneProblem& pp, int m, 
 
 __device__ __forceinline__ void store_four(const GemmArgs& g, int m, int n, const float (&acc)[4]) {
     float* out_row = g.out + (size_t)m * g.ldc;
-    if ((g.N & 3) == 0 && (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(out_row) & 15) == 0) {
+    if (n + 3 < g.N && (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(out_row) & 15) == 0) {
         *reinterpret_cast<float4*>(out_row + n) = make_float4(acc[0], acc[1], acc[2], acc[3]);
     } else {
 #pragma unroll
@@ -450,7 +453,7 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // (3: up to 30 rows, five or more splits; 7: up to 64 rows).  BF16: bfloat16 operands.
 template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, bool BF16 = false>
 __global__ void __launch_bounds__(kPlThreads, 1)
-k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneMaps maps) {
+k_tc_planes(const __grid_constant__ PlaneSet gp, const __grid_constant__ PlaneMaps maps) {
     constexpr bool kLean = EPI >= 0;
     static_assert(BN == 64 || BN == 128, "tile widths: 64 or 128 columns");
     constexpr int CPT = BN / 2;  // accumulator columns per accumulating thread: a warp reads one half of its 32 lanes' columns
@@ -464,13 +467,14 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     __shared__ float s_cut_score[SIDE == SIDE_NORMS ? kBM : 1];            // their scores: a score below it cannot pass
     constexpr bool ROWSUM = SIDE != SIDE_NONE;
 
-    const int which = (int)blockIdx.x >= gp.tiles_m0 ? 1 : 0;
+    int which = 0;
+    while (which + 1 < gp.n_problems && (int)blockIdx.x >= gp.tiles_end[which]) ++which;
     const PlaneProblem& pp = gp.p[which];
     const GemmArgs& g = pp.g;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = ((int)blockIdx.x - (which ? gp.tiles_m0 : 0)) * kBM, n0 = blockIdx.y * BN;
+    const int m0 = ((int)blockIdx.x - (which ? gp.tiles_end[which - 1] : 0)) * kBM, n0 = blockIdx.y * BN;
     const unsigned total_blocks = gridDim.x * gridDim.y * gridDim.z;
-    if (n0 >= g.N || m0 >= g.M) {  // the two problems may differ in size (a whole cluster leaves together)
+    if (n0 >= g.N || m0 >= g.M) {  // the problems may differ in size (a whole cluster leaves together)
         grid_dependency_sync();
         exchange_signal(gp.sync, gp.signal_kind, total_blocks);
         return;
@@ -638,7 +642,8 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
 
     // Routing (hidden rows to their lookups): the finished rows and the staged lookups live in the
     // idle ring, behind what the k-split exchange uses.
-    const bool routing = (!kLean || EPI == EPI_ADD_TABLE_VALUE) && gp.route.perm != nullptr && gp.route.mode[which] != 0;
+    const bool routing = (!kLean || EPI == EPI_ADD_TABLE_VALUE) && gp.route_mode[which] != 0;
+    const RouteArgs& route = gp.route[gp.route_of[which]];
     float* fin = reinterpret_cast<float*>(smem + 150 * 1024);                              // [<= 64 rows][BN], or [128][BN] at offset 0 without a k split
     uint32_t* s_look = reinterpret_cast<uint32_t*>(smem + 184 * 1024);                      // [kRouteMaxLookups]
     uint32_t* s_rel = s_look + kRouteMaxLookups;                                            // [kRouteMaxLookups]
@@ -755,7 +760,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
                 if (u < n_units && mm < g.M && nn < g.N) load_x_four(g, mm, nn, xv[i], EPI);
             }
         }
-        if (routing) route_n = route_stage(gp.route, m0 + r_begin, max(0, min(r_end, g.M - m0) - r_begin), s_off, s_look, s_rel, kPlThreads);
+        if (routing) route_n = route_stage(route, m0 + r_begin, max(0, min(r_end, g.M - m0) - r_begin), s_off, s_look, s_rel, kPlThreads);
         __syncthreads();
         if (clustered) {
             cluster_wait();
@@ -839,7 +844,7 @@ k_tc_planes(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneM
     }
     if (routing) {
         __syncthreads();  // the finished rows are in `fin`
-        route_rows<BN>(gp.route, gp.route.mode[which], fin, s_look, s_rel, route_n, n0, g.N, kPlThreads);
+        route_rows<BN>(route, gp.route_mode[which], fin, s_look, s_rel, route_n, n0, g.N, kPlThreads);
     }
     tc_fence_before();
     __syncthreads();
@@ -885,7 +890,7 @@ __device__ __forceinline__ void accumulating_warps_sync() {
 // in this form, hidden rows 35.5 and 39.3; one kernel serves both launches, at 5 of the pass's 120 us less than the other form.
 template <int EPI>
 __global__ void __launch_bounds__(kHalfThreads, 1)
-k_half_tiles(const __grid_constant__ PlanePair gp, const __grid_constant__ PlaneMaps maps) {
+k_half_tiles(const __grid_constant__ PlaneSet gp, const __grid_constant__ PlaneMaps maps) {
     static_assert(EPI == EPI_STORE || EPI == EPI_L2_DISTANCE || EPI == EPI_ADD_TABLE_VALUE, "ranking's epilogues");
     constexpr int BN = 128, CPT = BN / 4, kQuads = BN / 4, kAccThreads = 32 * kHalfAccWarps;
     extern __shared__ uint8_t smem_raw[];
@@ -1307,37 +1312,45 @@ inline int max_resident_plane_clusters(int splits) {
 // A launch with its tensor maps encoded (encoding costs the host a few microseconds per map; a
 // launch that is repeated, or captured into a graph, pays it once).
 struct PlaneLaunch {
-    PlanePair gp;
+    PlaneSet gp;
     PlaneMaps maps;
     dim3 grid;
     int splits, tile_n;
 };
 
-// One or two contractions of the same kind in one launch, tiles of 128 x tile_n (64 or 128).
+// What the finished rows of a launch's problems go to: one set of lookups per shard, `per_shard` problems each, of which
+// the i-th routes what mode[i] says.
+struct Routing {
+    const RouteArgs* shards;
+    int n_shards, per_shard;
+    int mode[2];
+};
+
+// Contractions of the same kind in one launch, tiles of 128 x tile_n (64 or 128).
 // splits > 1: the blocks of a tile form a cluster (at most kMaxClusterSplits) and g.k_per_split
 // must be set accordingly by the caller.
 inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, int splits, int tile_n, PlaneLaunch* out,
                                   const ExchangeSync& sync = ExchangeSync{}, int wait_kind = -1, int signal_kind = -1,
-                                  const RouteArgs* route = nullptr) {
-    if (splits < 1 || splits > kMaxClusterSplits || (tile_n != 64 && tile_n != 128)) return cudaErrorInvalidValue;
-    PlanePair& gp = out->gp;
-    gp = PlanePair{};
-    gp.p[0] = problems[0];
-    gp.p[1] = problems[n_problems > 1 ? 1 : 0];
-    gp.tiles_m0 = (problems[0].g.M + kBM - 1) / kBM;
+                                  const Routing* routing = nullptr) {
+    if (splits < 1 || splits > kMaxClusterSplits || (tile_n != 64 && tile_n != 128) || n_problems < 1 || n_problems > kMaxPlaneProblems) return cudaErrorInvalidValue;
+    PlaneSet& gp = out->gp;
+    gp = PlaneSet{};
+    gp.n_problems = n_problems;
     gp.sync = sync;
     gp.wait_kind = wait_kind;
     gp.signal_kind = signal_kind;
-    if (route) gp.route = *route;
-    int tiles_m = gp.tiles_m0, tiles_n = (problems[0].g.N + tile_n - 1) / tile_n;
-    if (n_problems > 1) {
-        tiles_m += (problems[1].g.M + kBM - 1) / kBM;
-        tiles_n = std::max(tiles_n, (problems[1].g.N + tile_n - 1) / tile_n);
-    }
+    if (routing)
+        for (int i = 0; i < routing->n_shards; ++i) gp.route[i] = routing->shards[i];
+    int tiles_m = 0, tiles_n = 1;
     auto type_of = [](const PlaneOperand& op) { return op.elem_bytes == 16 ? 2 : op.elem_bytes == 2 ? 1 : 0; };
     gp.bf16 = type_of(problems[0].A);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < n_problems; ++i) {
         PlaneProblem& q = gp.p[i];
+        q = problems[i];
+        tiles_m += (q.g.M + kBM - 1) / kBM;
+        tiles_n = std::max(tiles_n, (q.g.N + tile_n - 1) / tile_n);
+        gp.tiles_end[i] = tiles_m;
+        if (routing) gp.route_of[i] = i / routing->per_shard, gp.route_mode[i] = routing->mode[i % routing->per_shard];
         if (type_of(q.A) != gp.bf16 || type_of(q.B) != gp.bf16) return cudaErrorInvalidValue;
         if (gp.bf16 == 1 && (q.A.lo || q.B.lo || q.g.k_per_split % 64)) return cudaErrorInvalidValue;
         if (gp.bf16 == 2 && (!q.B.lo || n_problems != 1 || splits != 1 || tile_n != 128)) return cudaErrorInvalidValue;
@@ -1389,7 +1402,7 @@ template <int SIDE>
 inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
     if (SIDE != SIDE_NONE && l.gp.bf16 == 1) return cudaErrorInvalidValue;  // the side sums read fp32 tiles
     if (SIDE == SIDE_NORMS)
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < l.gp.n_problems; ++i)
             if (l.gp.p[i].A.mn_major || l.gp.p[i].B.mn_major || l.gp.p[i].g.out_blocks) return cudaErrorInvalidValue;
     if (l.gp.bf16 == 2) {
         const int epilogue = l.gp.p[0].g.epilogue;
@@ -1402,7 +1415,9 @@ inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
     if (l.tile_n == 128) {
         // one epilogue for the launch: the instantiation for it
         const int epilogue = l.gp.p[0].g.epilogue;
-        if (l.gp.p[1].g.epilogue == epilogue) {
+        bool alike = true;
+        for (int i = 1; i < l.gp.n_problems; ++i) alike = alike && l.gp.p[i].g.epilogue == epilogue;
+        if (alike) {
             if constexpr (SIDE == SIDE_NONE) {
                 if (l.gp.bf16) {
                     if (epilogue == EPI_STORE) return l.splits > 1 ? launch_lean<SIDE_NONE, EPI_STORE, 7, true>(l, stream) : launch_lean<SIDE_NONE, EPI_STORE, 0, true>(l, stream);
@@ -1431,9 +1446,9 @@ inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
 template <int SIDE>
 inline cudaError_t launch_planes(const PlaneProblem* problems, int n_problems, int splits, int tile_n, cudaStream_t stream,
                                  const ExchangeSync& sync = ExchangeSync{}, int wait_kind = -1, int signal_kind = -1,
-                                 const RouteArgs* route = nullptr) {
+                                 const Routing* routing = nullptr) {
     PlaneLaunch l;
-    cudaError_t err = prepare_planes(problems, n_problems, splits, tile_n, &l, sync, wait_kind, signal_kind, route);
+    cudaError_t err = prepare_planes(problems, n_problems, splits, tile_n, &l, sync, wait_kind, signal_kind, routing);
     if (err != cudaSuccess) return err;
     return launch_prepared<SIDE>(l, stream);
 }

@@ -4,10 +4,9 @@
 //   pt_i = h_i - n_i (n_i . h_i) + r_i                  (the predicted tail)
 //   e_ijk = pt_ik - (t_jk - n_ik (n_i . t_j))
 //   score_ij = gamma - sum_k |e_ijk|                     (always the L1 form, whatever model.distance_fn says).
-// Four kernels: the predicted tails of a batch, the pairwise distances with the two [B, T]
-// matrices the backward needs (s_ij = n_i . t_j and u_ij = sum_k sign(e_ijk) n_ik), the gradients
-// of the distance with respect to pt, n and the tails, and the backward of the prediction down to
-// the head rows, the translation rows and the raw normals.  FP32-pipe kernels; every sum has a fixed order.
+// Here are the pairwise distances with the two [B, T] matrices the backward needs (s_ij = n_i . t_j and
+// u_ij = sum_k sign(e_ijk) n_ik) and the gradients of the distance with respect to pt, n and the tails; the prediction and
+// its backward down to the head rows, the translation rows and the raw normals are k_lookup and k_lookup_bwd.  FP32-pipe kernels; every sum has a fixed order.
 #pragma once
 
 #include <algorithm>
@@ -15,33 +14,6 @@
 #include "kernels.cuh"
 
 namespace kge {
-
-// pred[i] = pt_i, nrm[i] = n_i.  One block of 64 threads per triple.
-static __global__ void __launch_bounds__(64)
-k_transh_predict(const float* __restrict__ hid_h, const uint32_t* __restrict__ head, const uint32_t* __restrict__ relation,
-                 const float* __restrict__ rel_table, const float* __restrict__ normal_table, float* __restrict__ pred,
-                 float* __restrict__ nrm, int D) {
-    grid_dependency_sync();
-    __shared__ float scratch[2];
-    const int i = blockIdx.x;
-    const float* __restrict__ h = hid_h + (size_t)head[i] * D;
-    const float* __restrict__ r = rel_table + (size_t)relation[i] * D;
-    const float* __restrict__ w = normal_table + (size_t)relation[i] * D;
-    float ww = 0.f, wh = 0.f;
-    for (int k = threadIdx.x; k < D; k += 64) {
-        ww += w[k] * w[k];
-        wh += w[k] * h[k];
-    }
-    ww = block_sum<64>(ww, scratch);
-    wh = block_sum<64>(wh, scratch);
-    const float inv = 1.f / sqrtf(ww);
-    const float nh = wh * inv;  // n . h
-    for (int k = threadIdx.x; k < D; k += 64) {
-        const float n = w[k] * inv;
-        nrm[(size_t)i * D + k] = n;
-        pred[(size_t)i * D + k] = h[k] - n * nh + r[k];
-    }
-}
 
 // raw[i, j] = sum_k |e_ijk|, and (BACKWARD) S[i, j] = n_i . t_j, U[i, j] = sum_k sign(e_ijk) n_ik.
 // A warp owns 4 x 8 outputs with its lanes along k (lane l has k = l, l + 32, ...), so that a row is read in whole
@@ -68,10 +40,21 @@ __device__ __forceinline__ float reduce_to_lanes(float (&sums)[32]) {
     return sums[0];
 }
 
+struct TranshScoreArgs {
+    const float *pt, *nrm, *tails;
+    float *raw, *S, *U;  // [B, ld]
+};
+
 template <bool BACKWARD>
 __global__ void __launch_bounds__(32 * kTranshWarps, 2)
-k_transh_score(const float* __restrict__ pt, const float* __restrict__ nrm, const float* __restrict__ tails, float* __restrict__ raw,
-               float* __restrict__ S, float* __restrict__ U, int B, int T, int D, ExchangeSync sync) {
+k_transh_score(const __grid_constant__ ShardArgs<TranshScoreArgs> shards, int B, int T, int D, int ld, ExchangeSync sync) {
+    const TranshScoreArgs& args = shards.s[blockIdx.z];
+    const float* __restrict__ pt = args.pt;
+    const float* __restrict__ nrm = args.nrm;
+    const float* __restrict__ tails = args.tails;
+    float* __restrict__ raw = args.raw;
+    float* __restrict__ S = args.S;
+    float* __restrict__ U = args.U;
     grid_dependency_sync();
     exchange_wait(sync, XCHG_TAILS);  // the tails come from the other processes
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -94,7 +77,7 @@ k_transh_score(const float* __restrict__ pt, const float* __restrict__ nrm, cons
     for (int b = 0; b < kTranshCols; ++b) row_j[b] = (uint32_t)(min(j0 + b, T - 1) - from_j) * (uint32_t)D;
     const int i = i0 + lane / kTranshCols, j = j0 + lane % kTranshCols;  // the output whose totals this lane ends up with
     const bool live = i < B && j < T;
-    const size_t out = (size_t)i * T + j;
+    const size_t out = (size_t)i * ld + j;
 
     // two neighbouring tails at a time
     constexpr int kPairs = kTranshCols / 2;
@@ -167,14 +150,20 @@ k_transh_score(const float* __restrict__ pt, const float* __restrict__ nrm, cons
 }
 
 // S and U null: the distances alone (predict).
-inline cudaError_t launch_transh_score(const float* pt, const float* nrm, const float* tails, float* raw, float* S, float* U, int B, int T, int D,
-                                       const ExchangeSync& sync, cudaStream_t stream) {
+inline cudaError_t launch_transh_score(const ShardArgs<TranshScoreArgs>& shards, int n_shards, int B, int T, int D, int ld, const ExchangeSync& sync,
+                                       cudaStream_t stream) {
     constexpr int kCols = kTranshCols * kTranshWarps;
-    const dim3 grid((B + kTranshRows - 1) / kTranshRows, (T + kCols - 1) / kCols), block(32 * kTranshWarps);
-    if (S && (uint64_t)std::max(B, T) * D > UINT32_MAX) return cudaErrorInvalidValue;
+    const dim3 grid((B + kTranshRows - 1) / kTranshRows, (T + kCols - 1) / kCols, (unsigned)n_shards), block(32 * kTranshWarps);
+    const bool backward = shards.s[0].S != nullptr;
+    if (backward && (uint64_t)std::max(B, T) * D > UINT32_MAX) return cudaErrorInvalidValue;
     if (T > kTranshMaxTails) return cudaErrorInvalidValue;
-    if (S) return launch_dependent(k_transh_score<true>, grid, block, 0, stream, pt, nrm, tails, raw, S, U, B, T, D, sync);
-    return launch_dependent(k_transh_score<false>, grid, block, 0, stream, pt, nrm, tails, raw, S, U, B, T, D, sync);
+    if (backward) return launch_dependent(k_transh_score<true>, grid, block, 0, stream, shards, B, T, D, ld, sync);
+    return launch_dependent(k_transh_score<false>, grid, block, 0, stream, shards, B, T, D, ld, sync);
+}
+inline cudaError_t launch_transh_score(const float* pt, const float* nrm, const float* tails, float* raw, int B, int T, int D, cudaStream_t stream) {
+    ShardArgs<TranshScoreArgs> shards{};
+    shards.s[0] = TranshScoreArgs{pt, nrm, tails, raw, nullptr, nullptr};
+    return launch_transh_score(shards, 1, B, T, D, T, ExchangeSync{}, stream);
 }
 
 // Gradients of the distances times C [B, T] (C = d loss / d raw), with sg_ijk = sign(pt_ik - t_jk + n_ik S_ij):
@@ -189,7 +178,7 @@ struct TranshBwdArgs {
     const float *pt, *nrm, *tails, *C, *S, *U;
     float *d_pt, *d_n;
     float* const* d_tail_blocks;
-    int block_rows, B, T, D, blocks_i;
+    int block_rows, B, T, D, ld, blocks_i;  // ld: floats between rows of C, S and U; what lies between T and ld is zero
 };
 constexpr int kTranshBwdCols = 32, kTranshChunkI = 64, kTranshChunkJ = 32;
 constexpr int kTranshStage = 3 * kPairWarps * kTranshChunkI + kTranshChunkI * kTranshBwdCols;  // floats of one chunk
@@ -205,11 +194,11 @@ __device__ __forceinline__ void transh_bwd_triples(const TranshBwdArgs& g, int b
     const int D = g.D, T = g.T, col_tiles = (D + kCols - 1) / kCols;
     const int i0 = block / col_tiles * kPairWarps, k0 = block % col_tiles * kCols;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = i0 + warp, k = k0 + lane;
-    const bool t_vec = (D & 3) == 0, c_vec = (T & 3) == 0, live = i < g.B && k < D;
+    const bool t_vec = (D & 3) == 0, c_vec = (g.ld & 3) == 0, live = i < g.B && k < D;
     auto stage = [&](int j0, float* to) {
         const float* planes[3] = {g.C, g.S, g.U};
 #pragma unroll
-        for (int q = 0; q < 3; ++q) stage_rows<kPairWarps, kChunk>(to + q * kPlane, planes[q] + (size_t)i0 * T + j0, T, g.B - i0, T - j0, c_vec);
+        for (int q = 0; q < 3; ++q) stage_rows<kPairWarps, kChunk>(to + q * kPlane, planes[q] + (size_t)i0 * g.ld + j0, g.ld, g.B - i0, T - j0, c_vec);
         stage_rows<kChunk, kCols>(to + 3 * kPlane, g.tails + (size_t)j0 * D + k0, D, T - j0, D - k0, t_vec);
     };
     const float p = live ? g.pt[(size_t)i * D + k] : 0.f, n = live ? g.nrm[(size_t)i * D + k] : 0.f;
@@ -246,11 +235,11 @@ __device__ __forceinline__ void transh_bwd_tails(const TranshBwdArgs& g, int blo
     const int D = g.D, T = g.T, B = g.B, col_tiles = (D + kCols - 1) / kCols;
     const int j0 = block / col_tiles * kRows, k0 = block % col_tiles * kCols;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, j = j0 + 2 * warp, k = k0 + lane;
-    const bool vec = (D & 3) == 0, c_vec = (T & 3) == 0;
+    const bool vec = (D & 3) == 0, c_vec = (g.ld & 3) == 0;
     auto stage = [&](int i0, float* to) {
         const float* planes[3] = {g.C, g.S, g.U};
 #pragma unroll
-        for (int q = 0; q < 3; ++q) stage_rows<kChunk, kRows>(to + q * kPlane, planes[q] + (size_t)i0 * T + j0, T, B - i0, T - j0, c_vec);
+        for (int q = 0; q < 3; ++q) stage_rows<kChunk, kRows>(to + q * kPlane, planes[q] + (size_t)i0 * g.ld + j0, g.ld, B - i0, T - j0, c_vec);
         stage_rows<kChunk, kCols>(to + 3 * kPlane, g.pt + (size_t)i0 * D + k0, D, B - i0, D - k0, vec);
         stage_rows<kChunk, kCols>(to + 3 * kPlane + kWide, g.nrm + (size_t)i0 * D + k0, D, B - i0, D - k0, vec);
     };
@@ -282,53 +271,20 @@ __device__ __forceinline__ void transh_bwd_tails(const TranshBwdArgs& g, int blo
         if (j + r < T && k < D) g.d_tail_blocks[(j + r) / g.block_rows][(size_t)((j + r) % g.block_rows) * D + k] = acc[r];
 }
 
-static __global__ void __launch_bounds__(32 * kPairWarps, 4) k_transh_bwd(TranshBwdArgs g) {
+static __global__ void __launch_bounds__(32 * kPairWarps, 4) k_transh_bwd(const __grid_constant__ ShardArgs<TranshBwdArgs> shards) {
     grid_dependency_sync();
+    const TranshBwdArgs& g = shards.s[blockIdx.y];
     __shared__ __align__(16) float smem[2][kTranshStage];
     if ((int)blockIdx.x < g.blocks_i) transh_bwd_triples(g, blockIdx.x, smem);
     else transh_bwd_tails(g, (int)blockIdx.x - g.blocks_i, smem);
 }
 
-inline cudaError_t launch_transh_bwd(TranshBwdArgs g, cudaStream_t stream) {
+inline cudaError_t launch_transh_bwd(ShardArgs<TranshBwdArgs> shards, int n_shards, cudaStream_t stream) {
+    const TranshBwdArgs& g = shards.s[0];
     const int col_tiles = (g.D + kTranshBwdCols - 1) / kTranshBwdCols;
-    g.blocks_i = (g.B + kPairWarps - 1) / kPairWarps * col_tiles;
-    const int blocks_j = (g.T + 2 * kPairWarps - 1) / (2 * kPairWarps) * col_tiles;
-    return launch_dependent(k_transh_bwd, dim3(g.blocks_i + blocks_j), dim3(32 * kPairWarps), 0, stream, g);
-}
-
-// Backward of k_transh_predict for triple i:
-//   d_head = d_pt - n (n . d_pt),   d_relrow = d_pt,
-//   d_n (total) = d_n - (n . h) d_pt - h (n . d_pt),   d_normrow = (d_n - n (n . d_n)) / |w|.
-static __global__ void __launch_bounds__(64)
-k_transh_pred_bwd(const float* __restrict__ d_pt, const float* __restrict__ d_n, const float* __restrict__ hid_h,
-                  const uint32_t* __restrict__ head, const uint32_t* __restrict__ relation, const float* __restrict__ normal_table,
-                  const float* __restrict__ nrm, float* __restrict__ d_head, float* __restrict__ d_relrow,
-                  float* __restrict__ d_normrow, int D) {
-    grid_dependency_sync();
-    __shared__ float scratch[2];
-    const int i = blockIdx.x;
-    const float* __restrict__ h = hid_h + (size_t)head[i] * D;
-    const float* __restrict__ w = normal_table + (size_t)relation[i] * D;
-    const size_t o = (size_t)i * D;
-    float ww = 0.f, nh = 0.f, ndp = 0.f;
-    for (int k = threadIdx.x; k < D; k += 64) {
-        ww += w[k] * w[k];
-        nh += nrm[o + k] * h[k];
-        ndp += nrm[o + k] * d_pt[o + k];
-    }
-    ww = block_sum<64>(ww, scratch);
-    nh = block_sum<64>(nh, scratch);
-    ndp = block_sum<64>(ndp, scratch);
-    float ndn = 0.f;  // n . (total d_n)
-    for (int k = threadIdx.x; k < D; k += 64) ndn += nrm[o + k] * (d_n[o + k] - nh * d_pt[o + k] - h[k] * ndp);
-    ndn = block_sum<64>(ndn, scratch);
-    const float inv = 1.f / sqrtf(ww);
-    for (int k = threadIdx.x; k < D; k += 64) {
-        const float n = nrm[o + k], dp = d_pt[o + k];
-        d_head[o + k] = dp - n * ndp;
-        d_relrow[o + k] = dp;
-        d_normrow[o + k] = (d_n[o + k] - nh * dp - h[k] * ndp - n * ndn) * inv;
-    }
+    const int blocks_i = (g.B + kPairWarps - 1) / kPairWarps * col_tiles, blocks_j = (g.T + 2 * kPairWarps - 1) / (2 * kPairWarps) * col_tiles;
+    for (int s = 0; s < n_shards; ++s) shards.s[s].blocks_i = blocks_i;
+    return launch_dependent(k_transh_bwd, dim3(blocks_i + blocks_j, (unsigned)n_shards), dim3(32 * kPairWarps), 0, stream, shards);
 }
 
 }  // namespace kge

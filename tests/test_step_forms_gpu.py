@@ -58,3 +58,25 @@ def test_rows_straight_from_the_table(score_fn, distance_fn, d):
 def test_rows_straight_from_a_float16_table():
     # float16 rows: the bound of the other float16 tests
     _two_runs(_config("ComplEx", "MatMul", embedding_size=36, n_shard=2), seed=5, rtol=2e-2, dtype="float16")
+
+
+@pytest.mark.parametrize("n_shard", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("score_fn,distance_fn", [("TransE", "L1"), ("TransE", "L2"), ("DistMult", "MatMul"), ("RotatE", "L2"), ("TransH", "L1")])
+def test_batches_of_any_size(score_fn, distance_fn, n_shard):
+    """One launch for up to four shards, and a fifth in one of its own; batches and tails that fill no tile and no 16 bytes."""
+    cfg = _config(score_fn, distance_fn, n_shard=n_shard, batch_size=7 * n_shard, a2a_size=9, n_relation_type=2 * n_shard, embedding_size=20, entity_feature_size=n_shard * 6,
+                  loss_type="softmax", correction_weight=1.0)
+    _two_runs(cfg, seed=n_shard, rtol=1e-4, rel_rtol=2e-3 if score_fn == "RotatE" else None, feature_dtype="float16" if n_shard % 2 else None)
+
+
+@pytest.mark.parametrize("score_fn,distance_fn", [("TransE", "L1"), ("ComplEx", "MatMul"), ("TransH", "L1")])
+@pytest.mark.parametrize("fused", ["1", "0"])
+def test_shards_update_dense_parameters_together(monkeypatch, score_fn, distance_fn, fused):
+    """Relation rows that no, one and all shards name; the Adam step in the row update and in a kernel of its own."""
+    monkeypatch.setenv("KGE_FUSE_DENSE_UPDATE", fused)
+    cfg = _config(score_fn, distance_fn, n_shard=4, batch_size=8, a2a_size=5, n_relation_type=40, learning_rate_modifiers={"relation_embedding": 0.5})
+    _two_runs(cfg, seed=3, rtol=1e-4)
+
+
+def test_separate_networks_of_four_shards():
+    _two_runs(_config("TransE", "L2", n_shard=4, batch_size=12, a2a_size=7, embedding_size=36, entity_feature_size=12, share_feature_networks=False), seed=9, rtol=1e-4)
