@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "exchange.cuh"
 #include "pdl.cuh"
 
@@ -901,7 +903,7 @@ struct PairBwdProblem {
 struct PairBwdArgs {
     PairBwdProblem p[2];
     int D;
-    int tiles_m0;  // set by launch_pair_bwd
+    int longest;   // the problem with the longer sums, whose blocks start first; set by launch_pair_bwd
 };
 
 // Two neighbouring fp32 values in one 64-bit register pair.  An instruction issues both and holds the FP32 pipe as long as
@@ -929,6 +931,19 @@ __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, 0xbf800
 __device__ __forceinline__ float positive(float x, float infinity) {
     float r;
     asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(infinity));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// c with its sign flipped where e is negative: c * sign(e) unless e is 0 or NaN.
+__device__ __forceinline__ float flip_by(float c, float e) { return __uint_as_float(__float_as_uint(c) ^ (__float_as_uint(e) & 0x80000000u)); }
+// The smallest magnitude so far; NaN once one was.
+__device__ __forceinline__ float least_magnitude(float so_far, float a, float b) {
+    float r;
+    asm("min.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(so_far), "f"(a), "f"(b));
     return r;
 }
 // sign(e) of either value: 1, 0 or -1.  Comparisons run at half the FP32 pipe's rate; these products run at the full one.
@@ -975,22 +990,29 @@ __device__ __forceinline__ void store_pair(float* __restrict__ row, int k, int D
 // result: the coefficients of a softmax row add up to zero, so where (nearly) all differences of a column have one sign
 // the L1 gradient is the rounding left over from that sum, and Adam's first steps of a parameter do not depend on a
 // gradient's size.  (Dividing n over warps was no faster and moved relations by 1e-3.)  The block walks n in chunks of
-// 64, both operands staged in shared memory one chunk ahead.  Bound by the FP32 pipe, 4 issue slots a term, as many as
-// shared memory's wavefronts with one row per warp; two rows share a warp's reads of Y where the problem has blocks
-// enough for it.  The form before, 32 x 64 tiles of 128 threads without the look-ahead, had 48 blocks for a
-// 256 x 512 x 100 problem and stalled on every chunk (61 us for 256 x 320 x 64).
+// 64, both operands staged in shared memory one chunk ahead; two rows share a warp's reads of Y where the problem has
+// blocks enough for it.  Two L1 terms are a packed difference, two coefficients with the sign flipped by it, the smallest
+// magnitude so far and a packed sum: five instructions, where clamped products for the signs took eight.  A chunk in which
+// a difference was 0 or NaN, whose sign is 0 (a few per million terms of float32 values: too few to matter, and some in every
+// launch), is added up again with those products.  Bound by shared memory's wavefronts and by what is left uneven: blocks with
+// the longer sums start first, and two blocks per SM, not three or four, because a dependent launch's blocks pile up where
+// the kernel in front ends first (four shards of 256 x 512 x 100: 31 us, 43 and 56 with three and four blocks; 48 before
+// the three changes, when the blocks of a shard's two problems followed each other).  Four rows per warp: 51 us, too few
+// warps.  Tried and slower: threads dealt out over (rows, pairs of columns) without gaps, bulk copies of row pieces for
+// the staging (about 100 copies a chunk from one warp), and both operands read through L1 without any staging.
 constexpr int kPairChunk = 64;
 
 template <int FN, int ROWS>
-__global__ void __launch_bounds__(32 * kPairWarps, 3) k_pair_bwd(const __grid_constant__ ShardArgs<PairBwdArgs> shards) {
+__global__ void __launch_bounds__(32 * kPairWarps, 2) k_pair_bwd(const __grid_constant__ ShardArgs<PairBwdArgs> shards) {
     grid_dependency_sync();
     const PairBwdArgs& args = shards.s[blockIdx.y];
+    const int which = blockIdx.z == 0 ? args.longest : 1 - args.longest;
     constexpr int kRows = ROWS * kPairWarps, kCs = kRows * kPairChunk, kStage = kCs + kPairChunk * kPairCols;
     __shared__ __align__(16) float smem[2][kStage];  // C [kRows][chunk] or [chunk][kRows] | Y [chunk][cols]
     const int D = args.D, col_tiles = (D + kPairCols - 1) / kPairCols, tile_m = (int)blockIdx.x / col_tiles;
-    const int which = tile_m >= args.tiles_m0 ? 1 : 0;
     const PairBwdProblem& pr = args.p[which];
-    const int M = pr.M, N = pr.N, m0 = (tile_m - (which ? args.tiles_m0 : 0)) * kRows, k0 = (int)blockIdx.x % col_tiles * kPairCols;
+    const int M = pr.M, N = pr.N, m0 = tile_m * kRows, k0 = (int)blockIdx.x % col_tiles * kPairCols;
+    if (m0 >= M) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = m0 + warp * ROWS, k = k0 + lane * 2;
     const bool n_fast = pr.c_stride_n == 1, y_vec = (D & 3) == 0;  // else c_stride_m is 1
     const int c_stride = n_fast ? pr.c_stride_m : pr.c_stride_n;
@@ -1003,7 +1025,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, 3) k_pair_bwd(const __grid_co
     f32x2 x[ROWS], acc[ROWS];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
-        x[r] = m + r < M ? load_pair(pr.X + (size_t)(m + r) * D, k, D) : 0ull;
+        // (1 where there is no value: its difference to the zeros staged there is not 0)
+        x[r] = m + r < M && k < D ? load_pair(pr.X + (size_t)(m + r) * D, k, D) : 0x3f8000003f800000ull;
         acc[r] = 0ull;
     }
     stage(0, smem[0]);
@@ -1015,6 +1038,13 @@ __global__ void __launch_bounds__(32 * kPairWarps, 3) k_pair_bwd(const __grid_co
         __syncthreads();
         const float* cs = smem[half] + (n_fast ? warp * ROWS * kPairChunk : warp * ROWS);
         const float* ys = smem[half] + kCs + lane * 2;
+        f32x2 before[ROWS];
+        float least[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            before[r] = acc[r];
+            least[r] = 1.f;
+        }
 #pragma unroll 4
         for (int n = 0; n < kPairChunk; n += 4) {
             float c[ROWS][4];
@@ -1026,19 +1056,42 @@ __global__ void __launch_bounds__(32 * kPairWarps, 3) k_pair_bwd(const __grid_co
                 }
             } else {
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-#pragma unroll
-                    for (int r = 0; r < ROWS; ++r) c[r][u] = cs[(n + u) * kRows + r];
+                for (int u = 0; u < 4; ++u) {
+                    if (ROWS == 4) {
+                        const float4 q = load4(cs + (n + u) * kRows);
+                        c[0][u] = q.x; c[1 % ROWS][u] = q.y; c[2 % ROWS][u] = q.z; c[3 % ROWS][u] = q.w;
+                    } else if (ROWS == 2) {
+                        const float2 q = *reinterpret_cast<const float2*>(cs + (n + u) * kRows);
+                        c[0][u] = q.x; c[1 % ROWS][u] = q.y;
+                    } else {
+                        c[0][u] = cs[(n + u) * kRows];
+                    }
+                }
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const f32x2 y = *reinterpret_cast<const f32x2*>(ys + (n + u) * kPairCols);
 #pragma unroll
                 for (int r = 0; r < ROWS; ++r) {
-                    const f32x2 cc = pack2(c[r][u], c[r][u]);
-                    if (FN == DIST_DOT) acc[r] = fma2(cc, y, acc[r]);
-                    else if (FN == DIST_L2) acc[r] = fma2(cc, sub2(x[r], y), acc[r]);
-                    else acc[r] = fma2(cc, sign2(sub2(x[r], y)), acc[r]);
+                    if (FN == DIST_L1) {
+                        const float2 d = unpack2(sub2(x[r], y));
+                        least[r] = least_magnitude(least[r], d.x, d.y);
+                        acc[r] = add2(acc[r], pack2(flip_by(c[r][u], d.x), flip_by(c[r][u], d.y)));
+                    } else {
+                        acc[r] = fma2(pack2(c[r][u], c[r][u]), FN == DIST_DOT ? y : sub2(x[r], y), acc[r]);
+                    }
+                }
+            }
+        }
+        if (FN == DIST_L1) {
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                if (least[r] > 0.f) continue;
+                acc[r] = before[r];
+#pragma unroll 4
+                for (int n = 0; n < kPairChunk; ++n) {
+                    const float c = n_fast ? cs[r * kPairChunk + n] : cs[n * kRows + r];
+                    acc[r] = fma2(pack2(c, c), sign2(sub2(x[r], *reinterpret_cast<const f32x2*>(ys + n * kPairCols))), acc[r]);
                 }
             }
         }
@@ -1065,8 +1118,8 @@ inline cudaError_t launch_pair_bwd(ShardArgs<PairBwdArgs> shards, int n_shards, 
     auto tiles = [&](int which, int rows) { return (first.p[which].M + rows * kPairWarps - 1) / (rows * kPairWarps); };
     // two rows per warp where that still leaves two blocks per SM
     const int rows = (tiles(0, 2) + tiles(1, 2)) * col_tiles * n_shards >= 2 * 148 ? 2 : 1;
-    for (int s = 0; s < n_shards; ++s) shards.s[s].tiles_m0 = tiles(0, rows);
-    const dim3 grid((tiles(0, rows) + tiles(1, rows)) * col_tiles, (unsigned)n_shards), block(32 * kPairWarps);
+    for (int s = 0; s < n_shards; ++s) shards.s[s].longest = first.p[0].N >= first.p[1].N ? 0 : 1;
+    const dim3 grid(std::max(tiles(0, rows), tiles(1, rows)) * col_tiles, (unsigned)n_shards, 2), block(32 * kPairWarps);
     if (rows == 2) return launch_dependent(k_pair_bwd<FN, 2>, grid, block, 0, stream, shards);
     return launch_dependent(k_pair_bwd<FN, 1>, grid, block, 0, stream, shards);
 }
