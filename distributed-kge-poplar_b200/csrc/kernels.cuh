@@ -877,8 +877,8 @@ inline cudaError_t launch_loss(const ShardArgs<LossArgs>& shards, int n_shards, 
     // log-sigmoids, whose chains are longest, gets twice the threads: 256 x 1536 self-adversarial scores 12.7 to 9.5 us
     // (a softmax row of that length was 1 us slower with them).
     const dim3 grid((unsigned)B, (unsigned)n_shards);
-    if (lp.loss_fn == LOSS_LOGSIGMOID && lp.n_tail >= 1024) return launch_dependent(k_loss<512>, grid, dim3(512), 0, stream, shards, lp, inv_normaliser, lo_bf16);
-    return launch_dependent(k_loss<256>, grid, dim3(256), 0, stream, shards, lp, inv_normaliser, lo_bf16);
+    if (lp.loss_fn == LOSS_LOGSIGMOID && lp.n_tail >= 1024) return launch_spread<k_loss<512>>(grid, dim3(512), stream, shards, lp, inv_normaliser, lo_bf16);
+    return launch_spread<k_loss<256>>(grid, dim3(256), stream, shards, lp, inv_normaliser, lo_bf16);
 }
 
 // ---------------------------------------------------------------------------

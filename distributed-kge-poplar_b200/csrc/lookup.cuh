@@ -173,9 +173,9 @@ inline cudaError_t launch_lookup(const ShardArgs<LookupArgs>& shards, int n_shar
         constexpr int FN = decltype(fn)::value;
         const int warps = g.B * kHeadWarps<FN> + g.T + (shards.s[0].remote ? g.R : 0);
         const dim3 grid((unsigned)((warps + 7) / 8), (unsigned)n_shards);
-        if (value_type == 2) return launch_dependent(k_lookup<__nv_bfloat16, FN>, grid, dim3(256), 0, stream, shards, g);
-        if (value_type == 1) return launch_dependent(k_lookup<__half, FN>, grid, dim3(256), 0, stream, shards, g);
-        return launch_dependent(k_lookup<float, FN>, grid, dim3(256), 0, stream, shards, g);
+        if (value_type == 2) return launch_spread<k_lookup<__nv_bfloat16, FN>>(grid, dim3(256), stream, shards, g);
+        if (value_type == 1) return launch_spread<k_lookup<__half, FN>>(grid, dim3(256), stream, shards, g);
+        return launch_spread<k_lookup<float, FN>>(grid, dim3(256), stream, shards, g);
     };
     switch (score_fn) {
         case SCORE_DISTMULT: return with_type(std::integral_constant<int, SCORE_DISTMULT>{});
@@ -277,9 +277,9 @@ inline cudaError_t launch_lookup_bwd(const ShardArgs<LookupBwdArgs>& shards, int
     auto with_type = [&](auto fn) {
         constexpr int FN = decltype(fn)::value;
         const dim3 grid((unsigned)((B * kHeadWarps<FN> + 7) / 8), (unsigned)n_shards);
-        if (value_type == 2) return launch_dependent(k_lookup_bwd<__nv_bfloat16, FN>, grid, dim3(256), 0, stream, shards, rel_table, normal_table, B, D);
-        if (value_type == 1) return launch_dependent(k_lookup_bwd<__half, FN>, grid, dim3(256), 0, stream, shards, rel_table, normal_table, B, D);
-        return launch_dependent(k_lookup_bwd<float, FN>, grid, dim3(256), 0, stream, shards, rel_table, normal_table, B, D);
+        if (value_type == 2) return launch_spread<k_lookup_bwd<__nv_bfloat16, FN>>(grid, dim3(256), stream, shards, rel_table, normal_table, B, D);
+        if (value_type == 1) return launch_spread<k_lookup_bwd<__half, FN>>(grid, dim3(256), stream, shards, rel_table, normal_table, B, D);
+        return launch_spread<k_lookup_bwd<float, FN>>(grid, dim3(256), stream, shards, rel_table, normal_table, B, D);
     };
     switch (score_fn) {
         case SCORE_COMPLEX: return with_type(std::integral_constant<int, SCORE_COMPLEX>{});

@@ -15,6 +15,8 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 namespace kge {
 
 #ifdef __CUDACC__
@@ -69,6 +71,38 @@ template <typename... Params, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                     Args&&... args) {
     return launch_dependent_cluster(kernel, grid, block, smem, stream, 1u, static_cast<Args&&>(args)...);
+}
+
+// A launch whose blocks are spread evenly over the SMs.  A dependent kernel's blocks are placed while its predecessor still
+// runs, on whatever SM has room for them first, and where an SM has room for eight a grid of 512 small blocks ends up on
+// half of the SMs.  Unused shared memory leaves each SM room for its share of the blocks and no more.  (The loss and the
+// lookups of a step launched this way: RotatE with features 88.2 to 86.1 us a step, ComplEx 76.4 to 74.6.  Kernels whose
+// blocks are long enough to be dealt out as others end, as the pair gradients, gained nothing or lost.)
+constexpr int kSmCount = 148;
+template <auto Kernel, typename... Args>
+inline cudaError_t launch_spread(dim3 grid, dim3 block, cudaStream_t stream, Args&&... args) {
+    struct Info {
+        int natural, static_bytes;  // blocks of an SM without the unused memory; natural 0: not asked yet
+    };
+    static Info known[kMaxDeviceOrdinals] = {};
+    const int slot = current_device_slot();
+    Info info = slot >= 0 ? known[slot] : Info{};
+    if (info.natural == 0) {
+        cudaFuncAttributes attributes;
+        cudaError_t err = cudaFuncGetAttributes(&attributes, Kernel);
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(Kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        info.static_bytes = (int)attributes.sharedSizeBytes;
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - info.static_bytes);
+        if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&info.natural, Kernel, (int)(block.x * block.y * block.z), 0);
+        if (err != cudaSuccess) return err;
+        if (slot >= 0) known[slot] = info;
+    }
+    const int share = (int)(((long long)grid.x * grid.y * grid.z + kSmCount - 1) / kSmCount);
+    // a block takes its memory and 1 KB of the SM's 228: so much that share + 1 blocks do not fit
+    int unused = 0;
+    if (share < info.natural) unused = std::min(228 * 1024 / (share + 1) + 128, 228 * 1024 / share) - 1024 - info.static_bytes;
+    unused = std::max(0, std::min(unused, 227 * 1024 - info.static_bytes)) / 128 * 128;
+    return launch_dependent(Kernel, grid, block, (size_t)unused, stream, static_cast<Args&&>(args)...);
 }
 
 }  // namespace kge
