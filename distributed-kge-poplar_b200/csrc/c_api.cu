@@ -632,7 +632,7 @@ int kge_microbench_rows(int kind, size_t table_rows, size_t d, const uint32_t* i
 }
 
 // Scores of m queries against n shared tails, k deep, device-resident: fn 0 = L1 and 1 = L2 on the
-// FP32 pipe (k_score_wide), 2 = dot product and 3 = L2 in the form |a|^2 + |b|^2 - 2 a.b on the tensor
+// FP32 pipe (k_score_block, k_score_tile), 2 = dot product and 3 = L2 in the form |a|^2 + |b|^2 - 2 a.b on the tensor
 // cores (k_tc_planes, 3xTF32).
 int kge_microbench_scores(int fn, size_t m, size_t n, size_t k, int repeat, float* mean_us) {
     return guarded(g_error, [&] {

@@ -463,116 +463,175 @@ __global__ void __launch_bounds__(128) k_score(const __grid_constant__ ShardArgs
     }
 }
 
-// The same scores for rows that allow 16-byte copies (D a multiple of 4, 16-byte aligned bases).
-// A block owns a 32x32 tile of outputs and its 8 warps divide the k range in chunks of 32: warp w
-// copies its own 32x32 chunk of both operands into its private part of shared memory (asynchronous
-// 16-byte copies, row-major with a stride of 36 floats, which keeps the 128-bit reads below free of
-// bank conflicts), accumulates a 4x8 register tile per lane over the chunk, and the 8 partial tiles
-// are added through shared memory at the end.  Splitting k, not the tile, is what gives every SM
-// several warps of independent work on a problem of only B x T = 512 x 768 outputs.
-constexpr int kScoreStride = 36;
-constexpr int kScoreWarps = 8;
-constexpr size_t kScoreWideSmem = (size_t)kScoreWarps * 2 * 32 * kScoreStride * sizeof(float);
-
+// The same scores for rows that allow 16-byte copies (D a multiple of 4, 16-byte aligned bases).  A block owns 64 x 4 NB
+// outputs and its 8 warps take 32 rows each in four groups that divide k in chunks of 32: a group copies its chunks of both
+// operands into its own part of shared memory (asynchronous 16-byte copies, row-major with a stride of 36 floats, which
+// keeps the 128-bit reads below free of bank conflicts), one ahead of the one it adds up in register tiles of 4 x NB per lane.
+// A chunk is summed by itself (with the chunk eight further on, and so on), and the chunks' sums are added in order at the
+// end: the order is part of an L1 model's result (see k_pair_bwd).  Bound by the FP32 pipe, two instructions per pair of
+// elements, and by the operands' way from L2, of which wider tiles need less; the width is chosen so that the blocks come to
+// whole waves of 148.  512 x 768 x 256 L2 scores: 13.8 us back to back with 48 columns a block, 16.4 with 64, 17.9 with 32.
+// With 32 x 32 outputs per block, its 8 warps dividing k and no chunk ahead, steps took (us, before -> after) TransE-L2 at that
+// size 72.6 -> 71.3, two shards of it 113.2 -> 109.6, RotatE-L2 256 x 1536 x 256 86.1 -> 82.9, four shards of 256 x 512 x 100
+// L1 scores 63.4 -> 59.0.  (Two blocks per SM, and two or four steps of k unrolled, were no faster.)
+constexpr int kScoreStride = 36, kScoreRows = 64, kScoreGroups = 4;
 __device__ __forceinline__ void score_copy16(float* dst_smem, const float* src) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst_smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
 }
-
 template <int FN>
-__global__ void __launch_bounds__(32 * kScoreWarps, 3)
-k_score_wide(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, int D, int ld, ExchangeSync sync) {
+__device__ __forceinline__ void score_add(float& sum, float4 p, float4 t) {
+    const float pr[4] = {p.x, p.y, p.z, p.w}, tr[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        if (FN == DIST_L1) {
+            sum += fabsf(pr[c] - tr[c]);
+        } else if (FN == DIST_L2) {
+            const float d = pr[c] - tr[c];
+            sum = fmaf(d, d, sum);
+        } else {
+            sum = fmaf(pr[c], tr[c], sum);
+        }
+    }
+}
+template <int NB>
+constexpr int kScoreStage = (kScoreRows + 4 * NB) * kScoreStride;  // floats of a group's chunk
+template <int NB>
+constexpr size_t kScoreBlockSmem = (size_t)kScoreGroups * 2 * kScoreStage<NB> * sizeof(float);
+
+// WIDE: more than four chunks of k.
+template <int FN, int NB, bool WIDE>
+__global__ void __launch_bounds__(256, 1)
+k_score_block(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, int D, int ld, ExchangeSync sync) {
     const float* __restrict__ P = shards.s[blockIdx.z].P;
     const float* __restrict__ Tl = shards.s[blockIdx.z].Tl;
     float* __restrict__ raw = shards.s[blockIdx.z].raw;
     grid_dependency_sync();
     exchange_wait(sync, XCHG_TAILS);  // the tail rows come from the other processes
     extern __shared__ __align__(16) float score_smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
-    float* Ps = score_smem + (size_t)warp * 2 * 32 * kScoreStride;
-    float* Ts = Ps + 32 * kScoreStride;
-    const int ty = lane >> 2, tx = lane & 3;  // p rows ty + 8a, t rows tx + 4b
-    const int n_chunks = (D + 31) / 32;
-    float acc[4][8];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
-
-    for (int chunk = warp; chunk < n_chunks; chunk += kScoreWarps) {
-        const int k0 = chunk * 32;
-        __syncwarp();
-#pragma unroll 2
-        for (int it = 0; it < 8; ++it) {
-            const int row = it * 4 + (lane >> 3), k4 = (lane & 7) * 4;
-            float* pd = Ps + row * kScoreStride + k4;
-            float* td = Ts + row * kScoreStride + k4;
-            if (i0 + row < B && k0 + k4 < D) score_copy16(pd, P + (size_t)(i0 + row) * D + k0 + k4);
-            else *reinterpret_cast<float4*>(pd) = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (j0 + row < T && k0 + k4 < D) score_copy16(td, Tl + (size_t)(j0 + row) * D + k0 + k4);
-            else *reinterpret_cast<float4*>(td) = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, group = warp >> 1, in_group = threadIdx.x & 63;
+    const int i0 = blockIdx.y * kScoreRows, j0 = blockIdx.x * 4 * NB, n_chunks = (D + 31) / 32;
+    float* const mine = score_smem + group * 2 * kScoreStage<NB>;
+    auto stage = [&](int chunk, float* to) {
+        const int k0 = chunk * 32, k4 = (in_group & 7) * 4;
+#pragma unroll 4
+        for (int row = in_group >> 3; row < kScoreRows + 4 * NB; row += 8) {
+            const bool is_p = row < kScoreRows;
+            const int g = is_p ? i0 + row : j0 + row - kScoreRows;
+            float* d = to + row * kScoreStride + k4;
+            if (g < (is_p ? B : T) && k0 + k4 < D) score_copy16(d, (is_p ? P : Tl) + (size_t)g * D + k0 + k4);
+            else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncwarp();
-#pragma unroll 1
-        for (int k4 = 0; k4 < 32; k4 += 4) {
-            float4 pv[4];
+    };
+    auto group_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(group + 1) : "memory"); };
+    auto commit = [&] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    constexpr int kSets = WIDE ? 2 : 1;  // the sums of the group's chunks that are even and odd among its own
+    float acc[kSets][4][NB];
 #pragma unroll
-            for (int a = 0; a < 4; ++a) pv[a] = load4(Ps + (ty + 8 * a) * kScoreStride + k4);
-#pragma unroll
-            for (int half = 0; half < 4; ++half) {
-                float4 tv[2];
-#pragma unroll
-                for (int b = 0; b < 2; ++b) tv[b] = load4(Ts + (tx + 4 * (half * 2 + b)) * kScoreStride + k4);
-#pragma unroll
-                for (int a = 0; a < 4; ++a)
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        const float pr[4] = {pv[a].x, pv[a].y, pv[a].z, pv[a].w};
-                        const float tr[4] = {tv[b].x, tv[b].y, tv[b].z, tv[b].w};
-                        float& sum = acc[a][half * 2 + b];
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            if (FN == DIST_L1) {
-                                sum += fabsf(pr[c] - tr[c]);
-                            } else if (FN == DIST_L2) {
-                                const float d = pr[c] - tr[c];
-                                sum = fmaf(d, d, sum);
-                            } else {
-                                sum = fmaf(pr[c], tr[c], sum);
-                            }
-                        }
-                    }
-            }
-        }
-    }
-    // add the warps' partial tiles: red[warp][p row][t row], stride 33
-    __syncthreads();
-    float* red = score_smem;
-    const int n_active = n_chunks < kScoreWarps ? n_chunks : kScoreWarps;
-    if (warp < n_active) {
+    for (int s = 0; s < kSets; ++s)
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int b = 0; b < 8; ++b) red[(warp * 32 + ty + 8 * a) * 33 + tx + 4 * b] = acc[a][b];
-    }
-    __syncthreads();
+            for (int b = 0; b < NB; ++b) acc[s][a][b] = 0.f;
+    const int ty = lane >> 2, tx = lane & 3;  // rows ty + 8a of the warp's 32, columns tx + 4b
+    auto add_chunk = [&](int chunk, const float* from, float (&sums)[4][NB]) {
+        const float* Ps = from + ((warp & 1) * 32 + ty) * kScoreStride;
+        const float* Ts = from + (kScoreRows + tx) * kScoreStride;
+        const int k_end = min(32, D - chunk * 32);
+#pragma unroll 1
+        for (int k4 = 0; k4 < k_end; k4 += 4) {
+            float4 pv[4];
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        const int o = threadIdx.x + it * 32 * kScoreWarps, prow = o >> 5, trow = o & 31;
-        float sum = 0.f;
-        for (int w = 0; w < n_active; ++w) sum += red[(w * 32 + prow) * 33 + trow];
-        const int i = i0 + prow, j = j0 + trow;
-        if (i < B && j < T) raw[(size_t)i * ld + j] = FN == DIST_L2 ? sqrtf(sum) : sum;
+            for (int a = 0; a < 4; ++a) pv[a] = load4(Ps + 8 * a * kScoreStride + k4);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const float4 tv = load4(Ts + 4 * b * kScoreStride + k4);
+#pragma unroll
+                for (int a = 0; a < 4; ++a) score_add<FN>(sums[a][b], pv[a], tv);
+            }
+        }
+    };
+    if (group < n_chunks) stage(group, mine);
+    commit();
+    if (WIDE && group + kScoreGroups < n_chunks) stage(group + kScoreGroups, mine + kScoreStage<NB>);
+    commit();
+    for (int chunk = group; chunk < n_chunks; chunk += 2 * kScoreGroups) {
+#pragma unroll
+        for (int s = 0; s < kSets; ++s) {
+            const int c = chunk + s * kScoreGroups;
+            if (c >= n_chunks) break;
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            group_sync();
+            add_chunk(c, mine + s * kScoreStage<NB>, acc[s]);
+            if (WIDE && c + 2 * kScoreGroups < n_chunks) {
+                group_sync();
+                stage(c + 2 * kScoreGroups, mine + s * kScoreStage<NB>);
+            }
+            commit();
+        }
+    }
+    // add the chunks' sums: red[chunk modulo 8][row][column]
+    __syncthreads();
+    constexpr int kPitch = 4 * NB + 4;
+    static_assert((WIDE ? 8 : 4) * kScoreRows * kPitch <= kScoreGroups * 2 * kScoreStage<NB>, "the sums fit where the operands were");
+#pragma unroll
+    for (int s = 0; s < kSets; ++s)
+        if (group + s * kScoreGroups < n_chunks) {
+            float* red = score_smem + ((group + s * kScoreGroups) * kScoreRows + (warp & 1) * 32 + ty) * kPitch + tx;
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < NB; ++b) red[8 * a * kPitch + 4 * b] = acc[s][a][b];
+        }
+    __syncthreads();
+    const int n_sums = min(n_chunks, 8);
+    const bool vec = (ld & 3) == 0;
+#pragma unroll
+    for (int it = 0; it < kScoreRows * NB / 256; ++it) {
+        const int q = threadIdx.x + it * 256, row = q / NB, col = q % NB * 4, i = i0 + row, j = j0 + col;
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int w = 0; w < (WIDE ? 8 : 4); ++w) {
+            if (w >= n_sums) break;
+            const float4 v = load4(score_smem + (w * kScoreRows + row) * kPitch + col);
+            sum[0] += v.x; sum[1] += v.y; sum[2] += v.z; sum[3] += v.w;
+        }
+        if (i >= B || j >= T) continue;
+        float* dst = raw + (size_t)i * ld + j;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) sum[u] = FN == DIST_L2 ? sqrtf(sum[u]) : sum[u];
+        if (vec && j + 3 < T) {
+            store4(dst, make_float4(sum[0], sum[1], sum[2], sum[3]));
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (j + u < T) dst[u] = sum[u];
+        }
     }
 }
 
+template <int FN, int NB, bool WIDE>
+inline cudaError_t launch_score_block(const ShardArgs<ScoreArgs>& shards, int n_shards, int B, int T, int D, int ld, cudaStream_t stream, const ExchangeSync& sync) {
+    static bool configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
+    const int slot = current_device_slot();
+    if (slot < 0 || !configured[slot]) {
+        const cudaError_t err = cudaFuncSetAttribute(k_score_block<FN, NB, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreBlockSmem<NB>);
+        if (err != cudaSuccess) return err;
+        if (slot >= 0) configured[slot] = true;
+    }
+    const dim3 grid((T + 4 * NB - 1) / (4 * NB), (B + kScoreRows - 1) / kScoreRows, (unsigned)n_shards);
+    return launch_dependent(k_score_block<FN, NB, WIDE>, grid, dim3(256), kScoreBlockSmem<NB>, stream, shards, B, T, D, ld, sync);
+}
+template <int FN, int NB>
+inline cudaError_t launch_score_block(const ShardArgs<ScoreArgs>& shards, int n_shards, int B, int T, int D, int ld, cudaStream_t stream, const ExchangeSync& sync) {
+    if (D > 32 * kScoreGroups) return launch_score_block<FN, NB, true>(shards, n_shards, B, T, D, ld, stream, sync);
+    return launch_score_block<FN, NB, false>(shards, n_shards, B, T, D, ld, stream, sync);
+}
+
 // The same scores where there are enough of them to fill the GPU with tiles (ranking): a block owns 64 x 128 outputs, its
-// 8 warps 32 x 32 each, with k_score_wide's register tile; all of them walk all of k in chunks of 32 staged one ahead.
-// Each chunk is summed by itself and added to the total, as k_score_wide adds its warps' chunks.  Bound by the FP32
-// pipe.  (k_score_wide divides the chunks over its warps, half of which have none at 100 columns, and its blocks pay a
-// reduction for every 1024 outputs: 32 queries x 4 shards x 4096 rows x 100 columns took 13 us a pass.)
+// 8 warps 32 x 32 each; all of them walk all of k in chunks of 32 staged one ahead.  Each chunk is summed by itself and
+// added to the total, as k_score_block adds its groups' chunks.  Bound by the FP32 pipe.  (With k_score_block's division of k
+// half the warps have nothing to do at 100 columns, and 1024 outputs a block pay for a reduction.)
 constexpr int kScoreTileP = 64, kScoreTileT = 128;
 constexpr int kScoreTileStage = (kScoreTileP + kScoreTileT) * kScoreStride;
 constexpr size_t kScoreTileSmem = 2 * kScoreTileStage * sizeof(float);
@@ -695,8 +754,7 @@ inline cudaError_t launch_score(const ShardArgs<ScoreArgs>& shards, int n_shards
     static bool configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
     const int slot = current_device_slot();
     if (slot < 0 || !configured[slot]) {
-        cudaError_t err = cudaFuncSetAttribute(k_score_wide<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreWideSmem);
-        if (err == cudaSuccess) err = cudaFuncSetAttribute(k_score_tile<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreTileSmem);
+        const cudaError_t err = cudaFuncSetAttribute(k_score_tile<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreTileSmem);
         if (err != cudaSuccess) return err;
         if (slot >= 0) configured[slot] = true;
     }
@@ -704,7 +762,15 @@ inline cudaError_t launch_score(const ShardArgs<ScoreArgs>& shards, int n_shards
     const dim3 tiles((T + kScoreTileT - 1) / kScoreTileT, (B + kScoreTileP - 1) / kScoreTileP, n);
     if (sync.world <= 1 && (size_t)tiles.x * tiles.y * n >= 2 * 148)
         return launch_dependent(k_score_tile<FN>, tiles, dim3(256), kScoreTileSmem, stream, shards, B, T, D, ld);
-    return launch_dependent(k_score_wide<FN>, dim3((T + 31) / 32, (B + 31) / 32, n), dim3(32 * kScoreWarps), kScoreWideSmem, stream, shards, B, T, D, ld, sync);
+    // The width whose waves of 148 blocks end first: 4 NB D clocks for a block's sums, about 4 us for what does not depend
+    // on its width.
+    auto clocks = [&](int nb) {
+        const long long blocks = (long long)((T + 4 * nb - 1) / (4 * nb)) * ((B + kScoreRows - 1) / kScoreRows) * n_shards;
+        return (blocks + kSmCount - 1) / kSmCount * (4ll * nb * D + 7600);
+    };
+    if (clocks(16) <= clocks(12) && clocks(16) <= clocks(8)) return launch_score_block<FN, 16>(shards, n_shards, B, T, D, ld, stream, sync);
+    if (clocks(12) <= clocks(8)) return launch_score_block<FN, 12>(shards, n_shards, B, T, D, ld, stream, sync);
+    return launch_score_block<FN, 8>(shards, n_shards, B, T, D, ld, stream, sync);
 }
 inline cudaError_t launch_score(int dist_fn, const ShardArgs<ScoreArgs>& shards, int n_shards, int B, int T, int D, int ld, cudaStream_t stream,
                                 const ExchangeSync& sync = ExchangeSync{}) {

@@ -5,6 +5,7 @@ import pytest
 
 from distributed_kge_poplar_b200 import capi
 from helpers import assert_close, engine_settings, make_oracle, random_batch, random_state, read_rows, read_state, write_state
+from oracle import step_oracle as so
 from oracle.step_oracle import StepConfig
 
 pytestmark = pytest.mark.gpu
@@ -80,3 +81,16 @@ def test_shards_update_dense_parameters_together(monkeypatch, score_fn, distance
 
 def test_separate_networks_of_four_shards():
     _two_runs(_config("TransE", "L2", n_shard=4, batch_size=12, a2a_size=7, embedding_size=36, entity_feature_size=12, share_feature_networks=False), seed=9, rtol=1e-4)
+
+
+@pytest.mark.parametrize("fn", [capi.L1, capi.L2, capi.DOT], ids=["l1", "l2", "dot"])
+@pytest.mark.parametrize("shape", [(1, 1, 4), (64, 33, 128), (65, 49, 132), (130, 700, 260), (200, 1500, 288), (64, 64, 516)])
+def test_scores_in_blocks(fn, shape):
+    """Blocks of 32, 48 and 64 columns with and without a remainder; one chunk of k, four, five, eight and more."""
+    m, n, k = shape
+    rng = np.random.RandomState(n)
+    a, b = rng.normal(size=(m, k)).astype(np.float32), rng.normal(size=(n, k)).astype(np.float32)
+    b[-1] = a[0]
+    a64, b64 = a.astype(np.float64), b.astype(np.float64)
+    want = {capi.L1: so.l1_distance, capi.L2: so.l2_distance, capi.DOT: lambda x, y: x @ y.T}[fn](a64, b64)
+    assert_close(capi.op_pairwise(fn, a, b), want, 1e-5, f"scores {shape}")
