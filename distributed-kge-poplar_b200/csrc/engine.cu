@@ -1357,29 +1357,84 @@ void Engine::launch_tc(const char* name, tc::GemmArgs* problems, int n_problems,
     KGE_CUDA(err);
 }
 
+// How the k ranges of a launch's problems are divided over the blocks of clusters of `cluster` blocks: every problem over all
+// of them or, where the launch allows it, over the divisor with which its blocks have the fewest slices to add up while all
+// clusters are on the GPU at once.  Returns the longest chain of slices, 0 where the clusters do not fit.
+static unsigned divide_k(const tc::PlaneProblem* problems, int n_problems, unsigned cluster, unsigned tile_n, unsigned slice, bool mixed, int* splits) {
+    auto slices = [&](int i, unsigned s) { return std::max(1u, ceil_div(ceil_div((unsigned)problems[i].g.K, slice), s)); };
+    unsigned tiles_n = 1;
+    for (int i = 0; i < n_problems; ++i) tiles_n = std::max(tiles_n, ceil_div((unsigned)problems[i].g.N, tile_n));
+    auto clusters = [&] {
+        unsigned n = 0;
+        for (int i = 0; i < n_problems; ++i) n += ceil_div(ceil_div((unsigned)problems[i].g.M, 128u), cluster / (unsigned)splits[i]) * tiles_n;
+        return n;
+    };
+    const unsigned room = cluster > 1 ? (unsigned)tc::max_resident_plane_clusters((int)cluster) : ~0u;
+    for (int i = 0; i < n_problems; ++i) splits[i] = mixed ? 1 : (int)cluster;
+    if (clusters() > room) return 0;
+    // divide the problem with the longest chain further while there is room for the blocks that takes
+    for (bool further = mixed; further;) {
+        int longest = 0;
+        for (int i = 1; i < n_problems; ++i)
+            if (slices(i, (unsigned)splits[i]) > slices(longest, (unsigned)splits[longest])) longest = i;
+        int next = splits[longest] + 1;
+        while (next <= (int)cluster && cluster % (unsigned)next) ++next;
+        further = next <= (int)cluster;
+        if (!further) break;
+        const int before = splits[longest];
+        splits[longest] = next;
+        if (clusters() > room) splits[longest] = before, further = false;
+    }
+    unsigned chain = 0;
+    for (int i = 0; i < n_problems; ++i) chain = std::max(chain, slices(i, (unsigned)splits[i]));
+    return chain;
+}
+
 // One launch of the plane-fed contraction for problems of the same shape class, those of `n_shards` local shards.  Tiles
-// are 128 x 128 (128 x 64 for narrow outputs); the k range is split over the blocks of a cluster so
-// that about one block per SM is busy and every split keeps at least two 32-deep slices.
+// are 128 x 128 (128 x 64 for narrow outputs); the k range is divided over the blocks of a cluster so that about one block
+// per SM is busy and every split keeps at least two slices.  The two score gradients of a batch with many more tails than
+// triples have k ranges of very different length, and only the longer one wants dividing: with one number of splits for
+// both, 256 x 1536 x 256 gradients walked 12 slices where 6 do (RotatE 82.9 -> 77.6 us a step).  Gradients from bfloat16
+// operands stay with one number: their slices are short, the operands' way from L2 bounds them, and 1024 x 2048 x 512 with 16
+// slices a block in place of 32 took 2 us longer.
 void Engine::launch_planes(const char* name, tc::PlaneProblem* problems, int n_problems, int side, int wait_kind, int signal_kind,
                            const tc::Routing* routing, unsigned n_shards) {
     int max_n = 0, max_k = 0;
     unsigned tiles = 0;
-    for (int i = 0; i < n_problems; ++i) max_n = std::max(max_n, problems[i].g.N);
+    bool alike = true;
+    for (int i = 0; i < n_problems; ++i) {
+        max_n = std::max(max_n, problems[i].g.N);
+        alike = alike && problems[i].g.epilogue == problems[0].g.epilogue;
+    }
     const bool half = problems[0].A.elem_bytes == 16;  // float16 planes: whole tiles of 128 x 128 (launch_prepared)
     const int tile_n = max_n > 64 || half ? 128 : 64;
     for (int i = 0; i < n_problems; ++i) {
         tiles += ceil_div((unsigned)problems[i].g.M, 128) * ceil_div((unsigned)max_n, (unsigned)tile_n);
         max_k = std::max(max_k, problems[i].g.K);
     }
+    const unsigned slice = problems[0].A.elem_bytes == 2 || half ? 64u : 32u;  // slices of 16-bit operands are 64 deep
     int splits = (int)std::min<unsigned>({std::max(1u, 148u / std::max(1u, tiles)), std::max(1u, (unsigned)max_k / 64u),
                                           (unsigned)tc::kMaxClusterSplits});
     while (splits > 1 && (unsigned)tc::max_resident_plane_clusters(splits) < tiles) --splits;
     if (half) splits = 1;
+    int each[tc::kMaxPlaneProblems];
+    unsigned chain = divide_k(problems, n_problems, (unsigned)splits, (unsigned)tile_n, slice, false, each);
+    if (n_problems > 1 && alike && problems[0].A.elem_bytes != 2 && tc::mixed_splits_allowed(side, problems[0].g.epilogue, tile_n)) {
+        // worth it from two slices less on (a cluster's exchange where there was none costs about as much)
+        for (unsigned cluster = 2; cluster <= (unsigned)tc::kMaxClusterSplits; cluster *= 2) {
+            int other[tc::kMaxPlaneProblems];
+            const unsigned c = divide_k(problems, n_problems, cluster, (unsigned)tile_n, slice, true, other);
+            if (c == 0 || c + 2 > chain) continue;
+            chain = c;
+            splits = (int)cluster;
+            std::copy(other, other + n_problems, each);
+        }
+    }
     for (int i = 0; i < n_problems; ++i) {
         tc::GemmArgs& g = problems[i].g;
         g.status = d_tc_status_;
-        const unsigned slice = problems[i].A.elem_bytes == 2 || half ? 64u : 32u;  // slices of 16-bit operands are 64 deep
-        g.k_per_split = (int)std::max<size_t>(slice, round_up(ceil_div((unsigned)g.K, (unsigned)splits), slice));
+        g.cluster_splits = each[i];
+        g.k_per_split = (int)std::max<size_t>(slice, round_up(ceil_div((unsigned)g.K, (unsigned)each[i]), slice));
     }
     timing_begin(name);
     cudaError_t err;

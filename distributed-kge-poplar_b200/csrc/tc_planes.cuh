@@ -449,8 +449,8 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // EPI >= 0: an instantiation whose epilogue, operand type and k split are known at compile time.  A block runs
 // this kernel once on an SM whose instruction cache has never seen it, and most of it is
 // straight-line code executed once: what the instantiation does not need is not fetched.
-// SPLIT: 0 no k split; else the k range is split over a cluster and a block finishes at most SPLIT units per thread
-// (3: up to 30 rows, five or more splits; 7: up to 64 rows).  BF16: bfloat16 operands.
+// SPLIT: 0 no cluster; else a block finishes at most SPLIT units per thread (3: up to 30 rows, five or more k splits; 7: up to
+// 64 rows; 13: a whole tile, in a launch whose other problem is split).  BF16: bfloat16 operands.
 template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, bool BF16 = false>
 __global__ void __launch_bounds__(kPlThreads, 1)
 k_tc_planes(const __grid_constant__ PlaneSet gp, const __grid_constant__ PlaneMaps maps) {
@@ -472,9 +472,12 @@ k_tc_planes(const __grid_constant__ PlaneSet gp, const __grid_constant__ PlaneMa
     const PlaneProblem& pp = gp.p[which];
     const GemmArgs& g = pp.g;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = ((int)blockIdx.x - (which ? gp.tiles_end[which - 1] : 0)) * kBM, n0 = blockIdx.y * BN;
+    // a cluster of gridDim.z blocks works on gridDim.z / splits tiles of rows, each of them divided over `splits` blocks
+    const int splits = max(1, g.cluster_splits), split = (int)blockIdx.z % splits;
+    const int m_tile = ((int)blockIdx.x - (which ? gp.tiles_end[which - 1] : 0)) * ((int)gridDim.z / splits) + (int)blockIdx.z / splits;
+    const int m0 = m_tile * kBM, n0 = blockIdx.y * BN;
     const unsigned total_blocks = gridDim.x * gridDim.y * gridDim.z;
-    if (n0 >= g.N || m0 >= g.M) {  // the problems may differ in size (a whole cluster leaves together)
+    if (n0 >= g.N) {  // the problems may differ in size (a whole cluster leaves together)
         grid_dependency_sync();
         exchange_signal(gp.sync, gp.signal_kind, total_blocks);
         return;
@@ -482,7 +485,8 @@ k_tc_planes(const __grid_constant__ PlaneSet gp, const __grid_constant__ PlaneMa
 
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr uint32_t kATile = kBM * 128, kBTile = BN * 128;
-    const int k_begin = blockIdx.z * g.k_per_split, k_end = min(g.K, k_begin + g.k_per_split);
+    // (a block past the last tile of rows stays for its cluster's barriers, with nothing to add up and nothing to store)
+    const int k_begin = split * g.k_per_split, k_end = m0 < g.M ? min(g.K, k_begin + g.k_per_split) : 0;
     const int bf16 = kLean ? (BF16 ? 1 : 0) : gp.bf16, slice_k = bf16 ? 64 : kBK;
     const int n_slices = max(0, (k_end - k_begin + slice_k - 1) / slice_k);
     const bool a_two = pp.A.lo != nullptr, b_two = pp.B.lo != nullptr;
@@ -515,7 +519,7 @@ k_tc_planes(const __grid_constant__ PlaneSet gp, const __grid_constant__ PlaneMa
     grid_dependency_sync();
     exchange_wait(gp.sync, gp.wait_kind);
     const uint32_t tmem_base = tmem_slot;
-    if ((kLean ? EPI == EPI_ADD_TABLE_VALUE && SPLIT == 0 : g.epilogue == EPI_ADD_TABLE_VALUE && g.cluster_splits <= 1) && tid >= 64 && tid < 64 + kBM && m0 + tid - 64 < g.M) {
+    if ((kLean ? EPI == EPI_ADD_TABLE_VALUE && SPLIT == 0 : g.epilogue == EPI_ADD_TABLE_VALUE && gridDim.z == 1) && tid >= 64 && tid < 64 + kBM && m0 + tid - 64 < g.M) {
         // A whole tile without a k split (predict's hidden rows): the table values that the epilogue
         // adds are asked into L2 now, a row per thread, so that the finishing loop, which fetches
         // them one unit after the other, waits for L2 and not for DRAM.
@@ -661,9 +665,9 @@ k_tc_planes(const __grid_constant__ PlaneSet gp, const __grid_constant__ PlaneMa
         // barrier (arrive here, wait before the copies are issued).  Without a k split the block is
         // the only owner: its rows take the same way through shared memory, which turns one thread's
         // row of the accumulator into whole rows stored by neighbouring threads.
-        const bool clustered = kLean ? SPLIT > 0 : g.cluster_splits > 1;
+        const bool clustered = kLean ? SPLIT > 0 : gridDim.z > 1;
         if (clustered) cluster_arrive_relaxed();
-        const int n_split = clustered ? g.cluster_splits : 1, rank = clustered ? (int)cluster_rank() : 0;
+        const int n_split = clustered ? splits : 1, rank = clustered ? split : 0, first_rank = (int)blockIdx.z - split;  // of the blocks that share the tile
         const int rows_each = (kBM + n_split - 1) / n_split;
         const uint32_t off_rowsum = (uint32_t)rows_each * BN, off_colsum = off_rowsum + (uint32_t)((rows_each + 3) & ~3);
         const uint32_t slot_floats = off_colsum + (SIDE == SIDE_NORMS ? BN : 0);  // rows | row sums | column sums
@@ -747,7 +751,7 @@ k_tc_planes(const __grid_constant__ PlaneSet gp, const __grid_constant__ PlaneMa
         if (clustered) fence_async_shared();  // the copy engine reads what the threads have just written
         const int r_begin = rank * rows_each, r_end = min(kBM, r_begin + rows_each);
         constexpr int kQuads = BN / 4;
-        // a split owns at most 64 rows x BN / 4 quads
+        // (where all problems are split a block owns at most 64 rows x BN / 4 quads)
         constexpr int kUnits = kLean && SPLIT > 0 ? SPLIT : (64 * kQuads + kPlThreads - 1) / kPlThreads;
         const int n_units = max(0, r_end - r_begin) * kQuads;
         float xv[kUnits][4];
@@ -765,8 +769,8 @@ k_tc_planes(const __grid_constant__ PlaneSet gp, const __grid_constant__ PlaneMa
         if (clustered) {
             cluster_wait();
             if (warp == 0 && lane < n_split && lane != rank) {
-                const uint32_t dst = cluster_map(smem_u32(receive + (size_t)rank * slot_floats), (uint32_t)lane);
-                const uint32_t bar = cluster_map(smem_u32(&bar_reduce), (uint32_t)lane);
+                const uint32_t dst = cluster_map(smem_u32(receive + (size_t)rank * slot_floats), (uint32_t)(first_rank + lane));
+                const uint32_t bar = cluster_map(smem_u32(&bar_reduce), (uint32_t)(first_rank + lane));
                 asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                              ::"r"(dst), "r"(smem_u32(staging + (size_t)lane * slot_floats)), "r"(slot_bytes), "r"(bar) : "memory");
             }
@@ -1315,7 +1319,7 @@ struct PlaneLaunch {
     PlaneSet gp;
     PlaneMaps maps;
     dim3 grid;
-    int splits, tile_n;
+    int splits, fewest_splits, tile_n;  // blocks of a cluster, and how many of them the least divided problem's k is divided over
 };
 
 // What the finished rows of a launch's problems go to: one set of lookups per shard, `per_shard` problems each, of which
@@ -1327,8 +1331,8 @@ struct Routing {
 };
 
 // Contractions of the same kind in one launch, tiles of 128 x tile_n (64 or 128).
-// splits > 1: the blocks of a tile form a cluster (at most kMaxClusterSplits) and g.k_per_split
-// must be set accordingly by the caller.
+// splits > 1: clusters of that many blocks (at most kMaxClusterSplits).  A problem's k range is divided over all blocks of a
+// cluster, or over g.cluster_splits of them where the caller has set that to a divisor; g.k_per_split is set accordingly.
 inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, int splits, int tile_n, PlaneLaunch* out,
                                   const ExchangeSync& sync = ExchangeSync{}, int wait_kind = -1, int signal_kind = -1,
                                   const Routing* routing = nullptr) {
@@ -1341,13 +1345,17 @@ inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, 
     gp.signal_kind = signal_kind;
     if (routing)
         for (int i = 0; i < routing->n_shards; ++i) gp.route[i] = routing->shards[i];
-    int tiles_m = 0, tiles_n = 1;
+    int tiles_m = 0, tiles_n = 1, fewest = splits;
     auto type_of = [](const PlaneOperand& op) { return op.elem_bytes == 16 ? 2 : op.elem_bytes == 2 ? 1 : 0; };
     gp.bf16 = type_of(problems[0].A);
     for (int i = 0; i < n_problems; ++i) {
         PlaneProblem& q = gp.p[i];
         q = problems[i];
-        tiles_m += (q.g.M + kBM - 1) / kBM;
+        if (splits == 1 || q.g.cluster_splits < 1) q.g.cluster_splits = splits;
+        if (splits % q.g.cluster_splits) return cudaErrorInvalidValue;
+        const int tiles_each = splits / q.g.cluster_splits;  // of a cluster
+        tiles_m += ((q.g.M + kBM - 1) / kBM + tiles_each - 1) / tiles_each;
+        fewest = std::min(fewest, q.g.cluster_splits);
         tiles_n = std::max(tiles_n, (q.g.N + tile_n - 1) / tile_n);
         gp.tiles_end[i] = tiles_m;
         if (routing) gp.route_of[i] = i / routing->per_shard, gp.route_mode[i] = routing->mode[i % routing->per_shard];
@@ -1355,7 +1363,6 @@ inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, 
         if (gp.bf16 == 1 && (q.A.lo || q.B.lo || q.g.k_per_split % 64)) return cudaErrorInvalidValue;
         if (gp.bf16 == 2 && (!q.B.lo || n_problems != 1 || splits != 1 || tile_n != 128)) return cudaErrorInvalidValue;
         q.g.ws = nullptr;
-        q.g.cluster_splits = splits > 1 ? splits : 0;
         if (!planes_aligned(q.A) || !planes_aligned(q.B)) return cudaErrorInvalidValue;
         cudaError_t err = make_plane_map(q.A.hi, q.A, q.g.M, q.g.K, kBM, &out->maps.a_hi[i]);
         if (err == cudaSuccess) err = make_plane_map(q.A.lo ? q.A.lo : q.A.hi, q.A, q.g.M, q.g.K, kBM, &out->maps.a_lo[i]);
@@ -1367,6 +1374,7 @@ inline cudaError_t prepare_planes(const PlaneProblem* problems, int n_problems, 
     }
     out->grid = dim3(tiles_m, tiles_n, splits);
     out->splits = splits;
+    out->fewest_splits = fewest;
     out->tile_n = tile_n;
     return cudaSuccess;
 }
@@ -1381,9 +1389,15 @@ inline cudaError_t launch_lean(const PlaneLaunch& l, cudaStream_t stream) {
 // By the number of k splits: five or more leave at most 26 rows of a tile to a block.
 template <int SIDE, int EPI>
 inline cudaError_t launch_lean_split(const PlaneLaunch& l, cudaStream_t stream) {
-    if (l.splits >= 5) return launch_lean<SIDE, EPI, 3>(l, stream);
-    if (l.splits >= 2) return launch_lean<SIDE, EPI, 7>(l, stream);
-    return launch_lean<SIDE, EPI, 0>(l, stream);
+    if (l.splits == 1) return launch_lean<SIDE, EPI, 0>(l, stream);
+    if (l.fewest_splits >= 5) return launch_lean<SIDE, EPI, 3>(l, stream);
+    if (l.fewest_splits >= 2) return launch_lean<SIDE, EPI, 7>(l, stream);
+    if constexpr (EPI == EPI_STORE || EPI == EPI_ROWSUM_X_MINUS) return launch_lean<SIDE, EPI, 13>(l, stream);
+    return cudaErrorInvalidValue;
+}
+// Whether a launch's problems may be divided differently, with one that is not divided at all among them.
+inline bool mixed_splits_allowed(int side, int epilogue, int tile_n) {
+    return tile_n == 128 && ((side == SIDE_NONE && epilogue == EPI_STORE) || (side == SIDE_ROWSUM && epilogue == EPI_ROWSUM_X_MINUS));
 }
 
 template <int EPI>
@@ -1420,6 +1434,7 @@ inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
         if (alike) {
             if constexpr (SIDE == SIDE_NONE) {
                 if (l.gp.bf16) {
+                    if (l.splits > 1 && l.fewest_splits == 1) return cudaErrorInvalidValue;
                     if (epilogue == EPI_STORE) return l.splits > 1 ? launch_lean<SIDE_NONE, EPI_STORE, 7, true>(l, stream) : launch_lean<SIDE_NONE, EPI_STORE, 0, true>(l, stream);
                 } else {
                     if (epilogue == EPI_ADD_TABLE_VALUE) return launch_lean_split<SIDE_NONE, EPI_ADD_TABLE_VALUE>(l, stream);
@@ -1432,11 +1447,13 @@ inline cudaError_t launch_prepared(const PlaneLaunch& l, cudaStream_t stream) {
                 if (epilogue == EPI_L2_DISTANCE && l.splits == 1) return launch_lean<SIDE_NORMS, EPI_L2_DISTANCE, 0>(l, stream);
             }
         }
+        if (l.splits > 1 && l.fewest_splits == 1) return cudaErrorInvalidValue;
         cudaError_t err = configure_planes<128, SIDE>();
         if (err != cudaSuccess) return err;
         return launch_dependent_cluster(k_tc_planes<128, SIDE>, l.grid, dim3(kPlThreads), plane_smem_bytes(), stream,
                                         (unsigned)l.splits, l.gp, l.maps);
     }
+    if (l.splits > 1 && l.fewest_splits == 1) return cudaErrorInvalidValue;
     cudaError_t err = configure_planes<64, SIDE>();
     if (err != cudaSuccess) return err;
     return launch_dependent_cluster(k_tc_planes<64, SIDE>, l.grid, dim3(kPlThreads), plane_smem_bytes(), stream,

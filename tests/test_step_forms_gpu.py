@@ -94,3 +94,12 @@ def test_scores_in_blocks(fn, shape):
     a64, b64 = a.astype(np.float64), b.astype(np.float64)
     want = {capi.L1: so.l1_distance, capi.L2: so.l2_distance, capi.DOT: lambda x, y: x @ y.T}[fn](a64, b64)
     assert_close(capi.op_pairwise(fn, a, b), want, 1e-5, f"scores {shape}")
+
+
+@pytest.mark.parametrize("score_fn,distance_fn", [("RotatE", "L2"), ("ComplEx", "MatMul")])
+@pytest.mark.parametrize("batch,a2a", [(64, 1536), (70, 900), (1000, 150), (300, 2200)])
+def test_score_gradients_of_lopsided_batches(score_fn, distance_fn, batch, a2a):
+    """Many more tails than triples and the reverse: the two contractions' k ranges divided differently, with clusters whose
+    last tile has no rows.  Sums of up to 2200 cancelling terms: the bound of the other long contractions, 5e-5, over two steps."""
+    _two_runs(_config(score_fn, distance_fn, n_entity=4000, batch_size=batch, a2a_size=a2a, embedding_size=68, loss_type="softmax", correction_weight=1.0), seed=batch, rtol=1e-4,
+              rel_rtol=2e-3 if score_fn == "RotatE" else None, n_step=1)
