@@ -844,55 +844,70 @@ __device__ __forceinline__ void finish_step_loss(const float* loss_rows, int B, 
     }
 }
 
-template <int THREADS>
+// One block per row.  A thread keeps its PER columns (j, j + THREADS, ...) in registers, read once and all at the same time;
+// the sums take them in that order, which is part of an L1 model's result (see k_pair_bwd).  Bound by latency: a row's
+// read, two reductions over the block, a chain of exponentials.  With the row read again for the maximum, the sum and the
+// coefficients, one column after the other, steps took (us, before -> after) 70.6 -> 68.9 for 512 x 768 softmax scores, 110.0
+// -> 106.5 for two such shards, 64.8 -> 62.7 for 1024 x 2048 log-sigmoids, 59.0 -> 57.4 for four shards of 256 x 512.
+template <int THREADS, int PER>
 __global__ void __launch_bounds__(THREADS)
 k_loss(const __grid_constant__ ShardArgs<LossArgs> shards, LossParams lp, float inv_normaliser, int lo_bf16) {
-    grid_dependency_sync();
-    __shared__ float scratch[THREADS / 32];
+    __shared__ float scratch[2][THREADS / 32];
     const LossArgs& a = shards.s[blockIdx.y];
-    float* __restrict__ loss_rows = a.loss_rows;
     const int i = blockIdx.x, T = lp.n_tail;
+    const int lab = (int)a.label[i];  // (staged before the kernel in front began)
+    grid_dependency_sync();
+    float* __restrict__ loss_rows = a.loss_rows;
     const float* __restrict__ r = a.raw + (size_t)i * lp.ld;
     float* __restrict__ c = a.coeff + (size_t)i * lp.ld;
     // the companion plane for the tensor-core gradients: lower TF32 part, or the bf16 rounding
     float* __restrict__ c_lo = a.coeff_lo && !lo_bf16 ? a.coeff_lo + (size_t)i * lp.ld : nullptr;
     __nv_bfloat16* __restrict__ c16 = a.coeff_lo && lo_bf16 ? reinterpret_cast<__nv_bfloat16*>(a.coeff_lo) + (size_t)i * lp.ld : nullptr;
-    for (int j = T + (int)threadIdx.x; j < lp.ld; j += THREADS) {
-        c[j] = 0.f;
-        if (c_lo) c_lo[j] = 0.f;
-        if (c16) c16[j] = __float2bfloat16_rn(0.f);
+    auto store = [&](int j, float cj) {
+        c[j] = cj;
+        if (c_lo) c_lo[j] = tf32_lower(cj);
+        if (c16) c16[j] = __float2bfloat16_rn(cj);
+    };
+    float dist[PER];  // distances or dot products
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        const int j = threadIdx.x + u * THREADS;
+        dist[u] = j < T ? r[j] : 0.f;
     }
-    const int lab = (int)a.label[i];
+    for (int j = T + (int)threadIdx.x; j < lp.ld; j += THREADS) store(j, 0.f);
     const bool transe = score_is_gamma_minus_distance(lp.score_fn);
-    auto score_of = [&](int j) { return transe ? lp.gamma - r[j] : r[j]; };
-    auto to_coeff = [&](int j, float g_score) {
+    auto score_of = [&](int u) { return transe ? lp.gamma - dist[u] : dist[u]; };
+    auto to_coeff = [&](int u, float g_score) {
         float g = transe ? -g_score : g_score;  // d score / d raw
-        if (lp.dist_fn == DIST_L2) {
-            const float dist = r[j];
-            g = dist == 0.f ? 0.f : g / dist;
-        }
+        if (lp.dist_fn == DIST_L2) g = dist[u] == 0.f ? 0.f : g / dist[u];
         return g;
     };
     if (lp.loss_fn == LOSS_SOFTMAX) {
         float mx = -INFINITY;
-        for (int j = threadIdx.x; j < T; j += THREADS)
-            mx = fmaxf(mx, score_of(j) + (j == lab ? 0.f : lp.softmax_shift));
-        mx = block_max<THREADS>(mx, scratch);
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int j = threadIdx.x + u * THREADS;
+            if (j < T) mx = fmaxf(mx, score_of(u) + (j == lab ? 0.f : lp.softmax_shift));
+        }
+        mx = block_max<THREADS>(mx, scratch[0]);
         float sum = 0.f;
-        for (int j = threadIdx.x; j < T; j += THREADS)
-            sum += expf(score_of(j) + (j == lab ? 0.f : lp.softmax_shift) - mx);
-        sum = block_sum<THREADS>(sum, scratch);
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int j = threadIdx.x + u * THREADS;
+            if (j < T) sum += expf(score_of(u) + (j == lab ? 0.f : lp.softmax_shift) - mx);
+        }
+        sum = block_sum<THREADS>(sum, scratch[1]);
         const float log_z = logf(sum);
-        for (int j = threadIdx.x; j < T; j += THREADS) {
-            const float logp = score_of(j) + (j == lab ? 0.f : lp.softmax_shift) - mx - log_z;
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int j = threadIdx.x + u * THREADS;
+            if (j >= T) continue;
+            const float logp = score_of(u) + (j == lab ? 0.f : lp.softmax_shift) - mx - log_z;
             const float g = lp.grad_scale * (expf(logp) - (j == lab ? 1.f : 0.f));
-            const float cj = to_coeff(j, g);
-            c[j] = cj;
-            if (c_lo) c_lo[j] = tf32_lower(cj);
-            if (c16) c16[j] = __float2bfloat16_rn(cj);
+            store(j, to_coeff(u, g));
             if (j == lab) loss_rows[i] = -logp;
         }
-        if (a.loss_total) finish_step_loss<THREADS>(loss_rows, (int)gridDim.x, inv_normaliser, a.loss_total, a.loss_last, a.counter, scratch, a.extra_loss);
+        if (a.loss_total) finish_step_loss<THREADS>(loss_rows, (int)gridDim.x, inv_normaliser, a.loss_total, a.loss_last, a.counter, scratch[0], a.extra_loss);
         return;
     }
     // log-sigmoid, optionally with self-adversarial weights from a detached softmax
@@ -900,20 +915,26 @@ k_loss(const __grid_constant__ ShardArgs<LossArgs> shards, LossParams lp, float 
     const bool adv = lp.adversarial_scale > 0.f;
     if (adv) {
         float mx = -INFINITY;
-#pragma unroll 4
-        for (int j = threadIdx.x; j < T; j += THREADS)
-            mx = fmaxf(mx, lp.adversarial_scale * score_of(j) + (j == lab ? -10000.f : 0.f));
-        adv_max = block_max<THREADS>(mx, scratch);
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int j = threadIdx.x + u * THREADS;
+            if (j < T) mx = fmaxf(mx, lp.adversarial_scale * score_of(u) + (j == lab ? -10000.f : 0.f));
+        }
+        adv_max = block_max<THREADS>(mx, scratch[0]);
         float sum = 0.f;
-#pragma unroll 4
-        for (int j = threadIdx.x; j < T; j += THREADS)
-            sum += expf(lp.adversarial_scale * score_of(j) + (j == lab ? -10000.f : 0.f) - adv_max);
-        adv_sum = block_sum<THREADS>(sum, scratch);
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int j = threadIdx.x + u * THREADS;
+            if (j < T) sum += expf(lp.adversarial_scale * score_of(u) + (j == lab ? -10000.f : 0.f) - adv_max);
+        }
+        adv_sum = block_sum<THREADS>(sum, scratch[1]);
     }
     float part = 0.f;
-#pragma unroll 4
-    for (int j = threadIdx.x; j < T; j += THREADS) {
-        const float s = score_of(j);
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        const int j = threadIdx.x + u * THREADS;
+        if (j >= T) continue;
+        const float s = score_of(u);
         const bool pos = j == lab;
         float w = pos ? lp.w_pos : lp.w_neg;
         if (adv) {
@@ -925,26 +946,36 @@ k_loss(const __grid_constant__ ShardArgs<LossArgs> shards, LossParams lp, float 
         const float ls = x > -11.f ? -log1pf(expf(-fmaxf(x, -11.f))) : x;
         part += w * ls;
         const float dx = (-w * lp.grad_scale) / (1.f + expf(fminf(x, 11.f)));
-        const float cj = to_coeff(j, pos ? dx : -dx);
-        c[j] = cj;
-        if (c_lo) c_lo[j] = tf32_lower(cj);
-        if (c16) c16[j] = __float2bfloat16_rn(cj);
+        store(j, to_coeff(u, pos ? dx : -dx));
     }
-    part = block_sum<THREADS>(part, scratch);
+    part = block_sum<THREADS>(part, scratch[0]);
     if (threadIdx.x == 0) loss_rows[i] = -part;
     // (null loss_total: a later kernel of the step adds the rows' terms, off the step's critical chain)
-    if (a.loss_total) finish_step_loss<THREADS>(loss_rows, (int)gridDim.x, inv_normaliser, a.loss_total, a.loss_last, a.counter, scratch, a.extra_loss);
+    if (a.loss_total) finish_step_loss<THREADS>(loss_rows, (int)gridDim.x, inv_normaliser, a.loss_total, a.loss_last, a.counter, scratch[0], a.extra_loss);
 }
 
+template <int THREADS>
 inline cudaError_t launch_loss(const ShardArgs<LossArgs>& shards, int n_shards, const LossParams& lp, float inv_normaliser, int lo_bf16, int B,
                                cudaStream_t stream) {
-    // One block per row keeps about 130 thousand threads in flight for the metric's 512 x 768 scores; a warp
-    // per row (a sixth as many threads, each with a serial chain of exponentials) measured 4 us slower.  A long row of
+    const dim3 grid((unsigned)B, (unsigned)n_shards);
+    // columns per thread: as few as the row needs (a batch has at most kMaxSortItems tails)
+    const int per = (lp.n_tail + THREADS - 1) / THREADS;
+    if (per <= 1) return launch_spread<k_loss<THREADS, 1>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 2) return launch_spread<k_loss<THREADS, 2>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 3) return launch_spread<k_loss<THREADS, 3>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 4) return launch_spread<k_loss<THREADS, 4>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 6) return launch_spread<k_loss<THREADS, 6>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 8) return launch_spread<k_loss<THREADS, 8>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 16) return launch_spread<k_loss<THREADS, 16>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    return cudaErrorInvalidValue;
+}
+inline cudaError_t launch_loss(const ShardArgs<LossArgs>& shards, int n_shards, const LossParams& lp, float inv_normaliser, int lo_bf16, int B,
+                               cudaStream_t stream) {
+    // A warp per row, with a serial chain of exponentials, measured 4 us slower for 512 x 768 scores.  A long row of
     // log-sigmoids, whose chains are longest, gets twice the threads: 256 x 1536 self-adversarial scores 12.7 to 9.5 us
     // (a softmax row of that length was 1 us slower with them).
-    const dim3 grid((unsigned)B, (unsigned)n_shards);
-    if (lp.loss_fn == LOSS_LOGSIGMOID && lp.n_tail >= 1024) return launch_spread<k_loss<512>>(grid, dim3(512), stream, shards, lp, inv_normaliser, lo_bf16);
-    return launch_spread<k_loss<256>>(grid, dim3(256), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (lp.loss_fn == LOSS_LOGSIGMOID && lp.n_tail >= 1024) return launch_loss<512>(shards, n_shards, lp, inv_normaliser, lo_bf16, B, stream);
+    return launch_loss<256>(shards, n_shards, lp, inv_normaliser, lo_bf16, B, stream);
 }
 
 // ---------------------------------------------------------------------------

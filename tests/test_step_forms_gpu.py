@@ -103,3 +103,11 @@ def test_score_gradients_of_lopsided_batches(score_fn, distance_fn, batch, a2a):
     last tile has no rows.  Sums of up to 2200 cancelling terms: the bound of the other long contractions, 5e-5, over two steps."""
     _two_runs(_config(score_fn, distance_fn, n_entity=4000, batch_size=batch, a2a_size=a2a, embedding_size=68, loss_type="softmax", correction_weight=1.0), seed=batch, rtol=1e-4,
               rel_rtol=2e-3 if score_fn == "RotatE" else None, n_step=1)
+
+
+@pytest.mark.parametrize("loss_type,adversarial", [("softmax", 0.0), ("logsigmoid", 0.0), ("logsigmoid", 1.5)])
+@pytest.mark.parametrize("a2a", [2, 255, 257, 1023, 1025, 2049, 4090])
+def test_loss_rows_of_any_length(loss_type, adversarial, a2a):
+    """One column and more per thread, up to the longest row, the last of a thread's there and not; 256 and 512 threads."""
+    cfg = _config("DistMult", "MatMul", n_entity=4200, batch_size=4, a2a_size=a2a, embedding_size=8, loss_type=loss_type, negative_adversarial_scale=adversarial)
+    _two_runs(cfg, seed=a2a, rtol=1e-4, n_step=1, pad=1 if a2a == 2 else 3)
