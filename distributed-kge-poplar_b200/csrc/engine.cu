@@ -2551,7 +2551,8 @@ void Engine::launch_topk(ShardBuffers& b, unsigned c, uint32_t start, uint32_t l
     const unsigned Q = (unsigned)tp.n_query;
     if (start == 1) {  // nothing ranked yet: parts of at least 512 scores, as many lists as the candidates have room for
         const unsigned parts = std::max(1u, std::min({(unsigned)kTopkCandidates / (unsigned)tp.n_best, ceil_div(c, 512u), 64u}));
-        KGE_LAUNCH("predict_topk", k_topk_seed<<<dim3(ceil_div(Q, 4), parts), 128, 0, stream_>>>(p_raw_, (int)c, start, last, p_cand_, p_cand_count_, tp));
+        const auto seed = tp.n_best <= 32 ? k_topk_seed<true> : k_topk_seed<false>;
+        KGE_LAUNCH("predict_topk", seed<<<dim3(ceil_div(Q, 4), parts), 128, 0, stream_>>>(p_raw_, (int)c, start, last, p_cand_, p_cand_count_, tp));
     } else if (!filtered) {  // else the score kernel's epilogue has left the candidates
         const dim3 fgrid(std::max(1u, std::min(ceil_div(c, 4 * 256), 8u)), Q);
         KGE_LAUNCH("predict_topk", k_topk_filter<<<fgrid, 256, 0, stream_>>>(p_raw_, (int)c, start, last, b.topk_state, b.topk_count, p_cand_, p_cand_count_, tp));

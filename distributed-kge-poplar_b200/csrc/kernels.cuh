@@ -2563,13 +2563,44 @@ k_topk_filter(const float* __restrict__ raw, int n_cols, uint32_t first_row, uin
 }
 
 // One warp's list: up to kTopkCapacity keys in shared memory, sorted down to the n_best largest when it fills.
+// The lanes' keys in descending order.
+__device__ __forceinline__ unsigned long long lanes_sort_desc(unsigned long long key) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll 1
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, j);
+            const bool keep_larger = ((lane & j) == 0) == ((lane & k) == 0);
+            key = (key > other) == keep_larger ? key : other;
+        }
+    return key;
+}
+
+// The first `count` of kTopkCapacity keys in descending order, zeros behind them.
+static __device__ __noinline__ void topk_sort(unsigned long long* buf, int count) {
+    for (int i = count + (threadIdx.x & 31); i < kTopkCapacity; i += 32) buf[i] = 0ull;
+    __syncwarp();
+    warp_sort_desc(buf);
+}
+
 struct TopkList {
     unsigned long long* buf;
     int count, n_best;
     unsigned long long cutoff;  // keys up to it cannot be among the n_best
 
+    // A list of up to 32 keys, as a first scan with a cut-off leaves, is sorted a key per lane (15 exchanges); the register
+    // sort of 256 keys takes 36, of eight keys per lane each.
     __device__ __noinline__ void sort() {
         const int lane = threadIdx.x & 31;
+        if (count <= 32) {
+            const unsigned long long key = lanes_sort_desc(lane < count ? buf[lane] : 0ull);
+            count = min(count, n_best);
+            buf[lane] = lane < count ? key : 0ull;
+            __syncwarp();
+            cutoff = count >= n_best ? buf[n_best - 1] : 0ull;
+            return;
+        }
         warp_sort_desc(buf);
         count = min(count, n_best);
         for (int i = count + lane; i < kTopkCapacity; i += 32) buf[i] = 0ull;
@@ -2597,26 +2628,25 @@ struct TopkList {
         const int lane = threadIdx.x & 31;
         const bool few = n_best <= 32;
         unsigned long long top[4] = {0ull, 0ull, 0ull, 0ull};
-        for (int i = lane; i < n; i += 32) {
-            unsigned long long key = key_of(i);
+        constexpr int kAhead = 5;  // keys fetched before the first of them is looked at
+        for (int i0 = lane; i0 < n; i0 += 32 * kAhead) {
+            unsigned long long ahead[kAhead];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                if (r > 0 && few) break;
-                const unsigned long long less = key < top[r] ? key : top[r];
-                top[r] = key < top[r] ? top[r] : key;
-                key = less;
+            for (int u = 0; u < kAhead; ++u) ahead[u] = i0 + 32 * u < n ? key_of(i0 + 32 * u) : 0ull;
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                unsigned long long key = ahead[u];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    if (r > 0 && few) break;
+                    const unsigned long long less = key < top[r] ? key : top[r];
+                    top[r] = key < top[r] ? top[r] : key;
+                    key = less;
+                }
             }
         }
         if (few) {
-#pragma unroll 1
-            for (int k = 2; k <= 32; k <<= 1)
-#pragma unroll 1
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    const unsigned long long other = __shfl_xor_sync(0xffffffffu, top[0], j);
-                    const bool keep_larger = ((lane & j) == 0) == ((lane & k) == 0);
-                    top[0] = (top[0] > other) == keep_larger ? top[0] : other;
-                }
-            top[0] = __shfl_sync(0xffffffffu, top[0], n_best - 1);
+            top[0] = __shfl_sync(0xffffffffu, lanes_sort_desc(top[0]), n_best - 1);
         } else {
 #pragma unroll
             for (int r = 0; r < 4; ++r) buf[r * 32 + lane] = top[r];
@@ -2655,27 +2685,89 @@ struct TopkList {
 // The first batch of a ranking, when no query has a cut-off: gridDim.y warps per query each scan a part of its row and
 // leave their n_best keys (0 for missing ones) as candidates, which k_topk_update merges like any other.  One warp per
 // query took 25 us for every 4096 scores, on as many SMs as there are groups of four queries.
-static __global__ void __launch_bounds__(128)
+// FEW: up to 32 keys per query.
+template <bool FEW>
+__global__ void __launch_bounds__(128, FEW ? 8 : 4)
 k_topk_seed(const float* __restrict__ raw, int n_cols, uint32_t first_row, uint32_t last_valid_row, unsigned long long* __restrict__ cand,
             int* __restrict__ cand_count, TopkParams tp) {
     __shared__ __align__(16) unsigned long long buffers[4][kTopkCapacity];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = blockIdx.x * 4 + warp;
     if (q >= tp.n_query) return;
-    TopkList list{buffers[warp], 0, tp.n_best, 0ull};
-    for (int i = lane; i < kTopkCapacity; i += 32) list.buf[i] = 0ull;
-    __syncwarp();
+    unsigned long long* const buf = buffers[warp];
     const int part = ((n_cols + (int)gridDim.y - 1) / (int)gridDim.y + 31) / 32 * 32, begin = (int)blockIdx.y * part;
     const float* __restrict__ row = raw + (size_t)q * n_cols;
     const int end = min(n_cols, begin + part);
-    list.raise_cutoff(end - begin, [&](int i) {
-        const uint32_t table_row = first_row + (uint32_t)(begin + i);
-        return table_row <= last_valid_row ? topk_key(tp.score_is_gamma_minus ? tp.gamma - row[begin + i] : row[begin + i], table_row) : 0ull;
-    });
-    list.scan(row, begin, end, first_row, last_valid_row, tp);
-    list.sort();
+    auto score_at = [&](int j) { return tp.score_is_gamma_minus ? tp.gamma - row[j] : row[j]; };
     unsigned long long* __restrict__ out = cand + (size_t)q * kTopkCandidates + (size_t)blockIdx.y * tp.n_best;
-    for (int i = lane; i < tp.n_best; i += 32) out[i] = list.buf[i];
     if (blockIdx.y == 0 && lane == 0) cand_count[q] = (int)gridDim.y * tp.n_best;
+    if constexpr (FEW) {
+        // Scores are held in registers, all of a tile read at the same time, and compared as floats: only what reaches the
+        // cut-off's score becomes a key, and the few keys that do are sorted a key per lane.  (With every score made a key
+        // twice, its reads waited for a few at a time, and a 256-key sort at the end, 128 queries x 40 000 scores took 58 us; 24
+        // this way; with 20 scores held
+        // instead of ten, which do not fit 64 registers, 36.)
+        constexpr int kHold = 10;
+        const int valid = (int)min((long long)end, (long long)last_valid_row - (long long)first_row + 1);
+        int count = 0;
+        unsigned long long cutoff = 0ull;
+        for (int tile = begin; tile < end; tile += 32 * kHold) {
+            float score[kHold];
+#pragma unroll
+            for (int u = 0; u < kHold; ++u) {
+                const int j = tile + 32 * u + lane;
+                score[u] = j < valid ? score_at(j) : 0.f;
+            }
+            if (tile == begin) {
+                // the n_best-th of the lanes' largest keys: so many keys reach it
+                float best = -INFINITY;
+                int at = -1;
+#pragma unroll
+                for (int u = 0; u < kHold; ++u) {
+                    const int j = tile + 32 * u + lane;
+                    if (j < valid && (at < 0 || score[u] > best)) best = score[u], at = j;
+                }
+                const unsigned long long bound =
+                    __shfl_sync(0xffffffffu, lanes_sort_desc(at >= 0 ? topk_key(best, first_row + (uint32_t)at) : 0ull), tp.n_best - 1);
+                if (bound > 0ull) cutoff = bound - 1;
+            }
+#pragma unroll
+            for (int u = 0; u < kHold; ++u) {
+                const int j = tile + 32 * u + lane;
+                bool pass = j < valid && (cutoff == 0ull || !(score[u] < topk_score(cutoff)));
+                if (__ballot_sync(0xffffffffu, pass) == 0) continue;
+                const unsigned long long key = topk_key(score[u], first_row + (uint32_t)j);
+                pass = pass && key > cutoff;
+                const unsigned mask = __ballot_sync(0xffffffffu, pass);
+                if (pass) buf[count + __popc(mask & ((1u << lane) - 1))] = key;
+                count += __popc(mask);
+                __syncwarp();
+                if (count + 32 > kTopkCapacity) {
+                    topk_sort(buf, count);
+                    count = tp.n_best;
+                    cutoff = buf[tp.n_best - 1];
+                }
+            }
+        }
+        if (count <= 32) {
+            const unsigned long long key = lanes_sort_desc(lane < count ? buf[lane] : 0ull);
+            if (lane < tp.n_best) out[lane] = key;
+        } else {
+            topk_sort(buf, count);
+            if (lane < tp.n_best) out[lane] = buf[lane];
+        }
+        return;
+    } else {
+        TopkList list{buf, 0, tp.n_best, 0ull};
+        for (int i = lane; i < kTopkCapacity; i += 32) list.buf[i] = 0ull;
+        __syncwarp();
+        list.raise_cutoff(end - begin, [&](int i) {
+            const uint32_t table_row = first_row + (uint32_t)(begin + i);
+            return table_row <= last_valid_row ? topk_key(score_at(begin + i), table_row) : 0ull;
+        });
+        list.scan(row, begin, end, first_row, last_valid_row, tp);
+        list.sort();
+        for (int i = lane; i < tp.n_best; i += 32) out[i] = list.buf[i];
+    }
 }
 
 // raw [n_query, n_cols] holds distances / dot products against rows first_row .. first_row+n_cols-1;
@@ -2711,8 +2803,16 @@ k_topk_update(const float* __restrict__ raw, int n_cols, uint32_t first_row, uin
     if (ranked) list.sort();
     if (lane == 0) cand_count[q] = 0;
     if (n_cand <= kTopkCandidates) {
-        if (list.count == 0 && n_cand > kTopkCapacity) list.raise_cutoff(n_cand, [&](int i) { return keys[i]; });
-        for (int base = 0; base < n_cand; base += 32) list.add(base + lane < n_cand ? keys[base + lane] : 0ull);
+        // (a bound first, where what passes it is likely to be sorted a key per lane)
+        if (list.count == 0 && n_cand > (tp.n_best <= 16 ? 32 : kTopkCapacity)) list.raise_cutoff(n_cand, [&](int i) { return keys[i]; });
+        constexpr int kAhead = 8;  // keys fetched before the first of them is looked at
+        for (int base = 0; base < n_cand; base += 32 * kAhead) {
+            unsigned long long ahead[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) ahead[u] = base + 32 * u + lane < n_cand ? keys[base + 32 * u + lane] : 0ull;
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) list.add(ahead[u]);
+        }
     } else {  // more than the candidate list holds
         list.scan(raw + (size_t)q * n_cols, 0, n_cols, first_row, last_valid_row, tp);
     }

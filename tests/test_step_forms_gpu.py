@@ -111,3 +111,28 @@ def test_loss_rows_of_any_length(loss_type, adversarial, a2a):
     """One column and more per thread, up to the longest row, the last of a thread's there and not; 256 and 512 threads."""
     cfg = _config("DistMult", "MatMul", n_entity=4200, batch_size=4, a2a_size=a2a, embedding_size=8, loss_type=loss_type, negative_adversarial_scale=adversarial)
     _two_runs(cfg, seed=a2a, rtol=1e-4, n_step=1, pad=1 if a2a == 2 else 3)
+
+
+@pytest.mark.parametrize("rows,n_best", [(2, 1), (330, 5), (700, 32), (700, 33), (5200, 20)])
+@pytest.mark.parametrize("same", [False, True], ids=["different", "ties"])
+def test_first_scan_of_a_ranking(rows, n_best, same):
+    """Parts with fewer scores than a warp holds, one more and several times as many; lists of up to 32 keys and longer ones;
+    equal scores, of which every one reaches the cut-off (ties go to the lower row)."""
+    from test_predict_gpu import _clear, _predict
+
+    cfg = _config("TransE", "L1", n_shard=2, n_entity=rows + 1, batch_size=2, a2a_size=2, embedding_size=8)
+    state = random_state(cfg, rows)
+    if same:
+        state["entity_data"][..., :8] = state["entity_data"][:, 1:2, :8]
+    n_best = min(n_best, rows)
+    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW, **{"execution.predict_hr_batch_size": 3, "execution.predict_n_best": n_best}))
+    write_state(engine, cfg, state, RW)
+    rng = np.random.RandomState(1)
+    queries = np.stack([np.arange(6) % 2, 1 + rng.randint(rows, size=6), rng.randint(12, size=6)], axis=1)
+    counts = np.array([rows, max(n_best, rows - 3)])
+    got_idx, got_score = _predict(engine, cfg, queries, counts, 3, n_best)
+    engine.close()
+    want_idx, want_score = make_oracle(cfg, state).predict(queries, counts, n_best)
+    assert_close(got_score, want_score, 1e-5, "ranking: scores")
+    clear = np.ones_like(want_score, bool) if same or n_best == 1 else _clear(want_score)
+    np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
