@@ -2624,26 +2624,37 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
         KGE_CUDA(cudaEventRecord(io_event(0), stream_));
     }
 
-    // 1. predicted tails of the local queries, written into every process's gathered query buffer
-    for (unsigned l = 0; l < n; ++l) {
-        dim3 grid(ceil_div((unsigned)hr, 64), dtiles, 1);
-        KGE_LAUNCH("predict_hidden", KGE_DISPATCH_ROW(cfg_, k_hidden<ST, FT><<<grid, 256, 0, stream_>>>(
-                                                                shards_[l].table, layout_, d_head + l * hr, 0u, (int)hr, W_head,
-                                                                nullptr, p_head_hidden_, nullptr)));
-        if (mlp_on()) launch_mlp_forward(shards_[l].table, d_head + l * hr, 0u, (unsigned)hr, 0, p_head_hidden_, p_mlp_cat_, p_mlp_pre_, p_mlp_out_);
+    // 1. predicted tails of the local queries, written into every process's gathered query buffer: from the table itself
+    // without features, all shards at once, else from the hidden rows of one shard after the other
+    const bool from_table = cfg_.f == 0;
+    const unsigned at_once = from_table ? (unsigned)kShardBatch : 1u;
+    const int value_type = !from_table ? 0 : cfg_.value_bf16 ? 2 : cfg_.state_type == ST_F16 ? 1 : 0;
+    for (unsigned l0 = 0; l0 < n; l0 += at_once) {
+        const unsigned count_l = std::min<unsigned>(at_once, (unsigned)n - l0);
+        if (!from_table) {
+            dim3 grid(ceil_div((unsigned)hr, 64), dtiles, 1);
+            KGE_LAUNCH("predict_hidden", KGE_DISPATCH_ROW(cfg_, k_hidden<ST, FT><<<grid, 256, 0, stream_>>>(
+                                                                    shards_[l0].table, layout_, d_head + l0 * hr, 0u, (int)hr, W_head,
+                                                                    nullptr, p_head_hidden_, nullptr)));
+            if (mlp_on()) launch_mlp_forward(shards_[l0].table, d_head + l0 * hr, 0u, (unsigned)hr, 0, p_head_hidden_, p_mlp_cat_, p_mlp_pre_, p_mlp_out_);
+        }
         for (unsigned p = 0; p < cfg_.world; ++p) {
-            float* dst = (float*)(peer_arena_[p] + arena_offset_predict(0)) + (size_t)(shard0_ + l) * hr * D;
             ShardArgs<LookupArgs> query{};
-            query.s[0].rows = LookupRows{reinterpret_cast<const uint8_t*>(p_head_hidden_), nullptr, d_iota_, nullptr, D * 4};
-            query.s[0].relation = d_rel + l * hr;
-            query.s[0].pred = dst;
-            query.s[0].nrm = dst + Q * D;  // TransH
+            for (unsigned i = 0; i < count_l; ++i) {
+                const unsigned l = l0 + i;
+                LookupArgs& a = query.s[i];
+                a.rows = from_table ? LookupRows{shards_[l].table, nullptr, d_head + l * hr, nullptr, layout_.row_bytes}
+                                    : LookupRows{reinterpret_cast<const uint8_t*>(p_head_hidden_), nullptr, d_iota_, nullptr, D * 4};
+                a.relation = d_rel + l * hr;
+                a.pred = (float*)(peer_arena_[p] + arena_offset_predict(0)) + (size_t)(shard0_ + l) * hr * D;
+                a.nrm = a.pred + Q * D;  // TransH
+            }
             LookupSizes sizes{};
             sizes.rel_table = dense_;
             sizes.normal_table = dense_ + dense_bounds_[3];
             sizes.B = (int)hr;
             sizes.D = (int)D;
-            KGE_LAUNCH("predict_query", KGE_CUDA(kge::launch_lookup(query, 1, sizes, cfg_.score_fn, 0, stream_)));
+            KGE_LAUNCH("predict_query", KGE_CUDA(kge::launch_lookup(query, (int)count_l, sizes, cfg_.score_fn, value_type, stream_)));
         }
     }
     KGE_CUDA(cudaGetLastError());

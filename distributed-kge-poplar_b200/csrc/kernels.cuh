@@ -629,20 +629,23 @@ inline cudaError_t launch_score_block(const ShardArgs<ScoreArgs>& shards, int n_
 }
 
 // The same scores where there are enough of them to fill the GPU with tiles (ranking): a block owns 64 x 128 outputs, its
-// 8 warps 32 x 32 each; all of them walk all of k in chunks of 32 staged one ahead.  Each chunk is summed by itself and
-// added to the total, as k_score_block adds its groups' chunks.  Bound by the FP32 pipe.  (With k_score_block's division of k
+// 8 warps 32 x 32 each (or 64 x 96 and 32 x 24, where that ends sooner); all of them walk all of k in chunks of 32 staged one
+// ahead.  Each chunk is summed by itself and added to the total, as k_score_block adds its groups' chunks.  Bound by the FP32 pipe.  (With k_score_block's division of k
 // half the warps have nothing to do at 100 columns, and 1024 outputs a block pay for a reduction.)
-constexpr int kScoreTileP = 64, kScoreTileT = 128;
-constexpr int kScoreTileStage = (kScoreTileP + kScoreTileT) * kScoreStride;
-constexpr size_t kScoreTileSmem = 2 * kScoreTileStage * sizeof(float);
+constexpr int kScoreTileP = 64;
+template <int NB>
+constexpr int kScoreTileStage = (kScoreTileP + 16 * NB) * kScoreStride;
+template <int NB>
+constexpr size_t kScoreTileSmem = 2 * kScoreTileStage<NB> * sizeof(float);
 
-template <int FN>
+template <int FN, int NB>
 __global__ void __launch_bounds__(256, 2)
 k_score_tile(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, int D, int ld) {
     const float* __restrict__ P = shards.s[blockIdx.z].P;
     const float* __restrict__ Tl = shards.s[blockIdx.z].Tl;
     float* __restrict__ raw = shards.s[blockIdx.z].raw;
     grid_dependency_sync();
+    constexpr int kScoreTileT = 16 * NB;
     extern __shared__ __align__(16) float score_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ty = lane >> 2, tx = lane & 3;
     const int i0 = blockIdx.y * kScoreTileP, j0 = blockIdx.x * kScoreTileT;
@@ -657,33 +660,33 @@ k_score_tile(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, 
             else *reinterpret_cast<float4*>(d) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
-    float total[4][8];
+    float total[4][NB];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 8; ++b) total[a][b] = 0.f;
-    const int row_p = (warp >> 2) * 32 + ty, row_t = kScoreTileP + (warp & 3) * 32 + tx;
+        for (int b = 0; b < NB; ++b) total[a][b] = 0.f;
+    const int row_p = (warp >> 2) * 32 + ty, row_t = kScoreTileP + (warp & 3) * 4 * NB + tx;
     stage(0, score_smem);
     asm volatile("cp.async.commit_group;" ::: "memory");
     for (int k0 = 0, half = 0; k0 < D; k0 += 32, half ^= 1) {
-        if (k0 + 32 < D) stage(k0 + 32, score_smem + (half ^ 1) * kScoreTileStage);
+        if (k0 + 32 < D) stage(k0 + 32, score_smem + (half ^ 1) * kScoreTileStage<NB>);
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();
-        const float* Ps = score_smem + half * kScoreTileStage + row_p * kScoreStride;
-        const float* Ts = score_smem + half * kScoreTileStage + row_t * kScoreStride;
-        float acc[4][8];
+        const float* Ps = score_smem + half * kScoreTileStage<NB> + row_p * kScoreStride;
+        const float* Ts = score_smem + half * kScoreTileStage<NB> + row_t * kScoreStride;
+        float acc[4][NB];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
+            for (int b = 0; b < NB; ++b) acc[a][b] = 0.f;
 #pragma unroll 1
         for (int k4 = 0; k4 < min(32, D - k0); k4 += 4) {
             float4 pv[4];
 #pragma unroll
             for (int a = 0; a < 4; ++a) pv[a] = load4(Ps + 8 * a * kScoreStride + k4);
 #pragma unroll
-            for (int b = 0; b < 8; ++b) {
+            for (int b = 0; b < NB; ++b) {
                 const float4 tv = load4(Ts + 4 * b * kScoreStride + k4);
                 const float tr[4] = {tv.x, tv.y, tv.z, tv.w};
 #pragma unroll
@@ -706,16 +709,16 @@ k_score_tile(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, 
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int b = 0; b < 8; ++b) total[a][b] += acc[a][b];
+            for (int b = 0; b < NB; ++b) total[a][b] += acc[a][b];
         __syncthreads();
     }
     // through shared memory, so that whole rows are stored
     constexpr int kOut = kScoreTileT + 4;
-    static_assert(kScoreTileP * kOut <= 2 * kScoreTileStage, "the outputs fit");
+    static_assert(kScoreTileP * kOut <= 2 * kScoreTileStage<NB>, "the outputs fit");
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 8; ++b)
+        for (int b = 0; b < NB; ++b)
             score_smem[(row_p + 8 * a) * kOut + row_t - kScoreTileP + 4 * b] = FN == DIST_L2 ? sqrtf(total[a][b]) : total[a][b];
     __syncthreads();
     const bool vec = (ld & 3) == 0;
@@ -735,6 +738,18 @@ k_score_tile(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, 
     }
 }
 
+template <int FN, int NB>
+inline cudaError_t launch_score_tile(const ShardArgs<ScoreArgs>& shards, dim3 tiles, int B, int T, int D, int ld, cudaStream_t stream) {
+    static bool configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
+    const int slot = current_device_slot();
+    if (slot < 0 || !configured[slot]) {
+        const cudaError_t err = cudaFuncSetAttribute(k_score_tile<FN, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreTileSmem<NB>);
+        if (err != cudaSuccess) return err;
+        if (slot >= 0) configured[slot] = true;
+    }
+    return launch_dependent(k_score_tile<FN, NB>, tiles, dim3(256), kScoreTileSmem<NB>, stream, shards, B, T, D, ld);
+}
+
 // Picks the kernel: the 16-byte-copy form when the rows allow it, the general form otherwise.  Rows of the scores begin
 // `ld` floats apart.  `sync` with world > 1: the kernel waits for the tail rows of the other processes (only the
 // 16-byte-copy form can; returns cudaErrorNotSupported otherwise so that the caller waits first).
@@ -751,17 +766,16 @@ inline cudaError_t launch_score(const ShardArgs<ScoreArgs>& shards, int n_shards
         if (sync.world > 1) return cudaErrorNotSupported;
         return launch_dependent(k_score<FN>, dim3((T + 63) / 64, (B + 31) / 32, n), dim3(128), 0, stream, shards, B, T, D, ld);
     }
-    static bool configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
-    const int slot = current_device_slot();
-    if (slot < 0 || !configured[slot]) {
-        const cudaError_t err = cudaFuncSetAttribute(k_score_tile<FN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreTileSmem);
-        if (err != cudaSuccess) return err;
-        if (slot >= 0) configured[slot] = true;
+    // Whole tiles from two blocks per SM on; below that, and where tails are waited for, the k range is divided too.  96
+    // columns a tile where its waves of 296 blocks end before those of 128 (128 x 40 000 x 100: 834 tiles in three waves, not
+    // 626 in three, 62 -> 60 us with its timing).
+    auto tiles = [&](int width) { return dim3((T + width - 1) / width, (B + kScoreTileP - 1) / kScoreTileP, n); };
+    const dim3 wide = tiles(128), narrow = tiles(96);
+    if (sync.world <= 1 && (size_t)wide.x * wide.y * n >= 2 * kSmCount) {
+        auto waves = [&](const dim3& t) { return ((size_t)t.x * t.y * n + 2 * kSmCount - 1) / (2 * kSmCount); };
+        if (waves(narrow) * 96 < waves(wide) * 128) return launch_score_tile<FN, 6>(shards, narrow, B, T, D, ld, stream);
+        return launch_score_tile<FN, 8>(shards, wide, B, T, D, ld, stream);
     }
-    // whole tiles from two blocks per SM on; below that, and where tails are waited for, the k range is divided too
-    const dim3 tiles((T + kScoreTileT - 1) / kScoreTileT, (B + kScoreTileP - 1) / kScoreTileP, n);
-    if (sync.world <= 1 && (size_t)tiles.x * tiles.y * n >= 2 * 148)
-        return launch_dependent(k_score_tile<FN>, tiles, dim3(256), kScoreTileSmem, stream, shards, B, T, D, ld);
     // The width whose waves of 148 blocks end first: 4 NB D clocks for a block's sums, about 4 us for what does not depend
     // on its width.
     auto clocks = [&](int nb) {

@@ -136,3 +136,31 @@ def test_first_scan_of_a_ranking(rows, n_best, same):
     assert_close(got_score, want_score, 1e-5, "ranking: scores")
     clear = np.ones_like(want_score, bool) if same or n_best == 1 else _clear(want_score)
     np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
+
+
+@pytest.mark.parametrize("shape", [(64, 37888, 36), (65, 18945, 64), (64, 37889, 36)])
+def test_scores_in_tiles_of_both_widths(shape):
+    """One wave of 128-column tiles, the same with ragged ones, and one tile more: two waves, so tiles of 96 columns."""
+    test_scores_in_blocks(capi.L1, shape)
+
+
+@pytest.mark.parametrize("score_fn,distance_fn", [("TransE", "L1"), ("ComplEx", "MatMul"), ("RotatE", "L2"), ("TransH", "L1")])
+@pytest.mark.parametrize("d,dtype", [(4, "float32"), (6, "float32"), (38, "float16"), (132, "float16")])
+def test_ranked_queries_straight_from_the_table(score_fn, distance_fn, d, dtype):
+    """Five shards without features: queries of four shards in a launch and the fifth by itself; 16-byte rows and others."""
+    from test_predict_gpu import _clear, _predict
+
+    store = np.dtype(dtype).type
+    cfg = _config(score_fn, distance_fn, n_shard=5, n_entity=90, batch_size=10, a2a_size=4, n_relation_type=10, embedding_size=d)
+    state = random_state(cfg, d)
+    state["entity_data"] = state["entity_data"].astype(store).astype(np.float32)
+    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW, dtype=dtype, **{"execution.predict_hr_batch_size": 3}))
+    write_state(engine, cfg, state, RW, dtype=store)
+    rng = np.random.RandomState(1)
+    queries = np.stack([np.arange(15) % 5, 1 + rng.randint(89, size=15), rng.randint(10, size=15)], axis=1)
+    got_idx, got_score = _predict(engine, cfg, queries, np.full(5, 89), 3, 5)
+    engine.close()
+    want_idx, want_score = make_oracle(cfg, state).predict(queries, np.full(5, 89), 5)
+    assert_close(got_score, want_score, 1e-5, "ranking: scores")
+    clear = _clear(want_score)
+    np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
