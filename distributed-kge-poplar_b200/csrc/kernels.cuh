@@ -65,6 +65,10 @@ struct AdamParams {
     float epsilon;
     float weight_decay;
 };
+// a x + b y with the first product unrounded.  Which one the addition takes in is the compiler's choice in every kernel anew
+// unless it is written out, and an L1 model, whose gradients are what rounding leaves of a sum, carries a last bit on: rows
+// and dense parameters have one form each in all kernels.
+__device__ __forceinline__ float weighted_sum(float a, float x, float b, float y) { return __fmaf_rn(a, x, __fmul_rn(b, y)); }
 
 __device__ __forceinline__ float load_as_float(const float* p) { return *p; }
 __device__ __forceinline__ float load_as_float(const __half* p) { return __half2float(*p); }
@@ -1693,8 +1697,8 @@ __device__ __forceinline__ void relation_row_sum(const ShardArgs<EntityShard>& s
         }
         const size_t e = (size_t)rho * D + c;
         const float alpha = *g.step_size * g.rel_lr_modifier[table];
-        const float mo = ap.beta_m * g.rel_m[table][e] + ap.one_minus_beta_m * total;
-        const float ve = ap.beta_v * g.rel_v[table][e] + ap.one_minus_beta_v * total * total;
+        const float mo = weighted_sum(ap.beta_m, g.rel_m[table][e], ap.one_minus_beta_m, total);
+        const float ve = weighted_sum(ap.beta_v, g.rel_v[table][e], __fmul_rn(ap.one_minus_beta_v, total), total);
         const float x = g.rel_w[table][e];
         g.rel_w[table][e] = x - alpha * (mo / (sqrtf(ve) + ap.epsilon) + ap.weight_decay * x);
         g.rel_m[table][e] = mo;
@@ -1713,8 +1717,8 @@ __device__ __forceinline__ void relation_row_sum(const ShardArgs<EntityShard>& s
         float mo[4] = {m4.x, m4.y, m4.z, m4.w}, ve[4] = {v4.x, v4.y, v4.z, v4.w}, x[4] = {x4.x, x4.y, x4.z, x4.w};
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            mo[u] = ap.beta_m * mo[u] + ap.one_minus_beta_m * total[u];
-            ve[u] = ap.beta_v * ve[u] + ap.one_minus_beta_v * total[u] * total[u];
+            mo[u] = weighted_sum(ap.beta_m, mo[u], ap.one_minus_beta_m, total[u]);
+            ve[u] = weighted_sum(ap.beta_v, ve[u], __fmul_rn(ap.one_minus_beta_v, total[u]), total[u]);
             x[u] = x[u] - alpha * (mo[u] / (sqrtf(ve[u]) + ap.epsilon) + ap.weight_decay * x[u]);
         }
         store4(g.rel_w[table] + e, make_float4(x[0], x[1], x[2], x[3]));
@@ -2002,9 +2006,8 @@ k_entity_update(const __grid_constant__ ShardArgs<EntityShard> shards, const __g
         }
 #pragma unroll
         for (int u = 0; u < V; ++u) {
-            float v = qq[u] * qq[u];
-            m[u] = ap.beta_m * m[u] + ap.one_minus_beta_m * gv[u];
-            v = ap.beta_v * v + ap.one_minus_beta_v * gv[u] * gv[u];
+            const float v = weighted_sum(__fmul_rn(ap.one_minus_beta_v, gv[u]), gv[u], ap.beta_v, __fmul_rn(qq[u], qq[u]));
+            m[u] = weighted_sum(ap.one_minus_beta_m, gv[u], ap.beta_m, m[u]);
             x[u] = x[u] - alpha * (m[u] / (sqrtf(v) + ap.epsilon) + ap.weight_decay * x[u]);
             qq[u] = sqrtf(v);
         }
@@ -2345,8 +2348,8 @@ __device__ __forceinline__ int dense_param_of(const DenseUpdateArgs& a, size_t e
 }
 
 __device__ __forceinline__ float dense_adam(float x, float g, float& m, float& v, float alpha, const AdamParams& ap) {
-    m = ap.beta_m * m + ap.one_minus_beta_m * g;
-    v = ap.beta_v * v + ap.one_minus_beta_v * g * g;
+    m = weighted_sum(ap.beta_m, m, ap.one_minus_beta_m, g);
+    v = weighted_sum(ap.beta_v, v, __fmul_rn(ap.one_minus_beta_v, g), g);
     return x - alpha * (m / (sqrtf(v) + ap.epsilon) + ap.weight_decay * x);
 }
 

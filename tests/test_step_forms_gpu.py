@@ -164,3 +164,30 @@ def test_ranked_queries_straight_from_the_table(score_fn, distance_fn, d, dtype)
     assert_close(got_score, want_score, 1e-5, "ranking: scores")
     clear = _clear(want_score)
     np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
+
+
+@pytest.mark.parametrize("d,features", [(6, 0), (16, 0), (16, 12)], ids=["odd rows", "table rows", "gathered rows"])
+def test_row_moments_round_alike(d, features):
+    """Every form of the row update rounds the moments' old part and not the gradient's: the bits of that sum."""
+    cfg = _config("TransE", "L1", embedding_size=d, entity_feature_size=features, loss_type="softmax", correction_weight=1.0)
+    state = random_state(cfg, d, warm=True)
+    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW))
+    write_state(engine, cfg, state, RW)
+    batch = random_batch(cfg, 1, 3, pad=3)
+    engine.run("train_step_loop", dict(learning_rate=np.full(1, 1e-3, np.float32), loss=np.zeros(1, np.float32), **batch))
+    grad = engine.debug_fetch("d_hidden", 0, cfg.n_remote * d).reshape(-1, d)
+    got = read_rows(engine, cfg, RW, 1, np.float32)[0]
+    engine.close()
+    remote = batch["remote"][0, 0]
+    rows, slots = np.unique(remote, return_index=True)
+    rows, slots = rows[rows > 0], slots[rows > 0]
+    g, old = grad[slots], state["entity_data"][0][rows]
+    mul = lambda a, b: np.float32(a) * np.float32(b)
+
+    def after(a, x, b, y):  # in 64 bits of mantissa: a x is exact, the sum rounded once more than in hardware, at 2^-40 odds
+        return (np.longdouble(a) * x.astype(np.longdouble) + mul(b, y)).astype(np.float32)
+
+    one_m, one_v = np.float32(1) - np.float32(cfg.adam_beta_m), np.float32(1) - np.float32(cfg.adam_beta_v)
+    np.testing.assert_array_equal(got[rows, d : 2 * d], after(one_m, g, cfg.adam_beta_m, old[:, d : 2 * d]))
+    root = old[:, 2 * d : 3 * d]
+    np.testing.assert_array_equal(got[rows, 2 * d : 3 * d], np.sqrt(after(mul(one_v, g).astype(np.longdouble), g, cfg.adam_beta_v, mul(root, root))))
