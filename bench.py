@@ -250,7 +250,7 @@ def step_traffic(n_shard: int) -> dict:
         "gather": 2 * R * (row_state + row_feat),
         # reads value + features of R rows and the projection, writes the hidden rows
         "hidden": R * (D * 4 + row_feat) + F * D * 4 + R * D * 4,
-        "route": 2 * (T + B) * D * 4 + B * D * 4,
+        "lookup": 2 * (T + B) * D * 4 + B * D * 4,
         "score": (B + T) * D * 4 + B * T * 4,
         "loss": 2 * B * T * 4,
         "score_bwd": 2 * B * T * 4 + 2 * (B + T) * D * 4,

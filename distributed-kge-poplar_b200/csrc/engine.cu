@@ -1704,7 +1704,7 @@ EntityStep Engine::entity_step(unsigned step, unsigned n) const {
 // wrote (the upper TF32 plane) plus a lower plane the same producer wrote next to it.
 // With a stream per shard instead, forked and joined three times a step, and a dense update of its own (us per step,
 // before -> after): demo preset, 2 shards, 40.4 -> 32.3; four shards of 256 x 320 L1 scores, 76.4 -> 67.2; four of 256 x 512
-// fp16 rows, 79.4 -> 83.1; two shards of the headline step 129.5 -> 112.9.
+// fp16 rows, 79.4 -> 83.1 (57.4 with the pair gradients of today); two shards of the headline step 129.5 -> 112.9.
 void Engine::launch_step_planes(unsigned step, const LossParams& lp, float normaliser) {
     const unsigned B = cfg_.batch_size, T = cfg_.n_tail(), R = cfg_.n_remote(), D = cfg_.d, F = cfg_.f;
     const unsigned n_rel = cfg_.n_relation_type, parity = step & 1, n_nets = cfg_.n_net(), ld = score_ld_;
