@@ -1028,13 +1028,6 @@ void Engine::last_run_stats(float* ms, unsigned long long* launches) const {
         ++launch_counter_;               \
     } while (0)
 
-// The same for a launch that works on `n` local shards, which counts as the n kernels it stands for.
-#define KGE_LAUNCH_SHARDS(name, n, ...)  \
-    do {                                 \
-        KGE_LAUNCH(name, __VA_ARGS__);   \
-        launch_counter_ += (n) - 1u;     \
-    } while (0)
-
 bool dependent_launch_enabled() {
     static const bool enabled = [] {
         const char* off = std::getenv("KGE_NO_DEPENDENT_LAUNCH");
@@ -1190,7 +1183,7 @@ void Engine::launch_gather(unsigned step, unsigned l0, unsigned n, cudaStream_t 
         const ShardBuffers& b = shards_[l0 + i];
         shards.s[i] = GatherArgs{b.table, d_remote_ + ((size_t)(l0 + i) * cfg_.n_step + step) * R, b.rows_c2[step & 1], feature_planes(b, step & 1)};
     }
-    KGE_LAUNCH_SHARDS("gather", n, KGE_CUDA(launch_dependent(k_gather_step_rows, dim3(ceil_div(R, 8), n), dim3(256), 0, stream, shards, layout_.row_bytes, (int)R)));
+    KGE_LAUNCH("gather", KGE_CUDA(launch_dependent(k_gather_step_rows, dim3(ceil_div(R, 8), n), dim3(256), 0, stream, shards, layout_.row_bytes, (int)R)));
 }
 
 FeaturePlanes Engine::feature_planes(const ShardBuffers& b, unsigned parity) const {
@@ -1390,7 +1383,7 @@ static unsigned divide_k(const tc::PlaneProblem* problems, int n_problems, unsig
     return chain;
 }
 
-// One launch of the plane-fed contraction for problems of the same shape class, those of `n_shards` local shards.  Tiles
+// One launch of the plane-fed contraction for problems of the same shape class, those of several local shards.  Tiles
 // are 128 x 128 (128 x 64 for narrow outputs); the k range is divided over the blocks of a cluster so that about one block
 // per SM is busy and every split keeps at least two slices.  The two score gradients of a batch with many more tails than
 // triples have k ranges of very different length, and only the longer one wants dividing: with one number of splits for
@@ -1398,7 +1391,7 @@ static unsigned divide_k(const tc::PlaneProblem* problems, int n_problems, unsig
 // operands stay with one number: their slices are short, the operands' way from L2 bounds them, and 1024 x 2048 x 512 with 16
 // slices a block in place of 32 took 2 us longer.
 void Engine::launch_planes(const char* name, tc::PlaneProblem* problems, int n_problems, int side, int wait_kind, int signal_kind,
-                           const tc::Routing* routing, unsigned n_shards) {
+                           const tc::Routing* routing) {
     int max_n = 0, max_k = 0;
     unsigned tiles = 0;
     bool alike = true;
@@ -1442,7 +1435,7 @@ void Engine::launch_planes(const char* name, tc::PlaneProblem* problems, int n_p
     else if (side == tc::SIDE_NORMS) err = tc::launch_planes<tc::SIDE_NORMS>(problems, n_problems, splits, tile_n, stream_, exchange_sync(), wait_kind, signal_kind, routing);
     else err = tc::launch_planes<tc::SIDE_NONE>(problems, n_problems, splits, tile_n, stream_, exchange_sync(), wait_kind, signal_kind, routing);
     timing_end();
-    launch_counter_ += n_shards;
+    ++launch_counter_;
     KGE_CUDA(err);
 }
 
@@ -1601,7 +1594,7 @@ void Engine::launch_lookup(unsigned l0, unsigned n, unsigned step) {
             a.hid = b.hid_h;
         }
     }
-    KGE_LAUNCH_SHARDS("lookup", n, KGE_CUDA(kge::launch_lookup(shards, (int)n, sizes, cfg_.score_fn, lookup_type(), stream_)));
+    KGE_LAUNCH("lookup", KGE_CUDA(kge::launch_lookup(shards, (int)n, sizes, cfg_.score_fn, lookup_type(), stream_)));
 }
 
 void Engine::launch_lookup_bwd(unsigned l0, unsigned n, unsigned step) {
@@ -1611,7 +1604,7 @@ void Engine::launch_lookup_bwd(unsigned l0, unsigned n, unsigned step) {
         const ShardBuffers& b = shards_[l0 + i];
         shards.s[i] = LookupBwdArgs{lookup_rows(l0 + i, step), d_relation_ + ((size_t)(l0 + i) * cfg_.n_step + step) * B, b.d_pred, b.d_head, b.d_relrow, b.nrm, b.d_nrm, b.d_normrow};
     }
-    KGE_LAUNCH_SHARDS("lookup_bwd", n, KGE_CUDA(kge::launch_lookup_bwd(shards, (int)n, dense_, dense_ + dense_bounds_[3], (int)B, (int)cfg_.d, cfg_.score_fn, lookup_type(), stream_)));
+    KGE_LAUNCH("lookup_bwd", KGE_CUDA(kge::launch_lookup_bwd(shards, (int)n, dense_, dense_ + dense_bounds_[3], (int)B, (int)cfg_.d, cfg_.score_fn, lookup_type(), stream_)));
 }
 
 ShardArgs<TranshScoreArgs> Engine::transh_scores(unsigned l0, unsigned n) const {
@@ -1766,7 +1759,7 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
             }
             const tc::Routing routing{routes, (int)n, (int)n_nets, {n_nets == 2 ? 1 : 3, 2}};
             launch_planes("hidden", problems, (int)(n * n_nets), tc::SIDE_NONE, XCHG_DENSE_PARAMS, fused_route && !heavy_route ? XCHG_TAILS : -1,
-                          fused_route ? &routing : nullptr, n);
+                          fused_route ? &routing : nullptr);
         } else {
             launch_exchange_wait(XCHG_DENSE_PARAMS);
         }
@@ -1796,7 +1789,7 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
         const unsigned n = std::min(group_, n_local_ - l0);
         // 2. scores
         if (transh) {
-            KGE_LAUNCH_SHARDS("score", n, KGE_CUDA(launch_transh_score(transh_scores(l0, n), (int)n, (int)B, (int)T, (int)D, (int)ld, sync, stream_)));
+            KGE_LAUNCH("score", KGE_CUDA(launch_transh_score(transh_scores(l0, n), (int)n, (int)B, (int)T, (int)D, (int)ld, sync, stream_)));
         } else if (dot || (l2 && cfg_.l2_contraction)) {
             // (the L2 distance as |p|^2 + |t|^2 - 2 p.t, in the direct form where that cancels)
             for (unsigned i = 0; i < n; ++i) {
@@ -1809,11 +1802,11 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                 p.g.epilogue = dot ? tc::EPI_STORE : tc::EPI_L2_DISTANCE;
                 p.g.out = b.raw; p.g.ldc = ld; p.g.block_rows = 1;
             }
-            launch_planes("score", problems, (int)n, dot ? tc::SIDE_NONE : tc::SIDE_NORMS, XCHG_TAILS, -1, nullptr, n);
+            launch_planes("score", problems, (int)n, dot ? tc::SIDE_NONE : tc::SIDE_NORMS, XCHG_TAILS, -1);
         } else {
             ShardArgs<ScoreArgs> shards{};
             for (unsigned i = 0; i < n; ++i) shards.s[i] = ScoreArgs{shards_[l0 + i].pred, shards_[l0 + i].tails, shards_[l0 + i].raw};
-            KGE_LAUNCH_SHARDS("score", n, KGE_CUDA(launch_score(cfg_.dist_fn, shards, (int)n, (int)B, (int)T, (int)D, (int)ld, stream_, sync)));
+            KGE_LAUNCH("score", KGE_CUDA(launch_score(cfg_.dist_fn, shards, (int)n, (int)B, (int)T, (int)D, (int)ld, stream_, sync)));
         }
         // 3. loss and the coefficients of the score gradients (the rows' loss terms are added up by a block of the entity update, off the chain)
         ShardArgs<LossArgs> loss{};
@@ -1821,10 +1814,10 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
             const ShardBuffers& b = shards_[l0 + i];
             loss.s[i] = LossArgs{b.raw, step_ptr(d_tail_, l0 + i, B), b.coeff, dot || l2 ? b.coeff_lo : nullptr, b.loss_rows, nullptr, nullptr, nullptr, nullptr};
         }
-        KGE_LAUNCH_SHARDS("loss", n, KGE_CUDA(launch_loss(loss, (int)n, lp, 1.0f / normaliser, bf16 ? 1 : 0, (int)B, stream_)));
+        KGE_LAUNCH("loss", KGE_CUDA(launch_loss(loss, (int)n, lp, 1.0f / normaliser, bf16 ? 1 : 0, (int)B, stream_)));
         // 4. score gradients; the tails' rows go straight to the shards that own them
         if (transh) {
-            KGE_LAUNCH_SHARDS("score_bwd", n, KGE_CUDA(launch_transh_bwd(transh_gradients(l0, n), (int)n, stream_)));
+            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_transh_bwd(transh_gradients(l0, n), (int)n, stream_)));
             launch_exchange_signal(XCHG_TAIL_GRADS);
         } else if (!dot && !l2) {
             ShardArgs<PairBwdArgs> shards{};
@@ -1835,7 +1828,7 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                 pa.p[0] = {b.pred, b.tails, b.coeff, (int)B, (int)T, (int)ld, 1, b.d_pred, nullptr, 1};
                 pa.p[1] = {b.tails, b.pred, b.coeff, (int)T, (int)B, 1, (int)ld, nullptr, b.grad_dst, (int)cfg_.a2a_size};
             }
-            KGE_LAUNCH_SHARDS("score_bwd", n, KGE_CUDA(launch_pair_bwd(DIST_L1, shards, (int)n, stream_)));
+            KGE_LAUNCH("score_bwd", KGE_CUDA(launch_pair_bwd(DIST_L1, shards, (int)n, stream_)));
             launch_exchange_signal(XCHG_TAIL_GRADS);
         } else {
             //   dot:  d_pred = C . tails,                          d_tails = C^T . pred
@@ -1857,7 +1850,7 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                 h.g.out = nullptr; h.g.out_blocks = b.grad_dst; h.g.block_rows = (int)cfg_.a2a_size; h.g.ldc = D;
                 h.g.x_base = reinterpret_cast<const uint8_t*>(b.tails); h.g.x_row_stride_bytes = (long long)D * 4;
             }
-            launch_planes("score_bwd", problems, (int)(2 * n), l2 ? tc::SIDE_ROWSUM : tc::SIDE_NONE, -1, XCHG_TAIL_GRADS, nullptr, n);
+            launch_planes("score_bwd", problems, (int)(2 * n), l2 ? tc::SIDE_ROWSUM : tc::SIDE_NONE, -1, XCHG_TAIL_GRADS);
         }
         if (cfg_.score_fn != SCORE_TRANSE) launch_lookup_bwd(l0, n, step);
     }
@@ -1881,7 +1874,7 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
             if (direct_rows_) return launch_entity_update<ST, 4, false, true>(shards, es, stream_);
             return launch_entity_update<ST, 4>(shards, es, stream_);
         };
-        KGE_LAUNCH_SHARDS("entity_update", n, KGE_CUDA(cfg_.state_type == ST_F32 ? update(float{}) : update(__half{})));
+        KGE_LAUNCH("entity_update", KGE_CUDA(cfg_.state_type == ST_F32 ? update(float{}) : update(__half{})));
         if (gather_beside) launch_gather(step + 1, l0, n, side_begin());
     }
     KGE_CUDA(cudaGetLastError());
@@ -1913,7 +1906,7 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                 }
             }
         }
-        if (F > 0) launch_planes("projection_bwd", problems, (int)(n_problems * n_nets), tc::SIDE_NONE, -1, XCHG_DENSE_PARTIALS, nullptr, n);
+        if (F > 0) launch_planes("projection_bwd", problems, (int)(n_problems * n_nets), tc::SIDE_NONE, -1, XCHG_DENSE_PARTIALS);
         else launch_exchange_signal(XCHG_DENSE_PARTIALS);  // the relation rows of the entity update are all there is
     }
     KGE_CUDA(cudaGetLastError());

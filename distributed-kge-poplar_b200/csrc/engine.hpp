@@ -188,7 +188,7 @@ class Engine {
                    int wait_kind = -1, int signal_kind = -1);
     // the plane-fed contraction: tile width and k splits chosen here
     void launch_planes(const char* name, tc::PlaneProblem* problems, int n_problems, int side, int wait_kind, int signal_kind,
-                       const tc::Routing* routing = nullptr, unsigned n_shards = 1);
+                       const tc::Routing* routing = nullptr);
     void launch_step_planes(unsigned step, const LossParams& lp, float normaliser);
     void refresh_lower_plane(size_t offset, size_t count);
     LookupRows lookup_rows(unsigned l, unsigned step) const;

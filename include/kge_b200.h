@@ -143,8 +143,7 @@ int kge_stage_batch(kge_engine* engine, const kge_array* arrays, size_t n_arrays
 int kge_train_staged(kge_engine* engine, float learning_rate, float* loss);
 
 /* Device time of the last kge_train_staged / "train_step_loop" run, from CUDA events on the
- * engine's stream, and the number of kernels it launched (graph nodes when replayed as a graph; a launch that works on
- * several local shards counts as the one per shard that it stands for). */
+ * engine's stream, and the number of kernels it launched (graph nodes when replayed as a graph). */
 int kge_last_run_stats(kge_engine* engine, float* device_ms, unsigned long long* kernel_launches);
 
 /* Per-kernel device times.  While switched on, the step loop is launched kernel by kernel (not as
