@@ -7,6 +7,7 @@
 #include <cstring>
 #include <mutex>
 #include <optional>
+#include <utility>
 
 namespace kge {
 
@@ -1554,6 +1555,16 @@ void Engine::launch_dropout(unsigned l, unsigned step, const uint8_t* rows_c) {
                                                         (int)R, dropout_params(l, step))));
 }
 
+static tc::PlaneOperand plane_operand(const float* hi, const float* lo, long long stride_bytes, bool mn_major) {
+    return tc::PlaneOperand{hi, lo, stride_bytes, mn_major ? 1 : 0, 0};
+}
+// The gathered features of a step as an operand of its contractions.
+tc::PlaneOperand Engine::features(const ShardBuffers& b, unsigned step, bool mn_major) const {
+    const unsigned parity = step & 1;
+    if (cfg_.feature_type == ST_F16) return plane_operand(b.feat_wide2[parity], nullptr, (long long)feat_stride_ * 4, mn_major);
+    return plane_operand(reinterpret_cast<const float*>(b.rows_c2[parity] + layout_.off_feat), b.feat_lo2[parity], (long long)layout_.row_bytes, mn_major);
+}
+
 // What the lookups of local shard l read: the table's values, or the hidden rows.
 LookupRows Engine::lookup_rows(unsigned l, unsigned step) const {
     const ShardBuffers& b = shards_[l];
@@ -1708,16 +1719,8 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
     auto plane16 = [](const float* values, long long row_elems, bool mn_major) {
         return tc::PlaneOperand{values, nullptr, row_elems * 2, mn_major ? 1 : 0, 2};
     };
-    const bool half_features = cfg_.feature_type == ST_F16;
     const ExchangeSync sync = exchange_sync();
     auto step_ptr = [&](uint32_t* base, unsigned l, size_t per_step) { return base + ((size_t)l * cfg_.n_step + step) * per_step; };
-    auto plane = [](const float* hi, const float* lo, long long stride_bytes, bool mn_major) {
-        return tc::PlaneOperand{hi, lo, stride_bytes, mn_major ? 1 : 0, 0};
-    };
-    auto features = [&](const ShardBuffers& b, bool mn_major) {
-        if (half_features) return plane(b.feat_wide2[parity], nullptr, (long long)feat_stride_ * 4, mn_major);
-        return plane(reinterpret_cast<const float*>(b.rows_c2[parity] + layout_.off_feat), b.feat_lo2[parity], (long long)layout_.row_bytes, mn_major);
-    };
     tc::PlaneProblem problems[tc::kMaxPlaneProblems];
 
     // 1. hidden = value + feature . W, and (elementwise score functions) from its epilogue the lookups and the send half of the exchange
@@ -1735,8 +1738,8 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                     tc::PlaneProblem& p = problems[i * n_nets + net];
                     p = tc::PlaneProblem{};
                     const size_t w = dense_bounds_[1 + net];
-                    p.A = features(b, false);
-                    p.B = plane(dense_ + w, dense_lo_ + w, (long long)D * 4, true);
+                    p.A = features(b, step, false);
+                    p.B = plane_operand(dense_ + w, dense_lo_ + w, (long long)D * 4, true);
                     tc::GemmArgs& g = p.g;
                     g.M = (int)R; g.N = (int)D; g.K = (int)F;
                     g.epilogue = tc::EPI_ADD_TABLE_VALUE;
@@ -1796,8 +1799,8 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                 const ShardBuffers& b = shards_[l0 + i];
                 tc::PlaneProblem& p = problems[i];
                 p = tc::PlaneProblem{};
-                p.A = bf16 ? plane16(b.pred_lo, D, false) : plane(b.pred, b.pred_lo, (long long)D * 4, false);
-                p.B = bf16 ? plane16(b.tails_lo, D, false) : plane(b.tails, b.tails_lo, (long long)D * 4, false);
+                p.A = bf16 ? plane16(b.pred_lo, D, false) : plane_operand(b.pred, b.pred_lo, (long long)D * 4, false);
+                p.B = bf16 ? plane16(b.tails_lo, D, false) : plane_operand(b.tails, b.tails_lo, (long long)D * 4, false);
                 p.g.M = (int)B; p.g.N = (int)T; p.g.K = (int)D;
                 p.g.epilogue = dot ? tc::EPI_STORE : tc::EPI_L2_DISTANCE;
                 p.g.out = b.raw; p.g.ldc = ld; p.g.block_rows = 1;
@@ -1837,14 +1840,14 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
                 const ShardBuffers& b = shards_[l0 + i];
                 tc::PlaneProblem &g = problems[2 * i], &h = problems[2 * i + 1];
                 g = h = tc::PlaneProblem{};
-                g.A = bf16 ? plane16(b.coeff_lo, ld, false) : plane(b.coeff, b.coeff_lo, (long long)ld * 4, false);
-                g.B = bf16 ? plane16(b.tails_lo, D, true) : plane(b.tails, b.tails_lo, (long long)D * 4, true);
+                g.A = bf16 ? plane16(b.coeff_lo, ld, false) : plane_operand(b.coeff, b.coeff_lo, (long long)ld * 4, false);
+                g.B = bf16 ? plane16(b.tails_lo, D, true) : plane_operand(b.tails, b.tails_lo, (long long)D * 4, true);
                 g.g.M = (int)B; g.g.N = (int)D; g.g.K = (int)T;
                 g.g.epilogue = l2 ? tc::EPI_ROWSUM_X_MINUS : tc::EPI_STORE;
                 g.g.out = b.d_pred; g.g.ldc = D; g.g.block_rows = 1;
                 g.g.x_base = reinterpret_cast<const uint8_t*>(b.pred); g.g.x_row_stride_bytes = (long long)D * 4;
-                h.A = bf16 ? plane16(b.coeff_lo, ld, true) : plane(b.coeff, b.coeff_lo, (long long)ld * 4, true);
-                h.B = bf16 ? plane16(b.pred_lo, D, true) : plane(b.pred, b.pred_lo, (long long)D * 4, true);
+                h.A = bf16 ? plane16(b.coeff_lo, ld, true) : plane_operand(b.coeff, b.coeff_lo, (long long)ld * 4, true);
+                h.B = bf16 ? plane16(b.pred_lo, D, true) : plane_operand(b.pred, b.pred_lo, (long long)D * 4, true);
                 h.g.M = (int)T; h.g.N = (int)D; h.g.K = (int)B;
                 h.g.epilogue = g.g.epilogue;
                 h.g.out = nullptr; h.g.out_blocks = b.grad_dst; h.g.block_rows = (int)cfg_.a2a_size; h.g.ldc = D;
@@ -1883,30 +1886,8 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
     // slices of each shard's partial dense gradient
     const unsigned at_once = fuse_dense_ ? n_local_ : group_;
     for (unsigned l0 = 0; l0 < n_local_; l0 += at_once) {
-        const unsigned n = std::min(at_once, n_local_ - l0), n_problems = fuse_dense_ ? 1 : n;
-        for (unsigned i = 0; i < n_problems; ++i) {
-            const ShardBuffers& b = shards_[l0 + i];
-            for (unsigned net = 0; net < n_nets; ++net) {
-                tc::PlaneProblem& p = problems[i * n_nets + net];
-                p = tc::PlaneProblem{};
-                p.A = features(b, true);
-                p.B = plane(net ? b.d_hid_t : b.d_hid_h, net ? b.d_hid_t_lo : b.d_hid_h_lo, (long long)D * 4, true);
-                tc::GemmArgs& g = p.g;
-                g.M = (int)F; g.N = (int)D; g.K = (int)(fuse_dense_ ? n * R : R);  // (shard behind shard in memory)
-                g.block_row_offset = (int)(n_rel + net * F); g.block_rows = 1; g.ldc = D;
-                if (fuse_dense_) {
-                    g.epilogue = tc::EPI_DENSE_ADAM;
-                    g.x_base = reinterpret_cast<const uint8_t*>(dense_ + dense_bounds_[1 + net]);
-                    g.x_row_stride_bytes = (long long)D * 4;
-                    g.adam = tc::DenseAdamArgs{dense_, dense_lo_, dense_m_, dense_v_, d_step_size_ + step, dense_lr_mod_[1 + net], adam_.beta_m, adam_.beta_v,
-                                               adam_.one_minus_beta_m, adam_.one_minus_beta_v, adam_.epsilon, adam_.weight_decay};
-                } else {
-                    g.epilogue = tc::EPI_STORE;
-                    g.out_blocks = b.dense_dst; g.block_cyclic = (int)cfg_.world;
-                }
-            }
-        }
-        if (F > 0) launch_planes("projection_bwd", problems, (int)(n_problems * n_nets), tc::SIDE_NONE, -1, XCHG_DENSE_PARTIALS);
+        const unsigned n = std::min(at_once, n_local_ - l0);
+        if (F > 0) launch_projection_bwd(l0, n, step, fuse_dense_);
         else launch_exchange_signal(XCHG_DENSE_PARTIALS);  // the relation rows of the entity update are all there is
     }
     KGE_CUDA(cudaGetLastError());
@@ -1915,6 +1896,57 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
     if (!fuse_dense_) launch_dense_update(step);
     KGE_CUDA(cudaGetLastError());
     if (gather_beside) side_join(1);
+}
+
+// d W = feature^T . d_hidden of local shards l0 .. l0 + n - 1.  `update`: one contraction over the rows of all of them (shard
+// behind shard in memory), which ends in the projection's Adam step; else each shard's goes to the owners' slices of its
+// partial dense gradient.
+void Engine::launch_projection_bwd(unsigned l0, unsigned n, unsigned step, bool update) {
+    const unsigned R = cfg_.n_remote(), D = cfg_.d, F = cfg_.f, n_nets = cfg_.n_net(), n_problems = update ? 1 : n;
+    tc::PlaneProblem problems[tc::kMaxPlaneProblems];
+    for (unsigned i = 0; i < n_problems; ++i) {
+        const ShardBuffers& b = shards_[l0 + i];
+        for (unsigned net = 0; net < n_nets; ++net) {
+            tc::PlaneProblem& p = problems[i * n_nets + net];
+            p = tc::PlaneProblem{};
+            p.A = features(b, step, true);
+            p.B = plane_operand(net ? b.d_hid_t : b.d_hid_h, net ? b.d_hid_t_lo : b.d_hid_h_lo, (long long)D * 4, true);
+            tc::GemmArgs& g = p.g;
+            g.M = (int)F; g.N = (int)D; g.K = (int)(update ? n * R : R);
+            g.block_row_offset = (int)(cfg_.n_relation_type + net * F); g.block_rows = 1; g.ldc = D;
+            if (update) {
+                g.epilogue = tc::EPI_DENSE_ADAM;
+                g.x_base = reinterpret_cast<const uint8_t*>(dense_ + dense_bounds_[1 + net]);
+                g.x_row_stride_bytes = (long long)D * 4;
+                g.adam = tc::DenseAdamArgs{dense_, dense_lo_, dense_m_, dense_v_, d_step_size_ + step, dense_lr_mod_[1 + net], adam_.beta_m, adam_.beta_v,
+                                           adam_.one_minus_beta_m, adam_.one_minus_beta_v, adam_.epsilon, adam_.weight_decay};
+            } else {
+                g.epilogue = tc::EPI_STORE;
+                g.out_blocks = b.dense_dst; g.block_cyclic = (int)cfg_.world;
+            }
+        }
+    }
+    launch_planes("projection_bwd", problems, (int)(n_problems * n_nets), tc::SIDE_NONE, -1, XCHG_DENSE_PARTIALS);
+}
+
+// Where the dense Adam steps are taken by the kernels that produce the gradients, these are never stored: the last step's
+// partial dense gradient of local shard l, from what that step has left of its operands (kge_debug_fetch).
+void Engine::restore_dense_partial(unsigned l) {
+    if (!staged_ || stage_fresh_)
+        fail(KGE_INVALID_ARGUMENT, "kge_debug_fetch: 'dense_grad' is made from the index streams of the last run: there has been none, or a newly staged batch has replaced them");
+    ShardBuffers& b = shards_[l];
+    const unsigned step = cfg_.n_step - 1, n_rel = cfg_.n_relation_type;
+    const size_t sidx = (size_t)l * cfg_.n_step + step;
+    const float* per_triple[2] = {b.d_relrow, b.d_normrow};
+    struct Untimed {  // (these launches belong to no run)
+        bool &timing, before;
+        ~Untimed() { timing = before; }
+    } untimed{kernel_timing_, std::exchange(kernel_timing_, false)};
+    for (int table = 0; table < (cfg_.score_fn == SCORE_TRANSH ? 2 : 1); ++table)
+        KGE_CUDA(launch_dependent(k_dense_partial<4>, dim3(n_rel), dim3(64 * kRelationLanes), 0, stream_, per_triple[table], d_rel_perm_ + sidx * cfg_.batch_size,
+                                  d_rel_off_ + sidx * (n_rel + 1), (int)n_rel, (int)cfg_.d, b.proj_partial, 0, 1, proj_elems_, b.dense_dst, (int)cfg_.world,
+                                  exchange_sync(), -1, table ? (int)(dense_bounds_[3] / cfg_.d) : 0));
+    if (cfg_.f) launch_projection_bwd(l, 1, step, false);
 }
 
 // Dense parameters: every process, also one that owns nothing, launches it, since the kernel carries two hand-overs.
@@ -2803,6 +2835,7 @@ size_t Engine::debug_fetch(const std::string& what, size_t shard, float* out, si
     else if (what == "grad_recv") { src = b.grad_recv; count = T * D; }
     else if (what == "dense_grad") {
         if (cfg_.world > 1) fail(KGE_INVALID_ARGUMENT, "kge_debug_fetch: 'dense_grad' is spread over the processes; fetch it with one process");
+        if (fuse_dense_ && n_dense_ <= capacity) restore_dense_partial((unsigned)shard);
         src = b.dense_partial; count = n_dense_;
     }
     else if (what == "loss_last") { src = d_loss_last_ + shard; count = 1; }

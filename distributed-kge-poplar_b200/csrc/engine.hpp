@@ -190,6 +190,9 @@ class Engine {
     void launch_planes(const char* name, tc::PlaneProblem* problems, int n_problems, int side, int wait_kind, int signal_kind,
                        const tc::Routing* routing = nullptr);
     void launch_step_planes(unsigned step, const LossParams& lp, float normaliser);
+    tc::PlaneOperand features(const ShardBuffers& b, unsigned step, bool mn_major) const;
+    void launch_projection_bwd(unsigned l0, unsigned n, unsigned step, bool update);
+    void restore_dense_partial(unsigned l);
     void refresh_lower_plane(size_t offset, size_t count);
     LookupRows lookup_rows(unsigned l, unsigned step) const;
     int lookup_type() const;

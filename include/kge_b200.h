@@ -157,6 +157,8 @@ int kge_kernel_time(kge_engine* engine, size_t index, const char** name, float* 
 
 /* Copies an intermediate of the last training step of local shard `shard` to the host, for
  * tests: "hidden", "tails", "pred", "raw_score", "coeff", "d_pred", "d_hidden", "dense_grad".
+ * "dense_grad" is the shard's part of the dense parameters' gradient, with one process; where no kernel
+ * stores it, it is made from the run's index streams, and refused once another batch is staged.
  * `capacity` is in floats; `*count` receives the number written. */
 int kge_debug_fetch(kge_engine* engine, const char* what, size_t shard, float* out, size_t capacity,
                     size_t* count);

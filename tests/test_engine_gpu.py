@@ -182,6 +182,50 @@ def _compare_state(engine, cfg, oracle, what, RTOL=RTOL, rel_rtol=None):
             assert_close(got[key], want[key], tol, f"{what}: {key}")
 
 
+def _check_dense_grad(engine, cfg, grads, what, rtol, rel_rtol=None):
+    """The shards' partial dense gradients add up to the oracle's, parameter by parameter in the dense vector's order."""
+    D, F, M = cfg.embedding_size, cfg.entity_feature_size, cfg.feature_mlp_size
+    got = np.sum([engine.debug_fetch("dense_grad", s, 1 << 24).astype(np.float64) for s in range(cfg.n_shard)], axis=0)
+    shapes = [("relation_embedding", (cfg.n_relation_type, D))]
+    shapes += [(name, (F, D)) for name in cfg.projection_names if F]
+    shapes += [("relation_normal", (cfg.n_relation_type, D))] if cfg.score_fn == "TransH" else []
+    for name in cfg.projection_names if F and M else []:
+        prefix = name[: -len("feature_projection")]
+        shapes += [(prefix + "mlp_up_projection", (2 * D, M)), (prefix + "mlp_down_projection", (M, D))]
+    assert got.size == sum(a * b for _, (a, b) in shapes)
+    for name, shape in shapes:
+        part, got = got[: shape[0] * shape[1]].reshape(shape), got[shape[0] * shape[1] :]
+        want = grads[name]
+        # (a RotatE relation has half as many angles as columns)
+        assert_close(part[:, : want.shape[1]], want, rel_rtol if rel_rtol and name == "relation_embedding" else rtol, f"{what}: gradient of {name}")
+
+
+@pytest.mark.parametrize("fused", ["1", "0"])
+def test_dense_gradients_of_the_last_step(monkeypatch, fused):
+    """Fetched where the kernels that make them take the Adam step themselves, and where another kernel does; refused
+    where there is nothing to fetch them from."""
+    monkeypatch.setenv("KGE_FUSE_DENSE_UPDATE", fused)
+    case = CASES["transe_l2_softmax_features"]
+    cfg, state, engine, batch = _build(case, n_step=3, warm=True, pad=2)
+    if fused == "1":
+        with pytest.raises(ValueError, match="last run"):
+            engine.debug_fetch("dense_grad", 0, 1 << 24)
+    oracle = make_oracle(cfg, state)
+    for run in range(2):
+        oracle.train_step_loop(1e-3, batch)
+        _run_engine(engine, cfg, batch, 1e-3)
+    before = read_state(engine, cfg, RW, cfg.n_shard)
+    _check_dense_grad(engine, cfg, oracle.last["grads"], "six steps", 1e-4)
+    after = read_state(engine, cfg, RW, cfg.n_shard)
+    for key in before:
+        np.testing.assert_array_equal(before[key], after[key])
+    engine.stage_batch(batch)
+    if fused == "1":
+        with pytest.raises(ValueError, match="newly staged"):
+            engine.debug_fetch("dense_grad", 0, 1 << 24)
+    engine.close()
+
+
 @pytest.mark.parametrize("name", sorted(CASES))
 @pytest.mark.parametrize("warm", [False, True], ids=["cold", "warm"])
 @pytest.mark.parametrize("tensor_cores", [True, False], ids=["tcgen05", "fp32pipe"])
@@ -218,10 +262,7 @@ def test_single_step_matches_oracle(name, warm, tensor_cores):
         d_hidden = engine.debug_fetch("d_hidden", s, R * D).reshape(R, D)
         if cfg.share_feature_networks or cfg.entity_feature_size == 0:
             assert_close(d_hidden, last["d_feature_hidden"][s], RTOL, f"{name}: d hidden[{s}]")
-    dense = engine.debug_fetch("dense_grad", 0, 1 << 24)
-    n_rel = cfg.n_relation_type * D
-    n_net = len(cfg.projection_names) * (cfg.entity_feature_size > 0)
-    assert dense.size == n_rel * (2 if cfg.score_fn == "TransH" else 1) + n_net * (cfg.entity_feature_size + 3 * cfg.feature_mlp_size) * D
+    _check_dense_grad(engine, cfg, last["grads"], name, RTOL, case.get("rel_rtol"))
     _compare_state(engine, cfg, oracle, name, RTOL, case.get("rel_rtol"))
     engine.close()
 
