@@ -1089,8 +1089,8 @@ __device__ __forceinline__ void stage_rows(float* dst, const float* __restrict__
 }
 __device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void stage_wait_previous() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-// Columns k and k + 1 of a row, zeros past the end.
-__device__ __forceinline__ f32x2 load_pair(const float* __restrict__ row, int k, int D) { return pack2(k < D ? row[k] : 0.f, k + 1 < D ? row[k + 1] : 0.f); }
+// Columns k and k + 1 of a row, ones past its end.
+__device__ __forceinline__ f32x2 load_pair(const float* __restrict__ row, int k, int D) { return pack2(k < D ? row[k] : 1.f, k + 1 < D ? row[k + 1] : 1.f); }
 __device__ __forceinline__ void store_pair(float* __restrict__ row, int k, int D, f32x2 v) {
     const float2 f = unpack2(v);
     if (k + 1 < D && (D & 1) == 0) {
@@ -1140,8 +1140,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, 2) k_pair_bwd(const __grid_co
     f32x2 x[ROWS], acc[ROWS];
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
-        // (1 where there is no value: its difference to the zeros staged there is not 0)
-        x[r] = m + r < M && k < D ? load_pair(pr.X + (size_t)(m + r) * D, k, D) : 0x3f8000003f800000ull;
+        // (1 where there is no value, the second of an odd row's last lane too: its difference to the zeros staged there is not 0)
+        x[r] = m + r < M ? load_pair(pr.X + (size_t)(m + r) * D, k, D) : 0x3f8000003f800000ull;
         acc[r] = 0ull;
     }
     stage(0, smem[0]);

@@ -83,6 +83,27 @@ def test_separate_networks_of_four_shards():
     _two_runs(_config("TransE", "L2", n_shard=4, batch_size=12, a2a_size=7, embedding_size=36, entity_feature_size=12, share_feature_networks=False), seed=9, rtol=1e-4)
 
 
+def test_odd_widths_count_no_ties():
+    """L1 gradients add a chunk up again where a difference is 0, which the missing neighbour of an odd row's last column must not
+    look like: 63 columns take as long as 62, whose blocks and copies are the same, and not as long as all chunks twice."""
+    def us_per_step(d):
+        cfg = _config("TransE", "L1", n_entity=2000, embedding_size=d, batch_size=512, a2a_size=768)
+        engine = capi.CEngine(engine_settings(cfg, n_step=20, rw_batch=RW))
+        write_state(engine, cfg, random_state(cfg, 1), RW)
+        run = dict(learning_rate=np.full(1, 1e-3, np.float32), loss=np.zeros(1, np.float32), **random_batch(cfg, 20, 2))
+        times = []
+        for _ in range(6):
+            engine.set_kernel_timing(True)
+            engine.run("train_step_loop", run)
+            ms, launches = engine.kernel_times()["score_bwd"]
+            times.append(1e3 * ms / launches)
+        engine.close()
+        return min(times[1:])
+
+    odd, even = us_per_step(63), us_per_step(62)
+    assert odd < 1.2 * even, f"{odd:.1f} us for 63 columns, {even:.1f} us for 62"
+
+
 @pytest.mark.parametrize("fn", [capi.L1, capi.L2, capi.DOT], ids=["l1", "l2", "dot"])
 @pytest.mark.parametrize("shape", [(1, 1, 4), (64, 33, 128), (65, 49, 132), (130, 700, 260), (200, 1500, 288), (64, 64, 516)])
 def test_scores_in_blocks(fn, shape):
