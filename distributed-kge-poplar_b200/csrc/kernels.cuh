@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "exchange.cuh"
 #include "pdl.cuh"
@@ -616,7 +617,7 @@ k_score_block(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T,
 
 template <int FN, int NB, bool WIDE>
 inline cudaError_t launch_score_block(const ShardArgs<ScoreArgs>& shards, int n_shards, int B, int T, int D, int ld, cudaStream_t stream, const ExchangeSync& sync) {
-    static bool configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
+    static std::atomic<bool> configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
     const int slot = current_device_slot();
     if (slot < 0 || !configured[slot]) {
         const cudaError_t err = cudaFuncSetAttribute(k_score_block<FN, NB, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreBlockSmem<NB>);
@@ -744,7 +745,7 @@ k_score_tile(const __grid_constant__ ShardArgs<ScoreArgs> shards, int B, int T, 
 
 template <int FN, int NB>
 inline cudaError_t launch_score_tile(const ShardArgs<ScoreArgs>& shards, dim3 tiles, int B, int T, int D, int ld, cudaStream_t stream) {
-    static bool configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
+    static std::atomic<bool> configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
     const int slot = current_device_slot();
     if (slot < 0 || !configured[slot]) {
         const cudaError_t err = cudaFuncSetAttribute(k_score_tile<FN, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScoreTileSmem<NB>);

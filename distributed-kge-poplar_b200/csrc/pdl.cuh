@@ -14,8 +14,10 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 
 namespace kge {
 
@@ -81,27 +83,28 @@ inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 b
 constexpr int kSmCount = 148;
 template <auto Kernel, typename... Args>
 inline cudaError_t launch_spread(dim3 grid, dim3 block, cudaStream_t stream, Args&&... args) {
-    struct Info {
-        int natural, static_bytes;  // blocks of an SM without the unused memory; natural 0: not asked yet
-    };
-    static Info known[kMaxDeviceOrdinals] = {};
+    // The blocks of an SM without the unused memory (high half, 0: not asked yet) and a block's static memory, in one word:
+    // engines on several threads ask and answer here.
+    static std::atomic<uint64_t> known[kMaxDeviceOrdinals] = {};
     const int slot = current_device_slot();
-    Info info = slot >= 0 ? known[slot] : Info{};
-    if (info.natural == 0) {
+    uint64_t answer = slot >= 0 ? known[slot].load() : 0;
+    if (answer == 0) {
         cudaFuncAttributes attributes;
+        int blocks = 0;
         cudaError_t err = cudaFuncGetAttributes(&attributes, Kernel);
         if (err == cudaSuccess) err = cudaFuncSetAttribute(Kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-        info.static_bytes = (int)attributes.sharedSizeBytes;
-        if (err == cudaSuccess) err = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - info.static_bytes);
-        if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&info.natural, Kernel, (int)(block.x * block.y * block.z), 0);
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)attributes.sharedSizeBytes);
+        if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, Kernel, (int)(block.x * block.y * block.z), 0);
         if (err != cudaSuccess) return err;
-        if (slot >= 0) known[slot] = info;
+        answer = (uint64_t)blocks << 32 | (uint32_t)attributes.sharedSizeBytes;
+        if (slot >= 0) known[slot].store(answer);
     }
+    const int natural = (int)(answer >> 32), static_bytes = (int)(uint32_t)answer;
     const int share = (int)(((long long)grid.x * grid.y * grid.z + kSmCount - 1) / kSmCount);
     // a block takes its memory and 1 KB of the SM's 228: so much that share + 1 blocks do not fit
     int unused = 0;
-    if (share < info.natural) unused = std::min(228 * 1024 / (share + 1) + 128, 228 * 1024 / share) - 1024 - info.static_bytes;
-    unused = std::max(0, std::min(unused, 227 * 1024 - info.static_bytes)) / 128 * 128;
+    if (share < natural) unused = std::min(228 * 1024 / (share + 1) + 128, 228 * 1024 / share) - 1024 - static_bytes;
+    unused = std::max(0, std::min(unused, 227 * 1024 - static_bytes)) / 128 * 128;
     return launch_dependent(Kernel, grid, block, (size_t)unused, stream, static_cast<Args&&>(args)...);
 }
 

@@ -1061,7 +1061,7 @@ static __global__ void __launch_bounds__(256) k_tc_reduce(const __grid_constant_
 // Host side: grid = (ceil(M / 128), ceil(N / BN), splits).
 template <int BN, bool A_EXACT, bool ROWSUM>
 inline cudaError_t launch(const GemmArgs& g, int splits, cudaStream_t stream) {
-    static bool configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
+    static std::atomic<bool> configured[kMaxDeviceOrdinals] = {};  // one attribute call per instantiation and device is enough
     const int slot = current_device_slot();
     auto kernel = k_tc_gemm<BN, A_EXACT, ROWSUM>;
     if (slot < 0 || !configured[slot]) {
@@ -1172,7 +1172,7 @@ inline cudaError_t launch_pair(const GemmArgs* problems, int n_problems, int spl
         }
         return cudaSuccess;
     }
-    static bool configured[kMaxDeviceOrdinals] = {};
+    static std::atomic<bool> configured[kMaxDeviceOrdinals] = {};
     const int slot = current_device_slot();
     auto kernel = k_tc_gemm_async<BN, A_EXACT, ROWSUM>;
     if (slot < 0 || !configured[slot]) {

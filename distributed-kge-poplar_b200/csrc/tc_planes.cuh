@@ -1276,7 +1276,7 @@ inline bool planes_aligned(const PlaneOperand& op) {
 
 template <int BN, int SIDE, int EPI = -1, int SPLIT = 7, bool BF16 = false>
 inline cudaError_t configure_planes() {
-    static bool configured[kMaxDeviceOrdinals] = {};
+    static std::atomic<bool> configured[kMaxDeviceOrdinals] = {};
     const int slot = current_device_slot();
     if (slot >= 0 && configured[slot]) return cudaSuccess;
     cudaError_t err = cudaFuncSetAttribute(k_tc_planes<BN, SIDE, EPI, SPLIT, BF16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem_bytes());
@@ -1402,7 +1402,7 @@ inline bool mixed_splits_allowed(int side, int epilogue, int tile_n) {
 
 template <int EPI>
 inline cudaError_t launch_half(const PlaneLaunch& l, cudaStream_t stream) {
-    static bool configured[kMaxDeviceOrdinals] = {};
+    static std::atomic<bool> configured[kMaxDeviceOrdinals] = {};
     const int slot = current_device_slot();
     if (slot < 0 || !configured[slot]) {
         const cudaError_t err = cudaFuncSetAttribute(k_half_tiles<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)half_smem_bytes());
