@@ -2609,6 +2609,7 @@ void Engine::cmd_predict(std::vector<HostArray>& arrays) {
     HostArray& count = find_array(arrays, "predict_entity_count", KGE_U32, {n});
     HostArray& scores = find_array(arrays, "predict_scores", KGE_F32, {n, cfg_.n_shard, hr, nb});
     HostArray& indices = find_array(arrays, "predict_indices", KGE_U32, {n, cfg_.n_shard, hr, nb});
+    if (hr == 0) fail(KGE_INVALID_ARGUMENT, "'execution.predict_hr_batch_size' must be positive to rank queries");
     if (nb == 0 || nb > kTopkCapacity / 2)
         fail(KGE_INVALID_ARGUMENT, msg() << "'execution.predict_n_best' must be between 1 and " << kTopkCapacity / 2);
     if (!connected_) fail(KGE_LOGIC_ERROR, "world_size > 1 but kge_comm_connect has not been called");

@@ -101,9 +101,9 @@ inline cudaError_t launch_spread(dim3 grid, dim3 block, cudaStream_t stream, Arg
     }
     const int natural = (int)(answer >> 32), static_bytes = (int)(uint32_t)answer;
     const int share = (int)(((long long)grid.x * grid.y * grid.z + kSmCount - 1) / kSmCount);
-    // a block takes its memory and 1 KB of the SM's 228: so much that share + 1 blocks do not fit
+    // a block takes its memory and 1 KB of the SM's 228: so much that share + 1 blocks do not fit (an empty grid is CUDA's to refuse)
     int unused = 0;
-    if (share < natural) unused = std::min(228 * 1024 / (share + 1) + 128, 228 * 1024 / share) - 1024 - static_bytes;
+    if (share > 0 && share < natural) unused = std::min(228 * 1024 / (share + 1) + 128, 228 * 1024 / share) - 1024 - static_bytes;
     unused = std::max(0, std::min(unused, 227 * 1024 - static_bytes)) / 128 * 128;
     return launch_dependent(Kernel, grid, block, (size_t)unused, stream, static_cast<Args&&>(args)...);
 }

@@ -82,3 +82,8 @@ def test_spread_launches_on_several_threads(program):
     its share of the blocks and no more."""
     run = subprocess.run([program], capture_output=True, text=True)
     assert run.returncode == 0, run.stderr[-3000:]
+
+
+def test_a_launch_of_no_blocks_is_an_error_status(program):
+    run = subprocess.run([program, "empty"], capture_output=True, text=True)
+    assert run.returncode == 0, run

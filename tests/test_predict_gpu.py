@@ -302,3 +302,17 @@ def test_whole_table_transfers_equal_chunked_ones(n_shard, n_entity, d, f, rw, d
     np.testing.assert_array_equal(got, want)
     np.testing.assert_array_equal(got[:, 1:, 3 * d :], features[:, 1:].astype(dtype))
     assert np.any(got[..., :d]) and not np.any(got[..., d : 3 * d])
+
+
+@pytest.mark.parametrize("score_fn,distance_fn,features", [("TransE", "L1", 0), ("TransE", "L2", 4)])
+def test_ranking_without_queries_is_refused(score_fn, distance_fn, features):
+    """No room for queries: an error before any launch, not the end of the process."""
+    cfg = StepConfig(n_shard=1, n_entity=40, n_relation_type=4, embedding_size=8, entity_feature_size=features, batch_size=4, a2a_size=3,
+                     score_fn=score_fn, distance_fn=distance_fn, gamma=4.0)
+    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW, **{"execution.predict_hr_batch_size": 0}))
+    write_state(engine, cfg, random_state(cfg, 1), RW)
+    with pytest.raises(ValueError, match="predict_hr_batch_size"):
+        engine.run("predict", dict(predict_head=np.zeros((1, 0), np.uint32), predict_relation=np.zeros((1, 0), np.uint32),
+                                   predict_entity_count=np.full(1, 39, np.uint32), predict_scores=np.zeros((1, 1, 0, 5), np.float32),
+                                   predict_indices=np.zeros((1, 1, 0, 5), np.uint32)))
+    engine.close()
