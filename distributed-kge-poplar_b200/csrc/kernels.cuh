@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "adam.cuh"
 #include "exchange.cuh"
 #include "pdl.cuh"
 
@@ -57,19 +58,6 @@ struct RowLayout {
     // embeddings with fp32 optimiser state; the reference has one type per row, src/poplar_kge.cpp:405-417)
     uint32_t value_bf16;
 };
-
-struct AdamParams {
-    float beta_m;
-    float beta_v;
-    float one_minus_beta_m;
-    float one_minus_beta_v;
-    float epsilon;
-    float weight_decay;
-};
-// a x + b y with the first product unrounded.  Which one the addition takes in is the compiler's choice in every kernel anew
-// unless it is written out, and an L1 model, whose gradients are what rounding leaves of a sum, carries a last bit on: rows
-// and dense parameters have one form each in all kernels.
-__device__ __forceinline__ float weighted_sum(float a, float x, float b, float y) { return __fmaf_rn(a, x, __fmul_rn(b, y)); }
 
 __device__ __forceinline__ float load_as_float(const float* p) { return *p; }
 __device__ __forceinline__ float load_as_float(const __half* p) { return __half2float(*p); }

@@ -139,9 +139,8 @@ k_row_adam(uint8_t* __restrict__ table, const uint8_t* __restrict__ rows_c, RowL
         float m = load_as_float(reinterpret_cast<const ST*>(src + L.off_m) + c);
         const float q = load_as_float(reinterpret_cast<const ST*>(src + L.off_q) + c);
         const float g = grad[idx];
-        float v = q * q;
-        m = ap.beta_m * m + ap.one_minus_beta_m * g;
-        v = ap.beta_v * v + ap.one_minus_beta_v * g * g;
+        const float v = weighted_sum(__fmul_rn(ap.one_minus_beta_v, g), g, ap.beta_v, __fmul_rn(q, q));
+        m = weighted_sum(ap.one_minus_beta_m, g, ap.beta_m, m);
         x = x - alpha * (m / (sqrtf(v) + ap.epsilon) + ap.weight_decay * x);
         store_value<ST>(L, dst, c, x);
         store_from_float(reinterpret_cast<ST*>(dst + L.off_m) + c, m);

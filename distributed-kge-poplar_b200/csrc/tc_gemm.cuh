@@ -32,6 +32,7 @@
 
 #include <atomic>
 
+#include "adam.cuh"
 #include "exchange.cuh"
 #include "pdl.cuh"
 
@@ -650,8 +651,8 @@ __device__ __forceinline__ void finish_four(const GemmArgs& g, float* out_base, 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float grad = acc[j];
-            mo[j] = a.beta_m * mo[j] + a.one_minus_beta_m * grad;
-            ve[j] = a.beta_v * ve[j] + a.one_minus_beta_v * grad * grad;
+            mo[j] = weighted_sum(a.beta_m, mo[j], a.one_minus_beta_m, grad);
+            ve[j] = weighted_sum(a.beta_v, ve[j], __fmul_rn(a.one_minus_beta_v, grad), grad);
             w[j] = x[j] - alpha * (mo[j] / (sqrtf(ve[j]) + a.epsilon) + a.weight_decay * x[j]);
             const float hi = __uint_as_float(__float_as_uint(w[j]) & 0xffffe000u);
             lo[j] = __uint_as_float(__float_as_uint(w[j] - hi) & 0xffffe000u);

@@ -187,28 +187,72 @@ def test_ranked_queries_straight_from_the_table(score_fn, distance_fn, d, dtype)
     np.testing.assert_array_equal(got_idx[clear], want_idx[clear])
 
 
-@pytest.mark.parametrize("d,features", [(6, 0), (16, 0), (16, 12)], ids=["odd rows", "table rows", "gathered rows"])
-def test_row_moments_round_alike(d, features):
+def _product_plus(a, x, y):
+    """a x + y in float32 with one rounding, as an FMA gives it: the product is exact in float64, the sum is rounded to odd there,
+    which float32's rounding of it cannot be misled by."""
+    p, y = np.float64(a) * np.asarray(x, np.float64), np.asarray(y, np.float64)
+    total = p + y
+    back = total - p
+    error = (p - (total - back)) + (y - back)
+    even = (total.view(np.int64) & 1) == 0
+    return np.where((error != 0) & even, np.nextafter(total, np.where(error > 0, np.inf, -np.inf)), total).astype(np.float32)
+
+
+def _product(a, b):
+    return np.float32(a) * np.float32(b)
+
+
+@pytest.mark.parametrize("d,features,mlp", [(6, 0, 0), (16, 0, 0), (16, 12, 0), (16, 12, 8)], ids=["odd rows", "table rows", "gathered rows", "mlp"])
+def test_row_moments_round_alike(d, features, mlp):
     """Every form of the row update rounds the moments' old part and not the gradient's: the bits of that sum."""
-    cfg = _config("TransE", "L1", embedding_size=d, entity_feature_size=features, loss_type="softmax", correction_weight=1.0)
+    cfg = _config("TransE", "L1", embedding_size=d, entity_feature_size=features, feature_mlp_size=mlp, loss_type="softmax", correction_weight=1.0)
     state = random_state(cfg, d, warm=True)
-    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW))
-    write_state(engine, cfg, state, RW)
     batch = random_batch(cfg, 1, 3, pad=3)
-    engine.run("train_step_loop", dict(learning_rate=np.full(1, 1e-3, np.float32), loss=np.zeros(1, np.float32), **batch))
-    grad = engine.debug_fetch("d_hidden", 0, cfg.n_remote * d).reshape(-1, d)
-    got = read_rows(engine, cfg, RW, 1, np.float32)[0]
-    engine.close()
+
+    def step(cfg, state):
+        engine = capi.CEngine(engine_settings(cfg, rw_batch=RW))
+        write_state(engine, cfg, state, RW)
+        engine.run("train_step_loop", dict(learning_rate=np.full(1, 1e-3, np.float32), loss=np.zeros(1, np.float32), **batch))
+        out = engine.debug_fetch("d_hidden", 0, cfg.n_remote * d).reshape(-1, d), read_rows(engine, cfg, RW, 1, np.float32)[0]
+        engine.close()
+        return out
+
+    if mlp:  # with a last layer of zeros the hidden rows are the values and nothing passes back: the gradients of the model without features
+        state["mlp_down_projection"][:] = 0
+        bare = {k: v for k, v in state.items() if "projection" not in k}
+        grad, _ = step(_config("TransE", "L1", embedding_size=d, loss_type="softmax", correction_weight=1.0), dict(bare, entity_data=state["entity_data"][..., : 3 * d]))
+        _, got = step(cfg, state)
+    else:
+        grad, got = step(cfg, state)
     remote = batch["remote"][0, 0]
     rows, slots = np.unique(remote, return_index=True)
     rows, slots = rows[rows > 0], slots[rows > 0]
     g, old = grad[slots], state["entity_data"][0][rows]
-    mul = lambda a, b: np.float32(a) * np.float32(b)
-
-    def after(a, x, b, y):  # in 64 bits of mantissa: a x is exact, the sum rounded once more than in hardware, at 2^-40 odds
-        return (np.longdouble(a) * x.astype(np.longdouble) + mul(b, y)).astype(np.float32)
-
     one_m, one_v = np.float32(1) - np.float32(cfg.adam_beta_m), np.float32(1) - np.float32(cfg.adam_beta_v)
-    np.testing.assert_array_equal(got[rows, d : 2 * d], after(one_m, g, cfg.adam_beta_m, old[:, d : 2 * d]))
+    np.testing.assert_array_equal(got[rows, d : 2 * d], _product_plus(one_m, g, _product(cfg.adam_beta_m, old[:, d : 2 * d])))
     root = old[:, 2 * d : 3 * d]
-    np.testing.assert_array_equal(got[rows, 2 * d : 3 * d], np.sqrt(after(mul(one_v, g).astype(np.longdouble), g, cfg.adam_beta_v, mul(root, root))))
+    want_v = _product_plus(_product(one_v, g), g, _product(cfg.adam_beta_v, _product(root, root)))
+    np.testing.assert_array_equal(got[rows, 2 * d : 3 * d], np.sqrt(want_v))
+
+
+@pytest.mark.parametrize("form", ["fused", "of its own", "separate kernels"])
+def test_dense_moments_round_alike(monkeypatch, form):
+    """Every form of the dense update rounds the gradient's part of the moments and not the old one's: the bits of that sum, for
+    the projection (a contraction's epilogue or k_dense_update) and for the relations (the row update or k_dense_update)."""
+    monkeypatch.setenv("KGE_FUSE_DENSE_UPDATE", "1" if form == "fused" else "0")
+    d = 10 if form == "separate kernels" else 16
+    cfg = _config("TransE", "L2", embedding_size=d, entity_feature_size=12, n_relation_type=12, batch_size=8, loss_type="softmax", correction_weight=1.0)
+    state = random_state(cfg, d, warm=True)
+    engine = capi.CEngine(engine_settings(cfg, rw_batch=RW))
+    write_state(engine, cfg, state, RW)
+    batch = random_batch(cfg, 1, 3, pad=3)
+    batch["relation"][:] = np.arange(8)  # a triple per relation: no order of a sum to agree on
+    engine.run("train_step_loop", dict(learning_rate=np.full(1, 1e-3, np.float32), loss=np.zeros(1, np.float32), **batch))
+    grads = engine.debug_fetch("dense_grad", 0, 1 << 12)
+    got = read_state(engine, cfg, RW, 1)
+    engine.close()
+    one_m, one_v = np.float32(1) - np.float32(cfg.adam_beta_m), np.float32(1) - np.float32(cfg.adam_beta_v)
+    for name, g in (("relation_embedding", grads[: 12 * d].reshape(12, d)), ("feature_projection", grads[12 * d :].reshape(12, d))):
+        m, v = state[name + "/adam_m"], state[name + "/adam_v"]
+        np.testing.assert_array_equal(got[name + "/adam_m"], _product_plus(cfg.adam_beta_m, m, _product(one_m, g)), err_msg=name)
+        np.testing.assert_array_equal(got[name + "/adam_v"], _product_plus(cfg.adam_beta_v, v, _product(_product(one_v, g), g)), err_msg=name)
