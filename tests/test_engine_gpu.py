@@ -641,14 +641,15 @@ def test_bf16_values_with_float32_optimiser_state(name):
     engine.close()
 
 
-def test_engines_on_two_threads_capture_their_first_runs_side_by_side():
-    """Two engines with several shards record their first program runs at the same time, each with branches on streams
-    that a pool lends to both: the results are those of the same runs one after the other, bit for bit."""
+@pytest.mark.parametrize("name,tensor_cores", [("config1_transe_l1", True), ("config1_transe_l1", False), ("ragged_sizes", True), ("mlp_shared", True)])
+def test_engines_on_two_threads_capture_their_first_runs_side_by_side(name, tensor_cores):
+    """Two engines with several shards record their first program runs at the same time: the step of batched launches and (all
+    cases but the first) that of separate kernels, whose captures have branches on streams that a pool lends to both.  The
+    results are those of the same runs one after the other, bit for bit."""
     import threading
 
     def fresh(i):
-        case = CASES["config1_transe_l1"]
-        cfg, state, engine, batch = _build({**case, "seed": 40 + i}, n_step=6, warm=True, pad=2)
+        cfg, state, engine, batch = _build({**CASES[name], "seed": 40 + i}, n_step=6, warm=True, pad=2, tensor_cores=tensor_cores)
         return cfg, engine, batch
 
     want = []
