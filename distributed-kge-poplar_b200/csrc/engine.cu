@@ -1976,11 +1976,9 @@ void Engine::launch_one_step(unsigned step) {
     const unsigned n_rel = cfg_.n_relation_type;
     const bool two_nets = cfg_.n_net() == 2;
     const bool vec = (D % 4) == 0;
-    const float* rel_table = dense_;
     const float* W0 = cfg_.n_net() >= 1 ? dense_ + dense_bounds_[1] : nullptr;
     const float* W1 = two_nets ? dense_ + dense_bounds_[2] : W0;
     const bool transh = cfg_.score_fn == SCORE_TRANSH;
-    const float* normal_table = dense_ + dense_bounds_[3];
 
     LossParams lp{};
     lp.loss_fn = cfg_.loss_fn;

@@ -623,8 +623,9 @@ inline cudaError_t launch_score_block(const ShardArgs<ScoreArgs>& shards, int n_
 
 // The same scores where there are enough of them to fill the GPU with tiles (ranking): a block owns 64 x 128 outputs, its
 // 8 warps 32 x 32 each (or 64 x 96 and 32 x 24, where that ends sooner); all of them walk all of k in chunks of 32 staged one
-// ahead.  Each chunk is summed by itself and added to the total, as k_score_block adds its groups' chunks.  Bound by the FP32 pipe.  (With k_score_block's division of k
-// half the warps have nothing to do at 100 columns, and 1024 outputs a block pay for a reduction.)
+// ahead.  Each chunk is summed by itself and added to the total, as k_score_block adds its groups' chunks.  Bound by the FP32
+// pipe.  (With k_score_block's division of k half the warps have nothing to do at 100 columns, and 1024 outputs a block pay
+// for a reduction.)
 constexpr int kScoreTileP = 64;
 template <int NB>
 constexpr int kScoreTileStage = (kScoreTileP + 16 * NB) * kScoreStride;
@@ -1161,10 +1162,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 2) k_pair_bwd(const __grid_co
             } else {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    if (ROWS == 4) {
-                        const float4 q = load4(cs + (n + u) * kRows);
-                        c[0][u] = q.x; c[1 % ROWS][u] = q.y; c[2 % ROWS][u] = q.z; c[3 % ROWS][u] = q.w;
-                    } else if (ROWS == 2) {
+                    if (ROWS == 2) {
                         const float2 q = *reinterpret_cast<const float2*>(cs + (n + u) * kRows);
                         c[0][u] = q.x; c[1 % ROWS][u] = q.y;
                     } else {
@@ -2568,7 +2566,6 @@ k_topk_filter(const float* __restrict__ raw, int n_cols, uint32_t first_row, uin
     }
 }
 
-// One warp's list: up to kTopkCapacity keys in shared memory, sorted down to the n_best largest when it fills.
 // The lanes' keys in descending order.
 __device__ __forceinline__ unsigned long long lanes_sort_desc(unsigned long long key) {
     const int lane = threadIdx.x & 31;
@@ -2590,6 +2587,7 @@ static __device__ __noinline__ void topk_sort(unsigned long long* buf, int count
     warp_sort_desc(buf);
 }
 
+// One warp's list: up to kTopkCapacity keys in shared memory, sorted down to the n_best largest when it fills.
 struct TopkList {
     unsigned long long* buf;
     int count, n_best;
@@ -2708,10 +2706,9 @@ k_topk_seed(const float* __restrict__ raw, int n_cols, uint32_t first_row, uint3
     if (blockIdx.y == 0 && lane == 0) cand_count[q] = (int)gridDim.y * tp.n_best;
     if constexpr (FEW) {
         // Scores are held in registers, all of a tile read at the same time, and compared as floats: only what reaches the
-        // cut-off's score becomes a key, and the few keys that do are sorted a key per lane.  (With every score made a key
-        // twice, its reads waited for a few at a time, and a 256-key sort at the end, 128 queries x 40 000 scores took 58 us; 24
-        // this way; with 20 scores held
-        // instead of ten, which do not fit 64 registers, 36.)
+        // cut-off's score becomes a key, and the few keys that do are sorted a key per lane.  128 queries x 40 000 scores: 24 us.
+        // (58 with every score made a key twice, its reads waiting for a few at a time, and a 256-key sort at the end; 36 with
+        // 20 scores held instead of ten, which do not fit 64 registers.)
         constexpr int kHold = 10;
         const int valid = (int)min((long long)end, (long long)last_valid_row - (long long)first_row + 1);
         int count = 0;

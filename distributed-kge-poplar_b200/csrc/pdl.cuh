@@ -7,6 +7,9 @@
 // runs.  The kernel then calls grid_dependency_sync() before it touches global memory: that waits
 // for the predecessor to complete with its writes visible, and then lets this kernel's own
 // successor begin to launch, so at most one successor is resident and waiting at any time.
+// Before that call a kernel may read what was written by the kernels ahead of its predecessor: all
+// of the predecessor's blocks have passed their own wait by then, so those are complete.  (k_loss
+// reads its labels and k_lookup its index streams there; prefetches into L2 are open too.)
 //
 // Every kernel launched with the attribute must call grid_dependency_sync() in every block that
 // does not return at once: completion of kernel N then implies completion of kernel N-1, which is

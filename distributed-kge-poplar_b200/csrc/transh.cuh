@@ -5,8 +5,9 @@
 //   e_ijk = pt_ik - (t_jk - n_ik (n_i . t_j))
 //   score_ij = gamma - sum_k |e_ijk|                     (always the L1 form, whatever model.distance_fn says).
 // Here are the pairwise distances with the two [B, T] matrices the backward needs (s_ij = n_i . t_j and
-// u_ij = sum_k sign(e_ijk) n_ik) and the gradients of the distance with respect to pt, n and the tails; the prediction and
-// its backward down to the head rows, the translation rows and the raw normals are k_lookup and k_lookup_bwd.  FP32-pipe kernels; every sum has a fixed order.
+// u_ij = sum_k sign(e_ijk) n_ik) and the gradients of the distance with respect to pt, n and the tails; the prediction and its
+// backward down to the head rows, the translation rows and the raw normals are k_lookup and k_lookup_bwd.  FP32-pipe kernels;
+// every sum has a fixed order.
 #pragma once
 
 #include <algorithm>
