@@ -1700,14 +1700,14 @@ EntityStep Engine::entity_step(unsigned step, unsigned n) const {
     return g;
 }
 
-// The training step of batched launches: six to nine on the step's chain (hidden rows, lookups + send, scores, loss, score
+// The training step of batched launches: five to nine on the step's chain (hidden rows, lookups + send, scores, loss, score
 // gradients + return, the prediction's backward, segment sums + Adam + relation gradients, projection gradient, dense
 // update; what a model has no use for is left out, and the lookups of the elementwise score functions are the hidden
 // kernel's epilogue) and the next step's gather beside the last two.  Every launch works on all local shards, which meet
 // at the exchange (the tails and the tails' gradients), and every operand of a contraction is the fp32 array its producer
 // wrote (the upper TF32 plane) plus a lower plane the same producer wrote next to it.
 // With a stream per shard instead, forked and joined three times a step, and a dense update of its own (us per step,
-// before -> after): demo preset, 2 shards, 40.4 -> 32.3; four shards of 256 x 320 L1 scores, 76.4 -> 67.2; four of 256 x 512
+// before -> after): demo preset, 2 shards, 40.4 -> 32.3; four shards of 256 x 320 L1 scores, 70.0 -> 67.2; four of 256 x 512
 // fp16 rows, 79.4 -> 83.1 (57.4 with the pair gradients of today); two shards of the headline step 129.5 -> 112.9.
 void Engine::launch_step_planes(unsigned step, const LossParams& lp, float normaliser) {
     const unsigned B = cfg_.batch_size, T = cfg_.n_tail(), R = cfg_.n_remote(), D = cfg_.d, F = cfg_.f;
