@@ -676,8 +676,8 @@ def test_engines_on_two_threads_capture_their_first_runs_side_by_side(name, tens
             assert got[i] is not None, "the run on this thread failed"
             np.testing.assert_array_equal(got[i], want[i][0])
             state = read_state(engine, cfg, RW, cfg.n_shard)
-            for name, value in want[i][1].items():
-                np.testing.assert_array_equal(state[name], value, err_msg=name)
+            for key, value in want[i][1].items():
+                np.testing.assert_array_equal(state[key], value, err_msg=key)
             engine.close()
 
 

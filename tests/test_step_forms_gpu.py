@@ -190,7 +190,7 @@ def test_ranked_queries_straight_from_the_table(score_fn, distance_fn, d, dtype)
 def _product_plus(a, x, y):
     """a x + y in float32 with one rounding, as an FMA gives it: the product is exact in float64, the sum is rounded to odd there,
     which float32's rounding of it cannot be misled by."""
-    p, y = np.float64(a) * np.asarray(x, np.float64), np.asarray(y, np.float64)
+    p, y = np.asarray(a, np.float32).astype(np.float64) * np.asarray(x, np.float64), np.asarray(y, np.float64)
     total = p + y
     back = total - p
     error = (p - (total - back)) + (y - back)
