@@ -382,6 +382,7 @@ Engine::Engine(const SettingMap& settings) : cfg_(parse_config(settings)) {
     direct_rows_ = planes_ && cfg_.f == 0 && !cfg_.regularised();
     // Shards of one launch.  With several processes the hand-over counters count the blocks of one shard's kernel at a time.
     group_ = cfg_.world == 1 ? std::min(n_local_, (unsigned)kShardBatch) : 1u;
+    alone_ = planes_ || n_local_ == 1 || cfg_.world > 1;
     // Where every shard is in every launch no gradient has to wait for another launch: the projection gradient's
     // contraction (over all shards' rows) and the relation rows' blocks of the entity update apply the Adam step
     // themselves and k_dense_update is not launched.
@@ -1605,7 +1606,7 @@ void Engine::launch_lookup(unsigned l0, unsigned n, unsigned step) {
             a.hid = b.hid_h;
         }
     }
-    KGE_LAUNCH("lookup", KGE_CUDA(kge::launch_lookup(shards, (int)n, sizes, cfg_.score_fn, lookup_type(), stream_)));
+    KGE_LAUNCH("lookup", KGE_CUDA(kge::launch_lookup(shards, (int)n, sizes, cfg_.score_fn, lookup_type(), stream_, alone_)));
 }
 
 void Engine::launch_lookup_bwd(unsigned l0, unsigned n, unsigned step) {
@@ -1615,7 +1616,7 @@ void Engine::launch_lookup_bwd(unsigned l0, unsigned n, unsigned step) {
         const ShardBuffers& b = shards_[l0 + i];
         shards.s[i] = LookupBwdArgs{lookup_rows(l0 + i, step), d_relation_ + ((size_t)(l0 + i) * cfg_.n_step + step) * B, b.d_pred, b.d_head, b.d_relrow, b.nrm, b.d_nrm, b.d_normrow};
     }
-    KGE_LAUNCH("lookup_bwd", KGE_CUDA(kge::launch_lookup_bwd(shards, (int)n, dense_, dense_ + dense_bounds_[3], (int)B, (int)cfg_.d, cfg_.score_fn, lookup_type(), stream_)));
+    KGE_LAUNCH("lookup_bwd", KGE_CUDA(kge::launch_lookup_bwd(shards, (int)n, dense_, dense_ + dense_bounds_[3], (int)B, (int)cfg_.d, cfg_.score_fn, lookup_type(), stream_, alone_)));
 }
 
 ShardArgs<TranshScoreArgs> Engine::transh_scores(unsigned l0, unsigned n) const {
@@ -1817,7 +1818,7 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
             const ShardBuffers& b = shards_[l0 + i];
             loss.s[i] = LossArgs{b.raw, step_ptr(d_tail_, l0 + i, B), b.coeff, dot || l2 ? b.coeff_lo : nullptr, b.loss_rows, nullptr, nullptr, nullptr, nullptr};
         }
-        KGE_LAUNCH("loss", KGE_CUDA(launch_loss(loss, (int)n, lp, 1.0f / normaliser, bf16 ? 1 : 0, (int)B, stream_)));
+        KGE_LAUNCH("loss", KGE_CUDA(launch_loss(loss, (int)n, lp, 1.0f / normaliser, bf16 ? 1 : 0, (int)B, stream_, alone_)));
         // 4. score gradients; the tails' rows go straight to the shards that own them
         if (transh) {
             KGE_LAUNCH("score_bwd", KGE_CUDA(launch_transh_bwd(transh_gradients(l0, n), (int)n, stream_)));
@@ -2078,7 +2079,7 @@ void Engine::launch_one_step(unsigned step) {
         }
         ShardArgs<LossArgs> loss{};
         loss.s[0] = LossArgs{b.raw, tail, b.coeff, nullptr, b.loss_rows, d_loss_total_ + l, d_loss_last_ + l, d_loss_counter_ + l, d_reg_loss_ ? d_reg_loss_ + 2 * l : nullptr};
-        KGE_LAUNCH("loss", KGE_CUDA(launch_loss(loss, 1, lp, 1.0f / normaliser, 0, (int)B, stream_)));
+        KGE_LAUNCH("loss", KGE_CUDA(launch_loss(loss, 1, lp, 1.0f / normaliser, 0, (int)B, stream_, alone_ && transh)));
         if (tc_bwd) {
             // Both input gradients are contractions with the coefficient matrix C [B, T]:
             //   dot:  d_pred = C . tails,                          d_tails = C^T . pred

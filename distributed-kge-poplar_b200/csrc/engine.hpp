@@ -229,6 +229,7 @@ class Engine {
     bool direct_rows_ = false;        // lookups and row update read the table: no gathered copy, no hidden rows
     bool planes_ = false;             // the step of batched launches, its contractions on the plane-fed tensor-core kernel
     unsigned group_ = 1;              // local shards of one launch
+    bool alone_ = false;              // no two shards' launches run side by side, on streams of their own
     unsigned score_ld_ = 0;           // floats between rows of scores, coefficients and TransH's pair matrices
     bool bf16_planes_ = false;        // scores and their gradients multiply bfloat16 copies of their operands
     uint32_t feat_stride_ = 0;        // floats per row of the widened / lower feature planes

@@ -964,26 +964,26 @@ k_loss(const __grid_constant__ ShardArgs<LossArgs> shards, LossParams lp, float 
 
 template <int THREADS>
 inline cudaError_t launch_loss(const ShardArgs<LossArgs>& shards, int n_shards, const LossParams& lp, float inv_normaliser, int lo_bf16, int B,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, bool spread) {
     const dim3 grid((unsigned)B, (unsigned)n_shards);
     // columns per thread: as few as the row needs (a batch has at most kMaxSortItems tails)
     const int per = (lp.n_tail + THREADS - 1) / THREADS;
-    if (per <= 1) return launch_spread<k_loss<THREADS, 1>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
-    if (per <= 2) return launch_spread<k_loss<THREADS, 2>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
-    if (per <= 3) return launch_spread<k_loss<THREADS, 3>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
-    if (per <= 4) return launch_spread<k_loss<THREADS, 4>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
-    if (per <= 6) return launch_spread<k_loss<THREADS, 6>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
-    if (per <= 8) return launch_spread<k_loss<THREADS, 8>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
-    if (per <= 16) return launch_spread<k_loss<THREADS, 16>>(grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 1) return launch_spread_if<k_loss<THREADS, 1>>(spread, grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 2) return launch_spread_if<k_loss<THREADS, 2>>(spread, grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 3) return launch_spread_if<k_loss<THREADS, 3>>(spread, grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 4) return launch_spread_if<k_loss<THREADS, 4>>(spread, grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 6) return launch_spread_if<k_loss<THREADS, 6>>(spread, grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 8) return launch_spread_if<k_loss<THREADS, 8>>(spread, grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
+    if (per <= 16) return launch_spread_if<k_loss<THREADS, 16>>(spread, grid, dim3(THREADS), stream, shards, lp, inv_normaliser, lo_bf16);
     return cudaErrorInvalidValue;
 }
 inline cudaError_t launch_loss(const ShardArgs<LossArgs>& shards, int n_shards, const LossParams& lp, float inv_normaliser, int lo_bf16, int B,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, bool spread) {
     // A warp per row, with a serial chain of exponentials, measured 4 us slower for 512 x 768 scores.  A long row of
     // log-sigmoids, whose chains are longest, gets twice the threads: 256 x 1536 self-adversarial scores 12.7 to 9.5 us
     // (a softmax row of that length was 1 us slower with them).
-    if (lp.loss_fn == LOSS_LOGSIGMOID && lp.n_tail >= 1024) return launch_loss<512>(shards, n_shards, lp, inv_normaliser, lo_bf16, B, stream);
-    return launch_loss<256>(shards, n_shards, lp, inv_normaliser, lo_bf16, B, stream);
+    if (lp.loss_fn == LOSS_LOGSIGMOID && lp.n_tail >= 1024) return launch_loss<512>(shards, n_shards, lp, inv_normaliser, lo_bf16, B, stream, spread);
+    return launch_loss<256>(shards, n_shards, lp, inv_normaliser, lo_bf16, B, stream, spread);
 }
 
 // ---------------------------------------------------------------------------

@@ -48,23 +48,36 @@ __device__ __forceinline__ void store_with_plane(float* out, float* lo, int lo_b
     else lo[row * D + c] = tf32_lower(v);
 }
 
-// A warp per row of `n_cols` columns: f(c, value) with a float4 where rows allow 16-byte accesses, four in flight a lane.
+// A warp per row of D columns and the same columns of N float rows beside it: f(c, value, beside) with float4s where rows allow
+// 16-byte accesses, four pieces of every row in flight a lane.
+template <int N, class VT, class F>
+__device__ __forceinline__ void for_row(const VT* __restrict__ src, const float* const (&rows)[N], int D, F f) {
+    const int lane = threadIdx.x & 31;
+    auto pieces = [&](auto zero, int stride, auto load_value, auto load_beside) {
+        using T = decltype(zero);
+        const int step = stride * 32;
+        for (int c0 = lane * stride; c0 < D; c0 += 4 * step) {
+            T v[4], beside[4][N];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (c0 + u * step >= D) continue;
+                v[u] = load_value(src + c0 + u * step);
+#pragma unroll
+                for (int i = 0; i < N; ++i)
+                    if (rows[i]) beside[u][i] = load_beside(rows[i] + c0 + u * step);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (c0 + u * step < D) f(c0 + u * step, v[u], beside[u]);
+        }
+    };
+    if ((D & 3) == 0) pieces(float4{}, 4, [](const VT* p) { return load4(p); }, [](const float* p) { return load4(p); });
+    else pieces(0.f, 1, [](const VT* p) { return load_as_float(p); }, [](const float* p) { return *p; });
+}
 template <class VT, class F>
 __device__ __forceinline__ void for_row(const VT* __restrict__ src, int D, F f) {
-    const int lane = threadIdx.x & 31;
-    if ((D & 3) == 0) {
-        for (int c0 = lane * 4; c0 < D; c0 += 4 * 128) {
-            float4 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (c0 + u * 128 < D) v[u] = load4(src + c0 + u * 128);
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (c0 + u * 128 < D) f(c0 + u * 128, v[u]);
-        }
-    } else {
-        for (int c = lane; c < D; c += 32) f(c, load_as_float(src + c));
-    }
+    const float* const none[1] = {nullptr};
+    for_row<1>(src, none, D, [&](int c, auto v, const auto&) { f(c, v); });
 }
 
 // Sums over a row's columns for a whole warp: add(c, sums) for the columns lane, lane + 64, ... into one set of sums and for
@@ -149,14 +162,13 @@ __global__ void __launch_bounds__(256) k_lookup(const __grid_constant__ ShardArg
                 a.pred[(size_t)i * D + c] = load_as_float(h + c) - n * nh + r[c];
             }
         } else {
-            for_row(h, D, [&](int c, auto v) {
-                auto with = [&](float x, float q) { return FN == SCORE_TRANSE ? x + q : x * q; };
-                if constexpr (sizeof(v) == sizeof(float4)) {
-                    const float4 q = load4(r + c);
-                    store_with_plane(a.pred, a.pred_lo, g.lo_bf16, (size_t)i, D, c, make_float4(with(v.x, q.x), with(v.y, q.y), with(v.z, q.z), with(v.w, q.w)));
-                } else {
-                    store_with_plane(a.pred, a.pred_lo, g.lo_bf16, (size_t)i, D, c, with(v, r[c]));
-                }
+            const float* const beside[1] = {r};
+            for_row<1>(h, beside, D, [&](int c, auto v, const auto& q) {
+                auto with = [&](float x, float y) { return FN == SCORE_TRANSE ? x + y : x * y; };
+                if constexpr (sizeof(v) == sizeof(float4))
+                    store_with_plane(a.pred, a.pred_lo, g.lo_bf16, (size_t)i, D, c, make_float4(with(v.x, q[0].x), with(v.y, q[0].y), with(v.z, q[0].z), with(v.w, q[0].w)));
+                else
+                    store_with_plane(a.pred, a.pred_lo, g.lo_bf16, (size_t)i, D, c, with(v, q[0]));
             });
         }
     } else if (a.remote && unit - g.B - g.T < g.R) {
@@ -168,14 +180,15 @@ __global__ void __launch_bounds__(256) k_lookup(const __grid_constant__ ShardArg
 }
 
 // `value_type` of the rows: 0 fp32, 1 fp16, 2 bf16.
-inline cudaError_t launch_lookup(const ShardArgs<LookupArgs>& shards, int n_shards, const LookupSizes& g, int score_fn, int value_type, cudaStream_t stream) {
+inline cudaError_t launch_lookup(const ShardArgs<LookupArgs>& shards, int n_shards, const LookupSizes& g, int score_fn, int value_type, cudaStream_t stream,
+                                 bool spread = true) {
     auto with_type = [&](auto fn) {
         constexpr int FN = decltype(fn)::value;
         const int warps = g.B * kHeadWarps<FN> + g.T + (shards.s[0].remote ? g.R : 0);
         const dim3 grid((unsigned)((warps + 7) / 8), (unsigned)n_shards);
-        if (value_type == 2) return launch_spread<k_lookup<__nv_bfloat16, FN>>(grid, dim3(256), stream, shards, g);
-        if (value_type == 1) return launch_spread<k_lookup<__half, FN>>(grid, dim3(256), stream, shards, g);
-        return launch_spread<k_lookup<float, FN>>(grid, dim3(256), stream, shards, g);
+        if (value_type == 2) return launch_spread_if<k_lookup<__nv_bfloat16, FN>>(spread, grid, dim3(256), stream, shards, g);
+        if (value_type == 1) return launch_spread_if<k_lookup<__half, FN>>(spread, grid, dim3(256), stream, shards, g);
+        return launch_spread_if<k_lookup<float, FN>>(spread, grid, dim3(256), stream, shards, g);
     };
     switch (score_fn) {
         case SCORE_DISTMULT: return with_type(std::integral_constant<int, SCORE_DISTMULT>{});
@@ -211,14 +224,15 @@ k_lookup_bwd(const __grid_constant__ ShardArgs<LookupBwdArgs> shards, const floa
     float* __restrict__ dh = a.d_head + (size_t)i * D;
     float* __restrict__ dr = a.d_relrow + (size_t)i * D;
     if (FN == SCORE_DISTMULT) {
-        for_row(h, D, [&](int c, auto v) {
+        const float* const beside[2] = {r, dp};
+        for_row<2>(h, beside, D, [&](int c, auto v, const auto& o) {
+            const auto &q = o[0], &g = o[1];
             if constexpr (sizeof(v) == sizeof(float4)) {
-                const float4 q = load4(r + c), g = load4(dp + c);
                 store4(dh + c, make_float4(g.x * q.x, g.y * q.y, g.z * q.z, g.w * q.w));
                 store4(dr + c, make_float4(g.x * v.x, g.y * v.y, g.z * v.z, g.w * v.w));
             } else {
-                dh[c] = dp[c] * r[c];
-                dr[c] = dp[c] * v;
+                dh[c] = g * q;
+                dr[c] = g * v;
             }
         });
     } else if (FN == SCORE_ROTATE) {
@@ -273,13 +287,13 @@ k_lookup_bwd(const __grid_constant__ ShardArgs<LookupBwdArgs> shards, const floa
 }
 
 inline cudaError_t launch_lookup_bwd(const ShardArgs<LookupBwdArgs>& shards, int n_shards, const float* rel_table, const float* normal_table, int B, int D,
-                                     int score_fn, int value_type, cudaStream_t stream) {
+                                     int score_fn, int value_type, cudaStream_t stream, bool spread = true) {
     auto with_type = [&](auto fn) {
         constexpr int FN = decltype(fn)::value;
         const dim3 grid((unsigned)((B * kHeadWarps<FN> + 7) / 8), (unsigned)n_shards);
-        if (value_type == 2) return launch_spread<k_lookup_bwd<__nv_bfloat16, FN>>(grid, dim3(256), stream, shards, rel_table, normal_table, B, D);
-        if (value_type == 1) return launch_spread<k_lookup_bwd<__half, FN>>(grid, dim3(256), stream, shards, rel_table, normal_table, B, D);
-        return launch_spread<k_lookup_bwd<float, FN>>(grid, dim3(256), stream, shards, rel_table, normal_table, B, D);
+        if (value_type == 2) return launch_spread_if<k_lookup_bwd<__nv_bfloat16, FN>>(spread, grid, dim3(256), stream, shards, rel_table, normal_table, B, D);
+        if (value_type == 1) return launch_spread_if<k_lookup_bwd<__half, FN>>(spread, grid, dim3(256), stream, shards, rel_table, normal_table, B, D);
+        return launch_spread_if<k_lookup_bwd<float, FN>>(spread, grid, dim3(256), stream, shards, rel_table, normal_table, B, D);
     };
     switch (score_fn) {
         case SCORE_COMPLEX: return with_type(std::integral_constant<int, SCORE_COMPLEX>{});

@@ -110,5 +110,14 @@ inline cudaError_t launch_spread(dim3 grid, dim3 block, cudaStream_t stream, Arg
     unused = std::max(0, std::min(unused, 227 * 1024 - static_bytes)) / 128 * 128;
     return launch_dependent(Kernel, grid, block, (size_t)unused, stream, static_cast<Args&&>(args)...);
 }
+// That memory keeps kernels of other streams off the SM too: the lookups and the loss of shards that run side by side, each on
+// a stream, are not spread (us a step, spread -> not: four shards of 256 x 320 x 10 L1 scores 60 -> 55, of 64 columns 62 -> 57).
+// In the step of separate kernels the loss of one shard is spread for TransH alone (512 x 768 x 50: 137, 150 without), not in
+// front of L1 gradients, whose blocks stay where its blocks have left room (512 x 768 x 63: 76 -> 74; its lookups not spread, 87).
+template <auto Kernel, typename... Args>
+inline cudaError_t launch_spread_if(bool spread, dim3 grid, dim3 block, cudaStream_t stream, Args&&... args) {
+    if (!spread) return launch_dependent(Kernel, grid, block, 0, stream, static_cast<Args&&>(args)...);
+    return launch_spread<Kernel>(grid, block, stream, static_cast<Args&&>(args)...);
+}
 
 }  // namespace kge

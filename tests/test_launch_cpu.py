@@ -46,7 +46,10 @@ static bool spread(unsigned blocks) {
     return share * each <= sm && ((share + 1) * each > sm || dynamic_bytes + kStatic >= 227 * 1024 - 128);
 }
 
+static bool not_spread() { return kge::launch_spread_if<kernel>(false, dim3(160), dim3(256), nullptr, 1) == cudaSuccess && dynamic_bytes == 0; }
+
 int main(int argc, char** argv) {
+    if (argc > 1 && !strcmp(argv[1], "beside")) return not_spread() ? 0 : 1;
     if (argc > 1) return kge::launch_spread<kernel>(dim3(0), dim3(256), nullptr, 1) == cudaErrorInvalidConfiguration ? 0 : 1;
     std::vector<std::thread> threads;
     bool ok[4] = {};
@@ -82,6 +85,12 @@ def test_spread_launches_on_several_threads(program):
     its share of the blocks and no more."""
     run = subprocess.run([program], capture_output=True, text=True)
     assert run.returncode == 0, run.stderr[-3000:]
+
+
+def test_a_launch_beside_others_leaves_them_room(program):
+    """Where shards run side by side, no block takes an SM's shared memory for itself."""
+    run = subprocess.run([program, "beside"], capture_output=True, text=True)
+    assert run.returncode == 0, run
 
 
 def test_a_launch_of_no_blocks_is_an_error_status(program):
