@@ -378,8 +378,10 @@ Engine::Engine(const SettingMap& settings) : cfg_(parse_config(settings)) {
     if (const char* v = std::getenv("KGE_PLANE_CONTRACTIONS")) planes_ = planes_ && std::atoi(v) != 0;
     if (mlp_on()) planes_ = false;  // the MLP sits between the projection and the lookups: the step of separate kernels
     score_ld_ = planes_ ? (unsigned)round_up(cfg_.n_tail(), 8) : cfg_.n_tail();
-    // Without features a hidden row is the stored value: the lookups and the row update read the table itself.
-    direct_rows_ = planes_ && cfg_.f == 0 && !cfg_.regularised();
+    // Without features a hidden row is the stored value: the lookups read the table itself and, but for the regularisers, which
+    // take the hidden rows and the state of a gathered copy, so does the row update.
+    table_lookups_ = planes_ && cfg_.f == 0;
+    direct_rows_ = table_lookups_ && !cfg_.regularised();
     // Shards of one launch.  With several processes the hand-over counters count the blocks of one shard's kernel at a time.
     group_ = cfg_.world == 1 ? std::min(n_local_, (unsigned)kShardBatch) : 1u;
     alone_ = planes_ || n_local_ == 1 || cfg_.world > 1;
@@ -567,7 +569,7 @@ void Engine::allocate() {
     d_rel_perm_ = (uint32_t*)device_alloc(steps * B * 4);
     d_rel_off_ = (uint32_t*)device_alloc(steps * (cfg_.n_relation_type + 1) * 4);
     d_first_slot_ = (uint32_t*)device_alloc(steps * R * 4);
-    if (direct_rows_) d_lookup_row_ = (uint32_t*)device_alloc(steps * (B + T) * 4);
+    if (table_lookups_) d_lookup_row_ = (uint32_t*)device_alloc(steps * (B + T) * 4);
     d_heavy_parts_ = (uint4*)device_alloc(steps * kHeavySlots * sizeof(uint4));
     d_row_info_ = (uint4*)device_alloc(steps * 2 * R * sizeof(uint4));
     d_heavy_count_ = (uint32_t*)device_alloc(steps * 4);
@@ -1513,22 +1515,23 @@ void Engine::launch_mlp_backward(unsigned l, unsigned step) {
                                                          (const float*)b.d_val, (const float*)(d_step_size_ + step), entity_lr_mod_, adam_, (int)R)));
 }
 
-// The norm regularisers of local shard l's gathered rows (k_regularise): after the hidden rows,
+// The norm regularisers of local shards' gathered rows (k_regularise): after the hidden rows,
 // before the loss (which adds their loss term) and the entity update (which adds their gradients).
-void Engine::launch_regularise(unsigned l, const uint8_t* rows_c) {
-    ShardBuffers& b = shards_[l];
+void Engine::launch_regularise(unsigned l0, unsigned n, unsigned step) {
     const size_t R = cfg_.n_remote();
     RegParams rp{};
     for (int i = 0; i < 3; ++i) rp.power[i] = cfg_.reg_power[i], rp.weight[i] = cfg_.reg_weight[i];
     rp.loss_scale = cfg_.loss_scale;
-    rp.shared = b.hid_t == b.hid_h ? 1 : 0;
-    float* loss = d_reg_loss_ + 2 * l;
-    if (cfg_.state_type == ST_F32)
-        KGE_LAUNCH("regularise", KGE_CUDA(launch_dependent(k_regularise<float>, dim3((unsigned)ceil_div(R, 8)), dim3(256), 0, stream_, rows_c, layout_, b.hid_h,
-                                                           b.hid_t, (int)R, rp, b.reg_val, b.reg_h, b.reg_t, b.reg_loss_rows, loss, loss + 1, d_reg_counter_ + l)));
-    else
-        KGE_LAUNCH("regularise", KGE_CUDA(launch_dependent(k_regularise<__half>, dim3((unsigned)ceil_div(R, 8)), dim3(256), 0, stream_, rows_c, layout_, b.hid_h,
-                                                           b.hid_t, (int)R, rp, b.reg_val, b.reg_h, b.reg_t, b.reg_loss_rows, loss, loss + 1, d_reg_counter_ + l)));
+    rp.shared = shards_[l0].hid_t == shards_[l0].hid_h ? 1 : 0;
+    ShardArgs<RegArgs> shards{};
+    for (unsigned i = 0; i < n; ++i) {
+        const ShardBuffers& b = shards_[l0 + i];
+        float* loss = d_reg_loss_ + 2 * (l0 + i);
+        shards.s[i] = RegArgs{b.rows_c2[step & 1], b.hid_h, b.hid_t, b.reg_val, b.reg_h, b.reg_t, b.reg_loss_rows, loss, loss + 1, d_reg_counter_ + l0 + i};
+    }
+    const dim3 grid((unsigned)ceil_div(R, 8), n);
+    if (cfg_.state_type == ST_F32) KGE_LAUNCH("regularise", KGE_CUDA(launch_dependent(k_regularise<float>, grid, dim3(256), 0, stream_, shards, layout_, (int)R, rp)));
+    else KGE_LAUNCH("regularise", KGE_CUDA(launch_dependent(k_regularise<__half>, grid, dim3(256), 0, stream_, shards, layout_, (int)R, rp)));
 }
 
 DropoutParams Engine::dropout_params(unsigned l, unsigned step) const {
@@ -1542,18 +1545,17 @@ DropoutParams Engine::dropout_params(unsigned l, unsigned step) const {
     return dp;
 }
 
-// hidden = value + dropout(hidden - value) for both calls of local shard l (k_dropout_hidden).
-void Engine::launch_dropout(unsigned l, unsigned step, const uint8_t* rows_c) {
-    ShardBuffers& b = shards_[l];
+// hidden = value + dropout(hidden - value) for both calls of local shards (k_dropout_hidden).
+void Engine::launch_dropout(unsigned l0, unsigned n, unsigned step) {
     const size_t R = cfg_.n_remote(), quads = ceil_div(cfg_.d, 4);
-    const float* tail_in = cfg_.n_net() == 2 ? b.hid_t : b.hid_h;
-    const dim3 grid((unsigned)ceil_div(R * quads, 256));
-    if (cfg_.state_type == ST_F32)
-        KGE_LAUNCH("dropout", KGE_CUDA(launch_dependent(k_dropout_hidden<float>, grid, dim3(256), 0, stream_, rows_c, layout_, b.hid_h, tail_in, b.hid_t,
-                                                        (int)R, dropout_params(l, step))));
-    else
-        KGE_LAUNCH("dropout", KGE_CUDA(launch_dependent(k_dropout_hidden<__half>, grid, dim3(256), 0, stream_, rows_c, layout_, b.hid_h, tail_in, b.hid_t,
-                                                        (int)R, dropout_params(l, step))));
+    ShardArgs<DropoutArgs> shards{};
+    for (unsigned i = 0; i < n; ++i) {
+        const ShardBuffers& b = shards_[l0 + i];
+        shards.s[i] = DropoutArgs{b.rows_c2[step & 1], b.hid_h, cfg_.n_net() == 2 ? b.hid_t : b.hid_h, b.hid_t, dropout_params(l0 + i, step)};
+    }
+    const dim3 grid((unsigned)ceil_div(R * quads, 256), n);
+    if (cfg_.state_type == ST_F32) KGE_LAUNCH("dropout", KGE_CUDA(launch_dependent(k_dropout_hidden<float>, grid, dim3(256), 0, stream_, shards, layout_, (int)R)));
+    else KGE_LAUNCH("dropout", KGE_CUDA(launch_dependent(k_dropout_hidden<__half>, grid, dim3(256), 0, stream_, shards, layout_, (int)R)));
 }
 
 static tc::PlaneOperand plane_operand(const float* hi, const float* lo, long long stride_bytes, bool mn_major) {
@@ -1570,13 +1572,13 @@ tc::PlaneOperand Engine::features(const ShardBuffers& b, unsigned step, bool mn_
 LookupRows Engine::lookup_rows(unsigned l, unsigned step) const {
     const ShardBuffers& b = shards_[l];
     const size_t B = cfg_.batch_size, T = cfg_.n_tail(), sidx = (size_t)l * cfg_.n_step + step;
-    if (direct_rows_) {
+    if (table_lookups_) {
         const uint32_t* row = d_lookup_row_ + sidx * (B + T);
         return LookupRows{b.table, b.table, row, row + B, layout_.row_bytes};
     }
     return LookupRows{reinterpret_cast<const uint8_t*>(b.hid_h), reinterpret_cast<const uint8_t*>(b.hid_t), d_head_ + sidx * B, d_a2a_ + sidx * T, (uint32_t)(cfg_.d * 4)};
 }
-int Engine::lookup_type() const { return !direct_rows_ ? 0 : cfg_.value_bf16 ? 2 : cfg_.state_type == ST_F16 ? 1 : 0; }
+int Engine::lookup_type() const { return !table_lookups_ ? 0 : cfg_.value_bf16 ? 2 : cfg_.state_type == ST_F16 ? 1 : 0; }
 
 // Lookups, predicted tails and the send half of the exchange for local shards whose hidden rows are ready.
 void Engine::launch_lookup(unsigned l0, unsigned n, unsigned step) {
@@ -1587,7 +1589,7 @@ void Engine::launch_lookup(unsigned l0, unsigned n, unsigned step) {
     sizes.normal_table = dense_ + dense_bounds_[3];
     sizes.B = (int)B; sizes.T = (int)cfg_.n_tail(); sizes.a2a = (int)cfg_.a2a_size; sizes.D = (int)cfg_.d; sizes.R = (int)R;
     sizes.lo_bf16 = bf16_planes_ ? 1 : 0;
-    sizes.prefetch = direct_rows_ && step > 0;  // the first step's index streams come from the kernel in front
+    sizes.prefetch = table_lookups_ && step > 0;  // the first step's index streams come from the kernel in front
     sizes.sync = exchange_sync();
     ShardArgs<LookupArgs> shards{};
     for (unsigned i = 0; i < n; ++i) {
@@ -1601,7 +1603,7 @@ void Engine::launch_lookup(unsigned l0, unsigned n, unsigned step) {
         a.pred = b.pred;
         a.pred_lo = companion ? b.pred_lo : nullptr;
         a.nrm = b.nrm;
-        if (direct_rows_ && step + 1 == cfg_.n_step) {  // kge_debug_fetch shows the last step's hidden rows
+        if (table_lookups_ && (!direct_rows_ || step + 1 == cfg_.n_step)) {  // the regularisers take them, kge_debug_fetch shows the last step's
             a.remote = d_remote_ + sidx * R;
             a.hid = b.hid_h;
         }
@@ -1767,25 +1769,19 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
         } else {
             launch_exchange_wait(XCHG_DENSE_PARAMS);
         }
-        for (unsigned l = l0; l < l0 + n; ++l) {
-            const ShardBuffers& b = shards_[l];
-            const size_t sidx = (size_t)l * cfg_.n_step + step;
-            if (F == 0 && !direct_rows_) {  // the hidden rows are the gathered values
-                dim3 grid(ceil_div(R, 64), ceil_div(D, 64), 1);
-                KGE_LAUNCH("hidden", KGE_DISPATCH_ROW(cfg_, KGE_CUDA(launch_dependent(k_hidden<ST, FT>, dim3(grid), dim3(256), 0, stream_, b.rows_c2[parity],
-                                                                                      layout_, nullptr, 0u, (int)R, nullptr, nullptr, b.hid_h, b.hid_t))));
-            }
-            if (heavy_route)
+        if (heavy_route)
+            for (unsigned l = l0; l < l0 + n; ++l) {
+                const ShardBuffers& b = shards_[l];
+                const size_t sidx = (size_t)l * cfg_.n_step + step;
                 KGE_LAUNCH("route_heavy", KGE_CUDA(launch_dependent(k_route_heavy, dim3(kHeavySlots), dim3(256), 0, stream_, (const float*)b.hid_h, (const float*)b.hid_t,
                                                                     (const uint4*)(d_heavy_parts_ + sidx * kHeavySlots), (const uint32_t*)(d_heavy_count_ + sidx),
                                                                     (const uint32_t*)(d_ent_perm_ + sidx * (B + T)), (const uint32_t*)step_ptr(d_relation_, l, B),
                                                                     (const float*)dense_, b.send_dst, b.send_lo_dst, b.pred, b.pred_lo, (int)B, (int)cfg_.a2a_size,
                                                                     (int)D, cfg_.score_fn, bf16 ? 1 : 0, sync)));
-            if (dropout_on()) launch_dropout(l, step, b.rows_c2[parity]);
-        }
+            }
+        if (dropout_on()) launch_dropout(l0, n, step);
         if (!fused_route) launch_lookup(l0, n, step);
-        if (cfg_.regularised())
-            for (unsigned l = l0; l < l0 + n; ++l) launch_regularise(l, shards_[l].rows_c2[parity]);
+        if (cfg_.regularised()) launch_regularise(l0, n, step);
     }
     KGE_CUDA(cudaGetLastError());
 
@@ -2042,9 +2038,9 @@ void Engine::launch_one_step(unsigned step) {
         if (mlp_on())
             for (unsigned net = 0; net < cfg_.n_net(); ++net)
                 launch_mlp_forward(rows_c, nullptr, 0u, R, (int)net, net ? b.hid_t : b.hid_h, b.mlp_cat[net], b.mlp_pre[net], b.mlp_out);
-        if (dropout_on()) launch_dropout(l, step, rows_c);
+        if (dropout_on()) launch_dropout(l, 1, step);
         launch_lookup(l, 1, step);
-        if (cfg_.regularised()) launch_regularise(l, rows_c);
+        if (cfg_.regularised()) launch_regularise(l, 1, step);
     }
     shards_join();
     KGE_CUDA(cudaGetLastError());

@@ -226,7 +226,8 @@ class Engine {
     cudaStream_t side_stream_ = nullptr;
     unsigned side_streams_ = 0;
     bool split_popular_rows_ = true;  // rows with many lookups are summed in parts by several blocks
-    bool direct_rows_ = false;        // lookups and row update read the table: no gathered copy, no hidden rows
+    bool table_lookups_ = false;      // lookups read the table: the hidden rows are its values
+    bool direct_rows_ = false;        // and so does the row update: no gathered copy, no hidden rows
     bool planes_ = false;             // the step of batched launches, its contractions on the plane-fed tensor-core kernel
     unsigned group_ = 1;              // local shards of one launch
     bool alone_ = false;              // no two shards' launches run side by side, on streams of their own
@@ -319,7 +320,7 @@ class Engine {
     uint32_t *d_ent_perm_ = nullptr, *d_ent_off_ = nullptr, *d_rel_perm_ = nullptr,
              *d_rel_off_ = nullptr, *d_first_slot_ = nullptr, *d_heavy_count_ = nullptr;
     uint4* d_heavy_parts_ = nullptr;
-    uint32_t* d_lookup_row_ = nullptr;  // [n_local * n_step][B + T] table rows by lookup (direct_rows_)
+    uint32_t* d_lookup_row_ = nullptr;  // [n_local * n_step][B + T] table rows by lookup (table_lookups_)
     uint4* d_row_info_ = nullptr;  // [n_local * n_step][R][2] per gathered row: offsets, flags, table row, first four lookups
     float *d_step_size_ = nullptr, *d_loss_total_ = nullptr, *d_loss_last_ = nullptr;
     unsigned* d_loss_counter_ = nullptr;
@@ -338,10 +339,10 @@ class Engine {
     uint32_t* d_step_key_ = nullptr;   // [n_step] numbers of the staged training steps (keys of the dropout masks)
     bool dropout_on() const { return cfg_.dropout > 0.f && cfg_.f > 0; }
     DropoutParams dropout_params(unsigned l, unsigned step) const;
-    void launch_dropout(unsigned l, unsigned step, const uint8_t* rows_c);
+    void launch_dropout(unsigned l0, unsigned n, unsigned step);
     float* d_reg_loss_ = nullptr;      // [n_local][2]: the step's regularisation loss, and a sink for its running sum
     unsigned* d_reg_counter_ = nullptr;
-    void launch_regularise(unsigned l, const uint8_t* rows_c);
+    void launch_regularise(unsigned l0, unsigned n, unsigned step);
     // What crosses to the GPU before a run and what comes back, laid out alike in pinned and in device memory: the five
     // index streams, then the run's words (step numbers, Adam step sizes, the loss totals' zeros), then the two status
     // words and ranking's flag.  Offsets in 32-bit words.

@@ -1510,11 +1510,23 @@ __device__ __forceinline__ uint32_t dropout_keep4(const DropoutParams& dp, uint3
 
 // hidden = value + dropout(hidden - value), in place on the hidden rows of each call.  With one
 // feature network both calls start from the same rows (hid_t_in == hid_h) and get their own masks.
+struct DropoutArgs {
+    const uint8_t* rows_c;
+    float* hid_h;
+    const float* hid_t_in;
+    float* hid_t;
+    DropoutParams dp;
+};
+
 template <class ST>
-__global__ void __launch_bounds__(256)
-k_dropout_hidden(const uint8_t* __restrict__ rows_c, RowLayout L, float* __restrict__ hid_h, const float* __restrict__ hid_t_in,
-                 float* __restrict__ hid_t, int R, DropoutParams dp) {
+__global__ void __launch_bounds__(256) k_dropout_hidden(const __grid_constant__ ShardArgs<DropoutArgs> shards, RowLayout L, int R) {
     grid_dependency_sync();
+    const DropoutArgs& a = shards.s[blockIdx.y];
+    const uint8_t* __restrict__ rows_c = a.rows_c;
+    float* hid_h = a.hid_h;
+    const float* hid_t_in = a.hid_t_in;
+    float* hid_t = a.hid_t;
+    const DropoutParams& dp = a.dp;
     const int D = (int)L.d, quads = (D + 3) / 4;
     const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= R * quads) return;
@@ -1559,12 +1571,23 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+struct RegArgs {
+    const uint8_t* rows_c;
+    const float *hid_h, *hid_t;
+    float *reg_val, *reg_h, *reg_t, *loss_rows, *loss_out, *loss_sink;
+    unsigned* counter;
+};
+
 template <class ST>
-__global__ void __launch_bounds__(256)
-k_regularise(const uint8_t* __restrict__ rows_c, RowLayout L, const float* __restrict__ hid_h, const float* __restrict__ hid_t, int R,
-             RegParams rp, float* __restrict__ reg_val, float* __restrict__ reg_h, float* __restrict__ reg_t,
-             float* __restrict__ loss_rows, float* __restrict__ loss_out, float* __restrict__ loss_sink, unsigned* __restrict__ counter) {
+__global__ void __launch_bounds__(256) k_regularise(const __grid_constant__ ShardArgs<RegArgs> shards, RowLayout L, int R, RegParams rp) {
     grid_dependency_sync();
+    const RegArgs& a = shards.s[blockIdx.y];
+    const uint8_t* __restrict__ rows_c = a.rows_c;
+    const float* __restrict__ hid_h = a.hid_h;
+    const float* __restrict__ hid_t = a.hid_t;
+    float* __restrict__ reg_val = a.reg_val;
+    float* __restrict__ reg_h = a.reg_h;
+    float* __restrict__ reg_t = a.reg_t;
     __shared__ float scratch[8];
     const int lane = threadIdx.x & 31, r = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), D = (int)L.d;
     if (r < R) {
@@ -1605,9 +1628,9 @@ k_regularise(const uint8_t* __restrict__ rows_c, RowLayout L, const float* __res
             }
             reg_val[(size_t)r * D + c] = gv;
         }
-        if (lane == 0) loss_rows[r] = loss;
+        if (lane == 0) a.loss_rows[r] = loss;
     }
-    finish_step_loss<256>(loss_rows, R, 1.f, loss_sink, loss_out, counter, scratch, nullptr);
+    finish_step_loss<256>(a.loss_rows, R, 1.f, a.loss_sink, a.loss_out, a.counter, scratch, nullptr);
 }
 
 struct HeavyRows {

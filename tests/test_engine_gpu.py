@@ -98,6 +98,12 @@ CASES = {
                                                    distance_fn="L1", gamma=3.0, loss_type="logsigmoid",
                                                    embedding_regularisation=(2.5, 0.02), hidden_regularisation=(2.0, 0.04)),
                                     seed=23),
+    # the same in the step of batched launches, whose lookups read the table and whose regularisers read the hidden rows
+    "regularised_table_rows": dict(cfg=StepConfig(n_shard=3, n_entity=101, n_relation_type=6, embedding_size=12,
+                                                  entity_feature_size=0, batch_size=9, a2a_size=5, score_fn="ComplEx",
+                                                  distance_fn="MatMul", loss_type="logsigmoid",
+                                                  embedding_regularisation=(2.5, 0.02), hidden_regularisation=(2.0, 0.04)),
+                                   seed=31),
     # Dropout of the feature network's output: each of the two calls draws its own mask, so the head
     # and tail rows differ even with one shared network; the oracle is given the engine's masks
     "dropout_shared": dict(cfg=StepConfig(n_shard=2, n_entity=300, n_relation_type=4, embedding_size=32,
@@ -285,11 +291,12 @@ def test_exchange_routing_is_bit_exact():
 
 
 # The kernels of a step, one launch each for all shards: lookup, score, loss, score_bwd, entity_update; with features also gather,
-# hidden, projection_bwd, and lookup_bwd but for TransE, whose lookups are the epilogue of "hidden".  Dropout and regularisers are
-# a launch per shard, and so is the MLP's step (hidden, four of the MLP, lookup, regularise, score, loss, score_bwd, dense_partial,
-# entity_update, seven of the MLP's backward, row_adam, projection_bwd) but for its dense_update and the first gather.
+# hidden, projection_bwd, and lookup_bwd but for TransE, whose lookups are the epilogue of "hidden"; dropout turns that epilogue off
+# and is a launch more, as the regularisers are (whose rows are gathered).  The MLP's step is a launch per shard (hidden, four of the
+# MLP, lookup, regularise, score, loss, score_bwd, dense_partial, entity_update, seven of the MLP's backward, row_adam,
+# projection_bwd) but for its dense_update and the first gather.
 LAUNCHES_OF_THREE_STEPS = {"config1_transe_l1": 3 * 5, "transe_l2_softmax_features": 3 * 7, "complex_softmax": 3 * 9,
-                           "dropout_shared": 3 * (8 + 2 * 2), "transh_logsigmoid": 3 * 9, "mlp_shared": 1 + 3 * (2 * 21 + 1) + 2 * 2}
+                           "dropout_shared": 3 * 10, "regularised_table_rows": 3 * 8, "transh_logsigmoid": 3 * 9, "mlp_shared": 1 + 3 * (2 * 21 + 1) + 2 * 2}
 
 
 @pytest.mark.parametrize("name", list(LAUNCHES_OF_THREE_STEPS))
