@@ -384,7 +384,8 @@ Engine::Engine(const SettingMap& settings) : cfg_(parse_config(settings)) {
     direct_rows_ = table_lookups_ && !cfg_.regularised();
     // Shards of one launch.  With several processes the hand-over counters count the blocks of one shard's kernel at a time.
     group_ = cfg_.world == 1 ? std::min(n_local_, (unsigned)kShardBatch) : 1u;
-    alone_ = planes_ || n_local_ == 1 || cfg_.world > 1;
+    branches_ = cfg_.world > 1 ? 1u : planes_ ? ceil_div(n_local_, group_) : n_local_;
+    alone_ = branches_ == 1;
     // Where every shard is in every launch no gradient has to wait for another launch: the projection gradient's
     // contraction (over all shards' rows) and the relation rows' blocks of the entity update apply the Adam step
     // themselves and k_dense_update is not launched.
@@ -1086,9 +1087,9 @@ class StreamPool {
 // steps, or until the steps themselves are over: StreamPool serves every engine of the process, and an engine on another
 // thread may borrow a stream the moment it is back.  After an error they are destroyed, not lent again.
 Engine::ShardStreams::ShardStreams(Engine& e) : engine_(e) {
-    if (e.n_local_ < 2 || e.cfg_.world > 1 || e.kernel_timing_ || e.planes_) return;
-    e.shard_streams_.assign(e.n_local_, nullptr);
-    for (unsigned l = 1; l < e.n_local_; ++l) e.shard_streams_[l] = StreamPool::instance().take();
+    if (e.branches_ < 2 || e.kernel_timing_) return;
+    e.shard_streams_.assign(e.branches_, nullptr);
+    for (unsigned l = 1; l < e.branches_; ++l) e.shard_streams_[l] = StreamPool::instance().take();
 }
 void Engine::ShardStreams::give_back() {
     for (cudaStream_t st : engine_.shard_streams_)
@@ -1218,21 +1219,21 @@ void Engine::side_join(int which) {
     KGE_CUDA(cudaStreamWaitEvent(stream_, ev_join_[which], 0));
 }
 
-// Several shards in one process: the kernels of a phase (hidden rows and lookups; scores and their gradients; row
-// updates and projection gradient) work on one shard each and meet only at the exchange, so every shard's part of a
-// phase is queued on a stream of its own (graph branches under capture).  The kernels of a step are short and mostly
-// far too small to fill 148 SMs: side by side they take little longer than one of them (program runs: the demo
-// preset's two shards, 5 steps, 475 to 342 us; four shards of 256 x 512 L1 scores, 20 steps, 9.5 to 3.7 ms; two
-// shards of the headline step, whose kernels do fill the GPU, 4.0 to 3.6 ms).  Only with one process: the hand-over
-// counters between processes count the blocks of one kernel at a time.
+// More local shards than a launch takes, or the step of separate kernels: the launches of a phase (hidden rows and lookups;
+// scores and their gradients; row updates and projection gradient) work on a group of shards, or one shard, each and meet
+// only at the exchange, so every branch of a phase is queued on a stream of its own (graph branches under capture).  The
+// kernels of a step are short and mostly far too small to fill 148 SMs: side by side they take little longer than one of
+// them.  us a step, groups of four one after the other -> side by side: sixteen shards of the demo's size 148 -> 62, eight of
+// 256 x 512 x 100 L1 scores 122 -> 109, eight of 512 x 768 with features 401 -> 366, eight of TransH at that size 792 -> 707.
+// Only with one process: the hand-over counters between processes count the blocks of one kernel at a time.
 void Engine::shards_fork() {
     if (!shards_beside()) return;
     KGE_CUDA(cudaEventRecord(ev_fork_, stream_));
-    for (unsigned l = 1; l < n_local_; ++l) KGE_CUDA(cudaStreamWaitEvent(shard_streams_[l], ev_fork_, 0));
+    for (unsigned l = 1; l < branches_; ++l) KGE_CUDA(cudaStreamWaitEvent(shard_streams_[l], ev_fork_, 0));
 }
 void Engine::shards_join() {
     if (!shards_beside()) return;
-    for (unsigned l = 1; l < n_local_; ++l) {
+    for (unsigned l = 1; l < branches_; ++l) {
         KGE_CUDA(cudaEventRecord(ev_shard_[l], shard_streams_[l]));
         KGE_CUDA(cudaStreamWaitEvent(stream_, ev_shard_[l], 0));
     }
@@ -1730,7 +1731,9 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
     const bool fused_route = F > 0 && (cfg_.score_fn == SCORE_TRANSE || cfg_.score_fn == SCORE_DISTMULT) && !dropout_on();
     // rows with many lookups are routed in parts by a kernel of their own, which then publishes the tails
     const bool heavy_route = fused_route && split_popular_rows_ && heavy_route_;
+    shards_fork();
     for (unsigned l0 = 0; l0 < n_local_; l0 += group_) {
+        const ShardScope on_stream(*this, l0 / group_);
         const unsigned n = std::min(group_, n_local_ - l0);
         if (F > 0) {
             tc::RouteArgs routes[kShardBatch] = {};
@@ -1783,9 +1786,12 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
         if (!fused_route) launch_lookup(l0, n, step);
         if (cfg_.regularised()) launch_regularise(l0, n, step);
     }
+    shards_join();
     KGE_CUDA(cudaGetLastError());
 
+    shards_fork();
     for (unsigned l0 = 0; l0 < n_local_; l0 += group_) {
+        const ShardScope on_stream(*this, l0 / group_);
         const unsigned n = std::min(group_, n_local_ - l0);
         // 2. scores
         if (transh) {
@@ -1854,6 +1860,7 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
         }
         if (cfg_.score_fn != SCORE_TRANSE) launch_lookup_bwd(l0, n, step);
     }
+    shards_join();
     KGE_CUDA(cudaGetLastError());
 
     // 5. segment sums + row-wise Adam, and the relation rows of the dense gradient
@@ -1862,7 +1869,9 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
     // with the table's own rows nothing reads the hidden rows' gradients but kge_debug_fetch, which shows the last step's
     const bool keep_d_hid = !direct_rows_ || step + 1 == cfg_.n_step;
     const bool extras = cfg_.regularised() || dropout_on();
+    shards_fork();
     for (unsigned l0 = 0; l0 < n_local_; l0 += group_) {
+        const ShardScope on_stream(*this, l0 / group_);
         const unsigned n = std::min(group_, n_local_ - l0);
         ShardArgs<EntityShard> shards{};
         for (unsigned i = 0; i < n; ++i) shards.s[i] = entity_shard(l0 + i, step, keep_d_hid);
@@ -1883,10 +1892,12 @@ void Engine::launch_step_planes(unsigned step, const LossParams& lp, float norma
     // slices of each shard's partial dense gradient
     const unsigned at_once = fuse_dense_ ? n_local_ : group_;
     for (unsigned l0 = 0; l0 < n_local_; l0 += at_once) {
+        const ShardScope on_stream(*this, l0 / group_);
         const unsigned n = std::min(at_once, n_local_ - l0);
         if (F > 0) launch_projection_bwd(l0, n, step, fuse_dense_);
         else launch_exchange_signal(XCHG_DENSE_PARTIALS);  // the relation rows of the entity update are all there is
     }
+    shards_join();
     KGE_CUDA(cudaGetLastError());
     if (gather_ahead && !gather_beside) launch_gather(step + 1, stream_);
     // 7. dense parameters: reduce over shards, Adam on the owned rows, new values and their lower planes into every replica

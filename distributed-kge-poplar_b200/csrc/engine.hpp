@@ -230,12 +230,13 @@ class Engine {
     bool direct_rows_ = false;        // and so does the row update: no gathered copy, no hidden rows
     bool planes_ = false;             // the step of batched launches, its contractions on the plane-fed tensor-core kernel
     unsigned group_ = 1;              // local shards of one launch
+    unsigned branches_ = 1;           // parts of a phase that run side by side, on streams of their own: groups of shards, or shards
     bool alone_ = false;              // no two shards' launches run side by side, on streams of their own
     unsigned score_ld_ = 0;           // floats between rows of scores, coefficients and TransH's pair matrices
     bool bf16_planes_ = false;        // scores and their gradients multiply bfloat16 copies of their operands
     uint32_t feat_stride_ = 0;        // floats per row of the widened / lower feature planes
     cudaEvent_t ev_fork_ = nullptr, ev_join_[2] = {nullptr, nullptr};
-    // One stream per local shard (the first one is stream_ itself) while steps are being queued; empty where the shards run one after the other.
+    // One stream per branch (the first one is stream_ itself) while steps are being queued; empty where there is one branch.
     std::vector<cudaStream_t> shard_streams_;
     std::vector<cudaEvent_t> ev_shard_;
     bool shards_beside() const { return !shard_streams_.empty() && !kernel_timing_; }
@@ -252,11 +253,11 @@ class Engine {
        private:
         Engine& engine_;
     };
-    // While alive, what the engine launches goes to local shard l's stream.
+    // While alive, what the engine launches goes to a branch's stream.
     class ShardScope {
        public:
-        ShardScope(Engine& e, unsigned l) : engine_(e), saved_(e.stream_) {
-            if (l > 0 && e.shards_beside()) e.stream_ = e.shard_streams_[l];
+        ShardScope(Engine& e, unsigned branch) : engine_(e), saved_(e.stream_) {
+            if (branch > 0 && e.shards_beside()) e.stream_ = e.shard_streams_[branch];
         }
         ~ShardScope() { engine_.stream_ = saved_; }
         ShardScope(const ShardScope&) = delete;

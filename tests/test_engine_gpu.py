@@ -146,6 +146,10 @@ CASES = {
                                                entity_feature_size=24, batch_size=32, a2a_size=24, score_fn="TransE",
                                                distance_fn="L2", gamma=10.0, loss_type="softmax", correction_weight=1.0),
                                 seed=30, feature_dtype="float16", settings={"execution.l2_contraction": True}),
+    # more shards than a launch takes: a group of four and one by itself, side by side
+    "five_shards": dict(cfg=StepConfig(n_shard=5, n_entity=200, n_relation_type=10, embedding_size=16, entity_feature_size=10,
+                                       batch_size=10, a2a_size=6, score_fn="TransE", distance_fn="L2", gamma=6.0,
+                                       loss_type="softmax", correction_weight=1.0), seed=32, feature_dtype="float16"),
     "single_shard": dict(cfg=StepConfig(n_shard=1, n_entity=400, n_relation_type=5, embedding_size=64,
                                         entity_feature_size=32, batch_size=64, a2a_size=96, score_fn="TransE",
                                         distance_fn="L2", gamma=10.0, loss_type="softmax", correction_weight=1.0),
@@ -648,11 +652,12 @@ def test_bf16_values_with_float32_optimiser_state(name):
     engine.close()
 
 
-@pytest.mark.parametrize("name,tensor_cores", [("config1_transe_l1", True), ("config1_transe_l1", False), ("ragged_sizes", True), ("mlp_shared", True)])
+@pytest.mark.parametrize("name,tensor_cores", [("config1_transe_l1", True), ("config1_transe_l1", False), ("ragged_sizes", True), ("mlp_shared", True),
+                                               ("five_shards", True)])
 def test_engines_on_two_threads_capture_their_first_runs_side_by_side(name, tensor_cores):
-    """Two engines with several shards record their first program runs at the same time: the step of batched launches and (all
-    cases but the first) that of separate kernels, whose captures have branches on streams that a pool lends to both.  The
-    results are those of the same runs one after the other, bit for bit."""
+    """Two engines with several shards record their first program runs at the same time: the step of batched launches and (the
+    next three cases) that of separate kernels.  All captures but the first case's have branches on streams that a pool lends to
+    both.  The results are those of the same runs one after the other, bit for bit."""
     import threading
 
     def fresh(i):
