@@ -38,6 +38,8 @@ enum LossFn : int { LOSS_LOGSIGMOID = 0, LOSS_SOFTMAX = 1 };
 
 // What belongs to each of the shards of one process that a launch works on, one per blockIdx.y (.z where y is taken).  The
 // kernels of a step are short and mostly far too small to fill 148 SMs, so the shards of a process share every launch.
+// More shards go in groups of so many, side by side on streams (Engine::shards_fork).  Four: a contraction's parameters are 8 KB
+// with that many, which every launch copies; larger groups have not been measured.
 constexpr int kShardBatch = 4;
 template <class A>
 struct ShardArgs {
