@@ -1106,11 +1106,12 @@ Engine::ShardStreams::~ShardStreams() {
 // every graph but the first (a single step) is captured and instantiated while its predecessor runs on the GPU.  That is
 // an engine's second run; the first goes out as plain launches, at about 3 us of host time each, while a graph costs 12 us
 // per kernel in a chain and up to 22 us among the branches of several shards (capture 1, instantiation 9 to 19, upload 2).
-// Milliseconds of an engine's first / second / later run, graphs made in the first and in the second:
-//   demo preset, 5 steps of 2 shards   1.45 / 0.31 / 0.29    0.58 / 1.46 / 0.29
-//   4 shards of TransE-L1, 20 steps    13.8 / 1.95 / 1.91    2.75 / 13.1 / 1.92
-//   2 shards of the headline, 20       7.36 / 3.66 / 2.98    4.26 / 7.14 / 3.00
-//   headline model, 100 steps          16.9 / 8.36 / 7.79    9.08 / 15.4 / 7.80
+// Milliseconds of an engine's first / second / later run, graphs made in the first and in the second (with a stream per shard),
+// and now that the shards share launches:
+//   demo preset, 5 steps of 2 shards   1.45 / 0.31 / 0.29    0.58 / 1.46 / 0.29    0.25 / 0.73 / 0.19
+//   4 shards of TransE-L1, 20 steps    13.8 / 1.95 / 1.91    2.75 / 13.1 / 1.92    1.37 / 1.54 / 1.26
+//   2 shards of the headline, 20       7.36 / 3.66 / 2.98    4.26 / 7.14 / 3.00    2.34 / 3.71 / 2.22
+//   headline model, 100 steps          16.9 / 8.36 / 7.79    9.08 / 15.4 / 7.80    7.53 / 14.6 / 7.21
 void Engine::launch_step_graphs() {
     if (graphs_.empty()) {
         unsigned length = 1;

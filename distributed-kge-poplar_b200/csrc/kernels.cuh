@@ -463,8 +463,8 @@ __global__ void __launch_bounds__(128) k_score(const __grid_constant__ ShardArgs
 // operands into its own part of shared memory (asynchronous 16-byte copies, row-major with a stride of 36 floats, which
 // keeps the 128-bit reads below free of bank conflicts), one ahead of the one it adds up in register tiles of 4 x NB per lane.
 // A chunk is summed by itself (with the chunk eight further on, and so on), and the chunks' sums are added in order at the
-// end: the order is part of an L1 model's result (see k_pair_bwd).  Bound by the FP32 pipe, two instructions per pair of
-// elements, and by the operands' way from L2, of which wider tiles need less; the width is chosen so that the blocks come to
+// end: the order is part of an L1 model's result (see k_pair_bwd).  Bound by FP32 issue, two instructions per pair of
+// elements (66 % of the slots of the SMs that have a block), and by the operands' way from L2, of which wider tiles need less; the width is chosen so that the blocks come to
 // whole waves of 148.  512 x 768 x 256 L2 scores: 13.8 us back to back with 48 columns a block, 16.4 with 64, 17.9 with 32.
 // With 32 x 32 outputs per block, its 8 warps dividing k and no chunk ahead, steps took (us, before -> after) TransE-L2 at that
 // size 72.6 -> 71.3, two shards of it 113.2 -> 109.6, RotatE-L2 256 x 1536 x 256 86.1 -> 82.9, four shards of 256 x 512 x 100
@@ -1101,8 +1101,8 @@ __device__ __forceinline__ void store_pair(float* __restrict__ row, int k, int D
 // blocks enough for it.  Two L1 terms are a packed difference, two coefficients with the sign flipped by it, the smallest
 // magnitude so far and a packed sum: five instructions, where clamped products for the signs took eight.  A chunk in which
 // a difference was 0 or NaN, whose sign is 0 (a few per million terms of float32 values: too few to matter, and some in every
-// launch), is added up again with those products.  Bound by shared memory's wavefronts and by what is left uneven: blocks with
-// the longer sums start first, and two blocks per SM, not three or four, because a dependent launch's blocks pile up where
+// launch), is added up again with those products.  Bound by instruction issue (four shards of 256 x 512 x 100: 68 % of the slots,
+// the FP32 pipe 41 % and shared memory's wavefronts 45 % of the time) and by what is left uneven: blocks with the longer sums start first, and two blocks per SM, not three or four, because a dependent launch's blocks pile up where
 // the kernel in front ends first (four shards of 256 x 512 x 100: 31 us, 43 and 56 with three and four blocks; 48 before
 // the three changes, when the blocks of a shard's two problems followed each other).  Four rows per warp: 51 us, too few
 // warps.  Tried and slower: threads dealt out over (rows, pairs of columns) without gaps, bulk copies of row pieces for
